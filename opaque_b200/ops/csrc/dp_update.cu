@@ -11,6 +11,8 @@
 // receives noise exactly once.
 #include <string.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "api.h"
 
@@ -170,167 +172,177 @@ struct ShardStepParams {
   const int* status;       // non-zero: a bounded wait expired earlier in this step; the kernel does nothing
 };
 
-__device__ __forceinline__ void ld8(const float* src, float* dst) {
-  *reinterpret_cast<float4*>(dst) = *reinterpret_cast<const float4*>(src);
-  *reinterpret_cast<float4*>(dst + 4) = *reinterpret_cast<const float4*>(src + 4);
+// V consecutive fp32 values (V = 4 or 8) as 16-byte accesses.  The state streams through once per step, so loads and
+// stores carry the evict-first hint: the bf16 weights of the next forward pass are what L2 should keep.
+template <int V>
+__device__ __forceinline__ void ldv(const float* src, float* dst) {
+#pragma unroll
+  for (int i = 0; i < V; i += 4) *reinterpret_cast<float4*>(dst + i) = __ldcs(reinterpret_cast<const float4*>(src + i));
 }
-__device__ __forceinline__ void st8(float* dst, const float* src) {
-  *reinterpret_cast<float4*>(dst) = *reinterpret_cast<const float4*>(src);
-  *reinterpret_cast<float4*>(dst + 4) = *reinterpret_cast<const float4*>(src + 4);
+template <int V>
+__device__ __forceinline__ void stv(float* dst, const float* src) {
+#pragma unroll
+  for (int i = 0; i < V; i += 4) __stcs(reinterpret_cast<float4*>(dst + i), *reinterpret_cast<const float4*>(src + i));
 }
 
-// Correlated-noise update for 8 consecutive coordinates with 32-byte vector accesses to the state buffers.
-// z: this step's raw N(0,1) draws; x: the correlated noise to add (row t of C^{-1} Z).
-__device__ __forceinline__ void ftrl_apply8(const ShardStepParams& p, long long base, const float* z, float* x) {
+// Correlated-noise update for V consecutive coordinates with vector accesses to the state buffers.
+// z: this step's raw N(0,1) draws; x: the correlated noise to add (row t of C^{-1} Z).  `keep` holds the first four BLT
+// buffers, which the caller loaded before it drew the noise.
+template <int V>
+__device__ __forceinline__ void ftrl_apply(const ShardStepParams& p, long long base, const float (*keep)[V], const float* z, float* x) {
   float* st = p.ftrl_state + base;
   if (p.ftrl_mode == 1) {
     // buffered-linear-Toeplitz C:  x = z - sum_b s_b S_b ;  S_b <- d_b S_b + x   (first four buffers stay in registers)
-    float keep[4][8], corr[8];
+    float corr[V];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) corr[j] = 0.f;
+    for (int j = 0; j < V; ++j) corr[j] = 0.f;
 #pragma unroll
     for (int b = 0; b < 8; ++b) {
       if (b < p.nbuf) {
-        float t[8];
-        ld8(st + b * p.n, t);
+        float t[V];
+        if (b < 4) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          corr[j] += p.coef[b] * t[j];
-          if (b < 4) keep[b][j] = t[j];
+          for (int j = 0; j < V; ++j) t[j] = keep[b][j];
+        } else {
+          ldv<V>(st + b * p.n, t);
         }
+#pragma unroll
+        for (int j = 0; j < V; ++j) corr[j] += p.coef[b] * t[j];
       }
     }
     for (int b = 8; b < p.nbuf; ++b) {          // beyond the unrolled eight: same recurrence, buffers re-read below
-      float t[8];
-      ld8(st + b * p.n, t);
+      float t[V];
+      ldv<V>(st + b * p.n, t);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) corr[j] += p.coef[b] * t[j];
+      for (int j = 0; j < V; ++j) corr[j] += p.coef[b] * t[j];
     }
 #pragma unroll
-    for (int j = 0; j < 8; ++j) x[j] = z[j] - corr[j];
+    for (int j = 0; j < V; ++j) x[j] = z[j] - corr[j];
 #pragma unroll
     for (int b = 0; b < 8; ++b) {
       if (b < p.nbuf) {
-        float t[8];
+        float t[V];
         if (b < 4) {
 #pragma unroll
-          for (int j = 0; j < 8; ++j) t[j] = keep[b][j];
+          for (int j = 0; j < V; ++j) t[j] = keep[b][j];
         } else {
-          ld8(st + b * p.n, t);
+          ldv<V>(st + b * p.n, t);
         }
 #pragma unroll
-        for (int j = 0; j < 8; ++j) t[j] = p.coef[p.nbuf + b] * t[j] + x[j];
-        st8(st + b * p.n, t);
+        for (int j = 0; j < V; ++j) t[j] = p.coef[p.nbuf + b] * t[j] + x[j];
+        stv<V>(st + b * p.n, t);
       }
     }
     for (int b = 8; b < p.nbuf; ++b) {
-      float t[8];
-      ld8(st + b * p.n, t);
+      float t[V];
+      ldv<V>(st + b * p.n, t);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) t[j] = p.coef[p.nbuf + b] * t[j] + x[j];
-      st8(st + b * p.n, t);
+      for (int j = 0; j < V; ++j) t[j] = p.coef[p.nbuf + b] * t[j] + x[j];
+      stv<V>(st + b * p.n, t);
     }
   } else {
     // ring of the previous nbuf values: mode 2 keeps outputs (banded C, IIR), mode 3 keeps raw draws (FIR)
-    float acc[8];
+    float acc[V];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[j] = (p.ftrl_mode == 3) ? p.coef[0] * z[j] : 0.f;
+    for (int j = 0; j < V; ++j) acc[j] = (p.ftrl_mode == 3) ? p.coef[0] * z[j] : 0.f;
 #pragma unroll
     for (int b = 1; b <= 8; ++b) {
       if (b <= p.nbuf) {
         int slot = p.ring_head - b;
         if (slot < 0) slot += p.nbuf;
-        float t[8];
-        ld8(st + slot * p.n, t);
+        float t[V];
+        ldv<V>(st + slot * p.n, t);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[j] += p.coef[b] * t[j];
+        for (int j = 0; j < V; ++j) acc[j] += p.coef[b] * t[j];
       }
     }
     for (int b = 9; b <= p.nbuf; ++b) {         // longer histories: a plain loop over the ring
       int slot = p.ring_head - b;
       if (slot < 0) slot += p.nbuf;
-      float t[8];
-      ld8(st + slot * p.n, t);
+      float t[V];
+      ldv<V>(st + slot * p.n, t);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) acc[j] += p.coef[b] * t[j];
+      for (int j = 0; j < V; ++j) acc[j] += p.coef[b] * t[j];
     }
     if (p.ftrl_mode == 2) {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) x[j] = (z[j] - acc[j]) / p.coef[0];
-      st8(st + p.ring_head * p.n, x);
+      for (int j = 0; j < V; ++j) x[j] = (z[j] - acc[j]) / p.coef[0];
+      stv<V>(st + p.ring_head * p.n, x);
     } else {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) x[j] = acc[j];
-      st8(st + p.ring_head * p.n, z);
+      for (int j = 0; j < V; ++j) x[j] = acc[j];
+      stv<V>(st + p.ring_head * p.n, z);
     }
   }
 }
 
-// Pull form of the gradient read: this shard's 8 coordinates from every rank's accumulation buffer, summed in rank
-// order.  Four ranks' 32-byte loads are in flight per thread before the first add (more would spill registers).
-__device__ __forceinline__ void pull_grad8(const ShardStepParams& p, long long base, float* g8) {
+// Pull form of the gradient read: this shard's V coordinates from every rank's accumulation buffer, summed in rank
+// order.  Four ranks' loads are in flight per thread before the first add (more would spill registers).
+template <int V>
+__device__ __forceinline__ void pull_grad(const ShardStepParams& p, long long base, float* g) {
 #pragma unroll
-  for (int j = 0; j < 8; ++j) g8[j] = 0.f;
+  for (int j = 0; j < V; ++j) g[j] = 0.f;
   for (int r0 = 0; r0 < p.world; r0 += 4) {
-    float4 a[4], b[4];
+    float4 a[4][V / 4];
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       if (r0 + r < p.world) {
         const float4* src = reinterpret_cast<const float4*>(p.peer_grad[r0 + r] + p.global_offset + base);
-        a[r] = __ldcg(src);
-        b[r] = __ldcg(src + 1);
+#pragma unroll
+        for (int i = 0; i < V / 4; ++i) a[r][i] = __ldcg(src + i);
       }
     }
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       if (r0 + r < p.world) {
-        g8[0] += a[r].x; g8[1] += a[r].y; g8[2] += a[r].z; g8[3] += a[r].w;
-        g8[4] += b[r].x; g8[5] += b[r].y; g8[6] += b[r].z; g8[7] += b[r].w;
+#pragma unroll
+        for (int i = 0; i < V / 4; ++i) {
+          g[4 * i] += a[r][i].x; g[4 * i + 1] += a[r][i].y; g[4 * i + 2] += a[r][i].z; g[4 * i + 3] += a[r][i].w;
+        }
       }
     }
   }
 }
 
-// PULL selects the gradient source at compile time, so the ordinary form keeps its register allocation.  FTRL = false is
-// the iid-noise step (DP-SGD): without the correlated-noise state it fits three blocks per SM, which this latency-bound
-// kernel (Philox rounds, accurate log / sincos / sqrt / divisions in a dependent chain) turns into bandwidth.
-template <bool PULL, bool FTRL>
-__global__ void __launch_bounds__(256, FTRL ? 2 : 3)
+// PULL selects the gradient source at compile time, so the ordinary form keeps its register allocation; FTRL = false is
+// the iid-noise step (DP-SGD).  V coordinates per thread: 4 when every store stays on this GPU (more warps in flight), 8
+// where parameters go to peers (one 16-byte store per peer and thread).
+//
+// Bound by memory: 34 B per coordinate iid, + 8 B per noise buffer.  The arithmetic (Philox rounds, accurate log / sincos
+// / sqrt / divisions, about 160 instructions per coordinate) takes about half that time, so the two must overlap: every
+// load of a thread is issued BEFORE its noise is drawn.  (With the loads behind the noise and 8 coordinates a thread the two
+// phases added up.)  Measured: 749 M coordinates with four BLT buffers 13.5 -> 9.0 ms, 124 M coordinates iid 0.99 -> 0.77 ms,
+// 5.5 TB/s both.
+template <bool PULL, bool FTRL, int V>
+__global__ void __launch_bounds__(256, V == 4 ? (FTRL ? 3 : 4) : (FTRL ? 2 : 3))
 shard_step_kernel(const ShardStepParams p) {
   // The gradient barrier before this kernel may have given up (status != 0): the shard is then not fully reduced, and
   // adding noise to it, stepping and clearing it would release and apply a partial sum.  Leave every buffer untouched;
   // the host reads the status word after the step and raises.
   if (p.status != nullptr && *reinterpret_cast<const volatile int*>(p.status) != 0) return;
-  // each thread owns 8 consecutive coordinates (two Philox blocks, one 16-byte bf16 store per peer)
-  const long long nv = (p.n + 7) >> 3;
+  const long long nv = (p.n + V - 1) / V;
   for (long long i = blockIdx.x * 256LL + threadIdx.x; i < nv; i += gridDim.x * 256LL) {
-    const long long base = i << 3;
-    const bool full = base + 8 <= p.n;
-    float z[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    if (p.noise_std != 0.f) {
-      const uint64_t blk = static_cast<uint64_t>((p.global_offset + base) >> 2);
-      const float4 r0 = philox_normal4(p.seed, blk, 0u), r1 = philox_normal4(p.seed, blk + 1, 0u);
-      z[0] = r0.x; z[1] = r0.y; z[2] = r0.z; z[3] = r0.w;
-      z[4] = r1.x; z[5] = r1.y; z[6] = r1.z; z[7] = r1.w;
+    const long long base = i * V;
+    const bool full = base + V <= p.n;
+    float gv[V], wv[V], mv[V], vv[V];
+    const bool vec_ftrl = FTRL && full && p.ftrl_mode != 0 && ((p.n & 3) == 0);
+    float keep[FTRL ? 4 : 1][V];
+    if (FTRL && vec_ftrl && p.ftrl_mode == 1) {
+#pragma unroll
+      for (int b = 0; b < (FTRL ? 4 : 1); ++b)
+        if (b < p.nbuf) ldv<V>(p.ftrl_state + b * p.n + base, keep[b]);
     }
-    float g8[8], w8[8], m8[8], v8[8];
     if (full) {
-      if (PULL) {
-        pull_grad8(p, base, g8);
-      } else {
-        *reinterpret_cast<float4*>(g8) = *reinterpret_cast<const float4*>(p.grad + base);
-        *reinterpret_cast<float4*>(g8 + 4) = *reinterpret_cast<const float4*>(p.grad + base + 4);
-      }
+      if (PULL) pull_grad<V>(p, base, gv);
+      else ldv<V>(p.grad + base, gv);
       if (!p.skip_update) {
-        *reinterpret_cast<float4*>(w8) = *reinterpret_cast<const float4*>(p.master + base);
-        *reinterpret_cast<float4*>(w8 + 4) = *reinterpret_cast<const float4*>(p.master + base + 4);
-        *reinterpret_cast<float4*>(m8) = *reinterpret_cast<const float4*>(p.m + base);
-        *reinterpret_cast<float4*>(m8 + 4) = *reinterpret_cast<const float4*>(p.m + base + 4);
-        *reinterpret_cast<float4*>(v8) = *reinterpret_cast<const float4*>(p.v + base);
-        *reinterpret_cast<float4*>(v8 + 4) = *reinterpret_cast<const float4*>(p.v + base + 4);
+        ldv<V>(p.master + base, wv);
+        ldv<V>(p.m + base, mv);
+        ldv<V>(p.v + base, vv);
       }
     } else {
-      for (int j = 0; j < 8; ++j) {
+#pragma unroll (PULL ? 1 : V)
+      for (int j = 0; j < V; ++j) {
         const long long k = base + j;
         const bool in = k < p.n;
         float gk = 0.f;
@@ -339,20 +351,32 @@ shard_step_kernel(const ShardStepParams p) {
         } else if (in) {
           gk = p.grad[k];
         }
-        g8[j] = gk;
-        w8[j] = (in && !p.skip_update) ? p.master[k] : 0.f;
-        m8[j] = (in && !p.skip_update) ? p.m[k] : 0.f;
-        v8[j] = (in && !p.skip_update) ? p.v[k] : 0.f;
+        gv[j] = gk;
+        wv[j] = (in && !p.skip_update) ? p.master[k] : 0.f;
+        mv[j] = (in && !p.skip_update) ? p.m[k] : 0.f;
+        vv[j] = (in && !p.skip_update) ? p.v[k] : 0.f;
       }
     }
-    float out8[8];
-    float x8[8];
-    const bool vec_ftrl = FTRL && full && p.ftrl_mode != 0 && ((p.n & 3) == 0);
-    if (vec_ftrl) ftrl_apply8(p, base, z, x8);
+    float z[V];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
+    for (int j = 0; j < V; ++j) z[j] = 0.f;
+    if (p.noise_std != 0.f) {
+      const uint64_t blk = static_cast<uint64_t>((p.global_offset + base) >> 2);
+#pragma unroll
+      for (int i4 = 0; i4 < V / 4; ++i4) {
+        const float4 r = philox_normal4(p.seed, blk + i4, 0u);
+        z[4 * i4] = r.x; z[4 * i4 + 1] = r.y; z[4 * i4 + 2] = r.z; z[4 * i4 + 3] = r.w;
+      }
+    }
+    float ov[V];
+    float xv[V];
+    if constexpr (FTRL) {
+      if (vec_ftrl) ftrl_apply<V>(p, base, keep, z, xv);
+    }
+#pragma unroll
+    for (int j = 0; j < V; ++j) {
       const long long k = base + j;
-      float x = vec_ftrl ? x8[j] : z[j];
+      float x = vec_ftrl ? xv[j] : z[j];
       if (FTRL && k < p.n && !vec_ftrl) {
         if (p.ftrl_mode == 1) {
           // row t of C^{-1} Z for a buffered-linear-Toeplitz C:  x = z - sum_b s_b S_b ;  S_b <- d_b S_b + x
@@ -385,73 +409,66 @@ shard_step_kernel(const ShardStepParams p) {
           x = acc;
         }
       }
-      const float g = (g8[j] + p.noise_std * x) * p.inv_normalize;
-      out8[j] = g;
-      float w = w8[j];
+      const float g = (gv[j] + p.noise_std * x) * p.inv_normalize;
+      ov[j] = g;
+      float w = wv[j];
       float ge = g;
       if (!p.decoupled_wd) ge += p.wd * w;
       float u;
       if (p.opt_mode == 0) {
-        const float m = p.b1 * m8[j] + (1.f - p.b1) * ge;
-        const float v = p.b2 * v8[j] + (1.f - p.b2) * ge * ge;
-        m8[j] = m;
-        v8[j] = v;
+        const float m = p.b1 * mv[j] + (1.f - p.b1) * ge;
+        const float v = p.b2 * vv[j] + (1.f - p.b2) * ge * ge;
+        mv[j] = m;
+        vv[j] = v;
         float vh = v / p.bc2;
         const float corrected = vh - p.phi_hat;
         if (corrected > 0.f) vh = corrected;
         u = (m / p.bc1) / (sqrtf(vh) + p.eps);
       } else if (p.opt_mode == 1) {
         // buf <- mu * buf + g (a zero buffer makes the first step buf = g); Nesterov looks ahead by one more mu * buf
-        const float m = p.b1 * m8[j] + ge;
-        m8[j] = m;
+        const float m = p.b1 * mv[j] + ge;
+        mv[j] = m;
         u = p.nesterov ? ge + p.b1 * m : m;
       } else {
-        const float c = p.b1 * m8[j] + (1.f - p.b1) * ge;
+        const float c = p.b1 * mv[j] + (1.f - p.b1) * ge;
         u = c > 0.f ? 1.f : (c < 0.f ? -1.f : 0.f);
-        m8[j] = p.b2 * m8[j] + (1.f - p.b2) * ge;
+        mv[j] = p.b2 * mv[j] + (1.f - p.b2) * ge;
       }
       if (p.decoupled_wd) u += p.wd * w;
-      w8[j] = w - p.lr * u;
+      wv[j] = w - p.lr * u;
     }
-    const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float zero[V] = {};
     if (full) {
-      if (!PULL) {
-        *reinterpret_cast<float4*>(p.grad + base) = zero4;
-        *reinterpret_cast<float4*>(p.grad + base + 4) = zero4;
-      }
-      if (p.noisy_out) {
-        *reinterpret_cast<float4*>(p.noisy_out + base) = *reinterpret_cast<const float4*>(out8);
-        *reinterpret_cast<float4*>(p.noisy_out + base + 4) = *reinterpret_cast<const float4*>(out8 + 4);
-      }
+      if (!PULL) stv<V>(p.grad + base, zero);
+      if (p.noisy_out) stv<V>(p.noisy_out + base, ov);
       if (!p.skip_update) {
-        *reinterpret_cast<float4*>(p.master + base) = *reinterpret_cast<const float4*>(w8);
-        *reinterpret_cast<float4*>(p.master + base + 4) = *reinterpret_cast<const float4*>(w8 + 4);
-        *reinterpret_cast<float4*>(p.m + base) = *reinterpret_cast<const float4*>(m8);
-        *reinterpret_cast<float4*>(p.m + base + 4) = *reinterpret_cast<const float4*>(m8 + 4);
-        *reinterpret_cast<float4*>(p.v + base) = *reinterpret_cast<const float4*>(v8);
-        *reinterpret_cast<float4*>(p.v + base + 4) = *reinterpret_cast<const float4*>(v8 + 4);
-        uint4 packed;
+        stv<V>(p.master + base, wv);
+        stv<V>(p.m + base, mv);
+        stv<V>(p.v + base, vv);
+        using Packed = typename std::conditional<V == 8, uint4, uint2>::type;
+        Packed packed;
         __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&packed);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) h[j] = __floats2bfloat162_rn(w8[2 * j], w8[2 * j + 1]);
+        for (int j = 0; j < V / 2; ++j) h[j] = __floats2bfloat162_rn(wv[2 * j], wv[2 * j + 1]);
         if (p.peer_params) {
           for (int r = 0; r < p.world; ++r)
-            *reinterpret_cast<uint4*>(p.peer_params[r] + p.global_offset + base) = packed;
+            *reinterpret_cast<Packed*>(p.peer_params[r] + p.global_offset + base) = packed;
         } else if (p.local_params) {
-          *reinterpret_cast<uint4*>(p.local_params + p.global_offset + base) = packed;
+          *reinterpret_cast<Packed*>(p.local_params + p.global_offset + base) = packed;
         }
       }
     } else {
-      for (int j = 0; j < 8; ++j) {
+#pragma unroll (PULL ? 1 : V)
+      for (int j = 0; j < V; ++j) {
         const long long k = base + j;
-        if (k >= p.n) break;
+        if (k >= p.n) continue;
         if (!PULL) p.grad[k] = 0.f;
-        if (p.noisy_out) p.noisy_out[k] = out8[j];
+        if (p.noisy_out) p.noisy_out[k] = ov[j];
         if (p.skip_update) continue;
-        p.master[k] = w8[j];
-        p.m[k] = m8[j];
-        p.v[k] = v8[j];
-        const __nv_bfloat16 wb = __float2bfloat16_rn(w8[j]);
+        p.master[k] = wv[j];
+        p.m[k] = mv[j];
+        p.v[k] = vv[j];
+        const __nv_bfloat16 wb = __float2bfloat16_rn(wv[j]);
         if (p.peer_params) {
           for (int r = 0; r < p.world; ++r) p.peer_params[r][p.global_offset + k] = wb;
         } else if (p.local_params) {
@@ -577,13 +594,19 @@ extern "C" int ob_shard_step(float* grad, const float* const* peer_grad, float* 
   p.opt_mode = opt_mode; p.nesterov = nesterov;
   if (opt_mode < 0 || opt_mode > 2) return -4;
   p.status = status;
-  const dim3 grid = grid_for((n + 7) / 8, sms);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const bool pull = peer_grad != nullptr, ftrl = ftrl_mode != 0;
-  if (pull && ftrl) shard_step_kernel<true, true><<<grid, 256, 0, st>>>(p);
-  else if (pull) shard_step_kernel<true, false><<<grid, 256, 0, st>>>(p);
-  else if (ftrl) shard_step_kernel<false, true><<<grid, 256, 0, st>>>(p);
-  else shard_step_kernel<false, false><<<grid, 256, 0, st>>>(p);
+  if (pull || peer_params != nullptr) {
+    const dim3 grid = grid_for((n + 7) / 8, sms);
+    if (pull && ftrl) shard_step_kernel<true, true, 8><<<grid, 256, 0, st>>>(p);
+    else if (pull) shard_step_kernel<true, false, 8><<<grid, 256, 0, st>>>(p);
+    else if (ftrl) shard_step_kernel<false, true, 8><<<grid, 256, 0, st>>>(p);
+    else shard_step_kernel<false, false, 8><<<grid, 256, 0, st>>>(p);
+  } else {
+    const dim3 grid = grid_for((n + 3) / 4, sms);
+    if (ftrl) shard_step_kernel<false, true, 4><<<grid, 256, 0, st>>>(p);
+    else shard_step_kernel<false, false, 4><<<grid, 256, 0, st>>>(p);
+  }
   return OB_CHECK_LAUNCH();
 }
 
