@@ -100,6 +100,10 @@ class Capture:
         self.parts, self.seg = held
         self.part_slots: list[str] = []
         self.records: list[tuple] = []
+        # norms of the captured layers, launched together when backward is over: (a, g, accumulator[, ...]).  The operands
+        # stay alive for the weight gradients anyway
+        self.ghost_jobs: list[tuple] = []
+        self.direct_jobs: list[tuple] = []
         self.status = engine.status
         self.direct_elems = sp.direct_elems
 
@@ -117,15 +121,14 @@ class Capture:
         if path == "direct" and self.tokens % 64 == 0 and x2d.shape[0] == self.batch_size * self.tokens \
                 and x2d.stride(1) == 1 and g2d.stride(1) == 1:
             # long sequences on a small layer: the per-example product itself is cheaper than the two Gram matrices
-            ops.direct_norm2(x2d, g2d, self._part(slot.name), self.tokens, status=self.status)
+            self.direct_jobs.append((x2d, g2d, self._part(slot.name)))
         else:
-            ops.ghost_norm(x2d, g2d, self._part(slot.name), self.tokens, status=self.status)
+            self.ghost_jobs.append((x2d, g2d, self._part(slot.name), self.tokens, None, None, None))
         self.records.append(("linear", slot, g2d, x2d))
 
     def add_embedding(self, weight: torch.nn.Parameter, ids: torch.Tensor, g2d: torch.Tensor) -> None:
         slot = self.engine.slot_of(weight)
-        ops.ghost_norm(None, g2d, self._part(slot.name), self.tokens, ids=ids.reshape(-1).to(torch.int32),
-                       status=self.status)
+        self.ghost_jobs.append((None, g2d, self._part(slot.name), self.tokens, ids.reshape(-1).to(torch.int32), None, None))
         self.records.append(("embedding", slot, g2d, ids.reshape(-1).to(torch.int64)))
 
     def add_grouped_linear(self, weight: torch.nn.Parameter, a_rows: torch.Tensor, g_rows: torch.Tensor,
@@ -138,8 +141,7 @@ class Capture:
         slot = self.engine.slot_of(weight)
         E = weight.shape[0]
         seg_out = (torch.arange(seg.numel() - 1, device=seg.device, dtype=torch.int32) % self.batch_size).contiguous()
-        ops.ghost_norm(a_rows, g_rows, self._part(slot.name + "#experts"), tokens, seg_offsets=seg, seg_out=seg_out,
-                       status=self.status)
+        self.ghost_jobs.append((a_rows, g_rows, self._part(slot.name + "#experts"), tokens, None, seg, seg_out))
         groups = torch.zeros(E + 1, dtype=torch.int32, device=seg.device)
         groups[1:] = expert_offs
         self.records.append(("grouped", slot, g_rows, (a_rows, groups, example_of_row)))
@@ -163,19 +165,17 @@ class Capture:
             raise RuntimeError("LoRA factors must be direct parameters of the flat space")
         r, d_in = lora_a.shape
         stride = self.pe.stride(0)
-        ops.wgrad_clip(x2d, q_pad, self.pe, seg_offsets=self.seg, num_groups=self.batch_size, out_offset=sa.offset,
-                       ldm=1, ldn=d_in, n_valid=r, accumulate=False, group_stride=stride, block_n=64,
-                       status=self.status)
-        ops.wgrad_clip(g2d, xa_pad, self.pe, seg_offsets=self.seg, num_groups=self.batch_size, out_offset=sb.offset,
-                       ldm=r, ldn=1, n_valid=r, accumulate=False, group_stride=stride, block_n=64,
-                       status=self.status)
+        common = dict(seg_offsets=self.seg, num_groups=self.batch_size, group_stride=stride, n_valid=r)
+        ops.wgrad_clip_batch([dict(a=x2d, b=q_pad, out_offset=sa.offset, ldm=1, ldn=d_in, **common),
+                              dict(a=g2d, b=xa_pad, out_offset=sb.offset, ldm=r, ldn=1, **common)],
+                             self.pe, accumulate=False, block_n=64, status=self.status)
 
     def add_lora_qkv(self, factors, x2d: torch.Tensor, xa: torch.Tensor, g_parts, q_all: torch.Tensor) -> None:
         """The three LoRA pairs of one attention block: ``factors = ((A_q, B_q), (A_k, B_k), (A_v, B_v))`` sharing ``x2d``.
 
         When the flat space holds ``A_q, A_k, A_v`` back to back (it does, see ``FlatSpace``), their per-example
-        gradients are ONE launch: ``[q_i | k_i | v_i]ᵀ x_i`` is the ``[3r, in]`` block that starts at ``A_q``'s offset,
-        and ``x`` is read once instead of three times.  The ``dB`` products have different left operands and stay separate.
+        gradients are ONE product: ``[q_i | k_i | v_i]ᵀ x_i`` is the ``[3r, in]`` block that starts at ``A_q``'s offset,
+        and ``x`` is read once instead of three times.  The three ``dB`` products share its launch.
         """
         r, d_in = factors[0][0].shape
         slots = [self.engine.slot_of(a) for a, _ in factors]
@@ -186,15 +186,14 @@ class Capture:
                 self.add_lora(a, b, x2d, xa[:, j * r:(j + 1) * r], g_parts[j], q_all[:, j * r:(j + 1) * r])
             return
         stride = self.pe.stride(0)
-        ops.wgrad_clip(x2d, q_all, self.pe, seg_offsets=self.seg, num_groups=self.batch_size, out_offset=slots[0].offset,
-                       ldm=1, ldn=d_in, n_valid=3 * r, accumulate=False, group_stride=stride, block_n=64, status=self.status)
+        common = dict(seg_offsets=self.seg, num_groups=self.batch_size, group_stride=stride)
+        jobs = [dict(a=x2d, b=q_all, out_offset=slots[0].offset, ldm=1, ldn=d_in, n_valid=3 * r, **common)]
         for j, (_, b) in enumerate(factors):
             sb = self.engine.slot_of(b)
             if not sb.direct:
                 raise RuntimeError("LoRA factors must be direct parameters of the flat space")
-            ops.wgrad_clip(g_parts[j], xa[:, j * r:(j + 1) * r], self.pe, seg_offsets=self.seg, num_groups=self.batch_size,
-                           out_offset=sb.offset, ldm=r, ldn=1, n_valid=r, accumulate=False, group_stride=stride, block_n=64,
-                           status=self.status)
+            jobs.append(dict(a=g_parts[j], b=xa[:, j * r:(j + 1) * r], out_offset=sb.offset, ldm=r, ldn=1, n_valid=r, **common))
+        ops.wgrad_clip_batch(jobs, self.pe, accumulate=False, block_n=64, status=self.status)
 
     def _tied_cross_term(self, slot_name: str) -> torch.Tensor | None:
         """``<g_embedding, g_head>`` per example for a weight used as input embedding AND output head.
@@ -247,6 +246,11 @@ class Capture:
         clipped on its own norm to its own threshold; the step's sensitivity is then ``sqrt(Σ C_g²)``.
         """
         eng, sp = self.engine, self.engine.space
+        if self.ghost_jobs:
+            ops.ghost_norm_batch(self.ghost_jobs, status=self.status)
+        if self.direct_jobs:
+            ops.direct_norm2_batch(self.direct_jobs, self.tokens, status=self.status)
+        self.ghost_jobs, self.direct_jobs = [], []
         by_slot: dict[str, list[int]] = {}
         for i, name in enumerate(self.part_slots):
             by_slot.setdefault(name, []).append(i)
@@ -280,29 +284,32 @@ class Capture:
                         expanded[g] = scales[g].repeat_interleave(self.tokens)
                     return expanded[g]
             row_scale = _RowScale()
+            uniform, ragged, narrow = [], [], []          # problems of one launch each
             for kind, slot, g2d, other in self.records:
                 g = label_of(slot.name)
                 if kind == "grouped":
                     a_rows, groups, ex_row = other
                     E, d_out, d_in = slot.shape
-                    ops.wgrad_clip(g2d, a_rows, tgt["out"], row_scale=scales[g].index_select(0, ex_row.long()),
-                                   seg_offsets=groups, num_groups=E, splits=1, out_offset=slot.offset, ldm=d_in, ldn=1,
-                                   accumulate=True, group_stride=d_out * d_in, peer_table=tgt["peer_table"],
-                                   shard_elems=tgt["shard_elems"], status=self.status)
+                    pr = dict(a=g2d, b=a_rows, row_scale=scales[g].index_select(0, ex_row.long()), seg_offsets=groups, num_groups=E,
+                              out_offset=slot.offset, ldm=d_in, group_stride=d_out * d_in)
                 elif kind == "linear":
                     if self.tokens % 64 == 0 and self.tokens >= 128 and g2d.shape[0] == self.batch_size * self.tokens:
                         # uniform examples: factor applied per example in the epilogue, operands untouched
-                        ops.wgrad_clip_per_example(g2d, other, tgt["out"], ex_scale=scales[g], rows_per_example=self.tokens,
-                                                   out_offset=slot.offset, ldm=slot.shape[1], accumulate=True,
-                                                   peer_table=tgt["peer_table"], shard_elems=tgt["shard_elems"],
-                                                   status=self.status)
-                    else:
-                        ops.wgrad_clip(g2d, other, tgt["out"], row_scale=row_scale[g], out_offset=slot.offset,
-                                       ldm=slot.shape[1], ldn=1, accumulate=True, peer_table=tgt["peer_table"],
-                                       shard_elems=tgt["shard_elems"], status=self.status)
+                        uniform.append((g2d, other, scales[g], slot.offset, slot.shape[1]))
+                        continue
+                    pr = dict(a=g2d, b=other, row_scale=row_scale[g], out_offset=slot.offset, ldm=slot.shape[1])
                 else:
                     ops.embedding_wgrad(g2d, other, tgt["out"], row_scale=row_scale[g], flat_offset=slot.offset,
                                         peer_table=tgt["peer_table"], shard_elems=tgt["shard_elems"])
+                    continue
+                (ragged if ops.pick_block_n(pr["b"].shape[1]) == 256 else narrow).append(pr)
+            dest = dict(peer_table=tgt["peer_table"], shard_elems=tgt["shard_elems"], status=self.status)
+            if uniform:
+                ops.wgrad_clip_per_example_batch(uniform, tgt["out"], self.tokens, **dest)
+            if ragged:
+                ops.wgrad_clip_batch(ragged, tgt["out"], **dest)
+            for pr in narrow:                             # layers of at most 128 inputs
+                ops.wgrad_clip(out=tgt["out"], accumulate=True, splits=1 if "seg_offsets" in pr else None, **pr, **dest)
         self.records = []
         if per_group:
             total = torch.sqrt(sum(n ** 2 for n in norms.values()))

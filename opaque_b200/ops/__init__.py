@@ -22,6 +22,7 @@ packages/opaque-optimizers/src/opaque/api/optimizers/_adam.py:120-270):
 from __future__ import annotations
 
 import math
+import struct
 from typing import Sequence
 
 import torch
@@ -69,18 +70,9 @@ def pick_splits(work_tiles: int, rows: int, sms: int, *, max_splits: int | None 
     return best
 
 
-def wgrad_clip(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None, *, row_scale: torch.Tensor | None = None,
-               seg_offsets: torch.Tensor | None = None, num_groups: int = 1, splits: int | None = None,
-               out_offset: int = 0, ldm: int | None = None, ldn: int = 1, n_valid: int = 0, accumulate: bool = True,
-               group_stride: int = 0, group_out_offset: torch.Tensor | None = None,
-               peer_table: torch.Tensor | None = None, shard_elems: int = 0, block_n: int | None = None,
-               status: StatusWord | None = None, wait_budget_s: float = DEFAULT_WAIT_BUDGET_S) -> None:
-    """``flat[out_offset + g_off + m*ldm + n*ldn] (+)= Σ_t s[t]·a[t, m]·b[t, n]`` over each segment.
-
-    ``a`` is ``[T, M]`` (scaled operand, e.g. output gradients), ``b`` is ``[T, N]`` (layer inputs),
-    both bf16 with 16-byte aligned rows.  ``out`` is the flat fp32 destination, or ``None`` with a
-    ``peer_table`` (int64 device tensor of per-rank shard base pointers) and ``shard_elems``.
-    """
+def _check_wgrad(a, b, out, num_groups, splits, out_offset, ldm, ldn, n_valid, accumulate, group_stride, group_out_offset, peer_table,
+                 shard_elems) -> tuple[int, int, int, int]:
+    """Argument checks of :func:`wgrad_clip`; returns ``(T, M, N, ldm)``."""
     _need_bf16(a, b)
     T, M = a.shape
     N = b.shape[1]
@@ -90,11 +82,6 @@ def wgrad_clip(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None, *, ro
         raise ValueError("operands must be row-major")
     if ldm is None:
         ldm = N
-    bn = block_n or pick_block_n(min(N, n_valid) if n_valid else N)
-    sms = lib.sm_count()
-    if splits is None:
-        tiles = num_groups * math.ceil(M / 128) * math.ceil(N / bn)
-        splits = pick_splits(tiles, T // max(num_groups, 1), sms) if accumulate else 1
     if not accumulate and splits != 1:
         raise ValueError("store mode cannot split K")
     n_lim = min(N, n_valid) if n_valid else N
@@ -108,6 +95,63 @@ def wgrad_clip(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None, *, ro
             raise ValueError(f"wgrad_clip would write element {hi} of a destination holding {room}")
     elif peer_table is None or shard_elems <= 0:
         raise ValueError("give either a destination tensor or a peer table with shard_elems")
+    return T, M, N, ldm
+
+
+_WGRAD_DESC, _WGRAD_PE_DESC, _GHOST_DESC = struct.Struct("5Q6q7i4x"), struct.Struct("4Q4q6i"), struct.Struct("6Q3q4i")
+
+
+def _batch_splits(tiles: int, rows: int, max_splits: int | None = None, peer: bool = False) -> int:
+    """K-splits of a launch that holds ``tiles`` output tiles over all of its problems: none once they make four waves
+    (the last, partly filled wave then costs little, and every split adds a pass of reductions over the outputs)."""
+    sms = lib.sm_count()
+    if tiles >= 4 * sms or (peer and tiles * 2 >= sms):
+        return 1
+    return pick_splits(max(tiles, 1), rows, sms, max_splits=max_splits)
+
+
+def wgrad_clip_batch(problems: Sequence[dict], out: torch.Tensor | None, *, accumulate: bool = True, peer_table: torch.Tensor | None = None,
+                     shard_elems: int = 0, block_n: int = 256, status: StatusWord | None = None,
+                     wait_budget_s: float = DEFAULT_WAIT_BUDGET_S) -> None:
+    """Several :func:`wgrad_clip` problems with one destination in one launch (per 64): dictionaries with that function's
+    ``a``, ``b`` and optional ``row_scale``, ``seg_offsets``, ``num_groups``, ``out_offset``, ``ldm``, ``ldn``, ``n_valid``,
+    ``group_stride``.  ``block_n`` is 256 or 64.  K is split (``accumulate`` only, ungrouped problems) when the whole list
+    would leave SMs idle."""
+    tiles = sum(pr.get("num_groups", 1) * math.ceil(pr["a"].shape[1] / 128) * math.ceil(pr["b"].shape[1] / block_n) for pr in problems)
+    jobs = []
+    for pr in problems:
+        a, b, groups = pr["a"], pr["b"], pr.get("num_groups", 1)
+        splits = _batch_splits(tiles, a.shape[0], peer=peer_table is not None) if accumulate and groups == 1 else 1
+        off, gstride, nv, ldn = pr.get("out_offset", 0), pr.get("group_stride", 0), pr.get("n_valid", 0), pr.get("ldn", 1)
+        T, M, N, ldm = _check_wgrad(a, b, out, groups, splits, off, pr.get("ldm"), ldn, nv, accumulate, gstride, None, peer_table, shard_elems)
+        jobs.append((T / (groups * splits), _WGRAD_DESC.pack(
+            a.data_ptr(), b.data_ptr(), lib.ptr(pr.get("row_scale")) or 0, lib.ptr(pr.get("seg_offsets")) or 0, 0, a.stride(0), b.stride(0),
+            gstride, off, ldm, ldn, T, M, N, groups, splits, nv, int(accumulate))))
+    jobs.sort(key=lambda j: -j[0])                       # longest items first: the tail of the launch is made of short ones
+    rc = lib.load().ob_wgrad_clip_batch(b"".join(j[1] for j in jobs), len(jobs), lib.ptr(out), lib.ptr(peer_table), shard_elems, block_n,
+                                        status.ptr() if status else None, wait_budget_s, lib.sm_count(), lib.stream())
+    lib.check(rc, "wgrad_clip_batch")
+
+
+def wgrad_clip(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None, *, row_scale: torch.Tensor | None = None,
+               seg_offsets: torch.Tensor | None = None, num_groups: int = 1, splits: int | None = None,
+               out_offset: int = 0, ldm: int | None = None, ldn: int = 1, n_valid: int = 0, accumulate: bool = True,
+               group_stride: int = 0, group_out_offset: torch.Tensor | None = None,
+               peer_table: torch.Tensor | None = None, shard_elems: int = 0, block_n: int | None = None,
+               status: StatusWord | None = None, wait_budget_s: float = DEFAULT_WAIT_BUDGET_S) -> None:
+    """``flat[out_offset + g_off + m*ldm + n*ldn] (+)= Σ_t s[t]·a[t, m]·b[t, n]`` over each segment.
+
+    ``a`` is ``[T, M]`` (scaled operand, e.g. output gradients), ``b`` is ``[T, N]`` (layer inputs),
+    both bf16 with 16-byte aligned rows.  ``out`` is the flat fp32 destination, or ``None`` with a
+    ``peer_table`` (int64 device tensor of per-rank shard base pointers) and ``shard_elems``.
+    """
+    bn = block_n or pick_block_n(min(b.shape[1], n_valid) if n_valid else b.shape[1])
+    sms = lib.sm_count()
+    if splits is None:
+        tiles = num_groups * math.ceil(a.shape[1] / 128) * math.ceil(b.shape[1] / bn)
+        splits = pick_splits(tiles, a.shape[0] // max(num_groups, 1), sms) if accumulate else 1
+    T, M, N, ldm = _check_wgrad(a, b, out, num_groups, splits, out_offset, ldm, ldn, n_valid, accumulate, group_stride, group_out_offset,
+                                peer_table, shard_elems)
     rc = lib.load().ob_wgrad_clip(
         a.data_ptr(), b.data_ptr(), T, M, N, a.stride(0), b.stride(0), lib.ptr(row_scale), lib.ptr(seg_offsets),
         num_groups, splits, lib.ptr(out), lib.ptr(peer_table), shard_elems, lib.ptr(group_out_offset), group_stride,
@@ -197,6 +241,59 @@ def wgrad_clip_per_example(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor |
     lib.check(rc, "wgrad_clip_per_example")
 
 
+def _check_pe(a, b, rows_per_example) -> tuple[int, int, int, int]:
+    _need_bf16(a, b)
+    T, M = a.shape
+    if b.shape[0] != T or a.stride(1) != 1 or b.stride(1) != 1:
+        raise ValueError("a [T, M] and b [T, N] must be row-major with the same number of rows")
+    if rows_per_example <= 0 or rows_per_example % 64 or T % rows_per_example:
+        raise ValueError("rows_per_example must be a multiple of 64 that divides the number of rows")
+    return T, M, b.shape[1], T // rows_per_example
+
+
+def wgrad_clip_per_example_batch(problems: Sequence[tuple], out: torch.Tensor | None, rows_per_example: int, *,
+                                 peer_table: torch.Tensor | None = None, shard_elems: int = 0, status: StatusWord | None = None,
+                                 wait_budget_s: float = DEFAULT_WAIT_BUDGET_S) -> None:
+    """Several accumulating :func:`wgrad_clip_per_example` problems ``(a, b, ex_scale, out_offset, ldm)`` in one launch (per 64)."""
+    tiles = sum(math.ceil(pr[0].shape[1] / 128) * math.ceil(pr[1].shape[1] / 256) for pr in problems)
+    descs = []
+    for a, b, ex_scale, off, ldm in problems:
+        T, M, N, B = _check_pe(a, b, rows_per_example)
+        if ex_scale is not None and (ex_scale.dtype != torch.float32 or ex_scale.numel() < B or not ex_scale.is_contiguous()):
+            raise ValueError("ex_scale must hold one contiguous fp32 factor per example")
+        if out is not None:
+            if out.dtype != torch.float32:
+                raise TypeError("the destination must be fp32")
+            hi = off + (M - 1) * ldm + N - 1
+            room = out.untyped_storage().nbytes() // 4 - out.storage_offset()
+            if min(off, ldm) < 0 or hi >= room:
+                raise ValueError(f"wgrad_clip_per_example would write element {hi} of a destination holding {room}")
+        elif peer_table is None or shard_elems <= 0:
+            raise ValueError("give either a destination tensor or a peer table with shard_elems")
+        splits = _batch_splits(tiles, T, B, peer_table is not None)
+        descs.append(_WGRAD_PE_DESC.pack(a.data_ptr(), b.data_ptr(), lib.ptr(ex_scale) or 0, 0, a.stride(0), b.stride(0), off, ldm, B,
+                                         rows_per_example, M, N, splits, 1))
+    rc = lib.load().ob_wgrad_clip_pe_batch(b"".join(descs), len(descs), lib.ptr(out), lib.ptr(peer_table), shard_elems,
+                                           status.ptr() if status else None, wait_budget_s, lib.sm_count(), lib.stream())
+    lib.check(rc, "wgrad_clip_per_example_batch")
+
+
+def direct_norm2_batch(problems: Sequence[tuple], rows_per_example: int, *, status: StatusWord | None = None,
+                       wait_budget_s: float = DEFAULT_WAIT_BUDGET_S) -> None:
+    """Several :func:`direct_norm2` problems ``(a, g, norm2)`` in one launch (per 64)."""
+    tiles = sum(math.ceil(pr[0].shape[1] / 128) * math.ceil(pr[1].shape[1] / 256) for pr in problems)
+    descs = []
+    for a, g, norm2 in problems:
+        T, M, N, B = _check_pe(a, g, rows_per_example)
+        if norm2.dtype != torch.float32 or norm2.numel() < B or not norm2.is_contiguous():
+            raise ValueError("norm2 must hold one contiguous fp32 value per example")
+        descs.append(_WGRAD_PE_DESC.pack(a.data_ptr(), g.data_ptr(), 0, norm2.data_ptr(), a.stride(0), g.stride(0), 0, N, B, rows_per_example,
+                                         M, N, _batch_splits(tiles, T, B), 0))
+    rc = lib.load().ob_wgrad_clip_pe_batch(b"".join(descs), len(descs), None, None, 0, status.ptr() if status else None, wait_budget_s,
+                                           lib.sm_count(), lib.stream())
+    lib.check(rc, "direct_norm2_batch")
+
+
 def wgrad_clip_ref(a, b, *, row_scale=None, seg_offsets=None, num_groups=1):
     """fp32 oracle: returns ``[num_groups, M, N]``."""
     af, bf = a.float(), b.float()
@@ -208,17 +305,8 @@ def wgrad_clip_ref(a, b, *, row_scale=None, seg_offsets=None, num_groups=1):
     return torch.stack([af[offs[g]:offs[g + 1]].t() @ bf[offs[g]:offs[g + 1]] for g in range(num_groups)])
 
 
-def ghost_norm(a: torch.Tensor | None, g: torch.Tensor, norm2: torch.Tensor, tokens_per_example: int, *,
-               ids: torch.Tensor | None = None, seg_offsets: torch.Tensor | None = None,
-               seg_out: torch.Tensor | None = None, status: StatusWord | None = None,
-               wait_budget_s: float = DEFAULT_WAIT_BUDGET_S) -> None:
-    """``norm2[i] += ‖A_iᵀ G_i‖_F²`` for every segment i of rows.
-
-    Uniform layout: segment i is rows ``[i·T, (i+1)·T)``.  Ragged layout: ``seg_offsets`` (int32 ``[S+1]``) gives the
-    row range of each segment (none longer than ``tokens_per_example``) and ``seg_out`` (int32 ``[S]``) the
-    accumulator each segment adds to (e.g. the example an (expert, example) group belongs to).
-    With ``ids`` (int32, one per row) the inputs are one-hot rows (embedding layer) and ``a`` is unused.
-    """
+def _check_ghost(a, g, norm2, tokens_per_example, ids, seg_offsets, seg_out):
+    """Argument checks of :func:`ghost_norm`; returns ``(rows, segments, d_in, d_out, input pitch, input pointer)``."""
     _need_bf16(g)
     rows, dg = g.shape
     if seg_offsets is None:
@@ -242,6 +330,35 @@ def ghost_norm(a: torch.Tensor | None, g: torch.Tensor, norm2: torch.Tensor, tok
         if ids.dtype != torch.int32 or ids.numel() != rows:
             raise TypeError("ids must be int32 with one entry per row")
         da, lda, ap = 0, 0, None
+    return rows, B, da, dg, lda, ap
+
+
+def ghost_norm_batch(problems: Sequence[tuple], *, status: StatusWord | None = None, wait_budget_s: float = DEFAULT_WAIT_BUDGET_S) -> None:
+    """Several :func:`ghost_norm` problems ``(a, g, norm2, tokens_per_example, ids, seg_offsets, seg_out)`` in one launch per
+    Gram block shape (and per 64 problems): their items share one work list, longest first."""
+    jobs = []
+    for a, g, norm2, tokens, ids, seg_offsets, seg_out in problems:
+        rows, B, da, dg, lda, ap = _check_ghost(a, g, norm2, tokens, ids, seg_offsets, seg_out)
+        jobs.append((da + dg, _GHOST_DESC.pack(ap or 0, g.data_ptr(), lib.ptr(ids) or 0, norm2.data_ptr(), lib.ptr(seg_offsets) or 0,
+                                               lib.ptr(seg_out) or 0, lda, g.stride(0), rows, B, tokens, da, dg)))
+    jobs.sort(key=lambda j: -j[0])
+    rc = lib.load().ob_ghost_norm_batch(b"".join(j[1] for j in jobs), len(jobs), status.ptr() if status else None, wait_budget_s,
+                                        lib.sm_count(), lib.stream())
+    lib.check(rc, "ghost_norm_batch")
+
+
+def ghost_norm(a: torch.Tensor | None, g: torch.Tensor, norm2: torch.Tensor, tokens_per_example: int, *,
+               ids: torch.Tensor | None = None, seg_offsets: torch.Tensor | None = None,
+               seg_out: torch.Tensor | None = None, status: StatusWord | None = None,
+               wait_budget_s: float = DEFAULT_WAIT_BUDGET_S) -> None:
+    """``norm2[i] += ‖A_iᵀ G_i‖_F²`` for every segment i of rows.
+
+    Uniform layout: segment i is rows ``[i·T, (i+1)·T)``.  Ragged layout: ``seg_offsets`` (int32 ``[S+1]``) gives the
+    row range of each segment (none longer than ``tokens_per_example``) and ``seg_out`` (int32 ``[S]``) the
+    accumulator each segment adds to (e.g. the example an (expert, example) group belongs to).
+    With ``ids`` (int32, one per row) the inputs are one-hot rows (embedding layer) and ``a`` is unused.
+    """
+    rows, B, da, dg, lda, ap = _check_ghost(a, g, norm2, tokens_per_example, ids, seg_offsets, seg_out)
     rc = lib.load().ob_ghost_norm(ap, g.data_ptr(), lib.ptr(ids), B, tokens_per_example, da, dg, lda, g.stride(0),
                                   norm2.data_ptr(), lib.ptr(seg_offsets), lib.ptr(seg_out), rows,
                                   status.ptr() if status else None, wait_budget_s, lib.sm_count(), lib.stream())
@@ -670,7 +787,7 @@ from .functional import (activation, cross_entropy, cross_entropy_ref, fused_add
                          layer_norm, merge_heads3, plain_torch_ops, rms_norm, rms_norm_ref, rope_qk, rope_qk_ref, rope_tables, rows_group_sum_, swiglu)
 
 __all__ = [
-    "gemm", "gemm_pair", "gemm_glu", "gemm_glu_bwd", "direct_norm2", "pick_norm_path", "pick_gemm_kernel", "die_map", "set_die_aware_tiles", "linear_ce_forward", "linear_ce_dlogits_", "gemm_glu_ref", "gemm_ref", "ghost_set_wide", "push_grad_", "wgrad_clip_per_example", "plain_torch_ops", "layer_norm", "activation", "rows_group_sum_", "merge_heads3",
+    "gemm", "gemm_pair", "gemm_glu", "gemm_glu_bwd", "direct_norm2", "pick_norm_path", "pick_gemm_kernel", "die_map", "set_die_aware_tiles", "linear_ce_forward", "linear_ce_dlogits_", "gemm_glu_ref", "gemm_ref", "ghost_set_wide", "push_grad_", "wgrad_clip_per_example", "wgrad_clip_batch", "wgrad_clip_per_example_batch", "direct_norm2_batch", "ghost_norm_batch", "plain_torch_ops", "layer_norm", "activation", "rows_group_sum_", "merge_heads3",
     "DeviceWaitTimeout", "KernelLibraryError", "StatusWord", "clip_weighted_sum", "cross_entropy",
     "cross_entropy_ref", "embedding_wgrad", "fused_add_rms_norm", "geglu", "ghost_norm", "ghost_norm_ref", "glu_ref",
     "philox_normal_add_", "pick_block_n", "pick_splits", "rms_norm", "rms_norm_ref", "rope_qk", "rope_qk_ref",

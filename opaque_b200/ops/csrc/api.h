@@ -26,6 +26,37 @@ int ob_ghost_norm(const void* a, const void* g, const int* ids, int B, int T, in
                   long long ldg, float* norm2, const int* seg, const int* seg_out, long long total_rows, int* status,
                   double wait_budget_s, int num_sms, void* stream);
 
+// Several problems in one launch (host arrays of descriptions; launches hold up to 64): the layers of a backward pass
+// share one work list.  Fields as in the single calls above; put problems with more work per item first.
+typedef struct {
+  const void *a, *g;
+  const int* ids;
+  float* norm2;
+  const int *seg, *seg_out;
+  long long lda, ldg, total_rows;
+  int B, T, Da, Dg;
+} ob_ghost_desc;
+typedef struct {
+  const void *a, *b;
+  const float* row_scale;
+  const int* seg_offsets;
+  const long long* group_out_offset;
+  long long lda, ldb, group_stride, out_offset, ldm, ldn;
+  int T, M, N, num_groups, splits, n_valid, accumulate;
+} ob_wgrad_desc;
+typedef struct {
+  const void *a, *b;
+  const float* ex_scale;
+  float* norm2;
+  long long lda, ldb, out_offset, ldm;
+  int num_examples, ex_rows, M, N, splits, accumulate;
+} ob_wgrad_pe_desc;
+int ob_ghost_norm_batch(const ob_ghost_desc* descs, int count, int* status, double wait_budget_s, int num_sms, void* stream);
+int ob_wgrad_clip_batch(const ob_wgrad_desc* descs, int count, float* out, float* const* peer_out, long long shard_elems,
+                        int block_n, int* status, double wait_budget_s, int num_sms, void* stream);
+int ob_wgrad_clip_pe_batch(const ob_wgrad_pe_desc* descs, int count, float* out, float* const* peer_out,
+                           long long shard_elems, int* status, double wait_budget_s, int num_sms, void* stream);
+
 // D[M, N] = A[M, K1] op(B) + A2[M, K2] B2[N, K2]^T + bias, bf16 in / bf16 out, fp32 accumulation.  b_kn = 0: B is
 // [N, K1] row-major (per group: [groups * N, K1]); b_kn = 1: B is [K1, N] row-major (per group: [groups * K1, N]).
 // group_offs (int32 device array [num_groups + 1]) switches on the grouped mode: rows [offs[e], offs[e+1]) use slab e.

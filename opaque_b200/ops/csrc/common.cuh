@@ -204,6 +204,30 @@ __host__ __device__ constexpr uint32_t make_idesc_bf16(int m, int n, int a_mn_ma
 }
 
 // ---------------------------------------------------------------------------------------------
+// Several problems of one kernel in one launch.  The persistent CTAs walk ONE work list: problem i owns items
+// [start[i], start[i + 1]).  A layer of a small model has fewer items than the chip has SMs; the layers of a backward pass
+// together fill it, and cost one launch.  The whole struct is a kernel parameter (tensor maps must be, or live in global
+// memory that a copy would have to fill first); 64 problems stay below the 32 764-byte parameter limit.
+constexpr int BATCH_CAP = 64;
+template <class Params, int CAP>
+struct alignas(64) TmaBatch {
+  CUtensorMap map_a[CAP];
+  CUtensorMap map_b[CAP];
+  Params p[CAP];
+  int start[CAP + 1];
+  int* status;
+  unsigned long long wait_budget_ns;
+  int count;
+  __device__ __forceinline__ int total() const { return start[CAP == 1 ? 1 : count]; }
+  // problem of item w; `cur` is the caller's monotone cursor
+  __device__ __forceinline__ int seek(int w, int cur) const {
+    if (CAP > 1)
+      while (w >= start[cur + 1]) ++cur;
+    return cur;
+  }
+};
+
+// ---------------------------------------------------------------------------------------------
 // Philox-4x32-10 (Salmon et al.), counter-based: same (key, counter) -> same 4 words.
 struct Philox4 {
   uint32_t x, y, z, w;

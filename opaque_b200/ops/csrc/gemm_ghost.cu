@@ -38,8 +38,19 @@ struct GhostParams {
   const int* seg;        // [B + 1] row offsets of ragged segments, or nullptr (segment b = rows [b*T, (b+1)*T))
   const int* seg_out;    // [B] accumulator index of every segment, or nullptr (identity)
   float* norm2;          // accumulated with atomics
-  int* status;
-  unsigned long long wait_budget_ns;
+};
+
+// tile counts of one problem
+struct GhostShape {
+  int nt, ncb, pairs, wide_items, ka, num_kb;
+  __host__ __device__ __forceinline__ explicit GhostShape(const GhostParams& p) {
+    nt = (p.T + GH_TILE - 1) / GH_TILE;
+    ncb = (nt + 1) / 2;
+    pairs = nt * (nt + 1) / 2;
+    wide_items = nt * ncb - (nt / 2) * (nt / 2) + ((nt & 1) ? 0 : nt / 2);   // sum over row blocks tb of ncb - tb / 2
+    ka = p.ids ? 0 : (p.Da + GH_BLOCK_K - 1) / GH_BLOCK_K;
+    num_kb = ka + (p.Dg + GH_BLOCK_K - 1) / GH_BLOCK_K;
+  }
 };
 
 struct GhostItem {
@@ -60,9 +71,9 @@ __device__ __forceinline__ GhostItem ghost_decode(int w, int pairs, int nt) {
   return it;
 }
 
+template <int CAP>
 __global__ void __launch_bounds__(GH_THREADS, 1)
-ghost_norm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_g,
-                  const GhostParams p) {
+ghost_norm_kernel(const __grid_constant__ TmaBatch<GhostParams, CAP> b) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + GH_STAGES * GH_STAGE_BYTES);
@@ -74,13 +85,8 @@ ghost_norm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nt = (p.T + GH_TILE - 1) / GH_TILE;
-  const int pairs = nt * (nt + 1) / 2;
-  const int total_work = p.B * pairs;
-  const int ka = p.ids ? 0 : (p.Da + GH_BLOCK_K - 1) / GH_BLOCK_K;
-  const int kg = (p.Dg + GH_BLOCK_K - 1) / GH_BLOCK_K;
-  const int num_kb = ka + kg;
-  const uint64_t budget = p.wait_budget_ns;
+  const int total_work = b.total();
+  const uint64_t budget = b.wait_budget_ns;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < GH_STAGES; ++s) {
@@ -93,8 +99,8 @@ ghost_norm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     }
     *abort_flag = 0;
     mbar_fence_init();
-    tma_prefetch_desc(&map_a);
-    tma_prefetch_desc(&map_g);
+    tma_prefetch_desc(&b.map_a[0]);
+    tma_prefetch_desc(&b.map_b[0]);
   }
   if (warp == 1) {
     tmem_alloc(tmem_slot, 512);
@@ -110,23 +116,27 @@ ghost_norm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       int stage = 0;
       uint32_t phase = 0, issued_mask = 0, issued_phase = 0;
       bool ok = true;
+      int cur = 0;
       for (int w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
-        const GhostItem it = ghost_decode(w, pairs, nt);
+        cur = b.seek(w, cur);
+        const GhostParams& p = b.p[cur];
+        const GhostShape sh(p);
+        const GhostItem it = ghost_decode(w - b.start[cur], sh.pairs, sh.nt);
         const int s0 = p.seg ? p.seg[it.ex] : it.ex * p.T;
         const int len = p.seg ? p.seg[it.ex + 1] - s0 : p.T;
         if (it.tb2 * GH_TILE >= len) continue;                 // tile pair lies outside this (ragged) segment
         const int r1 = s0 + it.tb * GH_TILE, r2 = s0 + it.tb2 * GH_TILE;
         const bool diag = it.tb == it.tb2;
-        for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, p.status, OB_ERR_WAIT_EMPTY, budget)) {
+        for (int kb = 0; kb < sh.num_kb; ++kb) {
+          if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, b.status, OB_ERR_WAIT_EMPTY, budget)) {
             ok = false;
             break;
           }
           // a diagonal tile multiplies a row block with itself: one load serves both operands
           mbar_expect_tx(&full[stage], diag ? GH_TILE_BYTES : GH_STAGE_BYTES);
           uint8_t* dst = smem + stage * GH_STAGE_BYTES;
-          const CUtensorMap* map = kb < ka ? &map_a : &map_g;
-          const int col = (kb < ka ? kb : kb - ka) * GH_BLOCK_K;
+          const CUtensorMap* map = kb < sh.ka ? &b.map_a[cur] : &b.map_b[cur];
+          const int col = (kb < sh.ka ? kb : kb - sh.ka) * GH_BLOCK_K;
           tma_load_2d(dst, map, &full[stage], col, r1);
           if (!diag) tma_load_2d(dst + GH_TILE_BYTES, map, &full[stage], col, r2);
           issued_mask |= 1u << stage;
@@ -138,7 +148,7 @@ ghost_norm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         for (int s = 0; s < GH_STAGES; ++s)
           if (issued_mask & (1u << s)) {
             int dummy_abort = 0;
-            mbar_wait(&full[s], (issued_phase >> s) & 1u, &dummy_abort, p.status, OB_ERR_DRAIN, budget);
+            mbar_wait(&full[s], (issued_phase >> s) & 1u, &dummy_abort, b.status, OB_ERR_DRAIN, budget);
           }
       }
     }
@@ -148,26 +158,30 @@ ghost_norm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       int stage = 0, acc_iter = 0;
       uint32_t phase = 0;
       bool ok = true;
+      int cur = 0;
       for (int w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
-        const GhostItem it = ghost_decode(w, pairs, nt);
+        cur = b.seek(w, cur);
+        const GhostParams& p = b.p[cur];
+        const GhostShape sh(p);
+        const GhostItem it = ghost_decode(w - b.start[cur], sh.pairs, sh.nt);
         if (p.seg && it.tb2 * GH_TILE >= p.seg[it.ex + 1] - p.seg[it.ex]) continue;
         const uint32_t b_off = it.tb == it.tb2 ? 0u : static_cast<uint32_t>(GH_TILE_BYTES);
         const int as = acc_iter & 1;
-        if (!mbar_wait(&tmem_empty[as], ((acc_iter >> 1) & 1) ^ 1, abort_flag, p.status, OB_ERR_WAIT_TMEM_EMPTY,
+        if (!mbar_wait(&tmem_empty[as], ((acc_iter >> 1) & 1) ^ 1, abort_flag, b.status, OB_ERR_WAIT_TMEM_EMPTY,
                        budget)) {
           ok = false;
           break;
         }
         tc_fence_after();
-        for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait(&full[stage], phase, abort_flag, p.status, OB_ERR_WAIT_FULL, budget)) {
+        for (int kb = 0; kb < sh.num_kb; ++kb) {
+          if (!mbar_wait(&full[stage], phase, abort_flag, b.status, OB_ERR_WAIT_FULL, budget)) {
             ok = false;
             break;
           }
           tc_fence_after();
           const uint32_t t1 = smem_u32(smem + stage * GH_STAGE_BYTES), t2 = t1 + b_off;
-          const uint32_t d_tmem = tmem_base + as * 256 + (kb < ka ? 0 : 128);
-          const bool first = (kb == 0) || (kb == ka);
+          const uint32_t d_tmem = tmem_base + as * 256 + (kb < sh.ka ? 0 : 128);
+          const bool first = (kb == 0) || (kb == sh.ka);
 #pragma unroll
           for (int kk = 0; kk < GH_BLOCK_K / 16; ++kk) {
             // K-major, 128-byte swizzle: rows are 128 B apart, 8-row groups 1024 B apart; a k-step
@@ -188,13 +202,17 @@ ghost_norm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     const int q = warp & 3;
     int acc_iter = 0;
     bool ok = true;
+    int cur = 0;
     for (int w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
-      const GhostItem it = ghost_decode(w, pairs, nt);
+      cur = b.seek(w, cur);
+      const GhostParams& p = b.p[cur];
+      const GhostShape sh(p);
+      const GhostItem it = ghost_decode(w - b.start[cur], sh.pairs, sh.nt);
       const int s0 = p.seg ? p.seg[it.ex] : it.ex * p.T;
       const int len = p.seg ? p.seg[it.ex + 1] - s0 : p.T;
       if (it.tb2 * GH_TILE >= len) continue;
       const int as = acc_iter & 1;
-      if (!mbar_wait(&tmem_full[as], (acc_iter >> 1) & 1, abort_flag, p.status, OB_ERR_WAIT_TMEM_FULL, budget)) {
+      if (!mbar_wait(&tmem_full[as], (acc_iter >> 1) & 1, abort_flag, b.status, OB_ERR_WAIT_TMEM_FULL, budget)) {
         ok = false;
         break;
       }
@@ -273,9 +291,9 @@ __device__ __forceinline__ GhostWideItem ghost_wide_decode(int w, int per_exampl
   return it;
 }
 
+template <int CAP>
 __global__ void __launch_bounds__(GW_THREADS, 1)
-ghost_norm_wide_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_g,
-                       const GhostParams p) {
+ghost_norm_wide_kernel(const __grid_constant__ TmaBatch<GhostParams, CAP> b) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + GW_STAGES * GW_STAGE_BYTES);
@@ -287,15 +305,8 @@ ghost_norm_wide_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nt = (p.T + GH_TILE - 1) / GH_TILE;
-  const int ncb = (nt + 1) / 2;
-  int per_example = 0;
-  for (int tb = 0; tb < nt; ++tb) per_example += ncb - (tb >> 1);
-  const int total_work = p.B * per_example;
-  const int ka = p.ids ? 0 : (p.Da + GH_BLOCK_K - 1) / GH_BLOCK_K;
-  const int kg = (p.Dg + GH_BLOCK_K - 1) / GH_BLOCK_K;
-  const int num_kb = ka + kg;
-  const uint64_t budget = p.wait_budget_ns;
+  const int total_work = b.total();
+  const uint64_t budget = b.wait_budget_ns;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < GW_STAGES; ++s) {
@@ -306,8 +317,8 @@ ghost_norm_wide_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     mbar_init(tmem_empty, 8);
     *abort_flag = 0;
     mbar_fence_init();
-    tma_prefetch_desc(&map_a);
-    tma_prefetch_desc(&map_g);
+    tma_prefetch_desc(&b.map_a[0]);
+    tma_prefetch_desc(&b.map_b[0]);
   }
   if (warp == 1) {
     tmem_alloc(tmem_slot, 512);
@@ -319,7 +330,7 @@ ghost_norm_wide_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
   const uint32_t tmem_base = *tmem_slot;
 
   // segment of example `ex`: first row and length; an item is skipped when its column blocks start past the end
-  auto segment = [&](int ex, int& s0, int& len) {
+  auto segment = [](const GhostParams& p, int ex, int& s0, int& len) {
     s0 = p.seg ? p.seg[ex] : ex * p.T;
     len = p.seg ? p.seg[ex + 1] - s0 : p.T;
   };
@@ -329,22 +340,26 @@ ghost_norm_wide_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
       int stage = 0;
       uint32_t phase = 0, issued_mask = 0, issued_phase = 0;
       bool ok = true;
+      int cur = 0;
       for (int w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
-        const GhostWideItem it = ghost_wide_decode(w, per_example, nt, ncb);
+        cur = b.seek(w, cur);
+        const GhostParams& p = b.p[cur];
+        const GhostShape sh(p);
+        const GhostWideItem it = ghost_wide_decode(w - b.start[cur], sh.wide_items, sh.nt, sh.ncb);
         int s0, len;
-        segment(it.ex, s0, len);
+        segment(p, it.ex, s0, len);
         if (it.tb * GH_TILE >= len || it.cb * GW_TILE_N >= len) continue;
         const int r1 = s0 + it.tb * GH_TILE, r2 = s0 + it.cb * GW_TILE_N;
         const bool diag = (it.tb >> 1) == it.cb;              // the row block is one of the two column blocks
-        for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, p.status, OB_ERR_WAIT_EMPTY, budget)) {
+        for (int kb = 0; kb < sh.num_kb; ++kb) {
+          if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, b.status, OB_ERR_WAIT_EMPTY, budget)) {
             ok = false;
             break;
           }
           mbar_expect_tx(&full[stage], diag ? GW_B_BYTES : GW_STAGE_BYTES);
           uint8_t* dst = smem + stage * GW_STAGE_BYTES;
-          const CUtensorMap* map = kb < ka ? &map_a : &map_g;
-          const int col = (kb < ka ? kb : kb - ka) * GH_BLOCK_K;
+          const CUtensorMap* map = kb < sh.ka ? &b.map_a[cur] : &b.map_b[cur];
+          const int col = (kb < sh.ka ? kb : kb - sh.ka) * GH_BLOCK_K;
           if (!diag) tma_load_2d(dst, map, &full[stage], col, r1);
           tma_load_2d(dst + GW_A_BYTES, map, &full[stage], col, r2);
           tma_load_2d(dst + GW_A_BYTES + GW_A_BYTES, map, &full[stage], col, r2 + GH_TILE);
@@ -357,7 +372,7 @@ ghost_norm_wide_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         for (int s = 0; s < GW_STAGES; ++s)
           if (issued_mask & (1u << s)) {
             int dummy_abort = 0;
-            mbar_wait(&full[s], (issued_phase >> s) & 1u, &dummy_abort, p.status, OB_ERR_DRAIN, budget);
+            mbar_wait(&full[s], (issued_phase >> s) & 1u, &dummy_abort, b.status, OB_ERR_DRAIN, budget);
           }
       }
     }
@@ -367,28 +382,32 @@ ghost_norm_wide_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
       int stage = 0, acc_iter = 0;
       uint32_t phase = 0;
       bool ok = true;
+      int cur = 0;
       for (int w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
-        const GhostWideItem it = ghost_wide_decode(w, per_example, nt, ncb);
+        cur = b.seek(w, cur);
+        const GhostParams& p = b.p[cur];
+        const GhostShape sh(p);
+        const GhostWideItem it = ghost_wide_decode(w - b.start[cur], sh.wide_items, sh.nt, sh.ncb);
         int s0, len;
-        segment(it.ex, s0, len);
+        segment(p, it.ex, s0, len);
         if (it.tb * GH_TILE >= len || it.cb * GW_TILE_N >= len) continue;
         // on a diagonal super-block the A operand is read from the copy of that row block inside the B operand
         const uint32_t a_off = (it.tb >> 1) == it.cb ? static_cast<uint32_t>(GW_A_BYTES + (it.tb & 1) * GW_A_BYTES) : 0u;
-        if (!mbar_wait(tmem_empty, (acc_iter & 1) ^ 1, abort_flag, p.status, OB_ERR_WAIT_TMEM_EMPTY, budget)) {
+        if (!mbar_wait(tmem_empty, (acc_iter & 1) ^ 1, abort_flag, b.status, OB_ERR_WAIT_TMEM_EMPTY, budget)) {
           ok = false;
           break;
         }
         tc_fence_after();
-        for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait(&full[stage], phase, abort_flag, p.status, OB_ERR_WAIT_FULL, budget)) {
+        for (int kb = 0; kb < sh.num_kb; ++kb) {
+          if (!mbar_wait(&full[stage], phase, abort_flag, b.status, OB_ERR_WAIT_FULL, budget)) {
             ok = false;
             break;
           }
           tc_fence_after();
           const uint32_t st0 = smem_u32(smem + stage * GW_STAGE_BYTES);
           const uint32_t t1 = st0 + a_off, t2 = st0 + GW_A_BYTES;
-          const uint32_t d_tmem = tmem_base + (kb < ka ? 0 : GW_TILE_N);
-          const bool first = (kb == 0) || (kb == ka);
+          const uint32_t d_tmem = tmem_base + (kb < sh.ka ? 0 : GW_TILE_N);
+          const bool first = (kb == 0) || (kb == sh.ka);
 #pragma unroll
           for (int kk = 0; kk < GH_BLOCK_K / 16; ++kk) {
             const uint64_t ad = make_smem_desc(t1 + kk * 32, 16, 1024, 2);
@@ -408,12 +427,16 @@ ghost_norm_wide_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     const int half = (warp - 2) >> 2;        // which of the two 128-column blocks
     int acc_iter = 0;
     bool ok = true;
+    int cur = 0;
     for (int w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
-      const GhostWideItem it = ghost_wide_decode(w, per_example, nt, ncb);
+      cur = b.seek(w, cur);
+      const GhostParams& p = b.p[cur];
+      const GhostShape sh(p);
+      const GhostWideItem it = ghost_wide_decode(w - b.start[cur], sh.wide_items, sh.nt, sh.ncb);
       int s0, len;
-      segment(it.ex, s0, len);
+      segment(p, it.ex, s0, len);
       if (it.tb * GH_TILE >= len || it.cb * GW_TILE_N >= len) continue;
-      if (!mbar_wait(tmem_full, acc_iter & 1, abort_flag, p.status, OB_ERR_WAIT_TMEM_FULL, budget)) {
+      if (!mbar_wait(tmem_full, acc_iter & 1, abort_flag, b.status, OB_ERR_WAIT_TMEM_FULL, budget)) {
         ok = false;
         break;
       }
@@ -473,56 +496,96 @@ extern "C" int ob_ghost_set_wide(int enabled) {
   return old;
 }
 
+namespace ob {
+
+template <int CAP>
+static int launch_ghost(const TmaBatch<GhostParams, CAP>& b, bool wide, int num_sms, cudaStream_t stream) {
+  static bool configured = false;
+  if (!configured) {
+    if (cudaFuncSetAttribute(ghost_norm_kernel<CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, GH_SMEM) != cudaSuccess ||
+        cudaFuncSetAttribute(ghost_norm_wide_kernel<CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, GW_SMEM) != cudaSuccess)
+      return -20;
+    configured = true;
+  }
+  const int total = b.start[b.count];
+  if (total <= 0) return 0;
+  const int grid = total < num_sms ? total : num_sms;
+  if (wide) ghost_norm_wide_kernel<CAP><<<grid, GW_THREADS, GW_SMEM, stream>>>(b);
+  else ghost_norm_kernel<CAP><<<grid, GH_THREADS, GH_SMEM, stream>>>(b);
+  return cudaGetLastError() == cudaSuccess ? 0 : -21;
+}
+
+// measured: the wide blocks win from about 1024 rows per example (less wasted work below the diagonal); below that the
+// 128 x 128 blocks with double-buffered accumulators are as fast or faster
+static bool ghost_use_wide(int T) {
+  const int nt = (T + GH_TILE - 1) / GH_TILE;
+  return wide_enabled == 2 ? nt >= 2 : (wide_enabled == 1 && nt >= 8);
+}
+
+// Appends one problem to the batch; 0 on success (also when it has no work).
+template <int CAP>
+static int ghost_append(TmaBatch<GhostParams, CAP>& b, const ob_ghost_desc& d, bool wide) {
+  if (d.B <= 0 || d.T <= 0 || d.Dg <= 0) return 0;
+  const long long rows = d.seg ? d.total_rows : static_cast<long long>(d.B) * d.T;
+  if (rows <= 0) return 0;
+  const int i = b.count;
+  int rc = make_bf16_map_2d(&b.map_b[i], d.g, rows, d.Dg, d.ldg, GH_BLOCK_K, GH_TILE);
+  if (rc) return rc;
+  if (d.ids == nullptr) {
+    rc = make_bf16_map_2d(&b.map_a[i], d.a, rows, d.Da, d.lda, GH_BLOCK_K, GH_TILE);
+    if (rc) return rc;
+  } else {
+    b.map_a[i] = b.map_b[i];
+  }
+  GhostParams& p = b.p[i];
+  p.B = d.B; p.T = d.T; p.Da = d.Da; p.Dg = d.Dg;
+  p.ids = d.ids; p.seg = d.seg; p.seg_out = d.seg_out; p.norm2 = d.norm2;
+  const GhostShape sh(p);
+  const long long end = b.start[i] + static_cast<long long>(d.B) * (wide ? sh.wide_items : sh.pairs);
+  if (end > 0x7fffffffLL - (1 << 16)) return -23;
+  b.start[i + 1] = static_cast<int>(end);
+  ++b.count;
+  return 0;
+}
+
+}  // namespace ob
+
 extern "C" int ob_ghost_norm(const void* a, const void* g, const int* ids, int B, int T, int Da, int Dg,
                              long long lda, long long ldg, float* norm2, const int* seg, const int* seg_out,
                              long long total_rows, int* status, double wait_budget_s, int num_sms, void* stream) {
   using namespace ob;
-  if (B <= 0 || T <= 0 || Dg <= 0) return 0;
-  const long long rows = seg ? total_rows : static_cast<long long>(B) * T;
-  if (rows <= 0) return 0;
-  CUtensorMap ma, mg;
-  int rc = make_bf16_map_2d(&mg, g, rows, Dg, ldg, GH_BLOCK_K, GH_TILE);
-  if (rc) return rc;
-  if (ids == nullptr) {
-    rc = make_bf16_map_2d(&ma, a, rows, Da, lda, GH_BLOCK_K, GH_TILE);
-    if (rc) return rc;
-  } else {
-    ma = mg;
-  }
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(ghost_norm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GH_SMEM) != cudaSuccess)
-      return -20;
-    configured = true;
-  }
-  GhostParams p;
-  p.B = B; p.T = T; p.Da = Da; p.Dg = Dg;
-  p.ids = ids;
-  p.seg = seg;
-  p.seg_out = seg_out;
-  p.norm2 = norm2;
-  p.status = status;
-  p.wait_budget_ns = static_cast<unsigned long long>(wait_budget_s * 1e9);
-  const int nt = (T + GH_TILE - 1) / GH_TILE;
-  // measured: the wide blocks win from about 1024 rows per example (less wasted work below the diagonal); below that
-  // the 128 x 128 blocks with double-buffered accumulators are as fast or faster
-  if (wide_enabled == 2 ? nt >= 2 : (wide_enabled == 1 && nt >= 8)) {
-    static bool configured_wide = false;
-    if (!configured_wide) {
-      if (cudaFuncSetAttribute(ghost_norm_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GW_SMEM) != cudaSuccess)
-        return -22;
-      configured_wide = true;
+  const ob_ghost_desc d = {a, g, ids, norm2, seg, seg_out, lda, ldg, total_rows, B, T, Da, Dg};
+  TmaBatch<GhostParams, 1> b;
+  b.count = 0;
+  b.start[0] = b.start[1] = 0;
+  b.status = status;
+  b.wait_budget_ns = static_cast<unsigned long long>(wait_budget_s * 1e9);
+  const bool wide = ghost_use_wide(T);
+  const int rc = ghost_append(b, d, wide);
+  return rc ? rc : launch_ghost(b, wide, num_sms, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int ob_ghost_norm_batch(const ob_ghost_desc* descs, int count, int* status, double wait_budget_s, int num_sms,
+                                   void* stream) {
+  using namespace ob;
+  // two groups by block shape, each in launches of up to BATCH_CAP problems
+  for (int wide = 0; wide < 2; ++wide) {
+    TmaBatch<GhostParams, BATCH_CAP> b;
+    b.status = status;
+    b.wait_budget_ns = static_cast<unsigned long long>(wait_budget_s * 1e9);
+    int i = 0;
+    while (i < count) {
+      b.count = 0;
+      b.start[0] = 0;
+      for (; i < count && b.count < BATCH_CAP; ++i) {
+        if (ghost_use_wide(descs[i].T) != (wide != 0)) continue;
+        const int rc = ghost_append(b, descs[i], wide != 0);
+        if (rc) return rc;
+      }
+      if (b.count == 0) continue;
+      const int rc = launch_ghost(b, wide != 0, num_sms, static_cast<cudaStream_t>(stream));
+      if (rc) return rc;
     }
-    const int ncb = (nt + 1) / 2;
-    long long per_example = 0;
-    for (int tb = 0; tb < nt; ++tb) per_example += ncb - (tb >> 1);
-    const long long total = static_cast<long long>(B) * per_example;
-    const int grid = static_cast<int>(total < num_sms ? total : num_sms);
-    ghost_norm_wide_kernel<<<grid, GW_THREADS, GW_SMEM, static_cast<cudaStream_t>(stream)>>>(ma, mg, p);
-    return cudaGetLastError() == cudaSuccess ? 0 : -21;
   }
-  const long long total = static_cast<long long>(B) * (nt * (nt + 1) / 2);
-  const int grid = static_cast<int>(total < num_sms ? total : num_sms);
-  ghost_norm_kernel<<<grid, GH_THREADS, GH_SMEM, static_cast<cudaStream_t>(stream)>>>(ma, mg, p);
-  return cudaGetLastError() == cudaSuccess ? 0 : -21;
+  return 0;
 }

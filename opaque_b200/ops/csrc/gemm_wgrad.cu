@@ -52,8 +52,6 @@ struct WgradParams {
   long long ldm, ldn;
   int n_valid;                       // only columns n < n_valid are written
   int accumulate;
-  int* status;
-  unsigned long long wait_budget_ns;
 };
 
 template <int BLOCK_N>
@@ -72,22 +70,22 @@ struct WorkItem {
   long long out_base;
 };
 
-__device__ __forceinline__ WorkItem decode_work(const WgradParams& p, int w, int tiles_m, int tiles_n,
-                                                int block_n) {
+__device__ __forceinline__ WorkItem decode_work(const WgradParams& p, int w, int block_n) {
   WorkItem it;
+  const int tiles_m = (p.M + WG_BLOCK_M - 1) / WG_BLOCK_M, tiles_n = (p.N + block_n - 1) / block_n;
   const int mn = tiles_m * tiles_n;
   const int gs = w / mn, r = w % mn;
   it.g = gs / p.splits;
   const int split = gs % p.splits;
   it.m0 = (r / tiles_n) * WG_BLOCK_M;
   it.n0 = (r % tiles_n) * block_n;
-  const int b = p.seg_offsets ? p.seg_offsets[it.g] : 0;
+  const int s0 = p.seg_offsets ? p.seg_offsets[it.g] : 0;
   const int e = p.seg_offsets ? p.seg_offsets[it.g + 1] : p.T;
-  const int nkb = (e - b + WG_BLOCK_K - 1) / WG_BLOCK_K;
+  const int nkb = (e - s0 + WG_BLOCK_K - 1) / WG_BLOCK_K;
   const int kb0 = static_cast<int>(static_cast<long long>(nkb) * split / p.splits);
   const int kb1 = static_cast<int>(static_cast<long long>(nkb) * (split + 1) / p.splits);
-  it.row_begin = b + kb0 * WG_BLOCK_K;
-  it.seg_end = min(e, b + kb1 * WG_BLOCK_K);
+  it.row_begin = s0 + kb0 * WG_BLOCK_K;
+  it.seg_end = min(e, s0 + kb1 * WG_BLOCK_K);
   it.num_kb = kb1 - kb0;
   it.out_base = p.out_offset + (p.group_out_offset ? p.group_out_offset[it.g]
                                                    : static_cast<long long>(it.g) * p.group_stride);
@@ -100,10 +98,9 @@ __device__ __forceinline__ float* resolve_out(const WgradParams& p, long long id
   return p.peer_out[owner] + (idx - owner * p.shard_elems);
 }
 
-template <int BLOCK_N>
+template <int BLOCK_N, int CAP>
 __global__ void __launch_bounds__(WG_THREADS, 1)
-wgrad_clip_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                  const WgradParams p) {
+wgrad_clip_kernel(const __grid_constant__ TmaBatch<WgradParams, CAP> b) {
   using S = WgradSmem<BLOCK_N>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -119,10 +116,8 @@ wgrad_clip_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tiles_m = (p.M + WG_BLOCK_M - 1) / WG_BLOCK_M;
-  const int tiles_n = (p.N + BLOCK_N - 1) / BLOCK_N;
-  const int total_work = p.num_groups * p.splits * tiles_m * tiles_n;
-  const uint64_t budget = p.wait_budget_ns;
+  const int total_work = b.total();
+  const uint64_t budget = b.wait_budget_ns;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < S::STAGES; ++s) {
@@ -136,8 +131,8 @@ wgrad_clip_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     }
     *abort_flag = 0;
     mbar_fence_init();
-    tma_prefetch_desc(&map_a);
-    tma_prefetch_desc(&map_b);
+    tma_prefetch_desc(&b.map_a[0]);
+    tma_prefetch_desc(&b.map_b[0]);
   }
   if (warp == 1) {
     tmem_alloc(tmem_slot, 2 * BLOCK_N);
@@ -155,10 +150,13 @@ wgrad_clip_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       uint32_t phase = 0;
       uint32_t issued_mask = 0, issued_phase = 0;
       bool ok = true;
+      int cur = 0;
       for (int w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
-        const WorkItem it = decode_work(p, w, tiles_m, tiles_n, BLOCK_N);
+        cur = b.seek(w, cur);
+        const WgradParams& p = b.p[cur];
+        const WorkItem it = decode_work(p, w - b.start[cur], BLOCK_N);
         for (int kb = 0; kb < it.num_kb; ++kb) {
-          if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, p.status, OB_ERR_WAIT_EMPTY, budget)) {
+          if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, b.status, OB_ERR_WAIT_EMPTY, budget)) {
             ok = false;
             break;
           }
@@ -168,10 +166,10 @@ wgrad_clip_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
           const int row = it.row_begin + kb * WG_BLOCK_K;
 #pragma unroll
           for (int j = 0; j < WG_BLOCK_M / 64; ++j)
-            tma_load_2d(a_dst + j * (WG_BLOCK_K * 128), &map_a, &full[stage], it.m0 + 64 * j, row);
+            tma_load_2d(a_dst + j * (WG_BLOCK_K * 128), &b.map_a[cur], &full[stage], it.m0 + 64 * j, row);
 #pragma unroll
           for (int j = 0; j < BLOCK_N / 64; ++j)
-            tma_load_2d(b_dst + j * (WG_BLOCK_K * 128), &map_b, &full[stage], it.n0 + 64 * j, row);
+            tma_load_2d(b_dst + j * (WG_BLOCK_K * 128), &b.map_b[cur], &full[stage], it.n0 + 64 * j, row);
           issued_mask |= 1u << stage;
           issued_phase = (issued_phase & ~(1u << stage)) | (phase << stage);
           if (++stage == S::STAGES) { stage = 0; phase ^= 1; }
@@ -182,7 +180,7 @@ wgrad_clip_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         for (int s = 0; s < S::STAGES; ++s)
           if (issued_mask & (1u << s)) {
             int dummy_abort = 0;
-            mbar_wait(&full[s], (issued_phase >> s) & 1u, &dummy_abort, p.status, OB_ERR_DRAIN, budget);
+            mbar_wait(&full[s], (issued_phase >> s) & 1u, &dummy_abort, b.status, OB_ERR_DRAIN, budget);
           }
       }
     }
@@ -194,11 +192,14 @@ wgrad_clip_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       uint32_t phase = 0;
       int acc_iter = 0;
       bool ok = true;
+      int cur = 0;
       for (int w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
-        const WorkItem it = decode_work(p, w, tiles_m, tiles_n, BLOCK_N);
+        cur = b.seek(w, cur);
+        const WgradParams& p = b.p[cur];
+        const WorkItem it = decode_work(p, w - b.start[cur], BLOCK_N);
         if (it.num_kb == 0) continue;
         const int as = acc_iter & 1;
-        if (!mbar_wait(&tmem_empty[as], ((acc_iter >> 1) & 1) ^ 1, abort_flag, p.status, OB_ERR_WAIT_TMEM_EMPTY,
+        if (!mbar_wait(&tmem_empty[as], ((acc_iter >> 1) & 1) ^ 1, abort_flag, b.status, OB_ERR_WAIT_TMEM_EMPTY,
                        budget)) {
           ok = false;
           break;
@@ -206,8 +207,8 @@ wgrad_clip_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + as * BLOCK_N;
         for (int kb = 0; kb < it.num_kb; ++kb) {
-          if (!mbar_wait(&full[stage], phase, abort_flag, p.status, OB_ERR_WAIT_FULL, budget) ||
-              !mbar_wait(&scaled[stage], phase, abort_flag, p.status, OB_ERR_WAIT_SCALED, budget)) {
+          if (!mbar_wait(&full[stage], phase, abort_flag, b.status, OB_ERR_WAIT_FULL, budget) ||
+              !mbar_wait(&scaled[stage], phase, abort_flag, b.status, OB_ERR_WAIT_SCALED, budget)) {
             ok = false;
             break;
           }
@@ -236,17 +237,19 @@ wgrad_clip_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     float* st = epi + (warp - 2) * 32 * WG_STAGE_LD;
     int acc_iter = 0;
     bool ok = true;
-    const int n_lim = min(p.N, p.n_valid);
-    const bool vec_ok = (p.ldn == 1) && ((n_lim & 3) == 0) && ((p.ldm & 3) == 0) &&
-                        (p.peer_out == nullptr || (p.shard_elems & 3) == 0);
+    int cur = 0;
     for (int w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
-      const WorkItem it = decode_work(p, w, tiles_m, tiles_n, BLOCK_N);
-      const bool row_major = vec_ok && ((it.out_base & 3) == 0);
+      cur = b.seek(w, cur);
+      const WgradParams& p = b.p[cur];
+      const WorkItem it = decode_work(p, w - b.start[cur], BLOCK_N);
+      const int n_lim = min(p.N, p.n_valid);
+      const bool row_major = (p.ldn == 1) && ((n_lim & 3) == 0) && ((p.ldm & 3) == 0) && ((it.out_base & 3) == 0) &&
+                             (p.peer_out == nullptr || (p.shard_elems & 3) == 0);
       if (it.num_kb == 0 && p.accumulate) continue;
       int as = 0;
       if (it.num_kb > 0) {
         as = acc_iter & 1;
-        if (!mbar_wait(&tmem_full[as], (acc_iter >> 1) & 1, abort_flag, p.status, OB_ERR_WAIT_TMEM_FULL, budget)) {
+        if (!mbar_wait(&tmem_full[as], (acc_iter >> 1) & 1, abort_flag, b.status, OB_ERR_WAIT_TMEM_FULL, budget)) {
           ok = false;
           break;
         }
@@ -314,8 +317,11 @@ wgrad_clip_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     const int my_row = tid >> 3;
     long long it_global = 0;                     // k-block counter over the whole work list
     bool ok = true;
+    int cur = 0;
     for (int w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
-      const WorkItem it = decode_work(p, w, tiles_m, tiles_n, BLOCK_N);
+      cur = b.seek(w, cur);
+      const WgradParams& p = b.p[cur];
+      const WorkItem it = decode_work(p, w - b.start[cur], BLOCK_N);
       // first k-block of this item that belongs to this group
       int kb = static_cast<int>((group - (it_global & 1) + 2) & 1);
       float sc[4];
@@ -342,7 +348,7 @@ wgrad_clip_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
           s2[i] = __halves2bfloat162(h, h);
         }
         if (kb + 2 < it.num_kb) fetch(kb + 2);   // prefetch for the next block of this group
-        if (!mbar_wait(&full[stage], phase, abort_flag, p.status, OB_ERR_WAIT_FULL, budget)) {
+        if (!mbar_wait(&full[stage], phase, abort_flag, b.status, OB_ERR_WAIT_FULL, budget)) {
           ok = false;
           break;
         }
@@ -402,8 +408,6 @@ struct WgradPeParams {
   long long ldm;
   int accumulate;
   float* norm2_out;                  // NORM kernel: [num_examples] squared Frobenius norms are added here; nothing else is written
-  int* status;
-  unsigned long long wait_budget_ns;
 };
 
 __device__ __forceinline__ float* resolve_out_pe(const WgradPeParams& p, long long idx) {
@@ -416,10 +420,9 @@ __device__ __forceinline__ float* resolve_out_pe(const WgradPeParams& p, long lo
 // tensor memory tile by tile, but the epilogue only sums their squares into norm2_out[e]; nothing is scaled, accumulated or
 // stored.  Costs 2 T d_in d_out FLOPs per example against T^2 (d_in + d_out) for the Gram-matrix form, so it is the
 // cheaper one for long sequences on small layers.
-template <bool NORM>
+template <bool NORM, int CAP>
 __global__ void __launch_bounds__(WP_THREADS, 1)
-wgrad_clip_pe_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                     const WgradPeParams p) {
+wgrad_clip_pe_kernel(const __grid_constant__ TmaBatch<WgradPeParams, CAP> b) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + WP_STAGES * WP_STAGE_BYTES);
@@ -431,11 +434,8 @@ wgrad_clip_pe_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tiles_m = (p.M + WG_BLOCK_M - 1) / WG_BLOCK_M;
-  const int tiles_n = (p.N + WP_BLOCK_N - 1) / WP_BLOCK_N;
-  const int total_work = p.splits * tiles_m * tiles_n;
-  const int kpe = p.ex_rows / WG_BLOCK_K;
-  const uint64_t budget = p.wait_budget_ns;
+  const int total_work = b.total();
+  const uint64_t budget = b.wait_budget_ns;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < WP_STAGES; ++s) {
@@ -448,8 +448,8 @@ wgrad_clip_pe_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     }
     *abort_flag = 0;
     mbar_fence_init();
-    tma_prefetch_desc(&map_a);
-    tma_prefetch_desc(&map_b);
+    tma_prefetch_desc(&b.map_a[0]);
+    tma_prefetch_desc(&b.map_b[0]);
   }
   if (warp == 1) {
     tmem_alloc(tmem_slot, 2 * WP_BLOCK_N);
@@ -461,7 +461,8 @@ wgrad_clip_pe_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
   const uint32_t tmem_base = *tmem_slot;
 
   // work item w -> (split, m tile, n tile); split s owns examples [e0, e1)
-  auto decode = [&](int w, int& m0, int& n0, int& e0, int& e1) {
+  auto decode = [](const WgradPeParams& p, int w, int& m0, int& n0, int& e0, int& e1) {
+    const int tiles_m = (p.M + WG_BLOCK_M - 1) / WG_BLOCK_M, tiles_n = (p.N + WP_BLOCK_N - 1) / WP_BLOCK_N;
     const int mn = tiles_m * tiles_n;
     const int split = w / mn, r = w % mn;
     m0 = (r / tiles_n) * WG_BLOCK_M;
@@ -475,13 +476,17 @@ wgrad_clip_pe_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
       int stage = 0;
       uint32_t phase = 0, issued_mask = 0, issued_phase = 0;
       bool ok = true;
+      int cur = 0;
       for (int w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
+        cur = b.seek(w, cur);
+        const WgradPeParams& p = b.p[cur];
+        const int kpe = p.ex_rows / WG_BLOCK_K;
         int m0, n0, e0, e1;
-        decode(w, m0, n0, e0, e1);
+        decode(p, w - b.start[cur], m0, n0, e0, e1);
         const int nkb = (e1 - e0) * kpe;
         const int row_begin = e0 * p.ex_rows;
         for (int kb = 0; kb < nkb; ++kb) {
-          if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, p.status, OB_ERR_WAIT_EMPTY, budget)) {
+          if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, b.status, OB_ERR_WAIT_EMPTY, budget)) {
             ok = false;
             break;
           }
@@ -491,10 +496,10 @@ wgrad_clip_pe_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
           const int row = row_begin + kb * WG_BLOCK_K;
 #pragma unroll
           for (int j = 0; j < WG_BLOCK_M / 64; ++j)
-            tma_load_2d(a_dst + j * (WG_BLOCK_K * 128), &map_a, &full[stage], m0 + 64 * j, row);
+            tma_load_2d(a_dst + j * (WG_BLOCK_K * 128), &b.map_a[cur], &full[stage], m0 + 64 * j, row);
 #pragma unroll
           for (int j = 0; j < WP_BLOCK_N / 64; ++j)
-            tma_load_2d(b_dst + j * (WG_BLOCK_K * 128), &map_b, &full[stage], n0 + 64 * j, row);
+            tma_load_2d(b_dst + j * (WG_BLOCK_K * 128), &b.map_b[cur], &full[stage], n0 + 64 * j, row);
           issued_mask |= 1u << stage;
           issued_phase = (issued_phase & ~(1u << stage)) | (phase << stage);
           if (++stage == WP_STAGES) { stage = 0; phase ^= 1; }
@@ -504,7 +509,7 @@ wgrad_clip_pe_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         for (int s = 0; s < WP_STAGES; ++s)
           if (issued_mask & (1u << s)) {
             int dummy_abort = 0;
-            mbar_wait(&full[s], (issued_phase >> s) & 1u, &dummy_abort, p.status, OB_ERR_DRAIN, budget);
+            mbar_wait(&full[s], (issued_phase >> s) & 1u, &dummy_abort, b.status, OB_ERR_DRAIN, budget);
           }
       }
     }
@@ -514,12 +519,16 @@ wgrad_clip_pe_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
       int stage = 0, acc_iter = 0;
       uint32_t phase = 0;
       bool ok = true;
+      int cur = 0;
       for (int w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
+        cur = b.seek(w, cur);
+        const WgradPeParams& p = b.p[cur];
+        const int kpe = p.ex_rows / WG_BLOCK_K;
         int m0, n0, e0, e1;
-        decode(w, m0, n0, e0, e1);
+        decode(p, w - b.start[cur], m0, n0, e0, e1);
         for (int e = e0; ok && e < e1; ++e) {
           const int as = acc_iter & 1;
-          if (!mbar_wait(&tmem_empty[as], ((acc_iter >> 1) & 1) ^ 1, abort_flag, p.status, OB_ERR_WAIT_TMEM_EMPTY,
+          if (!mbar_wait(&tmem_empty[as], ((acc_iter >> 1) & 1) ^ 1, abort_flag, b.status, OB_ERR_WAIT_TMEM_EMPTY,
                          budget)) {
             ok = false;
             break;
@@ -527,7 +536,7 @@ wgrad_clip_pe_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
           tc_fence_after();
           const uint32_t d_tmem = tmem_base + as * WP_BLOCK_N;
           for (int kb = 0; kb < kpe; ++kb) {
-            if (!mbar_wait(&full[stage], phase, abort_flag, p.status, OB_ERR_WAIT_FULL, budget)) {
+            if (!mbar_wait(&full[stage], phase, abort_flag, b.status, OB_ERR_WAIT_FULL, budget)) {
               ok = false;
               break;
             }
@@ -554,18 +563,21 @@ wgrad_clip_pe_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     const int half = (warp - 2) >> 2;            // which 128 of the tile's 256 columns
     int acc_iter = 0;
     bool ok = true;
-    const bool vec_ok = ((p.ldm & 3) == 0) && ((p.N & 3) == 0) && ((p.out_offset & 3) == 0) &&
-                        (p.peer_out == nullptr || (p.shard_elems & 3) == 0);
+    int cur = 0;
     for (int w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
+      cur = b.seek(w, cur);
+      const WgradPeParams& p = b.p[cur];
       int m0, n0, e0, e1;
-      decode(w, m0, n0, e0, e1);
+      decode(p, w - b.start[cur], m0, n0, e0, e1);
+      const bool vec_ok = ((p.ldm & 3) == 0) && ((p.N & 3) == 0) && ((p.out_offset & 3) == 0) &&
+                          (p.peer_out == nullptr || (p.shard_elems & 3) == 0);
       float acc[128];
 #pragma unroll
       for (int j = 0; j < 128; ++j) acc[j] = 0.f;
       for (int e = e0; e < e1; ++e) {
         const int as = acc_iter & 1;
         const float c = p.ex_scale ? __ldg(p.ex_scale + e) : 1.f;
-        if (!mbar_wait(&tmem_full[as], (acc_iter >> 1) & 1, abort_flag, p.status, OB_ERR_WAIT_TMEM_FULL, budget)) {
+        if (!mbar_wait(&tmem_full[as], (acc_iter >> 1) & 1, abort_flag, b.status, OB_ERR_WAIT_TMEM_FULL, budget)) {
           ok = false;
           break;
         }
@@ -687,23 +699,120 @@ int make_bf16_map_2d(CUtensorMap* map, const void* base, long long rows, long lo
   return r == CUDA_SUCCESS ? 0 : -12;
 }
 
-template <int BLOCK_N>
-static int launch_wgrad(const CUtensorMap& ma, const CUtensorMap& mb, const WgradParams& p, int sms,
-                        cudaStream_t stream) {
+template <int BLOCK_N, int CAP>
+static int launch_wgrad(const TmaBatch<WgradParams, CAP>& b, int sms, cudaStream_t stream) {
   using S = WgradSmem<BLOCK_N>;
   static bool configured = false;
   if (!configured) {
-    if (cudaFuncSetAttribute(wgrad_clip_kernel<BLOCK_N>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL) !=
+    if (cudaFuncSetAttribute(wgrad_clip_kernel<BLOCK_N, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL) !=
         cudaSuccess)
       return -20;
     configured = true;
   }
-  const int tiles_m = (p.M + WG_BLOCK_M - 1) / WG_BLOCK_M, tiles_n = (p.N + BLOCK_N - 1) / BLOCK_N;
-  const long long total = static_cast<long long>(p.num_groups) * p.splits * tiles_m * tiles_n;
+  const int total = b.start[b.count];
   if (total <= 0) return 0;
-  const int grid = static_cast<int>(total < sms ? total : sms);
-  wgrad_clip_kernel<BLOCK_N><<<grid, WG_THREADS, S::TOTAL, stream>>>(ma, mb, p);
+  const int grid = total < sms ? total : sms;
+  wgrad_clip_kernel<BLOCK_N, CAP><<<grid, WG_THREADS, S::TOTAL, stream>>>(b);
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
+}
+
+template <int CAP>
+static int launch_wgrad_bn(const TmaBatch<WgradParams, CAP>& b, int block_n, int sms, cudaStream_t st) {
+  if (block_n == 256) return launch_wgrad<256>(b, sms, st);
+  if (block_n == 128) return launch_wgrad<128>(b, sms, st);
+  if (block_n == 64) return launch_wgrad<64>(b, sms, st);
+  return -1;
+}
+
+// Appends one problem to the batch; 0 on success (also when it has no work).
+template <int CAP>
+static int wgrad_append(TmaBatch<WgradParams, CAP>& b, const ob_wgrad_desc& d, float* out, float* const* peer_out,
+                        long long shard_elems, int block_n) {
+  if (d.T <= 0 || d.M <= 0 || d.N <= 0 || d.num_groups <= 0) return 0;
+  const int i = b.count;
+  int rc = make_bf16_map_2d(&b.map_a[i], d.a, d.T, d.M, d.lda, 64, WG_BLOCK_K);
+  if (rc) return rc;
+  rc = make_bf16_map_2d(&b.map_b[i], d.b, d.T, d.N, d.ldb, 64, WG_BLOCK_K);
+  if (rc) return rc;
+  WgradParams& p = b.p[i];
+  p.M = d.M; p.N = d.N; p.T = d.T;
+  p.num_groups = d.num_groups;
+  p.seg_offsets = d.seg_offsets;
+  p.splits = d.splits < 1 ? 1 : d.splits;
+  p.row_scale = d.row_scale;
+  p.out = out;
+  p.peer_out = peer_out;
+  p.shard_elems = shard_elems;
+  p.group_out_offset = d.group_out_offset;
+  p.group_stride = d.group_stride;
+  p.out_offset = d.out_offset;
+  p.ldm = d.ldm; p.ldn = d.ldn;
+  p.n_valid = d.n_valid > 0 ? d.n_valid : d.N;
+  p.accumulate = d.accumulate;
+  const long long tiles = static_cast<long long>((d.M + WG_BLOCK_M - 1) / WG_BLOCK_M) * ((d.N + block_n - 1) / block_n);
+  const long long end = b.start[i] + tiles * d.num_groups * p.splits;
+  if (end > 0x7fffffffLL - (1 << 16)) return -5;
+  b.start[i + 1] = static_cast<int>(end);
+  ++b.count;
+  return 0;
+}
+
+template <bool NORM, int CAP>
+static int launch_wgrad_pe(const TmaBatch<WgradPeParams, CAP>& b, int sms, cudaStream_t stream) {
+  static bool configured = false;
+  if (!configured) {
+    if (cudaFuncSetAttribute(wgrad_clip_pe_kernel<NORM, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, WP_SMEM) != cudaSuccess)
+      return -20;
+    configured = true;
+  }
+  const int total = b.start[b.count];
+  if (total <= 0) return 0;
+  const int grid = total < sms ? total : sms;
+  wgrad_clip_pe_kernel<NORM, CAP><<<grid, WP_THREADS, WP_SMEM, stream>>>(b);
+  return cudaGetLastError() == cudaSuccess ? 0 : -21;
+}
+
+template <int CAP>
+static int wgrad_pe_append(TmaBatch<WgradPeParams, CAP>& b, const ob_wgrad_pe_desc& d, float* out, float* const* peer_out,
+                           long long shard_elems) {
+  if (d.num_examples <= 0 || d.ex_rows <= 0 || d.M <= 0 || d.N <= 0) return 0;
+  if (d.ex_rows % WG_BLOCK_K) return -3;
+  int splits = d.splits < 1 ? 1 : d.splits;
+  if (splits > d.num_examples) splits = d.num_examples;
+  if (splits > 1 && !d.accumulate && d.norm2 == nullptr) return -4;   // split partial sums must be reduced into the destination
+  const long long T = static_cast<long long>(d.num_examples) * d.ex_rows;
+  if (T > 0x7fffffffLL) return -5;
+  const int i = b.count;
+  int rc = make_bf16_map_2d(&b.map_a[i], d.a, T, d.M, d.lda, 64, WG_BLOCK_K);
+  if (rc) return rc;
+  rc = make_bf16_map_2d(&b.map_b[i], d.b, T, d.N, d.ldb, 64, WG_BLOCK_K);
+  if (rc) return rc;
+  WgradPeParams& p = b.p[i];
+  p.M = d.M; p.N = d.N;
+  p.num_examples = d.num_examples; p.ex_rows = d.ex_rows;
+  p.splits = splits;
+  p.ex_scale = d.ex_scale;
+  p.out = out;
+  p.peer_out = peer_out;
+  p.shard_elems = shard_elems;
+  p.out_offset = d.out_offset;
+  p.ldm = d.ldm;
+  p.accumulate = d.accumulate;
+  p.norm2_out = d.norm2;
+  const long long tiles = static_cast<long long>((d.M + WG_BLOCK_M - 1) / WG_BLOCK_M) * ((d.N + WP_BLOCK_N - 1) / WP_BLOCK_N);
+  const long long end = b.start[i] + tiles * splits;
+  if (end > 0x7fffffffLL - (1 << 16)) return -5;
+  b.start[i + 1] = static_cast<int>(end);
+  ++b.count;
+  return 0;
+}
+
+template <class P, int CAP>
+static void batch_begin(TmaBatch<P, CAP>& b, int* status, double wait_budget_s) {
+  b.count = 0;
+  b.start[0] = b.start[1] = 0;
+  b.status = status;
+  b.wait_budget_ns = static_cast<unsigned long long>(wait_budget_s * 1e9);
 }
 
 }  // namespace ob
@@ -715,91 +824,70 @@ extern "C" int ob_wgrad_clip(const void* a, const void* b, int T, int M, int N, 
                              long long ldm, long long ldn, int n_valid, int accumulate, int block_n, int* status,
                              double wait_budget_s, int num_sms, void* stream) {
   using namespace ob;
-  if (T <= 0 || M <= 0 || N <= 0 || num_groups <= 0) return 0;
-  if (splits < 1) splits = 1;
-  CUtensorMap ma, mb;
-  int rc = make_bf16_map_2d(&ma, a, T, M, lda, 64, WG_BLOCK_K);
-  if (rc) return rc;
-  rc = make_bf16_map_2d(&mb, b, T, N, ldb, 64, WG_BLOCK_K);
-  if (rc) return rc;
-  WgradParams p;
-  p.M = M; p.N = N; p.T = T;
-  p.num_groups = num_groups;
-  p.seg_offsets = seg_offsets;
-  p.splits = splits;
-  p.row_scale = row_scale;
-  p.out = out;
-  p.peer_out = peer_out;
-  p.shard_elems = shard_elems;
-  p.group_out_offset = group_out_offset;
-  p.group_stride = group_stride;
-  p.out_offset = out_offset;
-  p.ldm = ldm; p.ldn = ldn;
-  p.n_valid = n_valid > 0 ? n_valid : N;
-  p.accumulate = accumulate;
-  p.status = status;
-  p.wait_budget_ns = static_cast<unsigned long long>(wait_budget_s * 1e9);
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (block_n == 256) return launch_wgrad<256>(ma, mb, p, num_sms, st);
-  if (block_n == 128) return launch_wgrad<128>(ma, mb, p, num_sms, st);
-  if (block_n == 64) return launch_wgrad<64>(ma, mb, p, num_sms, st);
-  return -1;
+  const ob_wgrad_desc d = {a, b, row_scale, seg_offsets, group_out_offset, lda, ldb, group_stride, out_offset, ldm, ldn,
+                           T, M, N, num_groups, splits, n_valid, accumulate};
+  TmaBatch<WgradParams, 1> w;
+  batch_begin(w, status, wait_budget_s);
+  if (block_n != 64 && block_n != 128 && block_n != 256) return -1;
+  const int rc = wgrad_append(w, d, out, peer_out, shard_elems, block_n);
+  return rc ? rc : launch_wgrad_bn(w, block_n, num_sms, static_cast<cudaStream_t>(stream));
 }
 
-static int launch_wgrad_pe(const void* a, const void* b, int num_examples, int ex_rows, int M, int N, long long lda,
-                           long long ldb, const float* ex_scale, int splits, float* out, float* const* peer_out,
-                           long long shard_elems, long long out_offset, long long ldm, int accumulate, float* norm2_out,
-                           int* status, double wait_budget_s, int num_sms, void* stream) {
+extern "C" int ob_wgrad_clip_batch(const ob_wgrad_desc* descs, int count, float* out, float* const* peer_out,
+                                   long long shard_elems, int block_n, int* status, double wait_budget_s, int num_sms,
+                                   void* stream) {
   using namespace ob;
-  if (num_examples <= 0 || ex_rows <= 0 || M <= 0 || N <= 0) return 0;
-  if (ex_rows % WG_BLOCK_K) return -3;
-  if (splits < 1) splits = 1;
-  if (splits > num_examples) splits = num_examples;
-  if (splits > 1 && !accumulate && norm2_out == nullptr) return -4;   // split partial sums must be reduced into the destination
-  const long long T = static_cast<long long>(num_examples) * ex_rows;
-  if (T > 0x7fffffffLL) return -5;
-  CUtensorMap ma, mb;
-  int rc = make_bf16_map_2d(&ma, a, T, M, lda, 64, WG_BLOCK_K);
-  if (rc) return rc;
-  rc = make_bf16_map_2d(&mb, b, T, N, ldb, 64, WG_BLOCK_K);
-  if (rc) return rc;
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(wgrad_clip_pe_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, WP_SMEM) != cudaSuccess ||
-        cudaFuncSetAttribute(wgrad_clip_pe_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, WP_SMEM) != cudaSuccess)
-      return -20;
-    configured = true;
+  if (block_n != 64 && block_n != 256) return -1;
+  TmaBatch<WgradParams, BATCH_CAP> w;
+  for (int i = 0; i < count;) {
+    batch_begin(w, status, wait_budget_s);
+    for (; i < count && w.count < BATCH_CAP; ++i) {
+      const int rc = wgrad_append(w, descs[i], out, peer_out, shard_elems, block_n);
+      if (rc) return rc;
+    }
+    const int rc = block_n == 256 ? launch_wgrad<256>(w, num_sms, static_cast<cudaStream_t>(stream))
+                                  : launch_wgrad<64>(w, num_sms, static_cast<cudaStream_t>(stream));
+    if (rc) return rc;
   }
-  WgradPeParams p;
-  p.M = M; p.N = N;
-  p.num_examples = num_examples; p.ex_rows = ex_rows;
-  p.splits = splits;
-  p.ex_scale = ex_scale;
-  p.out = out;
-  p.peer_out = peer_out;
-  p.shard_elems = shard_elems;
-  p.out_offset = out_offset;
-  p.ldm = ldm;
-  p.accumulate = accumulate;
-  p.norm2_out = norm2_out;
-  p.status = status;
-  p.wait_budget_ns = static_cast<unsigned long long>(wait_budget_s * 1e9);
-  const long long tiles = static_cast<long long>((M + WG_BLOCK_M - 1) / WG_BLOCK_M) * ((N + WP_BLOCK_N - 1) / WP_BLOCK_N);
-  const long long total = tiles * splits;
-  const int grid = static_cast<int>(total < num_sms ? total : num_sms);
-  if (norm2_out != nullptr)
-    wgrad_clip_pe_kernel<true><<<grid, WP_THREADS, WP_SMEM, static_cast<cudaStream_t>(stream)>>>(ma, mb, p);
-  else
-    wgrad_clip_pe_kernel<false><<<grid, WP_THREADS, WP_SMEM, static_cast<cudaStream_t>(stream)>>>(ma, mb, p);
-  return cudaGetLastError() == cudaSuccess ? 0 : -21;
+  return 0;
+}
+
+// norm2 != NULL in every description: the direct per-example norms instead of the weighted gradients
+extern "C" int ob_wgrad_clip_pe_batch(const ob_wgrad_pe_desc* descs, int count, float* out, float* const* peer_out,
+                                      long long shard_elems, int* status, double wait_budget_s, int num_sms, void* stream) {
+  using namespace ob;
+  TmaBatch<WgradPeParams, BATCH_CAP> w;
+  for (int i = 0; i < count;) {
+    batch_begin(w, status, wait_budget_s);
+    const bool norm = descs[i].norm2 != nullptr;
+    for (; i < count && w.count < BATCH_CAP && (descs[i].norm2 != nullptr) == norm; ++i) {
+      const int rc = wgrad_pe_append(w, descs[i], out, peer_out, shard_elems);
+      if (rc) return rc;
+    }
+    const int rc = norm ? launch_wgrad_pe<true>(w, num_sms, static_cast<cudaStream_t>(stream))
+                        : launch_wgrad_pe<false>(w, num_sms, static_cast<cudaStream_t>(stream));
+    if (rc) return rc;
+  }
+  return 0;
+}
+
+static int wgrad_pe_one(const ob_wgrad_pe_desc& d, float* out, float* const* peer_out, long long shard_elems, int* status,
+                        double wait_budget_s, int num_sms, void* stream) {
+  using namespace ob;
+  TmaBatch<WgradPeParams, 1> w;
+  batch_begin(w, status, wait_budget_s);
+  const int rc = wgrad_pe_append(w, d, out, peer_out, shard_elems);
+  if (rc) return rc;
+  return d.norm2 != nullptr ? launch_wgrad_pe<true>(w, num_sms, static_cast<cudaStream_t>(stream))
+                            : launch_wgrad_pe<false>(w, num_sms, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int ob_wgrad_clip_pe(const void* a, const void* b, int num_examples, int ex_rows, int M, int N, long long lda,
                                 long long ldb, const float* ex_scale, int splits, float* out, float* const* peer_out,
                                 long long shard_elems, long long out_offset, long long ldm, int accumulate, int* status,
                                 double wait_budget_s, int num_sms, void* stream) {
-  return launch_wgrad_pe(a, b, num_examples, ex_rows, M, N, lda, ldb, ex_scale, splits, out, peer_out, shard_elems, out_offset,
-                         ldm, accumulate, nullptr, status, wait_budget_s, num_sms, stream);
+  const ob_wgrad_pe_desc d = {a, b, ex_scale, nullptr, lda, ldb, out_offset, ldm, num_examples, ex_rows, M, N, splits, accumulate};
+  return wgrad_pe_one(d, out, peer_out, shard_elems, status, wait_budget_s, num_sms, stream);
 }
 
 // Direct per-example gradient norms: norm2[e] += || a_e^T b_e ||_F^2 for example e = rows [e * ex_rows, (e + 1) * ex_rows)
@@ -808,8 +896,8 @@ extern "C" int ob_direct_norm2(const void* a, const void* b, int num_examples, i
                                long long ldb, int splits, float* norm2, int* status, double wait_budget_s, int num_sms,
                                void* stream) {
   if (norm2 == nullptr) return -6;
-  return launch_wgrad_pe(a, b, num_examples, ex_rows, M, N, lda, ldb, nullptr, splits, nullptr, nullptr, 0, 0, N, 0, norm2, status,
-                         wait_budget_s, num_sms, stream);
+  const ob_wgrad_pe_desc d = {a, b, nullptr, norm2, lda, ldb, 0, N, num_examples, ex_rows, M, N, splits, 0};
+  return wgrad_pe_one(d, nullptr, nullptr, 0, status, wait_budget_s, num_sms, stream);
 }
 
 extern "C" int ob_last_detail(char* buf, int len) {

@@ -21,6 +21,9 @@ _SIGNATURES = {
     "ob_wgrad_clip_pe": [P, P, I, I, I, I, LL, LL, P, I, P, P, LL, LL, LL, I, P, D, I, P],
     "ob_direct_norm2": [P, P, I, I, I, I, LL, LL, I, P, P, D, I, P],
     "ob_ghost_norm": [P, P, P, I, I, I, I, LL, LL, P, P, P, LL, P, D, I, P],
+    "ob_ghost_norm_batch": [c_char_p, I, P, D, I, P],
+    "ob_wgrad_clip_batch": [c_char_p, I, P, P, LL, I, P, D, I, P],
+    "ob_wgrad_clip_pe_batch": [c_char_p, I, P, P, LL, P, D, I, P],
     "ob_gemm_tn": [P, P, P, P, P, P, LL, I, I, I, LL, LL, LL, LL, LL, I, P, I, P, D, I, P],
     "ob_gemm_pair": [P, P, P, P, P, P, P, P, P, P, LL, I, I, I, LL, LL, LL, LL, LL, I, I, I, I, P, D, I, P],
     "ob_pair_init": [],
