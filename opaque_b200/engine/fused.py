@@ -412,9 +412,12 @@ class _GLUUp(Function):
     """
 
     @staticmethod
-    def forward(ctx, x, w_gate, w_up, act):
+    def forward(ctx, x, w_gate, w_up, act, keep=True):
         x2d = _rows(x)
-        h, g, u = ops.gemm_glu(x2d, w_gate, w_up, act=act)
+        h, g, u = ops.gemm_glu(x2d, w_gate, w_up, act=act, save_preact=keep)
+        ctx.act, ctx.xshape, ctx.trainable = act, x.shape, False
+        if not keep:
+            return h.view(*x.shape[:-1], w_gate.shape[0])
         trainable = w_gate.requires_grad or w_up.requires_grad
         ctx.save_for_backward(g, u, w_gate, w_up, *((x2d,) if trainable else ()))
         ctx.act, ctx.xshape, ctx.trainable = act, x.shape, trainable
@@ -434,13 +437,13 @@ class _GLUUp(Function):
             x2d = ctx.saved_tensors[4]
             cap = current_capture()
             if cap is None:
-                return dx, dg.t() @ x2d, du.t() @ x2d, None
+                return dx, dg.t() @ x2d, du.t() @ x2d, None, None
             dgc, duc = dg.contiguous(), du.contiguous()
             if w_gate.requires_grad:
                 cap.add_linear(w_gate, x2d, dgc)
             if w_up.requires_grad:
                 cap.add_linear(w_up, x2d, duc)
-        return dx, None, None, None
+        return dx, None, None, None, None
 
 
 def glu_up(x: torch.Tensor, w_gate: torch.nn.Parameter, w_up: torch.nn.Parameter, act: str = "silu") -> torch.Tensor | None:
@@ -452,7 +455,8 @@ def glu_up(x: torch.Tensor, w_gate: torch.nn.Parameter, w_up: torch.nn.Parameter
     trainable = w_gate.requires_grad or w_up.requires_grad
     if trainable and (current_capture() is None or w_gate.requires_grad != w_up.requires_grad):
         return None
-    return _GLUUp.apply(x, w_gate, w_up, act)
+    # the pre-activations are two thirds of what the launch writes; without a backward pass nobody reads them
+    return _GLUUp.apply(x, w_gate, w_up, act, torch.is_grad_enabled() and (trainable or x.requires_grad))
 
 
 class _GLUMLP(Function):
