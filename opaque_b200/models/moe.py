@@ -135,28 +135,45 @@ class _Experts(Function):
         h = grouped_linear(xs, w1, offs)
         act = ops.swiglu(h[:, :I], h[:, I:])
         y = grouped_linear(act, w2, offs)
-        wrow = topk_w.reshape(-1).index_select(0, slot_sorted).to(y.dtype)
-        out = torch.zeros_like(x).index_add_(0, token_sorted, y * wrow[:, None])
-        ctx.save_for_backward(xs, h, act, y, wrow, token_sorted, slot_sorted, offs, seg, w1, w2)
+        # row kernels: gather k rows per token instead of a scatter-add, one pass per gradient
+        ctx.rows = ops.functional.kernels_enabled() and y.is_cuda and y.dtype == topk_w.dtype == torch.bfloat16 and H % 8 == 0 and I % 8 == 0
+        if ctx.rows:
+            wts = topk_w.contiguous()
+            pos = torch.empty_like(slot_sorted)
+            pos[slot_sorted] = torch.arange(pos.numel(), device=pos.device)
+            out = ops.functional.moe_combine(y, pos, topk_idx.shape[1], wts)
+            ctx.save_for_backward(xs, h, act, y, wts, token_sorted, slot_sorted, offs, seg, w1, w2, pos)
+        else:
+            wrow = topk_w.reshape(-1).index_select(0, slot_sorted).to(y.dtype)
+            out = torch.zeros_like(x).index_add_(0, token_sorted, y * wrow[:, None])
+            ctx.save_for_backward(xs, h, act, y, wrow, token_sorted, slot_sorted, offs, seg, w1, w2)
         ctx.meta = (batch, tokens, topk_w.shape)
         return out
 
     @staticmethod
     def backward(ctx, dout):
-        xs, h, act, y, wrow, token_sorted, slot_sorted, offs, seg, w1, w2 = ctx.saved_tensors
+        xs, h, act, y, wrow, token_sorted, slot_sorted, offs, seg, w1, w2 = ctx.saved_tensors[:11]
         batch, tokens, wshape = ctx.meta
         I = w2.shape[2]
-        g = dout.index_select(0, token_sorted)
-        dw_rows = (g.float() * y.float()).sum(-1)
-        dtopk = torch.zeros(wshape, dtype=torch.float32, device=dout.device).reshape(-1).index_copy_(0, slot_sorted, dw_rows).view(wshape)
-        dy = (g * wrow[:, None]).contiguous()
-        dact = grouped_linear(dy, w2, offs, transposed=True)
-        gate, up = h[:, :I].float(), h[:, I:].float()
-        sig = torch.sigmoid(gate)
-        silu = gate * sig
-        dh = torch.cat([dact.float() * up * sig * (1 + gate * (1 - sig)), dact.float() * silu], dim=1).to(h.dtype)
-        dxs = grouped_linear(dh, w1, offs, transposed=True)
-        dx = torch.zeros_like(dout).index_add_(0, token_sorted, dxs)
+        if ctx.rows:
+            dy, dw = ops.functional.moe_row_grad(dout.contiguous(), y, wrow, token_sorted, slot_sorted)
+            dtopk = dw.view(wshape)
+            dact = grouped_linear(dy, w2, offs, transposed=True)
+            dh = ops.functional.glu_backward_packed(dact, h)
+            dxs = grouped_linear(dh, w1, offs, transposed=True)
+            dx = ops.functional.moe_combine(dxs, ctx.saved_tensors[11], wshape[1])
+        else:
+            g = dout.index_select(0, token_sorted)
+            dw_rows = (g.float() * y.float()).sum(-1)
+            dtopk = torch.zeros(wshape, dtype=torch.float32, device=dout.device).reshape(-1).index_copy_(0, slot_sorted, dw_rows).view(wshape)
+            dy = (g * wrow[:, None]).contiguous()
+            dact = grouped_linear(dy, w2, offs, transposed=True)
+            gate, up = h[:, :I].float(), h[:, I:].float()
+            sig = torch.sigmoid(gate)
+            silu = gate * sig
+            dh = torch.cat([dact.float() * up * sig * (1 + gate * (1 - sig)), dact.float() * silu], dim=1).to(h.dtype)
+            dxs = grouped_linear(dh, w1, offs, transposed=True)
+            dx = torch.zeros_like(dout).index_add_(0, token_sorted, dxs)
         cap = fused.current_capture()
         if cap is not None:
             ex_row = (token_sorted // tokens).to(torch.int32)

@@ -100,6 +100,13 @@ int ob_linear_ce_dlogits(void* logits, const long long* labels, const float* lse
                          int N, long long ld, float softcap, float smoothing, long long ignore_index, void* stream);
 unsigned int ob_debug_idesc_bf16(int m, int n, int a_mn_major, int b_mn_major);
 
+// Mixture of experts: out[t] = sum_j w[t * k + j] * y[pos[t * k + j]] (w NULL: plain sum), rows of H bf16 values, H % 8 == 0.
+int ob_moe_combine(const void* y, const void* w, const long long* pos, void* out, long long tokens, int k, int H, int sms,
+                   void* stream);
+// Its backward by sorted row i: dy[i] = w[slot[i]] * dout[token[i]], dw[slot[i]] = <dout[token[i]], y[i]> (fp32).
+int ob_moe_row_grad(const void* dout, const void* y, const void* w, const long long* token, const long long* slot, void* dy,
+                    float* dw, long long rows, int H, int sms, void* stream);
+
 // LayerNorm over the last dimension (bf16 in/out, fp32 statistics saved per row).
 int ob_layernorm_fwd(const void* x, const void* w, const void* b, void* y, float* mean, float* rstd, long long rows,
                      int H, float eps, void* stream);

@@ -332,6 +332,19 @@ def glu_backward(dh: torch.Tensor, gate: torch.Tensor, up: torch.Tensor, act: st
     return dg, du
 
 
+def glu_backward_packed(dh: torch.Tensor, gate_up: torch.Tensor) -> torch.Tensor:
+    """``[dGate | dUp]`` of ``silu(gate) * up`` for contiguous bf16 ``gate_up = [gate | up]`` (``[rows, 2I]``) and ``dh [rows, I]``."""
+    rows, two_i = gate_up.shape
+    I = two_i // 2
+    if dh.shape != (rows, I) or not dh.is_contiguous() or not gate_up.is_contiguous():
+        raise ValueError("glu_backward_packed: contiguous dh [rows, I] and gate_up [rows, 2I]")
+    both = torch.empty_like(gate_up)
+    rc = lib.load().ob_glu_bwd(dh.data_ptr(), gate_up.data_ptr(), gate_up[:, I:].data_ptr(), both.data_ptr(), both[:, I:].data_ptr(),
+                               rows, I, two_i, two_i, ACTIVATION_SWIGLU, lib.sm_count(), lib.stream())
+    lib.check(rc, "glu_bwd")
+    return both
+
+
 def swiglu(gate, up):
     """``silu(gate)·up``."""
     if _use_kernel(gate, up) and gate.shape[-1] % 8 == 0:
@@ -345,6 +358,39 @@ def geglu(gate, up, approximate=False):
     if _use_kernel(gate, up) and gate.shape[-1] % 8 == 0:
         return _GLU.apply(gate, up, act)
     return glu_ref(gate, up, act)
+
+
+# =============================================================================== mixture of experts
+
+def moe_combine(y, pos, k: int, w=None):
+    """``out[t] = Σ_j w[t, j] · y[pos[t·k + j]]`` for bf16 rows ``y [T·k, H]`` (``H % 8 == 0``) and int64 ``pos [T·k]``; ``w`` bf16
+    ``[T, k]`` or ``None`` for the plain sum.  fp32 sum in slot order, rounded once."""
+    rows, H = y.shape
+    if y.dtype != torch.bfloat16 or not y.is_contiguous() or pos.dtype != torch.int64 or pos.numel() != rows or rows % k:
+        raise ValueError("moe_combine: contiguous bf16 rows, one int64 position per row, k rows per token")
+    if w is not None and (w.dtype != torch.bfloat16 or w.numel() != rows or not w.is_contiguous()):
+        raise ValueError("moe_combine: one contiguous bf16 weight per row")
+    out = torch.empty(rows // k, H, dtype=y.dtype, device=y.device)
+    rc = lib.load().ob_moe_combine(y.data_ptr(), lib.ptr(w), pos.data_ptr(), out.data_ptr(), rows // k, k, H, lib.sm_count(),
+                                   lib.stream())
+    lib.check(rc, "moe_combine")
+    return out
+
+
+def moe_row_grad(dout, y, w, token_sorted, slot_sorted):
+    """Backward of the weighted combine by sorted row: ``(dy [R, H], dw)`` with ``dy[i] = w[slot_i] · dout[token_i]`` and
+    ``dw[slot_i] = <dout[token_i], y[i]>`` (fp32, in slot order)."""
+    rows, H = y.shape
+    if any(t.dtype != torch.bfloat16 or not t.is_contiguous() for t in (dout, y, w)) or dout.shape[1] != H or w.numel() != rows:
+        raise ValueError("moe_row_grad: contiguous bf16 operands, one weight per row")
+    if any(t.dtype != torch.int64 or t.numel() != rows for t in (token_sorted, slot_sorted)):
+        raise ValueError("moe_row_grad: int64 token and slot of every row")
+    dy = torch.empty_like(y)
+    dw = torch.empty(rows, dtype=torch.float32, device=y.device)
+    rc = lib.load().ob_moe_row_grad(dout.data_ptr(), y.data_ptr(), w.data_ptr(), token_sorted.data_ptr(), slot_sorted.data_ptr(),
+                                    dy.data_ptr(), dw.data_ptr(), rows, H, lib.sm_count(), lib.stream())
+    lib.check(rc, "moe_row_grad")
+    return dy, dw
 
 
 # =============================================================================== RoPE

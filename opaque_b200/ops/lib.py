@@ -33,6 +33,8 @@ _SIGNATURES = {
     "ob_gemm_pair_db": [P, P, P, P, P, P, LL, I, I, I, LL, LL, LL, LL, LL, I, I, P, D, I, P],
     "ob_linear_ce_fwd": [P, P, P, P, P, P, P, LL, I, I, LL, LL, LL, F, F, LL, P, D, I, P],
     "ob_linear_ce_dlogits": [P, P, P, P, LL, I, LL, F, F, LL, P],
+    "ob_moe_combine": [P, P, P, P, LL, I, I, I, P],
+    "ob_moe_row_grad": [P, P, P, P, P, P, P, LL, I, I, P],
     "ob_layernorm_fwd": [P, P, P, P, P, P, LL, I, F, P],
     "ob_layernorm_bwd_dx": [P, P, P, P, P, P, LL, I, P],
     "ob_rows_group_sum": [P, P, P, P, I, I, I, LL, P, LL, I, P, LL, P],

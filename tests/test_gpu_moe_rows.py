@@ -1,0 +1,45 @@
+"""Row kernels of the mixture of experts against fp64 (one rounding to bf16: 2^-9 relative)."""
+from __future__ import annotations
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _rel(x, y):
+    return float((x.double() - y.double()).norm() / y.double().norm())
+
+
+@pytest.mark.parametrize("T,k,H", [(1, 1, 8), (5, 4, 264), (130, 6, 2048), (33, 5, 72)])
+def test_combine_and_row_gradients(T, k, H):
+    from opaque_b200.ops import functional as F
+    g = torch.Generator(device="cuda").manual_seed(T)
+    y = torch.randn(T * k, H, device="cuda", generator=g, dtype=torch.bfloat16)
+    w = torch.rand(T, k, device="cuda", generator=g).to(torch.bfloat16)
+    dout = torch.randn(T, H, device="cuda", generator=g, dtype=torch.bfloat16)
+    slot = torch.randperm(T * k, device="cuda", generator=g)          # slot of every sorted row
+    token = slot // k
+    pos = torch.empty_like(slot)
+    pos[slot] = torch.arange(T * k, device="cuda")
+    rows = y.double()[pos].view(T, k, H)
+    assert _rel(F.moe_combine(y, pos, k, w), (rows * w.double()[..., None]).sum(1)) < 4e-3
+    assert _rel(F.moe_combine(y, pos, k), rows.sum(1)) < 4e-3
+    dy, dw = F.moe_row_grad(dout, y, w, token, slot)
+    gd = dout.double()[token]
+    assert _rel(dy, gd * w.double().view(-1)[slot][:, None]) < 4e-3
+    ref = torch.empty(T * k, device="cuda", dtype=torch.float64)
+    ref[slot] = (gd * y.double()).sum(1)
+    assert float((dw - ref).abs().max()) < 1e-6 * H * 16
+    with pytest.raises(ValueError):
+        F.moe_combine(y, pos[:-1], k, w)
+
+
+def test_packed_gated_backward():
+    from opaque_b200.ops import functional as F
+    for rows, I in ((1, 8), (37, 136)):
+        gu = torch.randn(rows, 2 * I, device="cuda", dtype=torch.bfloat16)
+        dh = torch.randn(rows, I, device="cuda", dtype=torch.bfloat16)
+        x = gu.double().requires_grad_(True)
+        (torch.nn.functional.silu(x[:, :I]) * x[:, I:]).backward(dh.double())
+        assert _rel(F.glu_backward_packed(dh, gu), x.grad) < 4e-3
