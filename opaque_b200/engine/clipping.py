@@ -222,6 +222,34 @@ def batched_clip_scales(batched: Any, bound: float | PerGroup, *, mode: str = "c
     return scale_for, norms.to(acc), None, finite
 
 
+def _tree_kernel_ok(leaves: Sequence[Any], dtype: torch.dtype | None, compute_dtype: torch.dtype | None) -> bool:
+    """True when the fused tree kernels give what the tensor operations below give: plain contiguous fp32 leaves on the current
+    B200, fp32 accumulation, nothing that records or transforms the operations."""
+    from .. import ops
+    if not 0 < len(leaves) <= ops.CLIP_TREE_MAX_LEAVES or dtype not in (None, torch.float32) or compute_dtype not in (None, torch.float32):
+        return False
+    wrapped = torch._C._functorch.is_functorch_wrapped_tensor
+    if not all(type(x) is torch.Tensor and x.is_cuda and x.dtype == torch.float32 and not wrapped(x) and x.ndim > 0
+               for x in leaves):
+        return False
+    x0 = leaves[0]
+    if any(x.device != x0.device or x.shape[0] != x0.shape[0] or (torch.is_grad_enabled() and x.requires_grad) for x in leaves):
+        return False
+    from ..device import fused_kernels_available
+    from torch.utils._python_dispatch import _get_current_dispatch_mode
+    return (0 < x0.shape[0] <= 65535 and x0.device.index == torch.cuda.current_device() and _get_current_dispatch_mode() is None
+            and torch.autograd.forward_ad._current_level < 0 and ops.functional.kernels_enabled() and fused_kernels_available())
+
+
+def _clip_tree(leaves: Sequence[torch.Tensor], bound: float, mode: str, gamma: float, factor: float):
+    """:func:`batched_clip_scales` and the weighted sums of every leaf in three launches: ``(sums, norms, clipped_norms)``."""
+    from .. import ops
+    rnd = norm_roundoff(torch.float32, torch.float64, len(leaves), _reduction_terms([x[0].numel() for x in leaves]))
+    fi = torch.finfo(torch.float32)
+    return ops.clip_tree([x.contiguous() for x in leaves], max(bound, 0.0), auto=mode == "auto", gamma=gamma, shrink=1.0 - 2.0 * (fi.eps / 2 + rnd),
+                         ulp=fi.smallest_normal * fi.eps, factor=factor)
+
+
 def clip_pytree(pytree: Any, clipping_norm: float | PerGroup, return_zero: bool = False, *,
                 compute_dtype: torch.dtype | None = None):
     """Clip ONE record's tree to L2 norm ``clipping_norm`` (guarded; non-finite values zeroed)."""
@@ -365,6 +393,7 @@ def clipped_fun(fun: Callable, has_aux: bool = False, *, batch_argnums: int | Se
         gnorm_parts: dict[str, list[torch.Tensor]] = {}
         num_clipped: Any = 0.0
         finite_all = True
+        scaled = False
         for lo in range(0, n, max(mb, 1)):
             hi = min(n, lo + mb)
             piece = _slice(args, b_nums, lo, hi)
@@ -373,6 +402,19 @@ def clipped_fun(fun: Callable, has_aux: bool = False, *, batch_argnums: int | Se
             raw_finite = all(bool(torch.isfinite(x).all()) for x in leaves if isinstance(x, torch.Tensor)) \
                 if return_stats else True
             finite_all = finite_all and raw_finite
+            if _scale_fn is None and not second_moment and not isinstance(clipping_norm, PerGroup) and _tree_kernel_ok(leaves, dtype, compute_dtype):
+                # the factor 1 / normalize_by is applied to the sum of ALL microbatches; with one, in the same pass
+                scaled = mb >= n
+                part, norms, cnorms = _clip_tree(leaves, float(clipping_norm), _mode, _gamma, 1.0 / normalize_by if scaled else 1.0)
+                sums = part if sums is None else [a + b for a, b in zip(sums, part)]
+                if _mode == "clip":
+                    num_clipped = num_clipped + float((norms > float(clipping_norm)).sum())
+                if return_aux:
+                    norm_parts.append(norms)
+                    cnorm_parts.append(cnorms)
+                    if has_aux:
+                        aux_parts.append(aux)
+                continue
             leaves = [_sanitize(x) if isinstance(x, torch.Tensor) else x for x in leaves]
             batched = tree_unflatten(td, leaves)
             if _scale_fn is not None:
@@ -414,7 +456,7 @@ def clipped_fun(fun: Callable, has_aux: bool = False, *, batch_argnums: int | Se
                     aux_parts.append(aux)
         if sums is None:  # empty batch
             raise _EmptyBatch()
-        inv = 1.0 / normalize_by
+        inv = 1.0 if scaled else 1.0 / normalize_by
         tree = tree_unflatten(td, [s * inv if inv != 1.0 else s for s in sums])
         result: Any = ClippedPytree(tree, max_norm)
         if second_moment:

@@ -720,6 +720,33 @@ def clip_weighted_sum(g: torch.Tensor, c: torch.Tensor, out: torch.Tensor | None
     lib.check(rc, "clip_weighted_sum")
 
 
+CLIP_TREE_MAX_LEAVES = 64
+
+
+def clip_tree(leaves: Sequence[torch.Tensor], bound: float, *, shrink: float, ulp: float, auto: bool = False, gamma: float = 0.0,
+              factor: float = 1.0) -> tuple[list[torch.Tensor], torch.Tensor, torch.Tensor]:
+    """Clip every example of a materialised fp32 gradient tree and sum: ``(sums, norms [E], clipped_norms [E])``.
+
+    ``leaves`` are contiguous ``[E, ...]`` fp32 CUDA tensors.  ``norm_e`` runs over all of them (fp32 squares, fp64 sums);
+    the factor of example e is ``bound / (norm + gamma)`` (``auto``) or ``min(1, bound / norm)``, shrunk to ``· shrink − ulp``
+    first and 0 where it is not finite; ``sums[i] = factor · Σ_e c_e · leaves[i][e]``.  Non-finite values count as 0.
+    """
+    import ctypes
+    E, n = leaves[0].shape[0], len(leaves)
+    if n > CLIP_TREE_MAX_LEAVES or any(x.dtype != torch.float32 or not x.is_contiguous() or x.shape[0] != E for x in leaves):
+        raise ValueError(f"clip_tree takes up to {CLIP_TREE_MAX_LEAVES} contiguous fp32 leaves with one leading example axis")
+    dev = leaves[0].device
+    sums = [torch.empty(x.shape[1:], dtype=torch.float32, device=dev) for x in leaves]
+    numel = (ctypes.c_longlong * n)(*[s.numel() for s in sums])
+    partial = torch.empty(max(E * lib.load().ob_clip_tree_chunks(numel, n), 1), dtype=torch.float64, device=dev)
+    rows = torch.empty(3, E, dtype=torch.float32, device=dev)
+    rc = lib.load().ob_clip_tree((ctypes.c_void_p * n)(*[x.data_ptr() for x in leaves]), (ctypes.c_void_p * n)(*[s.data_ptr() for s in sums]),
+                                 numel, n, E, bound, gamma, shrink, ulp, int(auto), factor, partial.data_ptr(), rows[0].data_ptr(),
+                                 rows[1].data_ptr(), rows[2].data_ptr(), lib.stream())
+    lib.check(rc, "clip_tree")
+    return sums, rows[0], rows[2]
+
+
 def embedding_wgrad(g: torch.Tensor, ids: torch.Tensor, out: torch.Tensor | None, *, row_scale=None, flat_offset=0,
                     peer_table=None, shard_elems=0) -> None:
     """``flat[flat_offset + ids[t]·D + d] += s[t]·g[t, d]``."""
@@ -788,7 +815,7 @@ from .functional import (activation, cross_entropy, cross_entropy_ref, fused_add
 
 __all__ = [
     "gemm", "gemm_pair", "gemm_glu", "gemm_glu_bwd", "direct_norm2", "pick_norm_path", "pick_gemm_kernel", "die_map", "set_die_aware_tiles", "linear_ce_forward", "linear_ce_dlogits_", "gemm_glu_ref", "gemm_ref", "ghost_set_wide", "push_grad_", "wgrad_clip_per_example", "wgrad_clip_batch", "wgrad_clip_per_example_batch", "direct_norm2_batch", "ghost_norm_batch", "plain_torch_ops", "layer_norm", "activation", "rows_group_sum_", "merge_heads3",
-    "DeviceWaitTimeout", "KernelLibraryError", "StatusWord", "clip_weighted_sum", "cross_entropy",
+    "DeviceWaitTimeout", "KernelLibraryError", "StatusWord", "clip_tree", "clip_weighted_sum", "cross_entropy",
     "cross_entropy_ref", "embedding_wgrad", "fused_add_rms_norm", "geglu", "ghost_norm", "ghost_norm_ref", "glu_ref",
     "philox_normal_add_", "pick_block_n", "pick_splits", "rms_norm", "rms_norm_ref", "rope_qk", "rope_qk_ref",
     "rope_tables", "rows_sumsq", "shard_step", "swiglu", "wgrad_clip", "wgrad_clip_ref",

@@ -107,6 +107,14 @@ int ob_moe_combine(const void* y, const void* w, const long long* pos, void* out
 int ob_moe_row_grad(const void* dout, const void* y, const void* w, const long long* token, const long long* slot, void* dy,
                     float* dw, long long rows, int H, int sms, void* stream);
 
+// Per-example clipping of a materialised fp32 gradient tree: leaf[i] is [E, numel[i]] contiguous, out[i] [numel[i]] receives
+// factor * sum_e scale[e] * leaf[i][e]; scale = bound / (norm + gamma) (automatic) or min(1, bound / norm), times `shrink`
+// minus `ulp`, 0 where not finite.  `partial` is scratch of E * ob_clip_tree_chunks(...) doubles.  At most 64 leaves.
+long long ob_clip_tree_chunks(const long long* numel, int leaves);
+int ob_clip_tree(const void* const* leaf, void* const* out, const long long* numel, int leaves, int E, double bound,
+                 double gamma, double shrink, double ulp, int automatic, float factor, double* partial, float* norms,
+                 float* scale, float* clipped, void* stream);
+
 // LayerNorm over the last dimension (bf16 in/out, fp32 statistics saved per row).
 int ob_layernorm_fwd(const void* x, const void* w, const void* b, void* y, float* mean, float* rstd, long long rows,
                      int H, float eps, void* stream);

@@ -35,6 +35,8 @@ _SIGNATURES = {
     "ob_linear_ce_dlogits": [P, P, P, P, LL, I, LL, F, F, LL, P],
     "ob_moe_combine": [P, P, P, P, LL, I, I, I, P],
     "ob_moe_row_grad": [P, P, P, P, P, P, P, LL, I, I, P],
+    "ob_clip_tree_chunks": [P, I],
+    "ob_clip_tree": [P, P, P, I, I, D, D, D, D, I, F, P, P, P, P, P],
     "ob_layernorm_fwd": [P, P, P, P, P, P, LL, I, F, P],
     "ob_layernorm_bwd_dx": [P, P, P, P, P, P, LL, I, P],
     "ob_rows_group_sum": [P, P, P, P, I, I, I, LL, P, LL, I, P, LL, P],
@@ -84,6 +86,7 @@ def load() -> ctypes.CDLL:
         fn = getattr(lib, name)
         fn.argtypes = argtypes
         fn.restype = c_int
+    lib.ob_clip_tree_chunks.restype = c_longlong
     lib.ob_debug_idesc_bf16.argtypes = [I, I, I, I]
     lib.ob_debug_idesc_bf16.restype = c_uint
     return lib
