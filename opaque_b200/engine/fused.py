@@ -104,6 +104,7 @@ class Capture:
         # stay alive for the weight gradients anyway
         self.ghost_jobs: list[tuple] = []
         self.direct_jobs: list[tuple] = []
+        self.bias_jobs: list[tuple] = []
         self.status = engine.status
         self.direct_elems = sp.direct_elems
 
@@ -250,7 +251,9 @@ class Capture:
             ops.ghost_norm_batch(self.ghost_jobs, status=self.status)
         if self.direct_jobs:
             ops.direct_norm2_batch(self.direct_jobs, self.tokens, status=self.status)
-        self.ghost_jobs, self.direct_jobs = [], []
+        for rows in {g.shape[0] for _, g in self.bias_jobs}:
+            ops.functional.rows_sum_batch_([j for j in self.bias_jobs if j[1].shape[0] == rows], self.batch_size)
+        self.ghost_jobs, self.direct_jobs, self.bias_jobs = [], [], []
         by_slot: dict[str, list[int]] = {}
         for i, name in enumerate(self.part_slots):
             by_slot.setdefault(name, []).append(i)
@@ -369,7 +372,7 @@ class _DPLinear(Function):
         cap.add_linear(weight, x2d, g2d)
         if ctx.bias is not None:
             if g2d.dtype == torch.bfloat16 and g2d.shape[1] % 8 == 0 and g2d.stride(0) % 8 == 0:
-                ops.rows_group_sum_(cap.pe_view(ctx.bias), g2d, cap.batch_size)
+                cap.bias_jobs.append((cap.pe_view(ctx.bias), g2d))
             else:
                 cap.pe_view(ctx.bias).add_(g2d.view(cap.batch_size, cap.tokens, -1).sum(1, dtype=torch.float32))
         return dx, None, None

@@ -70,16 +70,29 @@ class GPT2Block(nn.Module):
         self.mlp_c_proj = Linear(4 * d, d, bias=True, dtype=dtype, device=device)
 
     def forward(self, h):
-        B, T, d = h.shape
-        qkv = self.attn_c_attn(self.ln_1(h))
+        h = h + self._attention(self.ln_1(h))
+        return h + self._mlp(self.ln_2(h))
+
+    def forward_carried(self, x, residual):
+        """The block on a split stream ``h = x + residual`` (``residual`` may be ``None``): every residual addition happens inside
+        the next LayerNorm's kernel, and the two gradient branches meet in that kernel's backward.  Returns the pair."""
+        y, s = (self.ln_1(x), x) if residual is None else self.ln_1.add(x, residual)
+        y, s = self.ln_2.add(self._attention(y), s)
+        return self._mlp(y), s
+
+    def _mlp(self, y):
+        return self.mlp_c_proj(ops.activation(self.mlp_c_fc(y), "gelu_tanh"))
+
+    def _attention(self, y):
+        B, T, d = y.shape
+        qkv = self.attn_c_attn(y)
         if qkv.is_cuda and ops.functional.kernels_enabled():
             q, k, v = _SplitHeads.apply(qkv, self.nh)
         else:                                    # plain views (also what runs under vmap in the reference engine)
             v5 = qkv.view(B, T, 3, self.nh, d // self.nh)
             q, k, v = (v5[:, :, i].transpose(1, 2) for i in range(3))
         o = nn.functional.scaled_dot_product_attention(q, k, v, is_causal=True)
-        h = h + self.attn_c_proj(o.transpose(1, 2).reshape(B, T, d))
-        return h + self.mlp_c_proj(ops.activation(self.mlp_c_fc(self.ln_2(h)), "gelu_tanh"))
+        return self.attn_c_proj(o.transpose(1, 2).reshape(B, T, d))
 
 
 class GPT2LMHeadModel(nn.Module):
@@ -96,6 +109,11 @@ class GPT2LMHeadModel(nn.Module):
         B, T = input_ids.shape
         pos = torch.arange(T, device=input_ids.device).expand(B, T)
         h = self.wte(input_ids) + self.wpe(pos)
+        if h.is_cuda and ops.functional.kernels_enabled() and not (getattr(self, "activation_checkpointing", False) and torch.is_grad_enabled()):
+            x, residual = h, None
+            for blk in self.h:
+                x, residual = blk.forward_carried(x, residual)
+            return self.ln_f(x) if residual is None else self.ln_f.add(x, residual)[0]
         for blk in self.h:
             if getattr(self, "activation_checkpointing", False) and torch.is_grad_enabled():
                 h = (torch.utils.checkpoint.checkpoint(blk, h, use_reentrant=False) if ops.functional.kernels_enabled()

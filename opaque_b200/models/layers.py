@@ -148,6 +148,14 @@ class LayerNorm(nn.Module):
             return _LayerNormDP.apply(x, self.weight, self.bias, self.eps, self)
         return nn.functional.layer_norm(x, (x.shape[-1],), self.weight, self.bias, self.eps)
 
+    def add(self, x: torch.Tensor, residual: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
+        """``(layernorm(s), s)`` of ``s = x + residual``."""
+        if x.is_cuda and x.dtype == torch.bfloat16 and x.shape[-1] % 8 == 0 and self.weight.dtype == torch.bfloat16 \
+                and ops.functional.kernels_enabled():
+            return ops.add_layer_norm(x, residual, self.weight, self.bias, self.eps, layer=self)
+        s = x + residual
+        return self(s), s
+
 
 class _LinearCrossEntropy(Function):
     """Output head and token cross-entropy in one node; returns ``row_weight · nll`` per row.

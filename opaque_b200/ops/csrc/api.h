@@ -107,6 +107,10 @@ int ob_moe_combine(const void* y, const void* w, const long long* pos, void* out
 int ob_moe_row_grad(const void* dout, const void* y, const void* w, const long long* token, const long long* slot, void* dy,
                     float* dw, long long rows, int H, int sms, void* stream);
 
+// Plain row sums per example of several bf16 matrices g[i] [num_examples * rows_per_example, N[i]] (pitch ldg[i]) in one launch
+// per 128: out[i][e * ld_out[i] + n] += sum.
+int ob_rows_sum_batch(const void* const* g, const long long* ldg, const int* N, float* const* out, const long long* ld_out,
+                      int count, int num_examples, int rows_per_example, void* stream);
 // Per-example clipping of a materialised fp32 gradient tree: leaf[i] is [E, numel[i]] contiguous, out[i] [numel[i]] receives
 // factor * sum_e scale[e] * leaf[i][e]; scale = bound / (norm + gamma) (automatic) or min(1, bound / norm), times `shrink`
 // minus `ulp`, 0 where not finite.  `partial` is scratch of E * ob_clip_tree_chunks(...) doubles.  At most 64 leaves.
@@ -120,6 +124,11 @@ int ob_layernorm_fwd(const void* x, const void* w, const void* b, void* y, float
                      int H, float eps, void* stream);
 int ob_layernorm_bwd_dx(const void* dy, const void* x, const void* w, const float* mean, const float* rstd, void* dx,
                         long long rows, int H, void* stream);
+// The same with a residual addition in front (H <= 1024): sum = x + res (bf16), y = layernorm(sum); backward: dx = ... + ds.
+int ob_add_layernorm_fwd(const void* x, const void* res, const void* w, const void* b, void* y, void* sum, float* mean,
+                         float* rstd, long long rows, int H, float eps, void* stream);
+int ob_add_layernorm_bwd_dx(const void* dy, const void* x, const void* w, const float* mean, const float* rstd, const void* ds,
+                            void* dx, long long rows, int H, void* stream);
 // out[e, :N] += sum over the rows of example e of g (mode 0), g * (x - mean) * rstd (mode 1) or g * x * rstd (mode 2);
 // out row pitch ld_out.  In modes 1 and 2 a non-NULL out2 (row pitch ld_out2) also receives the plain sums of g.
 int ob_rows_group_sum(const void* g, const void* x, const float* mean, const float* rstd, int num_examples,

@@ -165,6 +165,24 @@ def rows_group_sum_(out: torch.Tensor, g2d: torch.Tensor, num_examples: int, *, 
     lib.check(rc, "rows_group_sum")
 
 
+def rows_sum_batch_(jobs, num_examples: int) -> None:
+    """``out[e] += Σ_{rows of example e} g`` for every ``(out, g2d)`` of ``jobs`` (the plain form of :func:`rows_group_sum_`; all
+    ``g2d`` with the same number of rows) in one launch per 128."""
+    rows = jobs[0][1].shape[0]
+    if rows % num_examples:
+        raise ValueError("rows_sum_batch_: rows must be a multiple of examples")
+    n = len(jobs)
+    g, o, ldg, ldo, cols = (ctypes.c_void_p * n)(), (ctypes.c_void_p * n)(), (ctypes.c_longlong * n)(), (ctypes.c_longlong * n)(), (ctypes.c_int * n)()
+    for i, (out, g2d) in enumerate(jobs):
+        if out.dtype != torch.float32 or out.shape != (num_examples, g2d.shape[1]) or out.stride(1) != 1:
+            raise ValueError("rows_sum_batch_: out must be fp32 [examples, N]")
+        if g2d.dtype != torch.bfloat16 or g2d.shape[0] != rows or g2d.stride(1) != 1:
+            raise ValueError("rows_sum_batch_: g must be bf16 matrices with the same number of rows")
+        g[i], o[i], ldg[i], ldo[i], cols[i] = g2d.data_ptr(), out.data_ptr(), g2d.stride(0), out.stride(0), g2d.shape[1]
+    rc = lib.load().ob_rows_sum_batch(g, ldg, cols, o, ldo, n, num_examples, rows // num_examples, lib.stream())
+    lib.check(rc, "rows_sum_batch")
+
+
 def merge_heads3(gq: torch.Tensor, gk: torch.Tensor, gv: torch.Tensor) -> torch.Tensor:
     """Three ``[B, heads, T, hd]`` bf16 tensors (any batch / head / token strides, contiguous head vectors) gathered into
     one ``[B, T, 3·heads·hd]`` tensor in ONE launch: the gradient of splitting a fused q/k/v projection into heads."""
@@ -182,6 +200,19 @@ def merge_heads3(gq: torch.Tensor, gk: torch.Tensor, gv: torch.Tensor) -> torch.
                                     lib.sm_count(), lib.stream())
     lib.check(rc, "merge_heads3")
     return out
+
+
+def _layer_norm_param_grads(dy2, x2, weight, stats, layer, has_bias):
+    """Weight and bias gradients of a LayerNorm: per example into the active capture (returns ``(None, None)``), else summed."""
+    cap = _param_grad_hook() if weight.requires_grad else None
+    if cap is not None:                      # per-example gradients straight into the capture's buffer rows
+        rows_group_sum_(cap.pe_view(layer.weight), dy2, cap.batch_size, x2d=x2, mean=stats[0], rstd=stats[1],
+                        out_plain=cap.pe_view(layer.bias) if has_bias else None)
+    elif weight.requires_grad:
+        acc = torch.zeros(2, 1, dy2.shape[1], dtype=torch.float32, device=x2.device)
+        rows_group_sum_(acc[0], dy2, 1, x2d=x2, mean=stats[0], rstd=stats[1], out_plain=acc[1])
+        return acc[0, 0].to(weight.dtype), (acc[1, 0].to(weight.dtype) if has_bias else None)
+    return None, None
 
 
 class _LayerNorm(Function):
@@ -213,15 +244,7 @@ class _LayerNorm(Function):
         rc = lib.load().ob_layernorm_bwd_dx(dy2.data_ptr(), x2.data_ptr(), weight.data_ptr(), stats[0].data_ptr(),
                                             stats[1].data_ptr(), dx.data_ptr(), rows, H, lib.stream())
         lib.check(rc, "layernorm_bwd_dx")
-        cap = _param_grad_hook() if weight.requires_grad else None
-        dw = db = None
-        if cap is not None:                      # per-example gradients straight into the capture's buffer rows
-            rows_group_sum_(cap.pe_view(layer.weight), dy2, cap.batch_size, x2d=x2, mean=stats[0], rstd=stats[1],
-                            out_plain=cap.pe_view(layer.bias) if has_bias else None)
-        elif weight.requires_grad:
-            acc = torch.zeros(2, 1, H, dtype=torch.float32, device=x2.device)
-            rows_group_sum_(acc[0], dy2, 1, x2d=x2, mean=stats[0], rstd=stats[1], out_plain=acc[1])
-            dw, db = acc[0, 0].to(weight.dtype), (acc[1, 0].to(weight.dtype) if has_bias else None)
+        dw, db = _layer_norm_param_grads(dy2, x2, weight, stats, layer, has_bias)
         return dx.view(shape), dw, db, None, None
 
 
@@ -230,6 +253,59 @@ def layer_norm(x, weight, bias=None, eps=1e-5, *, layer=None):
     if _use_kernel(x, weight) and x.shape[-1] % 8 == 0 and (bias is None or bias.dtype == torch.bfloat16):
         return _LayerNorm.apply(x, weight, bias, eps, layer)
     return torch.nn.functional.layer_norm(x, (x.shape[-1],), weight, bias, eps)
+
+
+class _AddLayerNorm(Function):
+    """``s = x + residual; y = layernorm(s)`` in one pass; both results are used, so both gradients meet in the backward pass."""
+
+    @staticmethod
+    def forward(ctx, x, residual, weight, bias, eps, layer):
+        shape, H = x.shape, x.shape[-1]
+        x2, r2 = x.reshape(-1, H), residual.reshape(-1, H)
+        x2 = x2 if x2.is_contiguous() else x2.contiguous()
+        r2 = r2 if r2.is_contiguous() else r2.contiguous()
+        rows = x2.shape[0]
+        y, s = torch.empty_like(x2), torch.empty_like(x2)
+        stats = torch.empty(2, rows, dtype=torch.float32, device=x.device)
+        rc = lib.load().ob_add_layernorm_fwd(x2.data_ptr(), r2.data_ptr(), weight.data_ptr(), lib.ptr(bias), y.data_ptr(), s.data_ptr(),
+                                             stats.data_ptr(), stats.data_ptr() + 4 * rows, rows, H, eps, lib.stream())
+        lib.check(rc, "add_layernorm_fwd")
+        ctx.save_for_backward(s, weight, stats)
+        ctx.meta = (shape, layer, bias is not None)
+        ctx.set_materialize_grads(False)
+        return y.view(shape), s.view(shape)
+
+    @staticmethod
+    def backward(ctx, dy, ds):
+        s, weight, stats = ctx.saved_tensors
+        shape, layer, has_bias = ctx.meta
+        rows, H = s.shape
+        if dy is None:                                   # only the sum is used
+            return ds, ds, None, None, None, None
+        dy2 = dy.reshape(-1, H)
+        dy2 = dy2 if dy2.is_contiguous() else dy2.contiguous()
+        dx = torch.empty_like(s)
+        mean, rstd = stats.data_ptr(), stats.data_ptr() + 4 * rows
+        if ds is None:                                   # nothing passes by the norm (the last one of a model)
+            rc = lib.load().ob_layernorm_bwd_dx(dy2.data_ptr(), s.data_ptr(), weight.data_ptr(), mean, rstd, dx.data_ptr(), rows, H, lib.stream())
+        else:
+            ds2 = ds.reshape(-1, H)
+            ds2 = ds2 if ds2.is_contiguous() else ds2.contiguous()
+            rc = lib.load().ob_add_layernorm_bwd_dx(dy2.data_ptr(), s.data_ptr(), weight.data_ptr(), mean, rstd, ds2.data_ptr(), dx.data_ptr(),
+                                                    rows, H, lib.stream())
+        lib.check(rc, "add_layernorm_bwd_dx")
+        dw, db = _layer_norm_param_grads(dy2, s, weight, stats, layer, has_bias)
+        dx = dx.view(shape)
+        return dx, dx, dw, db, None, None
+
+
+def add_layer_norm(x, residual, weight, bias=None, eps=1e-5, *, layer=None):
+    """``s = x + residual; y = layer_norm(s)``; returns ``(y, s)``."""
+    H = x.shape[-1]
+    if _use_kernel(x, residual, weight) and x.shape == residual.shape and H % 8 == 0 and H <= 1024 and (bias is None or bias.dtype == torch.bfloat16):
+        return _AddLayerNorm.apply(x, residual, weight, bias, eps, layer)
+    s = x + residual
+    return layer_norm(s, weight, bias, eps, layer=layer), s
 
 
 # =============================================================================== plain activations

@@ -1,0 +1,55 @@
+"""Residual addition fused into LayerNorm, and bias sums of many layers in one launch, against fp64 / the single-layer kernels."""
+from __future__ import annotations
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _rel(x, y):
+    return float((x.double() - y.double()).norm() / y.double().norm())
+
+
+@pytest.mark.parametrize("rows,H", [(1, 8), (7, 256), (9, 264), (130, 512), (33, 768), (5, 776), (17, 1024), (4, 1032)])
+@pytest.mark.parametrize("bias", [True, False])
+def test_add_layer_norm(rows, H, bias):
+    from opaque_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g, dtype=torch.bfloat16)          # noqa: E731
+    x, res, w, b = r(rows, H).requires_grad_(True), r(rows, H).requires_grad_(True), r(H).requires_grad_(True), r(H).requires_grad_(True) if bias else None
+    gy, gs = r(rows, H), r(rows, H)
+    s64 = (x.double() + res.double()).bfloat16().double().detach().requires_grad_(True)
+    w64, b64 = w.double().detach().requires_grad_(True), b.double().detach().requires_grad_(True) if bias else None
+    y64 = torch.nn.functional.layer_norm(s64, (H,), w64, b64, 1e-5)
+    for grads in ((gy, gs), (gy, None), (None, gs)):
+        leaves = [t for t in (x, res, w, b) if t is not None]
+        for t in leaves + [s64, w64] + ([b64] if bias else []):
+            t.grad = None
+        y, s = ops.add_layer_norm(x, res, w, b)
+        assert torch.equal(s.double(), s64) and _rel(y, y64) < 4e-3
+        used = [(o, q) for o, q in zip((y, s), grads) if q is not None]
+        torch.autograd.backward([o for o, _ in used], [q for _, q in used])
+        torch.autograd.backward([o for o, q in zip((y64, s64), grads) if q is not None], [q.double() for q in grads if q is not None], retain_graph=True)
+        assert torch.equal(x.grad, res.grad) and _rel(x.grad, s64.grad) < 6e-3
+        if grads[0] is not None:                 # parameters: fp32 sums over the rows, rounded to bf16
+            assert _rel(w.grad, w64.grad) < 6e-3 and (not bias or _rel(b.grad, b64.grad) < 6e-3)
+
+
+@pytest.mark.parametrize("count", [1, 3, 130])
+@pytest.mark.parametrize("B,T", [(1, 1), (3, 70), (2, 513)])
+def test_bias_sums_batched(count, B, T):
+    from opaque_b200.ops import functional as F
+    jobs, refs = [], []
+    for i in range(count):
+        N = 8 * (1 + (37 * i) % 70)
+        g = torch.randn(B * T, N + 8, device="cuda", dtype=torch.bfloat16)[:, :N]
+        buf = torch.full((B, N + 3), 2.0, device="cuda")
+        jobs.append((buf[:, :N], g))
+        refs.append((buf, g.double().view(B, T, N).sum(1) + 2.0))
+    F.rows_sum_batch_(jobs, B)
+    for buf, ref in refs:
+        # fp32 sums of T values of size one: T * 2^-24 * sqrt(T)
+        assert float((buf[:, :-3].double() - ref).abs().max()) < 1e-5 * max(T, 8) and bool((buf[:, -3:] == 2.0).all())
+    with pytest.raises(ValueError):
+        F.rows_sum_batch_([(jobs[0][0][:, :4], jobs[0][1])], B)
