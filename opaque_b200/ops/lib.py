@@ -132,7 +132,9 @@ def ptr(t: torch.Tensor | None) -> int | None:
 
 
 def stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """Handle of the current stream of the current device (``torch.cuda.current_stream()`` builds a stream object through
+    several Python layers: 3.2 us a call against 0.2, once per launch)."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 @functools.lru_cache(maxsize=None)
