@@ -21,6 +21,7 @@ packages/opaque-optimizers/src/opaque/api/optimizers/_adam.py:120-270):
 """
 from __future__ import annotations
 
+import functools
 import math
 import struct
 from typing import Sequence
@@ -428,6 +429,23 @@ def gemm_pair(a: torch.Tensor, b: torch.Tensor, *, b_layout: str = "nk", a2: tor
     return out
 
 
+def lora_pack(factors: Sequence[tuple[torch.Tensor, torch.Tensor]]) -> tuple[torch.Tensor, torch.Tensor]:
+    """``(a_cat [3r, in], b_block [Σout, 3r])`` of three LoRA pairs ``(A [r, in], B [out, r])``: the A factors stacked, the B
+    factors on the diagonal of a zero matrix (contiguous bf16, ``r % 8 == 0``)."""
+    (aq, bq), (ak, bk), (av, bv) = factors
+    r, d_in = aq.shape
+    outs = (bq.shape[0], bk.shape[0], bv.shape[0])
+    if any(a.shape != (r, d_in) or b.shape[1] != r or a.dtype != torch.bfloat16 or b.dtype != torch.bfloat16 or not a.is_contiguous()
+           or not b.is_contiguous() for a, b in factors):
+        raise ValueError("lora_pack: contiguous bf16 factors A [r, in], B [out, r] of one rank")
+    a_cat = torch.empty(3 * r, d_in, dtype=aq.dtype, device=aq.device)
+    b_block = torch.empty(sum(outs), 3 * r, dtype=aq.dtype, device=aq.device)
+    rc = lib.load().ob_lora_pack(aq.data_ptr(), ak.data_ptr(), av.data_ptr(), bq.data_ptr(), bk.data_ptr(), bv.data_ptr(), a_cat.data_ptr(),
+                                 b_block.data_ptr(), r, d_in, *outs, lib.sm_count(), lib.stream())
+    lib.check(rc, "lora_pack")
+    return a_cat, b_block
+
+
 def die_map() -> list[int] | None:
     """Die (0 / 1) of every SM of the current device by ``%smid``, or ``None`` when no two-die split was measured.
 
@@ -580,24 +598,61 @@ def pick_gemm_kernel(M: int, N: int, K: int, sms: int = 148) -> str:
     return "pair" if eff_pair >= eff_single else "single"
 
 
+@functools.lru_cache(maxsize=4096)
+def pick_gemm_plan(M: int, N: int, K: int, K2: int = 0, sms: int = 148) -> tuple[str, int]:
+    """``(kernel, splits)`` for an ungrouped ``[M, K] x [K, N]`` product (plus a ``K2`` segment).
+
+    Starts from :func:`pick_gemm_kernel`.  Where that kernel's tiles do not fill the chip once, the alternatives are weighed
+    by estimated microseconds, fitted to launches back to back in a CUDA graph with weights from HBM (32 shapes of 128 to
+    5439 rows; the estimates are within 10 % for most):
+
+      pair    6.6 + 0.567 per k-block   (256 x 2048 x 8192: 79.5 measured)
+      single  5.2 + 0.336 per k-block   (52.0)
+      split   the same with k-blocks / splits, + 3.2 for the second launch, + 1.14 per million partial values (18.6, 8 splits)
+
+    A split has to win a microsecond, or it is not worth the second launch's host time.
+    """
+    big = pick_gemm_kernel(M, N, K, sms)
+    nk = -(-K // 64) + -(-K2 // 64)
+    t1 = -(-M // 128) * -(-N // 256)
+    if (-(-M // 512) * -(-N // 256) >= max(sms // 2, 1)) if big == "pair" else t1 >= sms:
+        return (big, 1)
+    single = 5.2 + 0.336 * nk * -(-t1 // sms)
+    best = (6.6 + 0.567 * nk, "pair", 1) if big == "pair" and 6.6 + 0.567 * nk < single else (single, "single", 1)
+    for s in (2, 3, 4, 6, 8, 12, 16, 24):
+        if s > nk or t1 * s > 2 * sms or N % 4:
+            break
+        t = 5.2 + 0.336 * -(-nk // s) * -(-t1 * s // sms) + 3.2 + 1.14e-6 * M * N * s
+        if t + 1.0 < min(best[0], single):
+            best = (t + 1.0, "single", s)
+    return best[1:]
+
+
 def gemm(a: torch.Tensor, b: torch.Tensor, *, b_layout: str = "nk", a2: torch.Tensor | None = None,
          b2: torch.Tensor | None = None, bias: torch.Tensor | None = None, group_offs: torch.Tensor | None = None,
          out: torch.Tensor | None = None, status: StatusWord | None = None,
-         wait_budget_s: float = DEFAULT_WAIT_BUDGET_S, kernel: str = "auto") -> torch.Tensor:
+         wait_budget_s: float = DEFAULT_WAIT_BUDGET_S, kernel: str = "auto", b2_layout: str = "nk", alpha: float = 1.0,
+         splits: int = 1) -> torch.Tensor:
     """``a @ op(b) + a2 @ b2ᵀ + bias`` on the tcgen05 path (bf16 in/out, fp32 accumulation).
 
     ``b_layout="nk"``: ``b`` is ``[N, K]`` (a weight matrix as stored; ``op(b) = bᵀ``);  ``"kn"``: ``b`` is ``[K, N]``
     (``op(b) = b`` — data gradients ``dY @ W`` without a transposed copy).  ``a2 [M, r]``, ``b2 [N, r]`` add a
     low-rank segment accumulated in the same tile (LoRA-fused linear).  With ``group_offs`` (int32 ``[E + 1]`` row
     offsets, rows sorted by group) ``b`` is ``[E, N, K]`` / ``[E, K, N]`` and rows of group e use slab e (MoE experts).
-    ``kernel``: ``"pair"`` (two CTAs per 512 x 256 tile), ``"single"`` (one CTA per 128 x 256 tile) or ``"auto"``
-    (:func:`pick_gemm_kernel` for ungrouped products while :data:`PAIR_GEMM` is on; grouped products always run on
-    single CTAs).
+    ``kernel``: ``"pair"`` (two CTAs per 512 x 256 tile), ``"single"`` (one CTA per 128 x 256 tile, ``splits`` CTAs along K)
+    or ``"auto"`` (:func:`pick_gemm_plan` for ungrouped products while :data:`PAIR_GEMM` is on; grouped products always run
+    on single CTAs).  ``b2_layout="kn"``: ``b2`` is stored ``[r, N]``.  ``alpha`` scales the fp32 products (not the bias;
+    single-CTA kernel only, so ``"auto"`` takes it when ``alpha`` is given).
     """
     if group_offs is None and kernel == "auto" and PAIR_GEMM:
-        kernel = pick_gemm_kernel(a.shape[0], b.shape[1] if b_layout == "kn" else b.shape[0], a.shape[1], lib.sm_count())
+        kernel, splits = pick_gemm_plan(a.shape[0], b.shape[1] if b_layout == "kn" else b.shape[0], a.shape[1],
+                                        0 if a2 is None else a2.shape[1], lib.sm_count())
+        if alpha != 1.0:
+            kernel = "single"
     if group_offs is None and kernel == "pair":
-        return gemm_pair(a, b, b_layout=b_layout, a2=a2, b2=b2, bias=bias, out=out, status=status,
+        if alpha != 1.0:
+            raise ValueError("alpha runs on the single-CTA kernel")
+        return gemm_pair(a, b, b_layout=b_layout, a2=a2, b2=b2, b2_layout=b2_layout, bias=bias, out=out, status=status,
                          wait_budget_s=wait_budget_s)
     _need_bf16(a, b)
     if a.ndim != 2 or a.stride(1) != 1:
@@ -627,9 +682,9 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, b_layout: str = "nk", a2: torch.Te
     K2 = 0
     if a2 is not None:
         _need_bf16(a2, b2)
-        if a2.shape[0] != M or b2.shape[0] != N or a2.shape[1] != b2.shape[1] or a2.stride(1) != 1 or b2.stride(1) != 1:
-            raise ValueError("low-rank segment: a2 [M, r], b2 [N, r]")
         K2 = a2.shape[1]
+        if a2.shape[0] != M or a2.stride(1) != 1 or _check_b(b2, b2_layout, K2, "b2") != N:
+            raise ValueError("low-rank segment: a2 [M, r], b2 [N, r] (or [r, N])")
     if bias is not None:
         _need_bf16(bias)
         if bias.numel() != N or not bias.is_contiguous():
@@ -638,10 +693,11 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, b_layout: str = "nk", a2: torch.Te
         out = torch.empty(M, N, dtype=torch.bfloat16, device=a.device)
     elif out.shape != (M, N) or out.dtype != torch.bfloat16 or out.stride(1) != 1:
         raise ValueError("out must be a row-major bf16 [M, N] matrix")
+    scratch = torch.empty(splits * -(-M // 128) * 128 * N, dtype=torch.float32, device=a.device) if splits > 1 else None
     rc = lib.load().ob_gemm_tn(a.data_ptr(), b2d.data_ptr(), lib.ptr(a2), lib.ptr(b2), lib.ptr(bias), out.data_ptr(), M, N,
                                K, K2, a.stride(0), b2d.stride(0), a2.stride(0) if a2 is not None else 0,
-                               b2.stride(0) if b2 is not None else 0, out.stride(0), kn, lib.ptr(group_offs), E,
-                               status.ptr() if status else None, wait_budget_s, lib.sm_count(), lib.stream())
+                               b2.stride(0) if b2 is not None else 0, out.stride(0), kn, int(b2_layout == "kn"), alpha,
+                               lib.ptr(group_offs), E, splits, lib.ptr(scratch), status.ptr() if status else None, wait_budget_s, lib.sm_count(), lib.stream())
     lib.check(rc, "gemm")
     return out
 
@@ -814,7 +870,7 @@ from .functional import (activation, add_layer_norm, cross_entropy, cross_entrop
                          layer_norm, merge_heads3, plain_torch_ops, rms_norm, rms_norm_ref, rope_qk, rope_qk_ref, rope_tables, rows_group_sum_, swiglu)
 
 __all__ = [
-    "gemm", "gemm_pair", "gemm_glu", "gemm_glu_bwd", "direct_norm2", "pick_norm_path", "pick_gemm_kernel", "die_map", "set_die_aware_tiles", "linear_ce_forward", "linear_ce_dlogits_", "gemm_glu_ref", "gemm_ref", "ghost_set_wide", "push_grad_", "wgrad_clip_per_example", "wgrad_clip_batch", "wgrad_clip_per_example_batch", "direct_norm2_batch", "ghost_norm_batch", "plain_torch_ops", "layer_norm", "add_layer_norm", "activation", "rows_group_sum_", "merge_heads3",
+    "gemm", "gemm_pair", "lora_pack", "pick_gemm_plan", "gemm_glu", "gemm_glu_bwd", "direct_norm2", "pick_norm_path", "pick_gemm_kernel", "die_map", "set_die_aware_tiles", "linear_ce_forward", "linear_ce_dlogits_", "gemm_glu_ref", "gemm_ref", "ghost_set_wide", "push_grad_", "wgrad_clip_per_example", "wgrad_clip_batch", "wgrad_clip_per_example_batch", "direct_norm2_batch", "ghost_norm_batch", "plain_torch_ops", "layer_norm", "add_layer_norm", "activation", "rows_group_sum_", "merge_heads3",
     "DeviceWaitTimeout", "KernelLibraryError", "StatusWord", "clip_tree", "clip_weighted_sum", "cross_entropy",
     "cross_entropy_ref", "embedding_wgrad", "fused_add_rms_norm", "geglu", "ghost_norm", "ghost_norm_ref", "glu_ref",
     "philox_normal_add_", "pick_block_n", "pick_splits", "rms_norm", "rms_norm_ref", "rope_qk", "rope_qk_ref",

@@ -341,6 +341,22 @@ __device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.b
 // ... have finished altogether (before the kernel gives its shared memory back)
 __device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
+// This lane's row of 32 fp32 values into a 1024-byte aligned [32 x 32] slab in the 128-byte-swizzled layout of the tensor map.
+__device__ __forceinline__ void slab_row32(uint8_t* slab, const float* v, int lane) {
+#pragma unroll
+  for (int c = 0; c < 8; ++c)
+    *reinterpret_cast<float4*>(slab + lane * 128 + ((c ^ (lane & 7)) << 4)) =
+        make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+}
+
+// ... have finished reading shared memory, all but the latest one
+__device__ __forceinline__ void tma_store_wait_read1() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
+// fp32 tile in shared memory added to a 3-D tensor in global memory (elements outside the tensor are dropped)
+__device__ __forceinline__ void tma_reduce_add_3d(const CUtensorMap* map, const void* smem_src, int c0, int c1, int c2) {
+  asm volatile("cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4}], [%1];"
+               ::"l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(smem_src)), "r"(c0), "r"(c1), "r"(c2)
+               : "memory");
+}
 // pk[0 .. 31]: this lane's row of 64 bf16 values, two per register.  `use_tma` is warp-uniform.  Without it (unaligned
 // output, or rows that must be masked at a bound the tensor map does not know) the tile leaves through the slab as
 // 16-byte st.global row segments, or element by element when even that is not aligned.

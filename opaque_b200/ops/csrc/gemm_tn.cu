@@ -15,6 +15,12 @@
 // owns TMEM, warps 2-9 convert fp32 accumulators to bf16 and store them as whole 128-byte row segments (staged through
 // a swizzled shared-memory slab per warp): with a short K (768) the drain of one tile takes about as long as its MMAs,
 // so four warps storing one 16-byte piece per lane and row left the tensor pipe waiting.  Every wait is bounded.
+//
+// Few rows (short records, small microbatches) make few tiles: 128 x 2304 is nine, and nine SMs then pull the whole weight.
+// With `splits` > 1 a tile's k-blocks go to that many CTAs; each stores its fp32 partial tile to scratch (it stays in L2)
+// and gemm_split_sum_kernel adds them in a fixed order, so results repeat bit for bit.
+// Measured (us; launches back to back, weights from HBM; pair kernel / one CTA per tile / split): 256 x 2048 x 8192 79.5 / 52.0 /
+// 18.6 with 8 splits, 128 x 768 x 3072 33.8 / 21.3 / 11.2 with 8, 128 x 768 x 50304 444 / 279 / 27 with 24.
 #include "common.cuh"
 #include "api.h"
 
@@ -22,6 +28,8 @@ namespace ob {
 
 int make_bf16_map_2d(CUtensorMap* map, const void* base, long long rows, long long cols, long long ld,
                      int box_cols, int box_rows);
+int make_f32_map_2d(CUtensorMap* map, const void* base, long long rows, long long cols, long long ld,
+                    int box_cols, int box_rows);
 
 constexpr int GT_BM = 128;
 constexpr int GT_BN = 256;
@@ -45,19 +53,34 @@ struct GemmParams {
   int num_groups;
   int b_group_rows;        // distance, in rows of B, between consecutive groups' slabs
   int tma_store;           // the output leaves through bulk tensor stores (map_out is valid)
+  int b2_kn;               // B2 is [K2, N] (N-major) instead of [N, K2]
+  float alpha;             // scales the products
+  int splits;              // CTAs per tile; > 1: map_out is the fp32 scratch [splits * m_pad, N]
+  int m_pad;               // rows of one split's scratch matrix
   int* status;
   unsigned long long wait_budget_ns;
 };
 
 struct GtItem {
   int row0, row_end, n0, b_row;
+  int kb0, kb1, out_row;     // k-blocks of this item; output row (scratch row with splits) of the tile's first row
 };
 
 // Tile w of the persistent schedule.  `cursor` is the caller's monotone group cursor (grouped mode only).
-__device__ __forceinline__ GtItem gt_decode(const GemmParams& p, int w, int tiles_m, int tiles_n, const int* tile_start,
+template <bool SPLIT>
+__device__ __forceinline__ GtItem gt_decode(const GemmParams& p, int w, int tiles_m, int tiles_n, int num_kb, const int* tile_start,
                                             int& cursor) {
   GtItem it;
+  it.kb0 = 0;
+  it.kb1 = num_kb;
   if (p.group_offs == nullptr) {
+    int split = 0;
+    if constexpr (SPLIT) {
+      split = w / (tiles_m * tiles_n);
+      w -= split * (tiles_m * tiles_n);
+      it.kb0 = static_cast<int>(static_cast<long long>(num_kb) * split / p.splits);
+      it.kb1 = static_cast<int>(static_cast<long long>(num_kb) * (split + 1) / p.splits);
+    }
     const int band = GT_GROUP_M * tiles_n;
     const int b = w / band, r = w % band;
     const int m_in_band = min(GT_GROUP_M, tiles_m - b * GT_GROUP_M);
@@ -67,6 +90,7 @@ __device__ __forceinline__ GtItem gt_decode(const GemmParams& p, int w, int tile
     it.row_end = p.M;
     it.n0 = nt * GT_BN;
     it.b_row = 0;
+    it.out_row = it.row0 + split * p.m_pad;
   } else {
     const int g = w / tiles_n;
     while (g >= tile_start[cursor + 1]) ++cursor;
@@ -74,11 +98,13 @@ __device__ __forceinline__ GtItem gt_decode(const GemmParams& p, int w, int tile
     it.row_end = p.group_offs[cursor + 1];
     it.n0 = (w % tiles_n) * GT_BN;
     it.b_row = cursor * p.b_group_rows;
+    it.out_row = it.row0;
   }
   return it;
 }
 
-template <bool B_KN>
+// SPLIT is a template parameter so that the ordinary epilogue keeps its registers
+template <bool B_KN, bool SPLIT>
 __global__ void __launch_bounds__(GT_THREADS, 1)
 gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                const __grid_constant__ CUtensorMap map_a2, const __grid_constant__ CUtensorMap map_b2,
@@ -138,7 +164,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   const int tiles_m = p.group_offs ? tile_start[p.num_groups] : (p.M + GT_BM - 1) / GT_BM;
-  const int total_work = tiles_m * tiles_n;
+  const int total_work = tiles_m * tiles_n * p.splits;
 
   if (warp == 0) {
     if (lane == 0) {
@@ -146,8 +172,8 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       uint32_t phase = 0, issued_mask = 0, issued_phase = 0;
       bool ok = true;
       for (int w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
-        const GtItem it = gt_decode(p, w, tiles_m, tiles_n, tile_start, cursor);
-        for (int kb = 0; kb < num_kb; ++kb) {
+        const GtItem it = gt_decode<SPLIT>(p, w, tiles_m, tiles_n, num_kb, tile_start, cursor);
+        for (int kb = it.kb0; kb < it.kb1; ++kb) {
           if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, p.status, OB_ERR_WAIT_EMPTY, budget)) {
             ok = false;
             break;
@@ -166,7 +192,13 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             }
           } else {
             tma_load_2d(a_dst, &map_a2, &full[stage], (kb - nk1) * GT_BK, it.row0);
-            tma_load_2d(b_dst, &map_b2, &full[stage], (kb - nk1) * GT_BK, it.n0);
+            if (p.b2_kn) {
+#pragma unroll
+              for (int j = 0; j < GT_BN / 64; ++j)
+                tma_load_2d(b_dst + j * (GT_BK * 128), &map_b2, &full[stage], it.n0 + 64 * j, (kb - nk1) * GT_BK);
+            } else {
+              tma_load_2d(b_dst, &map_b2, &full[stage], (kb - nk1) * GT_BK, it.n0);
+            }
           }
           issued_mask |= 1u << stage;
           issued_phase = (issued_phase & ~(1u << stage)) | (phase << stage);
@@ -183,12 +215,13 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     }
   } else if (warp == 1) {
     if (lane == 0) {
-      constexpr uint32_t idesc_main = make_idesc_bf16(GT_BM, GT_BN, 0, B_KN ? 1 : 0);
+      constexpr uint32_t idesc_nmaj = make_idesc_bf16(GT_BM, GT_BN, 0, 1);
       constexpr uint32_t idesc_kmaj = make_idesc_bf16(GT_BM, GT_BN, 0, 0);
-      int stage = 0, acc_iter = 0;
+      int stage = 0, acc_iter = 0, cursor = 0;
       uint32_t phase = 0;
       bool ok = true;
       for (int w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
+        const GtItem it = gt_decode<SPLIT>(p, w, tiles_m, tiles_n, num_kb, tile_start, cursor);
         const int as = acc_iter & 1;
         if (!mbar_wait(&tmem_empty[as], ((acc_iter >> 1) & 1) ^ 1, abort_flag, p.status, OB_ERR_WAIT_TMEM_EMPTY,
                        budget)) {
@@ -197,7 +230,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + as * GT_BN;
-        for (int kb = 0; kb < num_kb; ++kb) {
+        for (int kb = it.kb0; kb < it.kb1; ++kb) {
           if (!mbar_wait(&full[stage], phase, abort_flag, p.status, OB_ERR_WAIT_FULL, budget)) {
             ok = false;
             break;
@@ -205,7 +238,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           tc_fence_after();
           const uint32_t a_addr = smem_u32(smem + stage * GT_STAGE_BYTES);
           const uint32_t b_addr = a_addr + GT_A_BYTES;
-          const bool kn = B_KN && kb < nk1;
+          const bool kn = kb < nk1 ? B_KN : p.b2_kn != 0;
 #pragma unroll
           for (int kk = 0; kk < GT_BK / 16; ++kk) {
             // K-major operand: rows 128 B apart, 8-row groups 1024 B apart, 32 B per 16-element k-step.
@@ -213,7 +246,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             const uint64_t ad = make_smem_desc(a_addr + kk * 32, 16, 1024, 2);
             const uint64_t bd = kn ? make_smem_desc(b_addr + kk * (16 * 128), GT_BK * 128, 1024, 2)
                                    : make_smem_desc(b_addr + kk * 32, 16, 1024, 2);
-            umma_bf16(d_tmem, ad, bd, kn ? idesc_main : idesc_kmaj, (kb > 0 || kk > 0) ? 1u : 0u);
+            umma_bf16(d_tmem, ad, bd, kn ? idesc_nmaj : idesc_kmaj, (kb > it.kb0 || kk > 0) ? 1u : 0u);
           }
           umma_commit(&empty[stage]);
           if (++stage == GT_STAGES) { stage = 0; phase ^= 1; }
@@ -234,7 +267,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     bool ok = true;
     const bool vec_ok = ((p.ldo & 7) == 0) && ((reinterpret_cast<uintptr_t>(p.out) & 15) == 0);
     for (int w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
-      const GtItem it = gt_decode(p, w, tiles_m, tiles_n, tile_start, cursor);
+      const GtItem it = gt_decode<SPLIT>(p, w, tiles_m, tiles_n, num_kb, tile_start, cursor);
       const int as = acc_iter & 1;
       if (!mbar_wait(&tmem_full[as], (acc_iter >> 1) & 1, abort_flag, p.status, OB_ERR_WAIT_TMEM_FULL, budget)) {
         ok = false;
@@ -243,35 +276,67 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       tc_fence_after();
       const int row0 = it.row0 + q * 32;
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + as * GT_BN + g * (GT_BN / 2);
-      // Both 64-column rounds go to registers (packed bf16) first, so the accumulator is back with the tensor pipe before
-      // a single store is issued.  Tiles that end inside a group's rows are masked by hand; all others leave through
-      // bulk tensor stores, which clip at the tensor's own bounds.
-      uint32_t pk[2][32];
+      if constexpr (SPLIT) {
+        // partial product: fp32, 32 x 32 values per bulk tensor store (columns past N are clipped; rows past M land in the
+        // padding of this split's scratch matrix)
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        const int nc = it.n0 + g * (GT_BN / 2) + c * 64;
-        if (nc < p.N) {
-          float v[64];
-          tmem_ld32(t_row + c * 64, v);
-          tmem_ld32(t_row + c * 64 + 32, v + 32);
-          tmem_ld_wait();
-          if (p.bias != nullptr) add_bias64(v, p.bias, nc, p.N);
-#pragma unroll
-          for (int j = 0; j < 32; ++j) pk[c][j] = pack_bf16x2(v[2 * j], v[2 * j + 1]);
+        for (int c = 0; c < 4; ++c) {
+          const int nc = it.n0 + g * (GT_BN / 2) + c * 32;
+          if (nc < p.N) {
+            float v[32];
+            tmem_ld32(t_row + c * 32, v);
+            tmem_ld_wait();
+            if (lane == 0) tma_store_wait_read();
+            __syncwarp();
+            slab_row32(slab, v, lane);
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              tma_store_2d(&map_out, slab, nc, it.out_row + q * 32);
+              tma_store_commit();
+            }
+          }
         }
-      }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&tmem_empty[as]);
-      const bool use_tma = p.tma_store != 0 && (p.group_offs == nullptr || row0 + 32 <= it.row_end);
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&tmem_empty[as]);
+        ++acc_iter;
+        continue;
+      } else {
+        // Both 64-column rounds go to registers (packed bf16) first, so the accumulator is back with the tensor pipe before
+        // a single store is issued.  Tiles that end inside a group's rows are masked by hand; all others leave through
+        // bulk tensor stores, which clip at the tensor's own bounds.
+        uint32_t pk[2][32];
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        const int nc = it.n0 + g * (GT_BN / 2) + c * 64;
-        if (nc < p.N)
-          store_tile64_packed(slab, pk[c], &map_out, use_tma, nc, row0, p.out, p.ldo, it.row_end - row0, p.N - nc, vec_ok,
-                              lane);
+        for (int c = 0; c < 2; ++c) {
+          const int nc = it.n0 + g * (GT_BN / 2) + c * 64;
+          if (nc < p.N) {
+            float v[64];
+            tmem_ld32(t_row + c * 64, v);
+            tmem_ld32(t_row + c * 64 + 32, v + 32);
+            tmem_ld_wait();
+            if (p.alpha != 1.f) {
+#pragma unroll
+              for (int j = 0; j < 64; ++j) v[j] *= p.alpha;
+            }
+            if (p.bias != nullptr) add_bias64(v, p.bias, nc, p.N);
+#pragma unroll
+            for (int j = 0; j < 32; ++j) pk[c][j] = pack_bf16x2(v[2 * j], v[2 * j + 1]);
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&tmem_empty[as]);
+        const bool use_tma = p.tma_store != 0 && (p.group_offs == nullptr || row0 + 32 <= it.row_end);
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const int nc = it.n0 + g * (GT_BN / 2) + c * 64;
+          if (nc < p.N)
+            store_tile64_packed(slab, pk[c], &map_out, use_tma, nc, row0, p.out, p.ldo, it.row_end - row0, p.N - nc, vec_ok,
+                                lane);
+        }
+        ++acc_iter;
       }
-      ++acc_iter;
     }
     if (lane == 0) tma_store_wait_all();         // this lane's bulk stores are done before shared memory is given back
   }
@@ -284,17 +349,51 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   }
 }
 
+// out[m, n] = alpha * sum over splits of part[s][m][n] + bias[n], splits added in order; 4 columns per thread.
+__global__ void __launch_bounds__(256)
+gemm_split_sum_kernel(const float* __restrict__ part, const __nv_bfloat16* __restrict__ bias, __nv_bfloat16* __restrict__ out,
+                      int M, int N, int m_pad, int splits, long long ldo, float alpha, int vec) {
+  const int n4 = N >> 2;
+  const long long total = static_cast<long long>(M) * n4, step = static_cast<long long>(m_pad) * N;
+  for (long long i = blockIdx.x * 256LL + threadIdx.x; i < total; i += gridDim.x * 256LL) {
+    const int m = static_cast<int>(i / n4), n = static_cast<int>(i % n4) * 4;
+    const float* src = part + static_cast<long long>(m) * N + n;
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+    for (int s = 0; s < splits; ++s) {
+      const float4 v = __ldg(reinterpret_cast<const float4*>(src + s * step));
+      a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w;
+    }
+    float f[4] = {a.x * alpha, a.y * alpha, a.z * alpha, a.w * alpha};
+    if (bias != nullptr) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) f[j] += __bfloat162float(__ldg(bias + n + j));
+    }
+    __nv_bfloat16* dst = out + m * ldo + n;
+    if (vec) {
+      *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]));
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) dst[j] = __float2bfloat16_rn(f[j]);
+    }
+  }
+}
+
 }  // namespace ob
 
 extern "C" int ob_gemm_tn(const void* a, const void* b, const void* a2, const void* b2, const void* bias, void* out,
                           long long rows_a, int N, int K1, int K2, long long lda, long long ldb, long long lda2,
-                          long long ldb2, long long ldo, int b_kn, const int* group_offs, int num_groups,
-                          int* status, double wait_budget_s, int num_sms, void* stream) {
+                          long long ldb2, long long ldo, int b_kn, int b2_kn, float alpha, const int* group_offs, int num_groups,
+                          int splits, float* scratch, int* status, double wait_budget_s, int num_sms, void* stream) {
   using namespace ob;
   if (rows_a <= 0 || N <= 0 || K1 <= 0) return 0;
   if (rows_a > 0x7fffffffLL - GT_BM) return -40;
   if (group_offs != nullptr && (num_groups < 1 || num_groups > GT_MAX_GROUPS)) return -41;
   if (K2 > 0 && (a2 == nullptr || b2 == nullptr)) return -42;
+  const int nk = (K1 + GT_BK - 1) / GT_BK + (K2 + GT_BK - 1) / GT_BK;
+  if (splits < 1) splits = 1;
+  if (splits > 1 && (group_offs != nullptr || splits > nk || (N & 3) || scratch == nullptr || (reinterpret_cast<uintptr_t>(scratch) & 15)))
+    return -45;
   const int groups = group_offs ? num_groups : 1;
   CUtensorMap ma, mb, ma2, mb2;
   int rc = make_bf16_map_2d(&ma, a, rows_a, K1, lda, GT_BK, GT_BM);
@@ -307,7 +406,7 @@ extern "C" int ob_gemm_tn(const void* a, const void* b, const void* a2, const vo
   if (K2 > 0) {
     rc = make_bf16_map_2d(&ma2, a2, rows_a, K2, lda2, GT_BK, GT_BM);
     if (rc) return rc;
-    rc = make_bf16_map_2d(&mb2, b2, N, K2, ldb2, GT_BK, GT_BN);
+    rc = b2_kn ? make_bf16_map_2d(&mb2, b2, K2, N, ldb2, 64, GT_BK) : make_bf16_map_2d(&mb2, b2, N, K2, ldb2, GT_BK, GT_BN);
     if (rc) return rc;
   } else {
     ma2 = ma;
@@ -315,9 +414,10 @@ extern "C" int ob_gemm_tn(const void* a, const void* b, const void* a2, const vo
   }
   static bool configured = false;
   if (!configured) {
-    if (cudaFuncSetAttribute(gemm_tn_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, GT_SMEM) != cudaSuccess ||
-        cudaFuncSetAttribute(gemm_tn_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, GT_SMEM) != cudaSuccess)
-      return -43;
+    const void* kernels[4] = {reinterpret_cast<const void*>(gemm_tn_kernel<false, false>), reinterpret_cast<const void*>(gemm_tn_kernel<true, false>),
+                              reinterpret_cast<const void*>(gemm_tn_kernel<false, true>), reinterpret_cast<const void*>(gemm_tn_kernel<true, true>)};
+    for (const void* k : kernels)
+      if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, GT_SMEM) != cudaSuccess) return -43;
     configured = true;
   }
   GemmParams p;
@@ -333,16 +433,34 @@ extern "C" int ob_gemm_tn(const void* a, const void* b, const void* a2, const vo
   p.wait_budget_ns = static_cast<unsigned long long>(wait_budget_s * 1e9);
   const long long tiles_n = (N + GT_BN - 1) / GT_BN;
   const long long tiles_m_bound = (rows_a + GT_BM - 1) / GT_BM + (group_offs ? groups : 0);
-  const long long total = tiles_m_bound * tiles_n;
+  p.b2_kn = b2_kn;
+  p.alpha = alpha;
+  p.splits = splits;
+  const long long m_pad = (rows_a + GT_BM - 1) / GT_BM * GT_BM;
+  if (splits > 1 && m_pad * splits > 0x7fffffffLL) return -40;
+  p.m_pad = static_cast<int>(m_pad);
+  const long long total = tiles_m_bound * tiles_n * splits;
+  if (total > 0x7fffffffLL - num_sms) return -40;
   const int grid = static_cast<int>(total < num_sms ? total : num_sms);
   CUtensorMap mo = ma;
   p.tma_store = 0;
-  if ((reinterpret_cast<uintptr_t>(out) & 15) == 0 && ((ldo * 2) & 15) == 0 &&
+  if (splits > 1) {
+    rc = make_f32_map_2d(&mo, scratch, m_pad * splits, N, N, 32, 32);
+    if (rc) return rc;
+  } else if ((reinterpret_cast<uintptr_t>(out) & 15) == 0 && ((ldo * 2) & 15) == 0 &&
       make_bf16_map_2d(&mo, out, rows_a, N, ldo, 64, 32) == 0)
     p.tma_store = 1;
-  if (b_kn)
-    gemm_tn_kernel<true><<<grid, GT_THREADS, GT_SMEM, static_cast<cudaStream_t>(stream)>>>(ma, mb, ma2, mb2, mo, p);
-  else
-    gemm_tn_kernel<false><<<grid, GT_THREADS, GT_SMEM, static_cast<cudaStream_t>(stream)>>>(ma, mb, ma2, mb2, mo, p);
+  const cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (splits > 1) {
+    if (b_kn) gemm_tn_kernel<true, true><<<grid, GT_THREADS, GT_SMEM, st>>>(ma, mb, ma2, mb2, mo, p);
+    else gemm_tn_kernel<false, true><<<grid, GT_THREADS, GT_SMEM, st>>>(ma, mb, ma2, mb2, mo, p);
+    const long long blocks = (rows_a * (N >> 2) + 255) / 256, cap = num_sms * 8LL;
+    gemm_split_sum_kernel<<<static_cast<unsigned>(blocks < cap ? blocks : cap), 256, 0, st>>>(
+        scratch, p.bias, p.out, p.M, N, p.m_pad, splits, ldo, alpha, (ldo & 3) == 0 && (reinterpret_cast<uintptr_t>(out) & 7) == 0);
+  } else if (b_kn) {
+    gemm_tn_kernel<true, false><<<grid, GT_THREADS, GT_SMEM, st>>>(ma, mb, ma2, mb2, mo, p);
+  } else {
+    gemm_tn_kernel<false, false><<<grid, GT_THREADS, GT_SMEM, st>>>(ma, mb, ma2, mb2, mo, p);
+  }
   return cudaGetLastError() == cudaSuccess ? 0 : -44;
 }
