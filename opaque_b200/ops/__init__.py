@@ -114,7 +114,7 @@ def _batch_splits(tiles: int, rows: int, max_splits: int | None = None, peer: bo
 def wgrad_clip_batch(problems: Sequence[dict], out: torch.Tensor | None, *, accumulate: bool = True, peer_table: torch.Tensor | None = None,
                      shard_elems: int = 0, block_n: int = 256, status: StatusWord | None = None,
                      wait_budget_s: float = DEFAULT_WAIT_BUDGET_S) -> None:
-    """Several :func:`wgrad_clip` problems with one destination in one launch (per 64): dictionaries with that function's
+    """Several :func:`wgrad_clip` problems with one destination in one launch (per 56): dictionaries with that function's
     ``a``, ``b`` and optional ``row_scale``, ``seg_offsets``, ``num_groups``, ``out_offset``, ``ldm``, ``ldn``, ``n_valid``,
     ``group_stride``.  ``block_n`` is 256 or 64.  K is split (``accumulate`` only, ungrouped problems) when the whole list
     would leave SMs idle."""
@@ -255,7 +255,7 @@ def _check_pe(a, b, rows_per_example) -> tuple[int, int, int, int]:
 def wgrad_clip_per_example_batch(problems: Sequence[tuple], out: torch.Tensor | None, rows_per_example: int, *,
                                  peer_table: torch.Tensor | None = None, shard_elems: int = 0, status: StatusWord | None = None,
                                  wait_budget_s: float = DEFAULT_WAIT_BUDGET_S) -> None:
-    """Several accumulating :func:`wgrad_clip_per_example` problems ``(a, b, ex_scale, out_offset, ldm)`` in one launch (per 64)."""
+    """Several accumulating :func:`wgrad_clip_per_example` problems ``(a, b, ex_scale, out_offset, ldm)`` in one launch (per 56)."""
     tiles = sum(math.ceil(pr[0].shape[1] / 128) * math.ceil(pr[1].shape[1] / 256) for pr in problems)
     descs = []
     for a, b, ex_scale, off, ldm in problems:
@@ -281,7 +281,7 @@ def wgrad_clip_per_example_batch(problems: Sequence[tuple], out: torch.Tensor | 
 
 def direct_norm2_batch(problems: Sequence[tuple], rows_per_example: int, *, status: StatusWord | None = None,
                        wait_budget_s: float = DEFAULT_WAIT_BUDGET_S) -> None:
-    """Several :func:`direct_norm2` problems ``(a, g, norm2)`` in one launch (per 64)."""
+    """Several :func:`direct_norm2` problems ``(a, g, norm2)`` in one launch (per 56)."""
     tiles = sum(math.ceil(pr[0].shape[1] / 128) * math.ceil(pr[1].shape[1] / 256) for pr in problems)
     descs = []
     for a, g, norm2 in problems:
@@ -336,7 +336,7 @@ def _check_ghost(a, g, norm2, tokens_per_example, ids, seg_offsets, seg_out):
 
 def ghost_norm_batch(problems: Sequence[tuple], *, status: StatusWord | None = None, wait_budget_s: float = DEFAULT_WAIT_BUDGET_S) -> None:
     """Several :func:`ghost_norm` problems ``(a, g, norm2, tokens_per_example, ids, seg_offsets, seg_out)`` in one launch per
-    Gram block shape (and per 64 problems): their items share one work list, longest first."""
+    Gram block shape (and per 56 problems): their items share one work list, longest first."""
     jobs = []
     for a, g, norm2, tokens, ids, seg_offsets, seg_out in problems:
         rows, B, da, dg, lda, ap = _check_ghost(a, g, norm2, tokens, ids, seg_offsets, seg_out)

@@ -26,7 +26,7 @@ int ob_ghost_norm(const void* a, const void* g, const int* ids, int B, int T, in
                   long long ldg, float* norm2, const int* seg, const int* seg_out, long long total_rows, int* status,
                   double wait_budget_s, int num_sms, void* stream);
 
-// Several problems in one launch (host arrays of descriptions; launches hold up to 64): the layers of a backward pass
+// Several problems in one launch (host arrays of descriptions; launches hold up to 56): the layers of a backward pass
 // share one work list.  Fields as in the single calls above; put problems with more work per item first.
 typedef struct {
   const void *a, *g;

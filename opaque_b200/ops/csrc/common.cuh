@@ -207,12 +207,13 @@ __host__ __device__ constexpr uint32_t make_idesc_bf16(int m, int n, int a_mn_ma
 // Several problems of one kernel in one launch.  The persistent CTAs walk ONE work list: problem i owns items
 // [start[i], start[i + 1]).  A layer of a small model has fewer items than the chip has SMs; the layers of a backward pass
 // together fill it, and cost one launch.  The whole struct is a kernel parameter (tensor maps must be, or live in global
-// memory that a copy would have to fill first); 64 problems stay below the 32 764-byte parameter limit.
-constexpr int BATCH_CAP = 64;
+// memory that a copy would have to fill first); 56 problems stay below the 32 764-byte parameter limit.
+constexpr int BATCH_CAP = 56;
 template <class Params, int CAP>
 struct alignas(64) TmaBatch {
   CUtensorMap map_a[CAP];
   CUtensorMap map_b[CAP];
+  CUtensorMap map_out[CAP];      // kernels that reduce their tiles into memory through the TMA engine
   Params p[CAP];
   int start[CAP + 1];
   int* status;

@@ -1,5 +1,5 @@
 """Batched launches of the norm and weight-gradient kernels: the same problems one by one give the same numbers, whatever
-their number (one launch holds 64), shapes, order and destination.  Sums are fp32 in both; only atomics' order differs."""
+their number (one launch holds 56), shapes, order and destination.  Sums are fp32 in both; only atomics' order differs."""
 from __future__ import annotations
 
 import pytest
@@ -98,3 +98,32 @@ def test_per_example_kernels_batched(count):
     n2 = torch.zeros(count, B, device="cuda")
     ops.direct_norm2_batch([(p[0], p[1], n2[i]) for i, p in enumerate(probs)], R, status=st)
     assert st.read() == 0 and _rel(n2, torch.stack(norms)) < 2e-5
+
+
+@pytest.mark.parametrize("offset", [0, 4, 1])
+@pytest.mark.parametrize("M,N,ldm", [(8, 136, 136), (130, 140, 140), (257, 264, 300), (40, 520, 521)])
+def test_accumulating_destinations(offset, M, N, ldm):
+    """Grouped and dense accumulation into aligned destinations (reduced by the TMA engine) and unaligned ones (by the warps):
+    nothing outside the matrices is touched, empty groups add nothing."""
+    from opaque_b200 import ops
+    offs = torch.tensor([0, 70, 70, 199, 200], device="cuda", dtype=torch.int32)
+    a, b = (_r(200, (w + 7) // 8 * 8)[:, :w] for w in (M, N))
+    gstride = M * ldm + 4
+    ref = ops.wgrad_clip_ref(a, b, seg_offsets=offs, num_groups=4)
+    out = torch.full((offset + 5 * gstride,), 3.0, device="cuda")
+    want, inside = out.clone(), torch.zeros_like(out, dtype=torch.bool)
+    for g in range(5):
+        want[offset + g * gstride:][:M * ldm].view(M, ldm)[:, :N] += 2 * ref[g] if g < 4 else ref.sum(0)
+        inside[offset + g * gstride:][:M * ldm].view(M, ldm)[:, :N] = True
+    st = ops.StatusWord()
+    for _ in range(2):
+        ops.wgrad_clip_batch([dict(a=a, b=b, seg_offsets=offs, num_groups=4, out_offset=offset, ldm=ldm, group_stride=gstride)], out, status=st)
+    ops.wgrad_clip_batch([dict(a=a, b=b, out_offset=offset + 4 * gstride, ldm=ldm)], out, status=st)
+    assert st.read() == 0 and _rel(out, want) < 1e-5 and bool((out[~inside] == 3.0).all())
+    if offset == 0:                                       # the per-example kernel's destination, two examples of 64 rows
+        c = torch.tensor([0.5, 2.0], device="cuda")
+        out2 = torch.full((M * ldm + 8,), 3.0, device="cuda")
+        ops.wgrad_clip_per_example_batch([(a[:128], b[:128], c, 0, ldm)], out2, 64, status=st)
+        w2 = torch.full_like(out2, 3.0)
+        w2[:M * ldm].view(M, ldm)[:, :N] += ops.wgrad_clip_ref(a[:128], b[:128], row_scale=c.repeat_interleave(64))[0]
+        assert st.read() == 0 and _rel(out2, w2) < 1e-5 and bool((out2[:M * ldm].view(M, ldm)[:, N:] == 3.0).all()) and bool((out2[M * ldm:] == 3.0).all())
