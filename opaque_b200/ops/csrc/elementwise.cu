@@ -124,7 +124,11 @@ __device__ __forceinline__ float row_group_sum(float v, float* red) {     // red
   return t;
 }
 
-template <int VPT>
+// Bound by memory (x, residual in; sum, y out), and by how many loads a thread has in flight: ALL of its loads are issued
+// before the first value is used.  RES (the residual addition) is a template parameter so that no branch stands between
+// them: with a run-time test per vector the loads went out in VPT dependent groups.
+// Measured at 16384 x 4096 inside a training step: 139.6 -> 131.1 us forward, 124.7 -> 121.5 us backward.
+template <int VPT, bool RES>
 __global__ void __launch_bounds__(2 * RN_ROW_THREADS)
 rmsnorm_fwd_reg_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ residual,
                        const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
@@ -137,22 +141,33 @@ rmsnorm_fwd_reg_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16*
   const bool live = row < rows;
   const long long r = live ? row : rows - 1;               // dead group mirrors the last row (keeps the barriers uniform)
   const bf16x8* xr = reinterpret_cast<const bf16x8*>(x + r * H);
+  bf16x8 raw[VPT], add[RES ? VPT : 1];
+#pragma unroll
+  for (int v = 0; v < VPT; ++v) {
+    raw[v] = xr[t + v * RN_ROW_THREADS];
+    if constexpr (RES) add[v] = reinterpret_cast<const bf16x8*>(residual + r * H)[t + v * RN_ROW_THREADS];
+  }
   float f[VPT][8];
   float ss = 0.f;
 #pragma unroll
   for (int v = 0; v < VPT; ++v) {
-    unpack8(xr[t + v * RN_ROW_THREADS], f[v]);
-    if (residual != nullptr) {
+    unpack8(raw[v], f[v]);
+    if constexpr (RES) {
       float g[8];
-      unpack8(reinterpret_cast<const bf16x8*>(residual + r * H)[t + v * RN_ROW_THREADS], g);
+      unpack8(add[v], g);
 #pragma unroll
       for (int j = 0; j < 8; ++j) f[v][j] += g[j];
-      const bf16x8 sv = pack8(f[v]);
-      if (live) reinterpret_cast<bf16x8*>(sum_out + r * H)[t + v * RN_ROW_THREADS] = sv;
-      unpack8(sv, f[v]);                                    // the normalised tensor is the stored (rounded) sum
+      raw[v] = pack8(f[v]);
+      unpack8(raw[v], f[v]);                                // the normalised tensor is the stored (rounded) sum
     }
 #pragma unroll
     for (int j = 0; j < 8; ++j) ss += f[v][j] * f[v][j];
+  }
+  if constexpr (RES) {
+    if (live) {
+#pragma unroll
+      for (int v = 0; v < VPT; ++v) reinterpret_cast<bf16x8*>(sum_out + r * H)[t + v * RN_ROW_THREADS] = raw[v];
+    }
   }
   const float rs = rsqrtf(row_group_sum(ss, red_all[grp]) / H + eps);
   if (live && t == 0) rstd[row] = rs;
@@ -170,7 +185,9 @@ rmsnorm_fwd_reg_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16*
   }
 }
 
-template <int VPT>
+// As in the forward kernel every load is issued up front; the residual branch's gradient used to be loaded behind the row's
+// reduction, a second trip to memory per row.
+template <int VPT, bool RES>
 __global__ void __launch_bounds__(2 * RN_ROW_THREADS)
 rmsnorm_bwd_dx_reg_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                           const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd,
@@ -183,13 +200,20 @@ rmsnorm_bwd_dx_reg_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloa
   const bool live = row < rows;
   const long long r = live ? row : rows - 1;
   const float rs = rstd[r];
+  bf16x8 raw_g[VPT], raw_x[VPT], raw_d[RES ? VPT : 1];
+#pragma unroll
+  for (int v = 0; v < VPT; ++v) {
+    raw_g[v] = reinterpret_cast<const bf16x8*>(dy + r * H)[t + v * RN_ROW_THREADS];
+    raw_x[v] = reinterpret_cast<const bf16x8*>(x + r * H)[t + v * RN_ROW_THREADS];
+    if constexpr (RES) raw_d[v] = reinterpret_cast<const bf16x8*>(dsum_in + r * H)[t + v * RN_ROW_THREADS];
+  }
   float gw[VPT][8], xv[VPT][8];
   float dot = 0.f;
 #pragma unroll
   for (int v = 0; v < VPT; ++v) {
     float c[8];
-    unpack8(reinterpret_cast<const bf16x8*>(dy + r * H)[t + v * RN_ROW_THREADS], gw[v]);
-    unpack8(reinterpret_cast<const bf16x8*>(x + r * H)[t + v * RN_ROW_THREADS], xv[v]);
+    unpack8(raw_g[v], gw[v]);
+    unpack8(raw_x[v], xv[v]);
     unpack8(reinterpret_cast<const bf16x8*>(w)[t + v * RN_ROW_THREADS], c);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -201,11 +225,11 @@ rmsnorm_bwd_dx_reg_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloa
 #pragma unroll
   for (int v = 0; v < VPT; ++v) {
     float d[8];
-    if (dsum_in != nullptr) unpack8(reinterpret_cast<const bf16x8*>(dsum_in + r * H)[t + v * RN_ROW_THREADS], d);
+    if constexpr (RES) unpack8(raw_d[v], d);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       float g = rs * (gw[v][j] - xv[v][j] * mean);
-      if (dsum_in != nullptr) g += d[j];
+      if constexpr (RES) g += d[j];
       gw[v][j] = g;
     }
     if (live) reinterpret_cast<bf16x8*>(dx + r * H)[t + v * RN_ROW_THREADS] = pack8(gw[v]);
@@ -573,7 +597,11 @@ extern "C" int ob_rmsnorm_fwd(const void* x, const void* residual, const void* w
                       *wp = static_cast<const __nv_bfloat16*>(w);
   __nv_bfloat16 *yp = static_cast<__nv_bfloat16*>(y), *sp = static_cast<__nv_bfloat16*>(sum_out);
   const unsigned pairs = static_cast<unsigned>((rows + 1) / 2);
-#define OB_RN_FWD(V) rmsnorm_fwd_reg_kernel<V><<<pairs, 2 * RN_ROW_THREADS, 0, st>>>(xp, rp, wp, yp, sp, rstd, rows, eps, offset, mode)
+#define OB_RN_FWD(V)                                                                                                            \
+  do {                                                                                                                          \
+    if (rp != nullptr) rmsnorm_fwd_reg_kernel<V, true><<<pairs, 2 * RN_ROW_THREADS, 0, st>>>(xp, rp, wp, yp, sp, rstd, rows, eps, offset, mode); \
+    else rmsnorm_fwd_reg_kernel<V, false><<<pairs, 2 * RN_ROW_THREADS, 0, st>>>(xp, rp, wp, yp, sp, rstd, rows, eps, offset, mode);              \
+  } while (0)
   if (H == 1024) OB_RN_FWD(1);
   else if (H == 2048) OB_RN_FWD(2);
   else if (H == 4096) OB_RN_FWD(4);
@@ -594,7 +622,11 @@ extern "C" int ob_rmsnorm_bwd(const void* dy, const void* x, const void* w, cons
                         *wp = static_cast<const __nv_bfloat16*>(w), *dp = static_cast<const __nv_bfloat16*>(dsum_in);
     __nv_bfloat16* op = static_cast<__nv_bfloat16*>(dx);
     const unsigned pairs = static_cast<unsigned>((rows + 1) / 2);
-#define OB_RN_BWD(V) rmsnorm_bwd_dx_reg_kernel<V><<<pairs, 2 * RN_ROW_THREADS, 0, st>>>(gp, xp, wp, rstd, dp, op, rows, offset)
+#define OB_RN_BWD(V)                                                                                                            \
+  do {                                                                                                                          \
+    if (dp != nullptr) rmsnorm_bwd_dx_reg_kernel<V, true><<<pairs, 2 * RN_ROW_THREADS, 0, st>>>(gp, xp, wp, rstd, dp, op, rows, offset); \
+    else rmsnorm_bwd_dx_reg_kernel<V, false><<<pairs, 2 * RN_ROW_THREADS, 0, st>>>(gp, xp, wp, rstd, dp, op, rows, offset);              \
+  } while (0)
     if (H == 1024) OB_RN_BWD(1);
     else if (H == 2048) OB_RN_BWD(2);
     else if (H == 4096) OB_RN_BWD(4);
