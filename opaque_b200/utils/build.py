@@ -111,6 +111,97 @@ def build_kernels(force: bool = False, verbose: bool = False) -> Path:
     return KERNEL_LIB
 
 
+def launcher_ext_path() -> Path:
+    suffix = sysconfig.get_config_var("EXT_SUFFIX") or ".so"
+    return PKG / "ops" / ("_launch" + suffix)
+
+
+def launcher_source(signatures: dict[str, str]) -> str:
+    """C source of the extension that calls the kernel library's entry points.
+
+    ``signatures`` maps an entry point to one letter per argument: ``P`` pointer (an address, ``bytes`` or ``None``), ``I`` int,
+    ``L`` long long, ``U`` unsigned, ``Q`` unsigned long long, ``F`` float, ``D`` double.  Every entry point becomes a function
+    of the same name that converts its arguments and calls the address handed to ``bind``, without the interpreter lock.
+    """
+    ctype = {"P": "void*", "I": "int", "L": "long long", "U": "unsigned", "Q": "unsigned long long", "F": "float", "D": "double"}
+    out = ["#define PY_SSIZE_T_CLEAN", "#include <Python.h>", "#include <string.h>", """
+static int to_ptr(PyObject* o, void** v) {
+  if (o == Py_None) { *v = NULL; return 0; }
+  if (PyLong_Check(o)) { *v = PyLong_AsVoidPtr(o); return (*v == NULL && PyErr_Occurred()) ? -1 : 0; }
+  if (PyBytes_Check(o)) { *v = PyBytes_AS_STRING(o); return 0; }
+  PyErr_Format(PyExc_TypeError, "expected an address, bytes or None, got %.80s", Py_TYPE(o)->tp_name);
+  return -1;
+}
+static int to_ll(PyObject* o, long long* v) { *v = PyLong_AsLongLong(o); return (*v == -1 && PyErr_Occurred()) ? -1 : 0; }
+static int to_int(PyObject* o, int* v) {
+  long long x;
+  if (to_ll(o, &x)) return -1;
+  if (x < INT_MIN || x > INT_MAX) { PyErr_SetString(PyExc_OverflowError, "argument does not fit an int"); return -1; }
+  *v = (int)x;
+  return 0;
+}
+static int to_ull(PyObject* o, unsigned long long* v) { *v = PyLong_AsUnsignedLongLongMask(o); return (*v == (unsigned long long)-1 && PyErr_Occurred()) ? -1 : 0; }
+static int to_uint(PyObject* o, unsigned* v) { unsigned long long x; if (to_ull(o, &x)) return -1; *v = (unsigned)x; return 0; }
+static int to_double(PyObject* o, double* v) { *v = PyFloat_AsDouble(o); return (*v == -1.0 && PyErr_Occurred()) ? -1 : 0; }
+static int to_float(PyObject* o, float* v) { double x; if (to_double(o, &x)) return -1; *v = (float)x; return 0; }
+"""]
+    conv = {"P": "to_ptr", "I": "to_int", "L": "to_ll", "U": "to_uint", "Q": "to_ull", "F": "to_float", "D": "to_double"}
+    for name, sig in signatures.items():
+        params = ", ".join(ctype[c] for c in sig)
+        out.append(f"static int (*p_{name})({params});")
+        out.append(f"static PyObject* w_{name}(PyObject* self, PyObject* const* a, Py_ssize_t n) {{")
+        out.append(f'  if (n != {len(sig)}) {{ PyErr_Format(PyExc_TypeError, "{name} takes {len(sig)} arguments, got %zd", n); return NULL; }}')
+        out.append(f'  if (p_{name} == NULL) {{ PyErr_SetString(PyExc_RuntimeError, "{name} is not bound"); return NULL; }}')
+        for i, c in enumerate(sig):
+            out.append(f"  {ctype[c]} v{i}; if ({conv[c]}(a[{i}], &v{i})) return NULL;")
+        call = ", ".join(f"v{i}" for i in range(len(sig)))
+        out.append(f"  int rc; Py_BEGIN_ALLOW_THREADS rc = p_{name}({call}); Py_END_ALLOW_THREADS")
+        out.append("  return PyLong_FromLong(rc);\n}")
+    out.append("static PyObject* bind(PyObject* self, PyObject* const* a, Py_ssize_t n) {")
+    out.append('  if (n != 2 || !PyUnicode_Check(a[0])) { PyErr_SetString(PyExc_TypeError, "bind(name, address)"); return NULL; }')
+    out.append("  const char* s = PyUnicode_AsUTF8(a[0]); void* p; if (s == NULL || to_ptr(a[1], &p)) return NULL;")
+    for name in signatures:
+        out.append(f'  if (!strcmp(s, "{name}")) {{ *(void**)&p_{name} = p; Py_RETURN_NONE; }}')
+    out.append('  PyErr_Format(PyExc_KeyError, "%s", s); return NULL;\n}')
+    out.append("static PyMethodDef methods[] = {")
+    for name in signatures:
+        out.append(f'  {{"{name}", (PyCFunction)(void (*)(void))w_{name}, METH_FASTCALL, NULL}},')
+    out.append('  {"bind", (PyCFunction)(void (*)(void))bind, METH_FASTCALL, NULL}, {NULL, NULL, 0, NULL}};')
+    out.append('static struct PyModuleDef mod = {PyModuleDef_HEAD_INIT, "_launch", NULL, -1, methods};')
+    out.append("PyMODINIT_FUNC PyInit__launch(void) { return PyModule_Create(&mod); }")
+    return "\n".join(out) + "\n"
+
+
+def build_launcher(signatures: dict[str, str], force: bool = False) -> Path:
+    """Compile :func:`launcher_source` in-tree; rebuilt when the signatures change."""
+    target = launcher_ext_path()
+    source = launcher_source(signatures)
+    src_path = OBJ_DIR / "_launch.c"
+
+    def fresh() -> bool:
+        return target.exists() and src_path.exists() and src_path.read_text() == source
+    if not force and fresh():
+        return target
+    gcc = _find("gcc", ["/usr/bin/gcc"])
+    if gcc is None:
+        raise RuntimeError("gcc not found: cannot build the kernel launcher")
+    with _build_lock(target):
+        if not force and fresh():
+            return target
+        OBJ_DIR.mkdir(exist_ok=True)
+        tmp, tmp_src = target.with_suffix(f".tmp{os.getpid()}"), OBJ_DIR / f"_launch{os.getpid()}.c"
+        tmp_src.write_text(source)
+        res = subprocess.run([gcc, "-O2", "-shared", "-fPIC", "-fvisibility=hidden", f"-I{sysconfig.get_paths()['include']}", str(tmp_src),
+                              "-o", str(tmp)], capture_output=True, text=True)
+        if res.returncode != 0:
+            tmp.unlink(missing_ok=True)
+            tmp_src.unlink(missing_ok=True)
+            raise RuntimeError("gcc failed:\n" + res.stdout + res.stderr)
+        os.replace(tmp, target)
+        os.replace(tmp_src, src_path)
+    return target
+
+
 def accounting_ext_path() -> Path:
     suffix = sysconfig.get_config_var("EXT_SUFFIX") or ".so"
     return PKG / "accounting" / ("_native" + suffix)
@@ -146,6 +237,8 @@ def build_accounting(force: bool = False) -> Path:
 
 def build_all(force: bool = False) -> None:
     build_kernels(force)
+    from ..ops import lib
+    build_launcher(lib.launch_signatures(), force)
     build_accounting(force)
 
 
