@@ -238,7 +238,8 @@ def _tree_kernel_ok(leaves: Sequence[Any], dtype: torch.dtype | None, compute_dt
     from ..device import fused_kernels_available
     from torch.utils._python_dispatch import _get_current_dispatch_mode
     return (0 < x0.shape[0] <= 65535 and x0.device.index == torch.cuda.current_device() and _get_current_dispatch_mode() is None
-            and torch.autograd.forward_ad._current_level < 0 and ops.functional.kernels_enabled() and fused_kernels_available())
+            and torch.autograd.forward_ad._current_level < 0 and not torch.jit.is_tracing() and not torch.compiler.is_compiling()
+            and ops.functional.kernels_enabled() and fused_kernels_available())
 
 
 def _clip_tree(leaves: Sequence[torch.Tensor], bound: float, mode: str, gamma: float, factor: float):

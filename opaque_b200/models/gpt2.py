@@ -105,11 +105,20 @@ class GPT2LMHeadModel(nn.Module):
         self.ln_f = LayerNorm(cfg.n_embd, cfg.layer_norm_epsilon, dtype=dtype, device=device)
         self.activation_checkpointing = False      # set by the trainer's gradient_checkpointing
 
+    def _carries(self) -> bool:
+        """Whether the blocks may run on the split stream: blocks and norms of these very classes, with no hooks that expect to be
+        called with the unsplit tensors."""
+        norms = [n for blk in self.h if type(blk) is GPT2Block for n in (blk.ln_1, blk.ln_2)] + [self.ln_f]
+        return (all(type(blk) is GPT2Block for blk in self.h) and all(type(n) is LayerNorm for n in norms)
+                and not any(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks
+                            for m in (*self.h, *norms)))
+
     def hidden_states(self, input_ids):
         B, T = input_ids.shape
         pos = torch.arange(T, device=input_ids.device).expand(B, T)
         h = self.wte(input_ids) + self.wpe(pos)
-        if h.is_cuda and ops.functional.kernels_enabled() and not (getattr(self, "activation_checkpointing", False) and torch.is_grad_enabled()):
+        if h.is_cuda and ops.functional.kernels_enabled() and not (getattr(self, "activation_checkpointing", False) and torch.is_grad_enabled()) \
+                and self._carries():
             x, residual = h, None
             for blk in self.h:
                 x, residual = blk.forward_carried(x, residual)

@@ -53,3 +53,20 @@ def test_bias_sums_batched(count, B, T):
         assert float((buf[:, :-3].double() - ref).abs().max()) < 1e-5 * max(T, 8) and bool((buf[:, -3:] == 2.0).all())
     with pytest.raises(ValueError):
         F.rows_sum_batch_([(jobs[0][0][:, :4], jobs[0][1])], B)
+
+
+def test_gpt2_blocks_with_hooks_see_the_unsplit_stream():
+    from opaque_b200.models import GPT2Config, GPT2LMHeadModel
+    torch.manual_seed(0)
+    m = GPT2LMHeadModel(GPT2Config.tiny(), device="cuda")
+    ids = torch.randint(0, 500, (2, 33), device="cuda")
+    assert m._carries()
+    with torch.no_grad():
+        plain = m.hidden_states(ids)
+        seen = []
+        handle = m.h[1].register_forward_hook(lambda mod, args, out: seen.append((args[0].shape, out.shape)))
+        hooked = m.hidden_states(ids)
+        handle.remove()
+    assert not m.h[1]._forward_hooks and seen == [((2, 33, 128), (2, 33, 128))]
+    # the split stream adds in the norm's kernel what the plain one adds before it: the same bf16 sums
+    assert _rel(plain, hooked) < 1e-2
