@@ -190,10 +190,20 @@ def direct_norm2(a: torch.Tensor, g: torch.Tensor, norm2: torch.Tensor, rows_per
     return norm2
 
 
-def pick_norm_path(rows_per_example: int, d_in: int, d_out: int) -> str:
+def pick_norm_path(rows_per_example: int, d_in: int, d_out: int, examples: int | None = None, sms: int = 148) -> str:
     """``"ghost"`` (Gram matrices, ``R²·(d_in + d_out)`` FLOPs on the upper triangle) or ``"direct"`` (the per-example
     product itself, ``2·R·d_in·d_out``) for one layer.  The Gram kernel runs at about 0.7 of the product kernel's rate, so
-    the direct form wins once ``R > 1.4·d_in·d_out / (d_in + d_out)``; it needs ``R % 64 == 0``."""
+    the direct form wins once ``R > 1.4·d_in·d_out / (d_in + d_out)``; it needs ``R % 64 == 0``.
+
+    With few ``examples`` an output head is the exception, at any length: a Gram item runs all ``(d_in + d_out) / 64`` k-blocks
+    (about 280 clocks each, 530 off the diagonal) on one SM, and with fewer items than SMs the launch waits for it: with 3 x 199
+    rows and 2048 + 151936 columns 670 of the 735 us that the norms of a whole model took.  The direct form spreads over the
+    output tiles."""
+    if examples is not None and d_in + d_out > 16384:
+        blocks = -(-rows_per_example // 128)
+        tiles = -(-examples * -(-d_in // 128) * -(-d_out // 256) // sms) * (-(-rows_per_example // 64) * 512 + 1500)
+        if examples * blocks * (blocks + 1) <= sms and 1.5 * tiles < (d_in + d_out) / 64 * (280 if blocks == 1 else 530):
+            return "direct"
     if rows_per_example % 64:
         return "ghost"
     return "direct" if rows_per_example * (d_in + d_out) > 1.4 * d_in * d_out else "ghost"
@@ -247,15 +257,16 @@ def _check_pe(a, b, rows_per_example) -> tuple[int, int, int, int]:
     T, M = a.shape
     if b.shape[0] != T or a.stride(1) != 1 or b.stride(1) != 1:
         raise ValueError("a [T, M] and b [T, N] must be row-major with the same number of rows")
-    if rows_per_example <= 0 or rows_per_example % 64 or T % rows_per_example:
-        raise ValueError("rows_per_example must be a multiple of 64 that divides the number of rows")
+    if rows_per_example <= 0 or T % rows_per_example:
+        raise ValueError("rows_per_example must divide the number of rows")
     return T, M, b.shape[1], T // rows_per_example
 
 
 def wgrad_clip_per_example_batch(problems: Sequence[tuple], out: torch.Tensor | None, rows_per_example: int, *,
                                  peer_table: torch.Tensor | None = None, shard_elems: int = 0, status: StatusWord | None = None,
                                  wait_budget_s: float = DEFAULT_WAIT_BUDGET_S) -> None:
-    """Several accumulating :func:`wgrad_clip_per_example` problems ``(a, b, ex_scale, out_offset, ldm)`` in one launch (per 56)."""
+    """Several accumulating :func:`wgrad_clip_per_example` problems ``(a, b, ex_scale, out_offset, ldm)`` in one launch (per 56).
+    ``rows_per_example`` may have any length here: an example's last 64-row block is filled up with zeros."""
     tiles = sum(math.ceil(pr[0].shape[1] / 128) * math.ceil(pr[1].shape[1] / 256) for pr in problems)
     descs = []
     for a, b, ex_scale, off, ldm in problems:
@@ -281,7 +292,7 @@ def wgrad_clip_per_example_batch(problems: Sequence[tuple], out: torch.Tensor | 
 
 def direct_norm2_batch(problems: Sequence[tuple], rows_per_example: int, *, status: StatusWord | None = None,
                        wait_budget_s: float = DEFAULT_WAIT_BUDGET_S) -> None:
-    """Several :func:`direct_norm2` problems ``(a, g, norm2)`` in one launch (per 56)."""
+    """Several :func:`direct_norm2` problems ``(a, g, norm2)`` in one launch (per 56), for any ``rows_per_example``."""
     tiles = sum(math.ceil(pr[0].shape[1] / 128) * math.ceil(pr[1].shape[1] / 256) for pr in problems)
     descs = []
     for a, g, norm2 in problems:

@@ -54,6 +54,7 @@ typedef struct {
 int ob_ghost_norm_batch(const ob_ghost_desc* descs, int count, int* status, double wait_budget_s, int num_sms, void* stream);
 int ob_wgrad_clip_batch(const ob_wgrad_desc* descs, int count, float* out, float* const* peer_out, long long shard_elems,
                         int block_n, int* status, double wait_budget_s, int num_sms, void* stream);
+// (ex_rows of any length here)
 int ob_wgrad_clip_pe_batch(const ob_wgrad_pe_desc* descs, int count, float* out, float* const* peer_out,
                            long long shard_elems, int* status, double wait_budget_s, int num_sms, void* stream);
 

@@ -428,7 +428,8 @@ wgrad_clip_kernel(const __grid_constant__ TmaBatch<WgradParams, CAP> b) {
 
 // ---------------------------------------------------------------------------------------------
 // Per-example variant: every example owns a whole number of 64-row k-blocks (uniform rows_per_example), so the clip
-// factor is constant over an accumulation run.  The MMA warp accumulates ONE example's A_e^T G_e per TMEM buffer and
+// factor is constant over an accumulation run.  The operand maps are [example][row][column], so the last k-block of an
+// example whose length is no multiple of 64 is filled up with zeros, not with the next example's rows.  The MMA warp accumulates ONE example's A_e^T G_e per TMEM buffer and
 // the epilogue warps fold it into fp32 register accumulators as  acc += c_e * P_e  while the tensor core already
 // works on the next example in the other buffer.  Operands are never touched in shared memory (no scaling pass, no
 // extra barrier in the TMA -> MMA chain) and c_e is applied in full fp32 precision.
@@ -442,7 +443,7 @@ constexpr int WP_SMEM = WP_STAGES * WP_STAGE_BYTES + 8 * 4096 + 256 + 1024;    /
 
 struct WgradPeParams {
   int M, N;
-  int num_examples, ex_rows;         // ex_rows is a multiple of WG_BLOCK_K
+  int num_examples, ex_rows;
   int splits;                        // each split owns a contiguous range of examples
   const float* ex_scale;             // [num_examples] or nullptr (all ones)
   float* out;
@@ -520,11 +521,11 @@ wgrad_clip_pe_kernel(const __grid_constant__ TmaBatch<WgradPeParams, CAP> b) {
       for (int w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
         cur = b.seek(w, cur);
         const WgradPeParams& p = b.p[cur];
-        const int kpe = p.ex_rows / WG_BLOCK_K;
+        const int kpe = (p.ex_rows + WG_BLOCK_K - 1) / WG_BLOCK_K;
         int m0, n0, e0, e1;
         decode(p, w - b.start[cur], m0, n0, e0, e1);
         const int nkb = (e1 - e0) * kpe;
-        const int row_begin = e0 * p.ex_rows;
+        int ex = e0, row = 0;
         for (int kb = 0; kb < nkb; ++kb) {
           if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, b.status, OB_ERR_WAIT_EMPTY, budget)) {
             ok = false;
@@ -533,13 +534,17 @@ wgrad_clip_pe_kernel(const __grid_constant__ TmaBatch<WgradPeParams, CAP> b) {
           mbar_expect_tx(&full[stage], WP_STAGE_BYTES);
           uint8_t* a_dst = smem + stage * WP_STAGE_BYTES;
           uint8_t* b_dst = a_dst + WP_A_BYTES;
-          const int row = row_begin + kb * WG_BLOCK_K;
 #pragma unroll
           for (int j = 0; j < WG_BLOCK_M / 64; ++j)
-            tma_load_2d(a_dst + j * (WG_BLOCK_K * 128), &b.map_a[cur], &full[stage], m0 + 64 * j, row);
+            tma_load_3d(a_dst + j * (WG_BLOCK_K * 128), &b.map_a[cur], &full[stage], m0 + 64 * j, row, ex);
 #pragma unroll
           for (int j = 0; j < WP_BLOCK_N / 64; ++j)
-            tma_load_2d(b_dst + j * (WG_BLOCK_K * 128), &b.map_b[cur], &full[stage], n0 + 64 * j, row);
+            tma_load_3d(b_dst + j * (WG_BLOCK_K * 128), &b.map_b[cur], &full[stage], n0 + 64 * j, row, ex);
+          row += WG_BLOCK_K;
+          if (row >= kpe * WG_BLOCK_K) {
+            row = 0;
+            ++ex;
+          }
           issued_mask |= 1u << stage;
           issued_phase = (issued_phase & ~(1u << stage)) | (phase << stage);
           if (++stage == WP_STAGES) { stage = 0; phase ^= 1; }
@@ -563,7 +568,7 @@ wgrad_clip_pe_kernel(const __grid_constant__ TmaBatch<WgradPeParams, CAP> b) {
       for (int w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
         cur = b.seek(w, cur);
         const WgradPeParams& p = b.p[cur];
-        const int kpe = p.ex_rows / WG_BLOCK_K;
+        const int kpe = (p.ex_rows + WG_BLOCK_K - 1) / WG_BLOCK_K;
         int m0, n0, e0, e1;
         decode(p, w - b.start[cur], m0, n0, e0, e1);
         for (int e = e0; ok && e < e1; ++e) {
@@ -738,6 +743,9 @@ static EncodeTiledFn get_encode_fn() {
 static thread_local char g_map_detail[192] = {0};
 
 // 2-D bf16 tensor map over a row-major [rows, cols] matrix with row pitch `ld` elements.
+// bf16 [examples][rows][cols] with row pitch ld, 64 x 64 boxes (a box never crosses into the next example)
+static int make_bf16_map_3d(CUtensorMap* map, const void* base, long long examples, long long rows, long long cols, long long ld);
+
 static int make_map_2d(CUtensorMap* map, CUtensorMapDataType type, int elem, const void* base, long long rows, long long cols,
                        long long ld, int box_cols, int box_rows) {
   EncodeTiledFn enc = get_encode_fn();
@@ -768,6 +776,22 @@ static int make_map_2d(CUtensorMap* map, CUtensorMapDataType type, int elem, con
 int make_bf16_map_2d(CUtensorMap* map, const void* base, long long rows, long long cols, long long ld,
                      int box_cols, int box_rows) {
   return make_map_2d(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, rows, cols, ld, box_cols, box_rows);
+}
+static int make_bf16_map_3d(CUtensorMap* map, const void* base, long long examples, long long rows, long long cols, long long ld) {
+  CUtensorMap whole;                     // the checks (alignment, pitch) and the thread's context of the 2-D form
+  const int rc = make_bf16_map_2d(&whole, base, examples * rows, cols, ld, 64, WG_BLOCK_K);
+  if (rc) return rc;
+  cuuint64_t dims[3] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(examples)};
+  cuuint64_t strides[2] = {static_cast<cuuint64_t>(ld) * 2, static_cast<cuuint64_t>(ld) * 2 * rows};
+  cuuint32_t box[3] = {64, WG_BLOCK_K, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  const CUresult r = get_encode_fn()(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+                                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS)
+    snprintf(g_map_detail, sizeof(g_map_detail), "tensor map rejected (CUresult %d): base=%p examples=%lld rows=%lld cols=%lld ld=%lld",
+             static_cast<int>(r), base, examples, rows, cols, ld);
+  return r == CUDA_SUCCESS ? 0 : -12;
 }
 int make_f32_map_2d(CUtensorMap* map, const void* base, long long rows, long long cols, long long ld,
                     int box_cols, int box_rows) {
@@ -889,16 +913,15 @@ template <int CAP>
 static int wgrad_pe_append(TmaBatch<WgradPeParams, CAP>& b, const ob_wgrad_pe_desc& d, float* out, float* const* peer_out,
                            long long shard_elems) {
   if (d.num_examples <= 0 || d.ex_rows <= 0 || d.M <= 0 || d.N <= 0) return 0;
-  if (d.ex_rows % WG_BLOCK_K) return -3;
   int splits = d.splits < 1 ? 1 : d.splits;
   if (splits > d.num_examples) splits = d.num_examples;
   if (splits > 1 && !d.accumulate && d.norm2 == nullptr) return -4;   // split partial sums must be reduced into the destination
   const long long T = static_cast<long long>(d.num_examples) * d.ex_rows;
   if (T > 0x7fffffffLL) return -5;
   const int i = b.count;
-  int rc = make_bf16_map_2d(&b.map_a[i], d.a, T, d.M, d.lda, 64, WG_BLOCK_K);
+  int rc = make_bf16_map_3d(&b.map_a[i], d.a, d.num_examples, d.ex_rows, d.M, d.lda);
   if (rc) return rc;
-  rc = make_bf16_map_2d(&b.map_b[i], d.b, T, d.N, d.ldb, 64, WG_BLOCK_K);
+  rc = make_bf16_map_3d(&b.map_b[i], d.b, d.num_examples, d.ex_rows, d.N, d.ldb);
   if (rc) return rc;
   WgradPeParams& p = b.p[i];
   p.M = d.M; p.N = d.N;
@@ -989,6 +1012,7 @@ extern "C" int ob_wgrad_clip_pe_batch(const ob_wgrad_pe_desc* descs, int count, 
 static int wgrad_pe_one(const ob_wgrad_pe_desc& d, float* out, float* const* peer_out, long long shard_elems, int* status,
                         double wait_budget_s, int num_sms, void* stream) {
   using namespace ob;
+  if (d.ex_rows > 0 && d.ex_rows % WG_BLOCK_K) return -3;
   TmaBatch<WgradPeParams, 1> w;
   batch_begin(w, status, wait_budget_s);
   const int rc = wgrad_pe_append(w, d, out, peer_out, shard_elems);

@@ -127,3 +127,28 @@ def test_accumulating_destinations(offset, M, N, ldm):
         w2 = torch.full_like(out2, 3.0)
         w2[:M * ldm].view(M, ldm)[:, :N] += ops.wgrad_clip_ref(a[:128], b[:128], row_scale=c.repeat_interleave(64))[0]
         assert st.read() == 0 and _rel(out2, w2) < 1e-5 and bool((out2[:M * ldm].view(M, ldm)[:, N:] == 3.0).all()) and bool((out2[M * ldm:] == 3.0).all())
+
+
+@pytest.mark.parametrize("R", [1, 40, 63, 65, 129, 333])
+def test_per_example_kernels_take_any_length(R):
+    """An example's last 64-row block must not see the next example's rows."""
+    from opaque_b200 import ops
+    B, M, N = 3, 136, 264
+    a, b = _r(B * R, M), _r(B * R, N)
+    c = torch.tensor([0.5, 0.0, 1.5], device="cuda")
+    out, st = torch.zeros(M * N, device="cuda"), ops.StatusWord()
+    ops.wgrad_clip_per_example_batch([(a, b, c, 0, N)], out, R, status=st)
+    assert st.read() == 0 and _rel(out.view(M, N), ops.wgrad_clip_ref(a, b, row_scale=c.repeat_interleave(R))[0]) < 2e-5
+    n2 = torch.zeros(B, device="cuda")
+    ops.direct_norm2_batch([(a, b, n2)], R, status=st)
+    assert st.read() == 0 and _rel(n2, ops.ghost_norm_ref(a, b, R)) < 5e-5
+    if R % 64:
+        with pytest.raises(ValueError):                   # the single call still wants whole blocks
+            ops.wgrad_clip_per_example(a, b, out, ex_scale=c, rows_per_example=R)
+
+
+def test_few_records_on_a_wide_head_take_the_direct_norm():
+    from opaque_b200 import ops
+    assert ops.pick_norm_path(64, 768, 50304, 2) == "direct" and ops.pick_norm_path(199, 2048, 151936, 3) == "direct"
+    assert ops.pick_norm_path(64, 768, 50304) == "ghost" and ops.pick_norm_path(512, 768, 50304, 32) == "ghost"
+    assert ops.pick_norm_path(64, 768, 3072, 2) == "ghost"
