@@ -104,7 +104,7 @@ class Capture:
         # stay alive for the weight gradients anyway
         self.ghost_jobs: list[tuple] = []
         self.direct_jobs: list[tuple] = []
-        self.bias_jobs: list[tuple] = []
+        self.sum_jobs: list[tuple] = []
         self.status = engine.status
         self.direct_elems = sp.direct_elems
 
@@ -198,6 +198,16 @@ class Capture:
             jobs.append(dict(a=g_parts[j], b=xa[:, j * r:(j + 1) * r], out_offset=sb.offset, ldm=r, ldn=1, n_valid=r, **common))
         ops.wgrad_clip_batch(jobs, self.pe, accumulate=False, block_n=64, status=self.status)
 
+    def add_row_sums(self, out: torch.Tensor, g2d: torch.Tensor, x2d: torch.Tensor, mean: torch.Tensor | None, rstd: torch.Tensor,
+                     out_plain: torch.Tensor | None) -> None:
+        """Per-example weight (and bias) gradient of a norm layer.  Short matrices wait for the other layers' and share a launch;
+        long ones run at once: they fill the chip alone, and waiting would keep two activations per layer alive (16 MB a layer
+        at 4096 rows of 1024)."""
+        if g2d.shape[0] <= 4096 and g2d.shape[1] <= 8192 and x2d.stride(0) == g2d.stride(0) and (g2d.data_ptr() | x2d.data_ptr()) & 15 == 0:
+            self.sum_jobs.append((out, g2d, x2d, mean, rstd, out_plain))
+        else:
+            ops.functional.rows_group_sum_(out, g2d, self.batch_size, x2d=x2d, mean=mean, rstd=rstd, out_plain=out_plain)
+
     def _tied_cross_term(self, slot_name: str) -> torch.Tensor | None:
         """``<g_embedding, g_head>`` per example for a weight used as input embedding AND output head.
 
@@ -253,9 +263,9 @@ class Capture:
             ops.ghost_norm_batch(self.ghost_jobs, status=self.status)
         if self.direct_jobs:
             ops.direct_norm2_batch(self.direct_jobs, self.tokens, status=self.status)
-        for rows in {g.shape[0] for _, g in self.bias_jobs}:
-            ops.functional.rows_sum_batch_([j for j in self.bias_jobs if j[1].shape[0] == rows], self.batch_size)
-        self.ghost_jobs, self.direct_jobs, self.bias_jobs = [], [], []
+        for rows in {j[1].shape[0] for j in self.sum_jobs}:
+            ops.functional.rows_sum_batch_([j for j in self.sum_jobs if j[1].shape[0] == rows], self.batch_size)
+        self.ghost_jobs, self.direct_jobs, self.sum_jobs = [], [], []
         by_slot: dict[str, list[int]] = {}
         for i, name in enumerate(self.part_slots):
             by_slot.setdefault(name, []).append(i)
@@ -377,7 +387,7 @@ class _DPLinear(Function):
         cap.add_linear(weight, x2d, g2d)
         if ctx.bias is not None:
             if g2d.dtype == torch.bfloat16 and g2d.shape[1] % 8 == 0 and g2d.stride(0) % 8 == 0:
-                cap.bias_jobs.append((cap.pe_view(ctx.bias), g2d))
+                cap.sum_jobs.append((cap.pe_view(ctx.bias), g2d))        # g2d is kept for the weight gradient anyway
             else:
                 cap.pe_view(ctx.bias).add_(g2d.view(cap.batch_size, cap.tokens, -1).sum(1, dtype=torch.float32))
         return dx, None, None

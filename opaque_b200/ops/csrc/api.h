@@ -111,10 +111,16 @@ int ob_moe_combine(const void* y, const void* w, const long long* pos, void* out
 int ob_moe_row_grad(const void* dout, const void* y, const void* w, const long long* token, const long long* slot, void* dy,
                     float* dw, long long rows, int H, int sms, void* stream);
 
-// Plain row sums per example of several bf16 matrices g[i] [num_examples * rows_per_example, N[i]] (pitch ldg[i]) in one launch
-// per 128: out[i][e * ld_out[i] + n] += sum.
-int ob_rows_sum_batch(const void* const* g, const long long* ldg, const int* N, float* const* out, const long long* ld_out,
-                      int count, int num_examples, int rows_per_example, void* stream);
+// ob_rows_group_sum for several matrices with the same rows in one launch per 128 (host array of descriptions): g and x
+// [num_examples * rows_per_example, N] with pitch ldg, out / out2 rows with pitch ld_out / ld_out2, modes as there.
+typedef struct {
+  const void *g, *x;
+  const float *mean, *rstd;
+  float *out, *out2;
+  long long ldg, ld_out, ld_out2;
+  int N, mode;
+} ob_rowsum_desc;
+int ob_rows_sum_batch(const ob_rowsum_desc* descs, int count, int num_examples, int rows_per_example, void* stream);
 // a_cat [3r, in] = (aq; ak; av), b_block [oq + ok + ov, 3r] = blockdiag(bq, bk, bv); contiguous bf16, r % 8 == 0.
 int ob_lora_pack(const void* aq, const void* ak, const void* av, const void* bq, const void* bk, const void* bv, void* a_cat,
                  void* b_block, int r, int in, int oq, int ok, int ov, int sms, void* stream);

@@ -429,36 +429,36 @@ rows_group_sum_kernel(const __nv_bfloat16* __restrict__ g, const __nv_bfloat16* 
   }
 }
 
-// Plain sums (mode 0) of several matrices with the same rows in ONE launch: the bias gradients of a backward pass.  A block
-// finds its (matrix, 256-column block) in the table; otherwise as above.  One launch per layer left most of the chip idle
-// (a 768-column matrix has 3 column blocks) and cost a launch each.  Measured for the 48 biases of GPT-2 small: 0.71 -> 0.58 ms
-// with 32 x 512 tokens, 0.21 -> 0.01 with 2 x 64.
+// The same sums for several matrices with the same rows in ONE launch: the bias and norm-weight gradients of a backward pass.  A
+// block finds its (matrix, 256-column block) in the table; otherwise as above.  One launch per layer left most of the chip
+// idle (a 768-column matrix has 3 column blocks) and cost a launch each.  Measured for the 48 biases of GPT-2 small: 0.71 -> 0.58
+// ms with 32 x 512 tokens, 0.21 -> 0.01 with 2 x 64.
+// Measured, all norm and bias sums of GPT-2 small: 26 launches and 152 us -> one of 11.5 us with 2 x 64 tokens, 345 -> 197 us
+// with 11 x 333.  At 16,384 rows a launch per layer takes the operands while L2 still holds them (16.6 us each, 28 by HBM), so
+// longer sums are not deferred.
 constexpr int RS_CAP = 128;
 struct RowSumBatch {
-  const __nv_bfloat16* g[RS_CAP];
-  float* out[RS_CAP];
-  long long ld_out[RS_CAP];
-  int ldg[RS_CAP];
-  int N[RS_CAP];
+  ob_rowsum_desc d[RS_CAP];
   int start[RS_CAP + 1];     // first column block
 };
 
 __global__ void __launch_bounds__(256)
 rows_sum_batch_kernel(const __grid_constant__ RowSumBatch t, int rows_per_example) {
   __shared__ float red[8][256 + 8];
+  __shared__ float red2[8][256 + 8];
   int i = 0;
   while (static_cast<int>(blockIdx.y) >= t.start[i + 1]) ++i;
   const int e = blockIdx.x;
   const int cg = threadIdx.x & 31, rl = threadIdx.x >> 5;
   const int col0 = (blockIdx.y - t.start[i]) * 256, col = col0 + cg * 8;
-  const int N = t.N[i];
-  const long long ldg = t.ldg[i];
+  const int N = t.d[i].N, mode = t.d[i].mode;
+  const long long ldg = t.d[i].ldg;
   const int chunk = (rows_per_example + gridDim.z - 1) / gridDim.z;
   const int r0 = e * rows_per_example + blockIdx.z * chunk;
   const int r1 = min(r0 + chunk, (e + 1) * rows_per_example);
-  const __nv_bfloat16* g = t.g[i] + col;
-  float acc[8] = {};
-  if (col < N) {
+  const __nv_bfloat16* g = static_cast<const __nv_bfloat16*>(t.d[i].g) + col;
+  float acc[8] = {}, acc2[8] = {};
+  if (col < N && mode == 0) {
 #pragma unroll 4
     for (int r = r0 + rl; r < r1; r += 8) {
       float gv[8];
@@ -466,16 +466,40 @@ rows_sum_batch_kernel(const __grid_constant__ RowSumBatch t, int rows_per_exampl
 #pragma unroll
       for (int j = 0; j < 8; ++j) acc[j] += gv[j];
     }
-  }
+  } else if (col < N) {
+    const __nv_bfloat16* x = static_cast<const __nv_bfloat16*>(t.d[i].x) + col;
+    const float *mean = t.d[i].mean, *rstd = t.d[i].rstd;
+#pragma unroll 2
+    for (int r = r0 + rl; r < r1; r += 8) {
+      float gv[8], xv[8];
+      ln_unpack8(*reinterpret_cast<const ln_bf16x8*>(g + static_cast<long long>(r) * ldg), gv);
+      ln_unpack8(*reinterpret_cast<const ln_bf16x8*>(x + static_cast<long long>(r) * ldg), xv);
+      const float mu = mode == 1 ? __ldg(mean + r) : 0.f, rs = __ldg(rstd + r);
 #pragma unroll
-  for (int j = 0; j < 8; ++j) red[rl][cg * 8 + j] = acc[j];
+      for (int j = 0; j < 8; ++j) {
+        acc[j] += gv[j] * (xv[j] - mu) * rs;
+        acc2[j] += gv[j];
+      }
+    }
+  }
+  float* const out2 = t.d[i].out2;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    red[rl][cg * 8 + j] = acc[j];
+    if (out2 != nullptr) red2[rl][cg * 8 + j] = acc2[j];
+  }
   __syncthreads();
   const int c = threadIdx.x;
   if (col0 + c < N) {
-    float s = 0.f;
+    float s = 0.f, s2 = 0.f;
 #pragma unroll
     for (int k = 0; k < 8; ++k) s += red[k][c];
-    atomicAdd(t.out[i] + static_cast<long long>(e) * t.ld_out[i] + col0 + c, s);
+    atomicAdd(t.d[i].out + static_cast<long long>(e) * t.d[i].ld_out + col0 + c, s);
+    if (out2 != nullptr) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) s2 += red2[k][c];
+      atomicAdd(out2 + static_cast<long long>(e) * t.d[i].ld_out2 + col0 + c, s2);
+    }
   }
 }
 
@@ -651,8 +675,7 @@ extern "C" int ob_rows_group_sum(const void* g, const void* x, const float* mean
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }
 
-extern "C" int ob_rows_sum_batch(const void* const* g, const long long* ldg, const int* N, float* const* out,
-                                 const long long* ld_out, int count, int num_examples, int rows_per_example, void* stream) {
+extern "C" int ob_rows_sum_batch(const ob_rowsum_desc* descs, int count, int num_examples, int rows_per_example, void* stream) {
   if (num_examples <= 0 || rows_per_example <= 0) return 0;
   int splits = rows_per_example / 64;
   splits = splits < 1 ? 1 : (splits > 16 ? 16 : splits);
@@ -661,14 +684,13 @@ extern "C" int ob_rows_sum_batch(const void* const* g, const long long* ldg, con
     const int n = count - first < RS_CAP ? count - first : RS_CAP;
     t.start[0] = 0;
     for (int i = 0; i < n; ++i) {
-      const int k = first + i;
-      if (N[k] <= 0 || (N[k] & 7) || (ldg[k] & 7) || ldg[k] > 0x7fffffffLL || (reinterpret_cast<uintptr_t>(g[k]) & 15)) return -2;
-      t.g[i] = static_cast<const __nv_bfloat16*>(g[k]);
-      t.out[i] = out[k];
-      t.ldg[i] = static_cast<int>(ldg[k]);
-      t.ld_out[i] = ld_out[k];
-      t.N[i] = N[k];
-      t.start[i + 1] = t.start[i] + (N[k] + 255) / 256;
+      const ob_rowsum_desc& d = descs[first + i];
+      if (d.N <= 0 || (d.N & 7) || (d.ldg & 7) || (reinterpret_cast<uintptr_t>(d.g) & 15) || (reinterpret_cast<uintptr_t>(d.x) & 15)) return -2;
+      if (d.mode < 0 || d.mode > 2 || (d.mode > 0 && (d.x == nullptr || d.rstd == nullptr)) || (d.mode == 1 && d.mean == nullptr) ||
+          (d.mode == 0 && d.out2 != nullptr))
+        return -3;
+      t.d[i] = d;
+      t.start[i + 1] = t.start[i] + (d.N + 255) / 256;
     }
     if (t.start[n] > 65535) return -4;
     rows_sum_batch_kernel<<<dim3(num_examples, t.start[n], splits), 256, 0, static_cast<cudaStream_t>(stream)>>>(t, rows_per_example);

@@ -11,8 +11,9 @@ cross_entropy.py:585-681.
 from __future__ import annotations
 
 import contextlib
-import math
 import ctypes
+import math
+import struct
 
 import torch
 from torch.autograd import Function
@@ -119,7 +120,7 @@ class _RMSNorm(Function):
                                        rows, H, offset, lib.stream())
         lib.check(rc, "rmsnorm_bwd")
         if direct_pe:                # 16-byte-vector row sums straight into the capture's per-example buffer
-            rows_group_sum_(cap.pe_view(layer.weight), dy2, cap.batch_size, x2d=xs, rstd=rstd)
+            cap.add_row_sums(cap.pe_view(layer.weight), dy2, xs, None, rstd, None)
         elif cap is not None:
             cap.add_per_example_grad(layer, "weight", dw_pe)
         elif dw_pe is not None:
@@ -165,21 +166,29 @@ def rows_group_sum_(out: torch.Tensor, g2d: torch.Tensor, num_examples: int, *, 
     lib.check(rc, "rows_group_sum")
 
 
+_ROWSUM_DESC = struct.Struct("6Q3q2i")
+
+
 def rows_sum_batch_(jobs, num_examples: int) -> None:
-    """``out[e] += Σ_{rows of example e} g`` for every ``(out, g2d)`` of ``jobs`` (the plain form of :func:`rows_group_sum_`; all
-    ``g2d`` with the same number of rows) in one launch per 128."""
+    """:func:`rows_group_sum_` for several matrices with the same number of rows in one launch (per 128): ``jobs`` are
+    ``(out, g2d)`` (plain sums) or ``(out, g2d, x2d, mean | None, rstd, out_plain | None)``."""
     rows = jobs[0][1].shape[0]
     if rows % num_examples:
         raise ValueError("rows_sum_batch_: rows must be a multiple of examples")
-    n = len(jobs)
-    g, o, ldg, ldo, cols = (ctypes.c_void_p * n)(), (ctypes.c_void_p * n)(), (ctypes.c_longlong * n)(), (ctypes.c_longlong * n)(), (ctypes.c_int * n)()
-    for i, (out, g2d) in enumerate(jobs):
-        if out.dtype != torch.float32 or out.shape != (num_examples, g2d.shape[1]) or out.stride(1) != 1:
-            raise ValueError("rows_sum_batch_: out must be fp32 [examples, N]")
-        if g2d.dtype != torch.bfloat16 or g2d.shape[0] != rows or g2d.stride(1) != 1:
-            raise ValueError("rows_sum_batch_: g must be bf16 matrices with the same number of rows")
-        g[i], o[i], ldg[i], ldo[i], cols[i] = g2d.data_ptr(), out.data_ptr(), g2d.stride(0), out.stride(0), g2d.shape[1]
-    rc = lib.load().ob_rows_sum_batch(g, ldg, cols, o, ldo, n, num_examples, rows // num_examples, lib.stream())
+    descs = []
+    for out, g2d, *norm in jobs:
+        x2d, mean, rstd, plain = norm or (None, None, None, None)
+        N = g2d.shape[1]
+        for o in (out, plain):
+            if o is not None and (o.dtype != torch.float32 or o.shape != (num_examples, N) or o.stride(1) != 1):
+                raise ValueError("rows_sum_batch_: out must be fp32 [examples, N]")
+        for t in (g2d, x2d):
+            if t is not None and (t.dtype != torch.bfloat16 or t.shape != (rows, N) or t.stride(1) != 1 or t.stride(0) != g2d.stride(0)):
+                raise ValueError("rows_sum_batch_: operands must be bf16 matrices with the same rows and pitch")
+        descs.append(_ROWSUM_DESC.pack(g2d.data_ptr(), lib.ptr(x2d) or 0, lib.ptr(mean) or 0, lib.ptr(rstd) or 0, out.data_ptr(),
+                                       lib.ptr(plain) or 0, g2d.stride(0), out.stride(0), 0 if plain is None else plain.stride(0), N,
+                                       0 if x2d is None else (1 if mean is not None else 2)))
+    rc = lib.load().ob_rows_sum_batch(b"".join(descs), len(descs), num_examples, rows // num_examples, lib.stream())
     lib.check(rc, "rows_sum_batch")
 
 
@@ -206,8 +215,7 @@ def _layer_norm_param_grads(dy2, x2, weight, stats, layer, has_bias):
     """Weight and bias gradients of a LayerNorm: per example into the active capture (returns ``(None, None)``), else summed."""
     cap = _param_grad_hook() if weight.requires_grad else None
     if cap is not None:                      # per-example gradients straight into the capture's buffer rows
-        rows_group_sum_(cap.pe_view(layer.weight), dy2, cap.batch_size, x2d=x2, mean=stats[0], rstd=stats[1],
-                        out_plain=cap.pe_view(layer.bias) if has_bias else None)
+        cap.add_row_sums(cap.pe_view(layer.weight), dy2, x2, stats[0], stats[1], cap.pe_view(layer.bias) if has_bias else None)
     elif weight.requires_grad:
         acc = torch.zeros(2, 1, dy2.shape[1], dtype=torch.float32, device=x2.device)
         rows_group_sum_(acc[0], dy2, 1, x2d=x2, mean=stats[0], rstd=stats[1], out_plain=acc[1])

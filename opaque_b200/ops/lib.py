@@ -43,7 +43,7 @@ _SIGNATURES = {
     "ob_rows_group_sum": [P, P, P, P, I, I, I, LL, P, LL, I, P, LL, P],
     "ob_add_layernorm_fwd": [P, P, P, P, P, P, P, P, LL, I, F, P],
     "ob_add_layernorm_bwd_dx": [P, P, P, P, P, P, P, LL, I, P],
-    "ob_rows_sum_batch": [P, P, P, P, P, I, I, I, P],
+    "ob_rows_sum_batch": [c_char_p, I, I, I, P],
     "ob_merge_heads3": [P, P, P, P, P, LL, I, I, I, I, P],
     "ob_activation": [P, P, P, LL, I, I, P],
     "ob_ghost_set_wide": [I],
@@ -72,7 +72,7 @@ _SIGNATURES = {
 
 
 # entry points called with host arrays or handles (and once-only queries) stay with ctypes
-_CTYPES_ONLY = {"ob_die_map", "ob_pair_init", "ob_pair_set_die_aware", "ob_ghost_set_wide", "ob_merge_heads3", "ob_rows_sum_batch",
+_CTYPES_ONLY = {"ob_die_map", "ob_pair_init", "ob_pair_set_die_aware", "ob_ghost_set_wide", "ob_merge_heads3",
                 "ob_clip_tree_chunks", "ob_clip_tree", "ob_shard_step", "ob_peer_barrier", "ob_ipc_alloc", "ob_ipc_free", "ob_ipc_get_handle",
                 "ob_ipc_open_handle", "ob_ipc_close_handle", "ob_last_cuda_error", "ob_last_detail"}
 _LETTER = {P: "P", c_char_p: "P", I: "I", LL: "L", F: "F", D: "D", U: "U", ULL: "Q"}

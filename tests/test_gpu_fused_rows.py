@@ -55,6 +55,25 @@ def test_bias_sums_batched(count, B, T):
         F.rows_sum_batch_([(jobs[0][0][:, :4], jobs[0][1])], B)
 
 
+@pytest.mark.parametrize("B,T", [(1, 1), (3, 70), (2, 513)])
+def test_norm_weight_sums_batched(B, T):
+    from opaque_b200.ops import functional as F
+    jobs, one = [], []
+    for i, N in enumerate((8, 264, 768, 1032, 16)):
+        g, x = (torch.randn(B * T, N, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+        mean, rstd = torch.randn(B * T, device="cuda"), torch.rand(B * T, device="cuda")
+        args = (x, mean if i % 2 == 0 else None, rstd)
+        a, b, pa, pb = (torch.ones(B, N, device="cuda") for _ in range(4))
+        plain = i % 3 != 1
+        jobs.append((a, g, *args, pa if plain else None))
+        F.rows_group_sum_(b, g, B, x2d=x, mean=args[1], rstd=rstd, out_plain=pb if plain else None)
+        one.append((a, b, pa, pb))
+    jobs.append((torch.zeros(B, 8, device="cuda"), torch.randn(B * T, 8, device="cuda", dtype=torch.bfloat16)))
+    F.rows_sum_batch_(jobs, B)
+    for a, b, pa, pb in one:                     # the same arithmetic; only the order of the atomics differs
+        assert torch.allclose(a, b, rtol=1e-5, atol=1e-4) and torch.allclose(pa, pb, rtol=1e-5, atol=1e-4)
+
+
 def test_gpt2_blocks_with_hooks_see_the_unsplit_stream():
     from opaque_b200.models import GPT2Config, GPT2LMHeadModel
     torch.manual_seed(0)
