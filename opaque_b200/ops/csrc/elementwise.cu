@@ -338,25 +338,36 @@ glu_fwd_kernel(const __nv_bfloat16* __restrict__ gate, const __nv_bfloat16* __re
   }
 }
 
+// ACT and FLAT (every matrix contiguous, so a vector's place needs no division by the row length) are template parameters: the
+// 64-bit division and the run-time choice of the activation per element took longer than the memory they wait for.
+// Measured, SwiGLU inside a training step: 16384 x 14336 465 -> 452 us (360 at the copy rate), 5439 x 8192 78.7 -> 75.2.
+template <int ACT, bool FLAT>
 __global__ void __launch_bounds__(256)
 glu_bwd_kernel(const __nv_bfloat16* __restrict__ dh, const __nv_bfloat16* __restrict__ gate,
                const __nv_bfloat16* __restrict__ up, __nv_bfloat16* __restrict__ dgate,
-               __nv_bfloat16* __restrict__ dup, long long rows, int I, long long ld_in, long long ld_out, int act) {
+               __nv_bfloat16* __restrict__ dup, long long rows, int I, long long ld_in, long long ld_out) {
   const long long nvec = rows * (I >> 3);
   for (long long i = blockIdx.x * 256LL + threadIdx.x; i < nvec; i += gridDim.x * 256LL) {
-    const long long r = i / (I >> 3);
-    const int c = static_cast<int>(i % (I >> 3)) << 3;
+    long long at_h = i << 3, at_in = at_h, at_out = at_h;
+    if constexpr (!FLAT) {
+      const long long r = i / (I >> 3);
+      const int c = static_cast<int>(i - r * (I >> 3)) << 3;
+      at_in = r * ld_in + c;
+      at_out = r * ld_out + c;
+    }
     float d[8], e[8], g[8], de[8], dg[8];
-    unpack8(*reinterpret_cast<const bf16x8*>(dh + r * I + c), d);
-    unpack8(*reinterpret_cast<const bf16x8*>(gate + r * ld_in + c), e);
-    unpack8(*reinterpret_cast<const bf16x8*>(up + r * ld_in + c), g);
+    const bf16x8 pd = *reinterpret_cast<const bf16x8*>(dh + at_h), pe = *reinterpret_cast<const bf16x8*>(gate + at_in),
+                 pg = *reinterpret_cast<const bf16x8*>(up + at_in);
+    unpack8(pd, d);
+    unpack8(pe, e);
+    unpack8(pg, g);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      dg[j] = d[j] * act_fwd(e[j], act);
-      de[j] = d[j] * g[j] * act_bwd(e[j], act);
+      dg[j] = d[j] * act_fwd(e[j], ACT);
+      de[j] = d[j] * g[j] * act_bwd(e[j], ACT);
     }
-    *reinterpret_cast<bf16x8*>(dgate + r * ld_out + c) = pack8(de);
-    *reinterpret_cast<bf16x8*>(dup + r * ld_out + c) = pack8(dg);
+    *reinterpret_cast<bf16x8*>(dgate + at_out) = pack8(de);
+    *reinterpret_cast<bf16x8*>(dup + at_out) = pack8(dg);
   }
 }
 
@@ -400,20 +411,24 @@ struct RopeSrc {
   long long sb, st, sh;      // element strides of batch, token and head; the last dimension is contiguous
 };
 
+// Idx is 32 bits wide where the element count allows: two 64-bit divisions per vector cost more than its loads hid.  Measured on 16384 rows of
+// 32 + 8 heads of 128: 71.1 -> 65.9 us (51 at the copy rate).
+template <typename Idx>
 __global__ void __launch_bounds__(256)
 rope_qk_oop_kernel(RopeSrc qs, RopeSrc ks, __nv_bfloat16* __restrict__ qo, __nv_bfloat16* __restrict__ ko,
                    const float* __restrict__ cs, const float* __restrict__ sn, const int* __restrict__ pos,
                    long long rows, int seq_len, int Hq, int Hk, int D, float sign) {
   const int half = D >> 1;
   const int chunks = half >> 3;                          // 8-element chunks per half head
-  const long long per_row = static_cast<long long>(Hq + Hk) * chunks;
-  const long long total = rows * per_row;
-  for (long long i = blockIdx.x * 256LL + threadIdx.x; i < total; i += gridDim.x * 256LL) {
-    const long long r = i / per_row;
-    const int rem = static_cast<int>(i % per_row);
+  const unsigned per_row = static_cast<unsigned>(Hq + Hk) * chunks;
+  const Idx total = static_cast<Idx>(rows * per_row);
+  for (Idx i = static_cast<Idx>(blockIdx.x) * 256 + threadIdx.x; i < total; i += static_cast<Idx>(gridDim.x) * 256) {
+    const Idx r32 = i / per_row;
+    const int rem = static_cast<int>(i - r32 * per_row);
     const int h = rem / chunks;
-    const int d = (rem % chunks) << 3;
-    const long long b = r / seq_len, t = r % seq_len;
+    const int d = (rem - h * chunks) << 3;
+    const Idx b32 = r32 / static_cast<unsigned>(seq_len);
+    const long long r = r32, b = b32, t = r32 - b32 * static_cast<unsigned>(seq_len);
     const int pidx = pos ? pos[r] : static_cast<int>(t);
     const bool is_q = h < Hq;
     const int hh = is_q ? h : h - Hq;
@@ -657,10 +672,21 @@ extern "C" int ob_glu_bwd(const void* dh, const void* gate, const void* up, void
                           int I, long long ld_in, long long ld_out, int act, int sms, void* stream) {
   if (rows <= 0) return 0;
   if (I % 8 || ld_in % 8 || ld_out % 8) return -2;
-  glu_bwd_kernel<<<flat_grid(rows * (I / 8), 256, sms), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(dh), static_cast<const __nv_bfloat16*>(gate),
-      static_cast<const __nv_bfloat16*>(up), static_cast<__nv_bfloat16*>(dgate), static_cast<__nv_bfloat16*>(dup),
-      rows, I, ld_in, ld_out, act);
+  const unsigned grid = flat_grid(rows * (I / 8), 256, sms);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const __nv_bfloat16 *hp = static_cast<const __nv_bfloat16*>(dh), *gp = static_cast<const __nv_bfloat16*>(gate),
+                      *up_ = static_cast<const __nv_bfloat16*>(up);
+  __nv_bfloat16 *dgp = static_cast<__nv_bfloat16*>(dgate), *dup_ = static_cast<__nv_bfloat16*>(dup);
+  const bool flat = ld_in == I && ld_out == I;
+#define OB_GLU_BWD(A)                                                                                            \
+  do {                                                                                                           \
+    if (flat) glu_bwd_kernel<A, true><<<grid, 256, 0, st>>>(hp, gp, up_, dgp, dup_, rows, I, ld_in, ld_out);     \
+    else glu_bwd_kernel<A, false><<<grid, 256, 0, st>>>(hp, gp, up_, dgp, dup_, rows, I, ld_in, ld_out);         \
+  } while (0)
+  if (act == 0) OB_GLU_BWD(0);
+  else if (act == 1) OB_GLU_BWD(1);
+  else OB_GLU_BWD(2);
+#undef OB_GLU_BWD
   return OB_CHECK_LAUNCH();
 }
 
@@ -691,9 +717,14 @@ extern "C" int ob_rope_qk_oop(const void* q_in, const void* k_in, void* q_out, v
   RopeSrc qs{static_cast<const __nv_bfloat16*>(q_in), q_sb, q_st, q_sh};
   RopeSrc ks{static_cast<const __nv_bfloat16*>(k_in), k_sb, k_st, k_sh};
   const long long work = rows * (Hq + Hk) * (D / 16);
-  rope_qk_oop_kernel<<<flat_grid(work, 256, sms), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      qs, ks, static_cast<__nv_bfloat16*>(q_out), static_cast<__nv_bfloat16*>(k_out), cos_t, sin_t, pos, rows, seq_len, Hq,
-      Hk, D, backward ? -1.f : 1.f);
+  const unsigned grid = flat_grid(work, 256, sms);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  __nv_bfloat16 *qo = static_cast<__nv_bfloat16*>(q_out), *ko = static_cast<__nv_bfloat16*>(k_out);
+  const float sign = backward ? -1.f : 1.f;
+  if (work < 0x7fffffffLL)
+    rope_qk_oop_kernel<unsigned><<<grid, 256, 0, st>>>(qs, ks, qo, ko, cos_t, sin_t, pos, rows, seq_len, Hq, Hk, D, sign);
+  else
+    rope_qk_oop_kernel<unsigned long long><<<grid, 256, 0, st>>>(qs, ks, qo, ko, cos_t, sin_t, pos, rows, seq_len, Hq, Hk, D, sign);
   return OB_CHECK_LAUNCH();
 }
 

