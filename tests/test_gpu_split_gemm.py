@@ -73,3 +73,30 @@ def test_lora_operands_packed_in_one_launch():
         f = [(torch.randn(r, d, device="cuda", dtype=torch.bfloat16), torch.randn(o, r, device="cuda", dtype=torch.bfloat16)) for o in outs]
         a, b = ops.lora_pack(f)
         assert torch.equal(a, torch.cat([x for x, _ in f])) and torch.equal(b, torch.block_diag(*[y for _, y in f]))
+
+
+@pytest.mark.parametrize("M,N,K,splits", [(1, 8, 8, 1), (128, 64, 64, 1), (130, 72, 1000, 1), (130, 72, 1000, 5), (257, 328, 136, 2), (64, 16, 2048, 8),
+                                          (20000, 56, 72, 1)])
+def test_narrow_tiles(M, N, K, splits):
+    from opaque_b200 import ops
+    torch.manual_seed(M + N)
+    a, bias = torch.randn(M, K, device="cuda", dtype=torch.bfloat16), torch.randn(N, device="cuda", dtype=torch.bfloat16)
+    a2 = torch.randn(M, 16, device="cuda", dtype=torch.bfloat16)
+    for layout, layout2 in (("nk", "kn"), ("kn", "nk")):
+        w = torch.randn((N, K) if layout == "nk" else (K, N), device="cuda", dtype=torch.bfloat16)
+        b2 = torch.randn((N, 16) if layout2 == "nk" else (16, N), device="cuda", dtype=torch.bfloat16)
+        prod = a.float() @ (w.float().t() if layout == "nk" else w.float()) + a2.float() @ (b2.float().t() if layout2 == "nk" else b2.float())
+        buf = torch.full((M, N + 8), 7.0, device="cuda", dtype=torch.bfloat16)
+        kw = dict(b_layout=layout, a2=a2, b2=b2, b2_layout=layout2, bias=bias, alpha=0.5, kernel="single", splits=splits)
+        ops.gemm(a, w, out=buf[:, :N], block_n=64, **kw)
+        assert _rel(buf[:, :N], 0.5 * prod + bias.float()) < TOL and bool((buf[:, N:] == 7.0).all())
+        # a tile's k-blocks are added in the same order whatever its width
+        assert torch.equal(buf[:, :N], ops.gemm(a, w, block_n=256, **kw))
+    with pytest.raises(ops.KernelLibraryError):
+        ops.gemm(a, w, b_layout="kn", kernel="single", block_n=128)
+
+
+def test_tile_width_follows_the_number_of_narrow_tiles():
+    from opaque_b200 import ops
+    assert ops.pick_tile_width(10 ** 6, 64, 2) == 64 and ops.pick_tile_width(128, 768, 12) == 64 and ops.pick_tile_width(128, 768, 48, 12) == 64
+    assert ops.pick_tile_width(2048, 768, 12) == 256 and ops.pick_tile_width(16384, 3072, 12) == 256 and ops.pick_tile_width(128, 50304, 12) == 256
