@@ -315,7 +315,9 @@ layernorm_fwd_warp_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat
 // The backward kernel keeps one row per launched warp and re-reads the weight per row: the weight is a quarter of its
 // wavefronts (dy, x in, dx out), and the registers for a resident copy cost more occupancy than the re-reads cost
 // (measured inside the GPT-2 step: 17.0 us per launch this way, 19.2 us with the walking form of the forward kernel).
-// RES: `ds`, the gradient that reaches the row past the norm (the residual branch), is added in.
+// RES: `ds`, the gradient that reaches the row past the norm (the residual branch), is added in.  The norm's own gradient is
+// rounded to bf16 first and the sum after it, as two tensors of that type add up: where many rows' gradients nearly cancel (a
+// bias of the first block), one rounding instead of two moved single sums by more than their root mean square.
 template <int VPL, bool RES>
 __global__ void __launch_bounds__(32 * LN_WARPS)
 layernorm_bwd_dx_warp_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
@@ -360,7 +362,7 @@ layernorm_bwd_dx_warp_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bf
         float h[8];
         ln_unpack8(reinterpret_cast<const ln_bf16x8*>(ds + row * H)[i], h);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) gw[v][j] += h[j];
+        for (int j = 0; j < 8; ++j) gw[v][j] = __bfloat162float(__float2bfloat16_rn(gw[v][j])) + h[j];
       }
       or_[i] = ln_pack8(gw[v]);
     }
