@@ -609,60 +609,49 @@ def pick_gemm_kernel(M: int, N: int, K: int, sms: int = 148) -> str:
     return "pair" if eff_pair >= eff_single else "single"
 
 
-def _single_us(M: int, N: int, nk: int, splits: int, width: int, sms: int) -> float:
-    """Estimated microseconds of the single-CTA kernel, ``splits`` of it along ``nk`` k-blocks, tiles ``width`` columns wide.
+def _single_us(M: int, N: int, nk: int, width: int, sms: int) -> float:
+    """Estimated microseconds of the single-CTA kernel along ``nk`` k-blocks, tiles ``width`` columns wide.
 
-    Fitted to launches back to back in a CUDA graph with weights from HBM (41 shapes of 1 to 16384 rows, 1 to 24 splits): the
-    fastest choice by these estimates takes 604 us over all of them, the best of every shape 600."""
-    ctas = -(-M // 128) * -(-N // width) * splits
+    Fitted to launches back to back in a CUDA graph with weights from HBM: over 41 shapes of 1 to 16384 rows the width with the
+    smaller estimate was the faster one every time."""
+    ctas = -(-M // 128) * -(-N // width)
     waves, busy = -(-ctas // sms), min(ctas, sms)
     start, per_kb = (5.2, 0.346 + 0.0011 * busy) if width == 256 else (3.9, 0.298 + 0.00036 * busy)
-    return start + per_kb * -(-nk // splits) * waves + (2.2 + 0.76e-6 * M * N * splits if splits > 1 else 0.0)
+    return start + per_kb * nk * waves
 
 
 @functools.lru_cache(maxsize=4096)
-def pick_tile_width(M: int, N: int, nk: int, splits: int = 1, sms: int = 148) -> int:
+def pick_tile_width(M: int, N: int, nk: int, sms: int = 148) -> int:
     """Columns per tile of the single-CTA kernel: 64 where one such tile covers ``N`` (16384 x 48 x 4096: 27.6 us, 32.9 with 256),
     or where all narrow tiles run at once and are faster by :func:`_single_us` (128 x 768 x 768: 7.7 and 9.5); beyond one wave they
     lose (2048 x 768 x 768: 12.3 and 9.7)."""
     if N <= 64:
         return 64
-    fits = -(-M // 128) * -(-N // 64) * splits <= sms
-    return 64 if fits and _single_us(M, N, nk, splits, 64, sms) < _single_us(M, N, nk, splits, 256, sms) else 256
+    fits = -(-M // 128) * -(-N // 64) <= sms
+    return 64 if fits and _single_us(M, N, nk, 64, sms) < _single_us(M, N, nk, 256, sms) else 256
 
 
 @functools.lru_cache(maxsize=4096)
-def pick_gemm_plan(M: int, N: int, K: int, K2: int = 0, sms: int = 148) -> tuple[str, int]:
-    """``(kernel, splits)`` for an ungrouped ``[M, K] x [K, N]`` product (plus a ``K2`` segment).
+def pick_gemm_plan(M: int, N: int, K: int, K2: int = 0, sms: int = 148) -> str:
+    """``"pair"`` or ``"single"`` for an ungrouped ``[M, K] x [K, N]`` product (plus a ``K2`` segment): the same bits either way.
 
-    Starts from :func:`pick_gemm_kernel`.  Where that kernel's tiles do not fill the chip once, the alternatives are weighed
-    by estimated microseconds: a pair takes 6.6 + 0.567 per k-block (256 x 2048 x 8192: 79.5 measured), the single-CTA kernel
-    :func:`_single_us` at the better tile width (one CTA per tile 52.0, 8 splits 18.7).
-
-    A split has to win a microsecond (its second launch's host time) and an eighth: an unsplit product has the same bits in every
-    kernel and at every tile width, a split one's depend on the plan, which moves near-ties of an expert router behind it.
+    :func:`pick_gemm_kernel`'s choice; where a pair's tiles do not fill the chip once, the two are weighed by estimated
+    microseconds: a pair takes 6.6 + 0.567 per k-block (256 x 2048 x 8192: 79.5 measured), the single-CTA kernel
+    :func:`_single_us` at the better tile width (52.0).
     """
-    big = pick_gemm_kernel(M, N, K, sms)
+    if pick_gemm_kernel(M, N, K, sms) == "single":
+        return "single"
     nk = -(-K // 64) + -(-K2 // 64)
-    rows = -(-M // 128)
-    if (-(-M // 512) * -(-N // 256) >= max(sms // 2, 1)) if big == "pair" else rows * -(-N // 256) >= sms:
-        return (big, 1)
-    single = _single_us(M, N, nk, 1, pick_tile_width(M, N, nk, 1, sms), sms)
-    best = (6.6 + 0.567 * nk, "pair", 1) if big == "pair" and 6.6 + 0.567 * nk < single else (single, "single", 1)
-    for s in (2, 3, 4, 6, 8, 12, 16, 24):
-        if s > nk or rows * -(-N // 256) * s > 2 * sms or N % 4:
-            break
-        t = _single_us(M, N, nk, s, pick_tile_width(M, N, nk, s, sms), sms) + 1.0
-        if t < min(best[0], 0.87 * single):
-            best = (t, "single", s)
-    return best[1:]
+    if -(-M // 512) * -(-N // 256) >= max(sms // 2, 1):
+        return "pair"
+    return "pair" if 6.6 + 0.567 * nk < _single_us(M, N, nk, pick_tile_width(M, N, nk, sms), sms) else "single"
 
 
 def gemm(a: torch.Tensor, b: torch.Tensor, *, b_layout: str = "nk", a2: torch.Tensor | None = None,
          b2: torch.Tensor | None = None, bias: torch.Tensor | None = None, group_offs: torch.Tensor | None = None,
          out: torch.Tensor | None = None, status: StatusWord | None = None,
          wait_budget_s: float = DEFAULT_WAIT_BUDGET_S, kernel: str = "auto", b2_layout: str = "nk", alpha: float = 1.0,
-         splits: int = 1, block_n: int | None = None) -> torch.Tensor:
+         block_n: int | None = None) -> torch.Tensor:
     """``a @ op(b) + a2 @ b2ᵀ + bias`` on the tcgen05 path (bf16 in/out, fp32 accumulation).
 
     ``b_layout="nk"``: ``b`` is ``[N, K]`` (a weight matrix as stored; ``op(b) = bᵀ``);  ``"kn"``: ``b`` is ``[K, N]``
@@ -670,14 +659,13 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, b_layout: str = "nk", a2: torch.Te
     low-rank segment accumulated in the same tile (LoRA-fused linear).  With ``group_offs`` (int32 ``[E + 1]`` row
     offsets, rows sorted by group) ``b`` is ``[E, N, K]`` / ``[E, K, N]`` and rows of group e use slab e (MoE experts).
     ``kernel``: ``"pair"`` (two CTAs per 512 x 256 tile), ``"single"`` (one CTA per 128 x ``block_n`` tile, 256 or 64
-    columns, by default :func:`pick_tile_width`'s choice; ``splits`` CTAs along K)
-    or ``"auto"`` (:func:`pick_gemm_plan` for ungrouped products while :data:`PAIR_GEMM` is on; grouped products always run
-    on single CTAs).  ``b2_layout="kn"``: ``b2`` is stored ``[r, N]``.  ``alpha`` scales the fp32 products (not the bias;
+    columns, by default :func:`pick_tile_width`'s choice) or ``"auto"`` (:func:`pick_gemm_plan` for ungrouped products while
+    :data:`PAIR_GEMM` is on; grouped products always run on single CTAs).  ``b2_layout="kn"``: ``b2`` is stored ``[r, N]``.  ``alpha`` scales the fp32 products (not the bias;
     single-CTA kernel only, so ``"auto"`` takes it when ``alpha`` is given).
     """
     if group_offs is None and kernel == "auto" and PAIR_GEMM:
-        kernel, splits = pick_gemm_plan(a.shape[0], b.shape[1] if b_layout == "kn" else b.shape[0], a.shape[1],
-                                        0 if a2 is None else a2.shape[1], lib.sm_count())
+        kernel = pick_gemm_plan(a.shape[0], b.shape[1] if b_layout == "kn" else b.shape[0], a.shape[1], 0 if a2 is None else a2.shape[1],
+                                lib.sm_count())
         if alpha != 1.0:
             kernel = "single"
     if group_offs is None and kernel == "pair":
@@ -725,12 +713,11 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, b_layout: str = "nk", a2: torch.Te
     elif out.shape != (M, N) or out.dtype != torch.bfloat16 or out.stride(1) != 1:
         raise ValueError("out must be a row-major bf16 [M, N] matrix")
     if block_n is None:
-        block_n = 256 if grouped else pick_tile_width(M, N, -(-K // 64) + -(-K2 // 64), splits, lib.sm_count())
-    scratch = torch.empty(splits * -(-M // 128) * 128 * N, dtype=torch.float32, device=a.device) if splits > 1 else None
+        block_n = 256 if grouped else pick_tile_width(M, N, -(-K // 64) + -(-K2 // 64), lib.sm_count())
     rc = lib.load().ob_gemm_tn(a.data_ptr(), b2d.data_ptr(), lib.ptr(a2), lib.ptr(b2), lib.ptr(bias), out.data_ptr(), M, N,
                                K, K2, a.stride(0), b2d.stride(0), a2.stride(0) if a2 is not None else 0,
                                b2.stride(0) if b2 is not None else 0, out.stride(0), kn, int(b2_layout == "kn"), alpha,
-                               lib.ptr(group_offs), E, splits, block_n, lib.ptr(scratch), status.ptr() if status else None, wait_budget_s, lib.sm_count(), lib.stream())
+                               lib.ptr(group_offs), E, block_n, status.ptr() if status else None, wait_budget_s, lib.sm_count(), lib.stream())
     lib.check(rc, "gemm")
     return out
 

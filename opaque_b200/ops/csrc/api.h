@@ -61,13 +61,11 @@ int ob_wgrad_clip_pe_batch(const ob_wgrad_pe_desc* descs, int count, float* out,
 // D[M, N] = A[M, K1] op(B) + A2[M, K2] B2[N, K2]^T + bias, bf16 in / bf16 out, fp32 accumulation.  b_kn = 0: B is
 // [N, K1] row-major (per group: [groups * N, K1]); b_kn = 1: B is [K1, N] row-major (per group: [groups * K1, N]).
 // group_offs (int32 device array [num_groups + 1]) switches on the grouped mode: rows [offs[e], offs[e+1]) use slab e.
-// b2_kn = 1: B2 is [K2, N] row-major.  alpha scales the products, not the bias.  splits > 1 (ungrouped only) spreads each
-// tile's k-blocks over that many CTAs: fp32 partial products go to scratch (splits * ceil(rows_a / 128) * 128 * N floats,
-// 16-byte aligned, N % 4 == 0) and a second kernel adds them in split order.  block_n: columns per tile, 256 or (ungrouped) 64.
+// b2_kn = 1: B2 is [K2, N] row-major.  alpha scales the products, not the bias.  block_n: columns per tile, 256 or (ungrouped) 64.
 int ob_gemm_tn(const void* a, const void* b, const void* a2, const void* b2, const void* bias, void* out,
                long long rows_a, int N, int K1, int K2, long long lda, long long ldb, long long lda2, long long ldb2,
-               long long ldo, int b_kn, int b2_kn, float alpha, const int* group_offs, int num_groups, int splits, int block_n,
-               float* scratch, int* status, double wait_budget_s, int num_sms, void* stream);
+               long long ldo, int b_kn, int b2_kn, float alpha, const int* group_offs, int num_groups, int block_n,
+               int* status, double wait_budget_s, int num_sms, void* stream);
 
 // Dense GEMM on CTA pairs (tcgen05 cta_group::2, 256 x 256 tiles):  D = A op1(B) + A2 op2(B2) + bias.
 // b_kn / b2_kn = 1: that B operand is stored [K, N] row-major, 0: [N, K].  glu != 0: `b` holds the gate rows and `b_up`

@@ -16,11 +16,10 @@
 // a swizzled shared-memory slab per warp): with a short K (768) the drain of one tile takes about as long as its MMAs,
 // so four warps storing one 16-byte piece per lane and row left the tensor pipe waiting.  Every wait is bounded.
 //
-// Few rows (short records, small microbatches) make few tiles: 128 x 2304 is nine, and nine SMs then pull the whole weight.
-// With `splits` > 1 a tile's k-blocks go to that many CTAs; each stores its fp32 partial tile to scratch (it stays in L2)
-// and gemm_split_sum_kernel adds them in a fixed order, so results repeat bit for bit.
-// Measured (us; launches back to back, weights from HBM; pair kernel / one CTA per tile / split): 256 x 2048 x 8192 79.5 / 52.0 /
-// 18.7 with 8 splits, 128 x 768 x 3072 33.8 / 21.2 / 10.3 with 12, 128 x 768 x 50304 444 / 280 / 26.5 with 24.
+// A tile's k-blocks stay on one CTA and are added in order: every tile shape of this kernel and of the pair kernel gives the same
+// bits, so the choice between them (by size alone) never shows in a result.  Few rows make few tiles, and spreading a tile's
+// k-blocks over several CTAs is faster there (256 x 2048 x 8192: 52.0 us and 18.7 with 8 parts), but another order of the sums
+// moves bf16 roundings, and behind twelve layers single gradient sums by more than their root mean square.
 #include "common.cuh"
 #include "api.h"
 
@@ -28,16 +27,13 @@ namespace ob {
 
 int make_bf16_map_2d(CUtensorMap* map, const void* base, long long rows, long long cols, long long ld,
                      int box_cols, int box_rows);
-int make_f32_map_2d(CUtensorMap* map, const void* base, long long rows, long long cols, long long ld,
-                    int box_cols, int box_rows);
 
 constexpr int GT_BM = 128;
 constexpr int GT_BK = 64;
 constexpr int GT_A_BYTES = GT_BM * GT_BK * 2;
 // Tile width: 256 columns, or 64 where the wide tiles leave most SMs idle or N is narrower than that.  A k-block of a lone tile
-// takes about 0.34 us wide and 0.31 narrow, so what a narrow tile saves is its shorter start and epilogue, and what it gains
-// is four times as many tiles to split the k-blocks over.  Measured (us, wide / narrow, best split of each): 128 x 768 x 768
-// 9.5 / 7.7, 128 x 768 x 3072 10.3 / 8.0, 16384 x 48 x 4096 32.9 / 27.6; 2048 x 768 x 768 9.7 / 12.3 (two waves).
+// takes about 0.34 us wide and 0.31 narrow, so what a narrow tile saves is its shorter start and epilogue.  Measured (us, wide /
+// narrow): 128 x 768 x 768 9.5 / 7.7, 16384 x 48 x 4096 32.9 / 27.6; 2048 x 768 x 768 9.7 / 12.3 (two waves).
 template <int BN>
 struct GtTile {
   static constexpr int B_BYTES = BN * GT_BK * 2;
@@ -63,32 +59,19 @@ struct GemmParams {
   int tma_store;           // the output leaves through bulk tensor stores (map_out is valid)
   int b2_kn;               // B2 is [K2, N] (N-major) instead of [N, K2]
   float alpha;             // scales the products
-  int splits;              // CTAs per tile; > 1: map_out is the fp32 scratch [splits * m_pad, N]
-  int m_pad;               // rows of one split's scratch matrix
   int* status;
   unsigned long long wait_budget_ns;
 };
 
 struct GtItem {
   int row0, row_end, n0, b_row;
-  int kb0, kb1, out_row;     // k-blocks of this item; output row (scratch row with splits) of the tile's first row
 };
 
 // Tile w of the persistent schedule.  `cursor` is the caller's monotone group cursor (grouped mode only).
-template <bool SPLIT, int BN>
-__device__ __forceinline__ GtItem gt_decode(const GemmParams& p, int w, int tiles_m, int tiles_n, int num_kb, const int* tile_start,
-                                            int& cursor) {
+template <int BN>
+__device__ __forceinline__ GtItem gt_decode(const GemmParams& p, int w, int tiles_m, int tiles_n, const int* tile_start, int& cursor) {
   GtItem it;
-  it.kb0 = 0;
-  it.kb1 = num_kb;
   if (p.group_offs == nullptr) {
-    int split = 0;
-    if constexpr (SPLIT) {
-      split = w / (tiles_m * tiles_n);
-      w -= split * (tiles_m * tiles_n);
-      it.kb0 = static_cast<int>(static_cast<long long>(num_kb) * split / p.splits);
-      it.kb1 = static_cast<int>(static_cast<long long>(num_kb) * (split + 1) / p.splits);
-    }
     const int band = GT_GROUP_M * tiles_n;
     const int b = w / band, r = w % band;
     const int m_in_band = min(GT_GROUP_M, tiles_m - b * GT_GROUP_M);
@@ -98,7 +81,6 @@ __device__ __forceinline__ GtItem gt_decode(const GemmParams& p, int w, int tile
     it.row_end = p.M;
     it.n0 = nt * BN;
     it.b_row = 0;
-    it.out_row = it.row0 + split * p.m_pad;
   } else {
     const int g = w / tiles_n;
     while (g >= tile_start[cursor + 1]) ++cursor;
@@ -106,13 +88,11 @@ __device__ __forceinline__ GtItem gt_decode(const GemmParams& p, int w, int tile
     it.row_end = p.group_offs[cursor + 1];
     it.n0 = (w % tiles_n) * BN;
     it.b_row = cursor * p.b_group_rows;
-    it.out_row = it.row0;
   }
   return it;
 }
 
-// SPLIT is a template parameter so that the ordinary epilogue keeps its registers
-template <bool B_KN, bool SPLIT, int BN>
+template <bool B_KN, int BN>
 __global__ void __launch_bounds__(GT_THREADS, 1)
 gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                const __grid_constant__ CUtensorMap map_a2, const __grid_constant__ CUtensorMap map_b2,
@@ -173,7 +153,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   const int tiles_m = p.group_offs ? tile_start[p.num_groups] : (p.M + GT_BM - 1) / GT_BM;
-  const int total_work = tiles_m * tiles_n * p.splits;
+  const int total_work = tiles_m * tiles_n;
 
   if (warp == 0) {
     if (lane == 0) {
@@ -181,8 +161,8 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       uint32_t phase = 0, issued_mask = 0, issued_phase = 0;
       bool ok = true;
       for (int w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
-        const GtItem it = gt_decode<SPLIT, BN>(p, w, tiles_m, tiles_n, num_kb, tile_start, cursor);
-        for (int kb = it.kb0; kb < it.kb1; ++kb) {
+        const GtItem it = gt_decode<BN>(p, w, tiles_m, tiles_n, tile_start, cursor);
+        for (int kb = 0; kb < num_kb; ++kb) {
           if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, p.status, OB_ERR_WAIT_EMPTY, budget)) {
             ok = false;
             break;
@@ -230,7 +210,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       uint32_t phase = 0;
       bool ok = true;
       for (int w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
-        const GtItem it = gt_decode<SPLIT, BN>(p, w, tiles_m, tiles_n, num_kb, tile_start, cursor);
+        const GtItem it = gt_decode<BN>(p, w, tiles_m, tiles_n, tile_start, cursor);
         const int as = acc_iter & 1;
         if (!mbar_wait(&tmem_empty[as], ((acc_iter >> 1) & 1) ^ 1, abort_flag, p.status, OB_ERR_WAIT_TMEM_EMPTY,
                        budget)) {
@@ -239,7 +219,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + as * BN;
-        for (int kb = it.kb0; kb < it.kb1; ++kb) {
+        for (int kb = 0; kb < num_kb; ++kb) {
           if (!mbar_wait(&full[stage], phase, abort_flag, p.status, OB_ERR_WAIT_FULL, budget)) {
             ok = false;
             break;
@@ -255,7 +235,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             const uint64_t ad = make_smem_desc(a_addr + kk * 32, 16, 1024, 2);
             const uint64_t bd = kn ? make_smem_desc(b_addr + kk * (16 * 128), GT_BK * 128, 1024, 2)
                                    : make_smem_desc(b_addr + kk * 32, 16, 1024, 2);
-            umma_bf16(d_tmem, ad, bd, kn ? idesc_nmaj : idesc_kmaj, (kb > it.kb0 || kk > 0) ? 1u : 0u);
+            umma_bf16(d_tmem, ad, bd, kn ? idesc_nmaj : idesc_kmaj, (kb > 0 || kk > 0) ? 1u : 0u);
           }
           umma_commit(&empty[stage]);
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
@@ -276,7 +256,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     bool ok = true;
     const bool vec_ok = ((p.ldo & 7) == 0) && ((reinterpret_cast<uintptr_t>(p.out) & 15) == 0);
     for (int w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
-      const GtItem it = gt_decode<SPLIT, BN>(p, w, tiles_m, tiles_n, num_kb, tile_start, cursor);
+      const GtItem it = gt_decode<BN>(p, w, tiles_m, tiles_n, tile_start, cursor);
       const int as = acc_iter & 1;
       if (!mbar_wait(&tmem_full[as], (acc_iter >> 1) & 1, abort_flag, p.status, OB_ERR_WAIT_TMEM_FULL, budget)) {
         ok = false;
@@ -285,69 +265,41 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       tc_fence_after();
       const int row0 = it.row0 + q * 32;
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + as * BN + g * (BN / 2);
-      if constexpr (SPLIT) {
-        // partial product: fp32, 32 x 32 values per bulk tensor store (columns past N are clipped; rows past M land in the
-        // padding of this split's scratch matrix)
+      // Both 64-column rounds go to registers (packed bf16) first, so the accumulator is back with the tensor pipe before
+      // a single store is issued.  Tiles that end inside a group's rows are masked by hand; all others leave through
+      // bulk tensor stores, which clip at the tensor's own bounds.
+      constexpr int ROUNDS = BN == 256 ? 2 : 1;          // a narrow tile is one round of the first four warps
+      const bool mine = BN == 256 || g == 0;
+      uint32_t pk[ROUNDS][32];
 #pragma unroll
-        for (int c = 0; c < BN / 64; ++c) {
-          const int nc = it.n0 + g * (BN / 2) + c * 32;
-          if (nc < p.N) {
-            float v[32];
-            tmem_ld32(t_row + c * 32, v);
-            tmem_ld_wait();
-            if (lane == 0) tma_store_wait_read();
-            __syncwarp();
-            slab_row32(slab, v, lane);
-            fence_proxy_async_smem();
-            __syncwarp();
-            if (lane == 0) {
-              tma_store_2d(&map_out, slab, nc, it.out_row + q * 32);
-              tma_store_commit();
-            }
+      for (int c = 0; c < ROUNDS; ++c) {
+        const int nc = it.n0 + g * (BN / 2) + c * 64;
+        if (mine && nc < p.N) {
+          float v[64];
+          tmem_ld32(t_row + c * 64, v);
+          tmem_ld32(t_row + c * 64 + 32, v + 32);
+          tmem_ld_wait();
+          if (p.alpha != 1.f) {
+#pragma unroll
+            for (int j = 0; j < 64; ++j) v[j] *= p.alpha;
           }
+          if (p.bias != nullptr) add_bias64(v, p.bias, nc, p.N);
+#pragma unroll
+          for (int j = 0; j < 32; ++j) pk[c][j] = pack_bf16x2(v[2 * j], v[2 * j + 1]);
         }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&tmem_empty[as]);
-        ++acc_iter;
-        continue;
-      } else {
-        // Both 64-column rounds go to registers (packed bf16) first, so the accumulator is back with the tensor pipe before
-        // a single store is issued.  Tiles that end inside a group's rows are masked by hand; all others leave through
-        // bulk tensor stores, which clip at the tensor's own bounds.
-        constexpr int ROUNDS = BN == 256 ? 2 : 1;          // a narrow tile is one round of the first four warps
-        const bool mine = BN == 256 || g == 0;
-        uint32_t pk[ROUNDS][32];
-#pragma unroll
-        for (int c = 0; c < ROUNDS; ++c) {
-          const int nc = it.n0 + g * (BN / 2) + c * 64;
-          if (mine && nc < p.N) {
-            float v[64];
-            tmem_ld32(t_row + c * 64, v);
-            tmem_ld32(t_row + c * 64 + 32, v + 32);
-            tmem_ld_wait();
-            if (p.alpha != 1.f) {
-#pragma unroll
-              for (int j = 0; j < 64; ++j) v[j] *= p.alpha;
-            }
-            if (p.bias != nullptr) add_bias64(v, p.bias, nc, p.N);
-#pragma unroll
-            for (int j = 0; j < 32; ++j) pk[c][j] = pack_bf16x2(v[2 * j], v[2 * j + 1]);
-          }
-        }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&tmem_empty[as]);
-        const bool use_tma = p.tma_store != 0 && (p.group_offs == nullptr || row0 + 32 <= it.row_end);
-#pragma unroll
-        for (int c = 0; c < ROUNDS; ++c) {
-          const int nc = it.n0 + g * (BN / 2) + c * 64;
-          if (mine && nc < p.N)
-            store_tile64_packed(slab, pk[c], &map_out, use_tma, nc, row0, p.out, p.ldo, it.row_end - row0, p.N - nc, vec_ok,
-                                lane);
-        }
-        ++acc_iter;
       }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&tmem_empty[as]);
+      const bool use_tma = p.tma_store != 0 && (p.group_offs == nullptr || row0 + 32 <= it.row_end);
+#pragma unroll
+      for (int c = 0; c < ROUNDS; ++c) {
+        const int nc = it.n0 + g * (BN / 2) + c * 64;
+        if (mine && nc < p.N)
+          store_tile64_packed(slab, pk[c], &map_out, use_tma, nc, row0, p.out, p.ldo, it.row_end - row0, p.N - nc, vec_ok,
+                              lane);
+      }
+      ++acc_iter;
     }
     if (lane == 0) tma_store_wait_all();         // this lane's bulk stores are done before shared memory is given back
   }
@@ -360,63 +312,18 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   }
 }
 
-// out[m, n] = alpha * sum over splits of part[s][m][n] + bias[n], splits added in order; 4 columns per thread.  The loads of a
-// group of 8, 4 or 2 splits are in flight together: a remainder loaded one by one made 128 x 768 x 3072 with 12 splits 11.5 us
-// instead of 10.3.
-template <int COUNT>
-__device__ __forceinline__ void add_parts(float4& a, const float* src, long long step) {
-  float4 v[COUNT];                        // all loads in flight before the first addition
-#pragma unroll
-  for (int s = 0; s < COUNT; ++s) v[s] = __ldg(reinterpret_cast<const float4*>(src + s * step));
-#pragma unroll
-  for (int s = 0; s < COUNT; ++s) { a.x += v[s].x; a.y += v[s].y; a.z += v[s].z; a.w += v[s].w; }
-}
-
-__global__ void __launch_bounds__(256)
-gemm_split_sum_kernel(const float* __restrict__ part, const __nv_bfloat16* __restrict__ bias, __nv_bfloat16* __restrict__ out,
-                      int M, int N, int m_pad, int splits, long long ldo, float alpha, int vec) {
-  const int n4 = N >> 2;
-  const long long total = static_cast<long long>(M) * n4, step = static_cast<long long>(m_pad) * N;
-  for (long long i = blockIdx.x * 256LL + threadIdx.x; i < total; i += gridDim.x * 256LL) {
-    const int m = static_cast<int>(i / n4), n = static_cast<int>(i % n4) * 4;
-    const float* src = part + static_cast<long long>(m) * N + n;
-    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int s = 0; s + 8 <= splits; s += 8) add_parts<8>(a, src + s * step, step);
-    src += (splits & ~7) * step;
-    if (splits & 4) { add_parts<4>(a, src, step); src += 4 * step; }
-    if (splits & 2) { add_parts<2>(a, src, step); src += 2 * step; }
-    if (splits & 1) add_parts<1>(a, src, step);
-    float f[4] = {a.x * alpha, a.y * alpha, a.z * alpha, a.w * alpha};
-    if (bias != nullptr) {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) f[j] += __bfloat162float(__ldg(bias + n + j));
-    }
-    __nv_bfloat16* dst = out + m * ldo + n;
-    if (vec) {
-      *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]));
-    } else {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) dst[j] = __float2bfloat16_rn(f[j]);
-    }
-  }
-}
-
 }  // namespace ob
 
 extern "C" int ob_gemm_tn(const void* a, const void* b, const void* a2, const void* b2, const void* bias, void* out,
                           long long rows_a, int N, int K1, int K2, long long lda, long long ldb, long long lda2,
                           long long ldb2, long long ldo, int b_kn, int b2_kn, float alpha, const int* group_offs, int num_groups,
-                          int splits, int block_n, float* scratch, int* status, double wait_budget_s, int num_sms, void* stream) {
+                          int block_n, int* status, double wait_budget_s, int num_sms, void* stream) {
   using namespace ob;
   if (rows_a <= 0 || N <= 0 || K1 <= 0) return 0;
   if (rows_a > 0x7fffffffLL - GT_BM) return -40;
   if (group_offs != nullptr && (num_groups < 1 || num_groups > GT_MAX_GROUPS)) return -41;
   if (K2 > 0 && (a2 == nullptr || b2 == nullptr)) return -42;
-  const int nk = (K1 + GT_BK - 1) / GT_BK + (K2 + GT_BK - 1) / GT_BK;
-  if (splits < 1) splits = 1;
   if ((block_n != 64 && block_n != 256) || (block_n == 64 && group_offs != nullptr)) return -46;
-  if (splits > 1 && (group_offs != nullptr || splits > nk || (N & 3) || scratch == nullptr || (reinterpret_cast<uintptr_t>(scratch) & 15)))
-    return -45;
   const int groups = group_offs ? num_groups : 1;
   CUtensorMap ma, mb, ma2, mb2;
   int rc = make_bf16_map_2d(&ma, a, rows_a, K1, lda, GT_BK, GT_BM);
@@ -436,9 +343,7 @@ extern "C" int ob_gemm_tn(const void* a, const void* b, const void* a2, const vo
     mb2 = mb;
   }
   using Kernel = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap, const GemmParams);
-  static const Kernel kernels[8] = {gemm_tn_kernel<false, false, 256>, gemm_tn_kernel<true, false, 256>, gemm_tn_kernel<false, true, 256>,
-                                    gemm_tn_kernel<true, true, 256>,   gemm_tn_kernel<false, false, 64>, gemm_tn_kernel<true, false, 64>,
-                                    gemm_tn_kernel<false, true, 64>,   gemm_tn_kernel<true, true, 64>};
+  static const Kernel kernels[4] = {gemm_tn_kernel<false, 256>, gemm_tn_kernel<true, 256>, gemm_tn_kernel<false, 64>, gemm_tn_kernel<true, 64>};
   static bool configured = false;
   if (!configured) {
     for (Kernel k : kernels)
@@ -460,27 +365,14 @@ extern "C" int ob_gemm_tn(const void* a, const void* b, const void* a2, const vo
   const long long tiles_m_bound = (rows_a + GT_BM - 1) / GT_BM + (group_offs ? groups : 0);
   p.b2_kn = b2_kn;
   p.alpha = alpha;
-  p.splits = splits;
-  const long long m_pad = (rows_a + GT_BM - 1) / GT_BM * GT_BM;
-  if (splits > 1 && m_pad * splits > 0x7fffffffLL) return -40;
-  p.m_pad = static_cast<int>(m_pad);
-  const long long total = tiles_m_bound * tiles_n * splits;
+  const long long total = tiles_m_bound * tiles_n;
   if (total > 0x7fffffffLL - num_sms) return -40;
   const int grid = static_cast<int>(total < num_sms ? total : num_sms);
   CUtensorMap mo = ma;
   p.tma_store = 0;
-  if (splits > 1) {
-    rc = make_f32_map_2d(&mo, scratch, m_pad * splits, N, N, 32, 32);
-    if (rc) return rc;
-  } else if ((reinterpret_cast<uintptr_t>(out) & 15) == 0 && ((ldo * 2) & 15) == 0 &&
+  if ((reinterpret_cast<uintptr_t>(out) & 15) == 0 && ((ldo * 2) & 15) == 0 &&
       make_bf16_map_2d(&mo, out, rows_a, N, ldo, 64, 32) == 0)
     p.tma_store = 1;
-  const cudaStream_t st = static_cast<cudaStream_t>(stream);
-  kernels[(block_n == 64 ? 4 : 0) + (splits > 1 ? 2 : 0) + (b_kn ? 1 : 0)]<<<grid, GT_THREADS, GT_SMEM, st>>>(ma, mb, ma2, mb2, mo, p);
-  if (splits > 1) {
-    const long long blocks = (rows_a * (N >> 2) + 255) / 256, cap = num_sms * 8LL;
-    gemm_split_sum_kernel<<<static_cast<unsigned>(blocks < cap ? blocks : cap), 256, 0, st>>>(
-        scratch, p.bias, p.out, p.M, N, p.m_pad, splits, ldo, alpha, (ldo & 3) == 0 && (reinterpret_cast<uintptr_t>(out) & 7) == 0);
-  }
+  kernels[(block_n == 64 ? 2 : 0) + (b_kn ? 1 : 0)]<<<grid, GT_THREADS, GT_SMEM, static_cast<cudaStream_t>(stream)>>>(ma, mb, ma2, mb2, mo, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -44;
 }

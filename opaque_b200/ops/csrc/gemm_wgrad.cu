@@ -742,20 +742,20 @@ static EncodeTiledFn get_encode_fn() {
 
 static thread_local char g_map_detail[192] = {0};
 
-// 2-D bf16 tensor map over a row-major [rows, cols] matrix with row pitch `ld` elements.
 // bf16 [examples][rows][cols] with row pitch ld, 64 x 64 boxes (a box never crosses into the next example)
 static int make_bf16_map_3d(CUtensorMap* map, const void* base, long long examples, long long rows, long long cols, long long ld);
 
-static int make_map_2d(CUtensorMap* map, CUtensorMapDataType type, int elem, const void* base, long long rows, long long cols,
-                       long long ld, int box_cols, int box_rows) {
+// 2-D bf16 tensor map over a row-major [rows, cols] matrix with row pitch `ld` elements.
+int make_bf16_map_2d(CUtensorMap* map, const void* base, long long rows, long long cols, long long ld,
+                     int box_cols, int box_rows) {
   EncodeTiledFn enc = get_encode_fn();
   if (enc == nullptr) return -10;
-  if ((reinterpret_cast<uintptr_t>(base) & 15) != 0 || ((ld * elem) & 15) != 0) {
+  if ((reinterpret_cast<uintptr_t>(base) & 15) != 0 || ((ld * 2) & 15) != 0) {
     snprintf(g_map_detail, sizeof(g_map_detail), "operand not 16-byte aligned: base=%p ld=%lld", base, ld);
     return -11;
   }
   cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
-  cuuint64_t strides[1] = {static_cast<cuuint64_t>(ld) * elem};
+  cuuint64_t strides[1] = {static_cast<cuuint64_t>(ld) * 2};
   cuuint32_t box[2] = {static_cast<cuuint32_t>(box_cols), static_cast<cuuint32_t>(box_rows)};
   cuuint32_t estr[2] = {1, 1};
   // Driver entry points need a context bound to the calling thread; framework worker threads (autograd) may never
@@ -765,17 +765,13 @@ static int make_map_2d(CUtensorMap* map, CUtensorMapDataType type, int elem, con
     int dev = 0;
     if (cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess) bound = true;
   }
-  const CUresult r = enc(map, type, 2, const_cast<void*>(base), dims, strides, box,
+  const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box,
                          estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS)
     snprintf(g_map_detail, sizeof(g_map_detail), "tensor map rejected (CUresult %d): base=%p rows=%lld cols=%lld ld=%lld box=%dx%d",
              static_cast<int>(r), base, rows, cols, ld, box_cols, box_rows);
   return r == CUDA_SUCCESS ? 0 : -12;
-}
-int make_bf16_map_2d(CUtensorMap* map, const void* base, long long rows, long long cols, long long ld,
-                     int box_cols, int box_rows) {
-  return make_map_2d(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, rows, cols, ld, box_cols, box_rows);
 }
 static int make_bf16_map_3d(CUtensorMap* map, const void* base, long long examples, long long rows, long long cols, long long ld) {
   CUtensorMap whole;                     // the checks (alignment, pitch) and the thread's context of the 2-D form
@@ -792,10 +788,6 @@ static int make_bf16_map_3d(CUtensorMap* map, const void* base, long long exampl
     snprintf(g_map_detail, sizeof(g_map_detail), "tensor map rejected (CUresult %d): base=%p examples=%lld rows=%lld cols=%lld ld=%lld",
              static_cast<int>(r), base, examples, rows, cols, ld);
   return r == CUDA_SUCCESS ? 0 : -12;
-}
-int make_f32_map_2d(CUtensorMap* map, const void* base, long long rows, long long cols, long long ld,
-                    int box_cols, int box_rows) {
-  return make_map_2d(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, rows, cols, ld, box_cols, box_rows);
 }
 
 // Tensor map of an fp32 destination [groups][m][n] with row pitch ldm and group pitch gstride (elements), 32 x 32 boxes in the

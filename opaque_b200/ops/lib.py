@@ -24,7 +24,7 @@ _SIGNATURES = {
     "ob_ghost_norm_batch": [c_char_p, I, P, D, I, P],
     "ob_wgrad_clip_batch": [c_char_p, I, P, P, LL, I, P, D, I, P],
     "ob_wgrad_clip_pe_batch": [c_char_p, I, P, P, LL, P, D, I, P],
-    "ob_gemm_tn": [P, P, P, P, P, P, LL, I, I, I, LL, LL, LL, LL, LL, I, I, F, P, I, I, I, P, P, D, I, P],
+    "ob_gemm_tn": [P, P, P, P, P, P, LL, I, I, I, LL, LL, LL, LL, LL, I, I, F, P, I, I, P, D, I, P],
     "ob_lora_pack": [P, P, P, P, P, P, P, P, I, I, I, I, I, I, P],
     "ob_gemm_pair": [P, P, P, P, P, P, P, P, P, P, LL, I, I, I, LL, LL, LL, LL, LL, I, I, I, I, P, D, I, P],
     "ob_pair_init": [],

@@ -1,5 +1,5 @@
-"""Products whose k-blocks are split over several CTAs per tile: edges of rows, columns and k-blocks, both layouts of both
-segments, scale and bias, pitched outputs.
+"""Products on the single-CTA kernel: edges of rows, columns and k-blocks, both layouts of both segments, scale and bias, pitched
+outputs, narrow tiles; and the same bits from every kernel and tile shape that ``auto`` chooses between.
 
 Tolerance: operands are bf16 and products exact in fp32; the fp32 sum of K terms and the final rounding to bf16 leave a relative
 2-norm error of 2^-9 (rounding) + K * 2^-24, below 4e-3 for every K here.
@@ -17,9 +17,11 @@ def _rel(x, y):
     return float((x.float() - y.float()).norm() / y.float().norm())
 
 
-@pytest.mark.parametrize("M,N,K,K2", [(1, 8, 64, 0), (127, 64, 520, 16), (128, 264, 512, 64), (129, 136, 1000, 48), (300, 520, 4096, 8), (257, 200, 768, 768)])
+@pytest.mark.parametrize("M,N,K,K2", [(1, 8, 64, 0), (127, 64, 520, 16), (128, 264, 512, 64), (129, 136, 1000, 48), (300, 520, 4096, 8), (257, 200, 768, 768),
+                                      (128, 768, 3072, 0), (1285, 768, 3072, 0), (256, 2048, 8192, 0), (300, 768, 50304, 0)])
 @pytest.mark.parametrize("layout,layout2", [("nk", "nk"), ("kn", "kn"), ("nk", "kn"), ("kn", "nk")])
-def test_split_products_match_fp32(M, N, K, K2, layout, layout2):
+def test_products_match_fp32_and_have_the_same_bits_in_every_kernel(M, N, K, K2, layout, layout2):
+    """The choice of a kernel by size must not show in a result: the k-blocks of a tile are added in one order everywhere."""
     from opaque_b200 import ops
     g = torch.Generator(device="cuda").manual_seed(M * 7 + N)
     r = lambda *s: torch.randn(*s, device="cuda", generator=g, dtype=torch.bfloat16)      # noqa: E731
@@ -28,43 +30,30 @@ def test_split_products_match_fp32(M, N, K, K2, layout, layout2):
     prod = a.float() @ w.float().t() + (a2.float() @ w2.float().t() if K2 else 0.0)
     b = w if layout == "nk" else w.t().contiguous()
     b2 = None if not K2 else (w2 if layout2 == "nk" else w2.t().contiguous())
+    kw = dict(b_layout=layout, a2=a2, b2=b2, b2_layout=layout2, bias=bias)
     st = ops.StatusWord()
-    nk = -(-K // 64) + -(-K2 // 64)
-    for splits in sorted({1, min(2, nk), min(3, nk), min(7, nk), min(24, nk), nk}):
-        for alpha, bb in ((1.0, None), (0.5, bias)):
-            kw = dict(b_layout=layout, a2=a2, b2=b2, b2_layout=layout2, bias=bb, kernel="single", splits=splits, alpha=alpha)
-            got = ops.gemm(a, b, status=st, **kw)
-            assert st.read() == 0 and _rel(got, alpha * prod + (0.0 if bb is None else bb.float())) < TOL, (splits, alpha)
-            assert torch.equal(got, ops.gemm(a, b, **kw))
-    auto = ops.gemm(a, b, b_layout=layout, a2=a2, b2=b2, b2_layout=layout2, bias=bias)
-    assert _rel(auto, prod + bias.float()) < TOL
+    ref = ops.gemm(a, b, kernel="single", block_n=256, status=st, **kw)
+    assert st.read() == 0 and _rel(ref, prod + bias.float()) < TOL
+    for choice in (dict(), dict(kernel="single"), dict(kernel="single", block_n=64), dict(kernel="pair")):
+        assert torch.equal(ops.gemm(a, b, **choice, **kw), ref), choice
+    assert torch.equal(ops.gemm_pair(a, b, tile="256x256", **kw), ref)
+    assert _rel(ops.gemm(a, b, alpha=0.5, **kw), 0.5 * prod + bias.float()) < TOL
 
 
-def test_split_products_write_inside_a_pitched_output_only():
+def test_products_write_inside_a_pitched_output_only():
     from opaque_b200 import ops
     a, w = torch.randn(130, 256, device="cuda", dtype=torch.bfloat16), torch.randn(72, 256, device="cuda", dtype=torch.bfloat16)
     for pitch in (80, 75):                               # rows for vector stores and rows that need scalar stores
         buf = torch.full((130, pitch), 7.0, device="cuda", dtype=torch.bfloat16)
-        ops.gemm(a, w, out=buf[:, :72], kernel="single", splits=4)
+        ops.gemm(a, w, out=buf[:, :72], kernel="single")
         assert _rel(buf[:, :72], a.float() @ w.float().t()) < TOL and bool((buf[:, 72:] == 7.0).all())
 
 
-def test_split_argument_errors():
+def test_scale_runs_on_the_single_cta_kernel():
     from opaque_b200 import ops
     a, w = torch.randn(64, 128, device="cuda", dtype=torch.bfloat16), torch.randn(64, 128, device="cuda", dtype=torch.bfloat16)
-    with pytest.raises(ops.KernelLibraryError):
-        ops.gemm(a, w, kernel="single", splits=3)        # two k-blocks
     with pytest.raises(ValueError):
         ops.gemm(a, w, kernel="pair", alpha=2.0)
-
-
-def test_small_products_are_split_and_large_ones_are_not():
-    from opaque_b200 import ops
-    for M, N, K in [(1, 768, 3072), (128, 768, 50304), (130, 48, 4096), (256, 2048, 8192)]:
-        kernel, splits = ops.pick_gemm_plan(M, N, K)
-        assert kernel == "single" and splits > 1
-    for M, N, K in [(16384, 4096, 4096), (16384, 2304, 768), (8192, 128256, 4096)]:
-        assert ops.pick_gemm_plan(M, N, K) == (ops.pick_gemm_kernel(M, N, K), 1)
 
 
 def test_lora_operands_packed_in_one_launch():
@@ -75,9 +64,8 @@ def test_lora_operands_packed_in_one_launch():
         assert torch.equal(a, torch.cat([x for x, _ in f])) and torch.equal(b, torch.block_diag(*[y for _, y in f]))
 
 
-@pytest.mark.parametrize("M,N,K,splits", [(1, 8, 8, 1), (128, 64, 64, 1), (130, 72, 1000, 1), (130, 72, 1000, 5), (257, 328, 136, 2), (64, 16, 2048, 8),
-                                          (20000, 56, 72, 1)])
-def test_narrow_tiles(M, N, K, splits):
+@pytest.mark.parametrize("M,N,K", [(1, 8, 8), (128, 64, 64), (130, 72, 1000), (257, 328, 136), (64, 16, 2048), (20000, 56, 72)])
+def test_narrow_tiles(M, N, K):
     from opaque_b200 import ops
     torch.manual_seed(M + N)
     a, bias = torch.randn(M, K, device="cuda", dtype=torch.bfloat16), torch.randn(N, device="cuda", dtype=torch.bfloat16)
@@ -87,7 +75,7 @@ def test_narrow_tiles(M, N, K, splits):
         b2 = torch.randn((N, 16) if layout2 == "nk" else (16, N), device="cuda", dtype=torch.bfloat16)
         prod = a.float() @ (w.float().t() if layout == "nk" else w.float()) + a2.float() @ (b2.float().t() if layout2 == "nk" else b2.float())
         buf = torch.full((M, N + 8), 7.0, device="cuda", dtype=torch.bfloat16)
-        kw = dict(b_layout=layout, a2=a2, b2=b2, b2_layout=layout2, bias=bias, alpha=0.5, kernel="single", splits=splits)
+        kw = dict(b_layout=layout, a2=a2, b2=b2, b2_layout=layout2, bias=bias, alpha=0.5, kernel="single")
         ops.gemm(a, w, out=buf[:, :N], block_n=64, **kw)
         assert _rel(buf[:, :N], 0.5 * prod + bias.float()) < TOL and bool((buf[:, N:] == 7.0).all())
         # a tile's k-blocks are added in the same order whatever its width
@@ -98,5 +86,5 @@ def test_narrow_tiles(M, N, K, splits):
 
 def test_tile_width_follows_the_number_of_narrow_tiles():
     from opaque_b200 import ops
-    assert ops.pick_tile_width(10 ** 6, 64, 2) == 64 and ops.pick_tile_width(128, 768, 12) == 64 and ops.pick_tile_width(128, 768, 48, 12) == 64
+    assert ops.pick_tile_width(10 ** 6, 64, 2) == 64 and ops.pick_tile_width(128, 768, 12) == 64
     assert ops.pick_tile_width(2048, 768, 12) == 256 and ops.pick_tile_width(16384, 3072, 12) == 256 and ops.pick_tile_width(128, 50304, 12) == 256
