@@ -54,6 +54,10 @@ from ..random import RngKey
 _ACTIVE: "Capture | None" = None
 CLIP_GUARD = 1.0 - 2.0 ** -8 - 2.0 ** -12
 LORA_PAD = 64
+# Norm-weight sums that wait for one launch (see Capture.add_row_sums): values of one operand, and bytes that wait in all.  At 4 Mi
+# values (4096 rows of 1024) a launch of its own has 4 column blocks x 4096 / 64 row splits: the chip is full.
+SUM_MATRIX_ELEMS = 4 << 20
+SUM_HELD_BYTES = 256 << 20
 
 
 def current_capture() -> "Capture | None":
@@ -105,6 +109,7 @@ class Capture:
         self.ghost_jobs: list[tuple] = []
         self.direct_jobs: list[tuple] = []
         self.sum_jobs: list[tuple] = []
+        self.sum_held = 0                  # bytes that only ``sum_jobs`` keeps alive
         self.status = engine.status
         self.direct_elems = sp.direct_elems
 
@@ -201,12 +206,23 @@ class Capture:
     def add_row_sums(self, out: torch.Tensor, g2d: torch.Tensor, x2d: torch.Tensor, mean: torch.Tensor | None, rstd: torch.Tensor,
                      out_plain: torch.Tensor | None) -> None:
         """Per-example weight (and bias) gradient of a norm layer.  Short matrices wait for the other layers' and share a launch;
-        long ones run at once: they fill the chip alone, and waiting would keep two activations per layer alive (16 MB a layer
-        at 4096 rows of 1024)."""
-        if g2d.shape[0] <= 4096 and g2d.shape[1] <= 8192 and x2d.stride(0) == g2d.stride(0) and (g2d.data_ptr() | x2d.data_ptr()) & 15 == 0:
+        long or wide ones run at once: they fill the chip alone.  Waiting keeps the layer's input and its gradient alive, which
+        nothing else needs any more: at most :data:`SUM_MATRIX_ELEMS` values each, :data:`SUM_HELD_BYTES` over all layers, and
+        what waits is launched when that is reached."""
+        held = 4 * g2d.numel()
+        if g2d.shape[0] <= 4096 and g2d.numel() <= SUM_MATRIX_ELEMS and x2d.stride(0) == g2d.stride(0) \
+                and (g2d.data_ptr() | x2d.data_ptr()) & 15 == 0:
+            if self.sum_held + held > SUM_HELD_BYTES:
+                self._launch_sums()
             self.sum_jobs.append((out, g2d, x2d, mean, rstd, out_plain))
+            self.sum_held += held
         else:
             ops.functional.rows_group_sum_(out, g2d, self.batch_size, x2d=x2d, mean=mean, rstd=rstd, out_plain=out_plain)
+
+    def _launch_sums(self) -> None:
+        for rows in {j[1].shape[0] for j in self.sum_jobs}:
+            ops.functional.rows_sum_batch_([j for j in self.sum_jobs if j[1].shape[0] == rows], self.batch_size)
+        self.sum_jobs, self.sum_held = [], 0
 
     def _tied_cross_term(self, slot_name: str) -> torch.Tensor | None:
         """``<g_embedding, g_head>`` per example for a weight used as input embedding AND output head.
@@ -263,9 +279,8 @@ class Capture:
             ops.ghost_norm_batch(self.ghost_jobs, status=self.status)
         if self.direct_jobs:
             ops.direct_norm2_batch(self.direct_jobs, self.tokens, status=self.status)
-        for rows in {j[1].shape[0] for j in self.sum_jobs}:
-            ops.functional.rows_sum_batch_([j for j in self.sum_jobs if j[1].shape[0] == rows], self.batch_size)
-        self.ghost_jobs, self.direct_jobs, self.sum_jobs = [], [], []
+        self._launch_sums()
+        self.ghost_jobs, self.direct_jobs = [], []
         by_slot: dict[str, list[int]] = {}
         for i, name in enumerate(self.part_slots):
             by_slot.setdefault(name, []).append(i)
