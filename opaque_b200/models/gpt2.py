@@ -13,6 +13,7 @@ import dataclasses
 
 import torch
 from torch import nn
+from torch.nn.modules.module import _has_any_global_hook
 
 from .. import ops
 from ..functional import functional_checkpoint
@@ -95,6 +96,9 @@ class GPT2Block(nn.Module):
         return self.attn_c_proj(o.transpose(1, 2).reshape(B, T, d))
 
 
+_BLOCK_FORWARD, _NORM_FORWARD = GPT2Block.forward, LayerNorm.forward
+
+
 class GPT2LMHeadModel(nn.Module):
     def __init__(self, cfg: GPT2Config, *, dtype=torch.bfloat16, device=None):
         super().__init__()
@@ -106,12 +110,15 @@ class GPT2LMHeadModel(nn.Module):
         self.activation_checkpointing = False      # set by the trainer's gradient_checkpointing
 
     def _carries(self) -> bool:
-        """Whether the blocks may run on the split stream: blocks and norms of these very classes, with no hooks that expect to be
-        called with the unsplit tensors."""
+        """Whether the blocks may run on the split stream, which calls neither a block's nor most norms' ``forward``: blocks and norms of
+        these very classes with their own ``forward`` (none assigned to an instance or patched into the class, none compiled), and no
+        hooks, on them or on all modules, that expect to be called with the unsplit tensors."""
+        if _has_any_global_hook() or GPT2Block.forward is not _BLOCK_FORWARD or LayerNorm.forward is not _NORM_FORWARD:
+            return False
         norms = [n for blk in self.h if type(blk) is GPT2Block for n in (blk.ln_1, blk.ln_2)] + [self.ln_f]
         return (all(type(blk) is GPT2Block for blk in self.h) and all(type(n) is LayerNorm for n in norms)
                 and not any(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks
-                            for m in (*self.h, *norms)))
+                            or "forward" in m.__dict__ or m._compiled_call_impl is not None for m in (*self.h, *norms)))
 
     def hidden_states(self, input_ids):
         B, T = input_ids.shape

@@ -123,3 +123,35 @@ def test_moe_dense_reference_form_matches_the_sorted_form():
     assert torch.allclose(dense.detach(), sorted_loss, atol=1e-5)
     for n, g in sorted_grads.items():
         assert torch.allclose(dict(m.named_parameters())[n].grad, g, atol=1e-5, rtol=1e-4), n
+
+
+def test_gpt2_split_stream_gives_way_to_hooks_and_replaced_forwards(monkeypatch):
+    """The split stream passes by the blocks' and norms' ``forward``: whoever hooks or replaces one gets the plain stream."""
+    from opaque_b200.models import GPT2Config, GPT2LMHeadModel
+    from opaque_b200.models.gpt2 import GPT2Block
+    from opaque_b200.models.layers import LayerNorm
+
+    def fresh():
+        return GPT2LMHeadModel(GPT2Config.tiny())
+    assert fresh()._carries()
+    handles = [torch.nn.modules.module.register_module_forward_hook(lambda *a: None),
+               torch.nn.modules.module.register_module_forward_pre_hook(lambda *a: None),
+               torch.nn.modules.module.register_module_full_backward_hook(lambda *a: None)]
+    for h in handles:
+        assert not fresh()._carries()
+        h.remove()
+    for pick in (lambda m: m.h[1], lambda m: m.h[0].ln_2, lambda m: m.ln_f):
+        m = fresh()
+        pick(m).forward = pick(m).forward
+        assert not m._carries()
+        m = fresh()
+        pick(m).register_forward_pre_hook(lambda *a: None)
+        assert not m._carries()
+    m = fresh()
+    m.h[0].compile()
+    assert not m._carries()
+    for cls in (GPT2Block, LayerNorm):
+        with monkeypatch.context() as mp:
+            mp.setattr(cls, "forward", lambda self, x: x)
+            assert not fresh()._carries()
+    assert fresh()._carries()
