@@ -156,7 +156,7 @@ class _Experts(Function):
         batch, tokens, wshape = ctx.meta
         I = w2.shape[2]
         if ctx.rows:
-            dy, dw = ops.functional.moe_row_grad(dout.contiguous(), y, wrow, token_sorted, slot_sorted)
+            dy, dw = ops.functional.moe_row_grad(ops.functional._vec16(dout), y, wrow, token_sorted, slot_sorted)
             dtopk = dw.view(wshape)
             dact = grouped_linear(dy, w2, offs, transposed=True)
             dh = ops.functional.glu_backward_packed(dact, h)

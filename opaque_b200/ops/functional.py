@@ -48,6 +48,14 @@ def _use_kernel(*ts: torch.Tensor) -> bool:
     return _PLAIN == 0 and all(t.is_cuda and t.dtype == torch.bfloat16 for t in ts)
 
 
+def _vec16(t: torch.Tensor) -> torch.Tensor:
+    """``t`` contiguous and on a 16-byte boundary, as the kernels' vector accesses need it: a contiguous view may start anywhere in
+    its storage, and an access that is not aligned faults."""
+    if t.is_contiguous():
+        return t if t.data_ptr() & 15 == 0 else t.clone(memory_format=torch.contiguous_format)
+    return t.contiguous()
+
+
 def _param_grad_hook():
     """The fused DP engine's capture callback for small per-example parameter gradients, if active."""
     from ..engine import fused
@@ -74,11 +82,11 @@ class _RMSNorm(Function):
         shape = x.shape
         H = shape[-1]
         x2 = x.reshape(-1, H)
-        x2 = x2 if x2.is_contiguous() else x2.contiguous()
+        x2 = _vec16(x2)
         r2 = None
         if residual is not None:
             r2 = residual.reshape(-1, H)
-            r2 = r2 if r2.is_contiguous() else r2.contiguous()
+            r2 = _vec16(r2)
         rows = x2.shape[0]
         y = torch.empty_like(x2)
         s = torch.empty_like(x2) if r2 is not None else None
@@ -98,11 +106,11 @@ class _RMSNorm(Function):
         shape, offset, layer, fused_add = ctx.meta
         H = shape[-1]
         dy2 = dy.reshape(-1, H)
-        dy2 = dy2 if dy2.is_contiguous() else dy2.contiguous()
+        dy2 = _vec16(dy2)
         ds2 = None
         if ds is not None:
             ds2 = ds.reshape(-1, H)
-            ds2 = ds2 if ds2.is_contiguous() else ds2.contiguous()
+            ds2 = _vec16(ds2)
         rows = xs.shape[0]
         dx = torch.empty_like(xs)
         cap = _param_grad_hook() if weight.requires_grad else None
@@ -229,7 +237,7 @@ class _LayerNorm(Function):
         shape = x.shape
         H = shape[-1]
         x2 = x.reshape(-1, H)
-        x2 = x2 if x2.is_contiguous() else x2.contiguous()
+        x2 = _vec16(x2)
         rows = x2.shape[0]
         y = torch.empty_like(x2)
         stats = torch.empty(2, rows, dtype=torch.float32, device=x.device)
@@ -246,7 +254,7 @@ class _LayerNorm(Function):
         shape, layer, has_bias = ctx.meta
         H = shape[-1]
         dy2 = dy.reshape(-1, H)
-        dy2 = dy2 if dy2.is_contiguous() else dy2.contiguous()
+        dy2 = _vec16(dy2)
         rows = x2.shape[0]
         dx = torch.empty_like(x2)
         rc = lib.load().ob_layernorm_bwd_dx(dy2.data_ptr(), x2.data_ptr(), weight.data_ptr(), stats[0].data_ptr(),
@@ -270,8 +278,8 @@ class _AddLayerNorm(Function):
     def forward(ctx, x, residual, weight, bias, eps, layer):
         shape, H = x.shape, x.shape[-1]
         x2, r2 = x.reshape(-1, H), residual.reshape(-1, H)
-        x2 = x2 if x2.is_contiguous() else x2.contiguous()
-        r2 = r2 if r2.is_contiguous() else r2.contiguous()
+        x2 = _vec16(x2)
+        r2 = _vec16(r2)
         rows = x2.shape[0]
         y, s = torch.empty_like(x2), torch.empty_like(x2)
         stats = torch.empty(2, rows, dtype=torch.float32, device=x.device)
@@ -291,14 +299,14 @@ class _AddLayerNorm(Function):
         if dy is None:                                   # only the sum is used
             return ds, ds, None, None, None, None
         dy2 = dy.reshape(-1, H)
-        dy2 = dy2 if dy2.is_contiguous() else dy2.contiguous()
+        dy2 = _vec16(dy2)
         dx = torch.empty_like(s)
         mean, rstd = stats.data_ptr(), stats.data_ptr() + 4 * rows
         if ds is None:                                   # nothing passes by the norm (the last one of a model)
             rc = lib.load().ob_layernorm_bwd_dx(dy2.data_ptr(), s.data_ptr(), weight.data_ptr(), mean, rstd, dx.data_ptr(), rows, H, lib.stream())
         else:
             ds2 = ds.reshape(-1, H)
-            ds2 = ds2 if ds2.is_contiguous() else ds2.contiguous()
+            ds2 = _vec16(ds2)
             rc = lib.load().ob_add_layernorm_bwd_dx(dy2.data_ptr(), s.data_ptr(), weight.data_ptr(), mean, rstd, ds2.data_ptr(), dx.data_ptr(),
                                                     rows, H, lib.stream())
         lib.check(rc, "add_layernorm_bwd_dx")
@@ -324,7 +332,7 @@ _ACTS = {"silu": 0, "gelu": 1, "gelu_tanh": 2, "relu": 3}
 class _Activation(Function):
     @staticmethod
     def forward(ctx, x, act):
-        xc = x if x.is_contiguous() else x.contiguous()
+        xc = _vec16(x)
         out = torch.empty_like(xc)
         rc = lib.load().ob_activation(xc.data_ptr(), None, out.data_ptr(), xc.numel(), act, lib.sm_count(), lib.stream())
         lib.check(rc, "activation")
@@ -335,7 +343,7 @@ class _Activation(Function):
     @staticmethod
     def backward(ctx, dy):
         (xc,) = ctx.saved_tensors
-        dyc = dy if dy.is_contiguous() else dy.contiguous()
+        dyc = _vec16(dy)
         dx = torch.empty_like(xc)
         rc = lib.load().ob_activation(xc.data_ptr(), dyc.data_ptr(), dx.data_ptr(), xc.numel(), ctx.act, lib.sm_count(),
                                       lib.stream())
@@ -392,7 +400,7 @@ class _GLU(Function):
         shape, act = ctx.meta
         I = shape[-1]
         d2 = dh.reshape(-1, I)
-        d2 = d2 if d2.is_contiguous() else d2.contiguous()
+        d2 = _vec16(d2)
         both = torch.empty(g2.shape[0], 2 * I, dtype=g2.dtype, device=g2.device)
         dg, du = both[:, :I], both[:, I:]
         rc = lib.load().ob_glu_bwd(d2.data_ptr(), g2.data_ptr(), u2.data_ptr(), dg.data_ptr(), du.data_ptr(),

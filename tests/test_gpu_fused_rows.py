@@ -52,6 +52,25 @@ def test_add_layer_norm_has_the_bits_of_the_separate_operations(rows, H):
     assert torch.equal(xf.grad, s2.grad + gs) and torch.equal(rf.grad, xf.grad)
 
 
+def test_norms_and_activations_of_views_that_start_anywhere():
+    """Contiguous views off the 16-byte boundary give what their aligned copies give, in both directions."""
+    from opaque_b200 import ops
+    off = lambda t: torch.cat([t.new_zeros(1), t.flatten()])[1:].view(t.shape)            # noqa: E731
+    x, res, gy, gs = (torch.randn(5, 64, device="cuda", dtype=torch.bfloat16) for _ in range(4))
+    w, b = (torch.randn(64, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    assert off(x).is_contiguous() and off(x).data_ptr() % 16 == 2
+    for fn, grads in ((lambda p, q: ops.add_layer_norm(p, q, w, b), 2), (lambda p, q: ops.fused_add_rms_norm(p, q, w), 2),
+                      (lambda p, q: (ops.layer_norm(p + q, w, b),), 1), (lambda p, q: (ops.layer_norm(p, w, b),), 1),
+                      (lambda p, q: (ops.rms_norm(p, w),), 1), (lambda p, q: (ops.activation(p, "silu"),), 1)):
+        out = []
+        for shift in (lambda t: t, off):
+            p, q = shift(x).detach().requires_grad_(True), shift(res).detach().requires_grad_(True)
+            ys = fn(p, q)
+            torch.autograd.backward(list(ys), [shift(g) for g in (gy, gs)[:grads]])
+            out.append((*ys, p.grad))
+        assert all(torch.equal(u, v) for u, v in zip(*out))
+
+
 @pytest.mark.parametrize("count", [1, 3, 130])
 @pytest.mark.parametrize("B,T", [(1, 1), (3, 70), (2, 513)])
 def test_bias_sums_batched(count, B, T):

@@ -35,6 +35,25 @@ def test_combine_and_row_gradients(T, k, H):
         F.moe_combine(y, pos[:-1], k, w)
 
 
+def test_experts_take_gradients_that_start_anywhere():
+    """The gradient of an output that was flattened into a longer vector starts off the 16-byte boundary."""
+    from opaque_b200.models import MoEConfig, MoEForCausalLM
+    cfg = MoEConfig.tiny()
+    torch.manual_seed(0)
+    experts = MoEForCausalLM(cfg, device="cuda").layers[0].mlp.experts
+    T, k, H = 18, cfg.num_experts_per_tok, cfg.hidden_size
+    x, up = (torch.randn(T, H, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    idx = torch.stack([torch.randperm(cfg.num_experts, device="cuda")[:k] for _ in range(T)])
+    w = torch.rand(T, k, device="cuda").to(torch.bfloat16)
+    grads = []
+    for shift in (0, 1):
+        xi = x.clone().requires_grad_(True)
+        y = experts(xi, idx, w, 2, 9)
+        torch.cat([y.new_zeros(shift), y.flatten()]).backward(torch.cat([up.new_zeros(shift), up.flatten()]))
+        grads.append(xi.grad)
+    assert torch.equal(*grads)
+
+
 def test_packed_gated_backward():
     from opaque_b200.ops import functional as F
     for rows, I in ((1, 8), (37, 136)):

@@ -155,3 +155,13 @@ def test_gpt2_split_stream_gives_way_to_hooks_and_replaced_forwards(monkeypatch)
             mp.setattr(cls, "forward", lambda self, x: x)
             assert not fresh()._carries()
     assert fresh()._carries()
+
+
+def test_kernel_operands_are_contiguous_and_aligned():
+    from opaque_b200.ops.functional import _vec16
+    t = torch.randn(4, 8).to(torch.bfloat16)
+    flat = torch.randn(40).to(torch.bfloat16)
+    assert _vec16(t) is t
+    for view in (t.t(), t[:, 1:], flat[1:33].view(4, 8), flat[3:35].view(8, 4)):
+        v = _vec16(view)
+        assert v.is_contiguous() and v.data_ptr() % 16 == 0 and torch.equal(v, view)
