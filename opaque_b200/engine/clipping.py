@@ -229,8 +229,9 @@ def _tree_kernel_ok(leaves: Sequence[Any], dtype: torch.dtype | None, compute_dt
     if not 0 < len(leaves) <= ops.CLIP_TREE_MAX_LEAVES or dtype not in (None, torch.float32) or compute_dtype not in (None, torch.float32):
         return False
     wrapped = torch._C._functorch.is_functorch_wrapped_tensor
-    if not all(type(x) is torch.Tensor and x.is_cuda and x.dtype == torch.float32 and not wrapped(x) and x.ndim > 0
-               for x in leaves):
+    # (a view with the negation bit reads negated through tensor operations only)
+    if not all(type(x) is torch.Tensor and x.is_cuda and x.dtype == torch.float32 and x.layout is torch.strided and not x.is_neg()
+               and not wrapped(x) and x.ndim > 0 for x in leaves):
         return False
     x0 = leaves[0]
     if any(x.device != x0.device or x.shape[0] != x0.shape[0] or (torch.is_grad_enabled() and x.requires_grad) for x in leaves):

@@ -71,4 +71,15 @@ def test_what_the_kernels_do_not_take_keeps_the_tensor_path():
     assert not C._tree_kernel_ok([ok], torch.float64, None) and not C._tree_kernel_ok([ok], None, torch.float64)
     assert not C._tree_kernel_ok([ok, 3.0], None, None) and not C._tree_kernel_ok([ok] * 65, None, None) and not C._tree_kernel_ok([], None, None)
     assert not C._tree_kernel_ok([ok[:0]], None, None) and not C._tree_kernel_ok([ok.clone().requires_grad_(True)], None, None)
+    assert not C._tree_kernel_ok([torch._neg_view(ok)], None, None) and not C._tree_kernel_ok([ok.to_sparse()], None, None)
     torch.func.vmap(lambda t: (C._tree_kernel_ok([t], None, None), t)[1] if not C._tree_kernel_ok([t], None, None) else 1 / 0)(ok)
+
+
+@pytest.mark.parametrize("E", [1, 5])                 # one record's view is contiguous as it stands
+def test_negated_views_are_clipped_as_they_read(E):
+    from opaque_b200.dpsgd.clipping import clipped_fun
+    x, c = torch.randn(E, 3, device="cuda"), torch._neg_view(torch.ones(4, device="cuda"))
+    fn, st = clipped_fun(lambda a: {"a": 2 * a, "c": c}, clipping_norm=1e3)
+    got, _ = fn(x, state=st)
+    assert torch.allclose(got.pytree["c"], torch.full_like(x[0, :1], -E).expand(4), rtol=1e-5)
+    assert torch.allclose(got.pytree["a"], 2 * x.sum(0), rtol=1e-5, atol=1e-5)
