@@ -6,6 +6,7 @@ build is skipped when the artefact is newer than every source; ``force=True`` re
 from __future__ import annotations
 
 import contextlib
+import hashlib
 import os
 import shutil
 import subprocess
@@ -173,13 +174,14 @@ static int to_float(PyObject* o, float* v) { double x; if (to_double(o, &x)) ret
 
 
 def build_launcher(signatures: dict[str, str], force: bool = False) -> Path:
-    """Compile :func:`launcher_source` in-tree; rebuilt when the signatures change."""
+    """Compile :func:`launcher_source` in-tree.  The extension carries a digest of its source, so an installed copy is fresh
+    without any other file; it is rebuilt when the signatures change."""
     target = launcher_ext_path()
     source = launcher_source(signatures)
-    src_path = OBJ_DIR / "_launch.c"
+    mark = "opaque-launch:" + hashlib.sha256(source.encode()).hexdigest()
 
     def fresh() -> bool:
-        return target.exists() and src_path.exists() and src_path.read_text() == source
+        return target.exists() and mark.encode() in target.read_bytes()
     if not force and fresh():
         return target
     gcc = _find("gcc", ["/usr/bin/gcc"])
@@ -188,17 +190,17 @@ def build_launcher(signatures: dict[str, str], force: bool = False) -> Path:
     with _build_lock(target):
         if not force and fresh():
             return target
-        OBJ_DIR.mkdir(exist_ok=True)
-        tmp, tmp_src = target.with_suffix(f".tmp{os.getpid()}"), OBJ_DIR / f"_launch{os.getpid()}.c"
-        tmp_src.write_text(source)
-        res = subprocess.run([gcc, "-O2", "-shared", "-fPIC", "-fvisibility=hidden", f"-I{sysconfig.get_paths()['include']}", str(tmp_src),
-                              "-o", str(tmp)], capture_output=True, text=True)
-        if res.returncode != 0:
+        tmp, tmp_src = target.with_suffix(f".tmp{os.getpid()}"), target.with_suffix(f".tmp{os.getpid()}.c")
+        try:
+            tmp_src.write_text(source + f'__attribute__((used)) static const char digest[] = "{mark}";\n')
+            res = subprocess.run([gcc, "-O2", "-shared", "-fPIC", "-fvisibility=hidden", f"-I{sysconfig.get_paths()['include']}", str(tmp_src),
+                                  "-o", str(tmp)], capture_output=True, text=True)
+            if res.returncode != 0:
+                raise RuntimeError("gcc failed:\n" + res.stdout + res.stderr)
+            os.replace(tmp, target)
+        finally:
             tmp.unlink(missing_ok=True)
             tmp_src.unlink(missing_ok=True)
-            raise RuntimeError("gcc failed:\n" + res.stdout + res.stderr)
-        os.replace(tmp, target)
-        os.replace(tmp_src, src_path)
     return target
 
 

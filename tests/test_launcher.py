@@ -63,3 +63,14 @@ def test_every_launching_entry_point_goes_through_it():
         assert len(sig) == len(lib._SIGNATURES[name]) and type(getattr(entries, name)).__name__ == "builtin_function_or_method"
     # an empty problem returns before anything touches a device
     assert entries.ob_gemm_tn(*[{"P": None, "F": 1.0, "D": 1.0}.get(c, 0) for c in sigs["ob_gemm_tn"]]) == 0
+
+
+def test_an_installed_extension_needs_no_other_file_and_no_compiler(tmp_path, monkeypatch):
+    monkeypatch.setattr(build, "launcher_ext_path", lambda: tmp_path / "_launch.so")
+    path = build.build_launcher({"ob_a": "PI"})
+    assert {f.name for f in tmp_path.iterdir() if f.suffix != ".lock"} == {"_launch.so"}
+    monkeypatch.setattr(build, "OBJ_DIR", tmp_path / "nowhere")
+    monkeypatch.setattr(build, "_find", lambda *a: None)
+    assert build.build_launcher({"ob_a": "PI"}) == path
+    with pytest.raises(RuntimeError):
+        build.build_launcher({"ob_a": "PL"})                      # other signatures: not fresh
