@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import ctypes
 import functools
+import warnings
 from ctypes import c_char_p, c_double, c_float, c_int, c_longlong, c_uint, c_ulonglong, c_void_p
 
 import torch
@@ -101,6 +102,22 @@ class KernelLibraryError(RuntimeError):
     pass
 
 
+def _load_launcher(signatures: dict[str, str]):
+    """The compiled caller, or ``None`` (with a warning: every call stays with ctypes) where it can neither be built nor loaded."""
+    import importlib.util
+    for force in (False, True):                 # an extension that does not load (another machine's, damaged) is built afresh
+        try:
+            path = _build.build_launcher(signatures, force)
+            spec = importlib.util.spec_from_file_location("opaque_b200.ops._launch", path)
+            launch = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(launch)
+            return launch
+        except (RuntimeError, OSError, ImportError) as exc:
+            reason = exc
+    warnings.warn(f"no compiled caller, launches go through ctypes at 3 us more each: {reason}", RuntimeWarning, stacklevel=3)
+    return None
+
+
 @functools.lru_cache(maxsize=None)
 def load() -> _Entries:
     """The entry points of the kernel library (built on demand, loaded once)."""
@@ -122,14 +139,9 @@ def load() -> _Entries:
     lib.ob_debug_idesc_bf16.restype = c_uint
     entries = _Entries(lib)
     signatures = launch_signatures()
-    try:
-        path = _build.build_launcher(signatures)
-    except (RuntimeError, OSError):                               # no C compiler, nowhere to write: every call stays with ctypes
+    launch = _load_launcher(signatures)
+    if launch is None:
         return entries
-    import importlib.util
-    spec = importlib.util.spec_from_file_location("opaque_b200.ops._launch", path)
-    launch = importlib.util.module_from_spec(spec)
-    spec.loader.exec_module(launch)
     for name in signatures:
         launch.bind(name, ctypes.cast(getattr(lib, name), c_void_p).value)
         setattr(entries, name, getattr(launch, name))

@@ -74,3 +74,19 @@ def test_an_installed_extension_needs_no_other_file_and_no_compiler(tmp_path, mo
     assert build.build_launcher({"ob_a": "PI"}) == path
     with pytest.raises(RuntimeError):
         build.build_launcher({"ob_a": "PL"})                      # other signatures: not fresh
+
+
+def test_an_extension_that_does_not_load_is_built_afresh(tmp_path, monkeypatch):
+    monkeypatch.setattr(build, "launcher_ext_path", lambda: tmp_path / "_launch.so")
+    path = build.build_launcher({"ob_a": "PI"})
+
+    def damage():
+        data = path.read_bytes()
+        path.unlink()                                             # a loaded library's file is not written over
+        path.write_bytes(b"not a library " + data)                # carries the digest all the same
+    damage()
+    assert lib._load_launcher({"ob_a": "PI"}).ob_a.__name__ == "ob_a"
+    damage()
+    monkeypatch.setattr(build, "_find", lambda *a: None)
+    with pytest.warns(RuntimeWarning, match="ctypes"):
+        assert lib._load_launcher({"ob_a": "PI"}) is None
