@@ -77,16 +77,14 @@ def test_an_installed_extension_needs_no_other_file_and_no_compiler(tmp_path, mo
 
 
 def test_an_extension_that_does_not_load_is_built_afresh(tmp_path, monkeypatch):
-    monkeypatch.setattr(build, "launcher_ext_path", lambda: tmp_path / "_launch.so")
-    path = build.build_launcher({"ob_a": "PI"})
-
-    def damage():
-        data = path.read_bytes()
-        path.unlink()                                             # a loaded library's file is not written over
+    def damaged(name):
+        path = tmp_path / name
+        monkeypatch.setattr(build, "launcher_ext_path", lambda: path)
+        data = build.build_launcher({"ob_a": "PI"}).read_bytes()
         path.write_bytes(b"not a library " + data)                # carries the digest all the same
-    damage()
+    damaged("_launch.so")
     assert lib._load_launcher({"ob_a": "PI"}).ob_a.__name__ == "ob_a"
-    damage()
+    damaged("_launch_2.so")
     monkeypatch.setattr(build, "_find", lambda *a: None)
     with pytest.warns(RuntimeWarning, match="ctypes"):
         assert lib._load_launcher({"ob_a": "PI"}) is None
