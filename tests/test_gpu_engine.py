@@ -108,6 +108,63 @@ def test_gpt2_full_parameter():
     _check(GPT2LMHeadModel(GPT2Config.tiny(), device=dev), 500, 1.0, 1.0, 5e-3, 2e-2)
 
 
+@pytest.mark.parametrize("kw,taken,not_taken", [
+    # weight gradients: the per-example kernel up to a tenth of zero rows, the ragged one beyond and for short records
+    (dict(tokens=65), "wgrad_clip_batch", "wgrad_clip_per_example_batch"),
+    (dict(tokens=130), "wgrad_clip_batch", "wgrad_clip_per_example_batch"),
+    (dict(tokens=250), "wgrad_clip_per_example_batch", "wgrad_clip_batch"),
+    (dict(tokens=333), "wgrad_clip_batch", "wgrad_clip_per_example_batch"),
+    # norm-weight sums of more than 4096 rows run at once
+    (dict(tokens=1000, microbatch=6), "rows_group_sum_", "wgrad_clip_batch"),
+    # few records on a wide head: its norm from the product itself, at any length
+    (dict(tokens=37, records=3, vocab=16500), "direct_norm2_batch", "rows_group_sum_"),
+    (dict(tokens=199, records=2, vocab=16500), "direct_norm2_batch", "rows_group_sum_"),
+    (dict(tokens=70, records=2), "ghost_norm_batch", "direct_norm2_batch"),
+    # more layers than one launch holds: 56 norms or weight gradients, 128 sums
+    (dict(tokens=70, layers=32, width=192), "wgrad_clip_batch", "wgrad_clip_per_example_batch"),
+    (dict(tokens=128, layers=32, width=192), "wgrad_clip_per_example_batch", "wgrad_clip_batch"),
+])
+def test_gpt2_every_branch_of_the_capture(monkeypatch, kw, taken, not_taken):
+    from opaque_b200 import ops
+    from opaque_b200.models import GPT2Config, GPT2LMHeadModel
+    kw = dict(kw)
+    calls = set()
+    for mod, names in ((ops, ("wgrad_clip_batch", "wgrad_clip_per_example_batch", "direct_norm2_batch", "ghost_norm_batch")),
+                       (ops.functional, ("rows_group_sum_",))):
+        for name in names:
+            def spy(*a, _fn=getattr(mod, name), _name=name, **k):
+                calls.add(_name)
+                return _fn(*a, **k)
+            monkeypatch.setattr(mod, name, spy)
+    width = kw.pop("width", 256)              # layers of more than 128 inputs share the launches
+    cfg = GPT2Config(vocab_size=kw.pop("vocab", 500), n_positions=1024, n_embd=width, n_layer=kw.pop("layers", 2), n_head=4)
+    torch.manual_seed(2)
+    model = GPT2LMHeadModel(cfg, device=torch.device("cuda", 0))
+    _check_capture(model, cfg.vocab_size, calls, **kw)
+    assert taken in calls and not_taken not in calls, calls
+
+
+def _check_capture(model, vocab, calls, *, records=6, tokens, microbatch=4):
+    """Norms and clipped sums of one pass against the per-example loop; ``calls`` is emptied before the pass."""
+    from opaque_b200.engine.fused import CLIP_GUARD, FusedDPEngine
+    from opaque_b200.models import shift_labels
+    from opaque_b200.random import key
+    ids = torch.randint(0, vocab, (records, tokens), device="cuda")
+    labels = shift_labels(ids, 1.0)
+    total, norms = _oracle(model, ids, labels, 0.3, CLIP_GUARD)
+    assert float(norms.min()) > 0.3                                # every record is clipped
+    eng = FusedDPEngine(model, clipping_norm=0.3, noise_multiplier=0.0, normalize_by=1.0, key=key(0), microbatch_size=microbatch)
+    calls.clear()
+    res = eng.accumulate(model.per_example_loss, {"input_ids": ids, "labels": labels})
+    # With random weights the gradient of every row's target logit is nearly the same number, w (p - 1) with p = 1 / vocabulary, so
+    # its roundings to bf16 (one here, two in the loop: p - 1, then its product with w) shift a whole gradient: 3 * 2^-9
+    assert eng.status.read() == 0 and float(((res.norms - norms).abs() / norms).max()) < 6e-3
+    flat = eng.space.grad.local
+    for n, g in total.items():
+        s = eng.space.slots[n]
+        assert float((flat[s.offset:s.offset + s.numel].view(s.shape) - g).norm() / (g.norm() + 1e-12)) < 2e-2, n
+
+
 def test_moe_full_parameter_ragged_ghost_and_grouped_wgrad():
     from opaque_b200.models import MoEConfig, MoEForCausalLM
     dev = torch.device("cuda", 0)
