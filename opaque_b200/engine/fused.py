@@ -324,10 +324,10 @@ class Capture:
                               out_offset=slot.offset, ldm=d_in, group_stride=d_out * d_in)
                 elif kind == "linear":
                     # uniform examples: factor applied per example in the epilogue, operands untouched.  That kernel runs at
-                    # 1.07 - 1.25 PFLOP/s against 0.91 - 1.06 of the ragged one, which pays for a tenth of zero rows: 24 products of
-                    # about 4,000 rows take 356 and 318 us at 1,000 rows per example, 326 and 311 at 520 (1.11 with the zero
-                    # rows), 347 and 354 at 333 (1.15), 347 and 441 at 130 (1.48)
-                    if self.tokens >= 128 and -(-self.tokens // 64) * 64 <= 1.1 * self.tokens and g2d.shape[0] == self.batch_size * self.tokens:
+                    # 1.07 - 1.25 PFLOP/s against 0.91 - 1.06 of the ragged one, which pays for a ninth of zero rows: 24 products of
+                    # about 4,000 rows take (ragged, uniform) 356 and 318 us at 1,000 rows per example, 326 and 311 at 520 (1.108
+                    # with the zero rows), 347 and 354 at 333 (1.153), 347 and 441 at 130 (1.48)
+                    if self.tokens >= 128 and -(-self.tokens // 64) * 64 <= 1.11 * self.tokens and g2d.shape[0] == self.batch_size * self.tokens:
                         uniform.append((g2d, other, scales[g], slot.offset, slot.shape[1]))
                         continue
                     pr = dict(a=g2d, b=other, row_scale=row_scale[g], out_offset=slot.offset, ldm=slot.shape[1])

@@ -109,11 +109,12 @@ def test_gpt2_full_parameter():
 
 
 @pytest.mark.parametrize("kw,taken,not_taken", [
-    # weight gradients: the per-example kernel up to a tenth of zero rows, the ragged one beyond and for short records
+    # weight gradients: the per-example kernel up to a ninth of zero rows, the ragged one beyond and for short records
     (dict(tokens=65), "wgrad_clip_batch", "wgrad_clip_per_example_batch"),
     (dict(tokens=130), "wgrad_clip_batch", "wgrad_clip_per_example_batch"),
     (dict(tokens=250), "wgrad_clip_per_example_batch", "wgrad_clip_batch"),
     (dict(tokens=333), "wgrad_clip_batch", "wgrad_clip_per_example_batch"),
+    (dict(tokens=520), "wgrad_clip_per_example_batch", "wgrad_clip_batch"),
     # norm-weight sums of more than 4096 rows run at once
     (dict(tokens=1000, microbatch=6), "rows_group_sum_", "wgrad_clip_batch"),
     # few records on a wide head: its norm from the product itself, at any length
