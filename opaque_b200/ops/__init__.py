@@ -184,8 +184,9 @@ def direct_norm2(a: torch.Tensor, g: torch.Tensor, norm2: torch.Tensor, rows_per
     if splits is None:
         tiles = math.ceil(M / 128) * math.ceil(N / 256)
         splits = pick_splits(tiles, T, sms, max_splits=B)
-    rc = lib.load().ob_direct_norm2(a.data_ptr(), g.data_ptr(), B, rows_per_example, M, N, a.stride(0), g.stride(0), splits,
-                                    norm2.data_ptr(), status.ptr() if status else None, wait_budget_s, sms, lib.stream())
+    desc = _WGRAD_PE_DESC.pack(a.data_ptr(), g.data_ptr(), 0, norm2.data_ptr(), a.stride(0), g.stride(0), 0, N, B, rows_per_example, M, N,
+                               splits, 0)
+    rc = lib.load().ob_wgrad_clip_pe_batch(desc, 1, None, None, 0, status.ptr() if status else None, wait_budget_s, sms, lib.stream())
     lib.check(rc, "direct_norm2")
     return norm2
 
@@ -245,10 +246,10 @@ def wgrad_clip_per_example(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor |
             raise ValueError(f"wgrad_clip_per_example would write element {hi} of a destination holding {room}")
     elif peer_table is None or shard_elems <= 0:
         raise ValueError("give either a destination tensor or a peer table with shard_elems")
-    rc = lib.load().ob_wgrad_clip_pe(a.data_ptr(), b.data_ptr(), B, rows_per_example, M, N, a.stride(0), b.stride(0),
-                                     lib.ptr(ex_scale), splits, lib.ptr(out), lib.ptr(peer_table), shard_elems, out_offset,
-                                     ldm, int(accumulate), status.ptr() if status else None, wait_budget_s, sms,
-                                     lib.stream())
+    desc = _WGRAD_PE_DESC.pack(a.data_ptr(), b.data_ptr(), lib.ptr(ex_scale) or 0, 0, a.stride(0), b.stride(0), out_offset, ldm, B,
+                               rows_per_example, M, N, splits, int(accumulate))
+    rc = lib.load().ob_wgrad_clip_pe_batch(desc, 1, lib.ptr(out), lib.ptr(peer_table), shard_elems, status.ptr() if status else None,
+                                           wait_budget_s, sms, lib.stream())
     lib.check(rc, "wgrad_clip_per_example")
 
 
@@ -370,11 +371,7 @@ def ghost_norm(a: torch.Tensor | None, g: torch.Tensor, norm2: torch.Tensor, tok
     accumulator each segment adds to (e.g. the example an (expert, example) group belongs to).
     With ``ids`` (int32, one per row) the inputs are one-hot rows (embedding layer) and ``a`` is unused.
     """
-    rows, B, da, dg, lda, ap = _check_ghost(a, g, norm2, tokens_per_example, ids, seg_offsets, seg_out)
-    rc = lib.load().ob_ghost_norm(ap, g.data_ptr(), lib.ptr(ids), B, tokens_per_example, da, dg, lda, g.stride(0),
-                                  norm2.data_ptr(), lib.ptr(seg_offsets), lib.ptr(seg_out), rows,
-                                  status.ptr() if status else None, wait_budget_s, lib.sm_count(), lib.stream())
-    lib.check(rc, "ghost_norm")
+    ghost_norm_batch([(a, g, norm2, tokens_per_example, ids, seg_offsets, seg_out)], status=status, wait_budget_s=wait_budget_s)
 
 
 PAIR_GEMM = True          # dense (ungrouped) products run on CTA pairs (256 x 256 tiles, tcgen05 cta_group::2)

@@ -11,23 +11,14 @@ int ob_wgrad_clip(const void* a, const void* b, int T, int M, int N, long long l
                   long long group_stride, long long out_offset, long long ldm, long long ldn, int n_valid,
                   int accumulate, int block_n, int* status, double wait_budget_s, int num_sms, void* stream);
 
-// out[m, n] (+)= sum over examples e of ex_scale[e] * A_e^T B_e, where example e owns rows [e*ex_rows, (e+1)*ex_rows) of
-// a [T, M] and b [T, N] (ex_rows a multiple of 64).  The factor is applied to each example's fp32 partial product in
-// the epilogue; operands are not modified.  splits > 1 needs accumulate = 1.
-int ob_wgrad_clip_pe(const void* a, const void* b, int num_examples, int ex_rows, int M, int N, long long lda,
-                     long long ldb, const float* ex_scale, int splits, float* out, float* const* peer_out,
-                     long long shard_elems, long long out_offset, long long ldm, int accumulate, int* status,
-                     double wait_budget_s, int num_sms, void* stream);
-// Direct per-example gradient norms on the same kernel: norm2[e] += || a_e^T b_e ||_F^2 (nothing else is written).
-int ob_direct_norm2(const void* a, const void* b, int num_examples, int ex_rows, int M, int N, long long lda, long long ldb,
-                    int splits, float* norm2, int* status, double wait_budget_s, int num_sms, void* stream);
-
-int ob_ghost_norm(const void* a, const void* g, const int* ids, int B, int T, int Da, int Dg, long long lda,
-                  long long ldg, float* norm2, const int* seg, const int* seg_out, long long total_rows, int* status,
-                  double wait_budget_s, int num_sms, void* stream);
-
 // Several problems in one launch (host arrays of descriptions; launches hold up to 56): the layers of a backward pass
-// share one work list.  Fields as in the single calls above; put problems with more work per item first.
+// share one work list; put problems with more work per item first.
+//   ghost        norm2[i] += || A_i^T G_i ||_F^2 for every segment i of rows, from Gram matrices (ids: one-hot inputs)
+//   wgrad        ob_wgrad_clip
+//   wgrad_pe     out[m, n] (+)= sum over examples e of ex_scale[e] * A_e^T B_e, where example e owns rows
+//                [e * ex_rows, (e + 1) * ex_rows) of a [T, M] and b [T, N] (any ex_rows); the factor is applied to each example's
+//                fp32 partial product in the epilogue, operands are not modified; splits > 1 needs accumulate = 1.
+//                norm2 != NULL in every description: norm2[e] += || A_e^T B_e ||_F^2 instead, nothing else is written
 typedef struct {
   const void *a, *g;
   const int* ids;
@@ -54,7 +45,6 @@ typedef struct {
 int ob_ghost_norm_batch(const ob_ghost_desc* descs, int count, int* status, double wait_budget_s, int num_sms, void* stream);
 int ob_wgrad_clip_batch(const ob_wgrad_desc* descs, int count, float* out, float* const* peer_out, long long shard_elems,
                         int block_n, int* status, double wait_budget_s, int num_sms, void* stream);
-// (ex_rows of any length here)
 int ob_wgrad_clip_pe_batch(const ob_wgrad_pe_desc* descs, int count, float* out, float* const* peer_out,
                            long long shard_elems, int* status, double wait_budget_s, int num_sms, void* stream);
 

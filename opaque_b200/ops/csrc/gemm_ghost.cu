@@ -550,21 +550,6 @@ static int ghost_append(TmaBatch<GhostParams, CAP>& b, const ob_ghost_desc& d, b
 
 }  // namespace ob
 
-extern "C" int ob_ghost_norm(const void* a, const void* g, const int* ids, int B, int T, int Da, int Dg,
-                             long long lda, long long ldg, float* norm2, const int* seg, const int* seg_out,
-                             long long total_rows, int* status, double wait_budget_s, int num_sms, void* stream) {
-  using namespace ob;
-  const ob_ghost_desc d = {a, g, ids, norm2, seg, seg_out, lda, ldg, total_rows, B, T, Da, Dg};
-  TmaBatch<GhostParams, 1> b;
-  b.count = 0;
-  b.start[0] = b.start[1] = 0;
-  b.status = status;
-  b.wait_budget_ns = static_cast<unsigned long long>(wait_budget_s * 1e9);
-  const bool wide = ghost_use_wide(T);
-  const int rc = ghost_append(b, d, wide);
-  return rc ? rc : launch_ghost(b, wide, num_sms, static_cast<cudaStream_t>(stream));
-}
-
 extern "C" int ob_ghost_norm_batch(const ob_ghost_desc* descs, int count, int* status, double wait_budget_s, int num_sms,
                                    void* stream) {
   using namespace ob;

@@ -982,7 +982,6 @@ extern "C" int ob_wgrad_clip_batch(const ob_wgrad_desc* descs, int count, float*
   return 0;
 }
 
-// norm2 != NULL in every description: the direct per-example norms instead of the weighted gradients
 extern "C" int ob_wgrad_clip_pe_batch(const ob_wgrad_pe_desc* descs, int count, float* out, float* const* peer_out,
                                       long long shard_elems, int* status, double wait_budget_s, int num_sms, void* stream) {
   using namespace ob;
@@ -999,36 +998,6 @@ extern "C" int ob_wgrad_clip_pe_batch(const ob_wgrad_pe_desc* descs, int count, 
     if (rc) return rc;
   }
   return 0;
-}
-
-static int wgrad_pe_one(const ob_wgrad_pe_desc& d, float* out, float* const* peer_out, long long shard_elems, int* status,
-                        double wait_budget_s, int num_sms, void* stream) {
-  using namespace ob;
-  if (d.ex_rows > 0 && d.ex_rows % WG_BLOCK_K) return -3;
-  TmaBatch<WgradPeParams, 1> w;
-  batch_begin(w, status, wait_budget_s);
-  const int rc = wgrad_pe_append(w, d, out, peer_out, shard_elems);
-  if (rc) return rc;
-  return d.norm2 != nullptr ? launch_wgrad_pe<true>(w, num_sms, static_cast<cudaStream_t>(stream))
-                            : launch_wgrad_pe<false>(w, num_sms, static_cast<cudaStream_t>(stream));
-}
-
-extern "C" int ob_wgrad_clip_pe(const void* a, const void* b, int num_examples, int ex_rows, int M, int N, long long lda,
-                                long long ldb, const float* ex_scale, int splits, float* out, float* const* peer_out,
-                                long long shard_elems, long long out_offset, long long ldm, int accumulate, int* status,
-                                double wait_budget_s, int num_sms, void* stream) {
-  const ob_wgrad_pe_desc d = {a, b, ex_scale, nullptr, lda, ldb, out_offset, ldm, num_examples, ex_rows, M, N, splits, accumulate};
-  return wgrad_pe_one(d, out, peer_out, shard_elems, status, wait_budget_s, num_sms, stream);
-}
-
-// Direct per-example gradient norms: norm2[e] += || a_e^T b_e ||_F^2 for example e = rows [e * ex_rows, (e + 1) * ex_rows)
-// of a [T, M] and b [T, N] (ex_rows % 64 == 0).  `splits` spreads the examples of one tile over several CTAs.
-extern "C" int ob_direct_norm2(const void* a, const void* b, int num_examples, int ex_rows, int M, int N, long long lda,
-                               long long ldb, int splits, float* norm2, int* status, double wait_budget_s, int num_sms,
-                               void* stream) {
-  if (norm2 == nullptr) return -6;
-  const ob_wgrad_pe_desc d = {a, b, nullptr, norm2, lda, ldb, 0, N, num_examples, ex_rows, M, N, splits, 0};
-  return wgrad_pe_one(d, nullptr, nullptr, 0, status, wait_budget_s, num_sms, stream);
 }
 
 extern "C" int ob_last_detail(char* buf, int len) {
