@@ -309,9 +309,10 @@ __device__ __forceinline__ void pull_grad(const ShardStepParams& p, long long ba
 // where parameters go to peers (one 16-byte store per peer and thread).
 //
 // Bound by memory: 34 B per coordinate iid, + 8 B per noise buffer.  The arithmetic (Philox rounds, accurate log / sincos
-// / sqrt / divisions, about 160 instructions per coordinate) takes about half that time, so the two must overlap: every
-// load of a thread is issued BEFORE its noise is drawn.  (With the loads behind the noise and 8 coordinates a thread the two
-// phases added up.)  Measured: 749 M coordinates with four BLT buffers 13.5 -> 9.0 ms, 124 M coordinates iid 0.99 -> 0.77 ms,
+// / sqrt / divisions, about 160 instructions per coordinate) takes about half that time, so the two must overlap: with
+// iid noise and with up to four BLT buffers every load of a thread is issued BEFORE its noise is drawn.  (Further BLT buffers and the
+// rings of the banded modes are read behind the draw, in ftrl_apply: their registers would cost a resident block.  With all loads
+// behind the noise and 8 coordinates a thread the two phases added up.)  Measured: 749 M coordinates with four BLT buffers 13.5 -> 9.0 ms, 124 M coordinates iid 0.99 -> 0.77 ms,
 // 5.5 TB/s both.
 template <bool PULL, bool FTRL, int V>
 __global__ void __launch_bounds__(256, V == 4 ? (FTRL ? 3 : 4) : (FTRL ? 2 : 3))

@@ -439,7 +439,7 @@ rows_group_sum_kernel(const __nv_bfloat16* __restrict__ g, const __nv_bfloat16* 
 // ms with 32 x 512 tokens, 0.21 -> 0.01 with 2 x 64.
 // Measured, all norm and bias sums of GPT-2 small: 26 launches and 152 us -> one of 11.5 us with 2 x 64 tokens, 345 -> 197 us
 // with 11 x 333.  At 16,384 rows a launch per layer takes the operands while L2 still holds them (16.6 us each, 28 by HBM), so
-// longer sums are not deferred.
+// norm sums wait for one another up to 4,096 rows only.  Bias sums wait at any length (the 32 x 512 tokens above).
 constexpr int RS_CAP = 128;
 struct RowSumBatch {
   ob_rowsum_desc d[RS_CAP];
