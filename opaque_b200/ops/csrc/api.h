@@ -98,6 +98,8 @@ int ob_moe_combine(const void* y, const void* w, const long long* pos, void* out
 // Its backward by sorted row i: dy[i] = w[slot[i]] * dout[token[i]], dw[slot[i]] = <dout[token[i]], y[i]> (fp32).
 int ob_moe_row_grad(const void* dout, const void* y, const void* w, const long long* token, const long long* slot, void* dy,
                     float* dw, long long rows, int H, int sms, void* stream);
+// [dGate | dUp] (rows of 2I) of silu(gate) * up for gate_up = [gate | up], dh rows of I bf16 values, I % 8 == 0; exact fp32 steps.
+int ob_moe_glu_bwd(const void* dh, const void* gate_up, void* dgate_up, long long rows, int I, int sms, void* stream);
 
 // ob_rows_group_sum for several matrices with the same rows in one launch per 128 (host array of descriptions): g and x
 // [num_examples * rows_per_example, N] with pitch ldg, out / out2 rows with pitch ld_out / ld_out2, modes as there.

@@ -425,15 +425,15 @@ def glu_backward(dh: torch.Tensor, gate: torch.Tensor, up: torch.Tensor, act: st
 
 
 def glu_backward_packed(dh: torch.Tensor, gate_up: torch.Tensor) -> torch.Tensor:
-    """``[dGate | dUp]`` of ``silu(gate) * up`` for contiguous bf16 ``gate_up = [gate | up]`` (``[rows, 2I]``) and ``dh [rows, I]``."""
+    """``[dGate | dUp]`` of ``silu(gate) * up`` for contiguous bf16 ``gate_up = [gate | up]`` (``[rows, 2I]``) and ``dh [rows, I]``: the
+    bits of the separate fp32 operations."""
     rows, two_i = gate_up.shape
     I = two_i // 2
     if dh.shape != (rows, I) or not dh.is_contiguous() or not gate_up.is_contiguous():
         raise ValueError("glu_backward_packed: contiguous dh [rows, I] and gate_up [rows, 2I]")
     both = torch.empty_like(gate_up)
-    rc = lib.load().ob_glu_bwd(dh.data_ptr(), gate_up.data_ptr(), gate_up[:, I:].data_ptr(), both.data_ptr(), both[:, I:].data_ptr(),
-                               rows, I, two_i, two_i, ACTIVATION_SWIGLU, lib.sm_count(), lib.stream())
-    lib.check(rc, "glu_bwd")
+    rc = lib.load().ob_moe_glu_bwd(dh.data_ptr(), gate_up.data_ptr(), both.data_ptr(), rows, I, lib.sm_count(), lib.stream())
+    lib.check(rc, "moe_glu_bwd")
     return both
 
 

@@ -34,6 +34,7 @@ _SIGNATURES = {
     "ob_linear_ce_dlogits": [P, P, P, P, LL, I, LL, F, F, LL, P],
     "ob_moe_combine": [P, P, P, P, LL, I, I, I, P],
     "ob_moe_row_grad": [P, P, P, P, P, P, P, LL, I, I, P],
+    "ob_moe_glu_bwd": [P, P, P, LL, I, I, P],
     "ob_clip_tree_chunks": [P, I],
     "ob_clip_tree": [P, P, P, I, I, D, D, D, D, I, F, P, P, P, P, P],
     "ob_layernorm_fwd": [P, P, P, P, P, P, LL, I, F, P],

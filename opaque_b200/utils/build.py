@@ -21,10 +21,10 @@ ACC_SRC = PKG / "accounting" / "csrc"
 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC"]
 # Approximate division / exp / tanh are fine in the GEMM epilogues and activation kernels.  The translation units that draw
-# the DP noise, apply the optimizer and clip materialised gradients are compiled WITHOUT them: logarithm, sine / cosine, square
-# roots and divisions are the IEEE-accurate ones and subnormal values are kept.
+# the DP noise, apply the optimizer, clip materialised gradients and move the experts' rows are compiled WITHOUT them: exponential,
+# logarithm, sine / cosine, square roots and divisions are the IEEE-accurate ones and subnormal values are kept.
 FAST_MATH = "--use_fast_math"
-EXACT_MATH_SOURCES = {"dp_update.cu", "clip_tree.cu"}
+EXACT_MATH_SOURCES = {"dp_update.cu", "clip_tree.cu", "moe.cu"}
 OBJ_DIR = CSRC / "build"
 
 
