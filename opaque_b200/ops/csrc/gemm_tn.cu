@@ -206,11 +206,10 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     if (lane == 0) {
       constexpr uint32_t idesc_nmaj = make_idesc_bf16(GT_BM, BN, 0, 1);
       constexpr uint32_t idesc_kmaj = make_idesc_bf16(GT_BM, BN, 0, 0);
-      int stage = 0, acc_iter = 0, cursor = 0;
+      int stage = 0, acc_iter = 0;
       uint32_t phase = 0;
       bool ok = true;
       for (int w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
-        const GtItem it = gt_decode<BN>(p, w, tiles_m, tiles_n, tile_start, cursor);
         const int as = acc_iter & 1;
         if (!mbar_wait(&tmem_empty[as], ((acc_iter >> 1) & 1) ^ 1, abort_flag, p.status, OB_ERR_WAIT_TMEM_EMPTY,
                        budget)) {
