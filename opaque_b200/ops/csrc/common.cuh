@@ -12,6 +12,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <initializer_list>
+
 namespace ob {
 
 // ---------------------------------------------------------------------------------------------
@@ -233,6 +235,14 @@ struct alignas(64) TmaBatch {
     return cur;
   }
 };
+
+// ---------------------------------------------------------------------------------------------
+// Host check of what 16-byte accesses need (a null pointer passes): an entry point refuses an operand that would fault.
+static inline bool aligned16(std::initializer_list<const void*> ptrs) {
+  uintptr_t all = 0;
+  for (const void* q : ptrs) all |= reinterpret_cast<uintptr_t>(q);
+  return (all & 15) == 0;
+}
 
 // ---------------------------------------------------------------------------------------------
 // Philox-4x32-10 (Salmon et al.), counter-based: same (key, counter) -> same 4 words.

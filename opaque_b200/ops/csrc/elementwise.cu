@@ -606,7 +606,7 @@ static int flat_grid(long long work, int per_block, int sms) {
 extern "C" int ob_rmsnorm_fwd(const void* x, const void* residual, const void* w, void* y, void* sum_out,
                               float* rstd, long long rows, int H, float eps, float offset, int mode, void* stream) {
   if (rows <= 0) return 0;
-  if (H % 8) return -2;
+  if (H % 8 || !aligned16({x, residual, w, y, sum_out})) return -2;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const __nv_bfloat16 *xp = static_cast<const __nv_bfloat16*>(x), *rp = static_cast<const __nv_bfloat16*>(residual),
                       *wp = static_cast<const __nv_bfloat16*>(w);
@@ -630,7 +630,7 @@ extern "C" int ob_rmsnorm_bwd(const void* dy, const void* x, const void* w, cons
                               void* dx, float* dw_per_example, const int* seg_offsets, int num_examples,
                               int rows_per_example, long long rows, int H, float offset, void* stream) {
   if (rows <= 0) return 0;
-  if (H % 8) return -2;
+  if (H % 8 || !aligned16({dy, x, w, dsum_in, dx})) return -2;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (dx != nullptr) {
     const __nv_bfloat16 *gp = static_cast<const __nv_bfloat16*>(dy), *xp = static_cast<const __nv_bfloat16*>(x),
@@ -661,7 +661,7 @@ extern "C" int ob_rmsnorm_bwd(const void* dy, const void* x, const void* w, cons
 extern "C" int ob_glu_fwd(const void* gate, const void* up, void* out, long long rows, int I, long long ld_in,
                           int act, int sms, void* stream) {
   if (rows <= 0) return 0;
-  if (I % 8 || ld_in % 8) return -2;
+  if (I % 8 || ld_in % 8 || !aligned16({gate, up, out})) return -2;
   glu_fwd_kernel<<<flat_grid(rows * (I / 8), 256, sms), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const __nv_bfloat16*>(gate), static_cast<const __nv_bfloat16*>(up),
       static_cast<__nv_bfloat16*>(out), rows, I, ld_in, act);
@@ -671,7 +671,7 @@ extern "C" int ob_glu_fwd(const void* gate, const void* up, void* out, long long
 extern "C" int ob_glu_bwd(const void* dh, const void* gate, const void* up, void* dgate, void* dup, long long rows,
                           int I, long long ld_in, long long ld_out, int act, int sms, void* stream) {
   if (rows <= 0) return 0;
-  if (I % 8 || ld_in % 8 || ld_out % 8) return -2;
+  if (I % 8 || ld_in % 8 || ld_out % 8 || !aligned16({dh, gate, up, dgate, dup})) return -2;
   const unsigned grid = flat_grid(rows * (I / 8), 256, sms);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const __nv_bfloat16 *hp = static_cast<const __nv_bfloat16*>(dh), *gp = static_cast<const __nv_bfloat16*>(gate),

@@ -4,8 +4,6 @@
 // enough to materialise per example ([B, H] each), so they are reduced over an example's T token rows by a kernel and
 // added straight into that example's row of the per-example gradient buffer.
 // bf16 storage, fp32 math, 16-byte vector accesses, one CTA per row for the normalisation passes.
-#include <initializer_list>
-
 #include "common.cuh"
 #include "api.h"
 
@@ -594,7 +592,7 @@ static unsigned ln_warp_grid(long long rows, int H) {
 extern "C" int ob_layernorm_fwd(const void* x, const void* w, const void* b, void* y, float* mean, float* rstd,
                                 long long rows, int H, float eps, void* stream) {
   if (rows <= 0) return 0;
-  if (H % 8) return -2;
+  if (H % 8 || !aligned16({x, w, b, y})) return -2;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const __nv_bfloat16 *xp = static_cast<const __nv_bfloat16*>(x), *wp = static_cast<const __nv_bfloat16*>(w),
                       *bp = static_cast<const __nv_bfloat16*>(b);
@@ -611,17 +609,11 @@ extern "C" int ob_layernorm_fwd(const void* x, const void* w, const void* b, voi
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }
 
-static bool ln_aligned16(std::initializer_list<const void*> ptrs) {
-  uintptr_t all = 0;
-  for (const void* q : ptrs) all |= reinterpret_cast<uintptr_t>(q);
-  return (all & 15) == 0;
-}
-
 // With the residual addition in front (H <= 1024): sum = x + res, y = layernorm(sum); and its backward, dx += ds.
 extern "C" int ob_add_layernorm_fwd(const void* x, const void* res, const void* w, const void* b, void* y, void* sum, float* mean,
                                     float* rstd, long long rows, int H, float eps, void* stream) {
   if (rows <= 0) return 0;
-  if (H % 8 || H > 1024 || !ln_aligned16({x, res, w, b, y, sum})) return -2;
+  if (H % 8 || H > 1024 || !aligned16({x, res, w, b, y, sum})) return -2;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const __nv_bfloat16 *xp = static_cast<const __nv_bfloat16*>(x), *wp = static_cast<const __nv_bfloat16*>(w),
                       *bp = static_cast<const __nv_bfloat16*>(b), *rp = static_cast<const __nv_bfloat16*>(res);
@@ -637,7 +629,7 @@ extern "C" int ob_add_layernorm_fwd(const void* x, const void* res, const void* 
 extern "C" int ob_add_layernorm_bwd_dx(const void* dy, const void* x, const void* w, const float* mean, const float* rstd,
                                        const void* ds, void* dx, long long rows, int H, void* stream) {
   if (rows <= 0) return 0;
-  if (H % 8 || H > 1024 || !ln_aligned16({dy, x, w, ds, dx})) return -2;
+  if (H % 8 || H > 1024 || !aligned16({dy, x, w, ds, dx})) return -2;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const __nv_bfloat16 *gp = static_cast<const __nv_bfloat16*>(dy), *xp = static_cast<const __nv_bfloat16*>(x),
                       *wp = static_cast<const __nv_bfloat16*>(w), *dp = static_cast<const __nv_bfloat16*>(ds);
@@ -653,7 +645,7 @@ extern "C" int ob_add_layernorm_bwd_dx(const void* dy, const void* x, const void
 extern "C" int ob_layernorm_bwd_dx(const void* dy, const void* x, const void* w, const float* mean, const float* rstd,
                                    void* dx, long long rows, int H, void* stream) {
   if (rows <= 0) return 0;
-  if (H % 8) return -2;
+  if (H % 8 || !aligned16({dy, x, w, dx})) return -2;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const __nv_bfloat16 *gp = static_cast<const __nv_bfloat16*>(dy), *xp = static_cast<const __nv_bfloat16*>(x),
                       *wp = static_cast<const __nv_bfloat16*>(w);
@@ -739,7 +731,7 @@ extern "C" int ob_merge_heads3(const void* q, const void* k, const void* v, cons
 
 extern "C" int ob_activation(const void* x, const void* dy, void* out, long long numel, int act, int sms, void* stream) {
   if (numel <= 0) return 0;
-  if (numel % 8) return -2;
+  if (numel % 8 || !aligned16({x, dy, out})) return -2;
   const long long nvec = numel / 8;
   long long grid = (nvec + 255) / 256;
   const long long cap = static_cast<long long>(sms) * 16;

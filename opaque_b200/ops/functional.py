@@ -384,8 +384,8 @@ class _GLU(Function):
     def forward(ctx, gate, up, act):
         I = gate.shape[-1]
         g2, u2 = gate.reshape(-1, I), up.reshape(-1, I)
-        if g2.stride(1) != 1 or u2.stride(1) != 1 or g2.stride(0) != u2.stride(0):
-            g2, u2 = g2.contiguous(), u2.contiguous()
+        if g2.stride(1) != 1 or u2.stride(1) != 1 or g2.stride(0) != u2.stride(0) or (g2.data_ptr() | u2.data_ptr()) & 15:
+            g2, u2 = _vec16(g2), _vec16(u2)
         out = torch.empty(g2.shape, dtype=gate.dtype, device=gate.device)
         rc = lib.load().ob_glu_fwd(g2.data_ptr(), u2.data_ptr(), out.data_ptr(), g2.shape[0], I, g2.stride(0), act,
                                    lib.sm_count(), lib.stream())

@@ -61,14 +61,22 @@ def test_norms_and_activations_of_views_that_start_anywhere():
     assert off(x).is_contiguous() and off(x).data_ptr() % 16 == 2
     for fn, grads in ((lambda p, q: ops.add_layer_norm(p, q, w, b), 2), (lambda p, q: ops.fused_add_rms_norm(p, q, w), 2),
                       (lambda p, q: (ops.layer_norm(p + q, w, b),), 1), (lambda p, q: (ops.layer_norm(p, w, b),), 1),
-                      (lambda p, q: (ops.rms_norm(p, w),), 1), (lambda p, q: (ops.activation(p, "silu"),), 1)):
+                      (lambda p, q: (ops.rms_norm(p, w),), 1), (lambda p, q: (ops.activation(p, "silu"),), 1),
+                      (lambda p, q: (ops.swiglu(p, q),), 1), (lambda p, q: (ops.geglu(p, q),), 1)):
         out = []
         for shift in (lambda t: t, off):
             p, q = shift(x).detach().requires_grad_(True), shift(res).detach().requires_grad_(True)
             ys = fn(p, q)
             torch.autograd.backward(list(ys), [shift(g) for g in (gy, gs)[:grads]])
-            out.append((*ys, p.grad))
-        assert all(torch.equal(u, v) for u, v in zip(*out))
+            out.append((*ys, p.grad, q.grad))
+        assert all(torch.equal(u, v) if u is not None else v is None for u, v in zip(*out))
+    # gate and up as slices of rows that start elsewhere: one pitch for both, neither aligned
+    rows = torch.randn(5, 136, device="cuda", dtype=torch.bfloat16)
+    assert torch.equal(ops.swiglu(rows[:, 1:65], rows[:, 66:130]), ops.swiglu(rows[:, 1:65].contiguous(), rows[:, 66:130].contiguous()))
+    for fn in (lambda: ops.layer_norm(x, off(w)), lambda: ops.rms_norm(x, off(w)), lambda: ops.add_layer_norm(x, res, w, off(b)),
+               lambda: ops.fused_add_rms_norm(x, res, off(w))):
+        with pytest.raises(ops.KernelLibraryError):         # parameters are not copied: the entry points refuse what would fault
+            fn()
 
 
 @pytest.mark.parametrize("count", [1, 3, 130])
