@@ -81,6 +81,20 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
+// The question without the wait (try_wait may suspend the warp for microseconds).  A role asks it for its NEXT stage before it
+// issues the current one, so that the round trip (74 clocks) hides behind the issue.
+__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+
 // Bounded wait.  `abort_flag` is a CTA-shared word: once any role of the CTA has
 // given up, every other wait in the CTA returns false promptly as well.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
@@ -101,6 +115,35 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   }
 }
 
+// The roles that feed the tensor core (TMA producer, MMA issuer) run as WHOLE warps with warp-uniform control flow, and only the
+// copies, MMAs and commits stand inside `if (elect_one())`.  Inside `if (lane == 0)` the compiler has to keep descriptors and
+// addresses in per-thread registers and move each one to a uniform register before every instruction that wants it there: four
+// MMAs and a commit took 378 clocks to issue and a k-block 604, whatever the tile's width (the tensor pipe needs 512 for 256
+// columns, 256 for 64).  Values that are read from memory become uniform through uniform().
+__device__ __forceinline__ int uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
+__device__ __forceinline__ uint32_t uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
+
+// mbar_wait for a converged warp: all lanes ask, and the answer is warp-uniform.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status, int code,
+                                               uint64_t budget_ns) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  const uint64_t t0 = globaltimer_ns();
+  uint32_t spins = 0;
+  while (true) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    if ((++spins & 0xff) == 0) {
+      if (__any_sync(0xffffffffu, *abort_flag != 0)) return false;
+      if (__any_sync(0xffffffffu, globaltimer_ns() - t0 > budget_ns)) {
+        if ((threadIdx.x & 31) == 0) {
+          *abort_flag = 1;
+          set_error(status, code);
+        }
+        __syncwarp();
+        return false;
+      }
+    }
+  }
+}
 // generic-proxy writes to shared memory -> visible to the async proxy (UMMA / TMA reads)
 __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -159,6 +202,15 @@ __device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t adesc, uint6
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                : "memory");
+}
+// One 64-deep k-block, issued by the elected lane: D[tmem] (+)= the four 16-deep products of a stage, then a commit that arrives on
+// `bar` when they have read it.  A_STEP, B_STEP: distance of two k-steps in the operands, in the descriptors' 16-byte units.
+template <int A_STEP, int B_STEP>
+__device__ __forceinline__ void umma_bf16_kblock(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, bool accumulate,
+                                                 uint64_t* bar) {
+#pragma unroll
+  for (int kk = 0; kk < 4; ++kk) umma_bf16(d_tmem, adesc + kk * A_STEP, bdesc + kk * B_STEP, idesc, (accumulate || kk > 0) ? 1u : 0u);
+  umma_commit(bar);
 }
 // 32 lanes x 32 consecutive fp32 columns: thread i of the warp receives row (lane base + i).
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {

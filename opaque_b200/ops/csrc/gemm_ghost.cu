@@ -84,7 +84,7 @@ ghost_norm_kernel(const __grid_constant__ TmaBatch<GhostParams, CAP> b) {
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * GH_STAGES + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform(static_cast<int>(threadIdx.x >> 5)), lane = threadIdx.x & 31;
   const int total_work = b.total();
   const uint64_t budget = b.wait_budget_ns;
 
@@ -109,29 +109,29 @@ ghost_norm_kernel(const __grid_constant__ TmaBatch<GhostParams, CAP> b) {
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = uniform(*tmem_slot);
 
   if (warp == 0) {
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0, issued_mask = 0, issued_phase = 0;
-      bool ok = true;
-      int cur = 0;
-      for (int w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
-        cur = b.seek(w, cur);
-        const GhostParams& p = b.p[cur];
-        const GhostShape sh(p);
-        const GhostItem it = ghost_decode(w - b.start[cur], sh.pairs, sh.nt);
-        const int s0 = p.seg ? p.seg[it.ex] : it.ex * p.T;
-        const int len = p.seg ? p.seg[it.ex + 1] - s0 : p.T;
-        if (it.tb2 * GH_TILE >= len) continue;                 // tile pair lies outside this (ragged) segment
-        const int r1 = s0 + it.tb * GH_TILE, r2 = s0 + it.tb2 * GH_TILE;
-        const bool diag = it.tb == it.tb2;
-        for (int kb = 0; kb < sh.num_kb; ++kb) {
-          if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, b.status, OB_ERR_WAIT_EMPTY, budget)) {
-            ok = false;
-            break;
-          }
+    int stage = 0;
+    uint32_t phase = 0, issued_mask = 0, issued_phase = 0;
+    bool ok = true;
+    int cur = 0;
+    for (int w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
+      cur = b.seek(w, cur);
+      const GhostParams& p = b.p[cur];
+      const GhostShape sh(p);
+      const GhostItem it = ghost_decode(w - b.start[cur], sh.pairs, sh.nt);
+      const int s0 = p.seg ? uniform(p.seg[it.ex]) : it.ex * p.T;
+      const int len = p.seg ? uniform(p.seg[it.ex + 1]) - s0 : p.T;
+      if (it.tb2 * GH_TILE >= len) continue;                 // tile pair lies outside this (ragged) segment
+      const int r1 = s0 + it.tb * GH_TILE, r2 = s0 + it.tb2 * GH_TILE;
+      const bool diag = it.tb == it.tb2;
+      for (int kb = 0; kb < sh.num_kb; ++kb) {
+        if (!mbar_wait_warp(&empty[stage], phase ^ 1, abort_flag, b.status, OB_ERR_WAIT_EMPTY, budget)) {
+          ok = false;
+          break;
+        }
+        if (elect_one()) {
           // a diagonal tile multiplies a row block with itself: one load serves both operands
           mbar_expect_tx(&full[stage], diag ? GH_TILE_BYTES : GH_STAGE_BYTES);
           uint8_t* dst = smem + stage * GH_STAGE_BYTES;
@@ -139,64 +139,61 @@ ghost_norm_kernel(const __grid_constant__ TmaBatch<GhostParams, CAP> b) {
           const int col = (kb < sh.ka ? kb : kb - sh.ka) * GH_BLOCK_K;
           tma_load_2d(dst, map, &full[stage], col, r1);
           if (!diag) tma_load_2d(dst + GH_TILE_BYTES, map, &full[stage], col, r2);
-          issued_mask |= 1u << stage;
-          issued_phase = (issued_phase & ~(1u << stage)) | (phase << stage);
-          if (++stage == GH_STAGES) { stage = 0; phase ^= 1; }
         }
-      }
-      if (!ok) {
-        for (int s = 0; s < GH_STAGES; ++s)
-          if (issued_mask & (1u << s)) {
-            int dummy_abort = 0;
-            mbar_wait(&full[s], (issued_phase >> s) & 1u, &dummy_abort, b.status, OB_ERR_DRAIN, budget);
-          }
+        issued_mask |= 1u << stage;
+        issued_phase = (issued_phase & ~(1u << stage)) | (phase << stage);
+        if (++stage == GH_STAGES) { stage = 0; phase ^= 1; }
       }
     }
+    if (!ok) {
+      for (int s = 0; s < GH_STAGES; ++s)
+        if (issued_mask & (1u << s)) {
+          int dummy_abort = 0;
+          mbar_wait(&full[s], (issued_phase >> s) & 1u, &dummy_abort, b.status, OB_ERR_DRAIN, budget);
+        }
+    }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc_bf16(GH_TILE, GH_TILE, 0, 0);
-      int stage = 0, acc_iter = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      int cur = 0;
-      for (int w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
-        cur = b.seek(w, cur);
-        const GhostParams& p = b.p[cur];
-        const GhostShape sh(p);
-        const GhostItem it = ghost_decode(w - b.start[cur], sh.pairs, sh.nt);
-        if (p.seg && it.tb2 * GH_TILE >= p.seg[it.ex + 1] - p.seg[it.ex]) continue;
-        const uint32_t b_off = it.tb == it.tb2 ? 0u : static_cast<uint32_t>(GH_TILE_BYTES);
-        const int as = acc_iter & 1;
-        if (!mbar_wait(&tmem_empty[as], ((acc_iter >> 1) & 1) ^ 1, abort_flag, b.status, OB_ERR_WAIT_TMEM_EMPTY,
-                       budget)) {
+    constexpr uint32_t idesc = make_idesc_bf16(GH_TILE, GH_TILE, 0, 0);
+    const uint32_t ring = smem_u32(smem);
+    int stage = 0, acc_iter = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    int cur = 0;
+    for (int w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
+      cur = b.seek(w, cur);
+      const GhostParams& p = b.p[cur];
+      const GhostShape sh(p);
+      const GhostItem it = ghost_decode(w - b.start[cur], sh.pairs, sh.nt);
+      if (p.seg && it.tb2 * GH_TILE >= uniform(p.seg[it.ex + 1] - p.seg[it.ex])) continue;
+      const uint32_t b_off = it.tb == it.tb2 ? 0u : static_cast<uint32_t>(GH_TILE_BYTES);
+      const int as = acc_iter & 1;
+      if (!mbar_wait_warp(&tmem_empty[as], ((acc_iter >> 1) & 1) ^ 1, abort_flag, b.status, OB_ERR_WAIT_TMEM_EMPTY, budget)) {
+        ok = false;
+        break;
+      }
+      tc_fence_after();
+      bool ready = false;
+      for (int kb = 0; kb < sh.num_kb; ++kb) {
+        if (!ready && !mbar_wait_warp(&full[stage], phase, abort_flag, b.status, OB_ERR_WAIT_FULL, budget)) {
           ok = false;
           break;
         }
         tc_fence_after();
-        for (int kb = 0; kb < sh.num_kb; ++kb) {
-          if (!mbar_wait(&full[stage], phase, abort_flag, b.status, OB_ERR_WAIT_FULL, budget)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t t1 = smem_u32(smem + stage * GH_STAGE_BYTES), t2 = t1 + b_off;
-          const uint32_t d_tmem = tmem_base + as * 256 + (kb < sh.ka ? 0 : 128);
-          const bool first = (kb == 0) || (kb == sh.ka);
-#pragma unroll
-          for (int kk = 0; kk < GH_BLOCK_K / 16; ++kk) {
-            // K-major, 128-byte swizzle: rows are 128 B apart, 8-row groups 1024 B apart; a k-step
-            // of 16 elements moves the start address by 32 B inside the swizzled row.
-            const uint64_t ad = make_smem_desc(t1 + kk * 32, 16, 1024, 2);
-            const uint64_t bd = make_smem_desc(t2 + kk * 32, 16, 1024, 2);
-            umma_bf16(d_tmem, ad, bd, idesc, (first && kk == 0) ? 0u : 1u);
-          }
-          umma_commit(&empty[stage]);
-          if (++stage == GH_STAGES) { stage = 0; phase ^= 1; }
-        }
-        if (!ok) break;
-        umma_commit(&tmem_full[as]);
-        ++acc_iter;
+        // K-major, 128-byte swizzle: rows are 128 B apart, 8-row groups 1024 B apart; a k-step of 16 elements moves the start
+        // address by 32 B inside the swizzled row.
+        const uint32_t t1 = ring + stage * GH_STAGE_BYTES;
+        const uint64_t ad = make_smem_desc(t1, 16, 1024, 2), bd = make_smem_desc(t1 + b_off, 16, 1024, 2);
+        const uint32_t d_tmem = tmem_base + as * 256 + (kb < sh.ka ? 0 : 128);
+        const int next = stage + 1 == GH_STAGES ? 0 : stage + 1;
+        const bool peek = kb + 1 < sh.num_kb && mbar_test_wait(&full[next], next == 0 ? phase ^ 1 : phase);
+        const bool first = (kb == 0) || (kb == sh.ka);
+        if (elect_one()) umma_bf16_kblock<2, 2>(d_tmem, ad, bd, idesc, !first, &empty[stage]);
+        ready = __all_sync(0xffffffffu, peek);
+        if (++stage == GH_STAGES) { stage = 0; phase ^= 1; }
       }
+      if (!ok) break;
+      if (elect_one()) umma_commit(&tmem_full[as]);
+      ++acc_iter;
     }
   } else {
     const int q = warp & 3;
@@ -304,7 +301,7 @@ ghost_norm_wide_kernel(const __grid_constant__ TmaBatch<GhostParams, CAP> b) {
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * GW_STAGES + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform(static_cast<int>(threadIdx.x >> 5)), lane = threadIdx.x & 31;
   const int total_work = b.total();
   const uint64_t budget = b.wait_budget_ns;
 
@@ -327,7 +324,7 @@ ghost_norm_wide_kernel(const __grid_constant__ TmaBatch<GhostParams, CAP> b) {
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = uniform(*tmem_slot);
 
   // segment of example `ex`: first row and length; an item is skipped when its column blocks start past the end
   auto segment = [](const GhostParams& p, int ex, int& s0, int& len) {
@@ -336,26 +333,28 @@ ghost_norm_wide_kernel(const __grid_constant__ TmaBatch<GhostParams, CAP> b) {
   };
 
   if (warp == 0) {
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0, issued_mask = 0, issued_phase = 0;
-      bool ok = true;
-      int cur = 0;
-      for (int w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
-        cur = b.seek(w, cur);
-        const GhostParams& p = b.p[cur];
-        const GhostShape sh(p);
-        const GhostWideItem it = ghost_wide_decode(w - b.start[cur], sh.wide_items, sh.nt, sh.ncb);
-        int s0, len;
-        segment(p, it.ex, s0, len);
-        if (it.tb * GH_TILE >= len || it.cb * GW_TILE_N >= len) continue;
-        const int r1 = s0 + it.tb * GH_TILE, r2 = s0 + it.cb * GW_TILE_N;
-        const bool diag = (it.tb >> 1) == it.cb;              // the row block is one of the two column blocks
-        for (int kb = 0; kb < sh.num_kb; ++kb) {
-          if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, b.status, OB_ERR_WAIT_EMPTY, budget)) {
-            ok = false;
-            break;
-          }
+    int stage = 0;
+    uint32_t phase = 0, issued_mask = 0, issued_phase = 0;
+    bool ok = true;
+    int cur = 0;
+    for (int w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
+      cur = b.seek(w, cur);
+      const GhostParams& p = b.p[cur];
+      const GhostShape sh(p);
+      const GhostWideItem it = ghost_wide_decode(w - b.start[cur], sh.wide_items, sh.nt, sh.ncb);
+      int s0, len;
+      segment(p, it.ex, s0, len);
+      s0 = uniform(s0);
+      len = uniform(len);
+      if (it.tb * GH_TILE >= len || it.cb * GW_TILE_N >= len) continue;
+      const int r1 = s0 + it.tb * GH_TILE, r2 = s0 + it.cb * GW_TILE_N;
+      const bool diag = (it.tb >> 1) == it.cb;              // the row block is one of the two column blocks
+      for (int kb = 0; kb < sh.num_kb; ++kb) {
+        if (!mbar_wait_warp(&empty[stage], phase ^ 1, abort_flag, b.status, OB_ERR_WAIT_EMPTY, budget)) {
+          ok = false;
+          break;
+        }
+        if (elect_one()) {
           mbar_expect_tx(&full[stage], diag ? GW_B_BYTES : GW_STAGE_BYTES);
           uint8_t* dst = smem + stage * GW_STAGE_BYTES;
           const CUtensorMap* map = kb < sh.ka ? &b.map_a[cur] : &b.map_b[cur];
@@ -363,64 +362,65 @@ ghost_norm_wide_kernel(const __grid_constant__ TmaBatch<GhostParams, CAP> b) {
           if (!diag) tma_load_2d(dst, map, &full[stage], col, r1);
           tma_load_2d(dst + GW_A_BYTES, map, &full[stage], col, r2);
           tma_load_2d(dst + GW_A_BYTES + GW_A_BYTES, map, &full[stage], col, r2 + GH_TILE);
-          issued_mask |= 1u << stage;
-          issued_phase = (issued_phase & ~(1u << stage)) | (phase << stage);
-          if (++stage == GW_STAGES) { stage = 0; phase ^= 1; }
         }
-      }
-      if (!ok) {
-        for (int s = 0; s < GW_STAGES; ++s)
-          if (issued_mask & (1u << s)) {
-            int dummy_abort = 0;
-            mbar_wait(&full[s], (issued_phase >> s) & 1u, &dummy_abort, b.status, OB_ERR_DRAIN, budget);
-          }
+        issued_mask |= 1u << stage;
+        issued_phase = (issued_phase & ~(1u << stage)) | (phase << stage);
+        if (++stage == GW_STAGES) { stage = 0; phase ^= 1; }
       }
     }
+    if (!ok) {
+      for (int s = 0; s < GW_STAGES; ++s)
+        if (issued_mask & (1u << s)) {
+          int dummy_abort = 0;
+          mbar_wait(&full[s], (issued_phase >> s) & 1u, &dummy_abort, b.status, OB_ERR_DRAIN, budget);
+        }
+    }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc_bf16(GH_TILE, GW_TILE_N, 0, 0);
-      int stage = 0, acc_iter = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      int cur = 0;
-      for (int w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
-        cur = b.seek(w, cur);
-        const GhostParams& p = b.p[cur];
-        const GhostShape sh(p);
-        const GhostWideItem it = ghost_wide_decode(w - b.start[cur], sh.wide_items, sh.nt, sh.ncb);
-        int s0, len;
-        segment(p, it.ex, s0, len);
-        if (it.tb * GH_TILE >= len || it.cb * GW_TILE_N >= len) continue;
-        // on a diagonal super-block the A operand is read from the copy of that row block inside the B operand
-        const uint32_t a_off = (it.tb >> 1) == it.cb ? static_cast<uint32_t>(GW_A_BYTES + (it.tb & 1) * GW_A_BYTES) : 0u;
-        if (!mbar_wait(tmem_empty, (acc_iter & 1) ^ 1, abort_flag, b.status, OB_ERR_WAIT_TMEM_EMPTY, budget)) {
+    constexpr uint32_t idesc = make_idesc_bf16(GH_TILE, GW_TILE_N, 0, 0);
+    const uint32_t ring = smem_u32(smem);
+    int stage = 0, acc_iter = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    int cur = 0;
+    for (int w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
+      cur = b.seek(w, cur);
+      const GhostParams& p = b.p[cur];
+      const GhostShape sh(p);
+      const GhostWideItem it = ghost_wide_decode(w - b.start[cur], sh.wide_items, sh.nt, sh.ncb);
+      int s0, len;
+      segment(p, it.ex, s0, len);
+      s0 = uniform(s0);
+      len = uniform(len);
+      if (it.tb * GH_TILE >= len || it.cb * GW_TILE_N >= len) continue;
+      // on a diagonal super-block the A operand is read from the copy of that row block inside the B operand
+      const uint32_t a_off = (it.tb >> 1) == it.cb ? static_cast<uint32_t>(GW_A_BYTES + (it.tb & 1) * GW_A_BYTES) : 0u;
+      if (!mbar_wait_warp(tmem_empty, (acc_iter & 1) ^ 1, abort_flag, b.status, OB_ERR_WAIT_TMEM_EMPTY, budget)) {
+        ok = false;
+        break;
+      }
+      tc_fence_after();
+      bool ready = false;
+      for (int kb = 0; kb < sh.num_kb; ++kb) {
+        if (!ready && !mbar_wait_warp(&full[stage], phase, abort_flag, b.status, OB_ERR_WAIT_FULL, budget)) {
           ok = false;
           break;
         }
         tc_fence_after();
-        for (int kb = 0; kb < sh.num_kb; ++kb) {
-          if (!mbar_wait(&full[stage], phase, abort_flag, b.status, OB_ERR_WAIT_FULL, budget)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t st0 = smem_u32(smem + stage * GW_STAGE_BYTES);
-          const uint32_t t1 = st0 + a_off, t2 = st0 + GW_A_BYTES;
-          const uint32_t d_tmem = tmem_base + (kb < sh.ka ? 0 : GW_TILE_N);
-          const bool first = (kb == 0) || (kb == sh.ka);
-#pragma unroll
-          for (int kk = 0; kk < GH_BLOCK_K / 16; ++kk) {
-            const uint64_t ad = make_smem_desc(t1 + kk * 32, 16, 1024, 2);
-            const uint64_t bd = make_smem_desc(t2 + kk * 32, 16, 1024, 2);
-            umma_bf16(d_tmem, ad, bd, idesc, (first && kk == 0) ? 0u : 1u);
-          }
-          umma_commit(&empty[stage]);
-          if (++stage == GW_STAGES) { stage = 0; phase ^= 1; }
-        }
-        if (!ok) break;
-        umma_commit(tmem_full);
-        ++acc_iter;
+        // K-major, 128-byte swizzle: rows are 128 B apart, 8-row groups 1024 B apart; a k-step of 16 elements moves the start
+        // address by 32 B inside the swizzled row.
+        const uint32_t st0 = ring + stage * GW_STAGE_BYTES;
+        const uint64_t ad = make_smem_desc(st0 + a_off, 16, 1024, 2), bd = make_smem_desc(st0 + GW_A_BYTES, 16, 1024, 2);
+        const uint32_t d_tmem = tmem_base + (kb < sh.ka ? 0 : GW_TILE_N);
+        const int next = stage + 1 == GW_STAGES ? 0 : stage + 1;
+        const bool peek = kb + 1 < sh.num_kb && mbar_test_wait(&full[next], next == 0 ? phase ^ 1 : phase);
+        const bool first = (kb == 0) || (kb == sh.ka);
+        if (elect_one()) umma_bf16_kblock<2, 2>(d_tmem, ad, bd, idesc, !first, &empty[stage]);
+        ready = __all_sync(0xffffffffu, peek);
+        if (++stage == GW_STAGES) { stage = 0; phase ^= 1; }
       }
+      if (!ok) break;
+      if (elect_one()) umma_commit(tmem_full);
+      ++acc_iter;
     }
   } else {
     const int q = warp & 3;                  // TMEM lane quadrant

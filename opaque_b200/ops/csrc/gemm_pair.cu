@@ -46,9 +46,6 @@ constexpr int GP_BK = 64;
 #ifndef OB_PAIR_STAGES
 #define OB_PAIR_STAGES 4
 #endif
-#ifndef OB_PAIR_INTERLEAVE
-#define OB_PAIR_INTERLEAVE 1
-#endif
 #ifndef OB_PAIR_RELAXED
 #define OB_PAIR_RELAXED 0
 #endif
@@ -199,6 +196,9 @@ __device__ __forceinline__ GpSchedule gp_read_schedule(const int* sched_local) {
   asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(s.first) : "r"(a) : "memory");
   asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(s.end) : "r"(a + 4) : "memory");
   asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(s.stride) : "r"(a + 8) : "memory");
+  s.first = uniform(s.first);
+  s.end = uniform(s.end);
+  s.stride = uniform(s.stride);
   return s;
 }
 
@@ -376,7 +376,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* sched = reinterpret_cast<int*>(tmem_slot + 2);  // [3]: first, end, stride (valid in the leader CTA)
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform(static_cast<int>(threadIdx.x >> 5)), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const bool leader = rank == 0;
   const int tiles_n = EPI == GP_EPI_GLU ? (p.N / 2 + GP_BNH - 1) / GP_BNH : (p.N + GP_BN - 1) / GP_BN;
@@ -420,26 +420,26 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   __syncthreads();
   cluster_sync_all();                // both CTAs' barriers are initialised before any remote arrival or copy
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = uniform(*tmem_slot);
   const GpSchedule sc = gp_read_schedule(sched);
 
   if (warp == 0) {
-    if (lane == 0) {
-      // ---------------------------------------------------------------- TMA producer (one per CTA)
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      const CUtensorMap* mb1 = (EPI == GP_EPI_GLU && rank == 1) ? &map_b_up : &map_b;
-      const CUtensorMap* mb2 = (EPI == GP_EPI_GLU && rank == 1) ? &map_b2_up : &map_b2;
-      for (int w = sc.first; ok && w < sc.end; w += sc.stride) {
-        const GpItem it = gp_decode(w, tiles_m, tiles_n, rank, p.group_m);
-        // first column of N (= row of a [N, K] operand) of this CTA's half of the B tile
-        const int bn0 = EPI == GP_EPI_GLU ? it.nt * GP_BNH : it.nt * GP_BN + static_cast<int>(rank) * GP_BNH;
-        for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, p.status, OB_ERR_WAIT_EMPTY, budget)) {
-            ok = false;
-            break;
-          }
+    // ---------------------------------------------------------------- TMA producer (one per CTA)
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    const CUtensorMap* mb1 = (EPI == GP_EPI_GLU && rank == 1) ? &map_b_up : &map_b;
+    const CUtensorMap* mb2 = (EPI == GP_EPI_GLU && rank == 1) ? &map_b2_up : &map_b2;
+    for (int w = sc.first; ok && w < sc.end; w += sc.stride) {
+      const GpItem it = gp_decode(w, tiles_m, tiles_n, rank, p.group_m);
+      // first column of N (= row of a [N, K] operand) of this CTA's half of the B tile
+      const int bn0 = EPI == GP_EPI_GLU ? it.nt * GP_BNH : it.nt * GP_BN + static_cast<int>(rank) * GP_BNH;
+      for (int kb = 0; kb < num_kb; ++kb) {
+        if (!mbar_wait_warp(&empty[stage], phase ^ 1, abort_flag, p.status, OB_ERR_WAIT_EMPTY, budget)) {
+          ok = false;
+          break;
+        }
+        if (elect_one()) {
           if (leader) mbar_expect_tx(&full[stage], 2 * GP_STAGE_BYTES);
           const uint32_t bar = map_to_cta(smem_u32(&full[stage]), 0);
           uint8_t* a_dst = smem + stage * GP_STAGE_BYTES;
@@ -455,12 +455,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
           } else {
             tma_load_2d_pair(b_dst, mb, bar, k0, bn0);
           }
-          if (++stage == GP_STAGES) { stage = 0; phase ^= 1; }
         }
+        if (++stage == GP_STAGES) { stage = 0; phase ^= 1; }
       }
     }
   } else if (warp == 1) {
-    if (leader && lane == 0) {
+    if (leader) {
       // ---------------------------------------------------------------- MMA issuer (leader CTA only)
       // Each CTA holds 256 rows of A per stage: two 128-row halves, one accumulator (256 TMEM columns) each, both
       // multiplied with the SAME B tile, so a stage's 48 KB feed 2 x (128 x 256 x 64) of work per SM.
@@ -472,38 +472,24 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       int stage = 0, acc_iter = 0;
       uint32_t phase = 0;
       bool ok = true;
-      auto issue_one = [&](int h, int kb, int st, int kk) {
-        const uint32_t a_addr = smem_u32(smem + st * GP_STAGE_BYTES);
+      const uint32_t ring = smem_u32(smem);
+      // one accumulator half of one k-block, by one lane; `frees`: the stage's last reader hands it back in both CTAs
+      auto issue_half = [&](int h, int kb, int st, bool frees) {
+        const uint32_t a_addr = ring + st * GP_STAGE_BYTES;
         const uint32_t b_addr = a_addr + GP_A_BYTES;
         const bool kn = kb < nk1 ? p.kn1 != 0 : p.kn2 != 0;
         // K-major operand: rows 128 B apart, 8-row groups 1024 B apart, 32 B per 16-element k-step.
         // N-major operand: 64-column blocks GP_BK*128 B apart, 8-row (k) groups 1024 B apart, 2048 B per k-step.
-        const uint64_t ad = make_smem_desc(a_addr + h * (GP_MMA_M * 128) + kk * 32, 16, 1024, 2);
-        const uint64_t bd = kn ? make_smem_desc(b_addr + kk * (16 * 128), GP_BK * 128, 1024, 2)
-                               : make_smem_desc(b_addr + kk * 32, 16, 1024, 2);
-        umma_bf16_pair(tmem_base + h * GP_BN, ad, bd, kn ? idesc_n : idesc_k, (kb > 0 || kk > 0) ? 1u : 0u);
-      };
-      auto issue_half = [&](int h, int kb, int st) {
+        const uint64_t ad = make_smem_desc(a_addr + h * (GP_MMA_M * 128), 16, 1024, 2);
+        const uint64_t bd = kn ? make_smem_desc(b_addr, GP_BK * 128, 1024, 2) : make_smem_desc(b_addr, 16, 1024, 2);
+        const uint32_t b_step = kn ? 128u : 2u, idesc = kn ? idesc_n : idesc_k;
+        if (elect_one()) {
 #pragma unroll
-        for (int kk = 0; kk < GP_BK / 16; ++kk) issue_one(h, kb, st, kk);
-        if (kb == num_kb - 1) umma_commit_pair(&tmem_full[h], 3);   // this half's accumulators (both CTAs) are complete
-      };
-      // steady state: the two accumulators alternate k-step by k-step, so no instruction waits on the one before it
-      auto issue_both = [&](int kb, int st) {
-#if OB_PAIR_INTERLEAVE
-#pragma unroll
-        for (int kk = 0; kk < GP_BK / 16; ++kk) {
-          issue_one(0, kb, st, kk);
-          issue_one(1, kb, st, kk);
+          for (int kk = 0; kk < GP_BK / 16; ++kk)
+            umma_bf16_pair(tmem_base + h * GP_BN, ad + 2 * kk, bd + kk * b_step, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
+          if (kb == num_kb - 1) umma_commit_pair(&tmem_full[h], 3);   // this half's accumulators (both CTAs) are complete
+          if (frees) umma_commit_pair(&empty[st], 3);
         }
-        if (kb == num_kb - 1) {
-          umma_commit_pair(&tmem_full[0], 3);
-          umma_commit_pair(&tmem_full[1], 3);
-        }
-#else
-        issue_half(0, kb, st);
-        issue_half(1, kb, st);
-#endif
       };
       for (int w = sc.first; ok && w < sc.end; w += sc.stride) {
         const uint32_t acc_parity = static_cast<uint32_t>(acc_iter & 1);
@@ -513,24 +499,23 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
           int st = stage + i;
           uint32_t ph = phase;
           if (st >= GP_STAGES) { st -= GP_STAGES; ph ^= 1; }
-          if (!mbar_wait(&full[st], ph, abort_flag, p.status, OB_ERR_WAIT_FULL, budget)) { ok = false; break; }
-          if (i == 0 && !mbar_wait(&tmem_empty[0], acc_parity ^ 1, abort_flag, p.status, OB_ERR_WAIT_TMEM_EMPTY, budget)) {
+          if (!mbar_wait_warp(&full[st], ph, abort_flag, p.status, OB_ERR_WAIT_FULL, budget)) { ok = false; break; }
+          if (i == 0 && !mbar_wait_warp(&tmem_empty[0], acc_parity ^ 1, abort_flag, p.status, OB_ERR_WAIT_TMEM_EMPTY, budget)) {
             ok = false;
             break;
           }
           tc_fence_after();
-          issue_half(0, i, st);
+          issue_half(0, i, st, false);
         }
         for (int i = 0; ok && i < lead; ++i) {
           if (i == 0) {
-            if (!mbar_wait(&tmem_empty[1], acc_parity ^ 1, abort_flag, p.status, OB_ERR_WAIT_TMEM_EMPTY, budget)) {
+            if (!mbar_wait_warp(&tmem_empty[1], acc_parity ^ 1, abort_flag, p.status, OB_ERR_WAIT_TMEM_EMPTY, budget)) {
               ok = false;
               break;
             }
             tc_fence_after();
           }
-          issue_half(1, i, stage);
-          umma_commit_pair(&empty[stage], 3);          // frees the stage in both CTAs
+          issue_half(1, i, stage, true);
           if (++stage == GP_STAGES) { stage = 0; phase ^= 1; }
         }
         // tail of the tile, the mirror image: half 0 finishes its last `tail` k-blocks first and is handed to the epilogue
@@ -538,26 +523,25 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         // during the drain of half 0, and the drain of half 1 overlaps the head of the next tile.
         const int tail = num_kb - lead < GP_STAGES ? num_kb - lead : GP_STAGES;
         for (int kb = lead; ok && kb < num_kb - tail; ++kb) {
-          if (!mbar_wait(&full[stage], phase, abort_flag, p.status, OB_ERR_WAIT_FULL, budget)) {
+          if (!mbar_wait_warp(&full[stage], phase, abort_flag, p.status, OB_ERR_WAIT_FULL, budget)) {
             ok = false;
             break;
           }
           tc_fence_after();
-          issue_both(kb, stage);
-          umma_commit_pair(&empty[stage], 3);
+          issue_half(0, kb, stage, false);
+          issue_half(1, kb, stage, true);
           if (++stage == GP_STAGES) { stage = 0; phase ^= 1; }
         }
         for (int i = 0; ok && i < tail; ++i) {
           int st = stage + i;
           uint32_t ph = phase;
           if (st >= GP_STAGES) { st -= GP_STAGES; ph ^= 1; }
-          if (!mbar_wait(&full[st], ph, abort_flag, p.status, OB_ERR_WAIT_FULL, budget)) { ok = false; break; }
+          if (!mbar_wait_warp(&full[st], ph, abort_flag, p.status, OB_ERR_WAIT_FULL, budget)) { ok = false; break; }
           tc_fence_after();
-          issue_half(0, num_kb - tail + i, st);
+          issue_half(0, num_kb - tail + i, st, false);
         }
         for (int i = 0; ok && i < tail; ++i) {
-          issue_half(1, num_kb - tail + i, stage);
-          umma_commit_pair(&empty[stage], 3);
+          issue_half(1, num_kb - tail + i, stage, true);
           if (++stage == GP_STAGES) { stage = 0; phase ^= 1; }
         }
         ++acc_iter;
@@ -846,7 +830,7 @@ gemm_pair_db_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* sched = reinterpret_cast<int*>(tmem_slot + 2);  // [3]: first, end, stride (valid in the leader CTA)
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform(static_cast<int>(threadIdx.x >> 5)), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const bool leader = rank == 0;
   const int tiles_n = (p.N + GP_BN - 1) / GP_BN;
@@ -890,23 +874,23 @@ gemm_pair_db_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   __syncthreads();
   cluster_sync_all();                // both CTAs' barriers are initialised before any remote arrival or copy
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = uniform(*tmem_slot);
   const GpSchedule sc = gp_read_schedule(sched);
 
   if (warp == 0) {
-    if (lane == 0) {
-      // ---------------------------------------------------------------- TMA producer (one per CTA)
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      for (int w = sc.first; ok && w < sc.end; w += sc.stride) {
-        const GpItem it = gd_decode(w, tiles_m, tiles_n, rank);
-        const int bn0 = it.nt * GP_BN + static_cast<int>(rank) * GP_BNH;     // this CTA's half of the B tile
-        for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, p.status, OB_ERR_WAIT_EMPTY, budget)) {
-            ok = false;
-            break;
-          }
+    // ---------------------------------------------------------------- TMA producer (one per CTA)
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int w = sc.first; ok && w < sc.end; w += sc.stride) {
+      const GpItem it = gd_decode(w, tiles_m, tiles_n, rank);
+      const int bn0 = it.nt * GP_BN + static_cast<int>(rank) * GP_BNH;     // this CTA's half of the B tile
+      for (int kb = 0; kb < num_kb; ++kb) {
+        if (!mbar_wait_warp(&empty[stage], phase ^ 1, abort_flag, p.status, OB_ERR_WAIT_EMPTY, budget)) {
+          ok = false;
+          break;
+        }
+        if (elect_one()) {
           if (leader) mbar_expect_tx(&full[stage], 2 * GD_STAGE_BYTES);
           const uint32_t bar = map_to_cta(smem_u32(&full[stage]), 0);
           uint8_t* a_dst = smem + stage * GD_STAGE_BYTES;
@@ -922,50 +906,56 @@ gemm_pair_db_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
           } else {
             tma_load_2d_pair(b_dst, mb, bar, k0, bn0);
           }
-          if (++stage == GD_STAGES) { stage = 0; phase ^= 1; }
         }
+        if (++stage == GD_STAGES) { stage = 0; phase ^= 1; }
       }
     }
   } else if (warp == 1) {
-    if (leader && lane == 0) {
+    if (leader) {
       // ---------------------------------------------------------------- MMA issuer (leader CTA only)
       constexpr uint32_t idesc_k = make_idesc_bf16(2 * GD_BM, GP_BN, 0, 0);
       constexpr uint32_t idesc_n = make_idesc_bf16(2 * GD_BM, GP_BN, 0, 1);
+      const uint32_t ring = smem_u32(smem);
       int stage = 0, acc_iter = 0;
       uint32_t phase = 0;
       bool ok = true;
       for (int w = sc.first; ok && w < sc.end; w += sc.stride) {
         const int as = acc_iter & 1;
-        if (!mbar_wait(&tmem_empty[as], ((acc_iter >> 1) & 1) ^ 1, abort_flag, p.status, OB_ERR_WAIT_TMEM_EMPTY,
+        if (!mbar_wait_warp(&tmem_empty[as], ((acc_iter >> 1) & 1) ^ 1, abort_flag, p.status, OB_ERR_WAIT_TMEM_EMPTY,
                        budget)) {
           ok = false;
           break;
         }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + as * GP_BN;
+        bool ready = false;
         for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait(&full[stage], phase, abort_flag, p.status, OB_ERR_WAIT_FULL, budget)) {
+          if (!ready && !mbar_wait_warp(&full[stage], phase, abort_flag, p.status, OB_ERR_WAIT_FULL, budget)) {
             ok = false;
             break;
           }
           tc_fence_after();
-          const uint32_t a_addr = smem_u32(smem + stage * GD_STAGE_BYTES);
+          const uint32_t a_addr = ring + stage * GD_STAGE_BYTES;
           const uint32_t b_addr = a_addr + GD_A_BYTES;
           const bool kn = kb < nk1 ? p.kn1 != 0 : p.kn2 != 0;
+          // K-major operand: rows 128 B apart, 8-row groups 1024 B apart, 32 B per 16-element k-step.
+          // N-major operand: 64-column blocks GP_BK*128 B apart, 8-row (k) groups 1024 B apart, 2048 B per k-step.
+          const uint64_t ad = make_smem_desc(a_addr, 16, 1024, 2);
+          const uint64_t bd = kn ? make_smem_desc(b_addr, GP_BK * 128, 1024, 2) : make_smem_desc(b_addr, 16, 1024, 2);
+          const uint32_t b_step = kn ? 128u : 2u, idesc = kn ? idesc_n : idesc_k;
+          const int next = stage + 1 == GD_STAGES ? 0 : stage + 1;
+          const bool peek = kb + 1 < num_kb && mbar_test_wait(&full[next], next == 0 ? phase ^ 1 : phase);
+          if (elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < GP_BK / 16; ++kk) {
-            // K-major operand: rows 128 B apart, 8-row groups 1024 B apart, 32 B per 16-element k-step.
-            // N-major operand: 64-column blocks GP_BK*128 B apart, 8-row (k) groups 1024 B apart, 2048 B per k-step.
-            const uint64_t ad = make_smem_desc(a_addr + kk * 32, 16, 1024, 2);
-            const uint64_t bd = kn ? make_smem_desc(b_addr + kk * (16 * 128), GP_BK * 128, 1024, 2)
-                                   : make_smem_desc(b_addr + kk * 32, 16, 1024, 2);
-            umma_bf16_pair(d_tmem, ad, bd, kn ? idesc_n : idesc_k, (kb > 0 || kk > 0) ? 1u : 0u);
+            for (int kk = 0; kk < GP_BK / 16; ++kk)
+              umma_bf16_pair(d_tmem, ad + 2 * kk, bd + kk * b_step, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
+            umma_commit_pair(&empty[stage], 3);          // frees the stage in both CTAs
           }
-          umma_commit_pair(&empty[stage], 3);          // frees the stage in both CTAs
+          ready = __all_sync(0xffffffffu, peek);
           if (++stage == GD_STAGES) { stage = 0; phase ^= 1; }
         }
         if (!ok) break;
-        umma_commit_pair(&tmem_full[as], 3);           // this tile's accumulators (both CTAs) are complete
+        if (elect_one()) umma_commit_pair(&tmem_full[as], 3);           // this tile's accumulators (both CTAs) are complete
         ++acc_iter;
       }
     }

@@ -18,7 +18,7 @@
 //
 // A tile's k-blocks stay on one CTA and are added in order: every tile shape of this kernel and of the pair kernel gives the same
 // bits, so the choice between them (by size alone) never shows in a result.  Few rows make few tiles, and spreading a tile's
-// k-blocks over several CTAs is faster there (256 x 2048 x 8192: 52.0 us and 18.7 with 8 parts), but another order of the sums
+// k-blocks over several CTAs is faster there (256 x 2048 x 8192: 27.3 us and 18.7 with 8 parts), but another order of the sums
 // moves bf16 roundings, and behind twelve layers single gradient sums by more than their root mean square.
 #include "common.cuh"
 #include "api.h"
@@ -32,8 +32,9 @@ constexpr int GT_BM = 128;
 constexpr int GT_BK = 64;
 constexpr int GT_A_BYTES = GT_BM * GT_BK * 2;
 // Tile width: 256 columns, or 64 where the wide tiles leave most SMs idle or N is narrower than that.  A k-block of a lone tile
-// takes about 0.34 us wide and 0.31 narrow, so what a narrow tile saves is its shorter start and epilogue.  Measured (us, wide /
-// narrow): 128 x 768 x 768 9.5 / 7.7, 16384 x 48 x 4096 32.9 / 27.6; 2048 x 768 x 768 9.7 / 12.3 (two waves).
+// takes 512 clocks wide (the tensor pipe's own time) and 285 narrow; 604 both ways while a single thread ran the issue loop.
+// Measured (us, wide / narrow; in brackets with that loop): 128 x 768 x 768 8.9 / 6.1 (9.4 / 7.6), 256 x 2048 x 8192 41.7 / 27.3
+// (46.0 / 44.4); 3663 x 768 x 768 9.4 / 11.4 (two waves).
 template <int BN>
 struct GtTile {
   static constexpr int B_BYTES = BN * GT_BK * 2;
@@ -110,7 +111,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* tile_start = reinterpret_cast<int*>(slabs + 8 * GT_SLAB_BYTES + 256);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform(static_cast<int>(threadIdx.x >> 5)), lane = threadIdx.x & 31;
   const int tiles_n = (p.N + BN - 1) / BN;
   const int nk1 = (p.K1 + GT_BK - 1) / GT_BK;
   const int nk2 = (p.K2 + GT_BK - 1) / GT_BK;
@@ -151,98 +152,100 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
-  const int tiles_m = p.group_offs ? tile_start[p.num_groups] : (p.M + GT_BM - 1) / GT_BM;
+  const uint32_t tmem_base = uniform(*tmem_slot);
+  const int tiles_m = p.group_offs ? uniform(tile_start[p.num_groups]) : (p.M + GT_BM - 1) / GT_BM;
   const int total_work = tiles_m * tiles_n;
 
   if (warp == 0) {
-    if (lane == 0) {
-      int stage = 0, cursor = 0;
-      uint32_t phase = 0, issued_mask = 0, issued_phase = 0;
-      bool ok = true;
-      for (int w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
-        const GtItem it = gt_decode<BN>(p, w, tiles_m, tiles_n, tile_start, cursor);
-        for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, p.status, OB_ERR_WAIT_EMPTY, budget)) {
-            ok = false;
-            break;
-          }
+    int stage = 0, cursor = 0;
+    uint32_t phase = 0, issued_mask = 0, issued_phase = 0;
+    bool ok = true;
+    for (int w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
+      const GtItem it = gt_decode<BN>(p, w, tiles_m, tiles_n, tile_start, cursor);
+      const int row0 = uniform(it.row0), b_row = uniform(it.b_row), n0 = it.n0;
+      for (int kb = 0; kb < num_kb; ++kb) {
+        if (!mbar_wait_warp(&empty[stage], phase ^ 1, abort_flag, p.status, OB_ERR_WAIT_EMPTY, budget)) {
+          ok = false;
+          break;
+        }
+        if (elect_one()) {
           mbar_expect_tx(&full[stage], STAGE_BYTES);
           uint8_t* a_dst = smem + stage * STAGE_BYTES;
           uint8_t* b_dst = a_dst + GT_A_BYTES;
           if (kb < nk1) {
-            tma_load_2d(a_dst, &map_a, &full[stage], kb * GT_BK, it.row0);
+            tma_load_2d(a_dst, &map_a, &full[stage], kb * GT_BK, row0);
             if constexpr (B_KN) {
 #pragma unroll
               for (int j = 0; j < BN / 64; ++j)
-                tma_load_2d(b_dst + j * (GT_BK * 128), &map_b, &full[stage], it.n0 + 64 * j, it.b_row + kb * GT_BK);
+                tma_load_2d(b_dst + j * (GT_BK * 128), &map_b, &full[stage], n0 + 64 * j, b_row + kb * GT_BK);
             } else {
-              tma_load_2d(b_dst, &map_b, &full[stage], kb * GT_BK, it.b_row + it.n0);
+              tma_load_2d(b_dst, &map_b, &full[stage], kb * GT_BK, b_row + n0);
             }
           } else {
-            tma_load_2d(a_dst, &map_a2, &full[stage], (kb - nk1) * GT_BK, it.row0);
+            tma_load_2d(a_dst, &map_a2, &full[stage], (kb - nk1) * GT_BK, row0);
             if (p.b2_kn) {
 #pragma unroll
               for (int j = 0; j < BN / 64; ++j)
-                tma_load_2d(b_dst + j * (GT_BK * 128), &map_b2, &full[stage], it.n0 + 64 * j, (kb - nk1) * GT_BK);
+                tma_load_2d(b_dst + j * (GT_BK * 128), &map_b2, &full[stage], n0 + 64 * j, (kb - nk1) * GT_BK);
             } else {
-              tma_load_2d(b_dst, &map_b2, &full[stage], (kb - nk1) * GT_BK, it.n0);
+              tma_load_2d(b_dst, &map_b2, &full[stage], (kb - nk1) * GT_BK, n0);
             }
           }
-          issued_mask |= 1u << stage;
-          issued_phase = (issued_phase & ~(1u << stage)) | (phase << stage);
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
-      }
-      if (!ok) {
-        for (int s = 0; s < STAGES; ++s)
-          if (issued_mask & (1u << s)) {
-            int dummy_abort = 0;
-            mbar_wait(&full[s], (issued_phase >> s) & 1u, &dummy_abort, p.status, OB_ERR_DRAIN, budget);
-          }
+        issued_mask |= 1u << stage;
+        issued_phase = (issued_phase & ~(1u << stage)) | (phase << stage);
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
     }
+    if (!ok) {
+      for (int s = 0; s < STAGES; ++s)
+        if (issued_mask & (1u << s)) {
+          int dummy_abort = 0;
+          mbar_wait(&full[s], (issued_phase >> s) & 1u, &dummy_abort, p.status, OB_ERR_DRAIN, budget);
+        }
+    }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc_nmaj = make_idesc_bf16(GT_BM, BN, 0, 1);
-      constexpr uint32_t idesc_kmaj = make_idesc_bf16(GT_BM, BN, 0, 0);
-      int stage = 0, acc_iter = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      for (int w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
-        const int as = acc_iter & 1;
-        if (!mbar_wait(&tmem_empty[as], ((acc_iter >> 1) & 1) ^ 1, abort_flag, p.status, OB_ERR_WAIT_TMEM_EMPTY,
-                       budget)) {
+    constexpr uint32_t idesc_nmaj = make_idesc_bf16(GT_BM, BN, 0, 1);
+    constexpr uint32_t idesc_kmaj = make_idesc_bf16(GT_BM, BN, 0, 0);
+    const uint32_t ring = smem_u32(smem);
+    int stage = 0, acc_iter = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
+      const int as = acc_iter & 1;
+      if (!mbar_wait_warp(&tmem_empty[as], ((acc_iter >> 1) & 1) ^ 1, abort_flag, p.status, OB_ERR_WAIT_TMEM_EMPTY, budget)) {
+        ok = false;
+        break;
+      }
+      tc_fence_after();
+      const uint32_t d_tmem = tmem_base + as * BN;
+      bool ready = false;
+      for (int kb = 0; kb < num_kb; ++kb) {
+        if (!ready && !mbar_wait_warp(&full[stage], phase, abort_flag, p.status, OB_ERR_WAIT_FULL, budget)) {
           ok = false;
           break;
         }
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + as * BN;
-        for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait(&full[stage], phase, abort_flag, p.status, OB_ERR_WAIT_FULL, budget)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t a_addr = smem_u32(smem + stage * STAGE_BYTES);
-          const uint32_t b_addr = a_addr + GT_A_BYTES;
-          const bool kn = kb < nk1 ? B_KN : p.b2_kn != 0;
-#pragma unroll
-          for (int kk = 0; kk < GT_BK / 16; ++kk) {
-            // K-major operand: rows 128 B apart, 8-row groups 1024 B apart, 32 B per 16-element k-step.
-            // N-major operand: 64-column blocks GT_BK*128 B apart, 8-row (k) groups 1024 B apart, 2048 B per k-step.
-            const uint64_t ad = make_smem_desc(a_addr + kk * 32, 16, 1024, 2);
-            const uint64_t bd = kn ? make_smem_desc(b_addr + kk * (16 * 128), GT_BK * 128, 1024, 2)
-                                   : make_smem_desc(b_addr + kk * 32, 16, 1024, 2);
-            umma_bf16(d_tmem, ad, bd, kn ? idesc_nmaj : idesc_kmaj, (kb > 0 || kk > 0) ? 1u : 0u);
-          }
-          umma_commit(&empty[stage]);
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
+        // K-major operand: rows 128 B apart, 8-row groups 1024 B apart, 32 B per 16-element k-step.
+        // N-major operand: 64-column blocks GT_BK*128 B apart, 8-row (k) groups 1024 B apart, 2048 B per k-step.
+        const uint32_t a_addr = ring + stage * STAGE_BYTES;
+        const uint32_t b_addr = a_addr + GT_A_BYTES;
+        const uint64_t ad = make_smem_desc(a_addr, 16, 1024, 2);
+        const int next = stage + 1 == STAGES ? 0 : stage + 1;
+        const bool peek = kb + 1 < num_kb && mbar_test_wait(&full[next], next == 0 ? phase ^ 1 : phase);
+        const bool kn = kb < nk1 ? B_KN : p.b2_kn != 0;
+        if (elect_one()) {
+          if (kn)
+            umma_bf16_kblock<2, 128>(d_tmem, ad, make_smem_desc(b_addr, GT_BK * 128, 1024, 2), idesc_nmaj, kb > 0, &empty[stage]);
+          else
+            umma_bf16_kblock<2, 2>(d_tmem, ad, make_smem_desc(b_addr, 16, 1024, 2), idesc_kmaj, kb > 0, &empty[stage]);
         }
-        if (!ok) break;
-        umma_commit(&tmem_full[as]);
-        ++acc_iter;
+        ready = __all_sync(0xffffffffu, peek);
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
+      if (!ok) break;
+      if (elect_one()) umma_commit(&tmem_full[as]);
+      ++acc_iter;
     }
   } else {
     // Eight warps drain one 128 x 256 accumulator: warp w reads TMEM lanes 32 * (w % 4) .. (the lane quarter a warp may

@@ -126,7 +126,7 @@ wgrad_clip_kernel(const __grid_constant__ TmaBatch<WgradParams, CAP> b) {
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 3 * S::STAGES + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform(static_cast<int>(threadIdx.x >> 5)), lane = threadIdx.x & 31;
   const int total_work = b.total();
   const uint64_t budget = b.wait_budget_ns;
 
@@ -152,51 +152,54 @@ wgrad_clip_kernel(const __grid_constant__ TmaBatch<WgradParams, CAP> b) {
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = uniform(*tmem_slot);
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      uint32_t issued_mask = 0, issued_phase = 0;
-      bool ok = true;
-      int cur = 0;
-      for (int w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
-        cur = b.seek(w, cur);
-        const WgradParams& p = b.p[cur];
-        const WorkItem it = decode_work(p, w - b.start[cur], BLOCK_N);
-        for (int kb = 0; kb < it.num_kb; ++kb) {
-          if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, b.status, OB_ERR_WAIT_EMPTY, budget)) {
-            ok = false;
-            break;
-          }
+    int stage = 0;
+    uint32_t phase = 0;
+    uint32_t issued_mask = 0, issued_phase = 0;
+    bool ok = true;
+    int cur = 0;
+    for (int w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
+      cur = b.seek(w, cur);
+      const WgradParams& p = b.p[cur];
+      const WorkItem it = decode_work(p, w - b.start[cur], BLOCK_N);
+      const int num_kb = uniform(it.num_kb), row_begin = uniform(it.row_begin);
+      for (int kb = 0; kb < num_kb; ++kb) {
+        if (!mbar_wait_warp(&empty[stage], phase ^ 1, abort_flag, b.status, OB_ERR_WAIT_EMPTY, budget)) {
+          ok = false;
+          break;
+        }
+        if (elect_one()) {
           mbar_expect_tx(&full[stage], S::STAGE_BYTES);
           uint8_t* a_dst = stage_base + stage * S::STAGE_BYTES;
           uint8_t* b_dst = a_dst + S::A_BYTES;
-          const int row = it.row_begin + kb * WG_BLOCK_K;
+          const int row = row_begin + kb * WG_BLOCK_K;
 #pragma unroll
           for (int j = 0; j < WG_BLOCK_M / 64; ++j)
             tma_load_2d(a_dst + j * (WG_BLOCK_K * 128), &b.map_a[cur], &full[stage], it.m0 + 64 * j, row);
 #pragma unroll
           for (int j = 0; j < BLOCK_N / 64; ++j)
             tma_load_2d(b_dst + j * (WG_BLOCK_K * 128), &b.map_b[cur], &full[stage], it.n0 + 64 * j, row);
-          issued_mask |= 1u << stage;
-          issued_phase = (issued_phase & ~(1u << stage)) | (phase << stage);
-          if (++stage == S::STAGES) { stage = 0; phase ^= 1; }
         }
+        issued_mask |= 1u << stage;
+        issued_phase = (issued_phase & ~(1u << stage)) | (phase << stage);
+        if (++stage == S::STAGES) { stage = 0; phase ^= 1; }
       }
-      if (!ok) {
-        // unwind: let every copy this thread started land before the CTA's shared memory goes away
-        for (int s = 0; s < S::STAGES; ++s)
-          if (issued_mask & (1u << s)) {
-            int dummy_abort = 0;
-            mbar_wait(&full[s], (issued_phase >> s) & 1u, &dummy_abort, b.status, OB_ERR_DRAIN, budget);
-          }
-      }
+    }
+    if (!ok) {
+      // unwind: let every copy this thread started land before the CTA's shared memory goes away
+      for (int s = 0; s < S::STAGES; ++s)
+        if (issued_mask & (1u << s)) {
+          int dummy_abort = 0;
+          mbar_wait(&full[s], (issued_phase >> s) & 1u, &dummy_abort, b.status, OB_ERR_DRAIN, budget);
+        }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
+    // One thread issues here: the MMAs follow the scalers, and issued by the whole warp (four times as fast) they only crowd the
+    // scalers out of shared memory: 8192 x 2048 x 2048 72 us by the warp, 62 by the thread, 60 experts' 32768 x 1408 x 2048 288 and 293.
     if (lane == 0) {
       constexpr uint32_t idesc = make_idesc_bf16(WG_BLOCK_M, BLOCK_N, 1, 1);
       int stage = 0;
@@ -474,7 +477,7 @@ wgrad_clip_pe_kernel(const __grid_constant__ TmaBatch<WgradPeParams, CAP> b) {
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * WP_STAGES + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform(static_cast<int>(threadIdx.x >> 5)), lane = threadIdx.x & 31;
   const int total_work = b.total();
   const uint64_t budget = b.wait_budget_ns;
 
@@ -499,7 +502,7 @@ wgrad_clip_pe_kernel(const __grid_constant__ TmaBatch<WgradPeParams, CAP> b) {
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = uniform(*tmem_slot);
 
   // work item w -> (split, m tile, n tile); split s owns examples [e0, e1)
   auto decode = [](const WgradPeParams& p, int w, int& m0, int& n0, int& e0, int& e1) {
@@ -513,24 +516,24 @@ wgrad_clip_pe_kernel(const __grid_constant__ TmaBatch<WgradPeParams, CAP> b) {
   };
 
   if (warp == 0) {
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0, issued_mask = 0, issued_phase = 0;
-      bool ok = true;
-      int cur = 0;
-      for (int w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
-        cur = b.seek(w, cur);
-        const WgradPeParams& p = b.p[cur];
-        const int kpe = (p.ex_rows + WG_BLOCK_K - 1) / WG_BLOCK_K;
-        int m0, n0, e0, e1;
-        decode(p, w - b.start[cur], m0, n0, e0, e1);
-        const int nkb = (e1 - e0) * kpe;
-        int ex = e0, row = 0;
-        for (int kb = 0; kb < nkb; ++kb) {
-          if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, b.status, OB_ERR_WAIT_EMPTY, budget)) {
-            ok = false;
-            break;
-          }
+    int stage = 0;
+    uint32_t phase = 0, issued_mask = 0, issued_phase = 0;
+    bool ok = true;
+    int cur = 0;
+    for (int w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
+      cur = b.seek(w, cur);
+      const WgradPeParams& p = b.p[cur];
+      const int kpe = (p.ex_rows + WG_BLOCK_K - 1) / WG_BLOCK_K;
+      int m0, n0, e0, e1;
+      decode(p, w - b.start[cur], m0, n0, e0, e1);
+      const int nkb = (e1 - e0) * kpe;
+      int ex = e0, row = 0;
+      for (int kb = 0; kb < nkb; ++kb) {
+        if (!mbar_wait_warp(&empty[stage], phase ^ 1, abort_flag, b.status, OB_ERR_WAIT_EMPTY, budget)) {
+          ok = false;
+          break;
+        }
+        if (elect_one()) {
           mbar_expect_tx(&full[stage], WP_STAGE_BYTES);
           uint8_t* a_dst = smem + stage * WP_STAGE_BYTES;
           uint8_t* b_dst = a_dst + WP_A_BYTES;
@@ -545,62 +548,59 @@ wgrad_clip_pe_kernel(const __grid_constant__ TmaBatch<WgradPeParams, CAP> b) {
             row = 0;
             ++ex;
           }
-          issued_mask |= 1u << stage;
-          issued_phase = (issued_phase & ~(1u << stage)) | (phase << stage);
-          if (++stage == WP_STAGES) { stage = 0; phase ^= 1; }
         }
-      }
-      if (!ok) {
-        for (int s = 0; s < WP_STAGES; ++s)
-          if (issued_mask & (1u << s)) {
-            int dummy_abort = 0;
-            mbar_wait(&full[s], (issued_phase >> s) & 1u, &dummy_abort, b.status, OB_ERR_DRAIN, budget);
-          }
+        issued_mask |= 1u << stage;
+        issued_phase = (issued_phase & ~(1u << stage)) | (phase << stage);
+        if (++stage == WP_STAGES) { stage = 0; phase ^= 1; }
       }
     }
+    if (!ok) {
+      for (int s = 0; s < WP_STAGES; ++s)
+        if (issued_mask & (1u << s)) {
+          int dummy_abort = 0;
+          mbar_wait(&full[s], (issued_phase >> s) & 1u, &dummy_abort, b.status, OB_ERR_DRAIN, budget);
+        }
+    }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc_bf16(WG_BLOCK_M, WP_BLOCK_N, 1, 1);
-      int stage = 0, acc_iter = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      int cur = 0;
-      for (int w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
-        cur = b.seek(w, cur);
-        const WgradPeParams& p = b.p[cur];
-        const int kpe = (p.ex_rows + WG_BLOCK_K - 1) / WG_BLOCK_K;
-        int m0, n0, e0, e1;
-        decode(p, w - b.start[cur], m0, n0, e0, e1);
-        for (int e = e0; ok && e < e1; ++e) {
-          const int as = acc_iter & 1;
-          if (!mbar_wait(&tmem_empty[as], ((acc_iter >> 1) & 1) ^ 1, abort_flag, b.status, OB_ERR_WAIT_TMEM_EMPTY,
-                         budget)) {
+    constexpr uint32_t idesc = make_idesc_bf16(WG_BLOCK_M, WP_BLOCK_N, 1, 1);
+    const uint32_t ring = smem_u32(smem);
+    int stage = 0, acc_iter = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    int cur = 0;
+    for (int w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
+      cur = b.seek(w, cur);
+      const WgradPeParams& p = b.p[cur];
+      const int kpe = (p.ex_rows + WG_BLOCK_K - 1) / WG_BLOCK_K;
+      int m0, n0, e0, e1;
+      decode(p, w - b.start[cur], m0, n0, e0, e1);
+      for (int e = e0; ok && e < e1; ++e) {
+        const int as = acc_iter & 1;
+        if (!mbar_wait_warp(&tmem_empty[as], ((acc_iter >> 1) & 1) ^ 1, abort_flag, b.status, OB_ERR_WAIT_TMEM_EMPTY, budget)) {
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        const uint32_t d_tmem = tmem_base + as * WP_BLOCK_N;
+        bool ready = false;
+        for (int kb = 0; kb < kpe; ++kb) {
+          if (!ready && !mbar_wait_warp(&full[stage], phase, abort_flag, b.status, OB_ERR_WAIT_FULL, budget)) {
             ok = false;
             break;
           }
           tc_fence_after();
-          const uint32_t d_tmem = tmem_base + as * WP_BLOCK_N;
-          for (int kb = 0; kb < kpe; ++kb) {
-            if (!mbar_wait(&full[stage], phase, abort_flag, b.status, OB_ERR_WAIT_FULL, budget)) {
-              ok = false;
-              break;
-            }
-            tc_fence_after();
-            const uint32_t a_addr = smem_u32(smem + stage * WP_STAGE_BYTES);
-            const uint32_t b_addr = a_addr + WP_A_BYTES;
-#pragma unroll
-            for (int kk = 0; kk < WG_BLOCK_K / WG_UMMA_K; ++kk) {
-              const uint64_t ad = make_smem_desc(a_addr + kk * (WG_UMMA_K * 128), WG_BLOCK_K * 128, 1024, 2);
-              const uint64_t bd = make_smem_desc(b_addr + kk * (WG_UMMA_K * 128), WG_BLOCK_K * 128, 1024, 2);
-              umma_bf16(d_tmem, ad, bd, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
-            }
-            umma_commit(&empty[stage]);
-            if (++stage == WP_STAGES) { stage = 0; phase ^= 1; }
-          }
-          if (!ok) break;
-          umma_commit(&tmem_full[as]);
-          ++acc_iter;
+          const uint32_t a_addr = ring + stage * WP_STAGE_BYTES;
+          const uint64_t ad = make_smem_desc(a_addr, WG_BLOCK_K * 128, 1024, 2);
+          const uint64_t bd = make_smem_desc(a_addr + WP_A_BYTES, WG_BLOCK_K * 128, 1024, 2);
+          const int next = stage + 1 == WP_STAGES ? 0 : stage + 1;
+          const bool peek = kb + 1 < kpe && mbar_test_wait(&full[next], next == 0 ? phase ^ 1 : phase);
+          if (elect_one()) umma_bf16_kblock<128, 128>(d_tmem, ad, bd, idesc, kb > 0, &empty[stage]);
+          ready = __all_sync(0xffffffffu, peek);
+          if (++stage == WP_STAGES) { stage = 0; phase ^= 1; }
         }
+        if (!ok) break;
+        if (elect_one()) umma_commit(&tmem_full[as]);
+        ++acc_iter;
       }
     }
   } else {
