@@ -386,16 +386,25 @@ def _check_b(b: torch.Tensor, layout: str, K: int, what: str) -> int:
     return b.shape[1] if kn else b.shape[0]
 
 
+_PAIR_TILES = {"auto": -1, "512x256": 0, "256x256": 1}
+
+
+def _pair_tile(tile: str) -> int:
+    if tile not in _PAIR_TILES:
+        raise ValueError("tile must be '512x256', '256x256' or 'auto'")
+    return _PAIR_TILES[tile]
+
+
 def gemm_pair(a: torch.Tensor, b: torch.Tensor, *, b_layout: str = "nk", a2: torch.Tensor | None = None,
               b2: torch.Tensor | None = None, b2_layout: str = "nk", bias: torch.Tensor | None = None,
               out: torch.Tensor | None = None, status: StatusWord | None = None,
-              wait_budget_s: float = DEFAULT_WAIT_BUDGET_S, tile: str = "512x256") -> torch.Tensor:
+              wait_budget_s: float = DEFAULT_WAIT_BUDGET_S, tile: str = "auto") -> torch.Tensor:
     """``a @ op(b) + a2 @ op(b2) + bias`` on CTA pairs (``tcgen05 … cta_group::2``; bf16 in/out, fp32 accumulation).
 
     Layouts as in :func:`gemm`; the second segment has its own layout, so ``dX = dG·Wg + dU·Wu`` (both weights
     stored ``[K, N]`` from the product's point of view) and the LoRA data gradient ``dY·W + q·A`` are one launch each.
-    ``tile``: ``"512x256"`` (one tile fills tensor memory; fewest operand bytes per FLOP, for long K) or ``"256x256"``
-    (two accumulators alternate, so a tile drains during the whole main loop of the next; for short K).
+    ``tile``: ``"512x256"`` (one tile fills tensor memory; fewest operand bytes per FLOP), ``"256x256"`` (two accumulators
+    alternate, so a tile drains during the whole main loop of the next) or ``"auto"`` (by size); the same bits either way.
     """
     _need_bf16(a, b)
     if a.ndim != 2 or a.stride(1) != 1:
@@ -418,20 +427,10 @@ def gemm_pair(a: torch.Tensor, b: torch.Tensor, *, b_layout: str = "nk", a2: tor
         out = torch.empty(M, N, dtype=torch.bfloat16, device=a.device)
     elif out.shape != (M, N) or out.dtype != torch.bfloat16 or out.stride(1) != 1:
         raise ValueError("out must be a row-major bf16 [M, N] matrix")
-    if tile == "256x256":
-        rc = lib.load().ob_gemm_pair_db(
-            a.data_ptr(), b.data_ptr(), lib.ptr(a2), lib.ptr(b2), lib.ptr(bias), out.data_ptr(),
-            M, N, K, K2, a.stride(0), b.stride(0), a2.stride(0) if a2 is not None else 0,
-            b2.stride(0) if b2 is not None else 0, out.stride(0), int(b_layout == "kn"), int(b2_layout == "kn"),
-            status.ptr() if status else None, wait_budget_s, lib.sm_count(), lib.stream())
-        lib.check(rc, "gemm_pair (256x256)")
-        return out
-    if tile != "512x256":
-        raise ValueError("tile must be '512x256' or '256x256'")
     rc = lib.load().ob_gemm_pair(
         a.data_ptr(), b.data_ptr(), None, lib.ptr(a2), lib.ptr(b2), None, lib.ptr(bias), out.data_ptr(), None, None,
         M, N, K, K2, a.stride(0), b.stride(0), a2.stride(0) if a2 is not None else 0,
-        b2.stride(0) if b2 is not None else 0, out.stride(0), int(b_layout == "kn"), int(b2_layout == "kn"), 0, 0,
+        b2.stride(0) if b2 is not None else 0, out.stride(0), int(b_layout == "kn"), int(b2_layout == "kn"), 0, 0, _pair_tile(tile),
         status.ptr() if status else None, wait_budget_s, lib.sm_count(), lib.stream())
     lib.check(rc, "gemm_pair")
     return out
@@ -498,7 +497,7 @@ def gemm_glu(a: torch.Tensor, w_gate: torch.Tensor, w_up: torch.Tensor, *, act: 
     u = torch.empty_like(h) if save_preact else None
     rc = lib.load().ob_gemm_pair(
         a.data_ptr(), w_gate.data_ptr(), w_up.data_ptr(), None, None, None, None, h.data_ptr(), lib.ptr(g), lib.ptr(u),
-        M, 2 * inter, K, 0, a.stride(0), w_gate.stride(0), 0, 0, h.stride(0), 0, 0, 1, _GLU_ACT[act],
+        M, 2 * inter, K, 0, a.stride(0), w_gate.stride(0), 0, 0, h.stride(0), 0, 0, 1, _GLU_ACT[act], -1,
         status.ptr() if status else None, wait_budget_s, lib.sm_count(), lib.stream())
     lib.check(rc, "gemm_glu")
     return h, g, u
@@ -589,7 +588,8 @@ def linear_ce_dlogits_(logits: torch.Tensor, labels: torch.Tensor, lse: torch.Te
 
 
 def pick_gemm_kernel(M: int, N: int, K: int, sms: int = 148) -> str:
-    """``"pair"`` or ``"single"`` for an ungrouped ``[M, K] x [K, N]`` product.
+    """``"pair"`` or ``"single"`` between the 512 x 256 pair tile and the single-CTA kernel (:func:`gemm` asks :func:`pick_gemm_plan`,
+    which knows the smaller pair tile).
 
     The pair kernel (512 x 256 output tiles on SM pairs, half the operand bytes per FLOP) wins on large products; its
     tiles are coarse, so a product with few tiles or a short K leaves SM pairs idle in the last wave or pays the
@@ -606,22 +606,32 @@ def pick_gemm_kernel(M: int, N: int, K: int, sms: int = 148) -> str:
     return "pair" if eff_pair >= eff_single else "single"
 
 
+def _waves_us(tiles: int, slots: int, nk: int, start: float, per_kb: float, per_busy: float, per_tile: float) -> float:
+    """``start`` plus, for every wave of ``tiles`` over ``slots``, ``nk`` k-blocks (dearer the more slots are busy) and a tile's own cost."""
+    full, rest = divmod(tiles, slots)
+    us = start + full * (nk * (per_kb + per_busy * slots) + per_tile)
+    return us + (nk * (per_kb + per_busy * rest) + per_tile if rest else 0.0)
+
+
 def _single_us(M: int, N: int, nk: int, width: int, sms: int) -> float:
     """Estimated microseconds of the single-CTA kernel along ``nk`` k-blocks, tiles ``width`` columns wide.
 
-    Fitted to launches back to back in a CUDA graph with weights from HBM: over 41 shapes of 1 to 16384 rows the width with the
-    smaller estimate was the faster one every time."""
-    ctas = -(-M // 128) * -(-N // width)
-    waves, busy = -(-ctas // sms), min(ctas, sms)
-    start, per_kb = (5.2, 0.346 + 0.0011 * busy) if width == 256 else (3.9, 0.298 + 0.00036 * busy)
-    return start + per_kb * nk * waves
+    This and :func:`_pair_us` are fitted to launches back to back in a CUDA graph with weights from HBM: over 238 shapes of 1 to 16384
+    rows the kernel and width with the smallest estimate took 0.25 % longer than the best one on average (4.6 % at most from 64 rows on)."""
+    tiles = -(-M // 128) * -(-N // width)
+    return _waves_us(tiles, sms, nk, *((3.95, 0.3506, 0.00026, 0.96) if width == 256 else (4.07, 0.1804, 0.00012, 0.12)))
+
+
+def _pair_us(M: int, N: int, nk: int, sms: int) -> float:
+    """The same for CTA pairs on 256 x 256 tiles."""
+    return _waves_us(-(-M // 256) * -(-N // 256), max(sms // 2, 1), nk, 5.80, 0.2715, 0.00103, 0.64)
 
 
 @functools.lru_cache(maxsize=4096)
 def pick_tile_width(M: int, N: int, nk: int, sms: int = 148) -> int:
     """Columns per tile of the single-CTA kernel: 64 where one such tile covers ``N`` (16384 x 48 x 4096: 27.6 us, 32.9 with 256),
-    or where all narrow tiles run at once and are faster by :func:`_single_us` (128 x 768 x 768: 7.7 and 9.5); beyond one wave they
-    lose (2048 x 768 x 768: 12.3 and 9.7)."""
+    or where all narrow tiles run at once and are faster by :func:`_single_us` (128 x 768 x 768: 6.1 and 8.6; 128 x 2048 x 8192: 28.5
+    and 51.7); beyond one wave they lose (3663 x 768 x 768: 11.3 and 9.3)."""
     if N <= 64:
         return 64
     fits = -(-M // 128) * -(-N // 64) <= sms
@@ -632,16 +642,11 @@ def pick_tile_width(M: int, N: int, nk: int, sms: int = 148) -> int:
 def pick_gemm_plan(M: int, N: int, K: int, K2: int = 0, sms: int = 148) -> str:
     """``"pair"`` or ``"single"`` for an ungrouped ``[M, K] x [K, N]`` product (plus a ``K2`` segment): the same bits either way.
 
-    :func:`pick_gemm_kernel`'s choice; where a pair's tiles do not fill the chip once, the two are weighed by estimated
-    microseconds: a pair takes 6.6 + 0.567 per k-block (256 x 2048 x 8192: 79.5 measured), the single-CTA kernel
-    :func:`_single_us` at the better tile width (52.0).
+    The one with the smaller estimate of :func:`_pair_us` and :func:`_single_us` at the better tile width (256 x 2048 x 8192: 42.1 and
+    27.3 us measured; 3663 x 3072 x 768: 18.7 and 20.5; 3663 x 768 x 768: 10.3 and 9.3; 8192 x 4096 x 4096: 167 and 182).
     """
-    if pick_gemm_kernel(M, N, K, sms) == "single":
-        return "single"
     nk = -(-K // 64) + -(-K2 // 64)
-    if -(-M // 512) * -(-N // 256) >= max(sms // 2, 1):
-        return "pair"
-    return "pair" if 6.6 + 0.567 * nk < _single_us(M, N, nk, pick_tile_width(M, N, nk, sms), sms) else "single"
+    return "pair" if _pair_us(M, N, nk, sms) <= _single_us(M, N, nk, pick_tile_width(M, N, nk, sms), sms) else "single"
 
 
 def gemm(a: torch.Tensor, b: torch.Tensor, *, b_layout: str = "nk", a2: torch.Tensor | None = None,
@@ -655,7 +660,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, b_layout: str = "nk", a2: torch.Te
     (``op(b) = b`` — data gradients ``dY @ W`` without a transposed copy).  ``a2 [M, r]``, ``b2 [N, r]`` add a
     low-rank segment accumulated in the same tile (LoRA-fused linear).  With ``group_offs`` (int32 ``[E + 1]`` row
     offsets, rows sorted by group) ``b`` is ``[E, N, K]`` / ``[E, K, N]`` and rows of group e use slab e (MoE experts).
-    ``kernel``: ``"pair"`` (two CTAs per 512 x 256 tile), ``"single"`` (one CTA per 128 x ``block_n`` tile, 256 or 64
+    ``kernel``: ``"pair"`` (two CTAs per tile, :func:`gemm_pair`), ``"single"`` (one CTA per 128 x ``block_n`` tile, 256 or 64
     columns, by default :func:`pick_tile_width`'s choice) or ``"auto"`` (:func:`pick_gemm_plan` for ungrouped products while
     :data:`PAIR_GEMM` is on; grouped products always run on single CTAs).  ``b2_layout="kn"``: ``b2`` is stored ``[r, N]``.  ``alpha`` scales the fp32 products (not the bias;
     single-CTA kernel only, so ``"auto"`` takes it when ``alpha`` is given).

@@ -7,8 +7,8 @@
 // (cluster rank 0) issues `tcgen05.mma.cta_group::2` (M = 256 across the pair) over both CTAs' shared memory, twice per
 // k-step: once for each 128-row half of a CTA's A tile, each half with its own 256-column accumulator in that CTA's tensor
 // memory.  Per k-block an SM stages 48 KB for 2 x (128 x 256 x 64) of tensor work: half the bytes per FLOP of a single-CTA
-// 128 x 256 tile.  Measured need for it: with 32 KB per (128 x 256 x 64) the tensor pipe was 81 % busy at 11.4 TB/s of
-// L2-to-SM traffic, whatever the number of stages.
+// 128 x 256 tile, which pays under the power cap once K is long (see pair_small_tile).  All other products, and the activation
+// and cross-entropy epilogues, run on the 256 x 256 tiles of gemm_pair_db_kernel below.
 //
 // Protocol (every wait bounded; a timeout records a code in the status word and the kernel unwinds):
 //   * full[s]  (leader only, 1 arrival + 96 KB of transactions): the leader's producer arms it for both CTAs' bytes;
@@ -357,6 +357,203 @@ __device__ __forceinline__ void ce_fold64(const uint32_t* pk, int nc, int N, int
 }
 
 template <int EPI>
+__device__ __forceinline__ bool pair_vec_ok(const PairParams& p) {
+  return ((p.ldo & 7) == 0) && ((reinterpret_cast<uintptr_t>(p.out) & 15) == 0) &&
+         (EPI != GP_EPI_GLU || p.out_gate == nullptr ||
+          (((reinterpret_cast<uintptr_t>(p.out_gate) | reinterpret_cast<uintptr_t>(p.out_up)) & 15) == 0)) &&
+         (EPI != GP_EPI_GLUBWD || (reinterpret_cast<uintptr_t>(p.out_up) & 15) == 0);
+}
+
+// Epilogue of one 128 x 256 accumulator per CTA, by one of the eight epilogue warps: TMEM lanes 32 * (warp % 4) .., column group g.
+// `t_row`: the accumulator's tensor-memory address with this warp's lanes, `row`: this lane's row of the output, `nt`: tile index
+// along N.  `release` hands the accumulator back to the MMA issuer; every form calls it once, when it has READ the accumulator.
+template <int EPI, class Release>
+__device__ __forceinline__ void pair_epilogue(const PairParams& p, const CUtensorMap& map_out, const CUtensorMap& map_out_gate,
+                                              const CUtensorMap& map_out_up, uint8_t* slab, uint32_t t_row, int row, int nt,
+                                              int tiles_n, int g, int lane, bool vec_ok, Release release) {
+  if constexpr (EPI == GP_EPI_STORE) {
+    // Both 64-column rounds of this warp's share go to registers (packed bf16) first, so the accumulator half is
+    // back with the tensor pipe before a single store is issued; the stores then overlap the next MMAs.
+    const int n0 = nt * GP_BN + g * (GP_BN / 2);
+    const int row0w = row - lane;
+    uint32_t pk[2][32];
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const int nc = n0 + c * 64;
+      if (nc < p.N) {
+        float v[64];
+        tmem_ld32(t_row + g * (GP_BN / 2) + c * 64, v);
+        tmem_ld32(t_row + g * (GP_BN / 2) + c * 64 + 32, v + 32);
+        tmem_ld_wait();
+        if (p.bias != nullptr) add_bias64(v, p.bias, nc, p.N);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) pk[c][j] = pack_bf16x2(v[2 * j], v[2 * j + 1]);
+      }
+    }
+    release();
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const int nc = n0 + c * 64;
+      if (nc < p.N)
+        store_tile64_packed(slab, pk[c], &map_out, p.tma_store != 0, nc, row0w, p.out, p.ldo, p.M - row0w, p.N - nc,
+                            vec_ok, lane);
+    }
+  } else if constexpr (EPI == GP_EPI_CE) {
+    // Output head: the logits tile never leaves the SM unless `out` asks for it.  Each thread owns one row and folds
+    // its 128 columns of the tile into (max, sum exp, label logit, plain sum); the partials (two per tile and row)
+    // are combined per row in a fixed order by lce_combine_kernel, so the result does not depend on which CTA ran
+    // which tile.
+    const int n0 = nt * GP_BN + g * (GP_BN / 2);
+    const long long label = row < p.M ? p.labels[row] : -1;
+    const int lab = (label >= 0 && label < p.N) ? static_cast<int>(label) : -(1 << 30);     // never matches a column
+    float m = -INFINITY, ssum = 0.f, zlab = 0.f, ztot = 0.f;
+    if (p.out != nullptr) {
+      // Training: the logits are stored (bf16) for the backward pass, and the statistics are taken from the stored,
+      // rounded values.  So the accumulator is read, soft-capped and packed to bf16 first and handed back; the
+      // exponentials and the stores then run beside the next tile's MMAs (with K = 768 the drain of a tile is
+      // otherwise longer than its main loop).
+      const int row0w = row - lane;
+      uint32_t pk[2][32];
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const int nc = n0 + c * 64;
+        if (nc < p.N) {
+          float v[64];
+          tmem_ld32(t_row + g * (GP_BN / 2) + c * 64, v);
+          tmem_ld32(t_row + g * (GP_BN / 2) + c * 64 + 32, v + 32);
+          tmem_ld_wait();
+          if (p.softcap > 0.f) {
+#pragma unroll
+            for (int j = 0; j < 64; ++j) v[j] = p.softcap * tanhf(v[j] / p.softcap);
+          }
+#pragma unroll
+          for (int j = 0; j < 32; ++j) pk[c][j] = pack_bf16x2(v[2 * j], v[2 * j + 1]);
+        }
+      }
+      release();
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const int nc = n0 + c * 64;
+        if (nc < p.N) {
+          if (nc + 64 <= p.N) ce_fold64<true>(pk[c], nc, p.N, lab, m, ssum, zlab, ztot);
+          else ce_fold64<false>(pk[c], nc, p.N, lab, m, ssum, zlab, ztot);
+          store_tile64_packed(slab, pk[c], &map_out, p.tma_store != 0, nc, row0w, p.out, p.ldo, p.M - row0w, p.N - nc,
+                              vec_ok, lane);
+        }
+      }
+    } else {
+      // Forward only (evaluation, reference log-probabilities): fp32 statistics, nothing stored.
+#pragma unroll 1
+      for (int c = 0; c < GP_BN / 2 / 32; ++c) {
+        const int nc = n0 + c * 32;
+        if (nc >= p.N) break;
+        float v[32];
+        tmem_ld32(t_row + g * (GP_BN / 2) + c * 32, v);
+        tmem_ld_wait();
+        if (p.softcap > 0.f) {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] = p.softcap * tanhf(v[j] / p.softcap);
+        }
+        float lm = -INFINITY;
+        const int d = lab - nc;
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+          const bool in = nc + j < p.N;
+          const float z = v[j];
+          v[j] = in ? z : -INFINITY;
+          if (in) {
+            ztot += z;
+            lm = fmaxf(lm, z);
+          }
+          if (d == j) zlab = z;
+        }
+        if (lm > m) {
+          ssum *= __expf(m - lm);
+          m = lm;
+        }
+#pragma unroll
+        for (int j = 0; j < 32; ++j) ssum += __expf(v[j] - m);      // exp(-inf) = 0 for masked columns
+      }
+      release();
+    }
+    if (row < p.M)
+      p.ce_partials[static_cast<long long>(row) * (2 * tiles_n) + 2 * nt + g] = make_float4(m, ssum, zlab, ztot);
+  } else if constexpr (EPI == GP_EPI_GLUBWD) {
+    // Data gradient of the down projection with the gated activation's backward in the epilogue: the tile is dH;
+    // it is read, rounded to bf16 and packed, the accumulator half goes back, and the row's gate / up
+    // pre-activations turn it into dGate and dUp tiles, which leave through the slab.  N % 64 == 0 (host-checked).
+    const int n0 = nt * GP_BN + g * (GP_BN / 2);
+    const int row0w = row - lane;
+    uint32_t pd[2][32];
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const int nc = n0 + c * 64;
+      if (nc < p.N) {
+        float v[64];
+        tmem_ld32(t_row + g * (GP_BN / 2) + c * 64, v);
+        tmem_ld32(t_row + g * (GP_BN / 2) + c * 64 + 32, v + 32);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 32; ++j) pd[c][j] = pack_bf16x2(v[2 * j], v[2 * j + 1]);
+      }
+    }
+    release();
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const int nc = n0 + c * 64;
+      if (nc < p.N) {
+        const bool in_row = row < p.M;
+        const __nv_bfloat16* grow = p.glu_g + static_cast<long long>(row) * p.ld_gu + nc;
+        const __nv_bfloat16* urow = p.glu_u + static_cast<long long>(row) * p.ld_gu + nc;
+        uint32_t og[32], ou[32];
+        if (p.act == 0) gp_glu_bwd64<0>(pd[c], grow, urow, in_row, og, ou);
+        else if (p.act == 1) gp_glu_bwd64<1>(pd[c], grow, urow, in_row, og, ou);
+        else gp_glu_bwd64<2>(pd[c], grow, urow, in_row, og, ou);
+        const bool tma = p.tma_store != 0;
+        store_tile64_packed(slab, og, &map_out, tma, nc, row0w, p.out, p.ldo, p.M - row0w, p.N - nc, vec_ok, lane);
+        store_tile64_packed(slab, ou, &map_out_up, tma, nc, row0w, p.out_up, p.ldo, p.M - row0w, p.N - nc, vec_ok, lane);
+      }
+    }
+  } else {
+    // GLU: this warp's 64 columns of h come from 64 gate and 64 up columns of the same rows.  Everything is read
+    // and packed first (four rounds of 16 + 16 columns), the accumulator half is released, then up to three
+    // [32 x 64] tiles (gate, up, h) leave through the slab.
+    const int nh = p.N / 2;
+    const int n0 = nt * GP_BNH + g * (GP_BNH / 2);
+    const int row0w = row - lane;
+    uint32_t pkg[32], pku[32];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {            // 16 + 16 columns per round: few fp32 registers in flight
+      if (n0 + c * 16 < nh) {
+        float gt[16], up[16];
+        tmem_ld16(t_row + g * (GP_BNH / 2) + c * 16, gt);
+        tmem_ld16(t_row + GP_BNH + g * (GP_BNH / 2) + c * 16, up);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          pkg[8 * c + j] = pack_bf16x2(gt[2 * j], gt[2 * j + 1]);
+          pku[8 * c + j] = pack_bf16x2(up[2 * j], up[2 * j + 1]);
+        }
+      }
+    }
+    release();
+    // h is formed from the ROUNDED pre-activations (what the backward pass reads when they are stored), after the
+    // accumulator has gone back (the activation needs no tensor memory) and in place, to keep registers free
+    if (n0 < nh) {
+      const bool tma = p.tma_store != 0;
+      if (p.out_gate != nullptr) {
+        store_tile64_packed(slab, pkg, &map_out_gate, tma, n0, row0w, p.out_gate, p.ldo, p.M - row0w, nh - n0, vec_ok, lane);
+        store_tile64_packed(slab, pku, &map_out_up, tma, n0, row0w, p.out_up, p.ldo, p.M - row0w, nh - n0, vec_ok, lane);
+      }
+      if (p.act == 0) gp_glu_inplace<0>(pkg, pku);
+      else if (p.act == 1) gp_glu_inplace<1>(pkg, pku);
+      else gp_glu_inplace<2>(pkg, pku);
+      store_tile64_packed(slab, pkg, &map_out, tma, n0, row0w, p.out, p.ldo, p.M - row0w, nh - n0, vec_ok, lane);
+    }
+  }
+}
+
+template <int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                  const __grid_constant__ CUtensorMap map_b_up, const __grid_constant__ CUtensorMap map_a2,
@@ -557,10 +754,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     uint8_t* slab = slabs + (warp - 2) * GP_SLAB_BYTES;
     int acc_iter = 0;
     bool ok = true;
-    const bool vec_ok = ((p.ldo & 7) == 0) && ((reinterpret_cast<uintptr_t>(p.out) & 15) == 0) &&
-                        (EPI != GP_EPI_GLU || p.out_gate == nullptr ||
-                         (((reinterpret_cast<uintptr_t>(p.out_gate) | reinterpret_cast<uintptr_t>(p.out_up)) & 15) == 0)) &&
-                        (EPI != GP_EPI_GLUBWD || (reinterpret_cast<uintptr_t>(p.out_up) & 15) == 0);
+    const bool vec_ok = pair_vec_ok<EPI>(p);
     for (int w = sc.first; ok && w < sc.end; w += sc.stride) {
       const GpItem it = gp_decode(w, tiles_m, tiles_n, rank, p.group_m);
       auto release_half = [&](int hh) {          // this warp is done READING accumulator half hh
@@ -580,186 +774,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         tc_fence_after();
         const int row = it.row0 + h * GP_MMA_M + q * 32 + lane;
         const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + h * GP_BN;
-        if constexpr (EPI == GP_EPI_STORE) {
-          // Both 64-column rounds of this warp's share go to registers (packed bf16) first, so the accumulator half is
-          // back with the tensor pipe before a single store is issued; the stores then overlap the next MMAs.
-          const int n0 = it.nt * GP_BN + g * (GP_BN / 2);
-          const int row0w = row - lane;
-          uint32_t pk[2][32];
-#pragma unroll
-          for (int c = 0; c < 2; ++c) {
-            const int nc = n0 + c * 64;
-            if (nc < p.N) {
-              float v[64];
-              tmem_ld32(t_row + g * (GP_BN / 2) + c * 64, v);
-              tmem_ld32(t_row + g * (GP_BN / 2) + c * 64 + 32, v + 32);
-              tmem_ld_wait();
-              if (p.bias != nullptr) add_bias64(v, p.bias, nc, p.N);
-#pragma unroll
-              for (int j = 0; j < 32; ++j) pk[c][j] = pack_bf16x2(v[2 * j], v[2 * j + 1]);
-            }
-          }
-          release_half(h);
-#pragma unroll
-          for (int c = 0; c < 2; ++c) {
-            const int nc = n0 + c * 64;
-            if (nc < p.N)
-              store_tile64_packed(slab, pk[c], &map_out, p.tma_store != 0, nc, row0w, p.out, p.ldo, p.M - row0w, p.N - nc,
-                                  vec_ok, lane);
-          }
-        } else if constexpr (EPI == GP_EPI_CE) {
-          // Output head: the logits tile never leaves the SM unless `out` asks for it.  Each thread owns one row and folds
-          // its 128 columns of the tile into (max, sum exp, label logit, plain sum); the partials (two per tile and row)
-          // are combined per row in a fixed order by lce_combine_kernel, so the result does not depend on which CTA ran
-          // which tile.
-          const int n0 = it.nt * GP_BN + g * (GP_BN / 2);
-          const long long label = row < p.M ? p.labels[row] : -1;
-          const int lab = (label >= 0 && label < p.N) ? static_cast<int>(label) : -(1 << 30);     // never matches a column
-          float m = -INFINITY, ssum = 0.f, zlab = 0.f, ztot = 0.f;
-          if (p.out != nullptr) {
-            // Training: the logits are stored (bf16) for the backward pass, and the statistics are taken from the stored,
-            // rounded values.  So the accumulator is read, soft-capped and packed to bf16 first and handed back; the
-            // exponentials and the stores then run beside the next tile's MMAs (with K = 768 the drain of a tile is
-            // otherwise longer than its main loop).
-            const int row0w = row - lane;
-            uint32_t pk[2][32];
-#pragma unroll
-            for (int c = 0; c < 2; ++c) {
-              const int nc = n0 + c * 64;
-              if (nc < p.N) {
-                float v[64];
-                tmem_ld32(t_row + g * (GP_BN / 2) + c * 64, v);
-                tmem_ld32(t_row + g * (GP_BN / 2) + c * 64 + 32, v + 32);
-                tmem_ld_wait();
-                if (p.softcap > 0.f) {
-#pragma unroll
-                  for (int j = 0; j < 64; ++j) v[j] = p.softcap * tanhf(v[j] / p.softcap);
-                }
-#pragma unroll
-                for (int j = 0; j < 32; ++j) pk[c][j] = pack_bf16x2(v[2 * j], v[2 * j + 1]);
-              }
-            }
-            release_half(h);
-#pragma unroll
-            for (int c = 0; c < 2; ++c) {
-              const int nc = n0 + c * 64;
-              if (nc < p.N) {
-                if (nc + 64 <= p.N) ce_fold64<true>(pk[c], nc, p.N, lab, m, ssum, zlab, ztot);
-                else ce_fold64<false>(pk[c], nc, p.N, lab, m, ssum, zlab, ztot);
-                store_tile64_packed(slab, pk[c], &map_out, p.tma_store != 0, nc, row0w, p.out, p.ldo, p.M - row0w, p.N - nc,
-                                    vec_ok, lane);
-              }
-            }
-          } else {
-            // Forward only (evaluation, reference log-probabilities): fp32 statistics, nothing stored.
-#pragma unroll 1
-            for (int c = 0; c < GP_BN / 2 / 32; ++c) {
-              const int nc = n0 + c * 32;
-              if (nc >= p.N) break;
-              float v[32];
-              tmem_ld32(t_row + g * (GP_BN / 2) + c * 32, v);
-              tmem_ld_wait();
-              if (p.softcap > 0.f) {
-#pragma unroll
-                for (int j = 0; j < 32; ++j) v[j] = p.softcap * tanhf(v[j] / p.softcap);
-              }
-              float lm = -INFINITY;
-              const int d = lab - nc;
-#pragma unroll
-              for (int j = 0; j < 32; ++j) {
-                const bool in = nc + j < p.N;
-                const float z = v[j];
-                v[j] = in ? z : -INFINITY;
-                if (in) {
-                  ztot += z;
-                  lm = fmaxf(lm, z);
-                }
-                if (d == j) zlab = z;
-              }
-              if (lm > m) {
-                ssum *= __expf(m - lm);
-                m = lm;
-              }
-#pragma unroll
-              for (int j = 0; j < 32; ++j) ssum += __expf(v[j] - m);      // exp(-inf) = 0 for masked columns
-            }
-            release_half(h);
-          }
-          if (row < p.M)
-            p.ce_partials[static_cast<long long>(row) * (2 * tiles_n) + 2 * it.nt + g] = make_float4(m, ssum, zlab, ztot);
-        } else if constexpr (EPI == GP_EPI_GLUBWD) {
-          // Data gradient of the down projection with the gated activation's backward in the epilogue: the tile is dH;
-          // it is read, rounded to bf16 and packed, the accumulator half goes back, and the row's gate / up
-          // pre-activations turn it into dGate and dUp tiles, which leave through the slab.  N % 64 == 0 (host-checked).
-          const int n0 = it.nt * GP_BN + g * (GP_BN / 2);
-          const int row0w = row - lane;
-          uint32_t pd[2][32];
-#pragma unroll
-          for (int c = 0; c < 2; ++c) {
-            const int nc = n0 + c * 64;
-            if (nc < p.N) {
-              float v[64];
-              tmem_ld32(t_row + g * (GP_BN / 2) + c * 64, v);
-              tmem_ld32(t_row + g * (GP_BN / 2) + c * 64 + 32, v + 32);
-              tmem_ld_wait();
-#pragma unroll
-              for (int j = 0; j < 32; ++j) pd[c][j] = pack_bf16x2(v[2 * j], v[2 * j + 1]);
-            }
-          }
-          release_half(h);
-#pragma unroll
-          for (int c = 0; c < 2; ++c) {
-            const int nc = n0 + c * 64;
-            if (nc < p.N) {
-              const bool in_row = row < p.M;
-              const __nv_bfloat16* grow = p.glu_g + static_cast<long long>(row) * p.ld_gu + nc;
-              const __nv_bfloat16* urow = p.glu_u + static_cast<long long>(row) * p.ld_gu + nc;
-              uint32_t og[32], ou[32];
-              if (p.act == 0) gp_glu_bwd64<0>(pd[c], grow, urow, in_row, og, ou);
-              else if (p.act == 1) gp_glu_bwd64<1>(pd[c], grow, urow, in_row, og, ou);
-              else gp_glu_bwd64<2>(pd[c], grow, urow, in_row, og, ou);
-              const bool tma = p.tma_store != 0;
-              store_tile64_packed(slab, og, &map_out, tma, nc, row0w, p.out, p.ldo, p.M - row0w, p.N - nc, vec_ok, lane);
-              store_tile64_packed(slab, ou, &map_out_up, tma, nc, row0w, p.out_up, p.ldo, p.M - row0w, p.N - nc, vec_ok, lane);
-            }
-          }
-        } else {
-          // GLU: this warp's 64 columns of h come from 64 gate and 64 up columns of the same rows.  Everything is read
-          // and packed first (four rounds of 16 + 16 columns), the accumulator half is released, then up to three
-          // [32 x 64] tiles (gate, up, h) leave through the slab.
-          const int nh = p.N / 2;
-          const int n0 = it.nt * GP_BNH + g * (GP_BNH / 2);
-          const int row0w = row - lane;
-          uint32_t pkg[32], pku[32];
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {            // 16 + 16 columns per round: few fp32 registers in flight
-            if (n0 + c * 16 < nh) {
-              float gt[16], up[16];
-              tmem_ld16(t_row + g * (GP_BNH / 2) + c * 16, gt);
-              tmem_ld16(t_row + GP_BNH + g * (GP_BNH / 2) + c * 16, up);
-              tmem_ld_wait();
-#pragma unroll
-              for (int j = 0; j < 8; ++j) {
-                pkg[8 * c + j] = pack_bf16x2(gt[2 * j], gt[2 * j + 1]);
-                pku[8 * c + j] = pack_bf16x2(up[2 * j], up[2 * j + 1]);
-              }
-            }
-          }
-          release_half(h);
-          // h is formed from the ROUNDED pre-activations (what the backward pass reads when they are stored), after the
-          // accumulator has gone back (the activation needs no tensor memory) and in place, to keep registers free
-          if (n0 < nh) {
-            const bool tma = p.tma_store != 0;
-            if (p.out_gate != nullptr) {
-              store_tile64_packed(slab, pkg, &map_out_gate, tma, n0, row0w, p.out_gate, p.ldo, p.M - row0w, nh - n0, vec_ok, lane);
-              store_tile64_packed(slab, pku, &map_out_up, tma, n0, row0w, p.out_up, p.ldo, p.M - row0w, nh - n0, vec_ok, lane);
-            }
-            if (p.act == 0) gp_glu_inplace<0>(pkg, pku);
-            else if (p.act == 1) gp_glu_inplace<1>(pkg, pku);
-            else gp_glu_inplace<2>(pkg, pku);
-            store_tile64_packed(slab, pkg, &map_out, tma, n0, row0w, p.out, p.ldo, p.M - row0w, nh - n0, vec_ok, lane);
-          }
-        }
+        pair_epilogue<EPI>(p, map_out, map_out_gate, map_out_up, slab, t_row, row, it.nt, tiles_n, g, lane, vec_ok, [&] { release_half(h); });
       }
       ++acc_iter;
     }
@@ -785,15 +800,16 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 }
 
 // ------------------------------------------------------------------------------------------------------------------
-// Short-K variant: 256 x 256 pair tiles with DOUBLE-BUFFERED accumulators.
+// 256 x 256 pair tiles with DOUBLE-BUFFERED accumulators: most products, and every activation and cross-entropy epilogue.
 //
 // The 512 x 256 kernel above fills tensor memory with one tile, so its drain hides only behind the first k-blocks of the
 // next tile; with K = 768 (GPT-2's projections: 12 k-blocks) the drain is as long as the main loop and every SM pair
 // stores at the same moment.  Here each CTA owns 128 rows and one 128 x 256 accumulator per tile (256 TMEM columns),
 // two of them alternate, and the eight epilogue warps drain tile i during the whole main loop of tile i + 1.  A stage
 // is 32 KB per CTA (128 rows of A, 128 columns' worth of B) for 128 x 256 x 64 of work: 64 bytes per tensor clock,
-// against 96 for the single-CTA 128 x 256 tile and 48 for the 512 x 256 pair tile.  Plain store epilogue (+ bias,
-// + second K segment) only.  Same barrier protocol and unwind rules as gemm_pair_kernel.
+// against 96 for the single-CTA 128 x 256 tile and 48 for the 512 x 256 pair tile.  It runs at the tensor pipe's rate: 8192 x 4096 x
+// 4096 in 167 us, 1.64 PFLOP/s, the library's own burst rate (big tile 182; 186 while one thread ran the issue loop).  Same
+// epilogues, barrier protocol and unwind rules as gemm_pair_kernel.
 constexpr int GD_BM = 128;                              // rows of M per CTA (256 per pair)
 constexpr int GD_STAGES = 6;
 constexpr int GD_A_BYTES = GD_BM * GP_BK * 2;
@@ -814,10 +830,13 @@ __device__ __forceinline__ GpItem gd_decode(int w, int tiles_m, int tiles_n, int
   return it;
 }
 
+template <int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
 gemm_pair_db_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                    const __grid_constant__ CUtensorMap map_a2, const __grid_constant__ CUtensorMap map_b2,
-                    const __grid_constant__ CUtensorMap map_out, const PairParams p) {
+                    const __grid_constant__ CUtensorMap map_b_up, const __grid_constant__ CUtensorMap map_a2,
+                    const __grid_constant__ CUtensorMap map_b2, const __grid_constant__ CUtensorMap map_b2_up,
+                    const __grid_constant__ CUtensorMap map_out, const __grid_constant__ CUtensorMap map_out_gate,
+                    const __grid_constant__ CUtensorMap map_out_up, const PairParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* slabs = smem + GD_STAGES * GD_STAGE_BYTES;
@@ -833,7 +852,7 @@ gemm_pair_db_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   const int warp = uniform(static_cast<int>(threadIdx.x >> 5)), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const bool leader = rank == 0;
-  const int tiles_n = (p.N + GP_BN - 1) / GP_BN;
+  const int tiles_n = EPI == GP_EPI_GLU ? (p.N / 2 + GP_BNH - 1) / GP_BNH : (p.N + GP_BN - 1) / GP_BN;
   const int tiles_m = (p.M + 2 * GD_BM - 1) / (2 * GD_BM);
   const int total_work = tiles_m * tiles_n;
   const int nk1 = (p.K1 + GP_BK - 1) / GP_BK;
@@ -854,10 +873,10 @@ gemm_pair_db_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&map_a);
-    tma_prefetch_desc(&map_b);
+    tma_prefetch_desc(rank == 1 && EPI == GP_EPI_GLU ? &map_b_up : &map_b);
     if (nk2) {
       tma_prefetch_desc(&map_a2);
-      tma_prefetch_desc(&map_b2);
+      tma_prefetch_desc(rank == 1 && EPI == GP_EPI_GLU ? &map_b2_up : &map_b2);
     }
   }
   if (warp == 1) {                   // one warp of EACH CTA takes part in a pair allocation
@@ -882,9 +901,12 @@ gemm_pair_db_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
+    const CUtensorMap* mb1 = (EPI == GP_EPI_GLU && rank == 1) ? &map_b_up : &map_b;
+    const CUtensorMap* mb2 = (EPI == GP_EPI_GLU && rank == 1) ? &map_b2_up : &map_b2;
     for (int w = sc.first; ok && w < sc.end; w += sc.stride) {
       const GpItem it = gd_decode(w, tiles_m, tiles_n, rank);
-      const int bn0 = it.nt * GP_BN + static_cast<int>(rank) * GP_BNH;     // this CTA's half of the B tile
+      // this CTA's half of the B tile: its columns of N, or with GLU the gate (rank 0) or up (rank 1) columns
+      const int bn0 = EPI == GP_EPI_GLU ? it.nt * GP_BNH : it.nt * GP_BN + static_cast<int>(rank) * GP_BNH;
       for (int kb = 0; kb < num_kb; ++kb) {
         if (!mbar_wait_warp(&empty[stage], phase ^ 1, abort_flag, p.status, OB_ERR_WAIT_EMPTY, budget)) {
           ok = false;
@@ -898,7 +920,7 @@ gemm_pair_db_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
           const bool first = kb < nk1;
           const int k0 = (first ? kb : kb - nk1) * GP_BK;
           tma_load_2d_pair(a_dst, first ? &map_a : &map_a2, bar, k0, it.row0);
-          const CUtensorMap* mb = first ? &map_b : &map_b2;
+          const CUtensorMap* mb = first ? mb1 : mb2;
           if (first ? p.kn1 : p.kn2) {
 #pragma unroll
             for (int j = 0; j < GP_BNH / 64; ++j)
@@ -966,7 +988,7 @@ gemm_pair_db_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     uint8_t* slab = slabs + (warp - 2) * GP_SLAB_BYTES;
     int acc_iter = 0;
     bool ok = true;
-    const bool vec_ok = ((p.ldo & 7) == 0) && ((reinterpret_cast<uintptr_t>(p.out) & 15) == 0);
+    const bool vec_ok = pair_vec_ok<EPI>(p);
     for (int w = sc.first; ok && w < sc.end; w += sc.stride) {
       const GpItem it = gd_decode(w, tiles_m, tiles_n, rank);
       const int as = acc_iter & 1;
@@ -975,35 +997,15 @@ gemm_pair_db_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         break;
       }
       tc_fence_after();
-      const int row0 = it.row0 + q * 32;
-      const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + as * GP_BN + g * (GP_BN / 2);
-      uint32_t pk[2][32];                    // both rounds in registers, then the accumulator goes back (see above)
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        const int nc = it.nt * GP_BN + g * (GP_BN / 2) + c * 64;
-        if (nc < p.N) {
-          float v[64];
-          tmem_ld32(t_row + c * 64, v);
-          tmem_ld32(t_row + c * 64 + 32, v + 32);
-          tmem_ld_wait();
-          if (p.bias != nullptr) add_bias64(v, p.bias, nc, p.N);
-#pragma unroll
-          for (int j = 0; j < 32; ++j) pk[c][j] = pack_bf16x2(v[2 * j], v[2 * j + 1]);
+      const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + as * GP_BN;
+      pair_epilogue<EPI>(p, map_out, map_out_gate, map_out_up, slab, t_row, it.row0 + q * 32 + lane, it.nt, tiles_n, g, lane, vec_ok, [&] {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+          if (leader) mbar_arrive(&tmem_empty[as]);
+          else mbar_arrive_cluster(map_to_cta(smem_u32(&tmem_empty[as]), 0));
         }
-      }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) {
-        if (leader) mbar_arrive(&tmem_empty[as]);
-        else mbar_arrive_cluster(map_to_cta(smem_u32(&tmem_empty[as]), 0));
-      }
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        const int nc = it.nt * GP_BN + g * (GP_BN / 2) + c * 64;
-        if (nc < p.N)
-          store_tile64_packed(slab, pk[c], &map_out, p.tma_store != 0, nc, row0, p.out, p.ldo, p.M - row0, p.N - nc, vec_ok,
-                              lane);
-      }
+      });
       ++acc_iter;
     }
     if (lane == 0) tma_store_wait_all();
@@ -1248,14 +1250,61 @@ extern "C" int ob_die_map(unsigned char* out, int n) {
   return dm.sms;
 }
 
+namespace ob {
+// tensor maps of one launch
+struct PairMaps {
+  CUtensorMap a, b, b_up, a2, b2, b2_up, out, out_gate, out_up;
+};
+
+// Tile of a plain product [rows, K] x [K, cols]: 256 x 256, or 512 x 256 where K is long.  A wave of the small tiles reads
+// (16 + 74 / 16) * 256 rows of K values; from K = 5632 on that no longer stays in one die's half of the L2 and the big tile's fewer
+// bytes per FLOP win (power-capped loops, TFLOP/s, big / small: 16384 x 4096 x 4096 1365 / 1368, 16384 x 4096 x 6144 1387 / 1336,
+// 16384 x 4096 x 14336 1422 / 1346), unless its coarser tiles leave more of the last wave empty (5439 x 2048 x 8192 1022 / 1141,
+// 8192 x 4096 x 14336, 7 waves for 2 x 4, 1333 / 1343).
+static bool pair_small_tile(long long rows, long long cols, long long K, int clusters) {
+  if (K <= 4096) return true;
+  const long long tn = (cols + GP_BN - 1) / GP_BN;
+  const long long big = (rows + 2 * GP_BM - 1) / (2 * GP_BM) * tn, small = (rows + 2 * GD_BM - 1) / (2 * GD_BM) * tn;
+  const long long waves_big = (big + clusters - 1) / clusters, waves_small = (small + clusters - 1) / clusters;
+  return 10 * waves_small <= 9 * 2 * waves_big;
+}
+
+// The activation and cross-entropy epilogues always take the small tile (power-capped loops against the big one: gate + up + SwiGLU
+// 16384 x 4096 x 14336 2.87 -> 2.80 ms, 5439 x 2048 x 8192 0.312 -> 0.291; head + statistics 8192 x 2048 x 128256 3.42 -> 3.19 ms with
+// the logits stored, 3.48 -> 3.00 without; 3663 x 768 x 50304 0.332 -> 0.305), the GLU backward, longer than either tile's main
+// loop, the big one.
+template <int EPI>
+static int pair_launch(bool small, const PairMaps& m, PairParams& p, int num_sms, cudaStream_t st) {
+  using Kernel = decltype(&gemm_pair_db_kernel<GP_EPI_STORE>);
+  Kernel kernel;
+  if constexpr (EPI == GP_EPI_STORE) kernel = small ? gemm_pair_db_kernel<EPI> : gemm_pair_kernel<EPI>;
+  else if constexpr (EPI == GP_EPI_GLUBWD) kernel = gemm_pair_kernel<EPI>;
+  else kernel = gemm_pair_db_kernel<EPI>;
+  const int smem = small ? GD_SMEM : GP_SMEM;
+  static int max_clusters[2] = {0, 0};
+  if (max_clusters[small] == 0) {
+    if (cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -54;
+    max_clusters[small] = pair_grid(reinterpret_cast<const void*>(kernel), num_sms, smem);
+  }
+  const int rows_tile = small ? 2 * GD_BM : 2 * GP_BM;
+  const long long tiles_n = EPI == GP_EPI_GLU ? (p.N / 2 + GP_BNH - 1) / GP_BNH : (p.N + GP_BN - 1) / GP_BN;
+  const long long total = (static_cast<long long>(p.M) + rows_tile - 1) / rows_tile * tiles_n;
+  const int clusters = static_cast<int>(total < max_clusters[small] ? total : max_clusters[small]);
+  pair_set_schedule(&p, total, clusters, st);
+  kernel<<<2 * clusters, GP_THREADS, smem, st>>>(m.a, m.b, m.b_up, m.a2, m.b2, m.b2_up, m.out, m.out_gate, m.out_up, p);
+  return cudaGetLastError() == cudaSuccess ? 0 : -55;
+}
+}  // namespace ob
+
 // D = A op1(B) + A2 op2(B2) + bias on CTA pairs.  b_kn / b2_kn = 1: that operand is stored [K, N].
 // glu != 0: `b` holds the gate rows and `b_up` the up rows ([N/2, K] each, or [K, N/2] with b_kn); N counts gate and up
 // columns together; out [M, N/2] = act(gate) * up, and out_gate / out_up (optional, both or none) receive the
 // pre-activations.  glu_act: 0 silu, 1 gelu erf, 2 gelu tanh.  With a second segment in GLU mode b2 / b2_up likewise.
+// tile (without glu): 1 = 256 x 256, 0 = 512 x 256, -1 = pair_small_tile's choice (the same bits either way).
 extern "C" int ob_gemm_pair(const void* a, const void* b, const void* b_up, const void* a2, const void* b2,
                             const void* b2_up, const void* bias, void* out, void* out_gate, void* out_up,
                             long long rows_a, int N, int K1, int K2, long long lda, long long ldb, long long lda2,
-                            long long ldb2, long long ldo, int b_kn, int b2_kn, int glu, int glu_act, int* status,
+                            long long ldb2, long long ldo, int b_kn, int b2_kn, int glu, int glu_act, int tile, int* status,
                             double wait_budget_s, int num_sms, void* stream) {
   using namespace ob;
   if (rows_a <= 0 || N <= 0 || K1 <= 0) return 0;
@@ -1264,45 +1313,37 @@ extern "C" int ob_gemm_pair(const void* a, const void* b, const void* b_up, cons
   if (glu && (b_up == nullptr || (N & 1) || (K2 > 0 && b2_up == nullptr) || bias != nullptr)) return -52;
   if (glu && ((out_gate == nullptr) != (out_up == nullptr))) return -53;
   const int nb = glu ? N / 2 : N;               // columns of N covered by ONE B operand
-  CUtensorMap ma, mb, mbu, ma2, mb2, mb2u;
-  int rc = make_bf16_map_2d(&ma, a, rows_a, K1, lda, GP_BK, GP_BM);
+  const bool small = glu || (tile < 0 ? pair_small_tile(rows_a, N, static_cast<long long>(K1) + K2, num_sms / 2) : tile != 0);
+  const int box_rows = small ? GD_BM : GP_BM;
+  PairMaps m;
+  int rc = make_bf16_map_2d(&m.a, a, rows_a, K1, lda, GP_BK, box_rows);
   if (rc) return rc;
-  auto b_map = [&](CUtensorMap* m, const void* base, int K, long long ld, int kn) {
-    return kn ? make_bf16_map_2d(m, base, K, nb, ld, 64, GP_BK) : make_bf16_map_2d(m, base, nb, K, ld, GP_BK, GP_BNH);
+  auto b_map = [&](CUtensorMap* map, const void* base, int K, long long ld, int kn) {
+    return kn ? make_bf16_map_2d(map, base, K, nb, ld, 64, GP_BK) : make_bf16_map_2d(map, base, nb, K, ld, GP_BK, GP_BNH);
   };
-  rc = b_map(&mb, b, K1, ldb, b_kn);
+  rc = b_map(&m.b, b, K1, ldb, b_kn);
   if (rc) return rc;
   if (glu) {
-    rc = b_map(&mbu, b_up, K1, ldb, b_kn);
+    rc = b_map(&m.b_up, b_up, K1, ldb, b_kn);
     if (rc) return rc;
   } else {
-    mbu = mb;
+    m.b_up = m.b;
   }
   if (K2 > 0) {
-    rc = make_bf16_map_2d(&ma2, a2, rows_a, K2, lda2, GP_BK, GP_BM);
+    rc = make_bf16_map_2d(&m.a2, a2, rows_a, K2, lda2, GP_BK, box_rows);
     if (rc) return rc;
-    rc = b_map(&mb2, b2, K2, ldb2, b2_kn);
+    rc = b_map(&m.b2, b2, K2, ldb2, b2_kn);
     if (rc) return rc;
     if (glu) {
-      rc = b_map(&mb2u, b2_up, K2, ldb2, b2_kn);
+      rc = b_map(&m.b2_up, b2_up, K2, ldb2, b2_kn);
       if (rc) return rc;
     } else {
-      mb2u = mb2;
+      m.b2_up = m.b2;
     }
   } else {
-    ma2 = ma;
-    mb2 = mb;
-    mb2u = mbu;
-  }
-  static bool configured = false;
-  static int clusters_store = 0, clusters_glu = 0;
-  if (!configured) {
-    if (cudaFuncSetAttribute(gemm_pair_kernel<GP_EPI_STORE>, cudaFuncAttributeMaxDynamicSharedMemorySize, GP_SMEM) != cudaSuccess ||
-        cudaFuncSetAttribute(gemm_pair_kernel<GP_EPI_GLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, GP_SMEM) != cudaSuccess)
-      return -54;
-    clusters_store = pair_grid(reinterpret_cast<const void*>(gemm_pair_kernel<GP_EPI_STORE>), num_sms);
-    clusters_glu = pair_grid(reinterpret_cast<const void*>(gemm_pair_kernel<GP_EPI_GLU>), num_sms);
-    configured = true;
+    m.a2 = m.a;
+    m.b2 = m.b;
+    m.b2_up = m.b_up;
   }
   PairParams p = {};
   p.group_m = pair_group_m();
@@ -1317,22 +1358,12 @@ extern "C" int ob_gemm_pair(const void* a, const void* b, const void* b_up, cons
   p.act = glu_act;
   p.status = status;
   p.wait_budget_ns = static_cast<unsigned long long>(wait_budget_s * 1e9);
-  const long long tiles_m = (rows_a + 2 * GP_BM - 1) / (2 * GP_BM);
-  const long long tiles_n = glu ? (nb + GP_BNH - 1) / GP_BNH : (N + GP_BN - 1) / GP_BN;
-  const long long total = tiles_m * tiles_n;
-  const int avail = glu ? clusters_glu : clusters_store;
-  const int clusters = static_cast<int>(total < avail ? total : avail);
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  pair_set_schedule(&p, total, clusters, st);
-  CUtensorMap mo = ma, mog = ma, mou = ma;
-  p.tma_store = pair_out_map(&mo, out, rows_a, nb, ldo) ? 1 : 0;          // nb: the width of the output (N / 2 for GLU)
+  m.out = m.out_gate = m.out_up = m.a;
+  p.tma_store = pair_out_map(&m.out, out, rows_a, nb, ldo) ? 1 : 0;          // nb: the width of the output (N / 2 for GLU)
   if (glu && out_gate != nullptr && p.tma_store)
-    p.tma_store = (pair_out_map(&mog, out_gate, rows_a, nb, ldo) && pair_out_map(&mou, out_up, rows_a, nb, ldo)) ? 1 : 0;
-  if (glu)
-    gemm_pair_kernel<GP_EPI_GLU><<<2 * clusters, GP_THREADS, GP_SMEM, st>>>(ma, mb, mbu, ma2, mb2, mb2u, mo, mog, mou, p);
-  else
-    gemm_pair_kernel<GP_EPI_STORE><<<2 * clusters, GP_THREADS, GP_SMEM, st>>>(ma, mb, mbu, ma2, mb2, mb2u, mo, mog, mou, p);
-  return cudaGetLastError() == cudaSuccess ? 0 : -55;
+    p.tma_store = (pair_out_map(&m.out_gate, out_gate, rows_a, nb, ldo) && pair_out_map(&m.out_up, out_up, rows_a, nb, ldo)) ? 1 : 0;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  return glu ? pair_launch<GP_EPI_GLU>(true, m, p, num_sms, st) : pair_launch<GP_EPI_STORE>(small, m, p, num_sms, st);
 }
 
 // Data gradient of a gated MLP's down projection fused with the activation's backward:
@@ -1349,19 +1380,13 @@ extern "C" int ob_gemm_pair_glu_bwd(const void* dy, const void* w, const void* g
   if (gate == nullptr || up == nullptr || dgate == nullptr || dup == nullptr) return -57;
   auto al = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
   if ((N & 63) != 0 || (ld_gu & 7) != 0 || (ld_out & 7) != 0 || !al(gate) || !al(up) || !al(dgate) || !al(dup)) return -58;
-  CUtensorMap ma, mb;
-  int rc = make_bf16_map_2d(&ma, dy, rows_a, K, lddy, GP_BK, GP_BM);
+  PairMaps m;
+  int rc = make_bf16_map_2d(&m.a, dy, rows_a, K, lddy, GP_BK, GP_BM);
   if (rc) return rc;
-  rc = b_kn ? make_bf16_map_2d(&mb, w, K, N, ldw, 64, GP_BK) : make_bf16_map_2d(&mb, w, N, K, ldw, GP_BK, GP_BNH);
+  rc = b_kn ? make_bf16_map_2d(&m.b, w, K, N, ldw, 64, GP_BK) : make_bf16_map_2d(&m.b, w, N, K, ldw, GP_BK, GP_BNH);
   if (rc) return rc;
-  static bool configured = false;
-  static int clusters_gb = 0;
-  if (!configured) {
-    if (cudaFuncSetAttribute(gemm_pair_kernel<GP_EPI_GLUBWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, GP_SMEM) != cudaSuccess)
-      return -54;
-    clusters_gb = pair_grid(reinterpret_cast<const void*>(gemm_pair_kernel<GP_EPI_GLUBWD>), num_sms);
-    configured = true;
-  }
+  m.b_up = m.b2 = m.b2_up = m.b;
+  m.a2 = m.out = m.out_gate = m.out_up = m.a;
   PairParams p = {};
   p.group_m = pair_group_m();
   p.M = static_cast<int>(rows_a);
@@ -1376,72 +1401,42 @@ extern "C" int ob_gemm_pair_glu_bwd(const void* dy, const void* w, const void* g
   p.act = glu_act;
   p.status = status;
   p.wait_budget_ns = static_cast<unsigned long long>(wait_budget_s * 1e9);
-  const long long total = ((rows_a + 2 * GP_BM - 1) / (2 * GP_BM)) * ((N + GP_BN - 1) / GP_BN);
-  const int clusters = static_cast<int>(total < clusters_gb ? total : clusters_gb);
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  pair_set_schedule(&p, total, clusters, st);
-  CUtensorMap mog = ma, mou = ma;
-  p.tma_store = (pair_out_map(&mog, dgate, rows_a, N, ld_out) && pair_out_map(&mou, dup, rows_a, N, ld_out)) ? 1 : 0;
-  gemm_pair_kernel<GP_EPI_GLUBWD><<<2 * clusters, GP_THREADS, GP_SMEM, st>>>(ma, mb, mb, ma, mb, mb, mog, ma, mou, p);
-  return cudaGetLastError() == cudaSuccess ? 0 : -55;
-}
-
-// The double-buffered 256 x 256 pair-tile kernel (plain store epilogue); arguments as in ob_gemm_pair.
-extern "C" int ob_gemm_pair_db(const void* a, const void* b, const void* a2, const void* b2, const void* bias, void* out,
-                               long long rows_a, int N, int K1, int K2, long long lda, long long ldb, long long lda2,
-                               long long ldb2, long long ldo, int b_kn, int b2_kn, int* status, double wait_budget_s,
-                               int num_sms, void* stream) {
-  using namespace ob;
-  if (rows_a <= 0 || N <= 0 || K1 <= 0) return 0;
-  if (rows_a > 0x7fffffffLL - 2 * GD_BM) return -50;
-  if (K2 > 0 && (a2 == nullptr || b2 == nullptr)) return -51;
-  CUtensorMap ma, mb, ma2, mb2;
-  int rc = make_bf16_map_2d(&ma, a, rows_a, K1, lda, GP_BK, GD_BM);
-  if (rc) return rc;
-  auto b_map = [&](CUtensorMap* m, const void* base, int K, long long ld, int kn) {
-    return kn ? make_bf16_map_2d(m, base, K, N, ld, 64, GP_BK) : make_bf16_map_2d(m, base, N, K, ld, GP_BK, GP_BNH);
-  };
-  rc = b_map(&mb, b, K1, ldb, b_kn);
-  if (rc) return rc;
-  if (K2 > 0) {
-    rc = make_bf16_map_2d(&ma2, a2, rows_a, K2, lda2, GP_BK, GD_BM);
-    if (rc) return rc;
-    rc = b_map(&mb2, b2, K2, ldb2, b2_kn);
-    if (rc) return rc;
-  } else {
-    ma2 = ma;
-    mb2 = mb;
-  }
-  static bool configured = false;
-  static int clusters_db = 0;
-  if (!configured) {
-    if (cudaFuncSetAttribute(gemm_pair_db_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GD_SMEM) != cudaSuccess)
-      return -54;
-    clusters_db = pair_grid(reinterpret_cast<const void*>(gemm_pair_db_kernel), num_sms, GD_SMEM);
-    configured = true;
-  }
-  PairParams p = {};
-  p.M = static_cast<int>(rows_a);
-  p.N = N; p.K1 = K1; p.K2 = K2;
-  p.kn1 = b_kn; p.kn2 = b2_kn;
-  p.out = static_cast<__nv_bfloat16*>(out);
-  p.ldo = ldo;
-  p.bias = static_cast<const __nv_bfloat16*>(bias);
-  p.status = status;
-  p.wait_budget_ns = static_cast<unsigned long long>(wait_budget_s * 1e9);
-  const long long total = ((rows_a + 2 * GD_BM - 1) / (2 * GD_BM)) * ((N + GP_BN - 1) / GP_BN);
-  const int clusters = static_cast<int>(total < clusters_db ? total : clusters_db);
-  pair_set_schedule(&p, total, clusters, static_cast<cudaStream_t>(stream));
-  CUtensorMap mo = ma;
-  p.tma_store = pair_out_map(&mo, out, rows_a, N, ldo) ? 1 : 0;
-  gemm_pair_db_kernel<<<2 * clusters, GP_THREADS, GD_SMEM, static_cast<cudaStream_t>(stream)>>>(ma, mb, ma2, mb2, mo, p);
-  return cudaGetLastError() == cudaSuccess ? 0 : -55;
+  p.tma_store = (pair_out_map(&m.out, dgate, rows_a, N, ld_out) && pair_out_map(&m.out_up, dup, rows_a, N, ld_out)) ? 1 : 0;
+  return pair_launch<GP_EPI_GLUBWD>(false, m, p, num_sms, static_cast<cudaStream_t>(stream));
 }
 
 // Bit patterns of the descriptors the tensor-core kernels build, for host-side checks.
 extern "C" unsigned int ob_debug_idesc_bf16(int m, int n, int a_mn_major, int b_mn_major) {
   return ob::make_idesc_bf16(m, n, a_mn_major, b_mn_major);
 }
+
+namespace ob {
+// The product and its per-tile statistics; `logits_out` may be null.
+static int ce_forward(const void* hidden, const void* weight, const long long* labels, void* logits_out, float4* partials, long long rows,
+                      int N, int K, long long ldh, long long ldw, long long ldo, float softcap, int* status,
+                      double wait_budget_s, int num_sms, cudaStream_t st) {
+  PairMaps m;
+  int rc = make_bf16_map_2d(&m.a, hidden, rows, K, ldh, GP_BK, GD_BM);
+  if (rc) return rc;
+  rc = make_bf16_map_2d(&m.b, weight, N, K, ldw, GP_BK, GP_BNH);
+  if (rc) return rc;
+  m.b_up = m.b2 = m.b2_up = m.b;
+  m.a2 = m.out = m.out_gate = m.out_up = m.a;
+  PairParams p = {};
+  p.group_m = pair_group_m();
+  p.M = static_cast<int>(rows);
+  p.N = N; p.K1 = K; p.K2 = 0;
+  p.out = static_cast<__nv_bfloat16*>(logits_out);
+  p.ldo = ldo;
+  p.labels = labels;
+  p.ce_partials = partials;
+  p.softcap = softcap;
+  p.status = status;
+  p.wait_budget_ns = static_cast<unsigned long long>(wait_budget_s * 1e9);
+  p.tma_store = (logits_out != nullptr && pair_out_map(&m.out, logits_out, rows, N, ldo)) ? 1 : 0;
+  return pair_launch<GP_EPI_CE>(true, m, p, num_sms, st);
+}
+}  // namespace ob
 
 // Output head fused with the cross-entropy statistics:  logits = hidden[M, K] * weight[N, K]^T on CTA pairs; the epilogue
 // folds every 128-column half of a logits tile into per-row partials (scratch `partials`: M * 2 * ceil(N / 256) float4) and a second
@@ -1456,40 +1451,11 @@ extern "C" int ob_linear_ce_fwd(const void* hidden, const void* weight, const lo
   if (rows <= 0 || N <= 0 || K <= 0) return 0;
   if (rows > 0x7fffffffLL - 2 * GP_BM) return -50;
   if (labels == nullptr || partials == nullptr || nll == nullptr) return -56;
-  CUtensorMap ma, mb;
-  int rc = make_bf16_map_2d(&ma, hidden, rows, K, ldh, GP_BK, GP_BM);
-  if (rc) return rc;
-  rc = make_bf16_map_2d(&mb, weight, N, K, ldw, GP_BK, GP_BNH);
-  if (rc) return rc;
-  static bool configured = false;
-  static int clusters_ce = 0;
-  if (!configured) {
-    if (cudaFuncSetAttribute(gemm_pair_kernel<GP_EPI_CE>, cudaFuncAttributeMaxDynamicSharedMemorySize, GP_SMEM) != cudaSuccess)
-      return -54;
-    clusters_ce = pair_grid(reinterpret_cast<const void*>(gemm_pair_kernel<GP_EPI_CE>), num_sms);
-    configured = true;
-  }
-  PairParams p = {};
-  p.group_m = pair_group_m();
-  p.M = static_cast<int>(rows);
-  p.N = N; p.K1 = K; p.K2 = 0;
-  p.out = static_cast<__nv_bfloat16*>(logits_out);
-  p.ldo = ldo;
-  p.labels = labels;
-  p.ce_partials = reinterpret_cast<float4*>(partials);
-  p.softcap = softcap;
-  p.status = status;
-  p.wait_budget_ns = static_cast<unsigned long long>(wait_budget_s * 1e9);
-  const long long tiles_m = (rows + 2 * GP_BM - 1) / (2 * GP_BM);
   const int tiles_n = (N + GP_BN - 1) / GP_BN;
-  const long long total = tiles_m * tiles_n;
-  const int clusters = static_cast<int>(total < clusters_ce ? total : clusters_ce);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  pair_set_schedule(&p, total, clusters, st);
-  CUtensorMap mo = ma;
-  p.tma_store = (logits_out != nullptr && pair_out_map(&mo, logits_out, rows, N, ldo)) ? 1 : 0;
-  gemm_pair_kernel<GP_EPI_CE><<<2 * clusters, GP_THREADS, GP_SMEM, st>>>(ma, mb, mb, ma, mb, mb, mo, ma, ma, p);
-  if (cudaGetLastError() != cudaSuccess) return -55;
+  const int rc = ce_forward(hidden, weight, labels, logits_out, reinterpret_cast<float4*>(partials), rows, N, K, ldh, ldw, ldo, softcap,
+                            status, wait_budget_s, num_sms, st);
+  if (rc) return rc;
   const long long warps = rows;
   lce_combine_kernel<<<static_cast<unsigned>((warps * 32 + 255) / 256), 256, 0, st>>>(
       reinterpret_cast<const float4*>(partials), labels, nll, lse, rows, 2 * tiles_n, N, smoothing, ignore_index);
@@ -1576,45 +1542,24 @@ extern "C" int ob_linear_ce_fwd_noalloc(const void* hidden, const void* weight, 
   float4* partials = nullptr;
   int rc = lce_static_scratch(&partials);
   if (rc) return rc;
-  CUtensorMap ma, mb;
-  rc = make_bf16_map_2d(&ma, hidden, rows, K, ldh, GP_BK, GP_BM);
-  if (rc == 0) rc = make_bf16_map_2d(&mb, weight, N, K, ldw, GP_BK, GP_BNH);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  // forward only: the logits never reach memory
+  rc = ce_forward(hidden, weight, labels, nullptr, partials, rows, N, K, ldh, ldw, 0, softcap, status, wait_budget_s, num_sms, st);
+  if (rc == -54) {
+    snprintf(g_no_alloc_error, sizeof(g_no_alloc_error), "cudaFuncSetAttribute(shared memory) failed");
+    return rc;
+  }
+  if (rc == -55) {
+    snprintf(g_no_alloc_error, sizeof(g_no_alloc_error), "kernel launch failed");
+    return rc;
+  }
   if (rc) {
     snprintf(g_no_alloc_error, sizeof(g_no_alloc_error), "operands must have 16-byte aligned rows (tensor map code %d)", rc);
     return rc;
   }
-  static bool configured = false;
-  static int clusters_ce = 0;
-  if (!configured) {
-    if (cudaFuncSetAttribute(gemm_pair_kernel<GP_EPI_CE>, cudaFuncAttributeMaxDynamicSharedMemorySize, GP_SMEM) != cudaSuccess) {
-      snprintf(g_no_alloc_error, sizeof(g_no_alloc_error), "cudaFuncSetAttribute(shared memory) failed");
-      return -54;
-    }
-    clusters_ce = pair_grid(reinterpret_cast<const void*>(gemm_pair_kernel<GP_EPI_CE>), num_sms);
-    configured = true;
-  }
-  PairParams p = {};
-  p.group_m = pair_group_m();
-  p.M = static_cast<int>(rows);
-  p.N = N; p.K1 = K; p.K2 = 0;
-  p.out = nullptr;                    // forward only: the logits never reach memory
-  p.ldo = 0;
-  p.labels = labels;
-  p.ce_partials = partials;
-  p.softcap = softcap;
-  p.status = status;
-  p.wait_budget_ns = static_cast<unsigned long long>(wait_budget_s * 1e9);
-  const long long tiles_m = (rows + 2 * GP_BM - 1) / (2 * GP_BM);
-  const long long total = tiles_m * tiles_n;
-  const int clusters = static_cast<int>(total < clusters_ce ? total : clusters_ce);
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  gemm_pair_kernel<GP_EPI_CE><<<2 * clusters, GP_THREADS, GP_SMEM, st>>>(ma, mb, mb, ma, mb, mb, ma, ma, ma, p);
-  cudaError_t err = cudaGetLastError();
-  if (err == cudaSuccess) {
-    lce_combine_kernel<<<static_cast<unsigned>((rows * 32 + 255) / 256), 256, 0, st>>>(
-        partials, labels, nll, lse, rows, 2 * tiles_n, N, smoothing, ignore_index);
-    err = cudaGetLastError();
-  }
+  lce_combine_kernel<<<static_cast<unsigned>((rows * 32 + 255) / 256), 256, 0, st>>>(
+      partials, labels, nll, lse, rows, 2 * tiles_n, N, smoothing, ignore_index);
+  const cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) {
     snprintf(g_no_alloc_error, sizeof(g_no_alloc_error), "kernel launch failed: %s", cudaGetErrorString(err));
     return -55;

@@ -24,12 +24,11 @@ _SIGNATURES = {
     "ob_wgrad_clip_pe_batch": [c_char_p, I, P, P, LL, P, D, I, P],
     "ob_gemm_tn": [P, P, P, P, P, P, LL, I, I, I, LL, LL, LL, LL, LL, I, I, F, P, I, I, P, D, I, P],
     "ob_lora_pack": [P, P, P, P, P, P, P, P, I, I, I, I, I, I, P],
-    "ob_gemm_pair": [P, P, P, P, P, P, P, P, P, P, LL, I, I, I, LL, LL, LL, LL, LL, I, I, I, I, P, D, I, P],
+    "ob_gemm_pair": [P, P, P, P, P, P, P, P, P, P, LL, I, I, I, LL, LL, LL, LL, LL, I, I, I, I, I, P, D, I, P],
     "ob_pair_init": [],
     "ob_pair_set_die_aware": [I],
     "ob_die_map": [P, I],
     "ob_gemm_pair_glu_bwd": [P, P, P, P, P, P, LL, I, I, LL, LL, LL, LL, I, I, P, D, I, P],
-    "ob_gemm_pair_db": [P, P, P, P, P, P, LL, I, I, I, LL, LL, LL, LL, LL, I, I, P, D, I, P],
     "ob_linear_ce_fwd": [P, P, P, P, P, P, P, LL, I, I, LL, LL, LL, F, F, LL, P, D, I, P],
     "ob_linear_ce_dlogits": [P, P, P, P, LL, I, LL, F, F, LL, P],
     "ob_moe_combine": [P, P, P, P, LL, I, I, I, P],
