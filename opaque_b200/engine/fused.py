@@ -493,12 +493,12 @@ def glu_up(x: torch.Tensor, w_gate: torch.nn.Parameter, w_up: torch.nn.Parameter
 
 
 class _GLUMLP(Function):
-    """A whole FROZEN gated MLP ``(act(x Wgᵀ) * (x Wuᵀ)) Wdᵀ`` in four launches, forward and backward together.
+    """A whole gated MLP ``(act(x Wgᵀ) * (x Wuᵀ)) Wdᵀ``, its three weights all frozen or all trainable, in four launches.
 
     Forward: the fused gate/up launch (keeps the bf16 pre-activations) and the down projection.  Backward: the down
-    projection's data-gradient GEMM turns its accumulator ``dH`` into ``dG`` and ``dU`` in its epilogue (neither ``h``
-    nor ``dH`` is kept or written), and ``dX = dG·Wg + dU·Wu`` is one two-segment launch.  Against the separate
-    functions this drops one element-wise pass over ``[T, I]`` tensors and a third of the MLP's saved activations.
+    projection's data-gradient GEMM turns its accumulator ``dH`` into ``dG`` and ``dU`` in its epilogue, so ``dH`` is never
+    written (few tiles: two launches, :func:`ops.pick_glu_bwd`), and ``dX = dG·Wg + dU·Wu`` is one two-segment launch.  Trainable weights hand ``(h, dY)``, ``(x, dG)`` and
+    ``(x, dU)`` to the capture like any DP linear.  The same bits as :class:`_GLUUp` and the separate down projection.
     """
 
     @staticmethod
@@ -506,36 +506,47 @@ class _GLUMLP(Function):
         x2d = _rows(x)
         h, g, u = ops.gemm_glu(x2d, w_gate, w_up, act=act)
         y = ops.gemm(h, w_down)
-        ctx.save_for_backward(g, u, w_gate, w_up, w_down)
+        ctx.trainable = w_down.requires_grad
+        ctx.save_for_backward(g, u, w_gate, w_up, w_down, *((x2d, h) if ctx.trainable else ()))
         ctx.act, ctx.xshape = act, x.shape
         return y.view(*x.shape[:-1], w_down.shape[0])
 
     @staticmethod
     def backward(ctx, dy):
-        g, u, w_gate, w_up, w_down = ctx.saved_tensors
-        d2 = dy.reshape(-1, dy.shape[-1])
-        d2 = d2 if d2.is_contiguous() else d2.contiguous()
-        dg, du = ops.gemm_glu_bwd(d2, w_down, g, u, act=ctx.act)
+        g, u, w_gate, w_up, w_down = ctx.saved_tensors[:5]
+        d2 = ops.functional._vec16(dy.reshape(-1, dy.shape[-1]))
+        if ops.pick_glu_bwd(g.shape[0], g.shape[1], ops.lib.sm_count()):
+            dg, du = ops.gemm_glu_bwd(d2, w_down, g, u, act=ctx.act)
+        else:
+            dg, du = ops.functional.glu_backward(ops.gemm(d2, w_down, b_layout="kn"), g, u, ctx.act)
         dx = None
         if ctx.needs_input_grad[0]:
             dx = ops.gemm(dg, w_gate, b_layout="kn", a2=du, b2=w_up, b2_layout="kn").view(ctx.xshape)
+        if not ctx.trainable:
+            return dx, None, None, None, None
+        x2d, h = ctx.saved_tensors[5:]
+        cap = current_capture()
+        if cap is None:
+            return dx, dg.t() @ x2d, du.t() @ x2d, d2.t() @ h, None
+        cap.add_linear(w_down, h, d2)
+        cap.add_linear(w_gate, x2d, dg)
+        cap.add_linear(w_up, x2d, du)
         return dx, None, None, None, None
 
 
-# Off: measured on 16384 x 14336 x 4096 (sustained) the fused launch takes 1.92 ms against 1.43 ms for the plain data-gradient
-# GEMM + 0.43 ms for the element-wise GLU backward (1.86 ms): the epilogue's row-strided loads of the pre-activations make
-# it longer than the tile's main loop.  Kept as a tested option.
-FUSE_GLU_MLP = False
+FUSE_GLU_MLP = True
 
 
 def glu_mlp(x: torch.Tensor, w_gate, w_up, w_down, act: str = "silu") -> torch.Tensor | None:
-    """The frozen gated MLP as one autograd function, or ``None`` when it does not apply (any of the three weights
-    trainable, shapes the kernels do not take): the caller then composes :func:`glu_up` and the down projection."""
-    if not FUSE_GLU_MLP or w_gate.requires_grad or w_up.requires_grad or w_down.requires_grad:
+    """The gated MLP as one autograd function, or ``None`` when it does not apply (no backward pass ahead, some weights frozen and
+    others not, shapes the kernels do not take): the caller then composes :func:`glu_up` and the down projection."""
+    trainable = w_down.requires_grad
+    if not FUSE_GLU_MLP or w_gate.requires_grad != trainable or w_up.requires_grad != trainable or not torch.is_grad_enabled():
         return None
-    if not (_own_gemm_ok(x, w_gate) and _own_gemm_ok(x, w_up) and w_gate.shape == w_up.shape
-            and w_gate.stride(0) == w_up.stride(0) and w_down.dtype == torch.bfloat16 and w_down.is_contiguous()
-            and w_down.shape[1] == w_gate.shape[0] and w_gate.shape[0] % 64 == 0 and w_down.shape[0] % 8 == 0):
+    if current_capture() is None if trainable else not x.requires_grad:
+        return None
+    if not (_own_gemm_ok(x, w_gate) and _own_gemm_ok(x, w_up) and _own_gemm_ok(x, w_down) and w_gate.shape == w_up.shape
+            and w_gate.stride(0) == w_up.stride(0) and w_down.shape[1] == w_gate.shape[0] and w_gate.shape[0] % 64 == 0):
         return None
     return _GLUMLP.apply(x, w_gate, w_up, w_down, act)
 

@@ -18,6 +18,7 @@ import math
 import torch
 from torch import nn
 from torch.autograd import Function
+from torch.nn.modules.module import _has_any_global_hook
 
 from .. import ops
 from ..engine import fused
@@ -71,6 +72,16 @@ class Linear(nn.Module):
         if self.lora_A is not None and not _ADAPTERS_OFF:
             return fused.lora_linear(x, self.weight, self.bias, self.lora_A, self.lora_B, self.scaling)
         return fused.dp_linear(x, self.weight, self.bias)
+
+
+_LINEAR_FORWARD = Linear.forward
+
+
+def plain_linear(m: nn.Module) -> bool:
+    """Whether ``m`` may be passed by, its weight used without a call of the module: a :class:`Linear` with this file's ``forward``
+    (none patched in, assigned or compiled) and no hooks, on it or on all modules, that expect the call."""
+    return (type(m) is Linear and Linear.forward is _LINEAR_FORWARD and "forward" not in m.__dict__ and m._compiled_call_impl is None
+            and not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks or _has_any_global_hook()))
 
 
 class Embedding(nn.Module):

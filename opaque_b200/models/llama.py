@@ -19,7 +19,7 @@ from torch import nn
 from .. import ops
 from ..engine import fused
 from ..functional import functional_checkpoint
-from .layers import Embedding, LayerNorm, Linear, RMSNorm, linear_cross_entropy, per_example_token_weights
+from .layers import Embedding, LayerNorm, Linear, RMSNorm, linear_cross_entropy, per_example_token_weights, plain_linear
 
 
 @dataclasses.dataclass
@@ -222,9 +222,8 @@ class LlamaMLP(nn.Module):
         gp, up_ = self.gate_proj, self.up_proj
         if gp.lora_A is None and up_.lora_A is None and gp.bias is None and up_.bias is None:
             dp = self.down_proj
-            if dp.lora_A is None and dp.bias is None:
-                # frozen MLP: forward and backward as one function (the GLU backward rides in the down projection's
-                # data-gradient epilogue)
+            if dp.lora_A is None and dp.bias is None and plain_linear(dp):
+                # forward and backward as one function (the GLU backward rides in the down projection's data-gradient epilogue)
                 y = fused.glu_mlp(x, gp.weight, up_.weight, dp.weight, self.act)
                 if y is not None:
                     return y

@@ -529,6 +529,13 @@ def gemm_glu_bwd(dy: torch.Tensor, w_down: torch.Tensor, gate: torch.Tensor, up:
     return dg, du
 
 
+def pick_glu_bwd(M: int, inter: int, sms: int = 148) -> bool:
+    """Whether :func:`gemm_glu_bwd` beats a plain data gradient and the element-wise GLU backward (the same bits): once its 256 x 256
+    tiles are more than one wave.  A lone tile's epilogue has no main loop to hide behind (us, separate / fused: 128 x 8192 12.5 / 20.1,
+    597 x 5632 21.1 / 21.6, both K = 2048; 1024 x 14336 x 4096, three waves, 129 / 122; 5439 x 8192 x 2048 218 / 183)."""
+    return -(-M // 256) * -(-inter // 256) > sms // 2
+
+
 def gemm_glu_ref(a, w_gate, w_up, *, act="silu"):
     """fp32 oracle of :func:`gemm_glu` (returns ``h`` only)."""
     g, u = a.float() @ w_gate.float().t(), a.float() @ w_up.float().t()
@@ -892,7 +899,7 @@ from .functional import (activation, add_layer_norm, cross_entropy, cross_entrop
                          layer_norm, merge_heads3, plain_torch_ops, rms_norm, rms_norm_ref, rope_qk, rope_qk_ref, rope_tables, rows_group_sum_, swiglu)
 
 __all__ = [
-    "gemm", "gemm_pair", "lora_pack", "pick_gemm_plan", "gemm_glu", "gemm_glu_bwd", "direct_norm2", "pick_norm_path", "pick_gemm_kernel", "die_map", "set_die_aware_tiles", "linear_ce_forward", "linear_ce_dlogits_", "gemm_glu_ref", "gemm_ref", "ghost_set_wide", "push_grad_", "wgrad_clip_per_example", "wgrad_clip_batch", "wgrad_clip_per_example_batch", "direct_norm2_batch", "ghost_norm_batch", "plain_torch_ops", "layer_norm", "add_layer_norm", "activation", "rows_group_sum_", "merge_heads3",
+    "gemm", "gemm_pair", "lora_pack", "pick_gemm_plan", "gemm_glu", "gemm_glu_bwd", "pick_glu_bwd", "direct_norm2", "pick_norm_path", "pick_gemm_kernel", "die_map", "set_die_aware_tiles", "linear_ce_forward", "linear_ce_dlogits_", "gemm_glu_ref", "gemm_ref", "ghost_set_wide", "push_grad_", "wgrad_clip_per_example", "wgrad_clip_batch", "wgrad_clip_per_example_batch", "direct_norm2_batch", "ghost_norm_batch", "plain_torch_ops", "layer_norm", "add_layer_norm", "activation", "rows_group_sum_", "merge_heads3",
     "DeviceWaitTimeout", "KernelLibraryError", "StatusWord", "clip_tree", "clip_weighted_sum", "cross_entropy",
     "cross_entropy_ref", "embedding_wgrad", "fused_add_rms_norm", "geglu", "ghost_norm", "ghost_norm_ref", "glu_ref",
     "philox_normal_add_", "pick_block_n", "pick_splits", "rms_norm", "rms_norm_ref", "rope_qk", "rope_qk_ref",

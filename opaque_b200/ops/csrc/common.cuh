@@ -389,6 +389,28 @@ __device__ __forceinline__ void add_bias64(float* v, const __nv_bfloat16* bias, 
 }
 
 // ---------------------------------------------------------------------------------------------
+// Gated activations.  act: 0 = SwiGLU (silu), 1 = GeGLU exact (erf), 2 = GeGLU tanh approximation.
+__device__ __forceinline__ float act_fwd(float e, int act) {
+  if (act == 0) return e / (1.f + __expf(-e));
+  if (act == 1) return 0.5f * e * (1.f + erff(e * 0.70710678118654752f));
+  const float u = 0.7978845608028654f * (e + 0.044715f * e * e * e);
+  return 0.5f * e * (1.f + tanhf(u));
+}
+__device__ __forceinline__ float act_bwd(float e, int act) {
+  if (act == 0) {
+    const float s = 1.f / (1.f + __expf(-e));
+    return s * (1.f + e * (1.f - s));
+  }
+  if (act == 1) {
+    const float cdf = 0.5f * (1.f + erff(e * 0.70710678118654752f));
+    return cdf + e * 0.3989422804014327f * __expf(-0.5f * e * e);
+  }
+  const float u = 0.7978845608028654f * (e + 0.044715f * e * e * e);
+  const float t = tanhf(u);
+  return 0.5f * (1.f + t) + 0.5f * e * (1.f - t * t) * 0.7978845608028654f * (1.f + 0.134145f * e * e);
+}
+
+// ---------------------------------------------------------------------------------------------
 // Epilogue stores through the TMA engine.  A warp writes its [32 rows x 64 columns] bf16 tile into a 4 KB shared-memory
 // slab in the 128-byte-swizzled layout the tensor map expects (16-byte chunk j of row r at chunk position j ^ (r & 7);
 // the slab is 1024-byte aligned), and one lane issues a bulk tensor store.  Rows and columns outside the tensor are

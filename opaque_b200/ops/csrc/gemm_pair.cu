@@ -77,11 +77,6 @@ struct PairParams {
   int* status;
   unsigned long long wait_budget_ns;
   int tma_store;                     // STORE: the output leaves through bulk tensor stores (map_out is valid)
-  // GLU-backward epilogue (data gradient of a gated MLP's down projection): the accumulator is dH; with the stored
-  // pre-activations it becomes dGate (-> out) and dUp (-> out_up) without dH ever reaching memory
-  const __nv_bfloat16* glu_g;        // [M, N] gate pre-activations, pitch ld_gu
-  const __nv_bfloat16* glu_u;        // [M, N] up pre-activations
-  long long ld_gu;
   // Die-aware tile assignment (see gp_schedule); claim == nullptr: cluster c simply takes tiles c, c + clusters, ...
   unsigned long long* claim;         // this launch's claim word (zero on entry, zero again after the last claim)
   int n_front;                       // clusters expected on die 0: slots [0, n_front) walk tiles [0, split)
@@ -254,49 +249,33 @@ __device__ __forceinline__ float gp_act(float g) {
   return 0.5f * g * (1.0f + t);
 }
 
-// Value and derivative of the gate activation (compile-time choice, see gp_act).
+// One 16-byte piece (8 columns) of a row: packed bf16 dH and the pre-activations `g`, `u` -> dGate = dH * up * act'(gate) in `g` and
+// dUp = dH * act(gate) in `u`.  dH enters bf16-rounded, as it would from memory; the operations are glu_bwd_kernel's, in its order.
 template <int ACT>
-__device__ __forceinline__ void gp_act_grad(float g, float& a, float& da) {
-  if constexpr (ACT == 0) {
-    const float sg = 1.0f / (1.0f + __expf(-g));
-    a = g * sg;
-    da = sg * (1.0f + g * (1.0f - sg));
-  } else if constexpr (ACT == 1) {
-    const float cdf = 0.5f * (1.0f + erff(g * 0.70710678118654752f));
-    a = g * cdf;
-    da = cdf + g * 0.3989422804014327f * __expf(-0.5f * g * g);
-  } else {
-    const float t = tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g));
-    a = 0.5f * g * (1.0f + t);
-    da = 0.5f * (1.0f + t) + 0.5f * g * (1.0f - t * t) * 0.7978845608028654f * (1.0f + 0.134145f * g * g);
+__device__ __forceinline__ void gp_glu_bwd8(const uint32_t* pd, uint4& g4, uint4& u4) {
+  uint32_t gw[4] = {g4.x, g4.y, g4.z, g4.w}, uw[4] = {u4.x, u4.y, u4.z, u4.w};
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float dx = __uint_as_float(pd[j] << 16), dy = __uint_as_float(pd[j] & 0xffff0000u);
+    const float gx = __uint_as_float(gw[j] << 16), gy = __uint_as_float(gw[j] & 0xffff0000u);
+    const float ux = __uint_as_float(uw[j] << 16), uy = __uint_as_float(uw[j] & 0xffff0000u);
+    uw[j] = pack_bf16x2(dx * act_fwd(gx, ACT), dy * act_fwd(gy, ACT));
+    gw[j] = pack_bf16x2(dx * ux * act_bwd(gx, ACT), dy * uy * act_bwd(gy, ACT));
   }
+  g4 = make_uint4(gw[0], gw[1], gw[2], gw[3]);
+  u4 = make_uint4(uw[0], uw[1], uw[2], uw[3]);
 }
-
-// 64 columns of one row: packed bf16 dH (pd) and the row's gate / up pre-activations (16-byte loads) -> packed
-// dGate = dH * up * act'(gate) and dUp = dH * act(gate).  dH enters bf16-rounded, as it would from memory.
+// 64 columns of the warp's 32 rows, in place: the two slabs hold gate and up (128-byte swizzle) and receive dGate and dUp.
 template <int ACT>
-__device__ __forceinline__ void gp_glu_bwd64(const uint32_t* pd, const __nv_bfloat16* grow, const __nv_bfloat16* urow,
-                                             bool in_row, uint32_t* og, uint32_t* ou) {
+__device__ __forceinline__ void gp_glu_bwd_slabs(const uint32_t* pd, uint8_t* slab, int lane) {
 #pragma unroll
-  for (int s8 = 0; s8 < 8; ++s8) {
-    uint4 g4 = make_uint4(0u, 0u, 0u, 0u), u4 = g4;
-    if (in_row) {
-      g4 = __ldg(reinterpret_cast<const uint4*>(grow) + s8);
-      u4 = __ldg(reinterpret_cast<const uint4*>(urow) + s8);
-    }
-    const uint32_t gw[4] = {g4.x, g4.y, g4.z, g4.w}, uw[4] = {u4.x, u4.y, u4.z, u4.w};
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const uint32_t d2 = pd[4 * s8 + j];
-      const float dx = __uint_as_float(d2 << 16), dy = __uint_as_float(d2 & 0xffff0000u);
-      const float gx = __uint_as_float(gw[j] << 16), gy = __uint_as_float(gw[j] & 0xffff0000u);
-      const float ux = __uint_as_float(uw[j] << 16), uy = __uint_as_float(uw[j] & 0xffff0000u);
-      float ax, dax, ay, day;
-      gp_act_grad<ACT>(gx, ax, dax);
-      gp_act_grad<ACT>(gy, ay, day);
-      og[4 * s8 + j] = pack_bf16x2(dx * ux * dax, dy * uy * day);
-      ou[4 * s8 + j] = pack_bf16x2(dx * ax, dy * ay);
-    }
+  for (int c = 0; c < 8; ++c) {
+    uint4* gp = reinterpret_cast<uint4*>(slab + lane * 128 + ((c ^ (lane & 7)) << 4));
+    uint4* up = reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(gp) + GP_SLAB_BYTES);
+    uint4 g4 = *gp, u4 = *up;
+    gp_glu_bwd8<ACT>(pd + 4 * c, g4, u4);
+    *gp = g4;
+    *up = u4;
   }
 }
 
@@ -360,8 +339,7 @@ template <int EPI>
 __device__ __forceinline__ bool pair_vec_ok(const PairParams& p) {
   return ((p.ldo & 7) == 0) && ((reinterpret_cast<uintptr_t>(p.out) & 15) == 0) &&
          (EPI != GP_EPI_GLU || p.out_gate == nullptr ||
-          (((reinterpret_cast<uintptr_t>(p.out_gate) | reinterpret_cast<uintptr_t>(p.out_up)) & 15) == 0)) &&
-         (EPI != GP_EPI_GLUBWD || (reinterpret_cast<uintptr_t>(p.out_up) & 15) == 0);
+          (((reinterpret_cast<uintptr_t>(p.out_gate) | reinterpret_cast<uintptr_t>(p.out_up)) & 15) == 0));
 }
 
 // Epilogue of one 128 x 256 accumulator per CTA, by one of the eight epilogue warps: TMEM lanes 32 * (warp % 4) .., column group g.
@@ -478,42 +456,6 @@ __device__ __forceinline__ void pair_epilogue(const PairParams& p, const CUtenso
     }
     if (row < p.M)
       p.ce_partials[static_cast<long long>(row) * (2 * tiles_n) + 2 * nt + g] = make_float4(m, ssum, zlab, ztot);
-  } else if constexpr (EPI == GP_EPI_GLUBWD) {
-    // Data gradient of the down projection with the gated activation's backward in the epilogue: the tile is dH;
-    // it is read, rounded to bf16 and packed, the accumulator half goes back, and the row's gate / up
-    // pre-activations turn it into dGate and dUp tiles, which leave through the slab.  N % 64 == 0 (host-checked).
-    const int n0 = nt * GP_BN + g * (GP_BN / 2);
-    const int row0w = row - lane;
-    uint32_t pd[2][32];
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      const int nc = n0 + c * 64;
-      if (nc < p.N) {
-        float v[64];
-        tmem_ld32(t_row + g * (GP_BN / 2) + c * 64, v);
-        tmem_ld32(t_row + g * (GP_BN / 2) + c * 64 + 32, v + 32);
-        tmem_ld_wait();
-#pragma unroll
-        for (int j = 0; j < 32; ++j) pd[c][j] = pack_bf16x2(v[2 * j], v[2 * j + 1]);
-      }
-    }
-    release();
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      const int nc = n0 + c * 64;
-      if (nc < p.N) {
-        const bool in_row = row < p.M;
-        const __nv_bfloat16* grow = p.glu_g + static_cast<long long>(row) * p.ld_gu + nc;
-        const __nv_bfloat16* urow = p.glu_u + static_cast<long long>(row) * p.ld_gu + nc;
-        uint32_t og[32], ou[32];
-        if (p.act == 0) gp_glu_bwd64<0>(pd[c], grow, urow, in_row, og, ou);
-        else if (p.act == 1) gp_glu_bwd64<1>(pd[c], grow, urow, in_row, og, ou);
-        else gp_glu_bwd64<2>(pd[c], grow, urow, in_row, og, ou);
-        const bool tma = p.tma_store != 0;
-        store_tile64_packed(slab, og, &map_out, tma, nc, row0w, p.out, p.ldo, p.M - row0w, p.N - nc, vec_ok, lane);
-        store_tile64_packed(slab, ou, &map_out_up, tma, nc, row0w, p.out_up, p.ldo, p.M - row0w, p.N - nc, vec_ok, lane);
-      }
-    }
   } else {
     // GLU: this warp's 64 columns of h come from 64 gate and 64 up columns of the same rows.  Everything is read
     // and packed first (four rounds of 16 + 16 columns), the accumulator half is released, then up to three
@@ -811,13 +753,22 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 // 4096 in 167 us, 1.64 PFLOP/s, the library's own burst rate (big tile 182; 186 while one thread ran the issue loop).  Same
 // epilogues, barrier protocol and unwind rules as gemm_pair_kernel.
 constexpr int GD_BM = 128;                              // rows of M per CTA (256 per pair)
-constexpr int GD_STAGES = 6;
 constexpr int GD_A_BYTES = GD_BM * GP_BK * 2;
 constexpr int GD_B_BYTES = GP_BNH * GP_BK * 2;
 constexpr int GD_STAGE_BYTES = GD_A_BYTES + GD_B_BYTES;
 constexpr int GD_GROUP_M = 16;                          // pair tiles (256 rows each) per raster band
-constexpr int GD_SMEM = GD_STAGES * GD_STAGE_BYTES + 8 * GP_SLAB_BYTES + 256 + 1024;
-static_assert((2 * GD_STAGES + 4) * 8 + 8 <= 256, "barrier block");
+// The GLU backward keeps two slabs per epilogue warp: the TMA engine brings the pre-activations there during the main loop, and they
+// become dGate and dUp in place.  That costs one stage.  Its epilogue hides behind the main loop from K = 1024 on.  Power-capped loops,
+// plain data gradient and element-wise kernel against this one: 16384 x 4096 x 14336 1760 -> 1632 us, 5439 x 2048 x 8192 218 -> 183,
+// 4096 x 1024 x 4096 61 -> 54.  (With one 16-byte load per lane and row instead of the TMA engine, on the 512 x 256 tile, 1920 us.)
+template <int EPI>
+struct GdRing {
+  static constexpr int STAGES = EPI == GP_EPI_GLUBWD ? 5 : 6;
+  static constexpr int WARP_SLAB = EPI == GP_EPI_GLUBWD ? 2 * GP_SLAB_BYTES : GP_SLAB_BYTES;
+  static constexpr int SMEM = STAGES * GD_STAGE_BYTES + 8 * WARP_SLAB + 256 + 1024;
+  static_assert((2 * STAGES + 4 + 8) * 8 + 20 <= 256, "barrier block");
+  static_assert(SMEM <= 232448, "shared memory of an SM");
+};
 
 __device__ __forceinline__ GpItem gd_decode(int w, int tiles_m, int tiles_n, int rank) {
   const int band = GD_GROUP_M * tiles_n;
@@ -839,13 +790,15 @@ gemm_pair_db_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     const __grid_constant__ CUtensorMap map_out_up, const PairParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  constexpr int GD_STAGES = GdRing<EPI>::STAGES, WARP_SLAB = GdRing<EPI>::WARP_SLAB;
   uint8_t* slabs = smem + GD_STAGES * GD_STAGE_BYTES;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(slabs + 8 * GP_SLAB_BYTES);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(slabs + 8 * WARP_SLAB);
   uint64_t* full = bars;                               // used in the leader CTA only
   uint64_t* empty = bars + GD_STAGES;
   uint64_t* tmem_full = bars + 2 * GD_STAGES;          // [2]: one per accumulator buffer
   uint64_t* tmem_empty = bars + 2 * GD_STAGES + 2;     // [2], used in the leader CTA only
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * GD_STAGES + 4);
+  uint64_t* preact = bars + 2 * GD_STAGES + 4;         // [8]: GLU backward, one per epilogue warp
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * GD_STAGES + 12);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* sched = reinterpret_cast<int*>(tmem_slot + 2);  // [3]: first, end, stride (valid in the leader CTA)
 
@@ -870,6 +823,8 @@ gemm_pair_db_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       mbar_init(&tmem_full[a], 1);
       mbar_init(&tmem_empty[a], 16);                   // eight epilogue warps in each CTA
     }
+    if constexpr (EPI == GP_EPI_GLUBWD)
+      for (int a = 0; a < 8; ++a) mbar_init(&preact[a], 1);
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&map_a);
@@ -985,27 +940,81 @@ gemm_pair_db_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     // ------------------------------------------------------------------ epilogue warps (8 per CTA)
     const int q = warp & 3;                  // TMEM lane quarter this warp may read
     const int g = (warp - 2) >> 2;           // 128-column half of the tile
-    uint8_t* slab = slabs + (warp - 2) * GP_SLAB_BYTES;
+    uint8_t* slab = slabs + (warp - 2) * WARP_SLAB;
     int acc_iter = 0;
     bool ok = true;
-    const bool vec_ok = pair_vec_ok<EPI>(p);
+    [[maybe_unused]] uint32_t fetched = 0;   // parity of this warp's next pair of pre-activation tiles
+    [[maybe_unused]] const bool vec_ok = pair_vec_ok<EPI>(p);
     for (int w = sc.first; ok && w < sc.end; w += sc.stride) {
       const GpItem it = gd_decode(w, tiles_m, tiles_n, rank);
       const int as = acc_iter & 1;
+      const int row0w = it.row0 + q * 32, n0 = it.nt * GP_BN + g * (GP_BN / 2);
+      // GLU backward: the pre-activations [32 rows x 64 columns] of this warp's next round, into its two slabs
+      [[maybe_unused]] auto fetch = [&](int nc) {
+        if (lane == 0) {
+          tma_store_wait_read();             // the round before has left the slabs
+          mbar_expect_tx(&preact[warp - 2], 2 * GP_SLAB_BYTES);
+          tma_load_2d(slab, &map_a2, &preact[warp - 2], nc, row0w);
+          tma_load_2d(slab + GP_SLAB_BYTES, &map_b2, &preact[warp - 2], nc, row0w);
+        }
+      };
+      if constexpr (EPI == GP_EPI_GLUBWD) {
+        if (n0 < p.N) fetch(n0);             // arrives during the tile's main loop
+      }
       if (!mbar_wait_idle(&tmem_full[as], (acc_iter >> 1) & 1, abort_flag, p.status, OB_ERR_WAIT_TMEM_FULL, budget)) {
         ok = false;
         break;
       }
       tc_fence_after();
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + as * GP_BN;
-      pair_epilogue<EPI>(p, map_out, map_out_gate, map_out_up, slab, t_row, it.row0 + q * 32 + lane, it.nt, tiles_n, g, lane, vec_ok, [&] {
+      auto release = [&] {
         tc_fence_before();
         __syncwarp();
         if (lane == 0) {
           if (leader) mbar_arrive(&tmem_empty[as]);
           else mbar_arrive_cluster(map_to_cta(smem_u32(&tmem_empty[as]), 0));
         }
-      });
+      };
+      if constexpr (EPI == GP_EPI_GLUBWD) {
+        // Data gradient of a gated MLP's down projection: the accumulator is dH.  It is read, rounded to bf16 and packed, handed
+        // back, and turned into dGate and dUp in the slabs that hold the pre-activations.  N % 64 == 0 (host-checked).
+        uint32_t pd[2][32];
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          if (n0 + c * 64 < p.N) {
+            float v[64];
+            tmem_ld32(t_row + g * (GP_BN / 2) + c * 64, v);
+            tmem_ld32(t_row + g * (GP_BN / 2) + c * 64 + 32, v + 32);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 32; ++j) pd[c][j] = pack_bf16x2(v[2 * j], v[2 * j + 1]);
+          }
+        }
+        release();
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const int nc = n0 + c * 64;
+          if (nc < p.N) {
+            if (c > 0) fetch(nc);
+            ok = mbar_wait_warp(&preact[warp - 2], fetched, abort_flag, p.status, OB_ERR_WAIT_FULL, budget);
+            if (!ok) break;
+            fetched ^= 1;
+            if (p.act == 0) gp_glu_bwd_slabs<0>(pd[c], slab, lane);
+            else if (p.act == 1) gp_glu_bwd_slabs<1>(pd[c], slab, lane);
+            else gp_glu_bwd_slabs<2>(pd[c], slab, lane);
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              tma_store_2d(&map_out, slab, nc, row0w);
+              tma_store_2d(&map_out_up, slab + GP_SLAB_BYTES, nc, row0w);
+              tma_store_commit();
+            }
+          }
+        }
+        if (!ok) break;
+      } else {
+        pair_epilogue<EPI>(p, map_out, map_out_gate, map_out_up, slab, t_row, row0w + lane, it.nt, tiles_n, g, lane, vec_ok, release);
+      }
       ++acc_iter;
     }
     if (lane == 0) tma_store_wait_all();
@@ -1271,16 +1280,15 @@ static bool pair_small_tile(long long rows, long long cols, long long K, int clu
 
 // The activation and cross-entropy epilogues always take the small tile (power-capped loops against the big one: gate + up + SwiGLU
 // 16384 x 4096 x 14336 2.87 -> 2.80 ms, 5439 x 2048 x 8192 0.312 -> 0.291; head + statistics 8192 x 2048 x 128256 3.42 -> 3.19 ms with
-// the logits stored, 3.48 -> 3.00 without; 3663 x 768 x 50304 0.332 -> 0.305), the GLU backward, longer than either tile's main
-// loop, the big one.
+// the logits stored, 3.48 -> 3.00 without; 3663 x 768 x 50304 0.332 -> 0.305).  The GLU backward's epilogue is longest of all
+// and exists for the small tile alone.
 template <int EPI>
 static int pair_launch(bool small, const PairMaps& m, PairParams& p, int num_sms, cudaStream_t st) {
   using Kernel = decltype(&gemm_pair_db_kernel<GP_EPI_STORE>);
   Kernel kernel;
   if constexpr (EPI == GP_EPI_STORE) kernel = small ? gemm_pair_db_kernel<EPI> : gemm_pair_kernel<EPI>;
-  else if constexpr (EPI == GP_EPI_GLUBWD) kernel = gemm_pair_kernel<EPI>;
   else kernel = gemm_pair_db_kernel<EPI>;
-  const int smem = small ? GD_SMEM : GP_SMEM;
+  const int smem = small ? GdRing<EPI>::SMEM : GP_SMEM;
   static int max_clusters[2] = {0, 0};
   if (max_clusters[small] == 0) {
     if (cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -54;
@@ -1381,12 +1389,16 @@ extern "C" int ob_gemm_pair_glu_bwd(const void* dy, const void* w, const void* g
   auto al = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
   if ((N & 63) != 0 || (ld_gu & 7) != 0 || (ld_out & 7) != 0 || !al(gate) || !al(up) || !al(dgate) || !al(dup)) return -58;
   PairMaps m;
-  int rc = make_bf16_map_2d(&m.a, dy, rows_a, K, lddy, GP_BK, GP_BM);
+  int rc = make_bf16_map_2d(&m.a, dy, rows_a, K, lddy, GP_BK, GD_BM);
   if (rc) return rc;
   rc = b_kn ? make_bf16_map_2d(&m.b, w, K, N, ldw, 64, GP_BK) : make_bf16_map_2d(&m.b, w, N, K, ldw, GP_BK, GP_BNH);
   if (rc) return rc;
-  m.b_up = m.b2 = m.b2_up = m.b;
-  m.a2 = m.out = m.out_gate = m.out_up = m.a;
+  m.b_up = m.b2_up = m.b;
+  m.out_gate = m.a;
+  // no second segment: its maps hold the pre-activations, in boxes of one epilogue round
+  if ((rc = make_bf16_map_2d(&m.a2, gate, rows_a, N, ld_gu, 64, 32)) != 0 || (rc = make_bf16_map_2d(&m.b2, up, rows_a, N, ld_gu, 64, 32)) != 0)
+    return rc;
+  if (!pair_out_map(&m.out, dgate, rows_a, N, ld_out) || !pair_out_map(&m.out_up, dup, rows_a, N, ld_out)) return -58;
   PairParams p = {};
   p.group_m = pair_group_m();
   p.M = static_cast<int>(rows_a);
@@ -1395,14 +1407,11 @@ extern "C" int ob_gemm_pair_glu_bwd(const void* dy, const void* w, const void* g
   p.out = static_cast<__nv_bfloat16*>(dgate);
   p.out_up = static_cast<__nv_bfloat16*>(dup);
   p.ldo = ld_out;
-  p.glu_g = static_cast<const __nv_bfloat16*>(gate);
-  p.glu_u = static_cast<const __nv_bfloat16*>(up);
-  p.ld_gu = ld_gu;
   p.act = glu_act;
   p.status = status;
   p.wait_budget_ns = static_cast<unsigned long long>(wait_budget_s * 1e9);
-  p.tma_store = (pair_out_map(&m.out, dgate, rows_a, N, ld_out) && pair_out_map(&m.out_up, dup, rows_a, N, ld_out)) ? 1 : 0;
-  return pair_launch<GP_EPI_GLUBWD>(false, m, p, num_sms, static_cast<cudaStream_t>(stream));
+  p.tma_store = 1;
+  return pair_launch<GP_EPI_GLUBWD>(true, m, p, num_sms, static_cast<cudaStream_t>(stream));
 }
 
 // Bit patterns of the descriptors the tensor-core kernels build, for host-side checks.

@@ -106,7 +106,7 @@ def test_down_projection_data_gradient_with_glu_backward_epilogue(dev, M, I, K, 
     x = torch.randn(M, K, device=dev).bfloat16().requires_grad_(True)
     wg = (torch.randn(I, K, device=dev) / math.sqrt(K)).bfloat16()
     wu = (torch.randn(I, K, device=dev) / math.sqrt(K)).bfloat16()
-    old, fused.FUSE_GLU_MLP = fused.FUSE_GLU_MLP, True          # the fused form is an option (off by default)
+    old, fused.FUSE_GLU_MLP = fused.FUSE_GLU_MLP, True
     try:
         y = fused.glu_mlp(x, wg, wu, wd, "silu")
     finally:

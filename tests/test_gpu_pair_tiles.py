@@ -59,3 +59,57 @@ def test_head_statistics(M, V, K, softcap):
         assert float((nll - ref).abs().max()) < 1e-5 * max(1.0, float(zz.abs().max())) * 4
         if store:
             assert float((logits.float() - z).abs().max()) <= 2 ** -8 * float(z.abs().max())
+
+
+# one row; the edges of the epilogue's 64-column rounds and 128-column halves, of the tile and of its five stages; several waves
+@pytest.mark.parametrize("M,inter,K", [(1, 64, 64), (255, 192, 320), (257, 320, 384), (600, 448, 72), (2600, 2368, 200)])
+@pytest.mark.parametrize("act", ["silu", "gelu", "gelu_tanh"])
+def test_gated_activation_backward(M, inter, K, act):
+    """The fused launch equals the data gradient and the element-wise kernel bit for bit, with pre-activations of a wider pitch too."""
+    from opaque_b200 import ops
+    torch.manual_seed(M)
+    dy, wd = (torch.randn(*s, device="cuda", dtype=torch.bfloat16) / K ** 0.25 for s in ((M, K), (K, inter)))
+    g, u = (torch.randn(M, inter + 8, device="cuda", dtype=torch.bfloat16)[:, :inter] for _ in range(2))
+    g[0, :3] = torch.tensor([float("inf"), -100.0, 100.0])
+    want = ops.functional.glu_backward(ops.gemm(dy, wd, b_layout="kn"), g.contiguous(), u.contiguous(), act)
+    for pair in ((g, u), (g.contiguous(), u.contiguous())):
+        for got, ref in zip(ops.gemm_glu_bwd(dy, wd, *pair, act=act), want):
+            assert torch.equal(got.view(torch.int16), ref.view(torch.int16))
+
+
+@pytest.mark.parametrize("rows,inter", [(40, 192), (2600, 2368)])             # two launches and one (ops.pick_glu_bwd)
+@pytest.mark.parametrize("trainable", [False, True])
+def test_gated_mlp_as_one_function(rows, inter, trainable):
+    """Outputs and every gradient of the one-node MLP equal the separate nodes'; with a hook on the down projection it is not taken."""
+    from opaque_b200.engine import fused
+    from opaque_b200.engine.fused import FusedDPEngine
+    from opaque_b200.models import LlamaConfig, LlamaForCausalLM, shift_labels
+    from opaque_b200.random import key
+    results, nodes = [], []
+    for on in (True, False, "hook"):
+        torch.manual_seed(rows)
+        cfg = LlamaConfig.tiny()
+        cfg.intermediate_size, cfg.num_hidden_layers, cfg.max_position_embeddings = inter, 1, 4096
+        model = LlamaForCausalLM(cfg, device="cuda")
+        if not trainable:
+            model.add_lora(8, 16.0)
+            for n, p in model.named_parameters():
+                if n.endswith("lora_B"):
+                    torch.nn.init.normal_(p, std=0.05)
+        eng = FusedDPEngine(model, clipping_norm=1.0, noise_multiplier=0.0, normalize_by=2.0, key=key(0), microbatch_size=2)
+        if on == "hook":
+            model.model.layers[0].mlp.down_proj.register_forward_hook(lambda *a: nodes.append(1))
+        ids = torch.randint(0, 256, (2, rows // 2), device="cuda")
+        old, fused.FUSE_GLU_MLP = fused.FUSE_GLU_MLP, bool(on)
+        try:
+            res = eng.accumulate(model.per_example_loss, {"input_ids": ids, "labels": shift_labels(ids)})
+        finally:
+            fused.FUSE_GLU_MLP = old
+        results.append((res.losses, res.norms, eng.space.grad.local.clone()))
+    assert nodes == [1]
+    for other in results[1:]:
+        assert torch.equal(results[0][0], other[0])
+        # bf16 products and activations are the same bits; norms and gradients add fp32 values with atomics, and the library
+        # attention's backward may round differently between two runs (2^-8 of single values)
+        for a, b in zip(results[0][1:], other[1:]):
+            assert float((a - b).norm()) <= 2e-3 * float(b.norm())
