@@ -172,11 +172,7 @@ class Capture:
         if not (sa.direct and sb.direct):
             raise RuntimeError("LoRA factors must be direct parameters of the flat space")
         r, d_in = lora_a.shape
-        stride = self.pe.stride(0)
-        common = dict(seg_offsets=self.seg, num_groups=self.batch_size, group_stride=stride, n_valid=r)
-        ops.wgrad_clip_batch([dict(a=x2d, b=q_pad, out_offset=sa.offset, ldm=1, ldn=d_in, **common),
-                              dict(a=g2d, b=xa_pad, out_offset=sb.offset, ldm=r, ldn=1, **common)],
-                             self.pe, accumulate=False, block_n=64, status=self.status)
+        self._store_lora(((x2d, q_pad, sa.offset, 1, d_in, r), (g2d, xa_pad, sb.offset, r, 1, r)))
 
     def add_lora_qkv(self, factors, x2d: torch.Tensor, xa: torch.Tensor, g_parts, q_all: torch.Tensor) -> None:
         """The three LoRA pairs of one attention block: ``factors = ((A_q, B_q), (A_k, B_k), (A_v, B_v))`` sharing ``x2d``.
@@ -193,15 +189,24 @@ class Capture:
             for j, (a, b) in enumerate(factors):
                 self.add_lora(a, b, x2d, xa[:, j * r:(j + 1) * r], g_parts[j], q_all[:, j * r:(j + 1) * r])
             return
-        stride = self.pe.stride(0)
-        common = dict(seg_offsets=self.seg, num_groups=self.batch_size, group_stride=stride)
-        jobs = [dict(a=x2d, b=q_all, out_offset=slots[0].offset, ldm=1, ldn=d_in, n_valid=3 * r, **common)]
+        jobs = [(x2d, q_all, slots[0].offset, 1, d_in, 3 * r)]
         for j, (_, b) in enumerate(factors):
             sb = self.engine.slot_of(b)
             if not sb.direct:
                 raise RuntimeError("LoRA factors must be direct parameters of the flat space")
-            jobs.append(dict(a=g_parts[j], b=xa[:, j * r:(j + 1) * r], out_offset=sb.offset, ldm=r, ldn=1, n_valid=r, **common))
-        ops.wgrad_clip_batch(jobs, self.pe, accumulate=False, block_n=64, status=self.status)
+            jobs.append((g_parts[j], xa[:, j * r:(j + 1) * r], sb.offset, r, 1, r))
+        self._store_lora(tuple(jobs))
+
+    def _store_lora(self, jobs: tuple) -> None:
+        """Factor gradients of every example into the per-example buffer, one launch; jobs are
+        ``(a, b, out_offset, ldm, ldn, n_valid)`` of :func:`ops.wgrad_clip`."""
+        steps, stride = ops.block_steps(), self.pe.stride(0)
+        if steps is not None:
+            steps.store_wgrads(jobs, self.pe, self.seg, self.batch_size, stride, self.status.ptr() if self.status else 0)
+            return
+        ops.wgrad_clip_batch([dict(a=a, b=b, out_offset=off, ldm=ldm, ldn=ldn, n_valid=n, seg_offsets=self.seg, num_groups=self.batch_size,
+                                   group_stride=stride) for a, b, off, ldm, ldn, n in jobs],
+                             self.pe, accumulate=False, block_n=64, status=self.status)
 
     def add_row_sums(self, out: torch.Tensor, g2d: torch.Tensor, x2d: torch.Tensor, mean: torch.Tensor | None, rstd: torch.Tensor,
                      out_plain: torch.Tensor | None) -> None:
@@ -492,12 +497,19 @@ def glu_up(x: torch.Tensor, w_gate: torch.nn.Parameter, w_up: torch.nn.Parameter
     return _GLUUp.apply(x, w_gate, w_up, act, torch.is_grad_enabled() and (trainable or x.requires_grad))
 
 
+def glu_down_backward(d2: torch.Tensor, w_down: torch.Tensor, gate: torch.Tensor, up: torch.Tensor, act: str):
+    """``(dG, dU)`` of a gated MLP from the gradient ``d2`` of its output and the stored pre-activations."""
+    if ops.pick_glu_bwd(gate.shape[0], gate.shape[1], ops.lib.sm_count()):
+        return ops.gemm_glu_bwd(d2, w_down, gate, up, act=act)
+    return ops.functional.glu_backward(ops.gemm(d2, w_down, b_layout="kn"), gate, up, act)
+
+
 class _GLUMLP(Function):
     """A whole gated MLP ``(act(x Wgᵀ) * (x Wuᵀ)) Wdᵀ``, its three weights all frozen or all trainable, in four launches.
 
     Forward: the fused gate/up launch (keeps the bf16 pre-activations) and the down projection.  Backward: the down
     projection's data-gradient GEMM turns its accumulator ``dH`` into ``dG`` and ``dU`` in its epilogue, so ``dH`` is never
-    written (few tiles: two launches, :func:`ops.pick_glu_bwd`), and ``dX = dG·Wg + dU·Wu`` is one two-segment launch.  Trainable weights hand ``(h, dY)``, ``(x, dG)`` and
+    written (few tiles: two launches, :func:`glu_down_backward`), and ``dX = dG·Wg + dU·Wu`` is one two-segment launch.  Trainable weights hand ``(h, dY)``, ``(x, dG)`` and
     ``(x, dU)`` to the capture like any DP linear.  The same bits as :class:`_GLUUp` and the separate down projection.
     """
 
@@ -515,10 +527,7 @@ class _GLUMLP(Function):
     def backward(ctx, dy):
         g, u, w_gate, w_up, w_down = ctx.saved_tensors[:5]
         d2 = ops.functional._vec16(dy.reshape(-1, dy.shape[-1]))
-        if ops.pick_glu_bwd(g.shape[0], g.shape[1], ops.lib.sm_count()):
-            dg, du = ops.gemm_glu_bwd(d2, w_down, g, u, act=ctx.act)
-        else:
-            dg, du = ops.functional.glu_backward(ops.gemm(d2, w_down, b_layout="kn"), g, u, ctx.act)
+        dg, du = glu_down_backward(d2, w_down, g, u, ctx.act)
         dx = None
         if ctx.needs_input_grad[0]:
             dx = ops.gemm(dg, w_gate, b_layout="kn", a2=du, b2=w_up, b2_layout="kn").view(ctx.xshape)
@@ -766,6 +775,17 @@ def lora_qkv(x: torch.Tensor, q_proj, k_proj, v_proj):
         return None
     return _LoRAQKV.apply(x, w_all, bias_all, q_proj.scaling, q_proj.lora_A, q_proj.lora_B, k_proj.lora_A, k_proj.lora_B,
                           v_proj.lora_A, v_proj.lora_B)
+
+
+def lora_factors_ok(lora_a: torch.Tensor, lora_b: torch.Tensor) -> bool:
+    """Factors that the grouped and the fused LoRA products take as they are stored."""
+    return (lora_a.dtype == lora_b.dtype == torch.bfloat16 and lora_a.shape[0] % 8 == 0 and lora_a.is_contiguous() and lora_b.is_contiguous()
+            and (lora_a.data_ptr() | lora_b.data_ptr()) & 15 == 0)
+
+
+def one_node_lora() -> bool:
+    """Whether every form that a LoRA block's two nodes stand for is switched on."""
+    return GROUP_LORA_QKV and FUSE_LORA_GEMM and FUSE_GLU_MLP
 
 
 def lora_linear(x, weight, bias, lora_a, lora_b, scaling: float):

@@ -13,11 +13,11 @@ import dataclasses
 
 import torch
 from torch import nn
-from torch.nn.modules.module import _has_any_global_hook
 
 from .. import ops
+from ..engine import blocks, fused
 from ..functional import functional_checkpoint
-from .layers import Embedding, LayerNorm, Linear, linear_cross_entropy, per_example_token_weights
+from .layers import _FORWARDS, Embedding, LayerNorm, Linear, linear_cross_entropy, passable, per_example_token_weights
 
 
 @dataclasses.dataclass
@@ -77,9 +77,40 @@ class GPT2Block(nn.Module):
     def forward_carried(self, x, residual):
         """The block on a split stream ``h = x + residual`` (``residual`` may be ``None``): every residual addition happens inside
         the next LayerNorm's kernel, and the two gradient branches meet in that kernel's backward.  Returns the pair."""
+        if self._two_nodes(x):
+            m, n1, n2 = self._modules, self.ln_1, self.ln_2
+            wq, wo, w1, w2 = (m[k]._parameters for k in _PROJECTIONS)
+            q, k, v, s = blocks.GPT2In.apply(x, residual, n1.weight, n1.bias, wq["weight"], wq["bias"], n1.eps, self.nh, n1)
+            o = nn.functional.scaled_dot_product_attention(q, k, v, is_causal=True)
+            return blocks.GPT2Out.apply(o, x if s is None else s, wo["weight"], wo["bias"], n2.weight, n2.bias, w1["weight"], w1["bias"],
+                                        w2["weight"], w2["bias"], n2.eps, n2)
         y, s = (self.ln_1(x), x) if residual is None else self.ln_1.add(x, residual)
         y, s = self.ln_2.add(self._attention(y), s)
         return self._mlp(y), s
+
+    def _two_nodes(self, x) -> bool:
+        """Whether the block may run as two autograd nodes around the attention (``engine/blocks.py``): plain projections with biases on
+        the library's products, and its parameters all frozen, or all trained under a capture."""
+        if GPT2Block._attention is not _BLOCK_PARTS[0] or GPT2Block._mlp is not _BLOCK_PARTS[1] or "_attention" in self.__dict__ \
+                or "_mlp" in self.__dict__ or not blocks.available():
+            return False
+        m = self._modules
+        linears = [m[k] for k in _PROJECTIONS]
+        if not passable(*linears, m["ln_1"], m["ln_2"]):
+            return False
+        trained = linears[0].weight.requires_grad
+        if trained and fused.current_capture() is None:
+            return False
+        for lin in linears:
+            w, b = lin._parameters["weight"], lin.bias
+            if lin.lora_A is not None or b is None or w.requires_grad != trained or b.requires_grad != trained \
+                    or not fused._own_gemm_ok(x, w, b):
+                return False
+        for norm in (m["ln_1"], m["ln_2"]):
+            w, b = norm._parameters["weight"], norm.bias
+            if b is None or w.requires_grad != trained or b.requires_grad != trained or w.dtype != torch.bfloat16 or b.dtype != torch.bfloat16:
+                return False
+        return x.shape[-1] % 8 == 0 and x.shape[-1] <= 1024
 
     def _mlp(self, y):
         return self.mlp_c_proj(ops.activation(self.mlp_c_fc(y), "gelu_tanh"))
@@ -96,7 +127,9 @@ class GPT2Block(nn.Module):
         return self.attn_c_proj(o.transpose(1, 2).reshape(B, T, d))
 
 
-_BLOCK_FORWARD, _NORM_FORWARD = GPT2Block.forward, LayerNorm.forward
+_FORWARDS[GPT2Block] = GPT2Block.forward
+_BLOCK_PARTS = GPT2Block._attention, GPT2Block._mlp
+_PROJECTIONS = ("attn_c_attn", "attn_c_proj", "mlp_c_fc", "mlp_c_proj")
 
 
 class GPT2LMHeadModel(nn.Module):
@@ -113,12 +146,8 @@ class GPT2LMHeadModel(nn.Module):
         """Whether the blocks may run on the split stream, which calls neither a block's nor most norms' ``forward``: blocks and norms of
         these very classes with their own ``forward`` (none assigned to an instance or patched into the class, none compiled), and no
         hooks, on them or on all modules, that expect to be called with the unsplit tensors."""
-        if _has_any_global_hook() or GPT2Block.forward is not _BLOCK_FORWARD or LayerNorm.forward is not _NORM_FORWARD:
-            return False
-        norms = [n for blk in self.h if type(blk) is GPT2Block for n in (blk.ln_1, blk.ln_2)] + [self.ln_f]
-        return (all(type(blk) is GPT2Block for blk in self.h) and all(type(n) is LayerNorm for n in norms)
-                and not any(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks
-                            or "forward" in m.__dict__ or m._compiled_call_impl is not None for m in (*self.h, *norms)))
+        return all(type(blk) is GPT2Block and type(blk.ln_1) is LayerNorm and type(blk.ln_2) is LayerNorm for blk in self.h) \
+            and type(self.ln_f) is LayerNorm and passable(self.ln_f, *(m for blk in self.h for m in (blk, blk.ln_1, blk.ln_2)))
 
     def hidden_states(self, input_ids):
         B, T = input_ids.shape

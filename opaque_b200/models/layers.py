@@ -74,14 +74,21 @@ class Linear(nn.Module):
         return fused.dp_linear(x, self.weight, self.bias)
 
 
-_LINEAR_FORWARD = Linear.forward
+_FORWARDS: dict[type, object] = {}                       # classes whose modules may be passed by, with their own ``forward``
 
 
-def plain_linear(m: nn.Module) -> bool:
-    """Whether ``m`` may be passed by, its weight used without a call of the module: a :class:`Linear` with this file's ``forward``
-    (none patched in, assigned or compiled) and no hooks, on it or on all modules, that expect the call."""
-    return (type(m) is Linear and Linear.forward is _LINEAR_FORWARD and "forward" not in m.__dict__ and m._compiled_call_impl is None
-            and not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks or _has_any_global_hook()))
+def passable(*modules: nn.Module) -> bool:
+    """Whether the modules may be passed by, their parameters used without a call: of one of the framework's own classes (registered in
+    :data:`_FORWARDS`), with the class's ``forward`` (none patched in, assigned or compiled), and no hooks, on them or on all modules,
+    that expect the call."""
+    if _has_any_global_hook():
+        return False
+    for m in modules:
+        d = m.__dict__
+        if type(m).forward is not _FORWARDS.get(type(m), False) or "forward" in d or m._compiled_call_impl is not None \
+                or d["_forward_hooks"] or d["_forward_pre_hooks"] or d["_backward_hooks"] or d["_backward_pre_hooks"]:
+            return False
+    return True
 
 
 class Embedding(nn.Module):
@@ -166,6 +173,9 @@ class LayerNorm(nn.Module):
             return ops.add_layer_norm(x, residual, self.weight, self.bias, self.eps, layer=self)
         s = x + residual
         return self(s), s
+
+
+_FORWARDS.update({c: c.forward for c in (Linear, RMSNorm, LayerNorm)})
 
 
 class _LinearCrossEntropy(Function):

@@ -17,9 +17,10 @@ import torch
 from torch import nn
 
 from .. import ops
-from ..engine import fused
+from ..engine import blocks, fused
 from ..functional import functional_checkpoint
-from .layers import Embedding, LayerNorm, Linear, RMSNorm, linear_cross_entropy, per_example_token_weights, plain_linear
+from . import layers
+from .layers import _FORWARDS, Embedding, LayerNorm, Linear, RMSNorm, linear_cross_entropy, passable, per_example_token_weights
 
 
 @dataclasses.dataclass
@@ -222,7 +223,7 @@ class LlamaMLP(nn.Module):
         gp, up_ = self.gate_proj, self.up_proj
         if gp.lora_A is None and up_.lora_A is None and gp.bias is None and up_.bias is None:
             dp = self.down_proj
-            if dp.lora_A is None and dp.bias is None and plain_linear(dp):
+            if dp.lora_A is None and dp.bias is None and passable(dp):
                 # forward and backward as one function (the GLU backward rides in the down projection's data-gradient epilogue)
                 y = fused.glu_mlp(x, gp.weight, up_.weight, dp.weight, self.act)
                 if y is not None:
@@ -280,6 +281,18 @@ class LlamaDecoderLayer(nn.Module):
         inside the next norm kernel (forward), its two gradient branches only inside that kernel's backward.  Saves the
         four element-wise add launches per block that the plain form costs (two forward, two backward).
         Returns ``(mlp output, residual)``; the caller folds the last pair into the final norm."""
+        if self._two_nodes(x, cos, sin, pos):
+            att, mlp, n1, n2 = self.self_attn, self.mlp, self.input_layernorm, self.post_attention_layernorm
+            lq, lk, lv, lo = (att._modules[k]._parameters for k in _PROJECTIONS)
+            w_all = fused.stacked_weight_view([lq["weight"], lk["weight"], lv["weight"]])
+            if w_all is not None:
+                q, k, v, s = blocks.LoRAIn.apply(x, residual, n1.weight, w_all, lq["lora_A"], lq["lora_B"], lk["lora_A"], lk["lora_B"], lv["lora_A"],
+                                                 lv["lora_B"], cos, sin, att.q_proj.scaling, (n1.eps, n1.offset, ops.functional._MODES[n1.casting_mode]),
+                                                 (att.nh, att.nkv, att.hd))
+                o = nn.functional.scaled_dot_product_attention(q, k, v, is_causal=True, enable_gqa=att.nkv != att.nh, scale=att.scale)
+                return blocks.LoRAOut.apply(o, x if s is None else s, lo["weight"], lo["lora_A"], lo["lora_B"], n2.weight, mlp.gate_proj.weight,
+                                            mlp.up_proj.weight, mlp.down_proj.weight, att.o_proj.scaling,
+                                            (n2.eps, n2.offset, ops.functional._MODES[n2.casting_mode]), mlp.act, torch.is_grad_enabled())
         if residual is None:
             residual = x
             n = self.input_layernorm(x)
@@ -288,6 +301,34 @@ class LlamaDecoderLayer(nn.Module):
         a = self.self_attn(n, cos, sin, pos)
         n2, residual = self.post_attention_layernorm(a, residual)
         return self.mlp(n2), residual
+
+    def _two_nodes(self, x, cos, sin, pos) -> bool:
+        """Whether the block may run as two autograd nodes around the attention (``engine/blocks.py``): LoRA on all four projections of a
+        plain causal attention with rotary positions, everything else frozen and without biases, on the library's kernels."""
+        m = self._modules
+        att, mlp = m["self_attn"], m["mlp"]
+        if type(att) is not LlamaAttention or type(mlp) is not LlamaMLP or not att.use_rope or att.q_norm is not None or att.sinks is not None \
+                or att.softcap or att.local_rope or (att.window is not None and x.shape[1] > att.window) or pos is not None \
+                or not isinstance(cos, torch.Tensor) or att.hd % 16 or layers._ADAPTERS_OFF or not fused.one_node_lora() or not blocks.available() \
+                or any(t.dtype != torch.float32 or not t.is_contiguous() or t.data_ptr() & 15 for t in (cos, sin)):
+            return False
+        norms = m["input_layernorm"], m["post_attention_layernorm"]
+        adapted, plain = [att._modules[k] for k in _PROJECTIONS], [mlp._modules[k] for k in ("gate_proj", "up_proj", "down_proj")]
+        if not passable(self, att, mlp, *norms, *adapted, *plain):
+            return False
+        r, scaling = adapted[0].lora_A.shape[0] if adapted[0].lora_A is not None else 0, adapted[0].scaling
+        for i, lin in enumerate(adapted):
+            w, a, b = lin._parameters["weight"], lin.lora_A, lin.lora_B
+            if a is None or lin.bias is not None or w.requires_grad or not fused.lora_factors_ok(a, b) or not w.is_contiguous() \
+                    or not fused._own_gemm_ok(x, w) or (i < 3 and (a.shape[0] != r or lin.scaling != scaling)):
+                return False
+        for lin in plain:
+            w = lin._parameters["weight"]
+            if lin.lora_A is not None or lin.bias is not None or w.requires_grad or not fused._own_gemm_ok(x, w):
+                return False
+        wg, wu, wd = (lin._parameters["weight"] for lin in plain)
+        return (wg.shape == wu.shape and wg.stride(0) == wu.stride(0) and wd.shape[1] == wg.shape[0] and wg.shape[0] % 64 == 0
+                and all(type(n) is RMSNorm and not n.weight.requires_grad and n.weight.dtype == torch.bfloat16 for n in norms))
 
     def forward(self, h, cos, sin, pos):
         if self.parallel:
@@ -304,6 +345,10 @@ class LlamaDecoderLayer(nn.Module):
             return h + self.res * self.mlp(self.post_attention_layernorm(h))
         h = h + self.self_attn(self.input_layernorm(h), cos, sin, pos)
         return h + self.mlp(self.post_attention_layernorm(h))
+
+
+_FORWARDS.update({c: c.forward for c in (LlamaAttention, LlamaMLP, LlamaDecoderLayer)})
+_PROJECTIONS = ("q_proj", "k_proj", "v_proj", "o_proj")
 
 
 class LlamaModel(nn.Module):

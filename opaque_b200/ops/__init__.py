@@ -731,6 +731,18 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, b_layout: str = "nk", a2: torch.Te
     return out
 
 
+def _plan_code(M: int, N: int, K: int, K2: int, single: int) -> int:
+    """:func:`gemm`'s choice as a number: 0 for the pair kernel, else the single-CTA kernel's tile width."""
+    sms = lib.sm_count()
+    return 0 if not single and pick_gemm_plan(M, N, K, K2, sms) == "pair" else pick_tile_width(M, N, -(-K // 64) + -(-K2 // 64), sms)
+
+
+@functools.lru_cache(maxsize=None)
+def block_steps():
+    """The compiled launch sequences of whole sub-layers (``csrc/block_steps.cpp``), or ``None`` where they cannot be built or loaded."""
+    return lib.load_block_steps(_plan_code, DEFAULT_WAIT_BUDGET_S)
+
+
 def gemm_ref(a, b, *, b_layout="nk", a2=None, b2=None, bias=None, group_offs=None):
     """fp32 oracle of :func:`gemm`."""
     af = a.float()
@@ -899,7 +911,7 @@ from .functional import (activation, add_layer_norm, cross_entropy, cross_entrop
                          layer_norm, merge_heads3, plain_torch_ops, rms_norm, rms_norm_ref, rope_qk, rope_qk_ref, rope_tables, rows_group_sum_, swiglu)
 
 __all__ = [
-    "gemm", "gemm_pair", "lora_pack", "pick_gemm_plan", "gemm_glu", "gemm_glu_bwd", "pick_glu_bwd", "direct_norm2", "pick_norm_path", "pick_gemm_kernel", "die_map", "set_die_aware_tiles", "linear_ce_forward", "linear_ce_dlogits_", "gemm_glu_ref", "gemm_ref", "ghost_set_wide", "push_grad_", "wgrad_clip_per_example", "wgrad_clip_batch", "wgrad_clip_per_example_batch", "direct_norm2_batch", "ghost_norm_batch", "plain_torch_ops", "layer_norm", "add_layer_norm", "activation", "rows_group_sum_", "merge_heads3",
+    "gemm", "gemm_pair", "block_steps", "lora_pack", "pick_gemm_plan", "gemm_glu", "gemm_glu_bwd", "pick_glu_bwd", "direct_norm2", "pick_norm_path", "pick_gemm_kernel", "die_map", "set_die_aware_tiles", "linear_ce_forward", "linear_ce_dlogits_", "gemm_glu_ref", "gemm_ref", "ghost_set_wide", "push_grad_", "wgrad_clip_per_example", "wgrad_clip_batch", "wgrad_clip_per_example_batch", "direct_norm2_batch", "ghost_norm_batch", "plain_torch_ops", "layer_norm", "add_layer_norm", "activation", "rows_group_sum_", "merge_heads3",
     "DeviceWaitTimeout", "KernelLibraryError", "StatusWord", "clip_tree", "clip_weighted_sum", "cross_entropy",
     "cross_entropy_ref", "embedding_wgrad", "fused_add_rms_norm", "geglu", "ghost_norm", "ghost_norm_ref", "glu_ref",
     "philox_normal_add_", "pick_block_n", "pick_splits", "rms_norm", "rms_norm_ref", "rope_qk", "rope_qk_ref",

@@ -119,6 +119,20 @@ int ob_clip_tree(const void* const* leaf, void* const* out, const long long* num
                  double gamma, double shrink, double ulp, int automatic, float factor, double* partial, float* norms,
                  float* scale, float* clipped, void* stream);
 
+// RMSNorm: y = x * rsqrt(mean(x^2) + eps) * (offset + w); with `residual` x + residual first, stored to sum_out.  mode: casting.
+int ob_rmsnorm_fwd(const void* x, const void* residual, const void* w, void* y, void* sum_out, float* rstd, long long rows, int H,
+                   float eps, float offset, int mode, void* stream);
+int ob_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd, const void* dsum_in, void* dx,
+                   float* dw_per_example, const int* seg_offsets, int num_examples, int rows_per_example, long long rows, int H,
+                   float offset, void* stream);
+// dgate, dup (pitch ld_out) of act(gate) * up (pitch ld_in) for dh [rows, I]; act: 0 silu, 1 gelu erf, 2 gelu tanh.
+int ob_glu_bwd(const void* dh, const void* gate, const void* up, void* dgate, void* dup, long long rows, int I, long long ld_in,
+               long long ld_out, int act, int sms, void* stream);
+// Rotary embedding of q and k read through element strides (batch, token, head); contiguous outputs [rows, heads, D].
+int ob_rope_qk_oop(const void* q_in, const void* k_in, void* q_out, void* k_out, const float* cos_t, const float* sin_t,
+                   const int* pos, long long rows, int seq_len, int Hq, int Hk, int D, long long q_sb, long long q_st,
+                   long long q_sh, long long k_sb, long long k_st, long long k_sh, int backward, int sms, void* stream);
+
 // LayerNorm over the last dimension (bf16 in/out, fp32 statistics saved per row).
 int ob_layernorm_fwd(const void* x, const void* w, const void* b, void* y, float* mean, float* rstd, long long rows,
                      int H, float eps, void* stream);

@@ -1,0 +1,468 @@
+// Launch sequences of whole decoder sub-layers: what runs between two library attention calls, forward or backward, as ONE call from
+// Python.  Written in Python, a launch of these sequences costs 15 to 25 us of host time (allocation, strides, addresses, plan, call),
+// more than most kernels of a short batch run; here 3 to 4.
+//
+// The functions allocate their results and launch the library's kernels (bound by address, see api.h) on the current stream; they
+// keep nothing.  The callers (engine/blocks.py) have checked types, layouts and alignment.  A launch that fails raises through the
+// Python check that the other entry points use; no C++ exception leaves a function.
+#define PY_SSIZE_T_CLEAN
+#include <Python.h>
+
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <array>
+#include <initializer_list>
+#include <map>
+
+#include "api.h"
+
+#ifdef OB_DIGEST
+__attribute__((used)) static const char digest[] = OB_DIGEST;      // of this file, api.h and torch's version (utils/build.py)
+#endif
+
+namespace {
+
+using at::Tensor;
+
+#define OB_ENTRIES(X)                                                                                                          \
+  X(ob_gemm_tn) X(ob_gemm_pair) X(ob_gemm_pair_glu_bwd) X(ob_glu_bwd) X(ob_rmsnorm_fwd) X(ob_rmsnorm_bwd) X(ob_layernorm_fwd)  \
+  X(ob_layernorm_bwd_dx) X(ob_add_layernorm_fwd) X(ob_add_layernorm_bwd_dx) X(ob_activation) X(ob_merge_heads3) X(ob_lora_pack) \
+  X(ob_rope_qk_oop) X(ob_wgrad_clip_batch)
+#define X(name) decltype(&name) p_##name = nullptr;
+OB_ENTRIES(X)
+#undef X
+
+PyObject *g_check = nullptr, *g_plan = nullptr;      // lib.check(rc, what); (M, N, K, K2, single) -> 0 pair, 64 or 256: tile width
+int g_sms = 0;
+double g_budget = 0.0;
+
+struct PythonError {};                               // a Python exception is set
+
+void done(int rc, const char* what) {
+  PyObject* r = PyObject_CallFunction(g_check, "is", rc, what);
+  if (r == nullptr) throw PythonError();
+  Py_DECREF(r);
+}
+void* stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
+// Launches without the interpreter lock (a full launch queue blocks); the arguments are evaluated before it is given up.
+template <class F, class... A>
+void launch(const char* what, F entry, A... args) {
+  void* const st = stream();
+  PyThreadState* const thread = PyEval_SaveThread();
+  const int rc = entry(args..., st);
+  PyEval_RestoreThread(thread);
+  done(rc, what);
+}
+#define LAUNCH(name, ...) launch(#name, p_##name, __VA_ARGS__)
+
+void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
+const float* f32(const Tensor& t) { return static_cast<const float*>(ptr(t)); }
+Tensor empty(std::initializer_list<int64_t> shape, const Tensor& like) { return at::empty(shape, like.options()); }
+Tensor empty_f32(std::initializer_list<int64_t> shape, const Tensor& like) { return at::empty(shape, like.options().dtype(at::kFloat)); }
+// contiguous and on a 16-byte boundary
+Tensor vec16(const Tensor& t) {
+  if (!t.is_contiguous()) return t.contiguous();
+  return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0 ? t : t.clone(at::MemoryFormat::Contiguous);
+}
+Tensor rows(const Tensor& t) { return t.defined() ? vec16(t.reshape({-1, t.size(-1)})) : t; }
+
+// ------------------------------------------------------------------------------------------------------- single launches
+
+// The choice of kernel and tile is the Python rule's; it is asked once per shape.
+int plan(int64_t M, int64_t N, int64_t K, int64_t K2, bool single) {
+  static std::map<std::array<int64_t, 5>, int> known;
+  const std::array<int64_t, 5> key{M, N, K, K2, single};
+  const auto at = known.find(key);
+  if (at != known.end()) return at->second;
+  PyObject* r = PyObject_CallFunction(g_plan, "LLLLi", (long long)M, (long long)N, (long long)K, (long long)K2, (int)single);
+  if (r == nullptr) throw PythonError();
+  const int width = static_cast<int>(PyLong_AsLong(r));
+  Py_DECREF(r);
+  if (PyErr_Occurred()) throw PythonError();
+  if (known.size() >= 4096) known.clear();
+  return known[key] = width;
+}
+
+struct Opt {                                         // the optional parts of a product
+  Tensor bias, a2, b2;
+  bool kn2 = false, single = false;
+  float alpha = 1.f;
+};
+// a [M, K] times b ([N, K], or [K, N] with kn), as ops.gemm
+Tensor product(const Tensor& a, const Tensor& b, int64_t N, bool kn, const Opt& o = {}) {
+  const int64_t M = a.size(0), K = a.size(1), K2 = o.a2.defined() ? o.a2.size(1) : 0;
+  Tensor out = empty({M, N}, a);
+  const int width = plan(M, N, K, K2, o.single);
+  const int64_t lda2 = K2 ? o.a2.stride(0) : 0, ldb2 = K2 ? o.b2.stride(0) : 0;
+  if (width == 0)
+    LAUNCH(ob_gemm_pair, ptr(a), ptr(b), nullptr, ptr(o.a2), ptr(o.b2), nullptr, ptr(o.bias), ptr(out), nullptr, nullptr, M, (int)N, (int)K, (int)K2,
+           a.stride(0), b.stride(0), lda2, ldb2, N, kn, o.kn2, 0, 0, -1, nullptr, g_budget, g_sms);
+  else
+    LAUNCH(ob_gemm_tn, ptr(a), ptr(b), ptr(o.a2), ptr(o.b2), ptr(o.bias), ptr(out), M, (int)N, (int)K, (int)K2, a.stride(0), b.stride(0), lda2, ldb2,
+           N, kn, o.kn2, o.alpha, nullptr, 0, width, nullptr, g_budget, g_sms);
+  return out;
+}
+Opt with_bias(const Tensor& bias) { Opt o; o.bias = bias; return o; }
+Opt scaled(double alpha) { Opt o; o.alpha = static_cast<float>(alpha); o.single = true; return o; }
+Opt segment(const Tensor& a2, const Tensor& b2, bool kn2) { Opt o; o.a2 = a2; o.b2 = b2; o.kn2 = kn2; return o; }
+
+// s = x + r (s = x without r) and its norm; stats: mean and rstd [2, rows]
+struct Normed {
+  Tensor y, s, stats;
+};
+Normed layer_norm(const Tensor& x, const Tensor& r, const Tensor& w, const Tensor& b, double eps) {
+  const int64_t R = x.size(0);
+  Normed n{empty({R, x.size(1)}, x), x, empty_f32({2, R}, x)};
+  float* mean = n.stats.data_ptr<float>();
+  if (!r.defined()) {
+    LAUNCH(ob_layernorm_fwd, ptr(x), ptr(w), ptr(b), ptr(n.y), mean, mean + R, R, (int)x.size(1), (float)eps);
+  } else {
+    n.s = empty({R, x.size(1)}, x);
+    LAUNCH(ob_add_layernorm_fwd, ptr(x), ptr(r), ptr(w), ptr(b), ptr(n.y), ptr(n.s), mean, mean + R, R, (int)x.size(1), (float)eps);
+  }
+  return n;
+}
+Tensor layer_norm_bwd(const Tensor& dy, const Tensor& s, const Tensor& w, const Tensor& stats, const Tensor& ds) {
+  const int64_t R = s.size(0);
+  Tensor dx = empty({R, s.size(1)}, s);
+  const float* mean = f32(stats);
+  if (!ds.defined())
+    LAUNCH(ob_layernorm_bwd_dx, ptr(dy), ptr(s), ptr(w), mean, mean + R, ptr(dx), R, (int)s.size(1));
+  else
+    LAUNCH(ob_add_layernorm_bwd_dx, ptr(dy), ptr(s), ptr(w), mean, mean + R, ptr(ds), ptr(dx), R, (int)s.size(1));
+  return dx;
+}
+Normed rms_norm(const Tensor& x, const Tensor& r, const Tensor& w, double eps, double offset, int mode) {
+  const int64_t R = x.size(0);
+  Normed n{empty({R, x.size(1)}, x), r.defined() ? empty({R, x.size(1)}, x) : x, empty_f32({R}, x)};
+  LAUNCH(ob_rmsnorm_fwd, ptr(x), ptr(r), ptr(w), ptr(n.y), r.defined() ? ptr(n.s) : nullptr, n.stats.data_ptr<float>(), R, (int)x.size(1),
+         (float)eps, (float)offset, mode);
+  return n;
+}
+Tensor rms_norm_bwd(const Tensor& dy, const Tensor& s, const Tensor& w, const Tensor& rstd, const Tensor& ds, double offset) {
+  Tensor dx = empty({s.size(0), s.size(1)}, s);
+  LAUNCH(ob_rmsnorm_bwd, ptr(dy), ptr(s), ptr(w), f32(rstd), ptr(ds), ptr(dx), nullptr, nullptr, 0, 0, s.size(0), (int)s.size(1), (float)offset);
+  return dx;
+}
+constexpr int GELU_TANH = 2;
+Tensor gelu(const Tensor& x, const Tensor& dy) {
+  Tensor out = empty({x.size(0), x.size(1)}, x);
+  LAUNCH(ob_activation, ptr(x), ptr(dy), ptr(out), x.numel(), GELU_TANH, g_sms);
+  return out;
+}
+// q, k [B, T, heads, hd] through their strides -> rotated, contiguous
+bool rope_reads(const Tensor& t) {
+  return t.stride(3) == 1 && (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0 && ((t.stride(0) | t.stride(1) | t.stride(2)) & 7) == 0;
+}
+std::pair<Tensor, Tensor> rope(Tensor q, Tensor k, const Tensor& cs, const Tensor& sn, bool backward) {
+  if (!rope_reads(q)) q = q.clone(at::MemoryFormat::Contiguous);
+  if (!rope_reads(k)) k = k.clone(at::MemoryFormat::Contiguous);
+  const int64_t B = q.size(0), T = q.size(1), hd = q.size(3);
+  Tensor qo = empty({B, T, q.size(2), hd}, q), ko = empty({B, T, k.size(2), hd}, k);
+  LAUNCH(ob_rope_qk_oop, ptr(q), ptr(k), ptr(qo), ptr(ko), f32(cs), f32(sn), nullptr, B * T, (int)T, (int)q.size(2), (int)k.size(2), (int)hd, q.stride(0),
+         q.stride(1), q.stride(2), k.stride(0), k.stride(1), k.stride(2), backward, g_sms);
+  return {qo, ko};
+}
+// three gradients [B, heads, T, hd] -> [B * T, 3 * heads * hd]
+Tensor merge_heads(const Tensor& q, const Tensor& k, const Tensor& v) {
+  const int64_t B = q.size(0), H = q.size(1), T = q.size(2), hd = q.size(3);
+  Tensor out = empty({B * T, 3 * H * hd}, q);
+  const Tensor* parts[3] = {&q, &k, &v};
+  long long strides[9];
+  bool ok = hd % 8 == 0;
+  for (int i = 0; i < 3; ++i) {
+    ok = ok && parts[i]->scalar_type() == at::kBFloat16 && rope_reads(*parts[i]);
+    for (int j = 0; j < 3; ++j) strides[3 * i + j] = parts[i]->stride(j);
+  }
+  if (ok) {
+    LAUNCH(ob_merge_heads3, ptr(q), ptr(k), ptr(v), strides, ptr(out), B, (int)T, (int)H, (int)hd, g_sms);
+  } else {
+    Tensor v5 = out.view({B, T, 3, H, hd});
+    for (int i = 0; i < 3; ++i) v5.select(2, i).copy_(parts[i]->transpose(1, 2));
+  }
+  return out;
+}
+
+// ------------------------------------------------------------------------------------------------------- Python arguments
+
+struct Args {
+  PyObject* const* a;
+  Py_ssize_t n, i = 0;
+  PyObject* next() {
+    if (i >= n) {
+      PyErr_SetString(PyExc_TypeError, "too few arguments");
+      throw PythonError();
+    }
+    return a[i++];
+  }
+  Tensor tensor() {
+    PyObject* o = next();
+    if (!THPVariable_Check(o)) {
+      PyErr_Format(PyExc_TypeError, "expected a tensor, got %.80s", Py_TYPE(o)->tp_name);
+      throw PythonError();
+    }
+    return THPVariable_Unpack(o);
+  }
+  Tensor optional() {
+    if (i < n && a[i] == Py_None) {
+      ++i;
+      return Tensor();
+    }
+    return tensor();
+  }
+  double number() {
+    const double v = PyFloat_AsDouble(next());
+    if (v == -1.0 && PyErr_Occurred()) throw PythonError();
+    return v;
+  }
+  long long integer() {
+    const long long v = PyLong_AsLongLong(next());
+    if (v == -1 && PyErr_Occurred()) throw PythonError();
+    return v;
+  }
+};
+PyObject* pack(std::initializer_list<Tensor> ts) {
+  PyObject* out = PyTuple_New(static_cast<Py_ssize_t>(ts.size()));
+  if (out == nullptr) throw PythonError();
+  Py_ssize_t i = 0;
+  for (const Tensor& t : ts) {
+    PyObject* o = t.defined() ? THPVariable_Wrap(t) : Py_NewRef(Py_None);
+    if (o == nullptr) {
+      Py_DECREF(out);
+      throw PythonError();
+    }
+    PyTuple_SET_ITEM(out, i++, o);
+  }
+  return out;
+}
+template <PyObject* (*F)(Args&)>
+PyObject* call(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  Args args{a, n};
+  try {
+    return F(args);
+  } catch (const PythonError&) {
+  } catch (const std::exception& e) {
+    PyErr_SetString(PyExc_RuntimeError, e.what());
+  } catch (...) {
+    PyErr_SetString(PyExc_RuntimeError, "unknown C++ exception");
+  }
+  return nullptr;
+}
+
+// ------------------------------------------------------------------------------------------------------- GPT-2
+
+// (x, residual | None, ln_w, ln_b, w, b, eps) -> y, s, stats, qkv
+PyObject* gpt2_in(Args& a) {
+  const Tensor x = rows(a.tensor()), r = rows(a.optional()), lw = a.tensor(), lb = a.tensor(), w = a.tensor(), b = a.tensor();
+  const Normed n = layer_norm(x, r, lw, lb, a.number());
+  return pack({n.y, n.s, n.stats, product(n.y, w, w.size(0), false, with_bias(b))});
+}
+// (dq, dk, dv, w, s, ln_w, stats, ds | None, need_dx) -> g, dy, dx
+PyObject* gpt2_in_bwd(Args& a) {
+  const Tensor dq = a.tensor(), dk = a.tensor(), dv = a.tensor(), w = a.tensor(), s = a.tensor(), lw = a.tensor(), stats = a.tensor(),
+               ds = rows(a.optional()), g = merge_heads(dq, dk, dv);
+  Tensor dy, dx;
+  if (a.integer()) {
+    dy = product(g, w, s.size(1), true);
+    dx = layer_norm_bwd(dy, s, lw, stats, ds);
+  }
+  return pack({g, dy, dx});
+}
+// (o [B, heads, T, hd], residual, wo, bo, ln_w, ln_b, w1, b1, w2, b2, eps) -> o2, y, s, stats, f, h, m
+PyObject* gpt2_out(Args& a) {
+  const Tensor o = a.tensor(), r = rows(a.tensor()), wo = a.tensor(), bo = a.tensor(), lw = a.tensor(), lb = a.tensor(), w1 = a.tensor(),
+               b1 = a.tensor(), w2 = a.tensor(), b2 = a.tensor();
+  const Tensor o2 = vec16(o.transpose(1, 2).reshape({o.size(0) * o.size(2), -1}));
+  const Normed n = layer_norm(product(o2, wo, wo.size(0), false, with_bias(bo)), r, lw, lb, a.number());
+  const Tensor f = product(n.y, w1, w1.size(0), false, with_bias(b1)), h = gelu(f, Tensor());
+  return pack({o2, n.y, n.s, n.stats, f, h, product(h, w2, w2.size(0), false, with_bias(b2))});
+}
+// (dm, f, w2, w1, s, ln_w, stats, ds, wo) -> g2, g1, dy, dx, do [rows, heads * hd]
+PyObject* gpt2_out_bwd(Args& a) {
+  const Tensor g2 = rows(a.tensor()), f = a.tensor(), w2 = a.tensor(), w1 = a.tensor(), s = a.tensor(), lw = a.tensor(), stats = a.tensor(),
+               ds = rows(a.tensor()), wo = a.tensor();
+  const Tensor g1 = gelu(f, product(g2, w2, w2.size(1), true)), dy = product(g1, w1, w1.size(1), true);
+  const Tensor dx = layer_norm_bwd(dy, s, lw, stats, ds);
+  return pack({g2, g1, dy, dx, product(dx, wo, wo.size(1), true)});
+}
+
+// ------------------------------------------------------------------------------------------------------- Llama with LoRA
+
+// (x [B, T, d], residual | None, norm_w, eps, offset, mode, aq, bq, ak, bk, av, bv, scaling, w_all, cos, sin, heads, kv heads, hd)
+//   -> y, s, rstd, a_cat, b_block, xa, q, k [B, T, heads, hd] rotated, qkv
+PyObject* lora_in(Args& a) {
+  const Tensor x3 = a.tensor(), x = rows(x3), r = rows(a.optional()), nw = a.tensor();
+  const double eps = a.number(), offset = a.number();
+  const int mode = static_cast<int>(a.integer());
+  const Tensor aq = a.tensor(), bq = a.tensor(), ak = a.tensor(), bk = a.tensor(), av = a.tensor(), bv = a.tensor();
+  const double scaling = a.number();
+  const Tensor w_all = a.tensor(), cs = a.tensor(), sn = a.tensor();
+  const int64_t nh = a.integer(), nkv = a.integer(), hd = a.integer(), rank = aq.size(0);
+  const Normed n = rms_norm(x, r, nw, eps, offset, mode);
+  const Tensor a_cat = empty({3 * rank, aq.size(1)}, aq), b_block = empty({bq.size(0) + bk.size(0) + bv.size(0), 3 * rank}, aq);
+  LAUNCH(ob_lora_pack, ptr(aq), ptr(ak), ptr(av), ptr(bq), ptr(bk), ptr(bv), ptr(a_cat), ptr(b_block), (int)rank, (int)aq.size(1), (int)bq.size(0),
+         (int)bk.size(0), (int)bv.size(0), g_sms);
+  const Tensor xa = product(n.y, a_cat, 3 * rank, false, scaled(scaling)), qkv = product(n.y, w_all, w_all.size(0), false, segment(xa, b_block, false));
+  const Tensor heads = qkv.view({x3.size(0), x3.size(1), nh + 2 * nkv, hd});
+  const auto [q, k] = rope(heads.narrow(2, 0, nh), heads.narrow(2, nh, nkv), cs, sn, false);
+  return pack({n.y, n.s, n.stats, a_cat, b_block, xa, q, k, qkv});
+}
+// (dq, dk, dv [B, heads, T, hd], cos, sin, b_block, scaling, w_all, a_cat, s, norm_w, rstd, ds | None, offset, need_dx) -> g, q_all, dx
+PyObject* lora_in_bwd(Args& a) {
+  const Tensor dq = a.tensor(), dk = a.tensor(), dv = a.tensor(), cs = a.tensor(), sn = a.tensor(), b_block = a.tensor();
+  const double scaling = a.number();
+  const Tensor w_all = a.tensor(), a_cat = a.tensor(), s = a.tensor(), nw = a.tensor(), rstd = a.tensor(), ds = rows(a.optional());
+  const double offset = a.number();
+  const int64_t R = dq.size(0) * dq.size(2);
+  const auto [q, k] = rope(dq.transpose(1, 2), dk.transpose(1, 2), cs, sn, true);
+  const Tensor g = at::cat({q.view({R, -1}), k.view({R, -1}), dv.transpose(1, 2).reshape({R, -1})}, 1);
+  const Tensor q_all = product(g, b_block, b_block.size(1), true, scaled(scaling));
+  Tensor dx;
+  if (a.integer()) dx = rms_norm_bwd(product(g, w_all, w_all.size(1), true, segment(q_all, a_cat, true)), s, nw, rstd, ds, offset);
+  return pack({g, q_all, dx});
+}
+// (o [B, heads, T, hd], a, scaling, wo, b, residual, norm_w, eps, offset, mode, w_gate, w_up, act, w_down, keep)
+//   -> o2, xa, s, rstd, g | None, u | None, m
+PyObject* lora_out(Args& a) {
+  const Tensor o = a.tensor(), la = a.tensor();
+  const double scaling = a.number();
+  const Tensor wo = a.tensor(), lb = a.tensor(), r = rows(a.tensor()), nw = a.tensor();
+  const double eps = a.number(), offset = a.number();
+  const int mode = static_cast<int>(a.integer());
+  const Tensor wg = a.tensor(), wu = a.tensor();
+  const int act = static_cast<int>(a.integer());
+  const Tensor wd = a.tensor();
+  const bool keep = a.integer() != 0;
+  const Tensor o2 = vec16(o.transpose(1, 2).reshape({o.size(0) * o.size(2), -1})), xa = product(o2, la, la.size(0), false, scaled(scaling));
+  const Normed n = rms_norm(product(o2, wo, wo.size(0), false, segment(xa, lb, false)), r, nw, eps, offset, mode);
+  const int64_t M = o2.size(0), I = wg.size(0), K = wg.size(1);
+  const Tensor h = empty({M, I}, o2), g = keep ? empty({M, I}, o2) : Tensor(), u = keep ? empty({M, I}, o2) : Tensor();
+  LAUNCH(ob_gemm_pair, ptr(n.y), ptr(wg), ptr(wu), nullptr, nullptr, nullptr, nullptr, ptr(h), ptr(g), ptr(u), M, (int)(2 * I), (int)K, 0, K,
+         wg.stride(0), 0, 0, I, 0, 0, 1, act, -1, nullptr, g_budget, g_sms);
+  return pack({o2, xa, n.s, n.stats, g, u, product(h, wd, wd.size(0), false)});
+}
+// (dm, w_down, g, u, act, fused, w_gate, w_up, s, norm_w, rstd, ds, offset, b, scaling, wo, a) -> dx, q, do [rows, heads * hd]
+PyObject* lora_out_bwd(Args& a) {
+  const Tensor d2 = rows(a.tensor()), wd = a.tensor(), g = a.tensor(), u = a.tensor();
+  const int act = static_cast<int>(a.integer());
+  const bool one_launch = a.integer() != 0;
+  const Tensor wg = a.tensor(), wu = a.tensor(), s = a.tensor(), nw = a.tensor(), rstd = a.tensor(), ds = rows(a.tensor());
+  const double offset = a.number();
+  const Tensor lb = a.tensor();
+  const double scaling = a.number();
+  const Tensor wo = a.tensor(), la = a.tensor();
+  const int64_t M = g.size(0), I = g.size(1);
+  Tensor dg = empty({M, I}, g), du = empty({M, I}, g);
+  if (one_launch) {
+    LAUNCH(ob_gemm_pair_glu_bwd, ptr(d2), ptr(wd), ptr(g), ptr(u), ptr(dg), ptr(du), M, (int)I, (int)d2.size(1), d2.stride(0), wd.stride(0), I, I, 1,
+           act, nullptr, g_budget, g_sms);
+  } else {
+    const Tensor dh = product(d2, wd, I, true);
+    LAUNCH(ob_glu_bwd, ptr(dh), ptr(g), ptr(u), ptr(dg), ptr(du), M, (int)I, I, I, act, g_sms);
+  }
+  const Tensor dy = product(dg, wg, wg.size(1), true, segment(du, wu, true));
+  dg.reset();
+  du.reset();
+  const Tensor dx = rms_norm_bwd(dy, s, nw, rstd, ds, offset), q = product(dx, lb, lb.size(1), true, scaled(scaling));
+  return pack({dx, q, product(dx, wo, wo.size(1), true, segment(q, la, true))});
+}
+
+// Stored (not accumulated) weight gradients of every example, one launch:
+// (jobs, out, seg_offsets, groups, group_stride, status address), jobs: (a, b, out_offset, ldm, ldn, n_valid), tiles of 64 columns.
+PyObject* store_wgrads(Args& args) {
+  PyObject* jobs = args.next();
+  const Tensor out = args.tensor(), seg = args.tensor();
+  const long long groups = args.integer(), group_stride = args.integer(), status = args.integer();
+  if (!PyTuple_Check(jobs) || PyTuple_GET_SIZE(jobs) > 8 || out.scalar_type() != at::kFloat) {
+    PyErr_SetString(PyExc_TypeError, "store_wgrads: at most eight jobs and an fp32 destination");
+    throw PythonError();
+  }
+  const int count = static_cast<int>(PyTuple_GET_SIZE(jobs));
+  const long long room = static_cast<long long>(out.storage().nbytes() / 4) - out.storage_offset();
+  ob_wgrad_desc d[8] = {};
+  for (int i = 0; i < count; ++i) {
+    PyObject* t = PyTuple_GET_ITEM(jobs, i);
+    if (!PyTuple_Check(t) || PyTuple_GET_SIZE(t) != 6) {
+      PyErr_SetString(PyExc_TypeError, "store_wgrads: a job is (a, b, out_offset, ldm, ldn, n_valid)");
+      throw PythonError();
+    }
+    Args j{&PyTuple_GET_ITEM(t, 0), 6};
+    const Tensor a = j.tensor(), b = j.tensor();
+    ob_wgrad_desc& p = d[i];
+    p.out_offset = j.integer();
+    p.ldm = j.integer();
+    p.ldn = j.integer();
+    p.n_valid = static_cast<int>(j.integer());
+    p.a = ptr(a);
+    p.b = ptr(b);
+    p.seg_offsets = static_cast<const int*>(ptr(seg));
+    p.lda = a.stride(0);
+    p.ldb = b.stride(0);
+    p.group_stride = group_stride;
+    p.T = static_cast<int>(a.size(0));
+    p.M = static_cast<int>(a.size(1));
+    p.N = static_cast<int>(b.size(1));
+    p.num_groups = static_cast<int>(groups);
+    p.splits = 1;
+    const long long n_lim = p.n_valid && p.n_valid < p.N ? p.n_valid : p.N;
+    const long long hi = p.out_offset + (groups - 1) * group_stride + (p.M - 1) * p.ldm + (n_lim - 1) * p.ldn;
+    if (a.scalar_type() != at::kBFloat16 || b.scalar_type() != at::kBFloat16 || b.size(0) != p.T || a.stride(1) != 1 || b.stride(1) != 1 ||
+        p.out_offset < 0 || p.ldm < 0 || p.ldn < 0 || hi >= room) {
+      PyErr_Format(PyExc_ValueError, "store_wgrads: job %d is not a pair of row-major bf16 matrices or would write element %lld of %lld", i, hi, room);
+      throw PythonError();
+    }
+  }
+  LAUNCH(ob_wgrad_clip_batch, d, count, out.data_ptr<float>(), nullptr, 0, 64, reinterpret_cast<int*>(status), g_budget, g_sms);
+  Py_RETURN_NONE;
+}
+
+// bind(name, address); setup(check, plan, sms, budget)
+PyObject* bind(Args& a) {
+  const char* name = PyUnicode_AsUTF8(a.next());
+  if (name == nullptr) throw PythonError();
+  void* p = PyLong_AsVoidPtr(a.next());
+  if (p == nullptr) throw PythonError();
+#define X(entry) \
+  if (!strcmp(name, #entry)) { p_##entry = reinterpret_cast<decltype(&entry)>(p); Py_RETURN_NONE; }
+  OB_ENTRIES(X)
+#undef X
+  PyErr_Format(PyExc_KeyError, "%s", name);
+  throw PythonError();
+}
+PyObject* setup(Args& a) {
+  PyObject *check = a.next(), *plan_fn = a.next();
+  const long long sms = a.integer();
+  g_budget = a.number();
+  g_sms = static_cast<int>(sms);
+  Py_XDECREF(g_check);
+  Py_XDECREF(g_plan);
+  g_check = Py_NewRef(check);
+  g_plan = Py_NewRef(plan_fn);
+  const char* missing = nullptr;
+#define X(entry) \
+  if (p_##entry == nullptr) missing = #entry;
+  OB_ENTRIES(X)
+#undef X
+  if (missing != nullptr) {
+    PyErr_Format(PyExc_RuntimeError, "%s is not bound", missing);
+    throw PythonError();
+  }
+  Py_RETURN_NONE;
+}
+PyObject* entries(Args&) {
+#define X(entry) #entry " "
+  return PyUnicode_FromString(OB_ENTRIES(X));
+#undef X
+}
+
+#define METHOD(f) {#f, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(&call<f>)), METH_FASTCALL, nullptr}
+PyMethodDef methods[] = {METHOD(gpt2_in), METHOD(gpt2_in_bwd), METHOD(gpt2_out), METHOD(gpt2_out_bwd), METHOD(lora_in), METHOD(lora_in_bwd),
+                         METHOD(lora_out), METHOD(lora_out_bwd), METHOD(store_wgrads), METHOD(bind), METHOD(setup), METHOD(entries),
+                         {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_blocks", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__blocks(void) { return PyModule_Create(&module); }

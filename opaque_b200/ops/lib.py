@@ -145,6 +145,27 @@ def load() -> _Entries:
     return entries
 
 
+def load_block_steps(plan, budget: float):
+    """The extension of ``csrc/block_steps.cpp`` with the library's entry points bound, or ``None`` (with a warning) where it can neither
+    be built nor loaded: the callers then run their operations one by one."""
+    import importlib.util
+    entries = load()
+    for force in (False, True):                 # as for the compiled caller
+        try:
+            path = _build.build_block_steps(force)
+            spec = importlib.util.spec_from_file_location("opaque_b200.ops._blocks", path)
+            steps = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(steps)
+            for name in steps.entries().split():
+                steps.bind(name, ctypes.cast(getattr(entries._cdll, name), c_void_p).value)
+            steps.setup(check, plan, sm_count(), budget)
+            return steps
+        except (RuntimeError, OSError, ImportError) as exc:
+            reason = exc
+    warnings.warn(f"no compiled launch sequences, decoder blocks run operation by operation: {reason}", RuntimeWarning, stacklevel=3)
+    return None
+
+
 def available() -> bool:
     """True when a CUDA device is present and the library loads."""
     if not torch.cuda.is_available():

@@ -204,6 +204,46 @@ def build_launcher(signatures: dict[str, str], force: bool = False) -> Path:
     return target
 
 
+def block_steps_ext_path() -> Path:
+    suffix = sysconfig.get_config_var("EXT_SUFFIX") or ".so"
+    return PKG / "ops" / ("_blocks" + suffix)
+
+
+def build_block_steps(force: bool = False) -> Path:
+    """Compile ``ops/csrc/block_steps.cpp`` against torch's C++ headers, in-tree.  The extension carries a digest of its sources and of
+    torch's version, so an installed copy is fresh without any other file."""
+    import torch
+    target, sources = block_steps_ext_path(), [CSRC / "block_steps.cpp", CSRC / "api.h"]
+    text = torch.__version__ + "".join(p.read_text() for p in sources)
+    mark = "opaque-blocks:" + hashlib.sha256(text.encode()).hexdigest()
+
+    def fresh() -> bool:
+        return target.exists() and mark.encode() in target.read_bytes()
+    if not force and fresh():
+        return target
+    gxx = _find("g++", ["/usr/bin/g++"])
+    if gxx is None:
+        raise RuntimeError("g++ not found: cannot build the block steps")
+    from torch.utils import cpp_extension
+    with _build_lock(target):
+        if not force and fresh():
+            return target
+        tmp = target.with_suffix(f".tmp{os.getpid()}")
+        try:
+            cuda = Path(_find("nvcc", ["/usr/local/cuda/bin/nvcc"]) or "/usr/local/cuda/bin/nvcc").resolve().parent.parent
+            res = subprocess.run(
+                [gxx, "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+                 f'-DOB_DIGEST="{mark}"', *(f"-I{d}" for d in cpp_extension.include_paths()), f"-I{sysconfig.get_paths()['include']}",
+                 f"-I{cuda / 'include'}", str(sources[0]), "-o", str(tmp), *(f"-L{d}" for d in cpp_extension.library_paths()),
+                 "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"], capture_output=True, text=True)
+            if res.returncode != 0:
+                raise RuntimeError("g++ failed:\n" + res.stdout + res.stderr)
+            os.replace(tmp, target)
+        finally:
+            tmp.unlink(missing_ok=True)
+    return target
+
+
 def accounting_ext_path() -> Path:
     suffix = sysconfig.get_config_var("EXT_SUFFIX") or ".so"
     return PKG / "accounting" / ("_native" + suffix)
@@ -241,6 +281,7 @@ def build_all(force: bool = False) -> None:
     build_kernels(force)
     from ..ops import lib
     build_launcher(lib.launch_signatures(), force)
+    build_block_steps(force)
     build_accounting(force)
 
 

@@ -1,0 +1,133 @@
+"""Decoder blocks as two autograd nodes (engine/blocks.py) against the same blocks with one node per operation."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(model, batch, mode, unsplit):
+    """Losses, gradients and the number of nodes taken; ``unsplit``: a hook on one projection of every block forbids the two nodes."""
+    from opaque_b200.engine import blocks
+    from opaque_b200.engine.fused import FusedDPEngine
+    from opaque_b200.random import key
+    hooks = []
+    if unsplit:
+        layers = model.h if hasattr(model, "h") else model.model.layers
+        hooks = [(blk.mlp_c_fc if hasattr(blk, "mlp_c_fc") else blk.mlp.down_proj).register_forward_hook(lambda *a: None) for blk in layers]
+    taken, apply = [], {}
+    for cls in (blocks.GPT2In, blocks.GPT2Out, blocks.LoRAIn, blocks.LoRAOut):
+        apply[cls] = cls.forward
+        cls.forward = staticmethod(lambda ctx, *a, f=cls.forward: (taken.append(1), f(ctx, *a))[1])
+    try:
+        if mode == "capture":
+            eng = FusedDPEngine(model, clipping_norm=1.0, noise_multiplier=0.0, normalize_by=2.0, key=key(0), microbatch_size=batch["labels"].shape[0])
+            res = eng.accumulate(model.per_example_loss, batch)
+            out = [res.losses, res.norms, eng.space.grad.local.clone()]
+        elif mode == "autograd":                       # without a capture: gradients of the adapters through torch's engine
+            params = [p for p in model.parameters() if p.requires_grad]
+            nll = model.token_nll(**batch)
+            out = [nll.detach(), *torch.autograd.grad(nll.sum(), params)]
+        else:
+            with torch.no_grad():
+                out = [model.token_nll(**batch)]
+    finally:
+        for cls, f in apply.items():
+            cls.forward = staticmethod(f)
+        for h in hooks:
+            h.remove()
+    return out, len(taken)
+
+
+def _close(a, b):
+    # the same kernels on the same operands; norms and gradients add fp32 values with atomics, and two runs of the library's attention
+    # backward round single values differently (2^-8)
+    for i, (x, y) in enumerate(zip(a, b)):
+        assert torch.equal(x, y) if i == 0 else float((x.float() - y.float()).norm()) <= 2e-3 * float(y.float().norm()) + 1e-12
+
+
+@pytest.mark.parametrize("B,T", [(1, 1), (2, 64), (3, 77)])
+@pytest.mark.parametrize("mode", ["capture", "none"])
+def test_gpt2(B, T, mode):
+    from opaque_b200.models import GPT2Config, GPT2LMHeadModel, shift_labels
+    torch.manual_seed(T)
+    model = GPT2LMHeadModel(GPT2Config.tiny(), device="cuda").requires_grad_(mode == "capture")
+    for n, p in model.named_parameters():
+        if n.endswith("bias"):
+            torch.nn.init.normal_(p, std=0.1)
+    ids = torch.randint(0, 500, (B, T), device="cuda")
+    batch = {"input_ids": ids, "labels": shift_labels(ids)}
+    one, n1 = _run(model, batch, mode, False)
+    two, n2 = _run(model, batch, mode, True)
+    assert (n1, n2) == (4, 0)
+    _close(one, two)
+
+
+@pytest.mark.parametrize("B,T,r", [(1, 1, 8), (2, 64, 16), (3, 77, 8)])
+@pytest.mark.parametrize("mode", ["capture", "autograd", "none"])
+def test_llama_lora(B, T, r, mode):
+    from opaque_b200.models import LlamaConfig, LlamaForCausalLM, shift_labels
+    torch.manual_seed(T)
+    model = LlamaForCausalLM(LlamaConfig.tiny(), device="cuda")
+    model.add_lora(r, 2.0 * r)
+    for n, p in model.named_parameters():
+        if n.endswith("lora_B"):
+            torch.nn.init.normal_(p, std=0.05)
+    ids = torch.randint(0, 256, (B, T), device="cuda")
+    batch = {"input_ids": ids, "labels": shift_labels(ids)}
+    one, n1 = _run(model, batch, mode, False)
+    two, n2 = _run(model, batch, mode, True)
+    assert (n1, n2) == (4, 0)
+    _close(one, two)
+
+
+def test_without_the_compiled_sequences(monkeypatch):
+    """Where the extension is missing, blocks run node by node and the factor gradients go through the general batch entry point."""
+    from opaque_b200 import ops
+    from opaque_b200.models import LlamaConfig, LlamaForCausalLM, shift_labels
+    torch.manual_seed(0)
+    model = LlamaForCausalLM(LlamaConfig.tiny(), device="cuda")
+    model.add_lora(8, 16.0)
+    ids = torch.randint(0, 256, (2, 64), device="cuda")
+    batch = {"input_ids": ids, "labels": shift_labels(ids)}
+    one, n1 = _run(model, batch, "capture", False)
+    monkeypatch.setattr(ops, "block_steps", lambda: None)
+    two, n2 = _run(model, batch, "capture", False)
+    assert (n1, n2) == (4, 0)
+    _close(one, two)
+
+
+def test_errors_of_the_compiled_sequences():
+    """Refused arguments and failed launches are Python exceptions."""
+    from opaque_b200 import ops
+    from opaque_b200.ops import lib
+    steps = ops.block_steps()
+    x = torch.randn(4, 128, device="cuda", dtype=torch.bfloat16)
+    out, seg = torch.zeros(2, 64, device="cuda"), torch.tensor([0, 2, 4], dtype=torch.int32, device="cuda")
+    with pytest.raises(TypeError):
+        steps.gpt2_in(x, None, 3)
+    with pytest.raises(ValueError):                      # past the end of the destination
+        steps.store_wgrads(((x, x, 0, 128, 1, 128),), out, seg, 2, 64, 0)
+    w = torch.ones(132, device="cuda", dtype=torch.bfloat16)[:124]
+    with pytest.raises(lib.KernelLibraryError):          # a width that is no multiple of 8: refused by the kernel's entry point
+        steps.gpt2_in(x[:, :124].contiguous(), None, w, w, x, w, 1e-5)
+
+
+def test_blocks_that_keep_one_node_per_operation():
+    """Partly frozen or partly adapted blocks, another class's projection and given positions."""
+    from opaque_b200.models import GPT2Config, GPT2LMHeadModel, Linear, LlamaConfig, LlamaForCausalLM
+    x = torch.randn(1, 8, 128, device="cuda", dtype=torch.bfloat16)
+    gpt = GPT2LMHeadModel(GPT2Config.tiny(), device="cuda").requires_grad_(False)
+    assert gpt.h[0]._two_nodes(x)
+    gpt.h[0].mlp_c_fc.bias.requires_grad_(True)
+    assert not gpt.h[0]._two_nodes(x) and gpt.h[1]._two_nodes(x) and not gpt.h[1]._two_nodes(x.float())
+
+    class Other(Linear):
+        pass
+    model = LlamaForCausalLM(LlamaConfig.tiny(), device="cuda")
+    assert not model.model.layers[0]._two_nodes(x, model.rope_cos, model.rope_sin, None)
+    model.add_lora(8, 16.0)
+    a, b = model.model.layers
+    assert a._two_nodes(x, model.rope_cos, model.rope_sin, None) and not a._two_nodes(x, model.rope_cos, model.rope_sin, torch.arange(8, device="cuda")[None])
+    a.self_attn.o_proj.__class__ = Other
+    b.mlp.gate_proj.add_lora(8, 16.0)
+    assert not a._two_nodes(x, model.rope_cos, model.rope_sin, None) and not b._two_nodes(x, model.rope_cos, model.rope_sin, None)
