@@ -62,13 +62,14 @@ class GPT2In(Function):
 
 class GPT2Out(Function):
     """From the attention's output ``o [B, heads, T, hd]``: its projection, ``s = residual + that``, LayerNorm and the GELU MLP.
-    Returns ``(mlp output, s)``."""
+    Returns ``(mlp output, s)``; ``keep``: a backward pass may follow."""
 
     @staticmethod
-    def forward(ctx, o, residual, wo, bo, ln_w, ln_b, w1, b1, w2, b2, eps, norm):
-        o2, y, s, stats, f, h, m = ops.block_steps().gpt2_out(o, residual, wo, bo, ln_w, ln_b, w1, b1, w2, b2, eps)
+    def forward(ctx, o, residual, wo, bo, ln_w, ln_b, w1, b1, w2, b2, eps, norm, keep):
+        o2, y, s, stats, f, h, m = ops.block_steps().gpt2_out(o, residual, wo, bo, ln_w, ln_b, w1, b1, w2, b2, eps, keep)
         ctx.trainable, ctx.norm, ctx.biases, ctx.dims = w1.requires_grad, norm, (bo, b1, b2), (o.shape[0], o.shape[2], o.shape[1], o.shape[3])
-        ctx.save_for_backward(s, stats, f, ln_w, wo, w1, w2, *((o2, y, h) if ctx.trainable else ()))
+        if keep:
+            ctx.save_for_backward(s, stats, f, ln_w, wo, w1, w2, *((o2, y, h) if ctx.trainable else ()))
         return m.view(residual.shape), s.view(residual.shape)
 
     @staticmethod
@@ -83,7 +84,7 @@ class GPT2Out(Function):
             d1 = _weight_grads(cap, w1, b1, y, g1)
             dln = _layer_norm_param_grads(dy, s, ln_w, stats, ctx.norm, True)
             grads = (*_weight_grads(cap, wo, bo, o2, dx), *dln, *d1, *d2)
-        return (do.view(ctx.dims).transpose(1, 2), dx.view(dm.shape), *grads, None, None)
+        return (do.view(ctx.dims).transpose(1, 2), dx.view(dm.shape), *grads, None, None, None)
 
 
 class LoRAIn(Function):

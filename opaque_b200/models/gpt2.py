@@ -83,7 +83,7 @@ class GPT2Block(nn.Module):
             q, k, v, s = blocks.GPT2In.apply(x, residual, n1.weight, n1.bias, wq["weight"], wq["bias"], n1.eps, self.nh, n1)
             o = nn.functional.scaled_dot_product_attention(q, k, v, is_causal=True)
             return blocks.GPT2Out.apply(o, x if s is None else s, wo["weight"], wo["bias"], n2.weight, n2.bias, w1["weight"], w1["bias"],
-                                        w2["weight"], w2["bias"], n2.eps, n2)
+                                        w2["weight"], w2["bias"], n2.eps, n2, torch.is_grad_enabled())
         y, s = (self.ln_1(x), x) if residual is None else self.ln_1.add(x, residual)
         y, s = self.ln_2.add(self._attention(y), s)
         return self._mlp(y), s

@@ -529,6 +529,62 @@ def gemm_glu_bwd(dy: torch.Tensor, w_down: torch.Tensor, gate: torch.Tensor, up:
     return dg, du
 
 
+def _act_single(M: int, N: int, K: int, kernel: str) -> bool:
+    """Which kernel :func:`gemm_act` and :func:`gemm_act_bwd` run: the single-CTA one (64-column tiles) or the pair kernel."""
+    if kernel == "auto":
+        return N % 64 == 0 and _plan_code(M, N, K, 0, 0) != 0
+    return {"single": True, "pair": False}[kernel]
+
+
+def gemm_act(a: torch.Tensor, b: torch.Tensor, bias: torch.Tensor | None = None, *, act: str = "gelu_tanh", save_preact: bool = True,
+             kernel: str = "auto", status: StatusWord | None = None, wait_budget_s: float = DEFAULT_WAIT_BUDGET_S):
+    """``x = a bᵀ + bias`` and ``h = act(x)`` of the rounded ``x`` in one launch; returns ``(h, x)``, ``x`` ``None`` without
+    ``save_preact``.  ``kernel``: ``"pair"``, ``"single"`` (``N % 64 == 0``) or ``"auto"``; the same bits."""
+    _need_bf16(a, b)
+    if a.ndim != 2 or a.stride(1) != 1 or b.ndim != 2 or b.stride(1) != 1 or b.shape[1] != a.shape[1]:
+        raise ValueError("gemm_act: a [M, K] and b [N, K] row-major")
+    M, K = a.shape
+    N = b.shape[0]
+    if bias is not None:
+        _need_bf16(bias)
+        if bias.numel() != N or not bias.is_contiguous():
+            raise ValueError("bias must hold N contiguous values")
+    h = torch.empty(M, N, dtype=torch.bfloat16, device=a.device)
+    x = torch.empty_like(h) if save_preact else None
+    st = status.ptr() if status else None
+    if _act_single(M, N, K, kernel):
+        rc = lib.load().ob_gemm_tn_act(a.data_ptr(), b.data_ptr(), lib.ptr(bias), h.data_ptr(), lib.ptr(x), M, N, K, a.stride(0), b.stride(0), 0,
+                                       _GLU_ACT[act], 0, st, wait_budget_s, lib.sm_count(), lib.stream())
+    else:
+        rc = lib.load().ob_gemm_pair(a.data_ptr(), b.data_ptr(), None, None, None, None, lib.ptr(bias), h.data_ptr(), lib.ptr(x), None, M, N, K, 0,
+                                     a.stride(0), b.stride(0), 0, 0, N, 0, 0, 2, _GLU_ACT[act], -1, st, wait_budget_s, lib.sm_count(), lib.stream())
+    lib.check(rc, "gemm_act")
+    return h, x
+
+
+def gemm_act_bwd(dy: torch.Tensor, w: torch.Tensor, x: torch.Tensor, *, act: str = "gelu_tanh", kernel: str = "auto",
+                 status: StatusWord | None = None, wait_budget_s: float = DEFAULT_WAIT_BUDGET_S) -> torch.Tensor:
+    """``(dy @ w) * act'(x)`` in one launch, the product rounded to bf16 first: ``dy [M, K]``, ``w [K, N]`` as stored (the second
+    projection of an MLP), ``x [M, N]`` the contiguous pre-activations.  ``N % 64 == 0``; ``kernel`` as in :func:`gemm_act`."""
+    _need_bf16(dy, w, x)
+    if dy.ndim != 2 or dy.stride(1) != 1 or w.ndim != 2 or w.stride(1) != 1 or w.shape[0] != dy.shape[1]:
+        raise ValueError("gemm_act_bwd: dy [M, K] and w [K, N] must be row-major")
+    M, K = dy.shape
+    N = w.shape[1]
+    if x.shape != (M, N) or not x.is_contiguous() or N % 64:
+        raise ValueError("gemm_act_bwd: x must be a contiguous [M, N] with N % 64 == 0")
+    dx = torch.empty(M, N, dtype=torch.bfloat16, device=dy.device)
+    st = status.ptr() if status else None
+    if _act_single(M, N, K, kernel):
+        rc = lib.load().ob_gemm_tn_act(dy.data_ptr(), w.data_ptr(), None, dx.data_ptr(), x.data_ptr(), M, N, K, dy.stride(0), w.stride(0), 1,
+                                       _GLU_ACT[act], 1, st, wait_budget_s, lib.sm_count(), lib.stream())
+    else:
+        rc = lib.load().ob_gemm_pair_glu_bwd(dy.data_ptr(), w.data_ptr(), x.data_ptr(), None, dx.data_ptr(), None, M, N, K, dy.stride(0),
+                                             w.stride(0), N, N, 1, _GLU_ACT[act], st, wait_budget_s, lib.sm_count(), lib.stream())
+    lib.check(rc, "gemm_act_bwd")
+    return dx
+
+
 def pick_glu_bwd(M: int, inter: int, sms: int = 148) -> bool:
     """Whether :func:`gemm_glu_bwd` beats a plain data gradient and the element-wise GLU backward (the same bits): once its 256 x 256
     tiles are more than one wave.  A lone tile's epilogue has no main loop to hide behind (us, separate / fused: 128 x 8192 12.5 / 20.1,
@@ -911,7 +967,7 @@ from .functional import (activation, add_layer_norm, cross_entropy, cross_entrop
                          layer_norm, merge_heads3, plain_torch_ops, rms_norm, rms_norm_ref, rope_qk, rope_qk_ref, rope_tables, rows_group_sum_, swiglu)
 
 __all__ = [
-    "gemm", "gemm_pair", "block_steps", "lora_pack", "pick_gemm_plan", "gemm_glu", "gemm_glu_bwd", "pick_glu_bwd", "direct_norm2", "pick_norm_path", "pick_gemm_kernel", "die_map", "set_die_aware_tiles", "linear_ce_forward", "linear_ce_dlogits_", "gemm_glu_ref", "gemm_ref", "ghost_set_wide", "push_grad_", "wgrad_clip_per_example", "wgrad_clip_batch", "wgrad_clip_per_example_batch", "direct_norm2_batch", "ghost_norm_batch", "plain_torch_ops", "layer_norm", "add_layer_norm", "activation", "rows_group_sum_", "merge_heads3",
+    "gemm", "gemm_pair", "block_steps", "lora_pack", "pick_gemm_plan", "gemm_glu", "gemm_glu_bwd", "pick_glu_bwd", "gemm_act", "gemm_act_bwd", "direct_norm2", "pick_norm_path", "pick_gemm_kernel", "die_map", "set_die_aware_tiles", "linear_ce_forward", "linear_ce_dlogits_", "gemm_glu_ref", "gemm_ref", "ghost_set_wide", "push_grad_", "wgrad_clip_per_example", "wgrad_clip_batch", "wgrad_clip_per_example_batch", "direct_norm2_batch", "ghost_norm_batch", "plain_torch_ops", "layer_norm", "add_layer_norm", "activation", "rows_group_sum_", "merge_heads3",
     "DeviceWaitTimeout", "KernelLibraryError", "StatusWord", "clip_tree", "clip_weighted_sum", "cross_entropy",
     "cross_entropy_ref", "embedding_wgrad", "fused_add_rms_norm", "geglu", "ghost_norm", "ghost_norm_ref", "glu_ref",
     "philox_normal_add_", "pick_block_n", "pick_splits", "rms_norm", "rms_norm_ref", "rope_qk", "rope_qk_ref",

@@ -57,17 +57,23 @@ int ob_gemm_tn(const void* a, const void* b, const void* a2, const void* b2, con
                long long ldo, int b_kn, int b2_kn, float alpha, const int* group_offs, int num_groups, int block_n,
                int* status, double wait_budget_s, int num_sms, void* stream);
 
+// The same kernel (64-column tiles, N % 64 == 0, contiguous out and pre) with a plain activation in its epilogue (0 silu, 1 gelu erf,
+// 2 gelu tanh): out = act(D) and, where given, pre = D; backward: out = D * act'(pre).
+int ob_gemm_tn_act(const void* a, const void* b, const void* bias, void* out, void* pre, long long rows_a, int N, int K, long long lda,
+                   long long ldb, int b_kn, int act, int backward, int* status, double wait_budget_s, int num_sms, void* stream);
+
 // Dense GEMM on CTA pairs (tcgen05 cta_group::2):  D = A op1(B) + A2 op2(B2) + bias.
 // tile (without glu): 1 = 256 x 256 tiles with two alternating accumulators, 0 = 512 x 256 tiles, -1 = by size; the same bits.
 // b_kn / b2_kn = 1: that B operand is stored [K, N] row-major, 0: [N, K].  glu != 0: `b` holds the gate rows and `b_up`
 // the up rows of a gated MLP ([N/2, K] each; N counts both), out [M, N/2] = act(gate) * up (glu_act: 0 silu, 1 gelu erf,
-// 2 gelu tanh) and the optional out_gate / out_up receive the pre-activations.
+// 2 gelu tanh) and the optional out_gate / out_up receive the pre-activations; glu = 2: out = act(D), out_gate (optional) = D.
 int ob_gemm_pair(const void* a, const void* b, const void* b_up, const void* a2, const void* b2, const void* b2_up,
                  const void* bias, void* out, void* out_gate, void* out_up, long long rows_a, int N, int K1, int K2,
                  long long lda, long long ldb, long long lda2, long long ldb2, long long ldo, int b_kn, int b2_kn, int glu,
                  int glu_act, int tile, int* status, double wait_budget_s, int num_sms, void* stream);
 // Data gradient of a gated MLP's down projection with the activation's backward in the epilogue: dH = dY op(W) stays in
 // tensor memory; dGate = dH * up * act'(gate) and dUp = dH * act(gate) are stored (bf16 [M, N], pitch ld_out).  N % 64 == 0.
+// up = dup = NULL: a plain activation, dGate = dH * act'(gate).
 int ob_gemm_pair_glu_bwd(const void* dy, const void* w, const void* gate, const void* up, void* dgate, void* dup,
                          long long rows_a, int N, int K, long long lddy, long long ldw, long long ld_gu, long long ld_out,
                          int b_kn, int glu_act, int* status, double wait_budget_s, int num_sms, void* stream);

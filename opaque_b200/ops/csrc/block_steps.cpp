@@ -27,7 +27,7 @@ namespace {
 using at::Tensor;
 
 #define OB_ENTRIES(X)                                                                                                          \
-  X(ob_gemm_tn) X(ob_gemm_pair) X(ob_gemm_pair_glu_bwd) X(ob_glu_bwd) X(ob_rmsnorm_fwd) X(ob_rmsnorm_bwd) X(ob_layernorm_fwd)  \
+  X(ob_gemm_tn) X(ob_gemm_tn_act) X(ob_gemm_pair) X(ob_gemm_pair_glu_bwd) X(ob_glu_bwd) X(ob_rmsnorm_fwd) X(ob_rmsnorm_bwd) X(ob_layernorm_fwd)  \
   X(ob_layernorm_bwd_dx) X(ob_add_layernorm_fwd) X(ob_add_layernorm_bwd_dx) X(ob_activation) X(ob_merge_heads3) X(ob_lora_pack) \
   X(ob_rope_qk_oop) X(ob_wgrad_clip_batch)
 #define X(name) decltype(&name) p_##name = nullptr;
@@ -152,6 +152,41 @@ Tensor gelu(const Tensor& x, const Tensor& dy) {
   LAUNCH(ob_activation, ptr(x), ptr(dy), ptr(out), x.numel(), GELU_TANH, g_sms);
   return out;
 }
+// GPT-2's GELU in the epilogue of the product around it: the pair kernel's, or the single-CTA kernel's with 64-column tiles, also where
+// the plain product would take wide ones (us, both launches / this, N = 3072, K = 768: 128 rows 8.4 / 8.0, 512 12.5 / 10.6, 1024
+// 13.9 / 13.7, 1285 14.8 / 14.2, 3663 27.7 / 26.4, 16384 117 / 98; backward 8.0 / 7.8, 12.3 / 11.4, 13.9 / 14.4, 14.9 / 13.9,
+// 30.3 / 25.9, 127 / 106).
+// -> gelu(x b^T + bias) and, with `pre`, its argument there (allocated)
+Tensor product_gelu(const Tensor& x, const Tensor& b, const Tensor& bias, Tensor* pre) {
+  const int64_t M = x.size(0), N = b.size(0), K = x.size(1);
+  if (N % 64 != 0) {
+    const Tensor f = product(x, b, N, false, with_bias(bias));
+    if (pre != nullptr) *pre = f;
+    return gelu(f, Tensor());
+  }
+  Tensor h = empty({M, N}, x);
+  if (pre != nullptr) *pre = empty({M, N}, x);
+  void* const f = pre != nullptr ? ptr(*pre) : nullptr;
+  if (plan(M, N, K, 0, false) == 0)
+    LAUNCH(ob_gemm_pair, ptr(x), ptr(b), nullptr, nullptr, nullptr, nullptr, ptr(bias), ptr(h), f, nullptr, M, (int)N, (int)K, 0, x.stride(0),
+           b.stride(0), 0, 0, N, 0, 0, 2, GELU_TANH, -1, nullptr, g_budget, g_sms);
+  else
+    LAUNCH(ob_gemm_tn_act, ptr(x), ptr(b), ptr(bias), ptr(h), f, M, (int)N, (int)K, x.stride(0), b.stride(0), 0, GELU_TANH, 0, nullptr, g_budget, g_sms);
+  return h;
+}
+// -> (g w) * gelu'(f)
+Tensor product_gelu_bwd(const Tensor& g, const Tensor& w, const Tensor& f) {
+  const int64_t M = g.size(0), N = w.size(1), K = g.size(1);
+  if (N % 64 != 0) return gelu(f, product(g, w, N, true));
+  Tensor df = empty({M, N}, g);
+  if (plan(M, N, K, 0, false) == 0)
+    LAUNCH(ob_gemm_pair_glu_bwd, ptr(g), ptr(w), ptr(f), nullptr, ptr(df), nullptr, M, (int)N, (int)K, g.stride(0), w.stride(0), N, N, 1, GELU_TANH,
+           nullptr, g_budget, g_sms);
+  else
+    LAUNCH(ob_gemm_tn_act, ptr(g), ptr(w), nullptr, ptr(df), ptr(f), M, (int)N, (int)K, g.stride(0), w.stride(0), 1, GELU_TANH, 1, nullptr, g_budget,
+           g_sms);
+  return df;
+}
 // q, k [B, T, heads, hd] through their strides -> rotated, contiguous
 bool rope_reads(const Tensor& t) {
   return t.stride(3) == 1 && (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0 && ((t.stride(0) | t.stride(1) | t.stride(2)) & 7) == 0;
@@ -270,20 +305,21 @@ PyObject* gpt2_in_bwd(Args& a) {
   }
   return pack({g, dy, dx});
 }
-// (o [B, heads, T, hd], residual, wo, bo, ln_w, ln_b, w1, b1, w2, b2, eps) -> o2, y, s, stats, f, h, m
+// (o [B, heads, T, hd], residual, wo, bo, ln_w, ln_b, w1, b1, w2, b2, eps, keep) -> o2, y, s, stats, f | None, h, m
 PyObject* gpt2_out(Args& a) {
   const Tensor o = a.tensor(), r = rows(a.tensor()), wo = a.tensor(), bo = a.tensor(), lw = a.tensor(), lb = a.tensor(), w1 = a.tensor(),
                b1 = a.tensor(), w2 = a.tensor(), b2 = a.tensor();
   const Tensor o2 = vec16(o.transpose(1, 2).reshape({o.size(0) * o.size(2), -1}));
   const Normed n = layer_norm(product(o2, wo, wo.size(0), false, with_bias(bo)), r, lw, lb, a.number());
-  const Tensor f = product(n.y, w1, w1.size(0), false, with_bias(b1)), h = gelu(f, Tensor());
+  Tensor f;
+  const Tensor h = product_gelu(n.y, w1, b1, a.integer() ? &f : nullptr);
   return pack({o2, n.y, n.s, n.stats, f, h, product(h, w2, w2.size(0), false, with_bias(b2))});
 }
 // (dm, f, w2, w1, s, ln_w, stats, ds, wo) -> g2, g1, dy, dx, do [rows, heads * hd]
 PyObject* gpt2_out_bwd(Args& a) {
   const Tensor g2 = rows(a.tensor()), f = a.tensor(), w2 = a.tensor(), w1 = a.tensor(), s = a.tensor(), lw = a.tensor(), stats = a.tensor(),
                ds = rows(a.tensor()), wo = a.tensor();
-  const Tensor g1 = gelu(f, product(g2, w2, w2.size(1), true)), dy = product(g1, w1, w1.size(1), true);
+  const Tensor g1 = product_gelu_bwd(g2, w2, f), dy = product(g1, w1, w1.size(1), true);
   const Tensor dx = layer_norm_bwd(dy, s, lw, stats, ds);
   return pack({g2, g1, dy, dx, product(dx, wo, wo.size(1), true)});
 }

@@ -58,17 +58,19 @@ constexpr int GP_GROUP_M = 8;        // pair tiles (512 rows each) per raster ba
 constexpr int GP_SLAB_BYTES = 4096;   // per epilogue warp: a 32-row x 64-column (or 2 x 32-column) bf16 staging tile
 constexpr int GP_SMEM = GP_STAGES * GP_STAGE_BYTES + 8 * GP_SLAB_BYTES + 256 + 1024;
 
-enum : int { GP_EPI_STORE = 0, GP_EPI_GLU = 1, GP_EPI_CE = 2, GP_EPI_GLUBWD = 3 };
+enum : int { GP_EPI_STORE = 0, GP_EPI_GLU = 1, GP_EPI_CE = 2, GP_EPI_GLUBWD = 3, GP_EPI_ACT = 4, GP_EPI_ACTBWD = 5 };
+// pre-activation tiles that a backward epilogue reads: gate and up, or a plain activation's one
+__host__ __device__ constexpr int gp_pre_tiles(int epi) { return epi == GP_EPI_GLUBWD ? 2 : epi == GP_EPI_ACTBWD ? 1 : 0; }
 
 struct PairParams {
   int M, N, K1, K2;
   int kn1, kn2;                      // 1: the segment's B operand is stored [K, N] (N-major), 0: [N, K]
   __nv_bfloat16* out;                // STORE: [M, N];  GLU: [M, N / 2] activations
   long long ldo;
-  __nv_bfloat16* out_gate;           // GLU only, optional: pre-activations, pitch ldo
+  __nv_bfloat16* out_gate;           // GLU and ACT, optional: pre-activations, pitch ldo
   __nv_bfloat16* out_up;
-  const __nv_bfloat16* bias;         // STORE only
-  int act;                           // GLU: 0 silu, 1 gelu (erf), 2 gelu (tanh)
+  const __nv_bfloat16* bias;         // STORE and ACT
+  int act;                           // 0 silu, 1 gelu (erf), 2 gelu (tanh)
   int group_m;                       // pair tiles (512 rows each) per raster band
   // CE epilogue (output head + cross-entropy statistics; `out` optional: the bf16, soft-capped logits)
   const long long* labels;           // [M]
@@ -279,6 +281,31 @@ __device__ __forceinline__ void gp_glu_bwd_slabs(const uint32_t* pd, uint8_t* sl
   }
 }
 
+// The same for a plain activation: the slab holds x and receives dH * act'(x) (activation_kernel's operations).
+template <int ACT>
+__device__ __forceinline__ void gp_act_bwd_slab(const uint32_t* pd, uint8_t* slab, int lane) {
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    uint4* xp = reinterpret_cast<uint4*>(slab + lane * 128 + ((c ^ (lane & 7)) << 4));
+    const uint4 x4 = *xp;
+    uint32_t xw[4] = {x4.x, x4.y, x4.z, x4.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t d2 = pd[4 * c + j];
+      xw[j] = pack_bf16x2(__uint_as_float(d2 << 16) * act_bwd(__uint_as_float(xw[j] << 16), ACT),
+                          __uint_as_float(d2 & 0xffff0000u) * act_bwd(__uint_as_float(xw[j] & 0xffff0000u), ACT));
+    }
+    *xp = make_uint4(xw[0], xw[1], xw[2], xw[3]);
+  }
+}
+// pk[j] <- bf16x2(act(x)) of packed pairs
+template <int ACT>
+__device__ __forceinline__ void gp_act_inplace(uint32_t* pk) {
+#pragma unroll
+  for (int j = 0; j < 32; ++j)
+    pk[j] = pack_bf16x2(act_fwd(__uint_as_float(pk[j] << 16), ACT), act_fwd(__uint_as_float(pk[j] & 0xffff0000u), ACT));
+}
+
 // pkg[j] <- bf16x2(act(g) * u) from packed bf16 pairs of g and u (32 registers = 64 values per lane)
 template <int ACT>
 __device__ __forceinline__ void gp_glu_inplace(uint32_t* pkg, const uint32_t* pku) {
@@ -338,7 +365,7 @@ __device__ __forceinline__ void ce_fold64(const uint32_t* pk, int nc, int N, int
 template <int EPI>
 __device__ __forceinline__ bool pair_vec_ok(const PairParams& p) {
   return ((p.ldo & 7) == 0) && ((reinterpret_cast<uintptr_t>(p.out) & 15) == 0) &&
-         (EPI != GP_EPI_GLU || p.out_gate == nullptr ||
+         ((EPI != GP_EPI_GLU && EPI != GP_EPI_ACT) || p.out_gate == nullptr ||
           (((reinterpret_cast<uintptr_t>(p.out_gate) | reinterpret_cast<uintptr_t>(p.out_up)) & 15) == 0));
 }
 
@@ -349,7 +376,7 @@ template <int EPI, class Release>
 __device__ __forceinline__ void pair_epilogue(const PairParams& p, const CUtensorMap& map_out, const CUtensorMap& map_out_gate,
                                               const CUtensorMap& map_out_up, uint8_t* slab, uint32_t t_row, int row, int nt,
                                               int tiles_n, int g, int lane, bool vec_ok, Release release) {
-  if constexpr (EPI == GP_EPI_STORE) {
+  if constexpr (EPI == GP_EPI_STORE || EPI == GP_EPI_ACT) {
     // Both 64-column rounds of this warp's share go to registers (packed bf16) first, so the accumulator half is
     // back with the tensor pipe before a single store is issued; the stores then overlap the next MMAs.
     const int n0 = nt * GP_BN + g * (GP_BN / 2);
@@ -372,9 +399,16 @@ __device__ __forceinline__ void pair_epilogue(const PairParams& p, const CUtenso
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
       const int nc = n0 + c * 64;
-      if (nc < p.N)
-        store_tile64_packed(slab, pk[c], &map_out, p.tma_store != 0, nc, row0w, p.out, p.ldo, p.M - row0w, p.N - nc,
-                            vec_ok, lane);
+      if (nc >= p.N) continue;
+      if constexpr (EPI == GP_EPI_ACT) {       // act() of the rounded pre-activations, which leave first where a backward pass follows
+        if (p.out_gate != nullptr)
+          store_tile64_packed(slab, pk[c], &map_out_gate, p.tma_store != 0, nc, row0w, p.out_gate, p.ldo, p.M - row0w, p.N - nc, vec_ok, lane);
+        if (p.act == 0) gp_act_inplace<0>(pk[c]);
+        else if (p.act == 1) gp_act_inplace<1>(pk[c]);
+        else gp_act_inplace<2>(pk[c]);
+      }
+      store_tile64_packed(slab, pk[c], &map_out, p.tma_store != 0, nc, row0w, p.out, p.ldo, p.M - row0w, p.N - nc,
+                          vec_ok, lane);
     }
   } else if constexpr (EPI == GP_EPI_CE) {
     // Output head: the logits tile never leaves the SM unless `out` asks for it.  Each thread owns one row and folds
@@ -764,7 +798,7 @@ constexpr int GD_GROUP_M = 16;                          // pair tiles (256 rows 
 template <int EPI>
 struct GdRing {
   static constexpr int STAGES = EPI == GP_EPI_GLUBWD ? 5 : 6;
-  static constexpr int WARP_SLAB = EPI == GP_EPI_GLUBWD ? 2 * GP_SLAB_BYTES : GP_SLAB_BYTES;
+  static constexpr int WARP_SLAB = gp_pre_tiles(EPI) == 2 ? 2 * GP_SLAB_BYTES : GP_SLAB_BYTES;
   static constexpr int SMEM = STAGES * GD_STAGE_BYTES + 8 * WARP_SLAB + 256 + 1024;
   static_assert((2 * STAGES + 4 + 8) * 8 + 20 <= 256, "barrier block");
   static_assert(SMEM <= 232448, "shared memory of an SM");
@@ -797,7 +831,7 @@ gemm_pair_db_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   uint64_t* empty = bars + GD_STAGES;
   uint64_t* tmem_full = bars + 2 * GD_STAGES;          // [2]: one per accumulator buffer
   uint64_t* tmem_empty = bars + 2 * GD_STAGES + 2;     // [2], used in the leader CTA only
-  uint64_t* preact = bars + 2 * GD_STAGES + 4;         // [8]: GLU backward, one per epilogue warp
+  uint64_t* preact = bars + 2 * GD_STAGES + 4;         // [8]: activation backward, one per epilogue warp
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * GD_STAGES + 12);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* sched = reinterpret_cast<int*>(tmem_slot + 2);  // [3]: first, end, stride (valid in the leader CTA)
@@ -823,7 +857,7 @@ gemm_pair_db_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       mbar_init(&tmem_full[a], 1);
       mbar_init(&tmem_empty[a], 16);                   // eight epilogue warps in each CTA
     }
-    if constexpr (EPI == GP_EPI_GLUBWD)
+    if constexpr (gp_pre_tiles(EPI) > 0)
       for (int a = 0; a < 8; ++a) mbar_init(&preact[a], 1);
     *abort_flag = 0;
     mbar_fence_init();
@@ -949,16 +983,16 @@ gemm_pair_db_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       const GpItem it = gd_decode(w, tiles_m, tiles_n, rank);
       const int as = acc_iter & 1;
       const int row0w = it.row0 + q * 32, n0 = it.nt * GP_BN + g * (GP_BN / 2);
-      // GLU backward: the pre-activations [32 rows x 64 columns] of this warp's next round, into its two slabs
+      // activation backward: the pre-activations [32 rows x 64 columns] of this warp's next round, into its slabs
       [[maybe_unused]] auto fetch = [&](int nc) {
         if (lane == 0) {
           tma_store_wait_read();             // the round before has left the slabs
-          mbar_expect_tx(&preact[warp - 2], 2 * GP_SLAB_BYTES);
+          mbar_expect_tx(&preact[warp - 2], gp_pre_tiles(EPI) * GP_SLAB_BYTES);
           tma_load_2d(slab, &map_a2, &preact[warp - 2], nc, row0w);
-          tma_load_2d(slab + GP_SLAB_BYTES, &map_b2, &preact[warp - 2], nc, row0w);
+          if constexpr (gp_pre_tiles(EPI) == 2) tma_load_2d(slab + GP_SLAB_BYTES, &map_b2, &preact[warp - 2], nc, row0w);
         }
       };
-      if constexpr (EPI == GP_EPI_GLUBWD) {
+      if constexpr (gp_pre_tiles(EPI) > 0) {
         if (n0 < p.N) fetch(n0);             // arrives during the tile's main loop
       }
       if (!mbar_wait_idle(&tmem_full[as], (acc_iter >> 1) & 1, abort_flag, p.status, OB_ERR_WAIT_TMEM_FULL, budget)) {
@@ -975,9 +1009,9 @@ gemm_pair_db_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
           else mbar_arrive_cluster(map_to_cta(smem_u32(&tmem_empty[as]), 0));
         }
       };
-      if constexpr (EPI == GP_EPI_GLUBWD) {
-        // Data gradient of a gated MLP's down projection: the accumulator is dH.  It is read, rounded to bf16 and packed, handed
-        // back, and turned into dGate and dUp in the slabs that hold the pre-activations.  N % 64 == 0 (host-checked).
+      if constexpr (gp_pre_tiles(EPI) > 0) {
+        // Data gradient of an MLP's second projection: the accumulator is dH.  It is read, rounded to bf16 and packed, handed back, and
+        // turned into dGate and dUp (or the one gradient) in the slabs that hold the pre-activations.  N % 64 == 0 (host-checked).
         uint32_t pd[2][32];
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
@@ -999,14 +1033,20 @@ gemm_pair_db_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             ok = mbar_wait_warp(&preact[warp - 2], fetched, abort_flag, p.status, OB_ERR_WAIT_FULL, budget);
             if (!ok) break;
             fetched ^= 1;
-            if (p.act == 0) gp_glu_bwd_slabs<0>(pd[c], slab, lane);
-            else if (p.act == 1) gp_glu_bwd_slabs<1>(pd[c], slab, lane);
-            else gp_glu_bwd_slabs<2>(pd[c], slab, lane);
+            if constexpr (EPI == GP_EPI_ACTBWD) {
+              if (p.act == 0) gp_act_bwd_slab<0>(pd[c], slab, lane);
+              else if (p.act == 1) gp_act_bwd_slab<1>(pd[c], slab, lane);
+              else gp_act_bwd_slab<2>(pd[c], slab, lane);
+            } else {
+              if (p.act == 0) gp_glu_bwd_slabs<0>(pd[c], slab, lane);
+              else if (p.act == 1) gp_glu_bwd_slabs<1>(pd[c], slab, lane);
+              else gp_glu_bwd_slabs<2>(pd[c], slab, lane);
+            }
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) {
               tma_store_2d(&map_out, slab, nc, row0w);
-              tma_store_2d(&map_out_up, slab + GP_SLAB_BYTES, nc, row0w);
+              if constexpr (gp_pre_tiles(EPI) == 2) tma_store_2d(&map_out_up, slab + GP_SLAB_BYTES, nc, row0w);
               tma_store_commit();
             }
           }
@@ -1308,6 +1348,7 @@ static int pair_launch(bool small, const PairMaps& m, PairParams& p, int num_sms
 // glu != 0: `b` holds the gate rows and `b_up` the up rows ([N/2, K] each, or [K, N/2] with b_kn); N counts gate and up
 // columns together; out [M, N/2] = act(gate) * up, and out_gate / out_up (optional, both or none) receive the
 // pre-activations.  glu_act: 0 silu, 1 gelu erf, 2 gelu tanh.  With a second segment in GLU mode b2 / b2_up likewise.
+// glu = 2: a plain activation, out = act(D) and, in out_gate (optional), D itself.
 // tile (without glu): 1 = 256 x 256, 0 = 512 x 256, -1 = pair_small_tile's choice (the same bits either way).
 extern "C" int ob_gemm_pair(const void* a, const void* b, const void* b_up, const void* a2, const void* b2,
                             const void* b2_up, const void* bias, void* out, void* out_gate, void* out_up,
@@ -1318,10 +1359,15 @@ extern "C" int ob_gemm_pair(const void* a, const void* b, const void* b_up, cons
   if (rows_a <= 0 || N <= 0 || K1 <= 0) return 0;
   if (rows_a > 0x7fffffffLL - 2 * GP_BM) return -50;
   if (K2 > 0 && (a2 == nullptr || b2 == nullptr)) return -51;
+  const bool plain_act = glu == 2;
+  if (plain_act) {
+    if (b_up != nullptr || out_up != nullptr) return -52;
+    glu = 0;
+  }
   if (glu && (b_up == nullptr || (N & 1) || (K2 > 0 && b2_up == nullptr) || bias != nullptr)) return -52;
   if (glu && ((out_gate == nullptr) != (out_up == nullptr))) return -53;
   const int nb = glu ? N / 2 : N;               // columns of N covered by ONE B operand
-  const bool small = glu || (tile < 0 ? pair_small_tile(rows_a, N, static_cast<long long>(K1) + K2, num_sms / 2) : tile != 0);
+  const bool small = glu || plain_act || (tile < 0 ? pair_small_tile(rows_a, N, static_cast<long long>(K1) + K2, num_sms / 2) : tile != 0);
   const int box_rows = small ? GD_BM : GP_BM;
   PairMaps m;
   int rc = make_bf16_map_2d(&m.a, a, rows_a, K1, lda, GP_BK, box_rows);
@@ -1368,9 +1414,11 @@ extern "C" int ob_gemm_pair(const void* a, const void* b, const void* b_up, cons
   p.wait_budget_ns = static_cast<unsigned long long>(wait_budget_s * 1e9);
   m.out = m.out_gate = m.out_up = m.a;
   p.tma_store = pair_out_map(&m.out, out, rows_a, nb, ldo) ? 1 : 0;          // nb: the width of the output (N / 2 for GLU)
+  if (plain_act && out_gate != nullptr && p.tma_store) p.tma_store = pair_out_map(&m.out_gate, out_gate, rows_a, nb, ldo) ? 1 : 0;
   if (glu && out_gate != nullptr && p.tma_store)
     p.tma_store = (pair_out_map(&m.out_gate, out_gate, rows_a, nb, ldo) && pair_out_map(&m.out_up, out_up, rows_a, nb, ldo)) ? 1 : 0;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (plain_act) return pair_launch<GP_EPI_ACT>(true, m, p, num_sms, st);
   return glu ? pair_launch<GP_EPI_GLU>(true, m, p, num_sms, st) : pair_launch<GP_EPI_STORE>(small, m, p, num_sms, st);
 }
 
@@ -1378,6 +1426,7 @@ extern "C" int ob_gemm_pair(const void* a, const void* b, const void* b_up, cons
 //   dH = dY[M, K] * op(W)  (W stored [K, N] with b_kn = 1: the down-projection weight as stored),  N = intermediate size,
 //   dGate = dH * up * act'(gate),  dUp = dH * act(gate)   (bf16 [M, N], pitch ld_out);  dH never reaches memory.
 // gate / up: the stored pre-activations [M, N] (pitch ld_gu).  N % 64 == 0; all rows 16-byte aligned.
+// up = dup = nullptr: a plain activation, dgate = dH * act'(gate).
 extern "C" int ob_gemm_pair_glu_bwd(const void* dy, const void* w, const void* gate, const void* up, void* dgate, void* dup,
                                     long long rows_a, int N, int K, long long lddy, long long ldw, long long ld_gu,
                                     long long ld_out, int b_kn, int glu_act, int* status, double wait_budget_s,
@@ -1385,7 +1434,7 @@ extern "C" int ob_gemm_pair_glu_bwd(const void* dy, const void* w, const void* g
   using namespace ob;
   if (rows_a <= 0 || N <= 0 || K <= 0) return 0;
   if (rows_a > 0x7fffffffLL - 2 * GP_BM) return -50;
-  if (gate == nullptr || up == nullptr || dgate == nullptr || dup == nullptr) return -57;
+  if (gate == nullptr || dgate == nullptr || (up == nullptr) != (dup == nullptr)) return -57;
   auto al = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
   if ((N & 63) != 0 || (ld_gu & 7) != 0 || (ld_out & 7) != 0 || !al(gate) || !al(up) || !al(dgate) || !al(dup)) return -58;
   PairMaps m;
@@ -1393,12 +1442,12 @@ extern "C" int ob_gemm_pair_glu_bwd(const void* dy, const void* w, const void* g
   if (rc) return rc;
   rc = b_kn ? make_bf16_map_2d(&m.b, w, K, N, ldw, 64, GP_BK) : make_bf16_map_2d(&m.b, w, N, K, ldw, GP_BK, GP_BNH);
   if (rc) return rc;
-  m.b_up = m.b2_up = m.b;
-  m.out_gate = m.a;
+  m.b_up = m.b2 = m.b2_up = m.b;
+  m.out_gate = m.out_up = m.a;
   // no second segment: its maps hold the pre-activations, in boxes of one epilogue round
-  if ((rc = make_bf16_map_2d(&m.a2, gate, rows_a, N, ld_gu, 64, 32)) != 0 || (rc = make_bf16_map_2d(&m.b2, up, rows_a, N, ld_gu, 64, 32)) != 0)
-    return rc;
-  if (!pair_out_map(&m.out, dgate, rows_a, N, ld_out) || !pair_out_map(&m.out_up, dup, rows_a, N, ld_out)) return -58;
+  if ((rc = make_bf16_map_2d(&m.a2, gate, rows_a, N, ld_gu, 64, 32)) != 0) return rc;
+  if (up != nullptr && (rc = make_bf16_map_2d(&m.b2, up, rows_a, N, ld_gu, 64, 32)) != 0) return rc;
+  if (!pair_out_map(&m.out, dgate, rows_a, N, ld_out) || (dup != nullptr && !pair_out_map(&m.out_up, dup, rows_a, N, ld_out))) return -58;
   PairParams p = {};
   p.group_m = pair_group_m();
   p.M = static_cast<int>(rows_a);
@@ -1411,7 +1460,8 @@ extern "C" int ob_gemm_pair_glu_bwd(const void* dy, const void* w, const void* g
   p.status = status;
   p.wait_budget_ns = static_cast<unsigned long long>(wait_budget_s * 1e9);
   p.tma_store = 1;
-  return pair_launch<GP_EPI_GLUBWD>(true, m, p, num_sms, static_cast<cudaStream_t>(stream));
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  return up != nullptr ? pair_launch<GP_EPI_GLUBWD>(true, m, p, num_sms, st) : pair_launch<GP_EPI_ACTBWD>(true, m, p, num_sms, st);
 }
 
 // Bit patterns of the descriptors the tensor-core kernels build, for host-side checks.

@@ -60,6 +60,11 @@ struct GemmParams {
   int tma_store;           // the output leaves through bulk tensor stores (map_out is valid)
   int b2_kn;               // B2 is [K2, N] (N-major) instead of [N, K2]
   float alpha;             // scales the products
+  // Plain activation in the epilogue of 64-column tiles (act >= 0): forward, out = act(D) and D itself goes to
+  // `pre` where that is given; backward, out = D * act'(pre).  A launch of its own takes as long as such a product's main loop.
+  int act;                 // -1: none; 0 silu, 1 gelu (erf), 2 gelu (tanh)
+  int act_bwd;
+  __nv_bfloat16* pre;      // pitch ldo
   int* status;
   unsigned long long wait_budget_ns;
 };
@@ -93,11 +98,27 @@ __device__ __forceinline__ GtItem gt_decode(const GemmParams& p, int w, int tile
   return it;
 }
 
-template <bool B_KN, int BN>
+// dx[j] <- bf16x2(d * act'(x)), or bf16x2(act(x)) with d == nullptr, of packed pairs
+template <int ACT>
+__device__ __forceinline__ void gt_act(uint32_t* x, const uint32_t* d) {
+#pragma unroll
+  for (int j = 0; j < 32; ++j) {
+    const float a = __uint_as_float(x[j] << 16), b = __uint_as_float(x[j] & 0xffff0000u);
+    x[j] = d == nullptr ? pack_bf16x2(act_fwd(a, ACT), act_fwd(b, ACT))
+                        : pack_bf16x2(__uint_as_float(d[j] << 16) * act_bwd(a, ACT), __uint_as_float(d[j] & 0xffff0000u) * act_bwd(b, ACT));
+  }
+}
+__device__ __forceinline__ void gt_act_any(int act, uint32_t* x, const uint32_t* d) {
+  if (act == 0) gt_act<0>(x, d);
+  else if (act == 1) gt_act<1>(x, d);
+  else gt_act<2>(x, d);
+}
+
+template <bool B_KN, int BN, bool ACT>
 __global__ void __launch_bounds__(GT_THREADS, 1)
 gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                const __grid_constant__ CUtensorMap map_a2, const __grid_constant__ CUtensorMap map_b2,
-               const __grid_constant__ CUtensorMap map_out, const GemmParams p) {
+               const __grid_constant__ CUtensorMap map_out, const __grid_constant__ CUtensorMap map_pre, const GemmParams p) {
   constexpr int STAGES = GtTile<BN>::STAGES, STAGE_BYTES = GtTile<BN>::STAGE_BYTES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -260,6 +281,22 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     for (int w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
       const GtItem it = gt_decode<BN>(p, w, tiles_m, tiles_n, tile_start, cursor);
       const int as = acc_iter & 1;
+      [[maybe_unused]] uint32_t pre[32];
+      if constexpr (ACT) {
+        // activation backward: this lane's row of the pre-activations, on its way while the main loop runs (N % 64 == 0)
+        const int row = it.row0 + q * 32 + lane;
+        if (p.act_bwd && g == 0 && row < it.row_end) {
+          const uint4* src = reinterpret_cast<const uint4*>(p.pre + static_cast<long long>(row) * p.ldo + it.n0);
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            const uint4 t = __ldg(src + c);
+            pre[4 * c] = t.x; pre[4 * c + 1] = t.y; pre[4 * c + 2] = t.z; pre[4 * c + 3] = t.w;
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) pre[j] = 0u;
+        }
+      }
       if (!mbar_wait(&tmem_full[as], (acc_iter >> 1) & 1, abort_flag, p.status, OB_ERR_WAIT_TMEM_FULL, budget)) {
         ok = false;
         break;
@@ -297,6 +334,16 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 #pragma unroll
       for (int c = 0; c < ROUNDS; ++c) {
         const int nc = it.n0 + g * (BN / 2) + c * 64;
+        if constexpr (ACT) {
+          if (mine && p.act_bwd) {
+            gt_act_any(p.act, pre, pk[c]);
+#pragma unroll
+            for (int j = 0; j < 32; ++j) pk[c][j] = pre[j];
+          } else if (mine) {
+            if (p.pre != nullptr) store_tile64_packed(slab, pk[c], &map_pre, true, nc, row0, p.pre, p.ldo, it.row_end - row0, p.N - nc, vec_ok, lane);
+            gt_act_any(p.act, pk[c], nullptr);
+          }
+        }
         if (mine && nc < p.N)
           store_tile64_packed(slab, pk[c], &map_out, use_tma, nc, row0, p.out, p.ldo, it.row_end - row0, p.N - nc, vec_ok,
                               lane);
@@ -316,11 +363,11 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 
 }  // namespace ob
 
-extern "C" int ob_gemm_tn(const void* a, const void* b, const void* a2, const void* b2, const void* bias, void* out,
-                          long long rows_a, int N, int K1, int K2, long long lda, long long ldb, long long lda2,
-                          long long ldb2, long long ldo, int b_kn, int b2_kn, float alpha, const int* group_offs, int num_groups,
-                          int block_n, int* status, double wait_budget_s, int num_sms, void* stream) {
-  using namespace ob;
+namespace ob {
+static int gemm_tn(const void* a, const void* b, const void* a2, const void* b2, const void* bias, void* out, long long rows_a, int N, int K1,
+                   int K2, long long lda, long long ldb, long long lda2, long long ldb2, long long ldo, int b_kn, int b2_kn, float alpha,
+                   const int* group_offs, int num_groups, int block_n, int act, int act_bwd, void* pre, int* status, double wait_budget_s,
+                   int num_sms, void* stream) {
   if (rows_a <= 0 || N <= 0 || K1 <= 0) return 0;
   if (rows_a > 0x7fffffffLL - GT_BM) return -40;
   if (group_offs != nullptr && (num_groups < 1 || num_groups > GT_MAX_GROUPS)) return -41;
@@ -344,8 +391,10 @@ extern "C" int ob_gemm_tn(const void* a, const void* b, const void* a2, const vo
     ma2 = ma;
     mb2 = mb;
   }
-  using Kernel = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap, const GemmParams);
-  static const Kernel kernels[4] = {gemm_tn_kernel<false, 256>, gemm_tn_kernel<true, 256>, gemm_tn_kernel<false, 64>, gemm_tn_kernel<true, 64>};
+  using Kernel = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap,
+                          const GemmParams);
+  static const Kernel kernels[6] = {gemm_tn_kernel<false, 256, false>, gemm_tn_kernel<true, 256, false>, gemm_tn_kernel<false, 64, false>,
+                                    gemm_tn_kernel<true, 64, false>,   gemm_tn_kernel<false, 64, true>,  gemm_tn_kernel<true, 64, true>};
   static bool configured = false;
   if (!configured) {
     for (Kernel k : kernels)
@@ -375,6 +424,30 @@ extern "C" int ob_gemm_tn(const void* a, const void* b, const void* a2, const vo
   if ((reinterpret_cast<uintptr_t>(out) & 15) == 0 && ((ldo * 2) & 15) == 0 &&
       make_bf16_map_2d(&mo, out, rows_a, N, ldo, 64, 32) == 0)
     p.tma_store = 1;
-  kernels[(block_n == 64 ? 2 : 0) + (b_kn ? 1 : 0)]<<<grid, GT_THREADS, GT_SMEM, static_cast<cudaStream_t>(stream)>>>(ma, mb, ma2, mb2, mo, p);
+  p.act = act;
+  p.act_bwd = act_bwd;
+  p.pre = static_cast<__nv_bfloat16*>(pre);
+  CUtensorMap mp = mo;
+  if (act >= 0 && (p.tma_store == 0 || (pre != nullptr && !act_bwd && make_bf16_map_2d(&mp, pre, rows_a, N, ldo, 64, 32) != 0))) return -47;
+  kernels[(act >= 0 ? 4 : block_n == 64 ? 2 : 0) + (b_kn ? 1 : 0)]<<<grid, GT_THREADS, GT_SMEM, static_cast<cudaStream_t>(stream)>>>(ma, mb, ma2, mb2,
+                                                                                                                              mo, mp, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -44;
+}
+}  // namespace ob
+
+extern "C" int ob_gemm_tn(const void* a, const void* b, const void* a2, const void* b2, const void* bias, void* out,
+                          long long rows_a, int N, int K1, int K2, long long lda, long long ldb, long long lda2,
+                          long long ldb2, long long ldo, int b_kn, int b2_kn, float alpha, const int* group_offs, int num_groups,
+                          int block_n, int* status, double wait_budget_s, int num_sms, void* stream) {
+  return ob::gemm_tn(a, b, a2, b2, bias, out, rows_a, N, K1, K2, lda, ldb, lda2, ldb2, ldo, b_kn, b2_kn, alpha, group_offs, num_groups, block_n, -1,
+                     0, nullptr, status, wait_budget_s, num_sms, stream);
+}
+
+extern "C" int ob_gemm_tn_act(const void* a, const void* b, const void* bias, void* out, void* pre, long long rows_a, int N, int K,
+                              long long lda, long long ldb, int b_kn, int act, int backward, int* status, double wait_budget_s,
+                              int num_sms, void* stream) {
+  if (act < 0 || act > 2 || (backward && pre == nullptr)) return -47;
+  if ((N & 63) != 0 || (reinterpret_cast<uintptr_t>(out) & 15) != 0 || (reinterpret_cast<uintptr_t>(pre) & 15) != 0) return -48;
+  return ob::gemm_tn(a, b, nullptr, nullptr, bias, out, rows_a, N, K, 0, lda, ldb, 0, 0, N, b_kn, 0, 1.f, nullptr, 0, 64, act, backward, pre, status,
+                     wait_budget_s, num_sms, stream);
 }

@@ -113,3 +113,33 @@ def test_gated_mlp_as_one_function(rows, inter, trainable):
         # attention's backward may round differently between two runs (2^-8 of single values)
         for a, b in zip(results[0][1:], other[1:]):
             assert float((a - b).norm()) <= 2e-3 * float(b.norm())
+
+
+# one row, edges of the 64-, 128- and 256-wide tiles and of the rounds, several waves of either kernel
+@pytest.mark.parametrize("M,N,K", [(1, 64, 64), (127, 192, 320), (129, 320, 72), (257, 448, 384), (2600, 2368, 200)])
+@pytest.mark.parametrize("act", ["silu", "gelu", "gelu_tanh"])
+@pytest.mark.parametrize("kernel", ["single", "pair", "auto"])
+def test_plain_activation_epilogues(M, N, K, act, kernel):
+    """Forward and backward equal the product and the element-wise kernel bit for bit."""
+    from opaque_b200 import ops
+    from opaque_b200.ops import lib
+    code = {"silu": 0, "gelu": 1, "gelu_tanh": 2}[act]
+
+    def elementwise(x, dy=None):
+        out = torch.empty_like(x)
+        lib.check(lib.load().ob_activation(x.data_ptr(), lib.ptr(dy), out.data_ptr(), x.numel(), code, lib.sm_count(), lib.stream()), "activation")
+        return out
+    torch.manual_seed(M)
+    a, b, w = (torch.randn(*s, device="cuda", dtype=torch.bfloat16) / K ** 0.25 for s in ((M, K), (N, K), (K, N)))
+    bias = torch.randn(N, device="cuda", dtype=torch.bfloat16)
+    bias[:3] = torch.tensor([float("inf"), -100.0, 100.0])
+    st = ops.StatusWord("cuda")
+    f = ops.gemm(a, b, bias=bias)
+    h, x = ops.gemm_act(a, b, bias, act=act, kernel=kernel, status=st)
+    only, none = ops.gemm_act(a, b, bias, act=act, kernel=kernel, save_preact=False, status=st)
+    df = ops.gemm_act_bwd(a, w, f, act=act, kernel=kernel, status=st)
+    assert none is None and st.read() == 0
+    for got, want in ((x, f), (h, elementwise(f)), (only, h), (df, elementwise(f, ops.gemm(a, w, b_layout="kn")))):
+        assert torch.equal(got.view(torch.int16), want.view(torch.int16))
+    with pytest.raises(ValueError):
+        ops.gemm_act_bwd(a, w[:, :-8].contiguous(), f[:, :-8].contiguous(), act=act)
