@@ -33,6 +33,15 @@ def _weight_grads(cap, weight, bias, x2d, g2d):
     return None, None
 
 
+def _norm_sums(trainable, norm, rows):
+    """Where the backward kernel of a trained LayerNorm adds its per-example gradients (weight, bias), or ``(None, None)`` where they are
+    summed apart: few rows, whose sums share a launch with the other layers', or no capture."""
+    cap = fused.current_capture() if trainable else None
+    if cap is None or cap.sums_wait(rows, norm.weight.shape[0]) or rows % cap.batch_size:
+        return None, None
+    return cap.pe_view(norm.weight), cap.pe_view(norm.bias)
+
+
 class GPT2In(Function):
     """``s = x + residual``, its LayerNorm and the query / key / value projection: ``(q, k, v, s)`` with heads ``[B, heads, T, hd]``.
     Without ``residual`` the last output is ``None``: the stream goes on from ``x``."""
@@ -49,12 +58,14 @@ class GPT2In(Function):
     @staticmethod
     def backward(ctx, dq, dk, dv, ds):
         s, stats, y, ln_w, w = ctx.saved_tensors
+        sums = _norm_sums(ctx.trainable, ctx.norm, s.shape[0])
         g, dy, dx = ops.block_steps().gpt2_in_bwd(dq, dk, dv, w, s, ln_w, stats, ds if ctx.carried else None,
-                                                  ctx.needs_input_grad[0] or ctx.trainable)
+                                                  ctx.needs_input_grad[0] or ctx.trainable, *sums)
         dln = dlb = dw = db = None
         if ctx.trainable:
             dw, db = _weight_grads(fused.current_capture(), w, ctx.bias, y, g)
-            dln, dlb = _layer_norm_param_grads(dy, s, ln_w, stats, ctx.norm, True)
+            if sums[0] is None:
+                dln, dlb = _layer_norm_param_grads(dy, s, ln_w, stats, ctx.norm, True)
         if dx is not None:
             dx = dx.view(dq.shape[0], dq.shape[2], -1)
         return dx, (dx if ctx.carried else None), dln, dlb, dw, db, None, None, None
@@ -75,14 +86,15 @@ class GPT2Out(Function):
     @staticmethod
     def backward(ctx, dm, ds):
         s, stats, f, ln_w, wo, w1, w2 = ctx.saved_tensors[:7]
-        g2, g1, dy, dx, do = ops.block_steps().gpt2_out_bwd(dm, f, w2, w1, s, ln_w, stats, ds, wo)
+        sums = _norm_sums(ctx.trainable, ctx.norm, s.shape[0])
+        g2, g1, dy, dx, do = ops.block_steps().gpt2_out_bwd(dm, f, w2, w1, s, ln_w, stats, ds, wo, *sums)
         grads = (None,) * 8
         if ctx.trainable:
             o2, y, h = ctx.saved_tensors[7:]
             cap, (bo, b1, b2) = fused.current_capture(), ctx.biases
             d2 = _weight_grads(cap, w2, b2, h, g2)
             d1 = _weight_grads(cap, w1, b1, y, g1)
-            dln = _layer_norm_param_grads(dy, s, ln_w, stats, ctx.norm, True)
+            dln = _layer_norm_param_grads(dy, s, ln_w, stats, ctx.norm, True) if sums[0] is None else (None, None)
             grads = (*_weight_grads(cap, wo, bo, o2, dx), *dln, *d1, *d2)
         return (do.view(ctx.dims).transpose(1, 2), dx.view(dm.shape), *grads, None, None, None)
 

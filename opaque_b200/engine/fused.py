@@ -215,7 +215,7 @@ class Capture:
         nothing else needs any more: at most :data:`SUM_MATRIX_ELEMS` values each, :data:`SUM_HELD_BYTES` over all layers, and
         what waits is launched when that is reached."""
         held = 4 * g2d.numel()
-        if g2d.shape[0] <= 4096 and g2d.numel() <= SUM_MATRIX_ELEMS and x2d.stride(0) == g2d.stride(0) \
+        if self.sums_wait(*g2d.shape) and x2d.stride(0) == g2d.stride(0) \
                 and (g2d.data_ptr() | x2d.data_ptr()) & 15 == 0:
             if self.sum_held + held > SUM_HELD_BYTES:
                 self._launch_sums()
@@ -223,6 +223,11 @@ class Capture:
             self.sum_held += held
         else:
             ops.functional.rows_group_sum_(out, g2d, self.batch_size, x2d=x2d, mean=mean, rstd=rstd, out_plain=out_plain)
+
+    @staticmethod
+    def sums_wait(rows: int, width: int) -> bool:
+        """Whether the weight sums of a norm of this size wait for other layers'."""
+        return rows <= 4096 and rows * width <= SUM_MATRIX_ELEMS
 
     def _launch_sums(self) -> None:
         for rows in {j[1].shape[0] for j in self.sum_jobs}:

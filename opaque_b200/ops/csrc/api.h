@@ -149,6 +149,10 @@ int ob_add_layernorm_fwd(const void* x, const void* res, const void* w, const vo
                          float* rstd, long long rows, int H, float eps, void* stream);
 int ob_add_layernorm_bwd_dx(const void* dy, const void* x, const void* w, const float* mean, const float* rstd, const void* ds,
                             void* dx, long long rows, int H, void* stream);
+// Either backward (ds NULL or not, H <= 1024) with the per-example sums of ob_rows_group_sum mode 1 into out_w, out_b (may be NULL).
+int ob_layernorm_bwd_sums(const void* dy, const void* x, const void* w, const float* mean, const float* rstd, const void* ds,
+                          void* dx, int num_examples, int rows_per_example, int H, float* out_w, float* out_b, long long ld_out,
+                          void* stream);
 // out[e, :N] += sum over the rows of example e of g (mode 0), g * (x - mean) * rstd (mode 1) or g * x * rstd (mode 2);
 // out row pitch ld_out.  In modes 1 and 2 a non-NULL out2 (row pitch ld_out2) also receives the plain sums of g.
 int ob_rows_group_sum(const void* g, const void* x, const float* mean, const float* rstd, int num_examples,

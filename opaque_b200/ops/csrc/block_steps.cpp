@@ -28,7 +28,7 @@ using at::Tensor;
 
 #define OB_ENTRIES(X)                                                                                                          \
   X(ob_gemm_tn) X(ob_gemm_tn_act) X(ob_gemm_pair) X(ob_gemm_pair_glu_bwd) X(ob_glu_bwd) X(ob_rmsnorm_fwd) X(ob_rmsnorm_bwd) X(ob_layernorm_fwd)  \
-  X(ob_layernorm_bwd_dx) X(ob_add_layernorm_fwd) X(ob_add_layernorm_bwd_dx) X(ob_activation) X(ob_merge_heads3) X(ob_lora_pack) \
+  X(ob_layernorm_bwd_dx) X(ob_layernorm_bwd_sums) X(ob_add_layernorm_fwd) X(ob_add_layernorm_bwd_dx) X(ob_activation) X(ob_merge_heads3) X(ob_lora_pack) \
   X(ob_rope_qk_oop) X(ob_wgrad_clip_batch)
 #define X(name) decltype(&name) p_##name = nullptr;
 OB_ENTRIES(X)
@@ -124,11 +124,24 @@ Normed layer_norm(const Tensor& x, const Tensor& r, const Tensor& w, const Tenso
   }
   return n;
 }
-Tensor layer_norm_bwd(const Tensor& dy, const Tensor& s, const Tensor& w, const Tensor& stats, const Tensor& ds) {
+// sums_w, sums_b [examples, H] (windows of the per-example buffer): the weight's and bias's gradients of every example are added there
+struct Sums {
+  Tensor w, b;
+};
+Tensor layer_norm_bwd(const Tensor& dy, const Tensor& s, const Tensor& w, const Tensor& stats, const Tensor& ds, const Sums& sums) {
   const int64_t R = s.size(0);
   Tensor dx = empty({R, s.size(1)}, s);
   const float* mean = f32(stats);
-  if (!ds.defined())
+  if (sums.w.defined()) {
+    const int64_t E = sums.w.size(0);
+    if (R % E != 0 || sums.w.scalar_type() != at::kFloat || sums.b.scalar_type() != at::kFloat || sums.w.size(1) != s.size(1) ||
+        sums.b.sizes() != sums.w.sizes() || sums.b.stride(0) != sums.w.stride(0) || sums.w.stride(1) != 1 || sums.b.stride(1) != 1) {
+      PyErr_SetString(PyExc_ValueError, "layer_norm_bwd: the sums are fp32 [examples, H] windows of one buffer, rows a multiple of examples");
+      throw PythonError();
+    }
+    LAUNCH(ob_layernorm_bwd_sums, ptr(dy), ptr(s), ptr(w), mean, mean + R, ptr(ds), ptr(dx), (int)E, (int)(R / E), (int)s.size(1),
+           sums.w.data_ptr<float>(), sums.b.data_ptr<float>(), sums.w.stride(0));
+  } else if (!ds.defined())
     LAUNCH(ob_layernorm_bwd_dx, ptr(dy), ptr(s), ptr(w), mean, mean + R, ptr(dx), R, (int)s.size(1));
   else
     LAUNCH(ob_add_layernorm_bwd_dx, ptr(dy), ptr(s), ptr(w), mean, mean + R, ptr(ds), ptr(dx), R, (int)s.size(1));
@@ -294,14 +307,15 @@ PyObject* gpt2_in(Args& a) {
   const Normed n = layer_norm(x, r, lw, lb, a.number());
   return pack({n.y, n.s, n.stats, product(n.y, w, w.size(0), false, with_bias(b))});
 }
-// (dq, dk, dv, w, s, ln_w, stats, ds | None, need_dx) -> g, dy, dx
+// (dq, dk, dv, w, s, ln_w, stats, ds | None, need_dx, sums_w | None, sums_b | None) -> g, dy, dx
 PyObject* gpt2_in_bwd(Args& a) {
   const Tensor dq = a.tensor(), dk = a.tensor(), dv = a.tensor(), w = a.tensor(), s = a.tensor(), lw = a.tensor(), stats = a.tensor(),
                ds = rows(a.optional()), g = merge_heads(dq, dk, dv);
   Tensor dy, dx;
   if (a.integer()) {
+    const Tensor sums_w = a.optional(), sums_b = a.optional();
     dy = product(g, w, s.size(1), true);
-    dx = layer_norm_bwd(dy, s, lw, stats, ds);
+    dx = layer_norm_bwd(dy, s, lw, stats, ds, {sums_w, sums_b});
   }
   return pack({g, dy, dx});
 }
@@ -315,12 +329,12 @@ PyObject* gpt2_out(Args& a) {
   const Tensor h = product_gelu(n.y, w1, b1, a.integer() ? &f : nullptr);
   return pack({o2, n.y, n.s, n.stats, f, h, product(h, w2, w2.size(0), false, with_bias(b2))});
 }
-// (dm, f, w2, w1, s, ln_w, stats, ds, wo) -> g2, g1, dy, dx, do [rows, heads * hd]
+// (dm, f, w2, w1, s, ln_w, stats, ds, wo, sums_w | None, sums_b | None) -> g2, g1, dy, dx, do [rows, heads * hd]
 PyObject* gpt2_out_bwd(Args& a) {
   const Tensor g2 = rows(a.tensor()), f = a.tensor(), w2 = a.tensor(), w1 = a.tensor(), s = a.tensor(), lw = a.tensor(), stats = a.tensor(),
-               ds = rows(a.tensor()), wo = a.tensor();
+               ds = rows(a.tensor()), wo = a.tensor(), sums_w = a.optional(), sums_b = a.optional();
   const Tensor g1 = product_gelu_bwd(g2, w2, f), dy = product(g1, w1, w1.size(1), true);
-  const Tensor dx = layer_norm_bwd(dy, s, lw, stats, ds);
+  const Tensor dx = layer_norm_bwd(dy, s, lw, stats, ds, {sums_w, sums_b});
   return pack({g2, g1, dy, dx, product(dx, wo, wo.size(1), true)});
 }
 

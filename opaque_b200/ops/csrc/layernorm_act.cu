@@ -236,6 +236,7 @@ layernorm_bwd_dx_reg_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfl
 // per row the weight and bias re-reads cost as many wavefronts as the row itself), hence the register-resident
 // parameters; two rows per warp in flight measured slower than one (3.0 vs 3.3 TB/s at H = 768).
 constexpr int LN_WARPS = 8;
+constexpr int LN_WALK_STAGES = 3;
 
 // RES: the row is x + res (rounded to bf16 and stored to `sum`, the residual stream of the next block): the addition in front
 // of a norm costs no pass of its own.  Measured at 16384 x 768: 27.8 us against 12.8 + 11.4 apart forward, 26.0 against
@@ -366,6 +367,227 @@ layernorm_bwd_dx_warp_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bf
       }
       or_[i] = ln_pack8(gw[v]);
     }
+  }
+}
+
+// Rows on their way through shared memory, one warp's: every lane copies the 16-byte vectors that IT will use into its own slots
+// (cp.async; nothing to synchronise but the lane's own copies), STAGES - 1 rows ahead of the row being worked on.  A warp that walks
+// over rows otherwise waits for memory once per row.
+template <int VPL, int TENSORS, int STAGES>
+struct LnRowRing {
+  static constexpr int WARP_BYTES = STAGES * TENSORS * VPL * 512;
+  static constexpr int BYTES = LN_WARPS * WARP_BYTES;
+  const ln_bf16x8* at;      // this lane's slots: [STAGES][TENSORS][VPL] x 32 lanes
+  __device__ __forceinline__ LnRowRing(uint8_t* smem, int warp, int lane) : at(reinterpret_cast<const ln_bf16x8*>(smem + warp * WARP_BYTES) + lane) {}
+  __device__ __forceinline__ void fetch(int stage, int tensor, const __nv_bfloat16* row, int lane, int nv) const {
+#pragma unroll
+    for (int v = 0; v < VPL; ++v)
+      if (lane + v * 32 < nv)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(at + ((stage * TENSORS + tensor) * VPL + v) * 32)),
+                     "l"(reinterpret_cast<const ln_bf16x8*>(row) + lane + v * 32) : "memory");
+  }
+  static __device__ __forceinline__ void commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+  static __device__ __forceinline__ void wait_row() { asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 1) : "memory"); }
+  __device__ __forceinline__ const ln_bf16x8& get(int stage, int tensor, int v) const { return at[((stage * TENSORS + tensor) * VPL + v) * 32]; }
+};
+
+// layernorm_fwd_warp_kernel<VPL, true> for many rows: the same operations on rows that come through a ring.
+template <int VPL>
+__global__ void __launch_bounds__(32 * LN_WARPS, 2)
+add_layernorm_fwd_walk_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ b,
+                              __nv_bfloat16* __restrict__ y, float* __restrict__ mean, float* __restrict__ rstd, long long rows, int H, float eps,
+                              const __nv_bfloat16* __restrict__ res, __nv_bfloat16* __restrict__ sum) {
+  constexpr int STAGES = LN_WALK_STAGES;
+  extern __shared__ uint8_t ln_smem[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const LnRowRing<VPL, 2, STAGES> ring(ln_smem, warp, lane);
+  const long long stride = static_cast<long long>(gridDim.x) * LN_WARPS;
+  long long row = static_cast<long long>(blockIdx.x) * LN_WARPS + warp;
+  if (row >= rows) return;
+  const int nv = H >> 3;
+  const float inv_h = 1.f / H;
+  auto fetch = [&](long long r, int stage) {
+    if (r < rows) {
+      ring.fetch(stage, 0, x + r * H, lane, nv);
+      ring.fetch(stage, 1, res + r * H, lane, nv);
+    }
+    ring.commit();
+  };
+#pragma unroll
+  for (int s = 0; s < STAGES - 1; ++s) fetch(row + s * stride, s);
+  ln_bf16x8 wp[VPL], bp[VPL];
+#pragma unroll
+  for (int v = 0; v < VPL; ++v) {
+    const int i = lane + v * 32;
+    if (i < nv) {
+      wp[v] = reinterpret_cast<const ln_bf16x8*>(w)[i];
+      if (b != nullptr) bp[v] = reinterpret_cast<const ln_bf16x8*>(b)[i];
+    }
+  }
+  int stage = 0;
+  for (; row < rows; row += stride) {
+    fetch(row + (STAGES - 1) * stride, stage == 0 ? STAGES - 1 : stage - 1);
+    ring.wait_row();
+    float f[VPL][8];
+    float s = 0.f, ss = 0.f;
+#pragma unroll
+    for (int v = 0; v < VPL; ++v)
+      if (lane + v * 32 < nv) {
+        float h[8];
+        ln_unpack8(ring.get(stage, 0, v), f[v]);
+        ln_unpack8(ring.get(stage, 1, v), h);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) f[v][j] += h[j];
+        const ln_bf16x8 q = ln_pack8(f[v]);
+        reinterpret_cast<ln_bf16x8*>(sum + row * H)[lane + v * 32] = q;
+        ln_unpack8(q, f[v]);
+      }
+#pragma unroll
+    for (int v = 0; v < VPL; ++v)
+      if (lane + v * 32 < nv) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          s += f[v][j];
+          ss += f[v][j] * f[v][j];
+        }
+      }
+    s = warp_sum(s);
+    ss = warp_sum(ss);
+    const float mu = s * inv_h;
+    const float rs = rsqrtf(fmaxf(ss * inv_h - mu * mu, 0.f) + eps);
+    if (lane == 0) {
+      mean[row] = mu;
+      rstd[row] = rs;
+    }
+#pragma unroll
+    for (int v = 0; v < VPL; ++v) {
+      const int i = lane + v * 32;
+      if (i < nv) {
+        float g[8], h[8];
+        ln_unpack8(wp[v], g);
+        if (b != nullptr) ln_unpack8(bp[v], h);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) f[v][j] = (f[v][j] - mu) * rs * g[j] + (b != nullptr ? h[j] : 0.f);
+        reinterpret_cast<ln_bf16x8*>(y + row * H)[i] = ln_pack8(f[v]);
+      }
+    }
+    if (++stage == STAGES) stage = 0;
+  }
+}
+
+// layernorm_bwd_dx_warp_kernel with the per-example weight and bias sums (rows_group_sum_kernel's mode 1) of the same rows: dy and x are
+// read once for both.  grid = examples x chunks of an example's rows; a warp walks over its chunk with its columns' sums in
+// registers, the block adds its warps' up and adds them to the example's row with atomics.
+// Bound by memory.  Measured with the operands in memory (hot in L2), against layernorm_bwd_dx_warp_kernel and rows_group_sum_kernel: 32 x 512
+// rows of 768 48.1 -> 30.7 us (34.3 -> 22.1), 8 x 1024 31.7 -> 20.5 (18.0 -> 14.3), 16 x 1024 rows of 1024 68.6 -> 47.1 (52.7 -> 41.3);
+// the copy rate allows 15.4, 7.7 and 20.5.  The sums' error against 64 bits is no larger (7.0e-8 and 7.3e-8 of their size).
+template <int VPL, bool RES>
+__global__ void __launch_bounds__(32 * LN_WARPS, 2)
+layernorm_bwd_sums_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
+                          const float* __restrict__ mean, const float* __restrict__ rstd, const __nv_bfloat16* __restrict__ ds,
+                          __nv_bfloat16* __restrict__ dx, int rows_per_example, int chunks, int H, float* __restrict__ out_w,
+                          float* __restrict__ out_b, long long ld_out) {
+  constexpr int TENSORS = RES ? 3 : 2, STAGES = LN_WALK_STAGES;
+  extern __shared__ uint8_t ln_smem[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const LnRowRing<VPL, TENSORS, STAGES> ring(ln_smem, warp, lane);
+  const int e = blockIdx.x / chunks, per = (rows_per_example + chunks - 1) / chunks;
+  const long long r0 = static_cast<long long>(e) * rows_per_example + (blockIdx.x % chunks) * per;
+  const long long r1 = min(r0 + per, static_cast<long long>(e + 1) * rows_per_example);
+  const int nv = H >> 3;
+  auto fetch = [&](long long r, int stage) {
+    if (r < r1) {
+      ring.fetch(stage, 0, dy + r * H, lane, nv);
+      ring.fetch(stage, 1, x + r * H, lane, nv);
+      if constexpr (RES) ring.fetch(stage, 2, ds + r * H, lane, nv);
+    }
+    ring.commit();
+  };
+#pragma unroll
+  for (int s = 0; s < STAGES - 1; ++s) fetch(r0 + warp + s * LN_WARPS, s);
+  ln_bf16x8 wp[VPL];
+  float aw[VPL][8] = {}, ab[VPL][8] = {};
+#pragma unroll
+  for (int v = 0; v < VPL; ++v)
+    if (lane + v * 32 < nv) wp[v] = reinterpret_cast<const ln_bf16x8*>(w)[lane + v * 32];
+  float mu_next = 0.f, rs_next = 0.f;
+  if (r0 + warp < r1) {
+    mu_next = mean[r0 + warp];
+    rs_next = rstd[r0 + warp];
+  }
+  int stage = 0;
+  for (long long row = r0 + warp; row < r1; row += LN_WARPS) {
+    const float mu = mu_next, rs = rs_next;
+    if (row + LN_WARPS < r1) {
+      mu_next = mean[row + LN_WARPS];
+      rs_next = rstd[row + LN_WARPS];
+    }
+    fetch(row + (STAGES - 1) * LN_WARPS, stage == 0 ? STAGES - 1 : stage - 1);
+    ring.wait_row();
+    // one vector of dy * w and of the normalised row, formed twice: kept from the first pass they would not fit the registers
+    auto load = [&](int v, float* g, float* xh, float* gw) {
+      ln_unpack8(ring.get(stage, 0, v), g);
+      ln_unpack8(ring.get(stage, 1, v), xh);
+      ln_unpack8(wp[v], gw);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        xh[j] = (xh[j] - mu) * rs;
+        gw[j] = g[j] * gw[j];
+      }
+    };
+    float s1 = 0.f, s2 = 0.f;
+#pragma unroll
+    for (int v = 0; v < VPL; ++v) {
+      if (lane + v * 32 < nv) {
+        float g[8], xh[8], gw[8];
+        load(v, g, xh, gw);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          ab[v][j] += g[j];
+          aw[v][j] += g[j] * xh[j];
+          s1 += gw[j];
+          s2 += gw[j] * xh[j];
+        }
+      }
+    }
+    const float m1 = warp_sum(s1) / H, m2 = warp_sum(s2) / H;
+#pragma unroll
+    for (int v = 0; v < VPL; ++v) {
+      if (lane + v * 32 < nv) {
+        float g[8], xh[8], gw[8];
+        load(v, g, xh, gw);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) gw[j] = rs * (gw[j] - m1 - xh[j] * m2);
+        if constexpr (RES) {
+          float h[8];
+          ln_unpack8(ring.get(stage, 2, v), h);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) gw[j] = __bfloat162float(__float2bfloat16_rn(gw[j])) + h[j];
+        }
+        reinterpret_cast<ln_bf16x8*>(dx + row * H)[lane + v * 32] = ln_pack8(gw);
+      }
+    }
+    if (++stage == STAGES) stage = 0;
+  }
+  // the block's sums, one of the two at a time through the ring's memory: [LN_WARPS][H]
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  float* red = reinterpret_cast<float*>(ln_smem);
+#pragma unroll
+  for (int which = 0; which < 2; ++which) {
+    __syncthreads();
+#pragma unroll
+    for (int v = 0; v < VPL; ++v)
+      if (lane + v * 32 < nv) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) red[warp * H + (lane + v * 32) * 8 + j] = which == 0 ? aw[v][j] : ab[v][j];
+      }
+    __syncthreads();
+    float* const out = which == 0 ? out_w : out_b;
+    if (out != nullptr)
+      for (int c = threadIdx.x; c < H; c += 32 * LN_WARPS) {
+        const float* q = red + c;
+        atomicAdd(out + e * ld_out + c, ((q[0] + q[H]) + (q[2 * H] + q[3 * H])) + ((q[4 * H] + q[5 * H]) + (q[6 * H] + q[7 * H])));
+      }
   }
 }
 
@@ -580,11 +802,46 @@ activation_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __re
 
 using namespace ob;
 
+static int ln_sms() {
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
+}
+
+template <int VPL>
+static int add_layernorm_fwd_walk(const __nv_bfloat16* x, const __nv_bfloat16* w, const __nv_bfloat16* b, __nv_bfloat16* y, float* mean, float* rstd,
+                                  long long rows, int H, float eps, const __nv_bfloat16* res, __nv_bfloat16* sum, cudaStream_t st) {
+  constexpr int smem = ob::LnRowRing<VPL, 2, ob::LN_WALK_STAGES>::BYTES;
+  static const cudaError_t configured = cudaFuncSetAttribute(add_layernorm_fwd_walk_kernel<VPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (configured != cudaSuccess) return -22;
+  add_layernorm_fwd_walk_kernel<VPL><<<2 * ln_sms(), 32 * LN_WARPS, smem, st>>>(x, w, b, y, mean, rstd, rows, H, eps, res, sum);
+  return cudaGetLastError() == cudaSuccess ? 0 : -21;
+}
+
+template <int VPL, bool RES>
+static int layernorm_bwd_sums(const __nv_bfloat16* dy, const __nv_bfloat16* x, const __nv_bfloat16* w, const float* mean, const float* rstd,
+                              const __nv_bfloat16* ds, __nv_bfloat16* dx, int examples, int rows_per_example, int H, float* out_w, float* out_b,
+                              long long ld_out, cudaStream_t st) {
+  constexpr int ring = ob::LnRowRing<VPL, RES ? 3 : 2, ob::LN_WALK_STAGES>::BYTES;
+  static_assert(ring >= ob::LN_WARPS * VPL * 256 * 4, "the block's sums fit the ring");
+  static const cudaError_t configured =
+      cudaFuncSetAttribute(layernorm_bwd_sums_kernel<VPL, RES>, cudaFuncAttributeMaxDynamicSharedMemorySize, ring);
+  if (configured != cudaSuccess) return -22;
+  // two blocks per SM where there are rows for them, at least a row per warp; 16 chunks at most, as rows_group_sum_kernel has: every
+  // chunk is one more rounding of the example's sum (300 chunks: 2.4e-7 of the sum's size against 1.1e-7)
+  long long chunks = 2LL * ln_sms() / examples;
+  if (chunks > 16) chunks = 16;
+  if (chunks > (rows_per_example + LN_WARPS - 1) / LN_WARPS) chunks = (rows_per_example + LN_WARPS - 1) / LN_WARPS;
+  if (chunks < 1) chunks = 1;
+  layernorm_bwd_sums_kernel<VPL, RES><<<static_cast<unsigned>(examples * chunks), 32 * LN_WARPS, ring, st>>>(
+      dy, x, w, mean, rstd, ds, dx, rows_per_example, static_cast<int>(chunks), H, out_w, out_b, ld_out);
+  return cudaGetLastError() == cudaSuccess ? 0 : -21;
+}
+
 // CTAs of the warp-per-row kernels: one warp per row while that fills fewer CTAs than are resident at once (two per SM
 // for rows wider than 512, else three), else that many CTAs, whose warps walk over the rows
 static unsigned ln_warp_grid(long long rows, int H) {
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = ln_sms();
   const long long want = (rows + ob::LN_WARPS - 1) / ob::LN_WARPS, cap = static_cast<long long>(sms) * (H > 512 ? 2 : 3);
   return static_cast<unsigned>(want < cap ? want : cap);
 }
@@ -618,6 +875,11 @@ extern "C" int ob_add_layernorm_fwd(const void* x, const void* res, const void* 
   const __nv_bfloat16 *xp = static_cast<const __nv_bfloat16*>(x), *wp = static_cast<const __nv_bfloat16*>(w),
                       *bp = static_cast<const __nv_bfloat16*>(b), *rp = static_cast<const __nv_bfloat16*>(res);
   __nv_bfloat16 *yp = static_cast<__nv_bfloat16*>(y), *sp = static_cast<__nv_bfloat16*>(sum);
+  // Rows in flight pay once a warp has more than two rows (us with the operands in memory, hot in L2 in brackets: 16384 x 768 32.8 -> 24.6
+  // (23.4 -> 16.7), 8192 x 768 22.5 -> 15.4 (10.8 -> 9.2), 5000 x 768 16.4 -> 12.3 (7.8 -> 5.9), 16384 x 1024 41.8 -> 31.6 (35.0 -> 26.3)).
+  if (H > 512 && rows > 2 * 2 * static_cast<long long>(ln_sms()) * LN_WARPS)
+    return H <= 768 ? add_layernorm_fwd_walk<3>(xp, wp, bp, yp, mean, rstd, rows, H, eps, rp, sp, st)
+                    : add_layernorm_fwd_walk<4>(xp, wp, bp, yp, mean, rstd, rows, H, eps, rp, sp, st);
   const unsigned octs = ln_warp_grid(rows, H);
   if (H <= 256) layernorm_fwd_warp_kernel<1, true><<<octs, 32 * LN_WARPS, 0, st>>>(xp, wp, bp, yp, mean, rstd, rows, H, eps, rp, sp);
   else if (H <= 512) layernorm_fwd_warp_kernel<2, true><<<octs, 32 * LN_WARPS, 0, st>>>(xp, wp, bp, yp, mean, rstd, rows, H, eps, rp, sp);
@@ -640,6 +902,27 @@ extern "C" int ob_add_layernorm_bwd_dx(const void* dy, const void* x, const void
   else if (H <= 768) layernorm_bwd_dx_warp_kernel<3, true><<<octs, 32 * LN_WARPS, 0, st>>>(gp, xp, wp, mean, rstd, op, rows, H, dp);
   else layernorm_bwd_dx_warp_kernel<4, true><<<octs, 32 * LN_WARPS, 0, st>>>(gp, xp, wp, mean, rstd, op, rows, H, dp);
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
+}
+
+// Either backward (ds may be NULL) with the per-example sums: out_w[e] += sum over example e's rows of dy (x - mean) rstd, out_b[e] += of dy
+// (fp32 rows of pitch ld_out; out_b may be NULL).  H <= 1024.
+extern "C" int ob_layernorm_bwd_sums(const void* dy, const void* x, const void* w, const float* mean, const float* rstd, const void* ds,
+                                     void* dx, int num_examples, int rows_per_example, int H, float* out_w, float* out_b, long long ld_out,
+                                     void* stream) {
+  if (num_examples <= 0 || rows_per_example <= 0) return 0;
+  if (H % 8 || H > 1024 || out_w == nullptr || !aligned16({dy, x, w, ds, dx})) return -2;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const __nv_bfloat16 *gp = static_cast<const __nv_bfloat16*>(dy), *xp = static_cast<const __nv_bfloat16*>(x),
+                      *wp = static_cast<const __nv_bfloat16*>(w), *dp = static_cast<const __nv_bfloat16*>(ds);
+  __nv_bfloat16* op = static_cast<__nv_bfloat16*>(dx);
+#define OB_LN_SUMS(V)                                                                                                                        \
+  return dp != nullptr ? layernorm_bwd_sums<V, true>(gp, xp, wp, mean, rstd, dp, op, num_examples, rows_per_example, H, out_w, out_b, ld_out, st) \
+                       : layernorm_bwd_sums<V, false>(gp, xp, wp, mean, rstd, dp, op, num_examples, rows_per_example, H, out_w, out_b, ld_out, st)
+  if (H <= 256) OB_LN_SUMS(1);
+  if (H <= 512) OB_LN_SUMS(2);
+  if (H <= 768) OB_LN_SUMS(3);
+  OB_LN_SUMS(4);
+#undef OB_LN_SUMS
 }
 
 extern "C" int ob_layernorm_bwd_dx(const void* dy, const void* x, const void* w, const float* mean, const float* rstd,

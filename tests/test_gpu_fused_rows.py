@@ -163,3 +163,44 @@ def test_activation_variants(rows, I, pitched, act):
     if act != "relu":
         dg, du = F.glu_backward(dh, gate, up, act)
         assert close(dg, d_act * up.double(), d * u * e_bwd) and close(du, dh.double() * fn(gate.double()), d * e_fwd)
+
+
+# one row per example, fewer rows than warps, ragged chunks, several rows per warp; widths at the edges of the vectors per lane
+@pytest.mark.parametrize("E,T,H", [(1, 1, 8), (3, 7, 256), (300, 2, 264), (5, 333, 512), (2, 1000, 768), (7, 130, 776), (9, 600, 1024)])
+@pytest.mark.parametrize("residual", [True, False])
+def test_layer_norm_backward_with_sums(E, T, H, residual):
+    """Data gradient: the bits of the kernels without the sums.  Sums: against 64 bits; fp32 sums of T terms, 2^-24 each times a factor
+    of two for the terms' own roundings and sqrt(T) for their number."""
+    from opaque_b200.ops import lib
+    torch.manual_seed(T)
+    rows = E * T
+    dy, x, ds = (torch.randn(rows, H, device="cuda").bfloat16() for _ in range(3))
+    w = torch.randn(H, device="cuda").bfloat16()
+    stats = torch.stack([x.float().mean(1), 1 / x.float().std(1, unbiased=False).clamp_min(0.1)]).contiguous()
+    mean, rstd = stats.data_ptr(), stats.data_ptr() + 4 * rows
+    L, want, got = lib.load(), torch.empty_like(dy), torch.empty_like(dy)
+    if residual:
+        lib.check(L.ob_add_layernorm_bwd_dx(dy.data_ptr(), x.data_ptr(), w.data_ptr(), mean, rstd, ds.data_ptr(), want.data_ptr(), rows, H, lib.stream()), "")
+    else:
+        lib.check(L.ob_layernorm_bwd_dx(dy.data_ptr(), x.data_ptr(), w.data_ptr(), mean, rstd, want.data_ptr(), rows, H, lib.stream()), "")
+    pe = torch.ones(E, 2 * H + 8, device="cuda")
+    lib.check(L.ob_layernorm_bwd_sums(dy.data_ptr(), x.data_ptr(), w.data_ptr(), mean, rstd, ds.data_ptr() if residual else None, got.data_ptr(), E, T, H,
+                                      pe.data_ptr(), pe.data_ptr() + 4 * H, pe.stride(0), lib.stream()), "layernorm_bwd_sums")
+    assert torch.equal(got, want)
+    xh = (x.double() - stats[0].double()[:, None]) * stats[1].double()[:, None]
+    ref = torch.cat([(dy.double() * xh).view(E, T, H).sum(1), dy.double().view(E, T, H).sum(1)], 1)
+    assert torch.all(pe[:, 2 * H:] == 1) and float((pe[:, :2 * H].double() - 1 - ref).norm()) <= 2 ** -23 * (T ** 0.5 + 2) * float((1 + ref.abs()).norm())
+
+
+@pytest.mark.parametrize("rows,H", [(4737, 520), (4800, 768), (9473, 776), (5000, 1024)])
+def test_add_layer_norm_of_many_rows(rows, H):
+    """Rows that come through the ring: against the fp32 statement, and the bits that the same rows have in a short call."""
+    from opaque_b200 import ops
+    torch.manual_seed(rows)
+    x, r = (torch.randn(rows, H, device="cuda").bfloat16() for _ in range(2))
+    w, b = (torch.randn(H, device="cuda").bfloat16() for _ in range(2))
+    y, s = ops.add_layer_norm(x, r, w, b)
+    assert torch.equal(s, x + r)
+    for lo in (0, rows - 100):
+        ys, _ = ops.add_layer_norm(x[lo:lo + 100], r[lo:lo + 100], w, b)
+        assert torch.equal(ys, y[lo:lo + 100])
