@@ -139,6 +139,10 @@ int ob_rope_qk_oop(const void* q_in, const void* k_in, void* q_out, void* k_out,
                    const int* pos, long long rows, int seq_len, int Hq, int Hk, int D, long long q_sb, long long q_st,
                    long long q_sh, long long k_sb, long long k_st, long long k_sh, int backward, int sms, void* stream);
 
+// The same with v, copied, and one output [rows, (Hq + 2 Hk) D]; strides[9] (host): batch, token, head stride of q, k, v.
+int ob_rope_qkv_gather(const void* q_in, const void* k_in, const void* v_in, void* out, const float* cos_t, const float* sin_t,
+                       const long long* strides, long long rows, int seq_len, int Hq, int Hk, int D, int backward, int sms, void* stream);
+
 // LayerNorm over the last dimension (bf16 in/out, fp32 statistics saved per row).
 int ob_layernorm_fwd(const void* x, const void* w, const void* b, void* y, float* mean, float* rstd, long long rows,
                      int H, float eps, void* stream);

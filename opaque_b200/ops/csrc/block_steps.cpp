@@ -29,7 +29,7 @@ using at::Tensor;
 #define OB_ENTRIES(X)                                                                                                          \
   X(ob_gemm_tn) X(ob_gemm_tn_act) X(ob_gemm_pair) X(ob_gemm_pair_glu_bwd) X(ob_glu_bwd) X(ob_rmsnorm_fwd) X(ob_rmsnorm_bwd) X(ob_layernorm_fwd)  \
   X(ob_layernorm_bwd_dx) X(ob_layernorm_bwd_sums) X(ob_add_layernorm_fwd) X(ob_add_layernorm_bwd_dx) X(ob_activation) X(ob_merge_heads3) X(ob_lora_pack) \
-  X(ob_rope_qk_oop) X(ob_wgrad_clip_batch)
+  X(ob_rope_qk_oop) X(ob_rope_qkv_gather) X(ob_wgrad_clip_batch)
 #define X(name) decltype(&name) p_##name = nullptr;
 OB_ENTRIES(X)
 #undef X
@@ -204,14 +204,25 @@ Tensor product_gelu_bwd(const Tensor& g, const Tensor& w, const Tensor& f) {
 bool rope_reads(const Tensor& t) {
   return t.stride(3) == 1 && (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0 && ((t.stride(0) | t.stride(1) | t.stride(2)) & 7) == 0;
 }
-std::pair<Tensor, Tensor> rope(Tensor q, Tensor k, const Tensor& cs, const Tensor& sn, bool backward) {
-  if (!rope_reads(q)) q = q.clone(at::MemoryFormat::Contiguous);
-  if (!rope_reads(k)) k = k.clone(at::MemoryFormat::Contiguous);
+std::pair<Tensor, Tensor> rope(const Tensor& q, const Tensor& k, const Tensor& cs, const Tensor& sn) {
   const int64_t B = q.size(0), T = q.size(1), hd = q.size(3);
   Tensor qo = empty({B, T, q.size(2), hd}, q), ko = empty({B, T, k.size(2), hd}, k);
   LAUNCH(ob_rope_qk_oop, ptr(q), ptr(k), ptr(qo), ptr(ko), f32(cs), f32(sn), nullptr, B * T, (int)T, (int)q.size(2), (int)k.size(2), (int)hd, q.stride(0),
-         q.stride(1), q.stride(2), k.stride(0), k.stride(1), k.stride(2), backward, g_sms);
+         q.stride(1), q.stride(2), k.stride(0), k.stride(1), k.stride(2), 0, g_sms);
   return {qo, ko};
+}
+// gradients [B, heads, T, hd] -> [B * T, (heads + 2 kv heads) * hd], query and key rotated back
+Tensor rope_backward(Tensor q, Tensor k, Tensor v, const Tensor& cs, const Tensor& sn) {
+  long long strides[9];
+  int i = 0;
+  for (Tensor* t : {&q, &k, &v}) {
+    if (!rope_reads(*t)) *t = t->clone(at::MemoryFormat::Contiguous);
+    for (int d : {0, 2, 1}) strides[i++] = t->stride(d);
+  }
+  const int64_t B = q.size(0), Hq = q.size(1), T = q.size(2), hd = q.size(3), Hk = k.size(1);
+  Tensor out = empty({B * T, (Hq + 2 * Hk) * hd}, q);
+  LAUNCH(ob_rope_qkv_gather, ptr(q), ptr(k), ptr(v), ptr(out), f32(cs), f32(sn), strides, B * T, (int)T, (int)Hq, (int)Hk, (int)hd, 1, g_sms);
+  return out;
 }
 // three gradients [B, heads, T, hd] -> [B * T, 3 * heads * hd]
 Tensor merge_heads(const Tensor& q, const Tensor& k, const Tensor& v) {
@@ -356,7 +367,7 @@ PyObject* lora_in(Args& a) {
          (int)bk.size(0), (int)bv.size(0), g_sms);
   const Tensor xa = product(n.y, a_cat, 3 * rank, false, scaled(scaling)), qkv = product(n.y, w_all, w_all.size(0), false, segment(xa, b_block, false));
   const Tensor heads = qkv.view({x3.size(0), x3.size(1), nh + 2 * nkv, hd});
-  const auto [q, k] = rope(heads.narrow(2, 0, nh), heads.narrow(2, nh, nkv), cs, sn, false);
+  const auto [q, k] = rope(heads.narrow(2, 0, nh), heads.narrow(2, nh, nkv), cs, sn);
   return pack({n.y, n.s, n.stats, a_cat, b_block, xa, q, k, qkv});
 }
 // (dq, dk, dv [B, heads, T, hd], cos, sin, b_block, scaling, w_all, a_cat, s, norm_w, rstd, ds | None, offset, need_dx) -> g, q_all, dx
@@ -365,10 +376,7 @@ PyObject* lora_in_bwd(Args& a) {
   const double scaling = a.number();
   const Tensor w_all = a.tensor(), a_cat = a.tensor(), s = a.tensor(), nw = a.tensor(), rstd = a.tensor(), ds = rows(a.optional());
   const double offset = a.number();
-  const int64_t R = dq.size(0) * dq.size(2);
-  const auto [q, k] = rope(dq.transpose(1, 2), dk.transpose(1, 2), cs, sn, true);
-  const Tensor g = at::cat({q.view({R, -1}), k.view({R, -1}), dv.transpose(1, 2).reshape({R, -1})}, 1);
-  const Tensor q_all = product(g, b_block, b_block.size(1), true, scaled(scaling));
+  const Tensor g = rope_backward(dq, dk, dv, cs, sn), q_all = product(g, b_block, b_block.size(1), true, scaled(scaling));
   Tensor dx;
   if (a.integer()) dx = rms_norm_bwd(product(g, w_all, w_all.size(1), true, segment(q_all, a_cat, true)), s, nw, rstd, ds, offset);
   return pack({g, q_all, dx});

@@ -393,14 +393,18 @@ struct RopeSrc {
 
 // Idx is 32 bits wide where the element count allows: two 64-bit divisions per vector cost more than its loads hid.  Measured on 16384 rows of
 // 32 + 8 heads of 128: 71.1 -> 65.9 us (51 at the copy rate).
-template <typename Idx>
+// GATHER: the outputs are slices of ONE buffer [rows, (Hq + 2 Hk) D] at `qo`, q then k then v (copied): the gradient of a fused q|k|v
+// projection, which three tensors and a concatenation had made.  power-capped, 16384 rows of 32 + 8 + 8
+// heads of 128 115 -> 67 us, 5439 rows with heads of 64 19.8 -> 9.7, 256 rows 4.1 -> 2.5.
+template <typename Idx, bool GATHER>
 __global__ void __launch_bounds__(256)
-rope_qk_oop_kernel(RopeSrc qs, RopeSrc ks, __nv_bfloat16* __restrict__ qo, __nv_bfloat16* __restrict__ ko,
+rope_qk_oop_kernel(RopeSrc qs, RopeSrc ks, RopeSrc vs, __nv_bfloat16* __restrict__ qo, __nv_bfloat16* __restrict__ ko,
                    const float* __restrict__ cs, const float* __restrict__ sn, const int* __restrict__ pos,
                    long long rows, int seq_len, int Hq, int Hk, int D, float sign) {
   const int half = D >> 1;
   const int chunks = half >> 3;                          // 8-element chunks per half head
-  const unsigned per_row = static_cast<unsigned>(Hq + Hk) * chunks;
+  const int heads = GATHER ? Hq + 2 * Hk : Hq + Hk;
+  const unsigned per_row = static_cast<unsigned>(heads) * chunks;
   const Idx total = static_cast<Idx>(rows * per_row);
   for (Idx i = static_cast<Idx>(blockIdx.x) * 256 + threadIdx.x; i < total; i += static_cast<Idx>(gridDim.x) * 256) {
     const Idx r32 = i / per_row;
@@ -410,11 +414,17 @@ rope_qk_oop_kernel(RopeSrc qs, RopeSrc ks, __nv_bfloat16* __restrict__ qo, __nv_
     const Idx b32 = r32 / static_cast<unsigned>(seq_len);
     const long long r = r32, b = b32, t = r32 - b32 * static_cast<unsigned>(seq_len);
     const int pidx = pos ? pos[r] : static_cast<int>(t);
-    const bool is_q = h < Hq;
-    const int hh = is_q ? h : h - Hq;
-    const RopeSrc& src = is_q ? qs : ks;
+    const bool is_q = h < Hq, is_v = GATHER && h >= Hq + Hk;
+    const int hh = is_q ? h : (is_v ? h - Hq - Hk : h - Hq);
+    const RopeSrc& src = is_q ? qs : (is_v ? vs : ks);
     const __nv_bfloat16* in = src.ptr + b * src.sb + t * src.st + hh * src.sh;
-    __nv_bfloat16* out = (is_q ? qo + r * Hq * D : ko + r * Hk * D) + static_cast<long long>(hh) * D;
+    __nv_bfloat16* out = GATHER ? qo + (r * heads + h) * D : (is_q ? qo + r * Hq * D : ko + r * Hk * D) + static_cast<long long>(hh) * D;
+    if (GATHER && is_v) {
+      const uint4 a = *reinterpret_cast<const uint4*>(in + d), z = *reinterpret_cast<const uint4*>(in + half + d);
+      *reinterpret_cast<uint4*>(out + d) = a;
+      *reinterpret_cast<uint4*>(out + half + d) = z;
+      continue;
+    }
     const uint4 lo4 = *reinterpret_cast<const uint4*>(in + d);
     const uint4 hi4 = *reinterpret_cast<const uint4*>(in + half + d);
     const float* cp = cs + static_cast<long long>(pidx) * half + d;
@@ -702,9 +712,32 @@ extern "C" int ob_rope_qk_oop(const void* q_in, const void* k_in, void* q_out, v
   __nv_bfloat16 *qo = static_cast<__nv_bfloat16*>(q_out), *ko = static_cast<__nv_bfloat16*>(k_out);
   const float sign = backward ? -1.f : 1.f;
   if (work < 0x7fffffffLL)
-    rope_qk_oop_kernel<unsigned><<<grid, 256, 0, st>>>(qs, ks, qo, ko, cos_t, sin_t, pos, rows, seq_len, Hq, Hk, D, sign);
+    rope_qk_oop_kernel<unsigned, false><<<grid, 256, 0, st>>>(qs, ks, ks, qo, ko, cos_t, sin_t, pos, rows, seq_len, Hq, Hk, D, sign);
   else
-    rope_qk_oop_kernel<unsigned long long><<<grid, 256, 0, st>>>(qs, ks, qo, ko, cos_t, sin_t, pos, rows, seq_len, Hq, Hk, D, sign);
+    rope_qk_oop_kernel<unsigned long long, false><<<grid, 256, 0, st>>>(qs, ks, ks, qo, ko, cos_t, sin_t, pos, rows, seq_len, Hq, Hk, D, sign);
+  return OB_CHECK_LAUNCH();
+}
+
+// The same with v, copied, and one output [rows, (Hq + 2 Hk) D]; strides[9]: batch, token, head stride of q, k, v in elements.
+extern "C" int ob_rope_qkv_gather(const void* q_in, const void* k_in, const void* v_in, void* out, const float* cos_t, const float* sin_t,
+                                  const long long* strides, long long rows, int seq_len, int Hq, int Hk, int D, int backward, int sms,
+                                  void* stream) {
+  if (rows <= 0) return 0;
+  if (D % 16) return -2;
+  long long all = 0;
+  for (int i = 0; i < 9; ++i) all |= strides[i];
+  if (!aligned16({q_in, k_in, v_in, out, cos_t, sin_t}) || (all & 7) != 0) return -3;
+  auto src = [&](const void* p, int i) { return RopeSrc{static_cast<const __nv_bfloat16*>(p), strides[3 * i], strides[3 * i + 1], strides[3 * i + 2]}; };
+  const long long work = rows * (Hq + 2 * Hk) * (D / 16);
+  const unsigned grid = flat_grid(work, 256, sms);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  __nv_bfloat16* o = static_cast<__nv_bfloat16*>(out);
+  const float sign = backward ? -1.f : 1.f;
+  const RopeSrc q = src(q_in, 0), k = src(k_in, 1), v = src(v_in, 2);
+  if (work < 0x7fffffffLL)
+    rope_qk_oop_kernel<unsigned, true><<<grid, 256, 0, st>>>(q, k, v, o, nullptr, cos_t, sin_t, nullptr, rows, seq_len, Hq, Hk, D, sign);
+  else
+    rope_qk_oop_kernel<unsigned long long, true><<<grid, 256, 0, st>>>(q, k, v, o, nullptr, cos_t, sin_t, nullptr, rows, seq_len, Hq, Hk, D, sign);
   return OB_CHECK_LAUNCH();
 }
 

@@ -29,6 +29,7 @@ _SIGNATURES = {
     "ob_pair_set_die_aware": [I],
     "ob_die_map": [P, I],
     "ob_layernorm_bwd_sums": [P, P, P, P, P, P, P, I, I, I, P, P, LL, P],
+    "ob_rope_qkv_gather": [P, P, P, P, P, P, P, LL, I, I, I, I, I, I, P],
     "ob_gemm_tn_act": [P, P, P, P, P, LL, I, I, LL, LL, I, I, I, P, D, I, P],
     "ob_gemm_pair_glu_bwd": [P, P, P, P, P, P, LL, I, I, LL, LL, LL, LL, I, I, P, D, I, P],
     "ob_linear_ce_fwd": [P, P, P, P, P, P, P, LL, I, I, LL, LL, LL, F, F, LL, P, D, I, P],

@@ -80,6 +80,24 @@ def test_llama_lora(B, T, r, mode):
     _close(one, two)
 
 
+@pytest.mark.parametrize("B,T,Hq,Hk,D", [(1, 1, 1, 1, 16), (2, 77, 4, 2, 32), (3, 130, 8, 8, 64), (2, 300, 6, 3, 128)])
+def test_rotary_gradients_into_one_buffer(B, T, Hq, Hk, D):
+    """q, k rotated back and v copied, from [B, heads, T, D] and from [B, T, heads, D] storage: the bits of the rotation and a concatenation."""
+    import ctypes
+    from opaque_b200 import ops
+    from opaque_b200.ops import lib
+    torch.manual_seed(T)
+    cos, sin = ops.rope_tables(D, 512, 10000.0, device="cuda")
+    q, k, v = (torch.randn(B, T, h, D, device="cuda", dtype=torch.bfloat16) for h in (Hq, Hk, Hk))
+    v = v.transpose(1, 2).contiguous().transpose(1, 2)
+    out = torch.empty(B * T, (Hq + 2 * Hk) * D, device="cuda", dtype=torch.bfloat16)
+    strides = (ctypes.c_longlong * 9)(*(t.stride(d) for t in (q, k, v) for d in range(3)))
+    lib.check(lib.load().ob_rope_qkv_gather(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), cos.data_ptr(), sin.data_ptr(),
+                                            ctypes.addressof(strides), B * T, T, Hq, Hk, D, 1, lib.sm_count(), lib.stream()), "rope_qkv_gather")
+    qr, kr = ops.functional._RoPE._run(q, k, cos, sin, None, 1)
+    assert torch.equal(out, torch.cat([t.reshape(B * T, -1) for t in (qr, kr, v)], 1))
+
+
 def test_without_the_compiled_sequences(monkeypatch):
     """Where the extension is missing, blocks run node by node and the factor gradients go through the general batch entry point."""
     from opaque_b200 import ops
