@@ -111,6 +111,17 @@ def _batch_splits(tiles: int, rows: int, max_splits: int | None = None, peer: bo
     return pick_splits(max(tiles, 1), rows, sms, max_splits=max_splits)
 
 
+@functools.lru_cache(maxsize=4096)
+def _packed_splits(tiles: int, rows: int, most: int, peer: int) -> int:
+    return _batch_splits(tiles, rows, most if most > 0 else None, bool(peer))
+
+
+def _native(name: str, wait_budget_s: float = DEFAULT_WAIT_BUDGET_S):
+    """The compiled packer of a batch entry point, or ``None``; it returns False for problems that Python should look at."""
+    steps = block_steps() if wait_budget_s == DEFAULT_WAIT_BUDGET_S else None
+    return None if steps is None else getattr(steps, name)
+
+
 def wgrad_clip_batch(problems: Sequence[dict], out: torch.Tensor | None, *, accumulate: bool = True, peer_table: torch.Tensor | None = None,
                      shard_elems: int = 0, block_n: int = 256, status: StatusWord | None = None,
                      wait_budget_s: float = DEFAULT_WAIT_BUDGET_S) -> None:
@@ -118,6 +129,9 @@ def wgrad_clip_batch(problems: Sequence[dict], out: torch.Tensor | None, *, accu
     ``a``, ``b`` and optional ``row_scale``, ``seg_offsets``, ``num_groups``, ``out_offset``, ``ldm``, ``ldn``, ``n_valid``,
     ``group_stride``.  ``block_n`` is 256 or 64.  K is split (``accumulate`` only, ungrouped problems) when the whole list
     would leave SMs idle."""
+    native = _native("wgrad_batch", wait_budget_s) if accumulate and block_n == 256 else None
+    if native is not None and native(problems, out, peer_table, shard_elems, status.ptr() if status else 0):
+        return
     tiles = sum(pr.get("num_groups", 1) * math.ceil(pr["a"].shape[1] / 128) * math.ceil(pr["b"].shape[1] / block_n) for pr in problems)
     jobs = []
     for pr in problems:
@@ -268,6 +282,9 @@ def wgrad_clip_per_example_batch(problems: Sequence[tuple], out: torch.Tensor | 
                                  wait_budget_s: float = DEFAULT_WAIT_BUDGET_S) -> None:
     """Several accumulating :func:`wgrad_clip_per_example` problems ``(a, b, ex_scale, out_offset, ldm)`` in one launch (per 56).
     ``rows_per_example`` may have any length here: an example's last 64-row block is filled up with zeros."""
+    native = _native("wgrad_pe_batch", wait_budget_s)
+    if native is not None and native(problems, out, rows_per_example, peer_table, shard_elems, status.ptr() if status else 0):
+        return
     tiles = sum(math.ceil(pr[0].shape[1] / 128) * math.ceil(pr[1].shape[1] / 256) for pr in problems)
     descs = []
     for a, b, ex_scale, off, ldm in problems:
@@ -349,6 +366,9 @@ def _check_ghost(a, g, norm2, tokens_per_example, ids, seg_offsets, seg_out):
 def ghost_norm_batch(problems: Sequence[tuple], *, status: StatusWord | None = None, wait_budget_s: float = DEFAULT_WAIT_BUDGET_S) -> None:
     """Several :func:`ghost_norm` problems ``(a, g, norm2, tokens_per_example, ids, seg_offsets, seg_out)`` in one launch per
     Gram block shape (and per 56 problems): their items share one work list, longest first."""
+    native = _native("ghost_batch", wait_budget_s)
+    if native is not None and native(problems, status.ptr() if status else 0):
+        return
     jobs = []
     for a, g, norm2, tokens, ids, seg_offsets, seg_out in problems:
         rows, B, da, dg, lda, ap = _check_ghost(a, g, norm2, tokens, ids, seg_offsets, seg_out)
@@ -532,7 +552,7 @@ def gemm_glu_bwd(dy: torch.Tensor, w_down: torch.Tensor, gate: torch.Tensor, up:
 def _act_single(M: int, N: int, K: int, kernel: str) -> bool:
     """Which kernel :func:`gemm_act` and :func:`gemm_act_bwd` run: the single-CTA one (64-column tiles) or the pair kernel."""
     if kernel == "auto":
-        return N % 64 == 0 and _plan_code(M, N, K, 0, 0) != 0
+        return N % 64 == 0 and _plan_code(M, N, K, 0, 2) != 0
     return {"single": True, "pair": False}[kernel]
 
 
@@ -787,16 +807,24 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, b_layout: str = "nk", a2: torch.Te
     return out
 
 
-def _plan_code(M: int, N: int, K: int, K2: int, single: int) -> int:
-    """:func:`gemm`'s choice as a number: 0 for the pair kernel, else the single-CTA kernel's tile width."""
+def _plan_code(M: int, N: int, K: int, K2: int, mode: int) -> int:
+    """:func:`gemm`'s choice as a number: 0 for the pair kernel, else the single-CTA kernel's tile width.  ``mode`` 1: single-CTA only.
+    2: a product with an activation in its epilogue, which wide single-CTA tiles do not have (us, element-wise launch apart / pair /
+    64-column tiles, N = 3072, K = 768, forward: 128 rows 8.4 / 13.1 / 8.0, 512 12.5 / 13.3 / 10.6, 1024 13.9 / 13.7 / 13.7, 1285 14.8 /
+    14.2 / 19.0, 3663 27.7 / 26.4, 16384 117 / 98)."""
     sms = lib.sm_count()
-    return 0 if not single and pick_gemm_plan(M, N, K, K2, sms) == "pair" else pick_tile_width(M, N, -(-K // 64) + -(-K2 // 64), sms)
+    nk = -(-K // 64) + -(-K2 // 64)
+    if mode == 2:
+        return 0 if _pair_us(M, N, nk, sms) <= _single_us(M, N, nk, 64, sms) else 64
+    return 0 if mode == 0 and pick_gemm_plan(M, N, K, K2, sms) == "pair" else pick_tile_width(M, N, nk, sms)
 
 
 @functools.lru_cache(maxsize=None)
 def block_steps():
-    """The compiled launch sequences of whole sub-layers (``csrc/block_steps.cpp``), or ``None`` where they cannot be built or loaded."""
-    return lib.load_block_steps(_plan_code, DEFAULT_WAIT_BUDGET_S)
+    """The compiled launch sequences (``csrc/block_steps.cpp``), or ``None`` without a GPU or where they cannot be built or loaded."""
+    if not torch.cuda.is_available():
+        return None
+    return lib.load_block_steps(_plan_code, _packed_splits, DEFAULT_WAIT_BUDGET_S)
 
 
 def gemm_ref(a, b, *, b_layout="nk", a2=None, b2=None, bias=None, group_offs=None):

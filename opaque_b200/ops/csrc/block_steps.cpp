@@ -12,9 +12,11 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <algorithm>
 #include <array>
 #include <initializer_list>
 #include <map>
+#include <vector>
 
 #include "api.h"
 
@@ -29,12 +31,14 @@ using at::Tensor;
 #define OB_ENTRIES(X)                                                                                                          \
   X(ob_gemm_tn) X(ob_gemm_tn_act) X(ob_gemm_pair) X(ob_gemm_pair_glu_bwd) X(ob_glu_bwd) X(ob_rmsnorm_fwd) X(ob_rmsnorm_bwd) X(ob_layernorm_fwd)  \
   X(ob_layernorm_bwd_dx) X(ob_layernorm_bwd_sums) X(ob_add_layernorm_fwd) X(ob_add_layernorm_bwd_dx) X(ob_activation) X(ob_merge_heads3) X(ob_lora_pack) \
-  X(ob_rope_qk_oop) X(ob_rope_qkv_gather) X(ob_wgrad_clip_batch)
+  X(ob_rope_qk_oop) X(ob_rope_qkv_gather) X(ob_wgrad_clip_batch) X(ob_wgrad_clip_pe_batch) \
+  X(ob_ghost_norm_batch) X(ob_rows_sum_batch)
 #define X(name) decltype(&name) p_##name = nullptr;
 OB_ENTRIES(X)
 #undef X
 
-PyObject *g_check = nullptr, *g_plan = nullptr;      // lib.check(rc, what); (M, N, K, K2, single) -> 0 pair, 64 or 256: tile width
+// lib.check(rc, what); (M, N, K, K2, mode) -> 0 pair, 64 or 256: tile width; (tiles, rows, most, peer) -> splits of a weight gradient
+PyObject *g_check = nullptr, *g_plan = nullptr, *g_splits = nullptr;
 int g_sms = 0;
 double g_budget = 0.0;
 
@@ -71,12 +75,13 @@ Tensor rows(const Tensor& t) { return t.defined() ? vec16(t.reshape({-1, t.size(
 // ------------------------------------------------------------------------------------------------------- single launches
 
 // The choice of kernel and tile is the Python rule's; it is asked once per shape.
-int plan(int64_t M, int64_t N, int64_t K, int64_t K2, bool single) {
+enum : int { ANY = 0, SINGLE = 1, ACTIVATION = 2 };
+int plan(int64_t M, int64_t N, int64_t K, int64_t K2, int mode) {
   static std::map<std::array<int64_t, 5>, int> known;
-  const std::array<int64_t, 5> key{M, N, K, K2, single};
+  const std::array<int64_t, 5> key{M, N, K, K2, mode};
   const auto at = known.find(key);
   if (at != known.end()) return at->second;
-  PyObject* r = PyObject_CallFunction(g_plan, "LLLLi", (long long)M, (long long)N, (long long)K, (long long)K2, (int)single);
+  PyObject* r = PyObject_CallFunction(g_plan, "LLLLi", (long long)M, (long long)N, (long long)K, (long long)K2, mode);
   if (r == nullptr) throw PythonError();
   const int width = static_cast<int>(PyLong_AsLong(r));
   Py_DECREF(r);
@@ -94,7 +99,7 @@ struct Opt {                                         // the optional parts of a 
 Tensor product(const Tensor& a, const Tensor& b, int64_t N, bool kn, const Opt& o = {}) {
   const int64_t M = a.size(0), K = a.size(1), K2 = o.a2.defined() ? o.a2.size(1) : 0;
   Tensor out = empty({M, N}, a);
-  const int width = plan(M, N, K, K2, o.single);
+  const int width = plan(M, N, K, K2, o.single ? SINGLE : ANY);
   const int64_t lda2 = K2 ? o.a2.stride(0) : 0, ldb2 = K2 ? o.b2.stride(0) : 0;
   if (width == 0)
     LAUNCH(ob_gemm_pair, ptr(a), ptr(b), nullptr, ptr(o.a2), ptr(o.b2), nullptr, ptr(o.bias), ptr(out), nullptr, nullptr, M, (int)N, (int)K, (int)K2,
@@ -165,10 +170,7 @@ Tensor gelu(const Tensor& x, const Tensor& dy) {
   LAUNCH(ob_activation, ptr(x), ptr(dy), ptr(out), x.numel(), GELU_TANH, g_sms);
   return out;
 }
-// GPT-2's GELU in the epilogue of the product around it: the pair kernel's, or the single-CTA kernel's with 64-column tiles, also where
-// the plain product would take wide ones (us, both launches / this, N = 3072, K = 768: 128 rows 8.4 / 8.0, 512 12.5 / 10.6, 1024
-// 13.9 / 13.7, 1285 14.8 / 14.2, 3663 27.7 / 26.4, 16384 117 / 98; backward 8.0 / 7.8, 12.3 / 11.4, 13.9 / 14.4, 14.9 / 13.9,
-// 30.3 / 25.9, 127 / 106).
+// GPT-2's GELU in the epilogue of the product around it: the pair kernel's or, with 64-column tiles, the single-CTA kernel's.
 // -> gelu(x b^T + bias) and, with `pre`, its argument there (allocated)
 Tensor product_gelu(const Tensor& x, const Tensor& b, const Tensor& bias, Tensor* pre) {
   const int64_t M = x.size(0), N = b.size(0), K = x.size(1);
@@ -180,7 +182,7 @@ Tensor product_gelu(const Tensor& x, const Tensor& b, const Tensor& bias, Tensor
   Tensor h = empty({M, N}, x);
   if (pre != nullptr) *pre = empty({M, N}, x);
   void* const f = pre != nullptr ? ptr(*pre) : nullptr;
-  if (plan(M, N, K, 0, false) == 0)
+  if (plan(M, N, K, 0, ACTIVATION) == 0)
     LAUNCH(ob_gemm_pair, ptr(x), ptr(b), nullptr, nullptr, nullptr, nullptr, ptr(bias), ptr(h), f, nullptr, M, (int)N, (int)K, 0, x.stride(0),
            b.stride(0), 0, 0, N, 0, 0, 2, GELU_TANH, -1, nullptr, g_budget, g_sms);
   else
@@ -192,7 +194,7 @@ Tensor product_gelu_bwd(const Tensor& g, const Tensor& w, const Tensor& f) {
   const int64_t M = g.size(0), N = w.size(1), K = g.size(1);
   if (N % 64 != 0) return gelu(f, product(g, w, N, true));
   Tensor df = empty({M, N}, g);
-  if (plan(M, N, K, 0, false) == 0)
+  if (plan(M, N, K, 0, ACTIVATION) == 0)
     LAUNCH(ob_gemm_pair_glu_bwd, ptr(g), ptr(w), ptr(f), nullptr, ptr(df), nullptr, M, (int)N, (int)K, g.stride(0), w.stride(0), N, N, 1, GELU_TANH,
            nullptr, g_budget, g_sms);
   else
@@ -476,7 +478,244 @@ PyObject* store_wgrads(Args& args) {
   Py_RETURN_NONE;
 }
 
-// bind(name, address); setup(check, plan, sms, budget)
+// ------------------------------------------------------------------------------------------------------- batches of problems
+//
+// The descriptions of ops.ghost_norm_batch, wgrad_clip_batch, wgrad_clip_per_example_batch and functional.rows_sum_batch_, packed here: 4 us a
+// problem in Python.  Each takes the same list of problems and returns True, or False, having launched nothing, where an argument is
+// not of the plain form: the Python function then says what is wrong with it, or packs it itself.
+
+bool bf16_rows(const Tensor& t) { return t.defined() && t.scalar_type() == at::kBFloat16 && t.dim() == 2 && t.is_cuda(); }
+struct Declined {};
+void need(bool ok) {
+  if (!ok) throw Declined();
+}
+Tensor tensor_or_none(PyObject* o) {
+  need(o != nullptr);
+  if (o == Py_None) return Tensor();
+  need(THPVariable_Check(o));
+  return THPVariable_Unpack(o);
+}
+long long whole(PyObject* o) {
+  need(o != nullptr && PyLong_Check(o));
+  const long long v = PyLong_AsLongLong(o);
+  if (v == -1 && PyErr_Occurred()) throw PythonError();
+  return v;
+}
+long long splits(long long tiles, long long rows, long long most, bool peer) {
+  PyObject* r = PyObject_CallFunction(g_splits, "LLLi", tiles, rows, most, (int)peer);
+  if (r == nullptr) throw PythonError();
+  const long long v = PyLong_AsLongLong(r);
+  Py_DECREF(r);
+  return v;
+}
+struct Problems {
+  PyObject* seq;
+  explicit Problems(PyObject* o) : seq(o) { need(PyList_Check(o) || PyTuple_Check(o)); }
+  Py_ssize_t size() const { return PySequence_Fast_GET_SIZE(seq); }
+  PyObject* at(Py_ssize_t i) const { return PySequence_Fast_GET_ITEM(seq, i); }
+  // item i, a tuple of `n` values
+  PyObject* tuple(Py_ssize_t i, Py_ssize_t n) const {
+    PyObject* t = at(i);
+    need(PyTuple_Check(t) && PyTuple_GET_SIZE(t) == n);
+    return t;
+  }
+};
+Tensor field(PyObject* tuple, Py_ssize_t i) { return tensor_or_none(PyTuple_GET_ITEM(tuple, i)); }
+long long room(const Tensor& out) { return static_cast<long long>(out.storage().nbytes() / 4) - out.storage_offset(); }
+template <PyObject* (*F)(Args&)>
+PyObject* or_false(Args& a) {
+  try {
+    return F(a);
+  } catch (const Declined&) {
+    Py_RETURN_FALSE;
+  }
+}
+
+// (problems (a | None, g, norm2, tokens, ids | None, seg | None, seg_out | None), status)
+PyObject* ghost_batch(Args& args) {
+  const Problems ps(args.next());
+  const long long status = args.integer();
+  std::vector<ob_ghost_desc> d;
+  for (Py_ssize_t i = 0; i < ps.size(); ++i) {
+    PyObject* t = ps.tuple(i, 7);
+    const Tensor a = field(t, 0), g = field(t, 1), norm2 = field(t, 2), ids = field(t, 4), seg = field(t, 5), seg_out = field(t, 6);
+    const long long tokens = whole(PyTuple_GET_ITEM(t, 3));
+    need(bf16_rows(g) && norm2.defined() && tokens > 0);
+    ob_ghost_desc p = {};
+    p.total_rows = g.size(0);
+    if (seg.defined()) {
+      need(seg.scalar_type() == at::kInt && (!seg_out.defined() || (seg_out.scalar_type() == at::kInt && seg_out.numel() == seg.numel() - 1)));
+      p.B = static_cast<int>(seg.numel() - 1);
+    } else {
+      p.B = static_cast<int>(p.total_rows / tokens);
+      need(p.B * tokens == p.total_rows && norm2.numel() >= p.B);
+    }
+    if (ids.defined()) {
+      need(ids.scalar_type() == at::kInt && ids.numel() == p.total_rows);
+    } else {
+      need(bf16_rows(a) && a.size(0) == p.total_rows);
+      p.a = ptr(a);
+      p.lda = a.stride(0);
+      p.Da = static_cast<int>(a.size(1));
+    }
+    p.g = ptr(g);
+    p.ids = static_cast<const int*>(ptr(ids));
+    p.norm2 = static_cast<float*>(ptr(norm2));
+    p.seg = static_cast<const int*>(ptr(seg));
+    p.seg_out = static_cast<const int*>(ptr(seg_out));
+    p.ldg = g.stride(0);
+    p.T = static_cast<int>(tokens);
+    p.Dg = static_cast<int>(g.size(1));
+    d.push_back(p);
+  }
+  std::stable_sort(d.begin(), d.end(), [](const ob_ghost_desc& x, const ob_ghost_desc& y) { return x.Da + x.Dg > y.Da + y.Dg; });
+  LAUNCH(ob_ghost_norm_batch, d.data(), (int)d.size(), reinterpret_cast<int*>(status), g_budget, g_sms);
+  Py_RETURN_TRUE;
+}
+
+// (problems {a, b, row_scale, seg_offsets, num_groups, out_offset, ldm, group_stride}, out | None, peer_table | None, shard_elems, status):
+// accumulating, tiles of 256 columns
+PyObject* wgrad_batch(Args& args) {
+  const Problems ps(args.next());
+  const Tensor out = args.optional(), peers = args.optional();
+  const long long shard = args.integer(), status = args.integer();
+  need(out.defined() ? out.scalar_type() == at::kFloat : peers.defined() && shard > 0);
+  struct Job {
+    double key;
+    ob_wgrad_desc d;
+  };
+  std::vector<Job> jobs;
+  long long tiles = 0;
+  for (Py_ssize_t i = 0; i < ps.size(); ++i) {
+    PyObject* o = ps.at(i);
+    need(PyDict_Check(o));
+    Tensor a, b, scale, seg;
+    ob_wgrad_desc p = {};
+    p.num_groups = 1;
+    p.ldn = 1;
+    p.ldm = -1;
+    p.accumulate = 1;
+    PyObject *k, *v;
+    Py_ssize_t pos = 0;
+    while (PyDict_Next(o, &pos, &k, &v)) {
+      const char* name = PyUnicode_Check(k) ? PyUnicode_AsUTF8(k) : nullptr;
+      need(name != nullptr);
+      if (!strcmp(name, "a")) a = tensor_or_none(v);
+      else if (!strcmp(name, "b")) b = tensor_or_none(v);
+      else if (!strcmp(name, "row_scale")) scale = tensor_or_none(v);
+      else if (!strcmp(name, "seg_offsets")) seg = tensor_or_none(v);
+      else if (!strcmp(name, "num_groups")) p.num_groups = static_cast<int>(whole(v));
+      else if (!strcmp(name, "out_offset")) p.out_offset = whole(v);
+      else if (!strcmp(name, "ldm")) p.ldm = whole(v);
+      else if (!strcmp(name, "group_stride")) p.group_stride = whole(v);
+      else throw Declined();
+    }
+    need(bf16_rows(a) && bf16_rows(b) && a.size(0) == b.size(0) && a.stride(1) == 1 && b.stride(1) == 1);
+    p.a = ptr(a);
+    p.b = ptr(b);
+    p.row_scale = f32(scale);
+    p.seg_offsets = static_cast<const int*>(ptr(seg));
+    p.lda = a.stride(0);
+    p.ldb = b.stride(0);
+    p.T = static_cast<int>(a.size(0));
+    p.M = static_cast<int>(a.size(1));
+    p.N = static_cast<int>(b.size(1));
+    if (p.ldm == -1) p.ldm = p.N;
+    if (out.defined())
+      need(p.out_offset >= 0 && p.ldm >= 0 &&
+           p.out_offset + (p.num_groups - 1) * p.group_stride + (p.M - 1) * p.ldm + p.N - 1 < room(out));
+    tiles += static_cast<long long>(p.num_groups) * ((p.M + 127) / 128) * ((p.N + 255) / 256);
+    jobs.push_back({0.0, p});
+  }
+  for (Job& j : jobs) {
+    j.d.splits = j.d.num_groups == 1 ? static_cast<int>(splits(tiles, j.d.T, -1, peers.defined())) : 1;
+    j.key = static_cast<double>(j.d.T) / (static_cast<double>(j.d.num_groups) * j.d.splits);
+  }
+  std::stable_sort(jobs.begin(), jobs.end(), [](const Job& x, const Job& y) { return x.key > y.key; });
+  std::vector<ob_wgrad_desc> d;
+  for (const Job& j : jobs) d.push_back(j.d);
+  LAUNCH(ob_wgrad_clip_batch, d.data(), (int)d.size(), static_cast<float*>(ptr(out)), static_cast<float* const*>(ptr(peers)), shard, 256,
+         reinterpret_cast<int*>(status), g_budget, g_sms);
+  Py_RETURN_TRUE;
+}
+
+// (problems (a, b, ex_scale | None, out_offset, ldm), out | None, rows_per_example, peer_table | None, shard_elems, status)
+PyObject* wgrad_pe_batch(Args& args) {
+  const Problems ps(args.next());
+  const Tensor out = args.optional();
+  const long long rows = args.integer();
+  const Tensor peers = args.optional();
+  const long long shard = args.integer(), status = args.integer();
+  need(rows > 0 && (out.defined() ? out.scalar_type() == at::kFloat : peers.defined() && shard > 0));
+  std::vector<ob_wgrad_pe_desc> d;
+  long long tiles = 0;
+  for (Py_ssize_t i = 0; i < ps.size(); ++i) {
+    PyObject* t = ps.tuple(i, 5);
+    const Tensor a = field(t, 0), b = field(t, 1), scale = field(t, 2);
+    need(bf16_rows(a) && bf16_rows(b) && a.size(0) == b.size(0) && a.stride(1) == 1 && b.stride(1) == 1 && a.size(0) % rows == 0);
+    ob_wgrad_pe_desc p = {};
+    p.a = ptr(a);
+    p.b = ptr(b);
+    p.ex_scale = f32(scale);
+    p.lda = a.stride(0);
+    p.ldb = b.stride(0);
+    p.out_offset = whole(PyTuple_GET_ITEM(t, 3));
+    p.ldm = whole(PyTuple_GET_ITEM(t, 4));
+    p.num_examples = static_cast<int>(a.size(0) / rows);
+    p.ex_rows = static_cast<int>(rows);
+    p.M = static_cast<int>(a.size(1));
+    p.N = static_cast<int>(b.size(1));
+    p.accumulate = 1;
+    need(!scale.defined() || (scale.scalar_type() == at::kFloat && scale.numel() >= p.num_examples && scale.is_contiguous()));
+    if (out.defined()) need(p.out_offset >= 0 && p.ldm >= 0 && p.out_offset + (p.M - 1) * p.ldm + p.N - 1 < room(out));
+    tiles += static_cast<long long>((p.M + 127) / 128) * ((p.N + 255) / 256);
+    d.push_back(p);
+  }
+  for (ob_wgrad_pe_desc& p : d)
+    p.splits = static_cast<int>(splits(tiles, static_cast<long long>(p.num_examples) * rows, p.num_examples, peers.defined()));
+  LAUNCH(ob_wgrad_clip_pe_batch, d.data(), (int)d.size(), static_cast<float*>(ptr(out)), static_cast<float* const*>(ptr(peers)), shard,
+         reinterpret_cast<int*>(status), g_budget, g_sms);
+  Py_RETURN_TRUE;
+}
+
+// (jobs (out, g) or (out, g, x, mean | None, rstd, out_plain | None), examples), all of the same rows
+PyObject* sums_batch(Args& args) {
+  const Problems ps(args.next());
+  const long long examples = args.integer();
+  std::vector<ob_rowsum_desc> d;
+  long long rows = -1;
+  for (Py_ssize_t i = 0; i < ps.size(); ++i) {
+    PyObject* t = ps.at(i);
+    need(PyTuple_Check(t) && (PyTuple_GET_SIZE(t) == 2 || PyTuple_GET_SIZE(t) == 6));
+    const bool norm = PyTuple_GET_SIZE(t) == 6;
+    const Tensor out = field(t, 0), g = field(t, 1), x = norm ? field(t, 2) : Tensor(), mean = norm ? field(t, 3) : Tensor(),
+                 rstd = norm ? field(t, 4) : Tensor(), plain = norm ? field(t, 5) : Tensor();
+    need(bf16_rows(g) && (rows < 0 || g.size(0) == rows) && g.stride(1) == 1 && examples > 0 && g.size(0) % examples == 0);
+    rows = g.size(0);
+    for (const Tensor* o : {&out, &plain})
+      need((!o->defined() && o == &plain) || (o->defined() && o->scalar_type() == at::kFloat && o->dim() == 2 && o->size(0) == examples &&
+                                              o->size(1) == g.size(1) && o->stride(1) == 1));
+    need(!x.defined() || (bf16_rows(x) && x.sizes() == g.sizes() && x.stride(1) == 1 && x.stride(0) == g.stride(0)));
+    ob_rowsum_desc p = {};
+    p.g = ptr(g);
+    p.x = ptr(x);
+    p.mean = f32(mean);
+    p.rstd = f32(rstd);
+    p.out = static_cast<float*>(ptr(out));
+    p.out2 = static_cast<float*>(ptr(plain));
+    p.ldg = g.stride(0);
+    p.ld_out = out.stride(0);
+    p.ld_out2 = plain.defined() ? plain.stride(0) : 0;
+    p.N = static_cast<int>(g.size(1));
+    p.mode = !x.defined() ? 0 : (mean.defined() ? 1 : 2);
+    d.push_back(p);
+  }
+  need(!d.empty());
+  LAUNCH(ob_rows_sum_batch, d.data(), (int)d.size(), (int)examples, (int)(rows / examples));
+  Py_RETURN_TRUE;
+}
+
+// bind(name, address); setup(check, plan, splits, sms, budget)
 PyObject* bind(Args& a) {
   const char* name = PyUnicode_AsUTF8(a.next());
   if (name == nullptr) throw PythonError();
@@ -490,12 +729,14 @@ PyObject* bind(Args& a) {
   throw PythonError();
 }
 PyObject* setup(Args& a) {
-  PyObject *check = a.next(), *plan_fn = a.next();
+  PyObject *check = a.next(), *plan_fn = a.next(), *splits_fn = a.next();
   const long long sms = a.integer();
   g_budget = a.number();
   g_sms = static_cast<int>(sms);
   Py_XDECREF(g_check);
   Py_XDECREF(g_plan);
+  Py_XDECREF(g_splits);
+  g_splits = Py_NewRef(splits_fn);
   g_check = Py_NewRef(check);
   g_plan = Py_NewRef(plan_fn);
   const char* missing = nullptr;
@@ -516,8 +757,10 @@ PyObject* entries(Args&) {
 }
 
 #define METHOD(f) {#f, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(&call<f>)), METH_FASTCALL, nullptr}
+#define BATCH(f) {#f, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(&call<or_false<f>>)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {METHOD(gpt2_in), METHOD(gpt2_in_bwd), METHOD(gpt2_out), METHOD(gpt2_out_bwd), METHOD(lora_in), METHOD(lora_in_bwd),
-                         METHOD(lora_out), METHOD(lora_out_bwd), METHOD(store_wgrads), METHOD(bind), METHOD(setup), METHOD(entries),
+                         METHOD(lora_out), METHOD(lora_out_bwd), METHOD(store_wgrads), BATCH(ghost_batch), BATCH(wgrad_batch),
+                         BATCH(wgrad_pe_batch), BATCH(sums_batch), METHOD(bind), METHOD(setup), METHOD(entries),
                          {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_blocks", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

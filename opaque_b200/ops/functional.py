@@ -180,6 +180,10 @@ _ROWSUM_DESC = struct.Struct("6Q3q2i")
 def rows_sum_batch_(jobs, num_examples: int) -> None:
     """:func:`rows_group_sum_` for several matrices with the same number of rows in one launch (per 128): ``jobs`` are
     ``(out, g2d)`` (plain sums) or ``(out, g2d, x2d, mean | None, rstd, out_plain | None)``."""
+    from . import _native
+    native = _native("sums_batch")
+    if native is not None and native(jobs, num_examples):
+        return
     rows = jobs[0][1].shape[0]
     if rows % num_examples:
         raise ValueError("rows_sum_batch_: rows must be a multiple of examples")

@@ -148,7 +148,7 @@ def load() -> _Entries:
     return entries
 
 
-def load_block_steps(plan, budget: float):
+def load_block_steps(plan, splits, budget: float):
     """The extension of ``csrc/block_steps.cpp`` with the library's entry points bound, or ``None`` (with a warning) where it can neither
     be built nor loaded: the callers then run their operations one by one."""
     import importlib.util
@@ -161,7 +161,7 @@ def load_block_steps(plan, budget: float):
             spec.loader.exec_module(steps)
             for name in steps.entries().split():
                 steps.bind(name, ctypes.cast(getattr(entries._cdll, name), c_void_p).value)
-            steps.setup(check, plan, sm_count(), budget)
+            steps.setup(check, plan, splits, sm_count(), budget)
             return steps
         except (RuntimeError, OSError, ImportError) as exc:
             reason = exc

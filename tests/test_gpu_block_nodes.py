@@ -114,6 +114,41 @@ def test_without_the_compiled_sequences(monkeypatch):
     _close(one, two)
 
 
+@pytest.mark.parametrize("B,T", [(3, 77), (2, 256), (19, 250)])           # ragged and uniform weight gradients, sums apart and in the norms
+def test_packed_batches(B, T, monkeypatch):
+    """Norms, sums and weight gradients whose problems are packed by the extension or in Python."""
+    from opaque_b200 import ops
+    from opaque_b200.models import GPT2Config, GPT2LMHeadModel, shift_labels
+    torch.manual_seed(T)
+    model = GPT2LMHeadModel(GPT2Config.tiny(), device="cuda")
+    ids = torch.randint(0, 500, (B, T), device="cuda")
+    batch = {"input_ids": ids, "labels": shift_labels(ids)}
+    one, _ = _run(model, batch, "capture", True)
+    monkeypatch.setattr(ops, "block_steps", lambda: None)
+    two, _ = _run(model, batch, "capture", True)
+    _close(one, two)
+
+
+def test_batches_that_python_looks_at():
+    """Problems that the packers decline raise what they raised."""
+    from opaque_b200 import ops
+    a, out = torch.randn(64, 128, device="cuda", dtype=torch.bfloat16), torch.zeros(128 * 128, device="cuda")
+    steps = ops.block_steps()
+    assert steps.wgrad_batch([dict(a=a, b=a, out_offset=1)], out, None, 0, 0) is False and steps.ghost_batch([(a, a.float(), out, 8, None, None, None)], 0) is False
+    with pytest.raises(ValueError):
+        ops.wgrad_clip_batch([dict(a=a, b=a, out_offset=1)], out)
+    with pytest.raises(TypeError):
+        ops.ghost_norm_batch([(a, a.float(), out, 8, None, None, None)])
+    with pytest.raises(ValueError):
+        ops.wgrad_clip_per_example_batch([(a, a, None, 0, 128)], out, 63)
+    with pytest.raises(ValueError):
+        ops.functional.rows_sum_batch_([(out.view(128, 128)[:7], a)], 8)
+    assert float(out.abs().max()) == 0.0
+    ops.wgrad_clip_batch([dict(a=a, b=a)], out)
+    ref = a.double().t() @ a.double()
+    assert float((out.view(128, 128) - ref).norm()) <= 2 ** -20 * float(ref.norm())
+
+
 def test_errors_of_the_compiled_sequences():
     """Refused arguments and failed launches are Python exceptions."""
     from opaque_b200 import ops
