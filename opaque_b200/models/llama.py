@@ -223,7 +223,7 @@ class LlamaMLP(nn.Module):
         gp, up_ = self.gate_proj, self.up_proj
         if gp.lora_A is None and up_.lora_A is None and gp.bias is None and up_.bias is None:
             dp = self.down_proj
-            if dp.lora_A is None and dp.bias is None and passable(dp):
+            if torch.is_grad_enabled() and dp.lora_A is None and dp.bias is None and passable(dp):
                 # forward and backward as one function (the GLU backward rides in the down projection's data-gradient epilogue)
                 y = fused.glu_mlp(x, gp.weight, up_.weight, dp.weight, self.act)
                 if y is not None:
@@ -307,6 +307,8 @@ class LlamaDecoderLayer(nn.Module):
         plain causal attention with rotary positions, everything else frozen and without biases, on the library's kernels."""
         m = self._modules
         att, mlp = m["self_attn"], m["mlp"]
+        if att._modules["q_proj"].lora_A is None:        # first: most blocks end here
+            return False
         if type(att) is not LlamaAttention or type(mlp) is not LlamaMLP or not att.use_rope or att.q_norm is not None or att.sinks is not None \
                 or att.softcap or att.local_rope or (att.window is not None and x.shape[1] > att.window) or pos is not None \
                 or not isinstance(cos, torch.Tensor) or att.hd % 16 or layers._ADAPTERS_OFF or not fused.one_node_lora() or not blocks.available() \
