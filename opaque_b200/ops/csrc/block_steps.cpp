@@ -336,7 +336,7 @@ PyObject* gpt2_in_bwd(Args& a) {
 PyObject* gpt2_out(Args& a) {
   const Tensor o = a.tensor(), r = rows(a.tensor()), wo = a.tensor(), bo = a.tensor(), lw = a.tensor(), lb = a.tensor(), w1 = a.tensor(),
                b1 = a.tensor(), w2 = a.tensor(), b2 = a.tensor();
-  const Tensor o2 = vec16(o.transpose(1, 2).reshape({o.size(0) * o.size(2), -1}));
+  const Tensor o2 = vec16(o.transpose(1, 2).reshape({o.size(0) * o.size(2), o.size(1) * o.size(3)}));
   const Normed n = layer_norm(product(o2, wo, wo.size(0), false, with_bias(bo)), r, lw, lb, a.number());
   Tensor f;
   const Tensor h = product_gelu(n.y, w1, b1, a.integer() ? &f : nullptr);
@@ -395,7 +395,7 @@ PyObject* lora_out(Args& a) {
   const int act = static_cast<int>(a.integer());
   const Tensor wd = a.tensor();
   const bool keep = a.integer() != 0;
-  const Tensor o2 = vec16(o.transpose(1, 2).reshape({o.size(0) * o.size(2), -1})), xa = product(o2, la, la.size(0), false, scaled(scaling));
+  const Tensor o2 = vec16(o.transpose(1, 2).reshape({o.size(0) * o.size(2), o.size(1) * o.size(3)})), xa = product(o2, la, la.size(0), false, scaled(scaling));
   const Normed n = rms_norm(product(o2, wo, wo.size(0), false, segment(xa, lb, false)), r, nw, eps, offset, mode);
   const int64_t M = o2.size(0), I = wg.size(0), K = wg.size(1);
   const Tensor h = empty({M, I}, o2), g = keep ? empty({M, I}, o2) : Tensor(), u = keep ? empty({M, I}, o2) : Tensor();

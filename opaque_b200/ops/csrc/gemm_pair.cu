@@ -3,7 +3,7 @@
 //     D[M, N] = A[M, K1] * op1(B) + A2[M, K2] * op2(B2) + bias          (bf16 in / bf16 out, fp32 accumulation)
 //
 // Two CTAs of a 2x1 cluster share one 512 x 256 output tile.  Each CTA loads ITS OWN 256 rows of A and ITS OWN half
-// (128 columns of N) of the B tile with ordinary TMA copies of this GPU's memory; one thread of the leader CTA
+// (128 columns of N) of the B tile with ordinary TMA copies of this GPU's memory; one lane of the leader CTA
 // (cluster rank 0) issues `tcgen05.mma.cta_group::2` (M = 256 across the pair) over both CTAs' shared memory, twice per
 // k-step: once for each 128-row half of a CTA's A tile, each half with its own 256-column accumulator in that CTA's tensor
 // memory.  Per k-block an SM stages 48 KB for 2 x (128 x 256 x 64) of tensor work: half the bytes per FLOP of a single-CTA
