@@ -60,7 +60,7 @@ class GPT2In(Function):
         s, stats, y, ln_w, w = ctx.saved_tensors
         sums = _norm_sums(ctx.trainable, ctx.norm, s.shape[0])
         g, dy, dx = ops.block_steps().gpt2_in_bwd(dq, dk, dv, w, s, ln_w, stats, ds if ctx.carried else None,
-                                                  ctx.needs_input_grad[0] or ctx.trainable, *sums)
+                                                  ctx.needs_input_grad[0] or ctx.needs_input_grad[1] or ctx.trainable, *sums)
         dln = dlb = dw = db = None
         if ctx.trainable:
             dw, db = _weight_grads(fused.current_capture(), w, ctx.bias, y, g)

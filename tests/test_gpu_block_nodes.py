@@ -184,3 +184,19 @@ def test_blocks_that_keep_one_node_per_operation():
     a.self_attn.o_proj.__class__ = Other
     b.mlp.gate_proj.add_lora(8, 16.0)
     assert not a._two_nodes(x, model.rope_cos, model.rope_sin, None) and not b._two_nodes(x, model.rope_cos, model.rope_sin, None)
+
+
+def test_gradient_of_the_residual_alone():
+    """A frozen block whose ``x`` asks for no gradient while its residual does: the residual's is what it is with both."""
+    from opaque_b200.models import GPT2Config, GPT2LMHeadModel
+    torch.manual_seed(0)
+    block = GPT2LMHeadModel(GPT2Config.tiny(), device="cuda").requires_grad_(False).h[0]
+    x, r, gm, gs = (torch.randn(2, 64, 128, device="cuda", dtype=torch.bfloat16) for _ in range(4))
+    assert block._two_nodes(x)
+    grads = []
+    for both in (False, True):
+        rr = r.clone().requires_grad_(True)
+        m, s = block.forward_carried(x.clone().requires_grad_(both), rr)
+        torch.autograd.backward((m, s), (gm, gs))
+        grads.append(rr.grad)
+    _close([m, grads[0]], [m, grads[1]])
