@@ -24,6 +24,11 @@ def available() -> bool:
     return ops.PAIR_GEMM and ops.block_steps() is not None
 
 
+def one_stream(x, residual) -> bool:
+    """Whether the two parts of a split stream are of one kind; a node's kernels read both the same way."""
+    return residual is None or (residual.shape == x.shape and residual.dtype == x.dtype and residual.device == x.device)
+
+
 def _weight_grads(cap, weight, bias, x2d, g2d):
     """A trained linear's gradients: to the capture (returns ``(None, None)``), or summed where no capture is active."""
     if cap is None:

@@ -77,7 +77,7 @@ class GPT2Block(nn.Module):
     def forward_carried(self, x, residual):
         """The block on a split stream ``h = x + residual`` (``residual`` may be ``None``): every residual addition happens inside
         the next LayerNorm's kernel, and the two gradient branches meet in that kernel's backward.  Returns the pair."""
-        if self._two_nodes(x):
+        if blocks.one_stream(x, residual) and self._two_nodes(x):
             m, n1, n2 = self._modules, self.ln_1, self.ln_2
             wq, wo, w1, w2 = (m[k]._parameters for k in _PROJECTIONS)
             q, k, v, s = blocks.GPT2In.apply(x, residual, n1.weight, n1.bias, wq["weight"], wq["bias"], n1.eps, self.nh, n1)

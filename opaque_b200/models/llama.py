@@ -281,7 +281,7 @@ class LlamaDecoderLayer(nn.Module):
         inside the next norm kernel (forward), its two gradient branches only inside that kernel's backward.  Saves the
         four element-wise add launches per block that the plain form costs (two forward, two backward).
         Returns ``(mlp output, residual)``; the caller folds the last pair into the final norm."""
-        if self._two_nodes(x, cos, sin, pos):
+        if blocks.one_stream(x, residual) and self._two_nodes(x, cos, sin, pos):
             att, mlp, n1, n2 = self.self_attn, self.mlp, self.input_layernorm, self.post_attention_layernorm
             lq, lk, lv, lo = (att._modules[k]._parameters for k in _PROJECTIONS)
             w_all = fused.stacked_weight_view([lq["weight"], lk["weight"], lv["weight"]])

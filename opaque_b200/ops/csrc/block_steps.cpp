@@ -3,7 +3,8 @@
 // more than most kernels of a short batch run; here 3 to 4.
 //
 // The functions allocate their results and launch the library's kernels (bound by address, see api.h) on the current stream; they
-// keep nothing.  The callers (engine/blocks.py) have checked types, layouts and alignment.  A launch that fails raises through the
+// keep nothing.  The callers (models/gpt2.py, models/llama.py) have checked types, layouts and alignment, fit() checks here that the
+// operands belong together.  A launch that fails raises through the
 // Python check that the other entry points use; no C++ exception leaves a function.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
@@ -61,6 +62,13 @@ void launch(const char* what, F entry, A... args) {
 }
 #define LAUNCH(name, ...) launch(#name, p_##name, __VA_ARGS__)
 
+// The shape checks of the Python entry points: a ValueError before a kernel is given a size that an operand does not have.
+void fit(bool ok, const char* what) {
+  if (ok) return;
+  PyErr_SetString(PyExc_ValueError, what);
+  throw PythonError();
+}
+
 void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
 const float* f32(const Tensor& t) { return static_cast<const float*>(ptr(t)); }
 Tensor empty(std::initializer_list<int64_t> shape, const Tensor& like) { return at::empty(shape, like.options()); }
@@ -98,6 +106,9 @@ struct Opt {                                         // the optional parts of a 
 // a [M, K] times b ([N, K], or [K, N] with kn), as ops.gemm
 Tensor product(const Tensor& a, const Tensor& b, int64_t N, bool kn, const Opt& o = {}) {
   const int64_t M = a.size(0), K = a.size(1), K2 = o.a2.defined() ? o.a2.size(1) : 0;
+  fit(b.dim() == 2 && b.size(kn ? 0 : 1) == K && b.size(kn ? 1 : 0) == N, "inner dimensions differ");
+  fit(K2 == 0 || (o.a2.size(0) == M && o.b2.size(o.kn2 ? 0 : 1) == K2 && o.b2.size(o.kn2 ? 1 : 0) == N), "low-rank segment: a2 [M, r], b2 [N, r] (or [r, N])");
+  fit(!o.bias.defined() || o.bias.numel() == N, "bias must hold N contiguous values");
   Tensor out = empty({M, N}, a);
   const int width = plan(M, N, K, K2, o.single ? SINGLE : ANY);
   const int64_t lda2 = K2 ? o.a2.stride(0) : 0, ldb2 = K2 ? o.b2.stride(0) : 0;
@@ -113,12 +124,18 @@ Opt with_bias(const Tensor& bias) { Opt o; o.bias = bias; return o; }
 Opt scaled(double alpha) { Opt o; o.alpha = static_cast<float>(alpha); o.single = true; return o; }
 Opt segment(const Tensor& a2, const Tensor& b2, bool kn2) { Opt o; o.a2 = a2; o.b2 = b2; o.kn2 = kn2; return o; }
 
+void fit_norm(const Tensor& x, const Tensor& r, const Tensor& w) {
+  fit(w.numel() == x.size(1), "a norm's weight and bias hold one value per column");
+  fit(!r.defined() || r.sizes() == x.sizes(), "the two parts of the stream have one shape");
+}
 // s = x + r (s = x without r) and its norm; stats: mean and rstd [2, rows]
 struct Normed {
   Tensor y, s, stats;
 };
 Normed layer_norm(const Tensor& x, const Tensor& r, const Tensor& w, const Tensor& b, double eps) {
   const int64_t R = x.size(0);
+  fit_norm(x, r, w);
+  fit_norm(x, r, b);
   Normed n{empty({R, x.size(1)}, x), x, empty_f32({2, R}, x)};
   float* mean = n.stats.data_ptr<float>();
   if (!r.defined()) {
@@ -154,6 +171,7 @@ Tensor layer_norm_bwd(const Tensor& dy, const Tensor& s, const Tensor& w, const 
 }
 Normed rms_norm(const Tensor& x, const Tensor& r, const Tensor& w, double eps, double offset, int mode) {
   const int64_t R = x.size(0);
+  fit_norm(x, r, w);
   Normed n{empty({R, x.size(1)}, x), r.defined() ? empty({R, x.size(1)}, x) : x, empty_f32({R}, x)};
   LAUNCH(ob_rmsnorm_fwd, ptr(x), ptr(r), ptr(w), ptr(n.y), r.defined() ? ptr(n.s) : nullptr, n.stats.data_ptr<float>(), R, (int)x.size(1),
          (float)eps, (float)offset, mode);
@@ -179,6 +197,8 @@ Tensor product_gelu(const Tensor& x, const Tensor& b, const Tensor& bias, Tensor
     if (pre != nullptr) *pre = f;
     return gelu(f, Tensor());
   }
+  fit(b.size(1) == K, "inner dimensions differ");
+  fit(bias.numel() == N, "bias must hold N contiguous values");
   Tensor h = empty({M, N}, x);
   if (pre != nullptr) *pre = empty({M, N}, x);
   void* const f = pre != nullptr ? ptr(*pre) : nullptr;
@@ -193,6 +213,7 @@ Tensor product_gelu(const Tensor& x, const Tensor& b, const Tensor& bias, Tensor
 Tensor product_gelu_bwd(const Tensor& g, const Tensor& w, const Tensor& f) {
   const int64_t M = g.size(0), N = w.size(1), K = g.size(1);
   if (N % 64 != 0) return gelu(f, product(g, w, N, true));
+  fit(w.size(0) == K && f.size(0) == M && f.size(1) == N, "inner dimensions differ");
   Tensor df = empty({M, N}, g);
   if (plan(M, N, K, 0, ACTIVATION) == 0)
     LAUNCH(ob_gemm_pair_glu_bwd, ptr(g), ptr(w), ptr(f), nullptr, ptr(df), nullptr, M, (int)N, (int)K, g.stride(0), w.stride(0), N, N, 1, GELU_TANH,
@@ -363,6 +384,8 @@ PyObject* lora_in(Args& a) {
   const double scaling = a.number();
   const Tensor w_all = a.tensor(), cs = a.tensor(), sn = a.tensor();
   const int64_t nh = a.integer(), nkv = a.integer(), hd = a.integer(), rank = aq.size(0);
+  for (const Tensor* f : {&aq, &ak, &av}) fit(f->sizes() == aq.sizes() && f->size(1) == x.size(1), "LoRA factors A [r, in] of one rank");
+  for (const Tensor* f : {&bq, &bk, &bv}) fit(f->size(1) == rank, "LoRA factors B [out, r] of one rank");
   const Normed n = rms_norm(x, r, nw, eps, offset, mode);
   const Tensor a_cat = empty({3 * rank, aq.size(1)}, aq), b_block = empty({bq.size(0) + bk.size(0) + bv.size(0), 3 * rank}, aq);
   LAUNCH(ob_lora_pack, ptr(aq), ptr(ak), ptr(av), ptr(bq), ptr(bk), ptr(bv), ptr(a_cat), ptr(b_block), (int)rank, (int)aq.size(1), (int)bq.size(0),
@@ -398,6 +421,7 @@ PyObject* lora_out(Args& a) {
   const Tensor o2 = vec16(o.transpose(1, 2).reshape({o.size(0) * o.size(2), o.size(1) * o.size(3)})), xa = product(o2, la, la.size(0), false, scaled(scaling));
   const Normed n = rms_norm(product(o2, wo, wo.size(0), false, segment(xa, lb, false)), r, nw, eps, offset, mode);
   const int64_t M = o2.size(0), I = wg.size(0), K = wg.size(1);
+  fit(K == n.y.size(1) && wu.sizes() == wg.sizes(), "gate and up projections [I, K]");
   const Tensor h = empty({M, I}, o2), g = keep ? empty({M, I}, o2) : Tensor(), u = keep ? empty({M, I}, o2) : Tensor();
   LAUNCH(ob_gemm_pair, ptr(n.y), ptr(wg), ptr(wu), nullptr, nullptr, nullptr, nullptr, ptr(h), ptr(g), ptr(u), M, (int)(2 * I), (int)K, 0, K,
          wg.stride(0), 0, 0, I, 0, 0, 1, act, -1, nullptr, g_budget, g_sms);
@@ -414,6 +438,7 @@ PyObject* lora_out_bwd(Args& a) {
   const double scaling = a.number();
   const Tensor wo = a.tensor(), la = a.tensor();
   const int64_t M = g.size(0), I = g.size(1);
+  fit(d2.size(0) == M && wd.size(0) == d2.size(1) && wd.size(1) == I, "inner dimensions differ");
   Tensor dg = empty({M, I}, g), du = empty({M, I}, g);
   if (one_launch) {
     LAUNCH(ob_gemm_pair_glu_bwd, ptr(d2), ptr(wd), ptr(g), ptr(u), ptr(dg), ptr(du), M, (int)I, (int)d2.size(1), d2.stride(0), wd.stride(0), I, I, 1,

@@ -200,3 +200,50 @@ def test_gradient_of_the_residual_alone():
         torch.autograd.backward((m, s), (gm, gs))
         grads.append(rr.grad)
     _close([m, grads[0]], [m, grads[1]])
+
+
+def _smaller(module, name, *shape):
+    p = getattr(module, name)
+    setattr(module, name, torch.nn.Parameter(torch.zeros(*shape, device="cuda", dtype=torch.bfloat16), requires_grad=p.requires_grad))
+
+
+def test_operands_that_do_not_fit_together():
+    """A parameter of another size is a ``ValueError`` of the product or norm that meets it, in a block that runs as two nodes."""
+    from opaque_b200.models import GPT2Config, GPT2LMHeadModel, LlamaConfig, LlamaForCausalLM
+    x = torch.randn(1, 8, 128, device="cuda", dtype=torch.bfloat16)
+    for path, name, shape in (("attn_c_attn", "weight", (384, 64)), ("attn_c_attn", "bias", (376,)), ("attn_c_proj", "weight", (128, 64)),
+                              ("mlp_c_fc", "weight", (512, 64)), ("mlp_c_fc", "bias", (504,)), ("mlp_c_proj", "weight", (128, 448)),
+                              ("mlp_c_proj", "weight", (120, 512)), ("ln_1", "weight", (120,)), ("ln_1", "bias", (120,)), ("ln_2", "bias", (8,))):
+        block = GPT2LMHeadModel(GPT2Config.tiny(), device="cuda").requires_grad_(False).h[0]
+        _smaller(getattr(block, path), name, *shape)
+        assert block._two_nodes(x)
+        with pytest.raises(ValueError):
+            block.forward_carried(x, x)
+    for path, name, shape in (("self_attn.q_proj", "lora_A", (8, 64)), ("self_attn.k_proj", "lora_A", (8, 64)), ("self_attn.v_proj", "lora_B", (64, 16)),
+                              ("self_attn.o_proj", "lora_A", (8, 64)), ("self_attn.o_proj", "lora_B", (128, 16)), ("self_attn.o_proj", "weight", (128, 64)),
+                              ("input_layernorm", "weight", (64,)), ("post_attention_layernorm", "weight", (64,))):
+        model = LlamaForCausalLM(LlamaConfig.tiny(), device="cuda")
+        model.add_lora(8, 16.0)
+        layer = model.model.layers[0]
+        _smaller(layer.get_submodule(path), name, *shape)
+        args = (model.rope_cos, model.rope_sin, None)
+        assert layer._two_nodes(x, *args)
+        with pytest.raises(ValueError):
+            layer.forward_carried(x, x, *args)
+
+
+def test_streams_of_two_kinds_keep_one_node_per_operation():
+    """A residual of another type or of a shape that only broadcasts is added as it was before blocks ran as two nodes."""
+    from opaque_b200.models import GPT2Config, GPT2LMHeadModel, LlamaConfig, LlamaForCausalLM
+    torch.manual_seed(0)
+    x = torch.randn(2, 8, 128, device="cuda", dtype=torch.bfloat16)
+    block = GPT2LMHeadModel(GPT2Config.tiny(), device="cuda").requires_grad_(False).h[0]
+    model = LlamaForCausalLM(LlamaConfig.tiny(), device="cuda")
+    model.add_lora(8, 16.0)
+    with torch.no_grad():
+        r = torch.randn(1, 8, 128, device="cuda", dtype=torch.bfloat16)
+        got, want = block.forward_carried(x, r), block.forward_carried(x, r.expand(2, 8, 128).contiguous())
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+        args = (model.rope_cos, model.rope_sin, None)
+        got, want = model.model.layers[0].forward_carried(x, x.float(), *args), model.model.layers[0].forward_carried(x, x.clone(), *args)
+        assert torch.equal(got[1], want[1]) and float((got[0] - want[0]).norm()) <= 2 ** -8 * float(want[0].norm())
