@@ -91,7 +91,7 @@ class GPT2Block(nn.Module):
     def _two_nodes(self, x) -> bool:
         """Whether the block may run as two autograd nodes around the attention (``engine/blocks.py``): plain projections with biases on
         the library's products, and its parameters all frozen, or all trained under a capture."""
-        if GPT2Block._attention is not _BLOCK_PARTS[0] or GPT2Block._mlp is not _BLOCK_PARTS[1] or "_attention" in self.__dict__ \
+        if type(self)._attention is not _BLOCK_PARTS[0] or type(self)._mlp is not _BLOCK_PARTS[1] or "_attention" in self.__dict__ \
                 or "_mlp" in self.__dict__ or not blocks.available():
             return False
         m = self._modules

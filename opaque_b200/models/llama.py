@@ -306,19 +306,24 @@ class LlamaDecoderLayer(nn.Module):
         """Whether the block may run as two autograd nodes around the attention (``engine/blocks.py``): LoRA on all four projections of a
         plain causal attention with rotary positions, everything else frozen and without biases, on the library's kernels."""
         m = self._modules
-        att, mlp = m["self_attn"], m["mlp"]
-        if att._modules["q_proj"].lora_A is None:        # first: most blocks end here
+        att, mlp = m.get("self_attn"), m.get("mlp")
+        if type(att) is not LlamaAttention or type(mlp) is not LlamaMLP:         # other modules need not have these projections
             return False
-        if type(att) is not LlamaAttention or type(mlp) is not LlamaMLP or not att.use_rope or att.q_norm is not None or att.sinks is not None \
+        q = att._modules.get("q_proj")
+        if type(q) is not Linear or q.lora_A is None:    # most blocks end here
+            return False
+        if not att.use_rope or att.q_norm is not None or att.sinks is not None \
                 or att.softcap or att.local_rope or (att.window is not None and x.shape[1] > att.window) or pos is not None \
                 or not isinstance(cos, torch.Tensor) or att.hd % 16 or layers._ADAPTERS_OFF or not fused.one_node_lora() or not blocks.available() \
                 or any(t.dtype != torch.float32 or not t.is_contiguous() or t.data_ptr() & 15 for t in (cos, sin)):
             return False
+        if not passable(self, att, mlp):
+            return False
         norms = m["input_layernorm"], m["post_attention_layernorm"]
         adapted, plain = [att._modules[k] for k in _PROJECTIONS], [mlp._modules[k] for k in ("gate_proj", "up_proj", "down_proj")]
-        if not passable(self, att, mlp, *norms, *adapted, *plain):
+        if not passable(*norms, *adapted, *plain):
             return False
-        r, scaling = adapted[0].lora_A.shape[0] if adapted[0].lora_A is not None else 0, adapted[0].scaling
+        r, scaling = q.lora_A.shape[0], q.scaling
         for i, lin in enumerate(adapted):
             w, a, b = lin._parameters["weight"], lin.lora_A, lin.lora_B
             if a is None or lin.bias is not None or w.requires_grad or not fused.lora_factors_ok(a, b) or not w.is_contiguous() \

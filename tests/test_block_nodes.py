@@ -1,0 +1,63 @@
+"""Which decoder blocks may run as two autograd nodes (engine/blocks.py): blocks with other modules in place of their own may not.
+The kernels are not asked for here, so these run without a GPU."""
+import pytest
+import torch
+from torch import nn
+
+from opaque_b200.engine import blocks, fused
+from opaque_b200.models import GPT2Config, GPT2LMHeadModel, LlamaConfig, LlamaForCausalLM
+from opaque_b200.models.gpt2 import GPT2Block
+
+
+@pytest.fixture(autouse=True)
+def _as_on_a_gpu(monkeypatch):
+    monkeypatch.setattr(blocks, "available", lambda: True)
+    monkeypatch.setattr(fused, "_own_gemm_ok", lambda *a: True)
+
+
+def _layer():
+    model = LlamaForCausalLM(LlamaConfig.tiny())
+    model.add_lora(8, 16.0)
+    layer = model.model.layers[0]
+    return layer, lambda: layer._two_nodes(torch.zeros(1, 8, 128, dtype=torch.bfloat16), model.rope_cos, model.rope_sin, None)
+
+
+class _Other(nn.Module):
+    def forward(self, x, *args):
+        return x
+
+
+def test_llama_blocks_with_other_modules():
+    layer, two_nodes = _layer()
+    assert two_nodes()
+    for part in ("self_attn", "mlp"):
+        own = getattr(layer, part)
+        for other in (torch.compile(own), _Other()):
+            setattr(layer, part, other)
+            assert not two_nodes()
+        setattr(layer, part, own)
+    att, own = layer.self_attn, layer.self_attn.q_proj
+    for other in (nn.Linear(128, 128), torch.compile(own)):
+        att.q_proj = other
+        assert not two_nodes()
+    att.q_proj = own
+    assert two_nodes()
+
+
+def test_llama_attention_patched_as_a_class(monkeypatch):
+    """The patched forward may need none of the projections."""
+    layer, two_nodes = _layer()
+    monkeypatch.setattr(type(layer.self_attn), "forward", lambda self, x, *a: x)
+    del layer.self_attn.k_proj
+    assert not two_nodes()
+
+
+def test_gpt2_blocks_that_override_a_part():
+    class Block(GPT2Block):
+        def _attention(self, y):
+            return y
+    block = GPT2LMHeadModel(GPT2Config.tiny()).requires_grad_(False).h[0]
+    x = torch.zeros(1, 8, 128, dtype=torch.bfloat16)
+    assert block._two_nodes(x)
+    block.__class__ = Block
+    assert not block._two_nodes(x)
