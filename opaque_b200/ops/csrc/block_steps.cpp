@@ -11,6 +11,7 @@
 
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <algorithm>
@@ -325,8 +326,8 @@ PyObject* call(PyObject*, PyObject* const* a, Py_ssize_t n) {
   try {
     return F(args);
   } catch (const PythonError&) {
-  } catch (const std::exception& e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what());
+  } catch (const std::exception&) {                 // of the type that torch's own calls raise: torch.OutOfMemoryError, IndexError, ...
+    torch::translate_exception_to_python(std::current_exception());
   } catch (...) {
     PyErr_SetString(PyExc_RuntimeError, "unknown C++ exception");
   }

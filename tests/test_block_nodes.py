@@ -61,3 +61,15 @@ def test_gpt2_blocks_that_override_a_part():
     assert block._two_nodes(x)
     block.__class__ = Block
     assert not block._two_nodes(x)
+
+
+def test_exceptions_of_the_compiled_sequences_keep_their_type():
+    """What torch's own call raises in Python: an IndexError here, as torch.OutOfMemoryError where an allocation fails."""
+    import importlib.util
+
+    from opaque_b200.utils import build
+    spec = importlib.util.spec_from_file_location("opaque_b200.ops._blocks", build.build_block_steps())
+    steps = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(steps)
+    with pytest.raises(IndexError):
+        steps.gpt2_in(torch.zeros(()), None, torch.zeros(1), torch.zeros(1), torch.zeros(1, 1), torch.zeros(1), 1e-5)

@@ -247,3 +247,22 @@ def test_streams_of_two_kinds_keep_one_node_per_operation():
         args = (model.rope_cos, model.rope_sin, None)
         got, want = model.model.layers[0].forward_carried(x, x.float(), *args), model.model.layers[0].forward_carried(x, x.clone(), *args)
         assert torch.equal(got[1], want[1]) and float((got[0] - want[0]).norm()) <= 2 ** -8 * float(want[0].norm())
+
+
+def test_allocations_that_fail():
+    """A sequence that finds no memory raises what torch's allocations raise, and the next call works."""
+    from opaque_b200 import ops
+    steps, kept = ops.block_steps(), []
+    x, w = torch.zeros(1 << 18, 128, device="cuda", dtype=torch.bfloat16), torch.ones(128, device="cuda", dtype=torch.bfloat16)
+    proj = torch.zeros(128, 128, device="cuda", dtype=torch.bfloat16)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    # results of 64 MB each, in what is left of the blocks that this process holds
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + 1) / torch.cuda.get_device_properties(0).total_memory)
+    try:
+        with pytest.raises(torch.OutOfMemoryError):
+            for _ in range(32):
+                kept.append(steps.gpt2_in(x, None, w, w, proj, w, 1e-5))
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert steps.gpt2_in(x, None, w, w, proj, w, 1e-5)[3].shape == x.shape
