@@ -56,19 +56,19 @@ class GPT2In(Function):
         B, T, d = x.shape
         y, s, stats, qkv = ops.block_steps().gpt2_in(x, residual, ln_w, ln_b, w, b, eps)
         ctx.trainable, ctx.norm, ctx.bias, ctx.carried = w.requires_grad, norm, b, residual is not None
-        ctx.save_for_backward(s, stats, y, ln_w, w)
+        ctx.save_for_backward(s, stats, ln_w, w, *((y,) if ctx.trainable else ()))
         q, k, v = qkv.view(B, T, 3, heads, d // heads).permute(2, 0, 3, 1, 4).unbind(0)
         return q, k, v, None if residual is None else s.view(x.shape)
 
     @staticmethod
     def backward(ctx, dq, dk, dv, ds):
-        s, stats, y, ln_w, w = ctx.saved_tensors
+        s, stats, ln_w, w, *trained = ctx.saved_tensors
         sums = _norm_sums(ctx.trainable, ctx.norm, s.shape[0])
         g, dy, dx = ops.block_steps().gpt2_in_bwd(dq, dk, dv, w, s, ln_w, stats, ds if ctx.carried else None,
                                                   ctx.needs_input_grad[0] or ctx.needs_input_grad[1] or ctx.trainable, *sums)
         dln = dlb = dw = db = None
         if ctx.trainable:
-            dw, db = _weight_grads(fused.current_capture(), w, ctx.bias, y, g)
+            dw, db = _weight_grads(fused.current_capture(), w, ctx.bias, *trained, g)
             if sums[0] is None:
                 dln, dlb = _layer_norm_param_grads(dy, s, ln_w, stats, ctx.norm, True)
         if dx is not None:

@@ -266,3 +266,29 @@ def test_allocations_that_fail():
     finally:
         torch.cuda.set_per_process_memory_fraction(1.0)
     assert steps.gpt2_in(x, None, w, w, proj, w, 1e-5)[3].shape == x.shape
+
+
+@pytest.mark.parametrize("family", ["gpt2", "llama"])
+def test_memory_kept_for_the_backward_pass(family):
+    """A block with frozen weights keeps no more as two nodes than with one node per operation."""
+    from opaque_b200.models import GPT2Config, GPT2LMHeadModel, LlamaConfig, LlamaForCausalLM
+    if family == "gpt2":
+        block, args = GPT2LMHeadModel(GPT2Config.tiny(), device="cuda").requires_grad_(False).h[0], ()
+        part = block.mlp_c_fc
+    else:
+        model = LlamaForCausalLM(LlamaConfig.tiny(), device="cuda")
+        model.add_lora(8, 16.0)
+        block, args = model.model.layers[0], (model.rope_cos, model.rope_sin, None)
+        part = block.mlp.down_proj
+    held = []
+    for unsplit in (False, True):
+        hook = part.register_forward_hook(lambda *a: None) if unsplit else None
+        x, r = (torch.randn(2, 64, 128, device="cuda", dtype=torch.bfloat16, requires_grad=True) for _ in range(2))
+        kept = {}
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: kept.setdefault(t.untyped_storage().data_ptr(), t), lambda t: t):
+            out = block.forward_carried(x, r, *args)
+        held.append(sum(t.untyped_storage().nbytes() for t in kept.values()))
+        del out
+        if hook is not None:
+            hook.remove()
+    assert held[0] <= held[1]
