@@ -40,9 +40,13 @@ def _weight_grads(cap, weight, bias, x2d, g2d):
 
 def _norm_sums(trainable, norm, rows):
     """Where the backward kernel of a trained LayerNorm adds its per-example gradients (weight, bias), or ``(None, None)`` where they are
-    summed apart: few rows, whose sums share a launch with the other layers', or no capture."""
+    summed apart: no capture; few rows, whose sums share a launch with the other layers'; or fewer examples than one per 256 columns.
+
+    The kernel has at most 16 blocks per example (each is one more rounding of the example's sum), which for few long examples is too few
+    for the chip, the sooner the wider the rows (us, apart / by the kernel: 8192 rows of 768 as 1, 2 and 4 examples 55 / 84, 36 / 45 and
+    27 / 25, of 1024 65 / 124, 45 / 66 and 35 / 36; of 512 as 1 and 2 51 / 58 and 32 / 32; of 256 as 1 45 / 41)."""
     cap = fused.current_capture() if trainable else None
-    if cap is None or cap.sums_wait(rows, norm.weight.shape[0]) or rows % cap.batch_size:
+    if cap is None or cap.sums_wait(rows, norm.weight.shape[0]) or rows % cap.batch_size or norm.weight.shape[0] > 256 * cap.batch_size:
         return None, None
     return cap.pe_view(norm.weight), cap.pe_view(norm.bias)
 

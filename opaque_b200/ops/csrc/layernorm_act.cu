@@ -478,9 +478,9 @@ add_layernorm_fwd_walk_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bf
 // layernorm_bwd_dx_warp_kernel with the per-example weight and bias sums (rows_group_sum_kernel's mode 1) of the same rows: dy and x are
 // read once for both.  grid = examples x chunks of an example's rows; a warp walks over its chunk with its columns' sums in
 // registers, the block adds its warps' up and adds them to the example's row with atomics.
-// Bound by memory.  Measured with the operands in memory (hot in L2), against layernorm_bwd_dx_warp_kernel and rows_group_sum_kernel: 32 x 512
-// rows of 768 48.1 -> 30.7 us (34.3 -> 22.1), 8 x 1024 31.7 -> 20.5 (18.0 -> 14.3), 16 x 1024 rows of 1024 68.6 -> 47.1 (52.7 -> 41.3);
-// the copy rate allows 15.4, 7.7 and 20.5.  The sums' error against 64 bits is no larger (7.0e-8 and 7.3e-8 of their size).
+// Bound by memory.  Measured in rotation over 300 MB of operands, against the data gradient's kernel and rows_group_sum_kernel: 32 x 512
+// rows of 768 37.8 -> 23.9 us, 8 x 1024 22.3 -> 15.7, 16 x 1024 rows of 1024 55.6 -> 34.9; the copy rate allows 15.4, 7.7 and 20.5.
+// The sums' error against 64 bits is no larger (7.0e-8 and 7.3e-8 of their size).  Which calls come here: _norm_sums in engine/blocks.py.
 template <int VPL, bool RES>
 __global__ void __launch_bounds__(32 * LN_WARPS, 2)
 layernorm_bwd_sums_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
@@ -829,10 +829,17 @@ static int layernorm_bwd_sums(const __nv_bfloat16* dy, const __nv_bfloat16* x, c
   if (configured != cudaSuccess) return -22;
   // two blocks per SM where there are rows for them, at least a row per warp; 16 chunks at most, as rows_group_sum_kernel has: every
   // chunk is one more rounding of the example's sum (300 chunks: 2.4e-7 of the sum's size against 1.1e-7)
-  long long chunks = 2LL * ln_sms() / examples;
+  const long long sms = ln_sms();
+  long long chunks = 2 * sms / examples;
   if (chunks > 16) chunks = 16;
   if (chunks > (rows_per_example + LN_WARPS - 1) / LN_WARPS) chunks = (rows_per_example + LN_WARPS - 1) / LN_WARPS;
   if (chunks < 1) chunks = 1;
+  // A few blocks too many share their SMs (half as long again where two fit), or are a second wave (above 768 columns with a residual,
+  // where one fits): one block per SM with longer chunks where that is shorter.  10 examples of 1024 rows, us: 1024 columns 39.9 -> 25.5
+  // with a residual, 29.2 -> 22.0 without, 768 columns 24.1 -> 18.0
+  const long long one = sms / examples;
+  const long long halves = 2 * ring <= 224 * 1024 ? 3 : 2 * ((examples * chunks + sms - 1) / sms);
+  if (one >= 1 && one < chunks && halves * one > 2 * chunks) chunks = one;
   layernorm_bwd_sums_kernel<VPL, RES><<<static_cast<unsigned>(examples * chunks), 32 * LN_WARPS, ring, st>>>(
       dy, x, w, mean, rstd, ds, dx, rows_per_example, static_cast<int>(chunks), H, out_w, out_b, ld_out);
   return cudaGetLastError() == cudaSuccess ? 0 : -21;

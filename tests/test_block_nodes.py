@@ -73,3 +73,19 @@ def test_exceptions_of_the_compiled_sequences_keep_their_type():
     spec.loader.exec_module(steps)
     with pytest.raises(IndexError):
         steps.gpt2_in(torch.zeros(()), None, torch.zeros(1), torch.zeros(1), torch.zeros(1, 1), torch.zeros(1), 1e-5)
+
+
+@pytest.mark.parametrize("examples,rows,width,in_kernel", [(1, 8192, 768, False), (2, 8192, 768, False), (3, 8193, 768, True), (3, 8193, 1024, False),
+                                                           (4, 8192, 1024, True), (1, 8192, 256, True), (5, 5000, 768, True), (32, 4096, 768, False),
+                                                           (3, 8192, 768, False)])
+def test_norm_sums_of_few_long_examples_are_apart(monkeypatch, examples, rows, width, in_kernel):
+    """The kernel that adds a norm's sums has at most 16 blocks per example; the last two: few rows, and rows that are no multiple."""
+    class Capture:
+        batch_size, sums_wait = examples, staticmethod(fused.Capture.sums_wait)
+
+        def pe_view(self, p):
+            return torch.zeros(examples, width)
+    monkeypatch.setattr(fused, "_ACTIVE", Capture())
+    sums = blocks._norm_sums(True, nn.LayerNorm(width), rows)
+    assert (sums[0] is not None) == in_kernel == (sums[1] is not None)
+    assert blocks._norm_sums(False, nn.LayerNorm(width), rows) == (None, None)

@@ -192,6 +192,13 @@ def test_layer_norm_backward_with_sums(E, T, H, residual):
     assert torch.all(pe[:, 2 * H:] == 1) and float((pe[:, :2 * H].double() - 1 - ref).norm()) <= 2 ** -23 * (T ** 0.5 + 2) * float((1 + ref.abs()).norm())
 
 
+# where 16 chunks per example are a few blocks more than SMs: one block per SM with longer chunks instead, down to the last row
+@pytest.mark.parametrize("E,T,H", [(10, 129, 256), (12, 140, 768), (10, 1024, 776), (16, 131, 1024), (74, 60, 1024)])
+@pytest.mark.parametrize("residual", [True, False])
+def test_layer_norm_backward_with_sums_in_one_wave(E, T, H, residual):
+    test_layer_norm_backward_with_sums(E, T, H, residual)
+
+
 @pytest.mark.parametrize("rows,H", [(4737, 520), (4800, 768), (9473, 776), (5000, 1024)])
 def test_add_layer_norm_of_many_rows(rows, H):
     """Rows that come through the ring: against the fp32 statement, and the bits that the same rows have in a short call."""
