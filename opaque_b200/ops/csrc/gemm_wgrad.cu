@@ -543,11 +543,11 @@ wgrad_clip_pe_kernel(const __grid_constant__ TmaBatch<WgradPeParams, CAP> b) {
 #pragma unroll
           for (int j = 0; j < WP_BLOCK_N / 64; ++j)
             tma_load_3d(b_dst + j * (WG_BLOCK_K * 128), &b.map_b[cur], &full[stage], n0 + 64 * j, row, ex);
-          row += WG_BLOCK_K;
-          if (row >= kpe * WG_BLOCK_K) {
-            row = 0;
-            ++ex;
-          }
+        }
+        row += WG_BLOCK_K;
+        if (row >= kpe * WG_BLOCK_K) {
+          row = 0;
+          ++ex;
         }
         issued_mask |= 1u << stage;
         issued_phase = (issued_phase & ~(1u << stage)) | (phase << stage);

@@ -40,3 +40,23 @@ def test_command_line_reports_and_returns_nonzero(tmp_path, capsys):
     assert "bad.cu:2: [unbounded-spin]" in out and "1 finding(s)" in out
     (tmp_path / "bad.cu").write_text("__global__ void k(int* f) { f[0] = 1; }\n")
     assert R.main([str(tmp_path)]) == 0
+
+
+def test_elected_lanes_change_nothing_that_outlives_the_election():
+    """Where one lane issues for its warp (``if (elect_one())``), what the next step depends on advances outside, in all lanes."""
+    import pathlib
+    import re
+    csrc = pathlib.Path(R.__file__).parent.parent / "ops" / "csrc"
+    blocks = 0
+    for path in sorted(csrc.glob("*.cu")):
+        lines = path.read_text().splitlines()
+        for n, line in enumerate(lines):
+            if not re.search(r"\bif \(elect_one\(\)\) \{", line):
+                continue
+            blocks += 1
+            indent = len(line) - len(line.lstrip())
+            for m in range(n + 1, len(lines)):
+                if lines[m].startswith(" " * indent + "}"):
+                    break
+                assert not re.match(r"\s*(\+\+|--)?\w+\s*(\+\+|--|[-+|^&]?=[^=]).*;|\s*(\+\+|--)\w+;", lines[m]), f"{path.name}:{m + 1}: {lines[m]}"
+    assert blocks >= 8
