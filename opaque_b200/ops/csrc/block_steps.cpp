@@ -619,8 +619,8 @@ PyObject* wgrad_batch(Args& args) {
     ob_wgrad_desc p = {};
     p.num_groups = 1;
     p.ldn = 1;
-    p.ldm = -1;
     p.accumulate = 1;
+    bool pitch = false;                              // given by the caller
     PyObject *k, *v;
     Py_ssize_t pos = 0;
     while (PyDict_Next(o, &pos, &k, &v)) {
@@ -632,7 +632,7 @@ PyObject* wgrad_batch(Args& args) {
       else if (!strcmp(name, "seg_offsets")) seg = tensor_or_none(v);
       else if (!strcmp(name, "num_groups")) p.num_groups = static_cast<int>(whole(v));
       else if (!strcmp(name, "out_offset")) p.out_offset = whole(v);
-      else if (!strcmp(name, "ldm")) p.ldm = whole(v);
+      else if (!strcmp(name, "ldm")) p.ldm = whole(v), pitch = true;
       else if (!strcmp(name, "group_stride")) p.group_stride = whole(v);
       else throw Declined();
     }
@@ -646,7 +646,8 @@ PyObject* wgrad_batch(Args& args) {
     p.T = static_cast<int>(a.size(0));
     p.M = static_cast<int>(a.size(1));
     p.N = static_cast<int>(b.size(1));
-    if (p.ldm == -1) p.ldm = p.N;
+    if (!pitch) p.ldm = p.N;
+    need(p.num_groups >= 1);
     if (out.defined())
       need(p.out_offset >= 0 && p.ldm >= 0 &&
            p.out_offset + (p.num_groups - 1) * p.group_stride + (p.M - 1) * p.ldm + p.N - 1 < room(out));

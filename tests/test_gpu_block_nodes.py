@@ -292,3 +292,14 @@ def test_memory_kept_for_the_backward_pass(family):
         if hook is not None:
             hook.remove()
     assert held[0] <= held[1]
+
+
+def test_pitches_and_groups_that_are_refused():
+    """A negative pitch is no pitch left out, and no group is no problem: refused by the packer and by the Python form alike."""
+    from opaque_b200 import ops
+    a, out = torch.ones(64, 128, device="cuda", dtype=torch.bfloat16), torch.zeros(128 * 128, device="cuda")
+    for bad, error in ((dict(ldm=-1), ValueError), (dict(num_groups=0), (ValueError, ZeroDivisionError))):
+        assert ops.block_steps().wgrad_batch([dict(a=a, b=a, **bad)], out, None, 0, 0) is False
+        with pytest.raises(error):
+            ops.wgrad_clip_batch([dict(a=a, b=a, **bad)], out)
+    assert float(out.abs().max()) == 0.0
