@@ -59,7 +59,7 @@ class GPT2In(Function):
     def forward(ctx, x, residual, ln_w, ln_b, w, b, eps, heads, norm):
         B, T, d = x.shape
         y, s, stats, qkv = ops.block_steps().gpt2_in(x, residual, ln_w, ln_b, w, b, eps)
-        ctx.trainable, ctx.norm, ctx.bias, ctx.carried = w.requires_grad, norm, b, residual is not None
+        ctx.trainable, ctx.norm, ctx.linear, ctx.carried = w.requires_grad, norm, (w, b), residual is not None
         ctx.save_for_backward(s, stats, ln_w, w, *((y,) if ctx.trainable else ()))
         q, k, v = qkv.view(B, T, 3, heads, d // heads).permute(2, 0, 3, 1, 4).unbind(0)
         return q, k, v, None if residual is None else s.view(x.shape)
@@ -72,7 +72,7 @@ class GPT2In(Function):
                                                   ctx.needs_input_grad[0] or ctx.needs_input_grad[1] or ctx.trainable, *sums)
         dln = dlb = dw = db = None
         if ctx.trainable:
-            dw, db = _weight_grads(fused.current_capture(), w, ctx.bias, *trained, g)
+            dw, db = _weight_grads(fused.current_capture(), *ctx.linear, *trained, g)
             if sums[0] is None:
                 dln, dlb = _layer_norm_param_grads(dy, s, ln_w, stats, ctx.norm, True)
         if dx is not None:
@@ -87,24 +87,24 @@ class GPT2Out(Function):
     @staticmethod
     def forward(ctx, o, residual, wo, bo, ln_w, ln_b, w1, b1, w2, b2, eps, norm, keep):
         o2, y, s, stats, f, h, m = ops.block_steps().gpt2_out(o, residual, wo, bo, ln_w, ln_b, w1, b1, w2, b2, eps, keep)
-        ctx.trainable, ctx.norm, ctx.biases, ctx.dims = w1.requires_grad, norm, (bo, b1, b2), (o.shape[0], o.shape[2], o.shape[1], o.shape[3])
+        ctx.trainable, ctx.norm, ctx.linears, ctx.dims = w1.requires_grad, norm, ((wo, bo), (w1, b1), (w2, b2)), (o.shape[0], o.shape[2], o.shape[1], o.shape[3])
         if keep:
             ctx.save_for_backward(s, stats, f, ln_w, wo, w1, w2, *((o2, y, h) if ctx.trainable else ()))
         return m.view(residual.shape), s.view(residual.shape)
 
     @staticmethod
     def backward(ctx, dm, ds):
-        s, stats, f, ln_w, wo, w1, w2 = ctx.saved_tensors[:7]
+        s, stats, f, ln_w, wo, w1, w2, *trained = ctx.saved_tensors
         sums = _norm_sums(ctx.trainable, ctx.norm, s.shape[0])
         g2, g1, dy, dx, do = ops.block_steps().gpt2_out_bwd(dm, f, w2, w1, s, ln_w, stats, ds, wo, *sums)
         grads = (None,) * 8
         if ctx.trainable:
-            o2, y, h = ctx.saved_tensors[7:]
-            cap, (bo, b1, b2) = fused.current_capture(), ctx.biases
-            d2 = _weight_grads(cap, w2, b2, h, g2)
-            d1 = _weight_grads(cap, w1, b1, y, g1)
+            o2, y, h = trained
+            cap, (lo, l1, l2) = fused.current_capture(), ctx.linears
+            d2 = _weight_grads(cap, *l2, h, g2)
+            d1 = _weight_grads(cap, *l1, y, g1)
             dln = _layer_norm_param_grads(dy, s, ln_w, stats, ctx.norm, True) if sums[0] is None else (None, None)
-            grads = (*_weight_grads(cap, wo, bo, o2, dx), *dln, *d1, *d2)
+            grads = (*_weight_grads(cap, *lo, o2, dx), *dln, *d1, *d2)
         return (do.view(ctx.dims).transpose(1, 2), dx.view(dm.shape), *grads, None, None, None)
 
 
@@ -120,6 +120,7 @@ class LoRAIn(Function):
                                                                               cos, sin, nh, nkv, hd)
         ctx.save_for_backward(s, rstd, norm_w, y, xa, w_all, a_cat, b_block, aq, bq, ak, bk, av, bv, cos, sin)
         ctx.scaling, ctx.offset, ctx.carried, ctx.dims = scaling, norm[1], residual is not None, (B, T, d, nh, nkv, hd)
+        ctx.factors = (aq, bq), (ak, bk), (av, bv)
         v = qkv.view(B, T, nh + 2 * nkv, hd).narrow(2, nh + nkv, nkv)
         return q.transpose(1, 2), k.transpose(1, 2), v.transpose(1, 2), None if residual is None else s.view(B, T, d)
 
@@ -133,7 +134,7 @@ class LoRAIn(Function):
         cap = fused.current_capture()
         grads = (None,) * 6
         if cap is not None:
-            cap.add_lora_qkv(((aq, bq), (ak, bk), (av, bv)), y, xa, parts, q_all)
+            cap.add_lora_qkv(ctx.factors, y, xa, parts, q_all)
         else:
             r = aq.shape[0]
             grads = [t for j in range(3) for t in (q_all[:, j * r:(j + 1) * r].t() @ y, parts[j].t() @ xa[:, j * r:(j + 1) * r])]
@@ -153,6 +154,7 @@ class LoRAOut(Function):
         if keep:
             ctx.save_for_backward(s, rstd, norm_w, o2, xa, wo, a, b, g, u, w_gate, w_up, w_down)
             ctx.scaling, ctx.offset, ctx.act, ctx.dims = scaling, norm[1], act, (o.shape[0], o.shape[2], o.shape[1], o.shape[3])
+            ctx.factors = a, b
         return m.view(residual.shape), s.view(residual.shape)
 
     @staticmethod
@@ -163,7 +165,7 @@ class LoRAOut(Function):
         cap = fused.current_capture()
         da = db = None
         if cap is not None:
-            cap.add_lora(a, b, o2, xa, dx, q)
+            cap.add_lora(*ctx.factors, o2, xa, dx, q)
         else:
             da, db = q.t() @ o2, dx.t() @ xa
         return do.view(ctx.dims).transpose(1, 2), dx.view(dm.shape), None, da, db, None, None, None, None, None, None, None, None

@@ -114,6 +114,8 @@ class Capture:
         self.direct_elems = sp.direct_elems
 
     # ---- called from layer backward passes --------------------------------------------------
+    # Parameters are looked up as objects, so nodes hand over those that their forward pass was given (kept on ``ctx``): what
+    # ``ctx.saved_tensors`` returns under saved-tensor hooks (activation checkpointing, offloading) are other tensors.
     def _part(self, slot_name: str) -> torch.Tensor:
         i = len(self.part_slots)
         if i >= self.MAX_GHOST:
@@ -388,7 +390,7 @@ class _DPLinear(Function):
     @staticmethod
     def forward(ctx, x, weight, bias):
         ctx.save_for_backward(x, weight)
-        ctx.bias = bias
+        ctx.weight, ctx.bias = weight, bias
         ctx.own = _own_gemm_ok(x, weight, bias)
         if ctx.own:
             return ops.gemm(_rows(x), weight, bias=bias).view(*x.shape[:-1], weight.shape[0])
@@ -409,7 +411,7 @@ class _DPLinear(Function):
             dw = g2d.t() @ x2d
             db = g2d.sum(0) if ctx.bias is not None else None
             return dx, dw, db
-        cap.add_linear(weight, x2d, g2d)
+        cap.add_linear(ctx.weight, x2d, g2d)
         if ctx.bias is not None:
             if g2d.dtype == torch.bfloat16 and g2d.shape[1] % 8 == 0 and g2d.stride(0) % 8 == 0:
                 cap.sum_jobs.append((cap.pe_view(ctx.bias), g2d))        # g2d is kept for the weight gradient anyway
@@ -463,12 +465,12 @@ class _GLUUp(Function):
             return h.view(*x.shape[:-1], w_gate.shape[0])
         trainable = w_gate.requires_grad or w_up.requires_grad
         ctx.save_for_backward(g, u, w_gate, w_up, *((x2d,) if trainable else ()))
-        ctx.act, ctx.xshape, ctx.trainable = act, x.shape, trainable
+        ctx.act, ctx.xshape, ctx.trainable, ctx.weights = act, x.shape, trainable, (w_gate, w_up)
         return h.view(*x.shape[:-1], w_gate.shape[0])
 
     @staticmethod
     def backward(ctx, dh):
-        g, u, w_gate, w_up = ctx.saved_tensors[:4]
+        g, u, w_gate, w_up, *kept = ctx.saved_tensors
         inter = g.shape[1]
         d2 = dh.reshape(-1, inter)
         d2 = d2 if d2.is_contiguous() else d2.contiguous()
@@ -477,15 +479,14 @@ class _GLUUp(Function):
         if ctx.needs_input_grad[0]:
             dx = ops.gemm(dg, w_gate, b_layout="kn", a2=du, b2=w_up, b2_layout="kn").view(ctx.xshape)
         if ctx.trainable:
-            x2d = ctx.saved_tensors[4]
+            (x2d,) = kept
             cap = current_capture()
             if cap is None:
                 return dx, dg.t() @ x2d, du.t() @ x2d, None, None
             dgc, duc = dg.contiguous(), du.contiguous()
-            if w_gate.requires_grad:
-                cap.add_linear(w_gate, x2d, dgc)
-            if w_up.requires_grad:
-                cap.add_linear(w_up, x2d, duc)
+            for w, gw in zip(ctx.weights, (dgc, duc)):
+                if w.requires_grad:
+                    cap.add_linear(w, x2d, gw)
         return dx, None, None, None, None
 
 
@@ -525,12 +526,12 @@ class _GLUMLP(Function):
         y = ops.gemm(h, w_down)
         ctx.trainable = w_down.requires_grad
         ctx.save_for_backward(g, u, w_gate, w_up, w_down, *((x2d, h) if ctx.trainable else ()))
-        ctx.act, ctx.xshape = act, x.shape
+        ctx.act, ctx.xshape, ctx.weights = act, x.shape, (w_gate, w_up, w_down)
         return y.view(*x.shape[:-1], w_down.shape[0])
 
     @staticmethod
     def backward(ctx, dy):
-        g, u, w_gate, w_up, w_down = ctx.saved_tensors[:5]
+        g, u, w_gate, w_up, w_down, *kept = ctx.saved_tensors
         d2 = ops.functional._vec16(dy.reshape(-1, dy.shape[-1]))
         dg, du = glu_down_backward(d2, w_down, g, u, ctx.act)
         dx = None
@@ -538,10 +539,11 @@ class _GLUMLP(Function):
             dx = ops.gemm(dg, w_gate, b_layout="kn", a2=du, b2=w_up, b2_layout="kn").view(ctx.xshape)
         if not ctx.trainable:
             return dx, None, None, None, None
-        x2d, h = ctx.saved_tensors[5:]
+        x2d, h = kept
         cap = current_capture()
         if cap is None:
             return dx, dg.t() @ x2d, du.t() @ x2d, d2.t() @ h, None
+        w_gate, w_up, w_down = ctx.weights
         cap.add_linear(w_down, h, d2)
         cap.add_linear(w_gate, x2d, dg)
         cap.add_linear(w_up, x2d, du)
@@ -569,6 +571,7 @@ class _DPEmbedding(Function):
     @staticmethod
     def forward(ctx, ids, weight):
         ctx.save_for_backward(ids, weight)
+        ctx.weight = weight
         return torch.nn.functional.embedding(ids, weight)
 
     @staticmethod
@@ -580,7 +583,7 @@ class _DPEmbedding(Function):
         if cap is None:
             dw = torch.zeros_like(weight, dtype=torch.float32).index_add_(0, ids.reshape(-1), g2d.float())
             return None, dw.to(weight.dtype)
-        cap.add_embedding(weight, ids, g2d)
+        cap.add_embedding(ctx.weight, ids, g2d)
         return None, None
 
 
@@ -629,7 +632,7 @@ class _LoRALinear(Function):
             y = torch.nn.functional.linear(x2d, weight, bias)
             y.addmm_(xa, lora_b.t())
         ctx.save_for_backward(x2d, xa, weight, lora_a, lora_b)
-        ctx.scaling = scaling
+        ctx.scaling, ctx.factors = scaling, (lora_a, lora_b)
         ctx.xshape = x.shape
         return y.view(*x.shape[:-1], weight.shape[0])
 
@@ -661,7 +664,7 @@ class _LoRALinear(Function):
             xa_op = torch.zeros(R, LORA_PAD, dtype=xa.dtype, device=xa.device)
             xa_op[:, :r] = xa
         xc = x2d if x2d.is_contiguous() else x2d.contiguous()
-        cap.add_lora(lora_a, lora_b, xc, xa_op, g2d, q_op)
+        cap.add_lora(*ctx.factors, xc, xa_op, g2d, q_op)
         return dx, None, None, None, None, None
 
 
@@ -724,7 +727,7 @@ class _LoRAQKV(Function):
         xa = _small_gemm(x2d, a_cat, "nk", scaling)                             # [R, 3r], kept for the backward pass
         y = ops.gemm(x2d, w_all, a2=xa, b2=b_block, bias=bias_all)
         ctx.save_for_backward(x2d, xa, w_all, a_cat, b_block, aq, bq, ak, bk, av, bv)
-        ctx.scaling, ctx.xshape, ctx.outs = scaling, x.shape, outs
+        ctx.scaling, ctx.xshape, ctx.outs, ctx.factors = scaling, x.shape, outs, ((aq, bq), (ak, bk), (av, bv))
         q, k, v = torch.split(y, outs, dim=1)
         lead = x.shape[:-1]
         return q.unflatten(0, lead) if len(lead) > 1 else q, k.unflatten(0, lead) if len(lead) > 1 else k, \
@@ -747,7 +750,7 @@ class _LoRAQKV(Function):
             for j in range(3):
                 parts.append(g_all[:, lo:lo + outs[j]])
                 lo += outs[j]
-            cap.add_lora_qkv(((aq, bq), (ak, bk), (av, bv)), x2d, xa, parts, q_all)
+            cap.add_lora_qkv(ctx.factors, x2d, xa, parts, q_all)
             return (dx,) + (None,) * 9
         grads = []
         lo = 0

@@ -147,12 +147,12 @@ class _Experts(Function):
             wrow = topk_w.reshape(-1).index_select(0, slot_sorted).to(y.dtype)
             out = torch.zeros_like(x).index_add_(0, token_sorted, y * wrow[:, None])
             ctx.save_for_backward(xs, h, act, y, wrow, token_sorted, slot_sorted, offs, seg, w1, w2)
-        ctx.meta = (batch, tokens, topk_w.shape)
+        ctx.meta, ctx.weights = (batch, tokens, topk_w.shape), (w1, w2)
         return out
 
     @staticmethod
     def backward(ctx, dout):
-        xs, h, act, y, wrow, token_sorted, slot_sorted, offs, seg, w1, w2 = ctx.saved_tensors[:11]
+        xs, h, act, y, wrow, token_sorted, slot_sorted, offs, seg, w1, w2, *kept = ctx.saved_tensors
         batch, tokens, wshape = ctx.meta
         I = w2.shape[2]
         if ctx.rows:
@@ -161,7 +161,7 @@ class _Experts(Function):
             dact = grouped_linear(dy, w2, offs, transposed=True)
             dh = ops.functional.glu_backward_packed(dact, h)
             dxs = grouped_linear(dh, w1, offs, transposed=True)
-            dx = ops.functional.moe_combine(dxs, ctx.saved_tensors[11], wshape[1])
+            dx = ops.functional.moe_combine(dxs, kept[0], wshape[1])
         else:
             g = dout.index_select(0, token_sorted)
             dw_rows = (g.float() * y.float()).sum(-1)
@@ -177,8 +177,8 @@ class _Experts(Function):
         cap = fused.current_capture()
         if cap is not None:
             ex_row = (token_sorted // tokens).to(torch.int32)
-            cap.add_grouped_linear(w1, xs, dh, offs, seg, ex_row, tokens)
-            cap.add_grouped_linear(w2, act.contiguous(), dy, offs, seg, ex_row, tokens)
+            cap.add_grouped_linear(ctx.weights[0], xs, dh, offs, seg, ex_row, tokens)
+            cap.add_grouped_linear(ctx.weights[1], act.contiguous(), dy, offs, seg, ex_row, tokens)
             return dx, None, dtopk.to(wrow.dtype), None, None, None, None
         E = w1.shape[0]
         gw1, gw2 = torch.zeros_like(w1, dtype=torch.float32), torch.zeros_like(w2, dtype=torch.float32)

@@ -1,4 +1,5 @@
 """Fused DP engine vs a per-example autograd loop on tiny models; smoke of a full DP step (B200)."""
+import contextlib
 import math
 
 import pytest
@@ -385,3 +386,31 @@ def test_direct_norm_path_gives_the_same_clipped_step_as_the_ghost_path():
     (n_g, g_g), (n_d, g_d) = results["ghost"], results["direct"]
     assert torch.allclose(n_g, n_d, rtol=5e-3)
     assert float((g_g - g_d).norm() / (g_g.norm() + 1e-30)) < 1e-2
+
+
+@pytest.mark.parametrize("family", ["gpt2", "llama", "lora", "moe"])
+@pytest.mark.parametrize("how", ["checkpointing", "offloading"])
+def test_saved_tensor_hooks_under_a_capture(family, how):
+    """Recomputed or offloaded activations (``gradient_checkpointing``, ``activation_offloading``): the gradient of the plain step."""
+    from opaque_b200.engine.fused import FusedDPEngine
+    from opaque_b200.models import GPT2Config, GPT2LMHeadModel, LlamaConfig, LlamaForCausalLM, MoEConfig, MoEForCausalLM, shift_labels
+    from opaque_b200.random import key
+    results = []
+    for on in (False, True):
+        torch.manual_seed(0)
+        cls, cfg = {"gpt2": (GPT2LMHeadModel, GPT2Config), "moe": (MoEForCausalLM, MoEConfig)}.get(family, (LlamaForCausalLM, LlamaConfig))
+        model = cls(cfg.tiny(), device="cuda")
+        if family == "lora":
+            model.add_lora(8, 16.0)
+            for n, p in model.named_parameters():
+                if n.endswith("lora_B"):
+                    torch.nn.init.normal_(p, std=0.05)
+        model.activation_checkpointing = on and how == "checkpointing"
+        eng = FusedDPEngine(model, clipping_norm=1.0, noise_multiplier=0.0, normalize_by=2.0, key=key(0), microbatch_size=2)
+        ids = torch.randint(0, 200, (2, 64), device="cuda")
+        with torch.autograd.graph.save_on_cpu(pin_memory=True) if on and how == "offloading" else contextlib.nullcontext():
+            res = eng.accumulate(model.per_example_loss, {"input_ids": ids, "labels": shift_labels(ids)})
+        results.append((res.losses, res.norms, eng.space.grad.local.clone()))
+    # the same kernels on the same operands, or on recomputed ones that went through other fusions of the residual stream (bf16)
+    for a, b in zip(*results):
+        assert float((a - b).norm()) <= 1e-2 * float(a.norm()), float((a - b).norm() / a.norm())
