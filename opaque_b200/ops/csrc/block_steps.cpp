@@ -230,6 +230,7 @@ bool rope_reads(const Tensor& t) {
 }
 std::pair<Tensor, Tensor> rope(const Tensor& q, const Tensor& k, const Tensor& cs, const Tensor& sn) {
   const int64_t B = q.size(0), T = q.size(1), hd = q.size(3);
+  for (const Tensor* t : {&cs, &sn}) fit(t->dim() == 2 && t->size(0) >= T && t->size(1) == hd / 2, "rotary tables [positions, head size / 2] of too few positions");
   Tensor qo = empty({B, T, q.size(2), hd}, q), ko = empty({B, T, k.size(2), hd}, k);
   LAUNCH(ob_rope_qk_oop, ptr(q), ptr(k), ptr(qo), ptr(ko), f32(cs), f32(sn), nullptr, B * T, (int)T, (int)q.size(2), (int)k.size(2), (int)hd, q.stride(0),
          q.stride(1), q.stride(2), k.stride(0), k.stride(1), k.stride(2), 0, g_sms);

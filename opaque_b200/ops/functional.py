@@ -638,6 +638,8 @@ class _RoPE(Function):
 def rope_qk(q, k, cos, sin, pos=None):
     """Joint rotary embedding of Q ``[B, T, Hq, D]`` and K ``[B, T, Hk, D]``."""
     if _use_kernel(q, k) and q.shape[-1] % 4 == 0 and cos.dtype == torch.float32:
+        if pos is None and min(cos.shape[0], sin.shape[0]) < q.shape[-3]:
+            raise ValueError(f"rope_qk: tables of {min(cos.shape[0], sin.shape[0])} positions for sequences of {q.shape[-3]}")
         return _RoPE.apply(q, k, cos, sin, pos)
     return rope_qk_ref(q, k, cos, sin, pos)
 

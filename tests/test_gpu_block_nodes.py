@@ -303,3 +303,15 @@ def test_pitches_and_groups_that_are_refused():
         with pytest.raises(error):
             ops.wgrad_clip_batch([dict(a=a, b=a, **bad)], out)
     assert float(out.abs().max()) == 0.0
+
+
+def test_sequences_longer_than_the_rotary_tables():
+    from opaque_b200.models import LlamaConfig, LlamaForCausalLM
+    model = LlamaForCausalLM(LlamaConfig.tiny(), device="cuda")
+    ids = torch.zeros(1, 257, dtype=torch.int64, device="cuda")
+    for adapters in (False, True):                       # one node per operation, and two nodes
+        if adapters:
+            model.add_lora(8, 16.0)
+        with torch.no_grad(), pytest.raises(ValueError):
+            model.token_nll(ids, ids)
+        model.token_nll(ids[:, :256], ids[:, :256])
