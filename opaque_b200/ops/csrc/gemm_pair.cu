@@ -1306,12 +1306,12 @@ struct PairMaps {
 };
 
 // Tile of a plain product [rows, K] x [K, cols]: 256 x 256, or 512 x 256 where K is long.  A wave of the small tiles reads
-// (16 + 74 / 16) * 256 rows of K values; from K = 5632 on that no longer stays in one die's half of the L2 and the big tile's fewer
-// bytes per FLOP win (power-capped loops, TFLOP/s, big / small: 16384 x 4096 x 4096 1365 / 1368, 16384 x 4096 x 6144 1387 / 1336,
-// 16384 x 4096 x 14336 1422 / 1346), unless its coarser tiles leave more of the last wave empty (5439 x 2048 x 8192 1022 / 1141,
-// 8192 x 4096 x 14336, 7 waves for 2 x 4, 1333 / 1343).
+// (16 + 74 / 16) * 256 rows of K values; towards K = 5632 that no longer stays in one die's half of the L2 and the big tile's fewer
+// bytes per FLOP win (power-capped loops, TFLOP/s, big / small: 16384 x 14336 x 4608 1341 / 1361, x 5120 1346 / 1344, x 5632 1350 / 1324,
+// x 8192 1354 / 1284; 16384 x 5120 x 4608 1318 / 1326, x 5120 1318 / 1308, x 5632 1317 / 1294), unless its coarser tiles leave more of the
+// last wave empty (5439 x 2048 x 5120 958 / 1084, x 8192 972 / 1092; 8192 x 4096 x 14336, 7 waves for 2 x 4, 1333 / 1343).
 static bool pair_small_tile(long long rows, long long cols, long long K, int clusters) {
-  if (K <= 4096) return true;
+  if (K <= 4608) return true;
   const long long tn = (cols + GP_BN - 1) / GP_BN;
   const long long big = (rows + 2 * GP_BM - 1) / (2 * GP_BM) * tn, small = (rows + 2 * GD_BM - 1) / (2 * GD_BM) * tn;
   const long long waves_big = (big + clusters - 1) / clusters, waves_small = (small + clusters - 1) / clusters;
