@@ -7,8 +7,8 @@
 // (cluster rank 0) issues `tcgen05.mma.cta_group::2` (M = 256 across the pair) over both CTAs' shared memory, twice per
 // k-step: once for each 128-row half of a CTA's A tile, each half with its own 256-column accumulator in that CTA's tensor
 // memory.  Per k-block an SM stages 48 KB for 2 x (128 x 256 x 64) of tensor work: half the bytes per FLOP of a single-CTA
-// 128 x 256 tile, which pays under the power cap once K is long (see pair_small_tile).  All other products, and the activation
-// and cross-entropy epilogues, run on the 256 x 256 tiles of gemm_pair_db_kernel below.
+// 128 x 256 tile, which pays under the power cap once K is long (see pair_small_tile).  All other products, and the gated, activation
+// and cross-entropy epilogues, run on the 256 x 256 tiles of gemm_pair_db_kernel below, with the same protocol.
 //
 // Protocol (every wait bounded; a timeout records a code in the status word and the kernel unwinds):
 //   * full[s]  (leader only, 1 arrival + 96 KB of transactions): the leader's producer arms it for both CTAs' bytes;
@@ -19,9 +19,10 @@
 //     All warps drain half 0 first, then half 1, and the next tile begins with half-0 work (see the MMA issuer).
 // No copy in this file uses cluster multicast.
 //
-// Epilogues: plain store (+ bias), or GLU: the B halves come from TWO weight matrices (gate rows to rank 0, up rows to
-// rank 1), so every accumulator row holds 128 gate and 128 up pre-activations and the epilogue writes
-// act(gate) * up, optionally together with gate and up themselves for the backward pass.
+// Epilogues: plain store (+ bias) with either tile.  With the 256 x 256 tile also GLU: the B halves come from TWO weight matrices (gate
+// rows to rank 0, up rows to rank 1), so every accumulator row holds 128 gate and 128 up pre-activations and the epilogue
+// writes act(gate) * up, optionally together with gate and up themselves for the backward pass; a plain activation; the backward
+// of both; and the cross-entropy statistics of an output head.
 // Second K segment: LoRA (x A^T)(s B)^T in the forward pass, or the second operand pair of dX = dG Wg + dU Wu.
 //
 // Reference counterpart: the library GEMMs inside packages/opaque-patches/src/opaque/api/patches/kernels/lora.py:217-293
@@ -529,13 +530,10 @@ __device__ __forceinline__ void pair_epilogue(const PairParams& p, const CUtenso
   }
 }
 
-template <int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                 const __grid_constant__ CUtensorMap map_b_up, const __grid_constant__ CUtensorMap map_a2,
-                 const __grid_constant__ CUtensorMap map_b2, const __grid_constant__ CUtensorMap map_b2_up,
-                 const __grid_constant__ CUtensorMap map_out, const __grid_constant__ CUtensorMap map_out_gate,
-                 const __grid_constant__ CUtensorMap map_out_up, const PairParams p) {
+                 const __grid_constant__ CUtensorMap map_a2, const __grid_constant__ CUtensorMap map_b2,
+                 const __grid_constant__ CUtensorMap map_out, const PairParams p) {
   extern __shared__ uint8_t smem_raw[];
   // the dynamic shared-memory window starts at the same offset in both CTAs, so the rounded offsets agree too
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -552,7 +550,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   const int warp = uniform(static_cast<int>(threadIdx.x >> 5)), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const bool leader = rank == 0;
-  const int tiles_n = EPI == GP_EPI_GLU ? (p.N / 2 + GP_BNH - 1) / GP_BNH : (p.N + GP_BN - 1) / GP_BN;
+  const int tiles_n = (p.N + GP_BN - 1) / GP_BN;
   const int tiles_m = (p.M + 2 * GP_BM - 1) / (2 * GP_BM);
   const int total_work = tiles_m * tiles_n;
   const int nk1 = (p.K1 + GP_BK - 1) / GP_BK;
@@ -573,10 +571,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&map_a);
-    tma_prefetch_desc(rank == 1 && EPI == GP_EPI_GLU ? &map_b_up : &map_b);
+    tma_prefetch_desc(&map_b);
     if (nk2) {
       tma_prefetch_desc(&map_a2);
-      tma_prefetch_desc(rank == 1 && EPI == GP_EPI_GLU ? &map_b2_up : &map_b2);
+      tma_prefetch_desc(&map_b2);
     }
   }
   if (warp == 1) {                   // one warp of EACH CTA takes part in a pair allocation
@@ -601,12 +599,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
-    const CUtensorMap* mb1 = (EPI == GP_EPI_GLU && rank == 1) ? &map_b_up : &map_b;
-    const CUtensorMap* mb2 = (EPI == GP_EPI_GLU && rank == 1) ? &map_b2_up : &map_b2;
     for (int w = sc.first; ok && w < sc.end; w += sc.stride) {
       const GpItem it = gp_decode(w, tiles_m, tiles_n, rank, p.group_m);
       // first column of N (= row of a [N, K] operand) of this CTA's half of the B tile
-      const int bn0 = EPI == GP_EPI_GLU ? it.nt * GP_BNH : it.nt * GP_BN + static_cast<int>(rank) * GP_BNH;
+      const int bn0 = it.nt * GP_BN + static_cast<int>(rank) * GP_BNH;
       for (int kb = 0; kb < num_kb; ++kb) {
         if (!mbar_wait_warp(&empty[stage], phase ^ 1, abort_flag, p.status, OB_ERR_WAIT_EMPTY, budget)) {
           ok = false;
@@ -620,7 +616,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
           const bool first = kb < nk1;
           const int k0 = (first ? kb : kb - nk1) * GP_BK;
           tma_load_2d_pair(a_dst, first ? &map_a : &map_a2, bar, k0, it.row0);          // 256 rows x 64 k in one box
-          const CUtensorMap* mb = first ? mb1 : mb2;
+          const CUtensorMap* mb = first ? &map_b : &map_b2;
           if (first ? p.kn1 : p.kn2) {
 #pragma unroll
             for (int j = 0; j < GP_BNH / 64; ++j)
@@ -730,7 +726,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     uint8_t* slab = slabs + (warp - 2) * GP_SLAB_BYTES;
     int acc_iter = 0;
     bool ok = true;
-    const bool vec_ok = pair_vec_ok<EPI>(p);
+    const bool vec_ok = pair_vec_ok<GP_EPI_STORE>(p);
     for (int w = sc.first; ok && w < sc.end; w += sc.stride) {
       const GpItem it = gp_decode(w, tiles_m, tiles_n, rank, p.group_m);
       auto release_half = [&](int hh) {          // this warp is done READING accumulator half hh
@@ -750,7 +746,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         tc_fence_after();
         const int row = it.row0 + h * GP_MMA_M + q * 32 + lane;
         const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + h * GP_BN;
-        pair_epilogue<EPI>(p, map_out, map_out_gate, map_out_up, slab, t_row, row, it.nt, tiles_n, g, lane, vec_ok, [&] { release_half(h); });
+        pair_epilogue<GP_EPI_STORE>(p, map_out, map_out, map_out, slab, t_row, row, it.nt, tiles_n, g, lane, vec_ok, [&] { release_half(h); });
       }
       ++acc_iter;
     }
@@ -786,6 +782,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 // against 96 for the single-CTA 128 x 256 tile and 48 for the 512 x 256 pair tile.  It runs at the tensor pipe's rate: 8192 x 4096 x
 // 4096 in 167 us, 1.64 PFLOP/s, the library's own burst rate (big tile 182; 186 while one thread ran the issue loop).  Same
 // epilogues, barrier protocol and unwind rules as gemm_pair_kernel.
+// 320 threads leave 168 registers a thread (they are shared out as for 384), and ptxas spills in three forms (bytes stored / loaded a
+// thread: plain 76 / 144, cross-entropy 88 / 124, activation 52 / 156).  Once per tile that is at most 50 KB through L1, beside 32 KB
+// per k-block of operands: less than two k-blocks' worth, and it overlaps the next tile's.
 constexpr int GD_BM = 128;                              // rows of M per CTA (256 per pair)
 constexpr int GD_A_BYTES = GD_BM * GP_BK * 2;
 constexpr int GD_B_BYTES = GP_BNH * GP_BK * 2;
@@ -1322,25 +1321,27 @@ static bool pair_small_tile(long long rows, long long cols, long long K, int clu
 // 16384 x 4096 x 14336 2.87 -> 2.80 ms, 5439 x 2048 x 8192 0.312 -> 0.291; head + statistics 8192 x 2048 x 128256 3.42 -> 3.19 ms with
 // the logits stored, 3.48 -> 3.00 without; 3663 x 768 x 50304 0.332 -> 0.305).  The GLU backward's epilogue is longest of all
 // and exists for the small tile alone.
+template <class Kernel, class... Maps>
+static int pair_launch_on(Kernel kernel, int smem, int rows_tile, long long tiles_n, int* max_clusters, PairParams& p, int num_sms,
+                          cudaStream_t st, const Maps&... maps) {
+  if (*max_clusters == 0) {
+    if (cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -54;
+    *max_clusters = pair_grid(reinterpret_cast<const void*>(kernel), num_sms, smem);
+  }
+  const long long total = (static_cast<long long>(p.M) + rows_tile - 1) / rows_tile * tiles_n;
+  const int clusters = static_cast<int>(total < *max_clusters ? total : *max_clusters);
+  pair_set_schedule(&p, total, clusters, st);
+  kernel<<<2 * clusters, GP_THREADS, smem, st>>>(maps..., p);
+  return cudaGetLastError() == cudaSuccess ? 0 : -55;
+}
 template <int EPI>
 static int pair_launch(bool small, const PairMaps& m, PairParams& p, int num_sms, cudaStream_t st) {
-  using Kernel = decltype(&gemm_pair_db_kernel<GP_EPI_STORE>);
-  Kernel kernel;
-  if constexpr (EPI == GP_EPI_STORE) kernel = small ? gemm_pair_db_kernel<EPI> : gemm_pair_kernel<EPI>;
-  else kernel = gemm_pair_db_kernel<EPI>;
-  const int smem = small ? GdRing<EPI>::SMEM : GP_SMEM;
   static int max_clusters[2] = {0, 0};
-  if (max_clusters[small] == 0) {
-    if (cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -54;
-    max_clusters[small] = pair_grid(reinterpret_cast<const void*>(kernel), num_sms, smem);
-  }
-  const int rows_tile = small ? 2 * GD_BM : 2 * GP_BM;
   const long long tiles_n = EPI == GP_EPI_GLU ? (p.N / 2 + GP_BNH - 1) / GP_BNH : (p.N + GP_BN - 1) / GP_BN;
-  const long long total = (static_cast<long long>(p.M) + rows_tile - 1) / rows_tile * tiles_n;
-  const int clusters = static_cast<int>(total < max_clusters[small] ? total : max_clusters[small]);
-  pair_set_schedule(&p, total, clusters, st);
-  kernel<<<2 * clusters, GP_THREADS, smem, st>>>(m.a, m.b, m.b_up, m.a2, m.b2, m.b2_up, m.out, m.out_gate, m.out_up, p);
-  return cudaGetLastError() == cudaSuccess ? 0 : -55;
+  if constexpr (EPI == GP_EPI_STORE)
+    if (!small) return pair_launch_on(gemm_pair_kernel, GP_SMEM, 2 * GP_BM, tiles_n, &max_clusters[0], p, num_sms, st, m.a, m.b, m.a2, m.b2, m.out);
+  return pair_launch_on(gemm_pair_db_kernel<EPI>, GdRing<EPI>::SMEM, 2 * GD_BM, tiles_n, &max_clusters[1], p, num_sms, st, m.a, m.b, m.b_up, m.a2,
+                        m.b2, m.b2_up, m.out, m.out_gate, m.out_up);
 }
 }  // namespace ob
 

@@ -143,3 +143,9 @@ def test_plain_activation_epilogues(M, N, K, act, kernel):
         assert torch.equal(got.view(torch.int16), want.view(torch.int16))
     with pytest.raises(ValueError):
         ops.gemm_act_bwd(a, w[:, :-8].contiguous(), f[:, :-8].contiguous(), act=act)
+
+
+@pytest.mark.parametrize("M,N,K", [(300, 264, 4608), (513, 520, 4616), (2600, 1032, 4672)])
+def test_tiles_agree_around_the_line_between_them(M, N, K):
+    """The last K that always takes the small tile, and the first ones that weigh the waves of both."""
+    test_tiles_agree_bit_for_bit(M, N, K, "nk")
