@@ -245,11 +245,11 @@ def compare_cases(impl: str):
             xx = torch.randn(M, K, **bf)
             ww = torch.randn(N, K, **bf) * 0.02
             fl = 2.0 * M * N * K
-            emit(f"gemm x W^T, CTA pairs {M}x{N}x{K}", timeit(lambda: ops.gemm_pair(xx, ww, status=st), 20, 5, flush), flops=fl)
+            emit(f"gemm x W^T, CTA pairs (tile by size) {M}x{N}x{K}", timeit(lambda: ops.gemm_pair(xx, ww, status=st), 20, 5, flush), flops=fl)
             emit(f"gemm x W^T, single CTA {M}x{N}x{K}", timeit(lambda: ops.gemm(xx, ww, status=st, kernel="single"), 20, 5, flush), flops=fl)
             emit(f"library x W^T {M}x{N}x{K}", timeit(lambda: torch.matmul(xx, ww.t()), 20, 5, flush), flops=fl)
             wk = ww.t().contiguous()
-            emit(f"gemm dY W ([K,N] operand), CTA pairs {M}x{N}x{K}", timeit(lambda: ops.gemm_pair(xx, wk, b_layout="kn", status=st), 20, 5, flush), flops=fl)
+            emit(f"gemm dY W ([K,N] operand), CTA pairs (tile by size) {M}x{N}x{K}", timeit(lambda: ops.gemm_pair(xx, wk, b_layout="kn", status=st), 20, 5, flush), flops=fl)
             emit(f"library dY W {M}x{N}x{K}", timeit(lambda: torch.matmul(xx, wk), 20, 5, flush), flops=fl)
             del xx, ww, wk
         M, I, K = 16384, 14336, 4096
@@ -273,7 +273,7 @@ def pair_small_case():
     w = (torch.randn(N, K, device=dev) * 0.02).bfloat16()
     st = ops.StatusWord(dev)
     for _ in range(2):
-        y = ops.gemm_pair(x, w, status=st)
+        y = ops.gemm_pair(x, w, status=st, tile="512x256")
         y2 = ops.gemm_pair(x, w, status=st, tile="256x256")
         y3 = ops.gemm(x, w, status=st, kernel="single")
         h, g, u = ops.gemm_glu(x, w[: N // 2], w[N // 2:], status=st)
@@ -327,13 +327,13 @@ def short_k_case():
         mk = lambda f: [(lambda i=i: f(i)) for i in range(nset)]
         row["single_nk_bias"] = _graph_time(mk(lambda i: ops.gemm(xs[i], w, bias=b, out=outs[i], status=st, kernel="single")))
         row["pair256_nk_bias"] = _graph_time(mk(lambda i: ops.gemm_pair(xs[i], w, bias=b, out=outs[i], status=st, tile="256x256")))
-        row["pair512_nk_bias"] = _graph_time(mk(lambda i: ops.gemm_pair(xs[i], w, bias=b, out=outs[i], status=st)))
+        row["pair512_nk_bias"] = _graph_time(mk(lambda i: ops.gemm_pair(xs[i], w, bias=b, out=outs[i], status=st, tile="512x256")))
         row["library_nk_bias"] = _graph_time(mk(lambda i: torch.addmm(b, xs[i], w.t(), out=outs[i])))
         row["single_kn"] = _graph_time(mk(lambda i: ops.gemm(xs[i], wk, b_layout="kn", out=outs[i], status=st, kernel="single")))
         row["pair256_kn"] = _graph_time(mk(lambda i: ops.gemm_pair(xs[i], wk, b_layout="kn", out=outs[i], status=st, tile="256x256")))
-        row["pair512_kn"] = _graph_time(mk(lambda i: ops.gemm_pair(xs[i], wk, b_layout="kn", out=outs[i], status=st)))
+        row["pair512_kn"] = _graph_time(mk(lambda i: ops.gemm_pair(xs[i], wk, b_layout="kn", out=outs[i], status=st, tile="512x256")))
         row["library_kn"] = _graph_time(mk(lambda i: torch.matmul(xs[i], wk, out=outs[i])))
-        row["auto_pick"] = ops.pick_gemm_kernel(M, N, K)
+        row["auto_pick"] = ops.pick_gemm_plan(M, N, K)
         print(json.dumps({k: (round(v, 4) if isinstance(v, float) else v) for k, v in row.items()}), flush=True)
     if st.read():
         raise SystemExit(f"a device wait timed out (status {st.read()})")
@@ -419,12 +419,12 @@ def sustained_case(seconds: float = 2.5):
         w = (torch.randn(N, K, device=dev) * 0.02).bfloat16()
         wk = w.t().contiguous()
         fl = 2.0 * M * N * K
-        for name, fn in (("pair 512x256", lambda: ops.gemm_pair(x, w, status=st)), ("library", lambda: torch.matmul(x, w.t())),
+        for name, fn in (("pair 512x256", lambda: ops.gemm_pair(x, w, status=st, tile="512x256")), ("library", lambda: torch.matmul(x, w.t())),
                          ("pair 256x256", lambda: ops.gemm_pair(x, w, status=st, tile="256x256")),
                          ("single CTA", lambda: ops.gemm(x, w, status=st, kernel="single")),
                          ("gate+up+SwiGLU fused", lambda: ops.gemm_glu(x, w[: N // 2], w[N // 2:], status=st)),
                          ("two library GEMMs + SwiGLU kernel", lambda: ops.swiglu(torch.matmul(x, w[: N // 2].t()), torch.matmul(x, w[N // 2:].t()))),
-                         ("pair 512x256, [K,N] operand", lambda: ops.gemm_pair(x, wk, b_layout="kn", status=st)),
+                         ("pair 512x256, [K,N] operand", lambda: ops.gemm_pair(x, wk, b_layout="kn", status=st, tile="512x256")),
                          ("library, [K,N] operand", lambda: torch.matmul(x, wk))):
             ms, clk, pw = sample(fn)
             print(json.dumps({"case": "sustained", "shape": [M, N, K], "kernel": name, "tflops": round(fl / ms / 1e9), "sm_mhz": clk,

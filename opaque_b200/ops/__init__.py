@@ -670,25 +670,6 @@ def linear_ce_dlogits_(logits: torch.Tensor, labels: torch.Tensor, lse: torch.Te
     return logits
 
 
-def pick_gemm_kernel(M: int, N: int, K: int, sms: int = 148) -> str:
-    """``"pair"`` or ``"single"`` between the 512 x 256 pair tile and the single-CTA kernel (:func:`gemm` asks :func:`pick_gemm_plan`,
-    which knows the smaller pair tile).
-
-    The pair kernel (512 x 256 output tiles on SM pairs, half the operand bytes per FLOP) wins on large products; its
-    tiles are coarse, so a product with few tiles or a short K leaves SM pairs idle in the last wave or pays the
-    un-overlapped part of its epilogue too often.  The estimate is work / (waves x capacity), times the measured
-    steady-state rate of each kernel, times K / (K + per-tile overhead in k).
-    """
-    clusters = max(sms // 2, 1)
-    t_pair = -(-M // 512) * -(-N // 256)
-    t_single = -(-M // 128) * -(-N // 256)
-    # constants fitted to sustained runs: single-CTA steady rate 0.93 of the pair kernel's; un-overlapped part of a tile
-    # worth about 128 (pair: one tile fills tensor memory) and 48 (single: double-buffered accumulators) elements of K
-    eff_pair = t_pair / (-(-t_pair // clusters) * clusters) * (K / (K + 128.0))
-    eff_single = 0.93 * t_single / (-(-t_single // sms) * sms) * (K / (K + 48.0))
-    return "pair" if eff_pair >= eff_single else "single"
-
-
 def _waves_us(tiles: int, slots: int, nk: int, start: float, per_kb: float, per_busy: float, per_tile: float) -> float:
     """``start`` plus, for every wave of ``tiles`` over ``slots``, ``nk`` k-blocks (dearer the more slots are busy) and a tile's own cost."""
     full, rest = divmod(tiles, slots)
@@ -995,7 +976,7 @@ from .functional import (activation, add_layer_norm, cross_entropy, cross_entrop
                          layer_norm, merge_heads3, plain_torch_ops, rms_norm, rms_norm_ref, rope_qk, rope_qk_ref, rope_tables, rows_group_sum_, swiglu)
 
 __all__ = [
-    "gemm", "gemm_pair", "block_steps", "lora_pack", "pick_gemm_plan", "gemm_glu", "gemm_glu_bwd", "pick_glu_bwd", "gemm_act", "gemm_act_bwd", "direct_norm2", "pick_norm_path", "pick_gemm_kernel", "die_map", "set_die_aware_tiles", "linear_ce_forward", "linear_ce_dlogits_", "gemm_glu_ref", "gemm_ref", "ghost_set_wide", "push_grad_", "wgrad_clip_per_example", "wgrad_clip_batch", "wgrad_clip_per_example_batch", "direct_norm2_batch", "ghost_norm_batch", "plain_torch_ops", "layer_norm", "add_layer_norm", "activation", "rows_group_sum_", "merge_heads3",
+    "gemm", "gemm_pair", "block_steps", "lora_pack", "pick_gemm_plan", "gemm_glu", "gemm_glu_bwd", "pick_glu_bwd", "gemm_act", "gemm_act_bwd", "direct_norm2", "pick_norm_path", "die_map", "set_die_aware_tiles", "linear_ce_forward", "linear_ce_dlogits_", "gemm_glu_ref", "gemm_ref", "ghost_set_wide", "push_grad_", "wgrad_clip_per_example", "wgrad_clip_batch", "wgrad_clip_per_example_batch", "direct_norm2_batch", "ghost_norm_batch", "plain_torch_ops", "layer_norm", "add_layer_norm", "activation", "rows_group_sum_", "merge_heads3",
     "DeviceWaitTimeout", "KernelLibraryError", "StatusWord", "clip_tree", "clip_weighted_sum", "cross_entropy",
     "cross_entropy_ref", "embedding_wgrad", "fused_add_rms_norm", "geglu", "ghost_norm", "ghost_norm_ref", "glu_ref",
     "philox_normal_add_", "pick_block_n", "pick_splits", "rms_norm", "rms_norm_ref", "rope_qk", "rope_qk_ref",

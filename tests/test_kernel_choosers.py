@@ -2,16 +2,40 @@
 from opaque_b200 import ops
 
 
-def test_gemm_kernel_choice_follows_tile_fill_and_k():
-    # long K and enough 512 x 256 tiles for every SM pair: CTA pairs
-    for shape in [(16384, 4096, 4096), (16384, 14336, 4096), (16384, 4096, 14336), (16384, 6144, 4096), (16384, 1024, 4096)]:
-        assert ops.pick_gemm_kernel(*shape) == "pair", shape
-    # short K (the big tile's drain is not amortised) or too few pair tiles: single CTA
-    for shape in [(16384, 2304, 768), (16384, 768, 768), (16384, 3072, 768), (16384, 768, 3072), (2048, 512, 4096)]:
-        assert ops.pick_gemm_kernel(*shape) == "single", shape
-    # the answer depends on the SM count it is asked for (a full last wave of pair tiles), not on a device being present
-    assert ops.pick_gemm_kernel(16384, 4096, 4096, sms=148) in ("pair", "single")
-    assert ops.pick_gemm_kernel(512, 256, 64, sms=148) in ("pair", "single")
+def test_gemm_plan_takes_the_kernel_that_measured_faster():
+    # both sides of the crossover in width at 3663 rows, and in size: (pair, single) us 18.7 / 20.5 and 10.3 / 9.3, 42.1 / 27.3 and 167 / 182
+    assert ops.pick_gemm_plan(3663, 3072, 768) == "pair" and ops.pick_gemm_plan(3663, 768, 768) == "single"
+    assert ops.pick_gemm_plan(256, 2048, 8192) == "single" and ops.pick_gemm_plan(8192, 4096, 4096) == "pair"
+    # large products run on pairs at any K, products of few tiles on single CTAs
+    for shape in [(16384, 4096, 4096), (16384, 14336, 4096), (16384, 4096, 14336), (16384, 2304, 768), (16384, 768, 3072)]:
+        assert ops.pick_gemm_plan(*shape) == "pair", shape
+    for shape in [(1, 8, 64), (128, 768, 768), (2048, 512, 4096), (16384, 48, 4096)]:
+        assert ops.pick_gemm_plan(*shape) == "single", shape
+    # a second K segment counts as its k-blocks
+    assert ops.pick_gemm_plan(3663, 768, 704, 64) == ops.pick_gemm_plan(3663, 768, 768)
+
+
+def test_tile_width_of_the_single_cta_kernel():
+    assert ops.pick_tile_width(16384, 48, 64) == 64 and ops.pick_tile_width(16384, 64, 64) == 64      # one narrow tile covers the columns
+    assert ops.pick_tile_width(128, 768, 12) == 64 and ops.pick_tile_width(128, 2048, 128) == 64      # all narrow tiles at once, and faster
+    assert ops.pick_tile_width(3663, 768, 12) == 256                                                  # beyond one wave
+
+
+def test_plan_code_is_the_plan_and_knows_activations(monkeypatch):
+    monkeypatch.setattr(ops.lib, "sm_count", lambda *a: 148)
+    for shape in [(3663, 3072, 768), (3663, 768, 768), (128, 768, 768), (16384, 768, 3072), (512, 256, 64), (1, 8, 64)]:
+        code = ops._plan_code(*shape, 0, 0)
+        assert (code == 0) == (ops.pick_gemm_plan(*shape) == "pair")
+        assert code in (0, ops.pick_tile_width(shape[0], shape[1], -(-shape[2] // 64)))
+        assert ops._plan_code(*shape, 0, 1) == ops.pick_tile_width(shape[0], shape[1], -(-shape[2] // 64))      # single CTAs only
+    # with an activation: 64-column tiles for few rows, pairs from where they measured faster (1285 rows: 14.2 us against 19.0)
+    assert [ops._plan_code(rows, 3072, 768, 0, 2) for rows in (128, 512, 1285, 3663, 16384)] == [64, 64, 0, 0, 0]
+
+
+def test_gated_backward_runs_in_the_epilogue_beyond_one_wave():
+    assert not ops.pick_glu_bwd(128, 8192) and not ops.pick_glu_bwd(597, 5632)
+    assert ops.pick_glu_bwd(1024, 14336) and ops.pick_glu_bwd(5439, 8192)
+    assert not ops.pick_glu_bwd(256, 74 * 256) and ops.pick_glu_bwd(256, 74 * 256 + 1)                # 74 SM pairs
 
 
 def test_norm_path_choice_crosses_over_with_sequence_length():
