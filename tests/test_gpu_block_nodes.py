@@ -315,3 +315,85 @@ def test_sequences_longer_than_the_rotary_tables():
         with torch.no_grad(), pytest.raises(ValueError):
             model.token_nll(ids, ids)
         model.token_nll(ids[:, :256], ids[:, :256])
+
+
+def _attention(q, k, v, is_causal=True, enable_gqa=False, scale=None):
+    """Attention whose backward pass gives the same bits every time (the library's varies)."""
+    B, H, T, hd = q.shape
+    if enable_gqa:
+        k, v = (t[:, :, None].expand(B, t.shape[1], H // t.shape[1], T, hd).reshape(B, H, T, hd) for t in (k, v))
+    s = (q @ k.transpose(2, 3)).float() * (hd ** -0.5 if scale is None else scale)
+    s = s.masked_fill(torch.ones(T, T, dtype=torch.bool, device=q.device).triu(1), float("-inf"))
+    return torch.softmax(s, -1).to(v.dtype) @ v
+
+
+@pytest.mark.parametrize("family,B,T", [("gpt2", 2, 64), ("gpt2", 3, 77), ("gpt2", 17, 250), ("llama", 2, 64), ("llama", 3, 77)])
+def test_same_operands_and_every_gradient(family, B, T, monkeypatch):
+    """With an attention that repeats its bits: what a pass hands to the capture is equal bit for bit, in the same order, and the gradient of
+    every parameter by itself differs by no more than the order of its fp32 sums.
+
+    The sums' terms are the same; a value of n terms moves by at most sqrt(n) 2^-24 of their size (n up to 4250 rows), and ten times that
+    allows for the terms that cancel."""
+    from opaque_b200.engine.fused import Capture, FusedDPEngine
+    from opaque_b200.models import GPT2Config, GPT2LMHeadModel, LlamaConfig, LlamaForCausalLM, shift_labels
+    from opaque_b200.random import key
+    monkeypatch.setattr(torch.nn.functional, "scaled_dot_product_attention", _attention)
+    handed, results = [], []                             # per run: (method, its operands without the parameters)
+    for name in ("add_linear", "add_embedding", "add_lora", "add_lora_qkv"):
+        def spy(self, *a, f=getattr(Capture, name), name=name):
+            flat = [t for x in a for t in (x if isinstance(x, (tuple, list)) else (x,)) if isinstance(t, torch.Tensor) and not isinstance(t, torch.nn.Parameter)]
+            handed[-1].append((name, [t.clone() for t in flat]))
+            return f(self, *a)
+        monkeypatch.setattr(Capture, name, spy)
+    for unsplit in (False, True):
+        handed.append([])
+        torch.manual_seed(T)
+        model = (GPT2LMHeadModel(GPT2Config.tiny(), device="cuda") if family == "gpt2" else LlamaForCausalLM(LlamaConfig.tiny(), device="cuda"))
+        if family == "llama":
+            model.add_lora(8, 16.0)
+        for n, p in model.named_parameters():
+            if n.endswith(("bias", "lora_B")):
+                torch.nn.init.normal_(p, std=0.1)
+        for blk in (model.h if family == "gpt2" else model.model.layers) if unsplit else ():
+            (blk.mlp_c_fc if family == "gpt2" else blk.mlp.down_proj).register_forward_hook(lambda *a: None)
+        eng = FusedDPEngine(model, clipping_norm=1.0, noise_multiplier=0.0, normalize_by=2.0, key=key(0), microbatch_size=B)
+        ids = torch.randint(0, 256, (B, T), device="cuda")
+        res = eng.accumulate(model.per_example_loss, {"input_ids": ids, "labels": shift_labels(ids)})
+        results.append((res, {n: eng.space.grad.local[s.offset:s.offset + s.numel].clone() for n, s in eng.space.slots.items()}))
+    two, one = handed
+    assert [n for n, _ in two] == [n for n, _ in one] and len(two) >= 4
+    for (name, a), (_, b) in zip(two, one):
+        assert len(a) == len(b) and all(torch.equal(x, y) for x, y in zip(a, b)), name
+    assert torch.equal(results[0][0].losses, results[1][0].losses)
+    for name, g in results[0][1].items():
+        ref = results[1][1][name]
+        assert float((g - ref).norm()) <= 10 * (B * T) ** 0.5 * 2 ** -24 * float(ref.norm()), (name, float((g - ref).norm() / ref.norm()))
+
+
+@pytest.mark.parametrize("family", ["gpt2", "llama"])
+@pytest.mark.parametrize("carried", [False, True])
+def test_gradients_through_frozen_weights_bit_for_bit(family, carried, monkeypatch):
+    """Data gradients of a block, and the factors' without a capture, with fixed incoming gradients and a repeatable attention."""
+    from opaque_b200.models import GPT2Config, GPT2LMHeadModel, LlamaConfig, LlamaForCausalLM
+    monkeypatch.setattr(torch.nn.functional, "scaled_dot_product_attention", _attention)
+    torch.manual_seed(0)
+    model = (GPT2LMHeadModel(GPT2Config.tiny(), device="cuda").requires_grad_(False) if family == "gpt2" else LlamaForCausalLM(LlamaConfig.tiny(), device="cuda"))
+    if family == "llama":
+        model.add_lora(8, 16.0)
+    for n, p in model.named_parameters():
+        if n.endswith(("bias", "lora_B")):
+            torch.nn.init.normal_(p, std=0.1)
+    block, args = (model.h[0], ()) if family == "gpt2" else (model.model.layers[0], (model.rope_cos, model.rope_sin, None))
+    x, r, gm, gs = (torch.randn(3, 77, 128, device="cuda", dtype=torch.bfloat16) for _ in range(4))
+    results = []
+    for unsplit in (False, True):
+        hook = (block.mlp_c_fc if family == "gpt2" else block.mlp.down_proj).register_forward_hook(lambda *a: None) if unsplit else None
+        xx, rr = x.clone().requires_grad_(True), (r.clone().requires_grad_(True) if carried else None)
+        out = block.forward_carried(xx, rr, *args)
+        inputs = [xx] + ([rr] if carried else []) + [p for p in block.parameters() if p.requires_grad]
+        results.append([*out, *torch.autograd.grad(out, inputs, (gm, gs))])
+        if hook is not None:
+            hook.remove()
+    assert len(results[0]) >= 3
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
