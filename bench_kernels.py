@@ -264,8 +264,9 @@ def compare_cases(impl: str):
 
 def pair_small_case():
     """Two rounds of one launch each: CTA-pair GEMM (512 x 256 tiles), its 256 x 256 variant, the single-CTA kernel, the
-    gated up-projection and the library GEMM on y[8192, 8192] = x[8192, 4096] W^T (inputs + output 192 MB > L2).  A small
-    case for counter captures (one launch per kernel and round; nothing is timed here)."""
+    gated up-projection and the library GEMM on y[8192, 8192] = x[8192, 4096] W^T (inputs + output 192 MB > L2), and on half of
+    its columns the GELU epilogue, its backward and the gated backward.  A small case for counter captures (one launch per
+    kernel and round; nothing is timed here)."""
     from opaque_b200 import ops
     dev = torch.device("cuda", 0)
     M, N, K = 8192, 8192, 4096
@@ -277,6 +278,9 @@ def pair_small_case():
         y2 = ops.gemm_pair(x, w, status=st, tile="256x256")
         y3 = ops.gemm(x, w, status=st, kernel="single")
         h, g, u = ops.gemm_glu(x, w[: N // 2], w[N // 2:], status=st)
+        ops.gemm_act(x, w[: N // 2], status=st, kernel="pair")
+        ops.gemm_act_bwd(x, w[: N // 2], g, status=st, kernel="pair")
+        ops.gemm_glu_bwd(x, w[: N // 2], g, u, status=st)
         ref = torch.matmul(x, w.t())
     torch.cuda.synchronize()
     if st.read():
@@ -555,6 +559,15 @@ def main():
         xl = torch.randn(rows_l, 768, device=dev).bfloat16()
         wl, bl = torch.ones(768, device=dev).bfloat16(), torch.zeros(768, device=dev).bfloat16()
         emit(f"layer_norm fwd {rows_l}x768", timeit(lambda: ops.layer_norm(xl, wl, bl), iters, warm, flush), bytes_=2 * xl.numel() * 2)
+        # the blocks' form: residual added in the norm, and its backward with the per-example weight and bias sums of 512-row examples
+        rl, ds, dx, E = torch.randn_like(xl), torch.randn_like(xl), torch.empty_like(xl), rows_l // 512
+        stats, pe = torch.rand(2, rows_l, device=dev), torch.zeros(E, 2 * 768, device=dev)
+        emit(f"add_layer_norm fwd {rows_l}x768", timeit(lambda: ops.add_layer_norm(xl, rl, wl, bl), iters, warm, flush), bytes_=4 * xl.numel() * 2)
+        emit(f"add_layer_norm bwd with sums {rows_l}x768",
+             timeit(lambda: ops.lib.check(ops.lib.load().ob_layernorm_bwd_sums(
+                 rl.data_ptr(), xl.data_ptr(), wl.data_ptr(), stats[0].data_ptr(), stats[1].data_ptr(), ds.data_ptr(), dx.data_ptr(), E, 512, 768,
+                 pe.data_ptr(), pe.data_ptr() + 4 * 768, pe.stride(0), ops.lib.stream()), "layernorm_bwd_sums"), iters, warm, flush),
+             bytes_=4 * xl.numel() * 2)
     if want("swiglu"):
         rows = 4096 if args.small else 16384
         g = torch.randn(rows, 14336, device=dev).bfloat16()
