@@ -26,7 +26,7 @@ def available() -> bool:
 
 def one_stream(x, residual) -> bool:
     """Whether the two parts of a split stream are of one kind; a node's kernels read both the same way."""
-    return residual is None or (residual.shape == x.shape and residual.dtype == x.dtype and residual.device == x.device)
+    return residual is None or (residual.dtype is x.dtype and residual.is_cuda and residual.is_same_size(x))
 
 
 def _weight_grads(cap, weight, bias, x2d, g2d):
