@@ -515,8 +515,10 @@ static int launch_ghost(const TmaBatch<GhostParams, CAP>& b, bool wide, int num_
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }
 
-// measured: the wide blocks win from about 1024 rows per example (less wasted work below the diagonal); below that the
-// 128 x 128 blocks with double-buffered accumulators are as fast or faster
+// The line was drawn where the wide blocks won while one thread issued copies and MMAs (from about 1024 rows per example).  Issued by
+// whole warps, the 128 x 128 blocks with their double-buffered accumulators win at 1024 rows as well, and the two are even from about 2048
+// on (us, 128 x 128 / 128 x 256: 8 x 1024 x 2048 x 2048 33.7 / 50.5, 8 x 1024 x 2048 x 8192 79 / 116, 4 x 1300 x 2048 x 2048 32 / 50,
+// 4 x 2048 x 2048 x 1408 52 / 52, 2 x 4096 x 768 x 3072 114 / 109).
 static bool ghost_use_wide(int T) {
   const int nt = (T + GH_TILE - 1) / GH_TILE;
   return wide_enabled == 2 ? nt >= 2 : (wide_enabled == 1 && nt >= 8);
