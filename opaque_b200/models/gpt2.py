@@ -102,13 +102,13 @@ class GPT2Block(nn.Module):
         if trained and fused.current_capture() is None:
             return False
         for lin in linears:
-            w, b = lin._parameters["weight"], lin.bias
-            if lin.lora_A is not None or b is None or w.requires_grad != trained or b.requires_grad != trained \
+            w, b = lin._parameters.get("weight"), lin._parameters.get("bias")          # None: no parameter of the module
+            if lin.lora_A is not None or w is None or b is None or w.requires_grad != trained or b.requires_grad != trained \
                     or not fused._own_gemm_ok(x, w, b):
                 return False
         for norm in (m["ln_1"], m["ln_2"]):
-            w, b = norm._parameters["weight"], norm.bias
-            if b is None or w.requires_grad != trained or b.requires_grad != trained or w.dtype != torch.bfloat16 or b.dtype != torch.bfloat16:
+            w, b = norm._parameters.get("weight"), norm._parameters.get("bias")
+            if w is None or b is None or w.requires_grad != trained or b.requires_grad != trained or w.dtype != torch.bfloat16 or b.dtype != torch.bfloat16:
                 return False
         return x.shape[-1] % 8 == 0 and x.shape[-1] <= 1024
 

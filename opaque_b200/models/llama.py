@@ -325,13 +325,13 @@ class LlamaDecoderLayer(nn.Module):
             return False
         r, scaling = q.lora_A.shape[0], q.scaling
         for i, lin in enumerate(adapted):
-            w, a, b = lin._parameters["weight"], lin.lora_A, lin.lora_B
-            if a is None or lin.bias is not None or w.requires_grad or not fused.lora_factors_ok(a, b) or not w.is_contiguous() \
+            w, a, b = (lin._parameters.get(k) for k in ("weight", "lora_A", "lora_B"))         # None: no parameter of the module
+            if w is None or a is None or b is None or lin.bias is not None or w.requires_grad or not fused.lora_factors_ok(a, b) or not w.is_contiguous() \
                     or not fused._own_gemm_ok(x, w) or (i < 3 and (a.shape[0] != r or lin.scaling != scaling)):
                 return False
         for lin in plain:
-            w = lin._parameters["weight"]
-            if lin.lora_A is not None or lin.bias is not None or w.requires_grad or not fused._own_gemm_ok(x, w):
+            w = lin._parameters.get("weight")
+            if w is None or lin.lora_A is not None or lin.bias is not None or w.requires_grad or not fused._own_gemm_ok(x, w):
                 return False
         wg, wu, wd = (lin._parameters["weight"] for lin in plain)
         return (wg.shape == wu.shape and wg.stride(0) == wu.stride(0) and wd.shape[1] == wg.shape[0] and wg.shape[0] % 64 == 0

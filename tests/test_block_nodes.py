@@ -63,6 +63,26 @@ def test_gpt2_blocks_that_override_a_part():
     assert not block._two_nodes(x)
 
 
+def _as_plain_tensor(module, name):
+    t = getattr(module, name).detach()
+    delattr(module, name)
+    setattr(module, name, t)
+
+
+@pytest.mark.parametrize("path,name", [("self_attn.q_proj", "weight"), ("self_attn.o_proj", "lora_B"), ("self_attn.k_proj", "lora_A"), ("mlp.down_proj", "weight")])
+def test_llama_blocks_with_plain_tensors_for_parameters(path, name):
+    layer, two_nodes = _layer()
+    _as_plain_tensor(layer.get_submodule(path), name)
+    assert not two_nodes()
+
+
+@pytest.mark.parametrize("path,name", [("attn_c_attn", "bias"), ("mlp_c_proj", "weight"), ("ln_2", "weight")])
+def test_gpt2_blocks_with_plain_tensors_for_parameters(path, name):
+    block = GPT2LMHeadModel(GPT2Config.tiny()).requires_grad_(False).h[0]
+    _as_plain_tensor(getattr(block, path), name)
+    assert not block._two_nodes(torch.zeros(1, 8, 128, dtype=torch.bfloat16))
+
+
 def test_exceptions_of_the_compiled_sequences_keep_their_type():
     """What torch's own call raises in Python: an IndexError here, as torch.OutOfMemoryError where an allocation fails."""
     import importlib.util
